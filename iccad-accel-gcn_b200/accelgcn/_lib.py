@@ -22,6 +22,7 @@ _vp, _i64, _int = ctypes.c_void_p, ctypes.c_int64, ctypes.c_int
 PROTOTYPES = {
     "agcn_last_error": (ctypes.c_char_p, []),
     "agcn_version": (_int, []),
+    "agcn_release_scratch": (_int, []),
     "agcn_partition_device": (_int, [_vp, _i64, _vp, _i64, ctypes.POINTER(_i64), _vp]),
     "agcn_partition_host": (_int, [_vp, _i64, _vp, _i64, ctypes.POINTER(_i64)]),
     "agcn_partition_device_noalloc": (_int, [_vp, _i64, _vp, _i64, ctypes.POINTER(_i64), _vp]),

@@ -22,7 +22,7 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
 
     const int64_t tiles = ceil_div(n_rows, SORT_TILE);
     const int64_t hist_len = tiles * RADIX_BINS;
-    DeviceScratch scratch;
+    DeviceScratch scratch(s);
     AGCN_ALLOC(keys_a, scratch, unsigned, n_rows + 1);
     AGCN_ALLOC(keys_b, scratch, unsigned, n_rows + 1);
     AGCN_ALLOC(rows_a, scratch, int, n_rows);
@@ -118,7 +118,7 @@ extern "C" int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_i
     const bool want_idx = h_new_indices != nullptr, want_val = h_new_vals != nullptr;
     AGCN_REQUIRE(!want_idx || (h_indices != nullptr && h_new_indptr != nullptr), "agcn_degree_sort_host: new_indices needs indices and new_indptr");
     AGCN_REQUIRE(!want_val || (h_vals != nullptr && want_idx), "agcn_degree_sort_host: new_vals needs vals and new_indices");
-    DeviceScratch scratch;
+    DeviceScratch scratch(nullptr);
     AGCN_ALLOC(d_indptr, scratch, int, n_rows + 1);
     AGCN_ALLOC(d_perm, scratch, int, n_rows);
     AGCN_ALLOC(d_new_indptr, scratch, int, n_rows + 1);

@@ -222,7 +222,7 @@ static int dist_set_graph(agcn_dist *d, const int *d_indptr, const int *d_indice
         AGCN_CUDA(cudaMemcpyAsync(d->val + light_nz, d_vals + h_indptr[L.heavy0[g]], (size_t)heavy_nz * 4, cudaMemcpyDeviceToDevice, s));
     }
     // column ids -> positions in the gathered operand
-    DeviceScratch scratch;
+    DeviceScratch scratch(s);
     AGCN_ALLOC(d_err, scratch, int, 1);
     AGCN_CUDA(cudaMemsetAsync(d_err, 0, sizeof(int), s));
     if (d->local_nnz > 0) {

@@ -45,35 +45,89 @@ void clear_error();
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// Device allocations that free themselves when the call returns.
+// Stream-ordered memory of the current device's pool (memory.cu).
+cudaError_t pool_alloc(void **out, size_t bytes, cudaStream_t s);
+void pool_free(void *p, cudaStream_t s);
+// for blocks that work on any stream may still use: waits for the device, as cudaFree does
+void pool_free_waiting(void *p);
+
+// Pool memory for the length of a call, used and given back on one stream.
 class DeviceScratch {
 public:
-    DeviceScratch() = default;
+    explicit DeviceScratch(cudaStream_t s) : s_(s) {}
     DeviceScratch(const DeviceScratch &) = delete;
     DeviceScratch &operator=(const DeviceScratch &) = delete;
-    ~DeviceScratch() { for (void *p : ptrs_) cudaFree(p); }
+    ~DeviceScratch() { for (void *p : ptrs_) pool_free(p, s_); }
     // returns nullptr (and records the error) on failure
     template <typename T> T *alloc(int64_t count)
     {
         void *p = nullptr;
         const size_t bytes = (size_t)(count > 0 ? count : 1) * sizeof(T);
-        cudaError_t e = cudaMalloc(&p, bytes);
+        cudaError_t e = pool_alloc(&p, bytes, s_);
         if (e != cudaSuccess) {
-            set_error("cudaMalloc(%zu bytes): %s", bytes, cudaGetErrorString(e));
+            set_error("device allocation of %zu bytes: %s", bytes, cudaGetErrorString(e));
             return nullptr;
         }
         ptrs_.push_back(p);
         return static_cast<T *>(p);
     }
 private:
+    cudaStream_t s_;
     std::vector<void *> ptrs_;
 };
+
+// Lays several arrays out in one allocation, each on a 256-byte boundary: take() every array first with a
+// null base to get the size, then again with the block.
+class Carver {
+public:
+    explicit Carver(void *base = nullptr) : base_(static_cast<unsigned char *>(base)) {}
+    template <typename T> T *take(int64_t count)
+    {
+        T *p = base_ != nullptr ? reinterpret_cast<T *>(base_ + used_) : nullptr;
+        used_ += ((size_t)(count > 0 ? count : 0) * sizeof(T) + 255) & ~(size_t)255;
+        return p;
+    }
+    size_t bytes() const { return used_; }
+private:
+    unsigned char *base_;
+    size_t used_ = 0;
+};
+
+// Words in pinned host memory that kernels store results and error codes into (memory.cu).
+struct HostWords {
+    enum { COUNT = 6 };
+    int64_t w[COUNT];
+};
+
+class HostWordsLease {
+public:
+    explicit HostWordsLease(cudaStream_t s);
+    ~HostWordsLease();
+    HostWordsLease(const HostWordsLease &) = delete;
+    HostWordsLease &operator=(const HostWordsLease &) = delete;
+    HostWords *device() { pending_ = true; return words_; }      // to hand to a kernel (null: no pinned memory)
+    cudaError_t sync() { pending_ = false; return cudaStreamSynchronize(s_); }
+    int64_t operator[](int i) const { return const_cast<const volatile HostWords *>(words_)->w[i]; }
+private:
+    HostWords *words_ = nullptr;
+    cudaStream_t s_;
+    bool pending_ = false;
+};
+
+#define AGCN_HOST_WORDS(var, stream)                                                      \
+    HostWordsLease var(stream);                                                           \
+    do {                                                                                  \
+        if ((var).device() == nullptr) {                                                  \
+            ::agcn::set_error("no pinned host memory for the result words");              \
+            return AGCN_ERR_CUDA;                                                         \
+        }                                                                                 \
+    } while (0)
 
 #define AGCN_ALLOC(var, scratch, type, count)                  \
     type *var = (scratch).alloc<type>(count);                  \
     if (var == nullptr) return AGCN_ERR_CUDA
 
-// Exclusive prefix sums used by several entry points (defined in scan.cu).
+// Exclusive prefix sums used by several entry points (defined in common.cu).
 // tile_sums must hold ceil(n / 2048) elements.  total_out may be null.
 int exclusive_scan_i32_i64(const int *in, int64_t *out, int64_t n, int64_t *tile_sums, int64_t *total_out, cudaStream_t s);
 int exclusive_scan_u32_u32(const unsigned *in, unsigned *out, int64_t n, unsigned *tile_sums, cudaStream_t s);

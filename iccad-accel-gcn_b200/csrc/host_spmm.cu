@@ -5,9 +5,8 @@
 // What crosses PCIe is fixed by the call (the graph, X per product up; Y per product down), so
 // the work is to keep both copy engines and the SMs busy at once:
 //  - uploads, kernels and downloads run on three streams chained by events;
-//  - a product is launched as several unit ranges (a unit = 8 consecutive tuples); each range is
-//    followed by the carry kernel over the carry slots of the rows it completes, and those rows are
-//    downloaded while the next range computes;
+//  - a product is launched as several unit ranges (a unit = 8 consecutive tuples), and the rows a
+//    range completes are downloaded while the next range computes;
 //  - when the graph itself is part of the call (agcn_spmm_host_batch), column ids and values are
 //    uploaded in the same ranges and every range is multiplied -- for all products -- as soon as
 //    it has arrived, so the kernels and the downloads hide under the upload of A.
@@ -36,9 +35,6 @@ struct agcn_host_ctx {
     int64_t n_rows = 0, n_cols = 0, nnz = 0, n_blocks = 0;
     // unit ranges a product is issued in, with the first row / first nonzero of each boundary
     std::vector<int64_t> part_unit, part_row, part_loc;
-    std::vector<int64_t> part_slot;                   // carry slots [part_slot[k], part_slot[k+1]) finish the rows of range k
-    std::vector<int2> h_unit_carry;                   // host copies of the plan's carry bookkeeping
-    std::vector<int> h_carry_row;
     int *d_abort = nullptr;                           // device word: set when a column id is out of range
     std::vector<cudaEvent_t> events;
     size_t events_used = 0;
@@ -96,7 +92,7 @@ static int ctx_sync(agcn_host_ctx *c)
 
 // Cuts the tuple list into about `want_parts` unit ranges of equal nonzero count, reading the
 // caller's host copy of .block4 (tuples tile [0, nnz) in order, so loc_begin is monotone).
-static void plan_part_cuts(agcn_host_ctx *c, const int *h_block4, int want_parts)
+static void plan_parts(agcn_host_ctx *c, const int *h_block4, int want_parts)
 {
     const int64_t n_units = ceil_div(c->n_blocks, HOST_SPMM_WARPS);
     c->part_unit.assign(1, 0);
@@ -123,41 +119,6 @@ static void plan_part_cuts(agcn_host_ctx *c, const int *h_block4, int want_parts
     c->part_unit.push_back(n_units);
     c->part_row.push_back(c->n_rows);
     c->part_loc.push_back(c->nnz);
-}
-
-// The carry slots of every unit range (needs the plan's bookkeeping: build_plan).
-static void plan_part_slots(agcn_host_ctx *c)
-{
-    const int64_t n_units = ceil_div(c->n_blocks, HOST_SPMM_WARPS);
-    // Carry slots are handed out in unit order (a slot for the row entering a unit from the left,
-    // one for the row leaving it to the right).  The rows a unit range completes own the slots up
-    // to the first slot of the row that runs on into the next range, or -- if none does -- up to the
-    // first slot of the next range's first unit.
-    const int n_parts = (int)c->part_unit.size() - 1;
-    const int64_t n_carry = (int64_t)c->h_carry_row.size();
-    c->part_slot.assign(n_parts + 1, n_carry);
-    c->part_slot[0] = 0;
-    int64_t next_slot = 0;                // slots handed out to the units before u
-    int k = 1;
-    for (int64_t u = 0; u < n_units && k < n_parts; u++) {
-        const int2 uc = c->h_unit_carry[u];
-        if (u == c->part_unit[k]) {
-            int64_t first = next_slot;
-            if (uc.x >= 0) {              // a row enters this unit from the previous range: back to its first slot
-                first = uc.x;
-                while (first > 0 && c->h_carry_row[first - 1] == c->h_carry_row[uc.x]) first--;
-            }
-            c->part_slot[k++] = first;
-        }
-        if (uc.x >= 0 && uc.x >= next_slot) next_slot = uc.x + 1;
-        if (uc.y >= 0 && uc.y >= next_slot) next_slot = uc.y + 1;
-    }
-}
-
-static void plan_parts(agcn_host_ctx *c, const int *h_block4, int want_parts)
-{
-    plan_part_cuts(c, h_block4, want_parts);
-    plan_part_slots(c);
 }
 
 static int check_graph_args(agcn_host_ctx *ctx, const int *h_block4, int64_t n_blocks, const int *h_indices,
@@ -189,22 +150,11 @@ static int upload_block4(agcn_host_ctx *c, const int *h_block4, int64_t n_blocks
 }
 
 // Builds the plan from the uploaded .block4 (tuple validation, carry slots, uncovered rows;
-// synchronises s_run) and fetches its carry bookkeeping for plan_parts.  Column ids are validated
-// by the caller (whole array, or range by range as they arrive).
+// synchronises s_run).  Column ids are validated by the caller (whole array, or range by range as they
+// arrive).
 static int build_plan(agcn_host_ctx *c)
 {
-    int rc = spmm_create(&c->plan, static_cast<const int *>(c->graph[0]), c->n_blocks, nullptr, c->n_rows, c->n_cols, c->nnz, c->s_run);
-    if (rc != AGCN_OK) return rc;
-    c->h_unit_carry.assign((size_t)c->plan->n_units, make_int2(-1, -1));
-    c->h_carry_row.assign((size_t)c->plan->n_carry, 0);
-    if (c->plan->n_carry > 0) {
-        AGCN_CUDA(cudaMemcpyAsync(c->h_unit_carry.data(), c->plan->unit_carry, c->h_unit_carry.size() * sizeof(int2),
-                                  cudaMemcpyDeviceToHost, c->s_run));
-        AGCN_CUDA(cudaMemcpyAsync(c->h_carry_row.data(), c->plan->carry_row, c->h_carry_row.size() * sizeof(int),
-                                  cudaMemcpyDeviceToHost, c->s_run));
-        AGCN_CUDA(cudaStreamSynchronize(c->s_run));
-    }
-    return AGCN_OK;
+    return spmm_create(&c->plan, static_cast<const int *>(c->graph[0]), c->n_blocks, nullptr, c->n_rows, c->n_cols, c->nnz, c->s_run);
 }
 
 static int host_set_graph(agcn_host_ctx *c, const int *h_block4, int64_t n_blocks, const int *h_indices,
@@ -253,8 +203,12 @@ static int reserve_products(agcn_host_ctx *c, int n, const int *dims, bool per_p
         int rc = reserve(&c->xbuf[i], &c->xcap[i], (size_t)c->n_cols * dims[i] * 4);
         if (rc == AGCN_OK) rc = reserve(&c->ybuf[i], &c->ycap[i], (size_t)c->n_rows * dims[i] * 4);
         // products whose unit ranges interleave each keep their own partial sums of the heavy rows
-        if (rc == AGCN_OK && per_product_carry && c->plan->n_carry > 0)
-            rc = reserve(&c->cbuf[i], &c->ccap[i], (size_t)c->plan->n_carry * HOST_SPMM_PANEL * 4);
+        if (rc == AGCN_OK && per_product_carry && c->plan->n_carry > 0) {
+            const int64_t n = c->plan->n_carry;
+            rc = reserve(&c->cbuf[i], &c->ccap[i], spmm_carry_bytes(n));
+            if (rc == AGCN_OK)
+                AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(c->cbuf[i], n), 0, (size_t)n * SPMM_CARRY_PASSES * sizeof(int), c->s_run));
+        }
         if (rc != AGCN_OK) return rc;
     }
     return AGCN_OK;
@@ -304,11 +258,9 @@ static int host_products(agcn_host_ctx *c, int n, const float *const *h_x, float
             continue;
         }
         for (int k = 0; k < n_parts; k++) {
-            // the units of the range, then the carry kernel over the rows the range completes
             SpmmLaunchPart part;
             part.unit0 = c->part_unit[k]; part.unit1 = c->part_unit[k + 1];
             part.zero_fill = k == 0;
-            part.carry_s0 = c->part_slot[k]; part.carry_s1 = c->part_slot[k + 1];
             rc = spmm_run_prepared(c->plan, idx, val, static_cast<const float *>(c->xbuf[i]), dim, true, y, dim, dim, c->s_run, 0, 0, part);
             if (rc == AGCN_OK) rc = ctx_chain(c, c->s_run, c->s_down);
             if (rc == AGCN_OK) rc = download_rows(c, i, h_y[i], dim, c->part_row[k], c->part_row[k + 1]);
@@ -378,8 +330,7 @@ static int host_graph_and_products(agcn_host_ctx *c, const int *h_block4, int64_
             SpmmLaunchPart part;
             part.unit0 = c->part_unit[k]; part.unit1 = c->part_unit[k + 1];
             part.zero_fill = k == 0; part.abort_flag = c->d_abort;
-            part.carry_s0 = c->part_slot[k]; part.carry_s1 = c->part_slot[k + 1];
-            part.carry_buf = static_cast<float *>(c->cbuf[i]);
+            part.carry = c->cbuf[i];
             rc = spmm_run_prepared(c->plan, idx, val, static_cast<const float *>(c->xbuf[i]), dims[i], true,
                                    static_cast<float *>(c->ybuf[i]), dims[i], dims[i], c->s_run, 0, 0, part);
         }

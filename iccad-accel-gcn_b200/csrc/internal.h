@@ -5,16 +5,18 @@
 struct agcn_spmm_plan {
     const int4 *block4 = nullptr;     // borrowed
     int64_t n_blocks = 0, n_units = 0, n_rows = 0, n_cols = 0, nnz = 0;
+    int device = -1;
+    void *memory = nullptr;           // one pool block that holds the arrays below
     int2 *unit_carry = nullptr;       // [n_units]
+    int2 *carry_span = nullptr;       // [n_carry]
     int *carry_row = nullptr;         // [n_carry]
-    float *carry = nullptr;           // [n_carry][SPMM_PANEL]
+    void *carry = nullptr;            // spmm_carry_bytes(n_carry): partial sums and arrival counters
     int *zero_rows = nullptr;         // [n_zero]
     int64_t n_carry = 0, n_zero = 0;
     int launches_last_run = 0;
     int l2_bytes = 0, sm_count = 0;   // of the device the plan was created on
     int panel_override = 0;           // AGCN_SPMM_PANEL at creation (0 = choose automatically)
     bool never_split = false;         // set for the ranges of a column-tiled product
-    int batch_override = 0;           // AGCN_SPMM_BATCH at creation: 8 or 16 gathers in flight per lane (experiments)
     int pad_unaligned = 1;            // AGCN_SPMM_PAD at creation: copy unaligned X into 16-byte-aligned rows
     float *x_pad = nullptr;           // [n_cols][dim rounded up to 4], grown on demand
     size_t x_pad_bytes = 0;
@@ -36,16 +38,21 @@ int spmm_check_run_args(const agcn_spmm_plan *p, const int *d_indices, const flo
                         const float *d_y, int64_t ldy, int dim, int activation);
 int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cudaStream_t s,
                    const float **x_use, int64_t *ldx_use, bool *x_vec);
+// Partial sums of the rows that cross unit boundaries: 128 floats per carry slot, and per slot one arrival
+// counter for every column pass a product of up to 128 columns can be cut into (products issued in unit
+// ranges have several passes under way).  The counters must be zero before a product and are zero after it.
+constexpr int SPMM_CARRY_PASSES = 32;
+inline size_t spmm_carry_bytes(int64_t n_carry) { return (size_t)n_carry * (128 * sizeof(float) + SPMM_CARRY_PASSES * sizeof(int)); }
+inline int *spmm_carry_counters(void *carry, int64_t n_carry) { return reinterpret_cast<int *>(static_cast<float *>(carry) + n_carry * 128); }
+
 // Which part of a product one call of spmm_run_prepared launches.  A product may be issued as
-// several unit ranges (a unit = 8 consecutive tuples = one thread block): the zero-fill of
-// uncovered rows goes with one of them and the carry kernel, which finishes the heavy rows that
-// cross unit boundaries, after the last.
+// several unit ranges (a unit = 8 consecutive tuples = one thread block); the zero-fill of uncovered
+// rows goes with one of them.  A heavy row that crosses into the next range is stored by that range.
 struct SpmmLaunchPart {
     int64_t unit0 = 0, unit1 = -1;      // units [unit0, unit1); -1 = to the end
-    bool zero_fill = true, carry = true;
-    int64_t carry_s0 = 0, carry_s1 = -1; // carry slots the carry kernel covers (-1 = to the last); row-aligned
+    bool zero_fill = true;
     const int *abort_flag = nullptr;    // optional device word: nonzero makes the kernels return at once
-    float *carry_buf = nullptr;         // optional carry scratch [n_carry][128] to use instead of the plan's (products in flight together)
+    void *carry = nullptr;              // optional carry scratch to use instead of the plan's (products in flight together)
 };
 int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *x_use, int64_t ldx_use,
                       bool x_vec, float *d_y, int64_t ldy, int dim, cudaStream_t s, int activation, int accumulate,

@@ -17,12 +17,17 @@
 // meet in shared memory and are added in tuple order; a row that is contained
 // in one unit is then stored directly.  A row that crosses a unit boundary
 // leaves one partial per unit in a small "carry" array (at most two per unit),
-// and spmm_carry_kernel adds those in unit order.  Every element of Y is thus
-// written exactly once with a plain store, in a fixed order of additions: no
-// atomics, no dependence on what Y held before, bit-identical from run to run.
+// and these are added in unit order: in a launch of few units by the unit that
+// arrives last at the row's counter, otherwise by spmm_carry_kernel.  (Waiting
+// for a counter keeps a thread block's registers for 1-2 us, 2 % of a product
+// of 50 000 units; a second launch costs 3 us, a third of a product of 2 048 rows.)
+// Every element of Y is thus written exactly once with a plain store, in a
+// fixed order of additions: no floating-point atomics, no dependence on what Y
+// held before, bit-identical from run to run.
 // Rows no tuple covers (degree 0) are zero-filled by extra blocks of the same
 // launch.
 #pragma once
+#include "../host_common.h"
 #include "primitives.cuh"
 #include "ptx.cuh"
 
@@ -62,6 +67,9 @@ struct SpmmParams {
     int dim;            // columns in this panel, 1..SPMM_PANEL
     const int2 *unit_carry;   // per unit: carry slot of a row entering / leaving the unit, or -1
     float *carry;             // [n_carry][SPMM_PANEL]
+    const int2 *carry_span;   // per slot: the first slot of its row, and how many the row has
+    int *carry_count;         // per slot (a row's first): units of the row that have arrived, zero between products;
+                              // null: spmm_carry_kernel follows
     const int *zero_rows;     // rows no tuple covers
     int64_t n_zero_rows;
     int relu;                 // nonzero: Y = max(A * X, 0) (fused GCN activation)
@@ -222,12 +230,58 @@ __device__ __forceinline__ void gather_scalar(const int2 *pairs, int count, cons
     }
 }
 
+// the partials warps w .. w_end - 1 left in shared memory, added in warp order
+__device__ __forceinline__ float4 sum_parts4(const float (*part)[SPMM_PANEL], int w, int w_end, int col)
+{
+    float4 sum = *reinterpret_cast<const float4 *>(&part[w][col]);
+    for (int ww = w + 1; ww < w_end; ww++) {
+        const float4 v = *reinterpret_cast<const float4 *>(&part[ww][col]);
+        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+    }
+    return sum;
+}
+__device__ __forceinline__ float sum_parts1(const float (*part)[SPMM_PANEL], int w, int w_end, int c)
+{
+    float sum = part[w][c];
+    for (int ww = w + 1; ww < w_end; ww++) sum += part[ww][c];
+    return sum;
+}
+
+// Stores a row whose partials lie in carry slots span.x .. span.x + span.y - 1, adding them in slot order.
+// VEC: `first` is the first of the four columns of this lane; otherwise the lane takes columns first, first + 32, ...
+template <bool VEC, bool PLAIN>
+__device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 span, int row, int first, uint64_t policy)
+{
+    const float *parts = p.carry + (int64_t)span.x * SPMM_PANEL;
+    float *yr = p.y + (int64_t)row * p.ldy;
+    if (VEC) {
+        if (first >= p.dim) return;
+        float4 sum = __ldcg(reinterpret_cast<const float4 *>(parts + first));
+#pragma unroll 8
+        for (int q = 1; q < span.y; q++) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(parts + (int64_t)q * SPMM_PANEL + first));
+            sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
+        }
+        emit_row4<PLAIN>(p, yr, first, sum, p.relu, policy);
+    } else {
+        for (int c = first; c < p.dim; c += 32) {
+            float sum = __ldcg(parts + c);
+#pragma unroll 8
+            for (int q = 1; q < span.y; q++) sum += __ldcg(parts + (int64_t)q * SPMM_PANEL + c);
+            emit_row1<PLAIN>(p, yr + c, sum, p.relu, policy);
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // main kernel.  S = lanes per slot in float4 mode (4, 8, 16 or 32; needs
 // dim % 4 == 0, dim <= 4*S and 16-byte aligned rows); S = 0 is the scalar
 // mode for every other dim (lane l owns columns l, l+32, l+64, l+96).
+// FINISH: rows that cross units are finished here (in launches of few units);
+// a template parameter because the code costs registers the large launches
+// do not have (two more spills, 3 % of a product of 500 000 rows).
 // ---------------------------------------------------------------------------
-template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN>
+template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH>
 __global__ void __launch_bounds__(SPMM_THREADS, MIN_BLOCKS)
 spmm_units_kernel(const SpmmParams p)
 {
@@ -332,76 +386,49 @@ spmm_units_kernel(const SpmmParams p)
     const int2 uc = __ldg(p.unit_carry + unit);
     const bool enters = w == 0 && uc.x >= 0;            // the row began in an earlier unit
     const bool leaves = w_end - 1 == w_last && uc.y >= 0;   // the row goes on in the next unit
-    const bool partial = enters || leaves;     // the row is finished by spmm_carry_kernel
-    float *dst = partial ? p.carry + (int64_t)(enters ? uc.x : uc.y) * SPMM_PANEL : p.y + (int64_t)t.row0 * p.ldy;
-    const int act = partial ? 0 : p.relu;
-    if (VEC) {
-        if (slot == 0 && active) {
-            float4 sum = *reinterpret_cast<const float4 *>(&s_part[w][col]);
-            for (int ww = w + 1; ww < w_end; ww++) {
-                const float4 v = *reinterpret_cast<const float4 *>(&s_part[ww][col]);
-                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-            }
-            if (partial) *reinterpret_cast<float4 *>(dst + col) = sum;      // carry slots are aligned and private
-            else emit_row4<PLAIN>(p, dst, col, sum, act, pol.stream);
+    const bool partial = enters || leaves;     // other units hold the rest of the row
+    float *yr = p.y + (int64_t)t.row0 * p.ldy;
+    if (!partial) {
+        if (VEC) {
+            if (slot == 0 && active) emit_row4<PLAIN>(p, yr, col, sum_parts4(s_part, w, w_end, col), p.relu, pol.stream);
+        } else {
+            for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, sum_parts1(s_part, w, w_end, c), p.relu, pol.stream);
         }
-    } else {
-        for (int c = lane; c < p.dim; c += 32) {
-            float sum = s_part[w][c];
-            for (int ww = w + 1; ww < w_end; ww++) sum += s_part[ww][c];
-            if (partial) dst[c] = sum;
-            else emit_row1<PLAIN>(p, dst + c, sum, act, pol.stream);
-        }
+        return;
     }
+    const int my_slot = enters ? uc.x : uc.y;
+    float *mine = p.carry + (int64_t)my_slot * SPMM_PANEL;
+    if (VEC) {
+        if (slot == 0 && active) *reinterpret_cast<float4 *>(mine + col) = sum_parts4(s_part, w, w_end, col);
+    } else {
+        for (int c = lane; c < p.dim; c += 32) mine[c] = sum_parts1(s_part, w, w_end, c);
+    }
+    if (!FINISH) return;                            // spmm_carry_kernel follows
+    // the row's last unit to arrive adds the partials
+    const int2 span = __ldg(p.carry_span + my_slot);
+    __threadfence();
+    __syncwarp();
+    int arrived = 0;
+    if (lane == 0) arrived = atomicAdd(p.carry_count + span.x, 1);
+    arrived = __shfl_sync(FULL_MASK, arrived, 0);
+    if (arrived != span.y - 1) return;
+    if (lane == 0) p.carry_count[span.x] = 0;       // ready for the next product
+    __threadfence();
+    finish_carried_row<VEC, PLAIN>(p, span, t.row0, VEC ? (slot == 0 && active ? col : SPMM_PANEL) : lane, pol.stream);
 }
 
-// Adds the carried partials of every row that crosses unit boundaries, in
-// unit order, and stores the row.  One warp per carry slot; the warp of the
-// first slot of a row does the work.  The launch covers slots [s0, s1), a range
-// that begins and ends between rows (all slots by default; a product issued in
-// unit ranges finishes the rows of each range as soon as its units have run).
+// Adds the carried partials of every row that crosses unit boundaries.  One warp per carry slot; the warp of
+// the first slot of a row does the work.  Bound by latency: the partials of a row are loaded eight at a time
+// (a hub row of 90 000 nonzeros has 30; loaded one by one they took 12 us).
 template <bool VEC>
 __global__ void __launch_bounds__(SPMM_THREADS)
-spmm_carry_kernel(const float *__restrict__ carry, const int *__restrict__ carry_row, int64_t s0, int64_t s1,
-                  float *y, int64_t ldy, int dim, int relu, int accumulate, int y_vec, int dim_store)
+spmm_carry_kernel(const SpmmParams p, const int *__restrict__ carry_row, int64_t n_carry)
 {
-    const int64_t s = s0 + (int64_t)blockIdx.x * SPMM_WARPS + warp_id();
-    if (s >= s1) return;
-    const int row = carry_row[s];
-    if (s > s0 && carry_row[s - 1] == row) return;
-    int64_t s_end = s + 1;
-    while (s_end < s1 && carry_row[s_end] == row) s_end++;
-    const int lane = lane_id();
-    if (VEC) {
-        const int col = lane * 4;
-        if (col < dim) {
-            float4 sum = *reinterpret_cast<const float4 *>(carry + s * SPMM_PANEL + col);
-            for (int64_t q = s + 1; q < s_end; q++) {
-                const float4 v = *reinterpret_cast<const float4 *>(carry + q * SPMM_PANEL + col);
-                sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-            }
-            float *yr = y + (int64_t)row * ldy;
-            if (y_vec) {
-                if (accumulate) {
-                    const float4 o = *reinterpret_cast<const float4 *>(yr + col);
-                    sum.x += o.x; sum.y += o.y; sum.z += o.z; sum.w += o.w;
-                }
-                *reinterpret_cast<float4 *>(yr + col) = relu4(sum, relu);
-            } else {
-                const float e[4] = {sum.x, sum.y, sum.z, sum.w};
-#pragma unroll
-                for (int k = 0; k < 4; k++)
-                    if (col + k < dim_store) yr[col + k] = relu1(accumulate ? e[k] + yr[col + k] : e[k], relu);
-            }
-        }
-    } else {
-        for (int c = lane; c < dim; c += 32) {
-            float sum = carry[s * SPMM_PANEL + c];
-            for (int64_t q = s + 1; q < s_end; q++) sum += carry[q * SPMM_PANEL + c];
-            float *ye = y + (int64_t)row * ldy + c;
-            *ye = relu1(accumulate ? sum + *ye : sum, relu);
-        }
-    }
+    const int64_t s = (int64_t)blockIdx.x * SPMM_WARPS + warp_id();
+    if (s >= n_carry) return;
+    const int2 span = p.carry_span[s];
+    if (span.x != s) return;
+    finish_carried_row<VEC, false>(p, span, carry_row[s], VEC ? lane_id() * 4 : lane_id(), make_l2_policies().stream);
 }
 
 // X[n_rows x dim] with row stride ldx  ->  XP[n_rows x ldp], ldp = dim rounded up to 4, tail zero:
@@ -435,73 +462,40 @@ constexpr int SPMM_ERR_COL = 8;       // column index outside [0, n_cols)
 __device__ __forceinline__ bool tuple_is_big(const int4 &b) { return b.x > SPMM_DEG_BOUND; }
 __device__ __forceinline__ int tuple_rows(const int4 &b) { return tuple_is_big(b) ? 1 : (b.w & 0xffff); }
 
-// Checks every tuple, and counts the rows that lie between tuple e-1 and
-// tuple e (gap[e]; gap[n_blocks] = rows after the last tuple).
-__global__ void __launch_bounds__(256)
-plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_rows, int64_t nnz,
-                  int *__restrict__ gap, int *__restrict__ err_flag)
+// Error bits are single words of the host so that blocks can store to them without atomics.
+constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_ERR = 2;      // then one word per SPMM_ERR_* bit
+constexpr int PLAN_ERR_BITS = 4;
+constexpr int PLAN_BLOCK = 256;      // units per thread block, one per thread
+
+__device__ __forceinline__ void plan_report(HostWords *out, int err)
 {
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e > n_blocks) return;
-    int err = 0;
-    int64_t prev_end = 0;       // first row not covered by tuples before e
-    int64_t prev_loc_end = 0;   // first nonzero not covered by tuples before e
-    if (e > 0) {
-        const int4 a = block4[e - 1];
-        prev_end = (int64_t)a.y + tuple_rows(a);
-        prev_loc_end = (int64_t)a.z + (tuple_is_big(a) ? (int64_t)a.w : (int64_t)tuple_rows(a) * a.x);
-    }
-    if (e == n_blocks) {
-        gap[e] = prev_end <= n_rows ? (int)(n_rows - prev_end) : 0;
-        return;
-    }
-    const int4 b = block4[e];
-    const bool big = tuple_is_big(b);
+#pragma unroll
+    for (int k = 0; k < PLAN_ERR_BITS; k++)
+        if (err & (1 << k)) out->w[PLAN_WORD_ERR + k] = 1;
+}
+
+__device__ __forceinline__ int64_t tuple_nz(const int4 &b) { return tuple_is_big(b) ? (int64_t)b.w : (int64_t)tuple_rows(b) * b.x; }
+
+// rows that lie between tuples a and b (a == nullptr: before the first); negative: out of order or overlapping
+__device__ __forceinline__ int64_t tuple_gap(bool has_prev, const int4 &a, const int4 &b)
+{
+    if (!has_prev) return b.y;
+    if (tuple_is_big(b) && tuple_is_big(a) && a.y == b.y) return 0;       // a later chunk of the same heavy row
+    return (int64_t)b.y - ((int64_t)a.y + tuple_rows(a));
+}
+
+__device__ __forceinline__ int tuple_errors(bool has_prev, const int4 &a, const int4 &b, int64_t n_rows, int64_t nnz)
+{
     const int rows = tuple_rows(b);
-    const int64_t nz = big ? (int64_t)b.w : (int64_t)rows * b.x;
+    const int64_t nz = tuple_nz(b);
+    const int64_t prev_loc_end = has_prev ? (int64_t)a.z + tuple_nz(a) : 0;
+    int err = 0;
     if (b.x < 1 || rows < 1 || nz < 1 || nz > SPMM_DEG_BOUND) err |= SPMM_ERR_TUPLE;
     // tuples take their nonzeros in order and without overlap (what lets A be uploaded and multiplied
     // range by range: a tuple never reaches into a range that has not arrived)
     if (b.z < 0 || (int64_t)b.z + nz > nnz || (int64_t)b.z < prev_loc_end) err |= SPMM_ERR_LOC;
-    int64_t g = (int64_t)b.y - prev_end;
-    if (big && e > 0) {
-        // a later chunk of the same heavy row repeats its row id
-        const int4 a = block4[e - 1];
-        if (tuple_is_big(a) && a.y == b.y) g = 0;
-    }
-    if (b.y < 0 || (int64_t)b.y + rows > n_rows || g < 0) { err |= SPMM_ERR_ROW; g = 0; }
-    gap[e] = (int)g;
-    if (err) atomicOr(err_flag, err);
-}
-
-__global__ void __launch_bounds__(256)
-plan_check_cols_kernel(const int *__restrict__ idx, int64_t nnz, int64_t n_cols, int *__restrict__ err_flag)
-{
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    bool bad = false;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += stride) {
-        const int c = idx[i];
-        bad |= c < 0 || c >= n_cols;
-    }
-    if (bad) atomicOr(err_flag, SPMM_ERR_COL);
-}
-
-// zero_rows[gap_offset[e] ...] = the rows of gap e
-__global__ void __launch_bounds__(256)
-plan_zero_rows_kernel(const int4 *__restrict__ block4, int64_t n_blocks, const int *__restrict__ gap,
-                      const int64_t *__restrict__ gap_offset, int *__restrict__ zero_rows)
-{
-    const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e > n_blocks) return;
-    const int g = gap[e];
-    if (g == 0) return;
-    int64_t prev_end = 0;
-    if (e > 0) {
-        const int4 a = block4[e - 1];
-        prev_end = (int64_t)a.y + tuple_rows(a);
-    }
-    int *dst = zero_rows + gap_offset[e];
-    for (int k = 0; k < g; k++) dst[k] = (int)(prev_end + k);
+    if (b.y < 0 || (int64_t)b.y + rows > n_rows || tuple_gap(has_prev, a, b) < 0) err |= SPMM_ERR_ROW;
+    return err;
 }
 
 // Does a heavy row enter unit u from the left / leave it to the right?
@@ -524,33 +518,170 @@ __device__ __forceinline__ void unit_crossings(const int4 *__restrict__ block4, 
     same_row = enters && leaves && first.y == last.y;
 }
 
-__global__ void __launch_bounds__(256)
-plan_count_carry_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int *__restrict__ count)
+// First pass over a `.block4` array: validates every tuple (and, in the blocks behind the tuple blocks,
+// every column id), and counts per PLAN_BLOCK units the rows no tuple covers and the carry slots.  One
+// launch and one read of 16 bytes per tuple and 4 per nonzero: bound by HBM for large graphs, by launch
+// latency for small ones.  ctl[0], ctl[1]: totals, ctl[2]: blocks done (zero at launch).
+__global__ void __launch_bounds__(PLAN_BLOCK)
+plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int64_t n_rows, int64_t nnz,
+                  const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned unit_grid,
+                  int64_t *__restrict__ tile_zero, int *__restrict__ tile_carry, unsigned long long *__restrict__ ctl,
+                  HostWords *out)
 {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n_units) return;
-    bool en, lv, same; int ri, ro;
-    unit_crossings(block4, n_blocks, u, en, lv, same, ri, ro);
-    count[u] = (en ? 1 : 0) + (lv ? 1 : 0) - (same ? 1 : 0);
+    if (blockIdx.x >= unit_grid) {
+        const int64_t stride = (int64_t)(gridDim.x - unit_grid) * blockDim.x;
+        bool bad = false;
+#pragma unroll 4
+        for (int64_t i = (int64_t)(blockIdx.x - unit_grid) * blockDim.x + threadIdx.x; i < n_idx; i += stride) {
+            const int c = __ldcs(idx + i);
+            bad |= c < 0 || c >= n_cols;
+        }
+        if (bad) plan_report(out, SPMM_ERR_COL);
+        return;
+    }
+    __shared__ int64_t s_zero[PLAN_BLOCK / 32];
+    __shared__ int s_carry[PLAN_BLOCK / 32];
+    const int64_t u = (int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x;
+    int64_t zero = 0;
+    int carry = 0, err = 0;
+    if (u < n_units || (n_units == 0 && u == 0)) {          // without any tuple, one thread counts the rows
+        const int64_t e0 = u * SPMM_WARPS;
+        const int64_t e1 = e0 + SPMM_WARPS < n_blocks ? e0 + SPMM_WARPS : n_blocks;
+        int4 a = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
+        for (int64_t e = e0; e < e1; e++) {
+            const int4 b = block4[e];
+            err |= tuple_errors(e > 0, a, b, n_rows, nnz);
+            const int64_t g = tuple_gap(e > 0, a, b);
+            zero += g > 0 ? g : 0;
+            a = b;
+        }
+        if (e1 == n_blocks) {                 // rows after the last tuple
+            const int64_t g = n_rows - ((int64_t)a.y + tuple_rows(a));
+            zero += g > 0 ? g : 0;
+        }
+        bool en = false, lv = false, same = false; int ri, ro;
+        if (u < n_units) unit_crossings(block4, n_blocks, u, en, lv, same, ri, ro);
+        carry = (en ? 1 : 0) + (lv ? 1 : 0) - (same ? 1 : 0);
+    }
+    if (err) plan_report(out, err);
+    zero = warp_reduce(zero, OpAdd());
+    carry = warp_reduce(carry, OpAdd());
+    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        zero = 0; carry = 0;
+        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; }
+        tile_zero[blockIdx.x] = zero;
+        tile_carry[blockIdx.x] = carry;
+        atomicAdd(ctl + 0, (unsigned long long)zero);
+        atomicAdd(ctl + 1, (unsigned long long)carry);
+        __threadfence();
+        if (atomicAdd(ctl + 2, 1ull) == unit_grid - 1) {
+            __threadfence();
+            out->w[PLAN_WORD_ZERO] = (int64_t)__ldcg(ctl + 0);
+            out->w[PLAN_WORD_CARRY] = (int64_t)__ldcg(ctl + 1);
+        }
+    }
 }
 
+// column ids of a range that has just been uploaded, for products that are streamed: raises a device flag
 __global__ void __launch_bounds__(256)
-plan_assign_carry_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units,
-                         const int64_t *__restrict__ slot_offset, int2 *__restrict__ unit_carry,
-                         int *__restrict__ carry_row)
+plan_check_cols_kernel(const int *__restrict__ idx, int64_t nnz, int64_t n_cols, int *__restrict__ err_flag)
 {
-    const int64_t u = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (u >= n_units) return;
-    bool en, lv, same; int ri, ro;
-    unit_crossings(block4, n_blocks, u, en, lv, same, ri, ro);
-    const int s = (int)slot_offset[u];
-    int2 uc = make_int2(-1, -1);
-    if (en) { uc.x = s; carry_row[s] = ri; }
-    if (lv) {
-        uc.y = same ? s : s + (en ? 1 : 0);
-        if (!same) carry_row[uc.y] = ro;
+    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
+    bool bad = false;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += stride) {
+        const int c = idx[i];
+        bad |= c < 0 || c >= n_cols;
     }
-    unit_carry[u] = uc;
+    if (bad) atomicOr(err_flag, SPMM_ERR_COL);
+}
+
+// first tuple whose row is >= row (tuples are in ascending row order)
+__device__ __forceinline__ int64_t tuple_lower_bound(const int4 *__restrict__ block4, int64_t n_blocks, int64_t row)
+{
+    int64_t lo = 0, hi = n_blocks;
+    while (lo < hi) {
+        const int64_t mid = lo + ((hi - lo) >> 1);
+        if ((int64_t)block4[mid].y < row) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+
+// Second pass: carry slots in unit order, and the list of rows no tuple covers.  A block adds up the counts
+// of the tiles before it itself (a few thousand words at most) -- no scan launches between the passes.
+// Gaps of many rows (the degree-0 rows of an ordered graph are one gap) are written by the whole block.
+constexpr int PLAN_INLINE_GAP = 16, PLAN_GAP_QUEUE = 64;
+
+__global__ void __launch_bounds__(PLAN_BLOCK)
+plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int64_t n_rows,
+                   const int64_t *__restrict__ tile_zero, const int *__restrict__ tile_carry,
+                   int2 *__restrict__ unit_carry, int2 *__restrict__ carry_span, int *__restrict__ carry_row,
+                   int *__restrict__ zero_rows)
+{
+    __shared__ int64_t s_scan64[PLAN_BLOCK / 32 + 1];
+    __shared__ int64_t s_gap_out[PLAN_GAP_QUEUE], s_gap_row[PLAN_GAP_QUEUE], s_gap_len[PLAN_GAP_QUEUE];
+    __shared__ int s_gaps;
+    if (threadIdx.x == 0) s_gaps = 0;
+    int64_t zb = 0, cb = 0;
+    for (int64_t k = threadIdx.x; k < blockIdx.x; k += PLAN_BLOCK) { zb += tile_zero[k]; cb += tile_carry[k]; }
+    int64_t zero_base, carry_base, total;
+    block_scan_exclusive<PLAN_BLOCK>(zb, OpAdd(), (int64_t)0, zero_base, s_scan64);
+    block_scan_exclusive<PLAN_BLOCK>(cb, OpAdd(), (int64_t)0, carry_base, s_scan64);
+
+    const int64_t u = (int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x;
+    const int64_t e0 = u * SPMM_WARPS;
+    const int64_t e1 = e0 + SPMM_WARPS < n_blocks ? e0 + SPMM_WARPS : n_blocks;
+    bool en = false, lv = false, same = false;
+    int ri = 0, ro = 0;
+    int64_t zero = 0;
+    const bool mine = u < n_units || (n_units == 0 && u == 0);
+    if (mine) {
+        if (u < n_units) unit_crossings(block4, n_blocks, u, en, lv, same, ri, ro);
+        if (zero_rows != nullptr) {
+            int4 a = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
+            for (int64_t e = e0; e < e1; e++) { const int4 b = block4[e]; zero += tuple_gap(e > 0, a, b); a = b; }
+            if (e1 == n_blocks) zero += n_rows - ((int64_t)a.y + tuple_rows(a));
+        }
+    }
+    const int64_t slot = carry_base + block_scan_exclusive<PLAN_BLOCK>((int64_t)((en ? 1 : 0) + (lv ? 1 : 0) - (same ? 1 : 0)),
+                                                                       OpAdd(), (int64_t)0, total, s_scan64);
+    int64_t out = zero_base + block_scan_exclusive<PLAN_BLOCK>(zero, OpAdd(), (int64_t)0, total, s_scan64);
+    if (mine) {
+        int2 uc = make_int2(-1, -1);
+        if (en) uc.x = (int)slot;
+        if (lv) uc.y = same ? (int)slot : (int)slot + (en ? 1 : 0);
+        if (u < n_units) unit_carry[u] = uc;
+        // a row has one slot in every unit it touches, and these are consecutive
+        for (int side = 0; side < 2; side++) {
+            const int s = side == 0 ? uc.x : uc.y;
+            if (s < 0 || (side == 1 && same)) continue;
+            const int row = side == 0 ? ri : ro;
+            const int64_t u0 = tuple_lower_bound(block4, n_blocks, row) / SPMM_WARPS;
+            const int64_t u1 = (tuple_lower_bound(block4, n_blocks, (int64_t)row + 1) - 1) / SPMM_WARPS;
+            carry_span[s] = make_int2(s - (int)(u - u0), (int)(u1 - u0 + 1));
+            carry_row[s] = row;
+        }
+        if (zero_rows != nullptr && zero > 0) {
+            int4 a = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
+            for (int64_t e = e0; e <= e1; e++) {
+                if (e == e1 && e1 != n_blocks) break;
+                const int4 b = e < e1 ? block4[e] : make_int4(0, 0, 0, 0);
+                const int64_t first = e > 0 ? (int64_t)a.y + tuple_rows(a) : 0;
+                const int64_t g = e < e1 ? tuple_gap(e > 0, a, b) : n_rows - first;
+                int q = PLAN_GAP_QUEUE;
+                if (g > PLAN_INLINE_GAP) q = atomicAdd(&s_gaps, 1);
+                if (q < PLAN_GAP_QUEUE) { s_gap_out[q] = out; s_gap_row[q] = first; s_gap_len[q] = g; }
+                else for (int64_t k = 0; k < g; k++) zero_rows[out + k] = (int)(first + k);
+                out += g;
+                a = b;
+            }
+        }
+    }
+    __syncthreads();
+    const int gaps = s_gaps < PLAN_GAP_QUEUE ? s_gaps : PLAN_GAP_QUEUE;
+    for (int q = 0; q < gaps; q++)
+        for (int64_t k = threadIdx.x; k < s_gap_len[q]; k += PLAN_BLOCK) zero_rows[s_gap_out[q] + k] = (int)(s_gap_row[q] + k);
 }
 
 }  // namespace agcn

@@ -1,0 +1,118 @@
+// Memory the entry points take for the length of a call, and the words kernels report to the host.
+//
+// A cudaMalloc / cudaFree pair costs 0.1 ms to several ms and stalls the whole device; the set-up calls
+// (degree sort, partitioner, plan) used to make up to a dozen of them for kernels of a few microseconds.
+// Scratch now comes from one stream-ordered pool per device (cudaMallocFromPoolAsync): safe for any number
+// of threads and streams, because the driver orders a block's next use after its last one.  What the pool
+// keeps between calls is bounded by POOL_KEEP_BYTES; agcn_release_scratch gives that back too.
+#include "host_common.h"
+
+#include <mutex>
+
+namespace agcn {
+
+constexpr int POOL_MAX_DEVICES = 64;
+// Enough for the scratch of a graph of 20 million rows, or of the host-array degree sort of 25 million
+// nonzeros; larger calls return the excess to the device at their next synchronisation.
+constexpr uint64_t POOL_KEEP_BYTES = (uint64_t)512 << 20;
+
+static std::mutex g_pool_mutex;
+static cudaMemPool_t g_pool_of[POOL_MAX_DEVICES] = {};
+
+static cudaError_t pool_of_current_device(cudaMemPool_t *out)
+{
+    int dev = -1;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= POOL_MAX_DEVICES) return cudaErrorInvalidDevice;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (g_pool_of[dev] == nullptr) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        e = cudaMemPoolCreate(&pool, &props);
+        if (e != cudaSuccess) return e;
+        uint64_t keep = POOL_KEEP_BYTES;
+        e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        if (e != cudaSuccess) { cudaMemPoolDestroy(pool); return e; }
+        g_pool_of[dev] = pool;
+    }
+    *out = g_pool_of[dev];
+    return cudaSuccess;
+}
+
+cudaError_t pool_alloc(void **out, size_t bytes, cudaStream_t s)
+{
+    *out = nullptr;
+    cudaMemPool_t pool = nullptr;
+    cudaError_t e = pool_of_current_device(&pool);
+    return e != cudaSuccess ? e : cudaMallocFromPoolAsync(out, bytes > 0 ? bytes : 16, pool, s);
+}
+
+void pool_free(void *p, cudaStream_t s)
+{
+    if (p != nullptr) cudaFreeAsync(p, s);
+}
+
+void pool_free_waiting(void *p)
+{
+    if (p == nullptr) return;
+    cudaDeviceSynchronize();             // what cudaFree did: whoever still uses the block is done
+    cudaFreeAsync(p, cudaStreamPerThread);
+}
+
+// ---------------------------------------------------------------------------
+// Host words: pinned, mapped, 64 bytes each, kept in a free list.  A kernel stores its result or error
+// code straight into one and the host reads it after the stream synchronisation it needs anyway, in place
+// of a device word, a memset and a device-to-host copy.
+// ---------------------------------------------------------------------------
+constexpr int HOST_WORDS_PER_CHUNK = 64;      // one 4 KiB page; more chunks only if more calls run at once
+
+struct HostWordsNode {
+    HostWords words;
+    HostWordsNode *next;
+    char pad[64 - (sizeof(HostWords) + sizeof(HostWordsNode *)) % 64];
+};
+
+static std::mutex g_words_mutex;
+static HostWordsNode *g_words_free = nullptr;
+
+HostWordsLease::HostWordsLease(cudaStream_t s) : s_(s)
+{
+    std::lock_guard<std::mutex> lock(g_words_mutex);
+    if (g_words_free == nullptr) {
+        void *chunk = nullptr;
+        if (cudaHostAlloc(&chunk, HOST_WORDS_PER_CHUNK * sizeof(HostWordsNode), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return;
+        HostWordsNode *n = static_cast<HostWordsNode *>(chunk);
+        for (int i = 0; i < HOST_WORDS_PER_CHUNK; i++) { n[i].next = g_words_free; g_words_free = &n[i]; }
+    }
+    HostWordsNode *n = g_words_free;
+    g_words_free = n->next;
+    words_ = &n->words;
+    for (int i = 0; i < HostWords::COUNT; i++) words_->w[i] = 0;
+}
+
+HostWordsLease::~HostWordsLease()
+{
+    if (words_ == nullptr) return;
+    if (pending_) cudaStreamSynchronize(s_);     // a call that gave up early: nothing may still write here
+    std::lock_guard<std::mutex> lock(g_words_mutex);
+    HostWordsNode *n = reinterpret_cast<HostWordsNode *>(words_);
+    n->next = g_words_free;
+    g_words_free = n;
+}
+
+}  // namespace agcn
+
+extern "C" int agcn_release_scratch(void)
+{
+    using namespace agcn;
+    clear_error();
+    cudaMemPool_t pool = nullptr;
+    AGCN_CUDA(pool_of_current_device(&pool));
+    AGCN_CUDA(cudaDeviceSynchronize());
+    AGCN_CUDA(cudaMemPoolTrimTo(pool, 0));
+    return AGCN_OK;
+}

@@ -73,7 +73,7 @@ int partition_device(const int *d_indptr, int64_t n_rows, int *d_block4, int64_t
     *n_blocks = 0;
 
     const int64_t tiles = ceil_div(n_rows, PART_TILE);
-    DeviceScratch scratch;
+    DeviceScratch scratch(s);
     PartScratch sc;
     AGCN_ALLOC(tile_head, scratch, int, tiles);
     AGCN_ALLOC(tile_count, scratch, int64_t, tiles);
@@ -100,7 +100,7 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
     AGCN_REQUIRE(h_indptr != nullptr && n_blocks != nullptr, "agcn_partition_host: null pointer");
     AGCN_REQUIRE(n_rows > 0, "agcn_partition_host: empty graph (n_rows = %lld); the reference script raises IndexError here",
                  (long long)n_rows);
-    DeviceScratch scratch;
+    DeviceScratch scratch(nullptr);
     AGCN_ALLOC(d_indptr, scratch, int, n_rows + 1);
     AGCN_CUDA(cudaMemcpy(d_indptr, h_indptr, (size_t)(n_rows + 1) * sizeof(int), cudaMemcpyHostToDevice));
     int rc = partition_device(d_indptr, n_rows, nullptr, 0, n_blocks, nullptr);

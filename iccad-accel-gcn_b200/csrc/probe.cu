@@ -60,7 +60,7 @@ extern "C" int agcn_probe_gather_bandwidth(int64_t table_rows, int row_floats, i
     const int64_t warps = ceil_div(total_rows, rows_per_warp);
     AGCN_REQUIRE(warps / 8 + 1 < ((int64_t)1 << 31), "agcn_probe_gather_bandwidth: too many rows per launch");
     const unsigned grid = (unsigned)ceil_div(warps, 8);
-    DeviceScratch scratch;
+    DeviceScratch scratch(nullptr);
     AGCN_ALLOC(table, scratch, float, table_rows * row_floats);
     AGCN_ALLOC(sink, scratch, float, (int64_t)grid * 8);
     AGCN_CUDA(cudaMemset(table, 0, (size_t)table_rows * row_floats * sizeof(float)));

@@ -18,14 +18,18 @@ int env_int(const char *name, int dflt)
 void plan_free(agcn_spmm_plan *p)
 {
     if (p == nullptr) return;
-    cudaFree(p->unit_carry);
-    cudaFree(p->carry_row);
-    cudaFree(p->carry);
-    cudaFree(p->zero_rows);
-    cudaFree(p->x_pad);
+    int dev = p->device;
+    cudaGetDevice(&dev);
+    if (dev != p->device) cudaSetDevice(p->device);
+    pool_free_waiting(p->memory);
+    if (p->x_pad != nullptr) pool_free_waiting(p->x_pad);
+    if (dev != p->device) cudaSetDevice(dev);
     delete p;
 }
 
+// Two launches: the first pass counts and validates, the host sizes the plan's one pool block from its
+// answer, the second pass fills it.  (Six cudaMalloc / cudaFree pairs and nine launches before; a plan of
+// 16 384 rows took about 1 ms, most of it in the allocator.)
 int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, const int *d_indices,
                        int64_t n_rows, int64_t n_cols, int64_t nnz, cudaStream_t s)
 {
@@ -40,34 +44,27 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
 
     const int4 *block4 = reinterpret_cast<const int4 *>(d_block4);
     const int64_t n_units = ceil_div(n_blocks, SPMM_WARPS);
-    DeviceScratch scratch;
-    AGCN_ALLOC(gap, scratch, int, n_blocks + 1);
-    AGCN_ALLOC(gap_offset, scratch, int64_t, n_blocks + 1);
-    AGCN_ALLOC(cnt, scratch, int, n_units);
-    AGCN_ALLOC(slot_offset, scratch, int64_t, n_units);
-    AGCN_ALLOC(tile_sums, scratch, int64_t, scan_tiles(n_blocks + 1));
-    AGCN_ALLOC(d_res, scratch, int64_t, 3);    // [0] zero rows, [1] carry slots, [2] error bits (low int)
-    AGCN_CUDA(cudaMemsetAsync(d_res, 0, 3 * sizeof(int64_t), s));
-    int *d_err = reinterpret_cast<int *>(d_res + 2);
-
-    AGCN_KERNEL(plan_check_kernel, (unsigned)ceil_div(n_blocks + 1, 256), 256, s, block4, n_blocks, n_rows, nnz, gap, d_err);
+    const int64_t tiles = n_units > 0 ? ceil_div(n_units, PLAN_BLOCK) : 1;
+    DeviceScratch scratch(s);
+    Carver size;
+    size.take<unsigned long long>(3); size.take<int64_t>(tiles); size.take<int>(tiles);
+    AGCN_ALLOC(block, scratch, unsigned char, (int64_t)size.bytes());
+    Carver c(block);
+    unsigned long long *ctl = c.take<unsigned long long>(3);
+    int64_t *tile_zero = c.take<int64_t>(tiles);
+    int *tile_carry = c.take<int>(tiles);
+    AGCN_HOST_WORDS(words, s);
+    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 3 * sizeof(*ctl), s));
+    // 16 column ids per thread, at most 64 thread blocks per SM's worth of them
+    const int64_t n_idx = d_indices != nullptr ? nnz : 0;
+    const int64_t col_grid = n_idx > 0 ? ceil_div(n_idx, PLAN_BLOCK * 16) : 0;
+    const unsigned grid = (unsigned)(tiles + (col_grid < 9472 ? col_grid : 9472));
+    AGCN_KERNEL(plan_check_kernel, grid, PLAN_BLOCK, s, block4, n_blocks, n_units, n_rows, nnz, d_indices, n_idx, n_cols, (unsigned)tiles,
+                tile_zero, tile_carry, ctl, words.device());
     AGCN_LAUNCH_CHECK("plan_check_kernel");
-    if (d_indices != nullptr && nnz > 0) {
-        int rc_cols = spmm_check_cols(d_indices, nnz, n_cols, d_err, s);
-        if (rc_cols != AGCN_OK) return rc_cols;
-    }
-    int rc = exclusive_scan_i32_i64(gap, gap_offset, n_blocks + 1, tile_sums, d_res + 0, s);
-    if (rc != AGCN_OK) return rc;
-    if (n_units > 0) {
-        AGCN_KERNEL(plan_count_carry_kernel, (unsigned)ceil_div(n_units, 256), 256, s, block4, n_blocks, n_units, cnt);
-        AGCN_LAUNCH_CHECK("plan_count_carry_kernel");
-        rc = exclusive_scan_i32_i64(cnt, slot_offset, n_units, tile_sums, d_res + 1, s);
-        if (rc != AGCN_OK) return rc;
-    }
-    int64_t res[3] = {0, 0, 0};
-    AGCN_CUDA(cudaMemcpyAsync(res, d_res, sizeof(res), cudaMemcpyDeviceToHost, s));
-    AGCN_CUDA(cudaStreamSynchronize(s));
-    const int err = (int)(res[2] & 0xffffffff);
+    AGCN_CUDA(words.sync());
+    int err = 0;
+    for (int k = 0; k < PLAN_ERR_BITS; k++) err |= words[PLAN_WORD_ERR + k] != 0 ? 1 << k : 0;
     if (err != 0) {
         set_error("agcn_spmm_create: invalid input:%s%s%s%s",
                   (err & SPMM_ERR_TUPLE) ? " malformed .block4 tuple;" : "",
@@ -79,41 +76,40 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
 
     agcn_spmm_plan *p = new (std::nothrow) agcn_spmm_plan;
     AGCN_REQUIRE(p != nullptr, "agcn_spmm_create: out of host memory");
+    struct Guard { agcn_spmm_plan *p; ~Guard() { plan_free(p); } } guard{p};       // frees the half-built plan on every early return
+    AGCN_CUDA(cudaGetDevice(&p->device));
     p->block4 = block4; p->n_blocks = n_blocks; p->n_units = n_units;
     p->n_rows = n_rows; p->n_cols = n_cols; p->nnz = nnz;
-    p->n_zero = res[0]; p->n_carry = res[1];
-    cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess && n_units > 0) e = cudaMalloc(&p->unit_carry, (size_t)n_units * sizeof(int2));
-    if (e == cudaSuccess && p->n_carry > 0) e = cudaMalloc(&p->carry_row, (size_t)p->n_carry * sizeof(int));
-    if (e == cudaSuccess && p->n_carry > 0) e = cudaMalloc(&p->carry, (size_t)p->n_carry * SPMM_PANEL * sizeof(float));
-    if (e == cudaSuccess && p->n_zero > 0) e = cudaMalloc(&p->zero_rows, (size_t)p->n_zero * sizeof(int));
-    if (e != cudaSuccess) {
-        set_error("agcn_spmm_create: cudaMalloc of plan scratch: %s", cudaGetErrorString(e));
-        plan_free(p);
-        return AGCN_ERR_CUDA;
+    p->n_zero = words[PLAN_WORD_ZERO]; p->n_carry = words[PLAN_WORD_CARRY];
+    for (int pass = 0; pass < 2; pass++) {
+        Carver m(p->memory);
+        p->unit_carry = m.take<int2>(n_units);
+        p->carry_span = m.take<int2>(p->n_carry);
+        p->carry_row = m.take<int>(p->n_carry);
+        p->carry = m.take<unsigned char>((int64_t)spmm_carry_bytes(p->n_carry));
+        p->zero_rows = m.take<int>(p->n_zero);
+        if (pass == 1 || m.bytes() == 0) break;
+        const cudaError_t e = pool_alloc(&p->memory, m.bytes(), s);
+        if (e != cudaSuccess) {
+            set_error("agcn_spmm_create: allocation of %zu bytes of plan scratch: %s", m.bytes(), cudaGetErrorString(e));
+            return AGCN_ERR_CUDA;
+        }
     }
-    if (p->n_zero > 0)
-        AGCN_KERNEL(plan_zero_rows_kernel, (unsigned)ceil_div(n_blocks + 1, 256), 256, s, block4, n_blocks, (const int *)gap,
-                    (const int64_t *)gap_offset, p->zero_rows);
-    if (n_units > 0)
-        AGCN_KERNEL(plan_assign_carry_kernel, (unsigned)ceil_div(n_units, 256), 256, s, block4, n_blocks, n_units,
-                    (const int64_t *)slot_offset, p->unit_carry, p->carry_row);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-    if (e != cudaSuccess) {
-        set_error("agcn_spmm_create: plan kernels: %s", cudaGetErrorString(e));
-        plan_free(p);
-        return AGCN_ERR_CUDA;
+    if (p->n_carry > 0)
+        AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(p->carry, p->n_carry), 0, (size_t)p->n_carry * SPMM_CARRY_PASSES * sizeof(int), s));
+    if (p->n_carry > 0 || p->n_zero > 0) {
+        AGCN_KERNEL(plan_assign_kernel, (unsigned)tiles, PLAN_BLOCK, s, block4, n_blocks, n_units, n_rows, (const int64_t *)tile_zero,
+                    (const int *)tile_carry, p->unit_carry, p->carry_span, p->carry_row, p->n_zero > 0 ? p->zero_rows : nullptr);
+        AGCN_LAUNCH_CHECK("plan_assign_kernel");
+    } else if (n_units > 0) {
+        AGCN_CUDA(cudaMemsetAsync(p->unit_carry, 0xff, (size_t)n_units * sizeof(int2), s));      // no row crosses units
     }
-    {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&p->l2_bytes, cudaDevAttrL2CacheSize, dev);
-        cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, dev);
-        p->panel_override = env_int("AGCN_SPMM_PANEL", 0);
-        p->pad_unaligned = env_int("AGCN_SPMM_PAD", 1);
-        p->batch_override = env_int("AGCN_SPMM_BATCH", 0);
-    }
+    AGCN_CUDA(cudaStreamSynchronize(s));          // products may run on any stream
+    AGCN_CUDA(cudaDeviceGetAttribute(&p->l2_bytes, cudaDevAttrL2CacheSize, p->device));
+    AGCN_CUDA(cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device));
+    p->panel_override = env_int("AGCN_SPMM_PANEL", 0);
+    p->pad_unaligned = env_int("AGCN_SPMM_PAD", 1);
+    guard.p = nullptr;
     *out = p;
     return AGCN_OK;
 }
@@ -128,31 +124,30 @@ int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag
     return AGCN_OK;
 }
 
-template <int S>
-static void launch_units(const SpmmParams &prm, unsigned grid, bool small_launch, bool plain, int batch, cudaStream_t s)
+template <int S, int BATCH, int MIN_BLOCKS, bool FINISH>
+static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaStream_t s)
 {
-    if (batch == 8) {          // experiment knob AGCN_SPMM_BATCH=8: 8 gathers in flight per lane at 3 thread blocks per SM
-        if (plain) { auto k = spmm_units_kernel<S, 8, 3, true>; AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm); }
-        else { auto k = spmm_units_kernel<S, 8, 3, false>; AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm); }
-        return;
-    }
-    if (small_launch || batch == 16) {
-        if (plain) { auto k = spmm_units_kernel<S, SPMM_SMALL_GATHER_BATCH, SPMM_SMALL_MIN_BLOCKS, true>; AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm); }
-        else { auto k = spmm_units_kernel<S, SPMM_SMALL_GATHER_BATCH, SPMM_SMALL_MIN_BLOCKS, false>; AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm); }
-    } else {
-        if (plain) { auto k = spmm_units_kernel<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, true>; AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm); }
-        else { auto k = spmm_units_kernel<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>; AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm); }
-    }
+    auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH>;
+    AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm);
 }
 
-static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, unsigned grid, bool small_launch, bool plain,
-                                   int batch, cudaStream_t s)
+// `small` launches always finish the rows that cross units themselves.
+template <int S>
+static void launch_units_for(const SpmmParams &prm, unsigned grid, bool small, bool plain, bool finish, cudaStream_t s)
 {
-    if (!vec) launch_units<0>(prm, grid, small_launch, plain, batch, s);
-    else if (width <= 16) launch_units<4>(prm, grid, small_launch, plain, batch, s);
-    else if (width <= 32) launch_units<8>(prm, grid, small_launch, plain, batch, s);
-    else if (width <= 64) launch_units<16>(prm, grid, small_launch, plain, batch, s);
-    else launch_units<32>(prm, grid, small_launch, plain, batch, s);
+    if (small) launch_units<S, SPMM_SMALL_GATHER_BATCH, SPMM_SMALL_MIN_BLOCKS, true>(prm, grid, plain, s);
+    else if (finish) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, true>(prm, grid, plain, s);
+    else launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, plain, s);
+}
+
+static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, unsigned grid, bool small, bool plain, bool finish,
+                                   cudaStream_t s)
+{
+    if (!vec) launch_units_for<0>(prm, grid, small, plain, finish, s);
+    else if (width <= 16) launch_units_for<4>(prm, grid, small, plain, finish, s);
+    else if (width <= 32) launch_units_for<8>(prm, grid, small, plain, finish, s);
+    else if (width <= 64) launch_units_for<16>(prm, grid, small, plain, finish, s);
+    else launch_units_for<32>(prm, grid, small, plain, finish, s);
 }
 
 // Rows of X that are not 16-byte aligned (dim % 4 != 0 with the reference's ld = dim, an odd
@@ -174,9 +169,9 @@ int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cu
     const size_t need = (size_t)p->n_cols * ldp * sizeof(float);
     if (need > p->x_pad_bytes) {
         // growing the scratch synchronises the device once per plan and width; steady state allocates nothing
-        if (p->x_pad != nullptr) AGCN_CUDA(cudaFree(p->x_pad));
+        pool_free_waiting(p->x_pad);
         p->x_pad = nullptr; p->x_pad_bytes = 0;
-        AGCN_CUDA(cudaMalloc(&p->x_pad, need));
+        AGCN_CUDA(pool_alloc(reinterpret_cast<void **>(&p->x_pad), need, s));
         p->x_pad_bytes = need;
     }
     const int64_t quads = p->n_cols * (ldp >> 2);
@@ -214,7 +209,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     const int64_t zero_blocks = !part.zero_fill || (accumulate && !activation) ? 0 : ceil_div(p->n_zero, SPMM_ZERO_ROWS_PER_BLOCK);
     const int64_t grid = (unit1 - unit0) + zero_blocks;
     AGCN_REQUIRE(grid < (int64_t)INT32_MAX, "agcn_spmm_run: grid too large");
-    const bool small_launch = p->n_units <= (int64_t)SPMM_SMALL_MIN_BLOCKS * p->sm_count;
+    const bool small = p->n_units <= (int64_t)SPMM_SMALL_MIN_BLOCKS * p->sm_count;
 
     // Column panels.  The gather re-reads a row of X once per nonzero of that column, so it runs
     // at L2 speed only while the X columns of a pass stay L2-resident.  When dim > 64 and the
@@ -233,12 +228,13 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         if (x_bytes > 0.75 * (double)p->l2_bytes && x_bytes <= 4.0 * (double)p->l2_bytes) panel = 64;
     }
     if (p->panel_override > 0) panel = p->panel_override;
-    const int64_t cs0 = part.carry_s0, cs1 = part.carry_s1 < 0 ? p->n_carry : part.carry_s1;
-    AGCN_REQUIRE(cs0 >= 0 && cs0 <= cs1 && cs1 <= p->n_carry, "agcn_spmm_run: carry slot range outside the plan");
-    const bool whole = unit0 == 0 && unit1 == p->n_units && part.carry && cs0 == 0 && cs1 == p->n_carry;
-    // A carry slot holds SPMM_PANEL floats and every column pass uses its own columns of it, so a
-    // product of up to SPMM_PANEL columns can be issued in parts (unit launches now, carry kernel
-    // later) whatever its passes are -- with the same passes, hence the same bits, as a whole run.
+    const bool whole = unit0 == 0 && unit1 == p->n_units;
+    // Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM),
+    // where a second launch costs more than blocks that wait for a counter; parts of a product always do that.
+    const bool carry_inside = !whole || p->n_units <= (int64_t)20 * p->sm_count;
+    // A carry slot holds SPMM_PANEL floats and every column pass uses its own columns (and arrival
+    // counters) of it, so a product of up to SPMM_PANEL columns can be issued in parts whatever its
+    // passes are -- with the same passes, hence the same bits, as a whole run.
     if (!whole) AGCN_REQUIRE(dim <= SPMM_PANEL, "agcn_spmm_run: a product issued in unit ranges is limited to %d columns", SPMM_PANEL);
     AGCN_REQUIRE(panel >= 1 && panel <= SPMM_PANEL, "agcn_spmm_run: AGCN_SPMM_PANEL must be 1..%d", SPMM_PANEL);
     if (x_vec && panel % 4 != 0) panel = (panel + 3) & ~3;         // keep every panel's first column 16-byte aligned
@@ -252,7 +248,10 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.x = x_use + col0; prm.ldx = ldx_use;
         prm.y = d_y + col0; prm.ldy = ldy;
         prm.unit_carry = p->unit_carry;
-        prm.carry = (part.carry_buf != nullptr ? part.carry_buf : p->carry) + col0 % SPMM_PANEL;
+        void *carry = part.carry != nullptr ? part.carry : p->carry;
+        prm.carry = static_cast<float *>(carry) + col0 % SPMM_PANEL;
+        prm.carry_span = p->carry_span;
+        prm.carry_count = spmm_carry_counters(carry, p->n_carry) + (int64_t)(col0 % SPMM_PANEL / 4) * p->n_carry;
         prm.zero_rows = p->zero_rows; prm.n_zero_rows = p->n_zero;
         prm.relu = activation;
         prm.accumulate = accumulate;
@@ -263,15 +262,13 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
         const bool plain = !accumulate && (vec ? y_vec : true);
         if (grid > 0) {
-            launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, small_launch, plain, p->batch_override, s);
+            launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, small, plain, carry_inside, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;
         }
-        if (cs1 > cs0 && part.carry) {
-            const unsigned cgrid = (unsigned)ceil_div(cs1 - cs0, SPMM_WARPS);
+        if (p->n_carry > 0 && !carry_inside) {
             auto k = vec ? spmm_carry_kernel<true> : spmm_carry_kernel<false>;
-            AGCN_KERNEL(k, cgrid, SPMM_THREADS, s, (const float *)prm.carry, (const int *)p->carry_row, cs0, cs1, prm.y, ldy,
-                        prm.dim, activation, accumulate, prm.y_vec, prm.dim_store);
+            AGCN_KERNEL(k, (unsigned)ceil_div(p->n_carry, SPMM_WARPS), SPMM_THREADS, s, prm, (const int *)p->carry_row, p->n_carry);
             AGCN_LAUNCH_CHECK("spmm_carry_kernel");
             p->launches_last_run++;
         }

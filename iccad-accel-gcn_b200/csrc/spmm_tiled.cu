@@ -61,7 +61,7 @@ static int tiled_create(agcn_spmm_tiled **out, const int *d_indptr, const int *d
                  ends[0], ends[1], (long long)nnz);
 
     const int64_t per = n_rows + 1, cells = per * n_ranges;
-    DeviceScratch scratch;
+    DeviceScratch scratch(s);
     AGCN_ALLOC(count, scratch, int, cells);
     AGCN_ALLOC(position, scratch, int64_t, cells);
     AGCN_ALLOC(tile_sums, scratch, int64_t, scan_tiles(cells));

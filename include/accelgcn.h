@@ -42,6 +42,10 @@ const char *agcn_last_error(void);
 /* Library version: major * 10000 + minor * 100 + patch. */
 int agcn_version(void);
 
+/* Scratch memory comes from a stream-ordered pool of the library, one per device, which keeps at most
+ * 512 MB between calls.  This returns what the current device's pool keeps (it waits for the device). */
+int agcn_release_scratch(void);
+
 /* ------------------------------------------------------------------------
  * Block-level partitioner.
  * Replaces the per-graph body of block_level_partition.py:38-106: row
