@@ -24,6 +24,8 @@ PROTOTYPES = {
     "agcn_version": (_int, []),
     "agcn_release_scratch": (_int, []),
     "agcn_partition_device": (_int, [_vp, _i64, _vp, _i64, ctypes.POINTER(_i64), _vp]),
+    "agcn_partition_begin": (_int, [_vp, _i64, ctypes.POINTER(_vp), ctypes.POINTER(_i64), _vp]),
+    "agcn_partition_finish": (_int, [_vp, _vp]),
     "agcn_partition_host": (_int, [_vp, _i64, _vp, _i64, ctypes.POINTER(_i64)]),
     "agcn_partition_device_noalloc": (_int, [_vp, _i64, _vp, _i64, ctypes.POINTER(_i64), _vp]),
     "agcn_degree_sort_device": (_int, [_vp, _vp, _vp, _i64, _i64, _int, _vp, _vp, _vp, _vp, _vp]),

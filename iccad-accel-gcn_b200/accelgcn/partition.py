@@ -46,11 +46,13 @@ def block_level_partition_device(indptr, stream=None):
     if n_rows <= 0:
         raise IndexError("empty graph")
     s = stream if stream is not None else torch.cuda.current_stream(indptr.device)
-    n_blocks = ctypes.c_int64(0)
+    n_blocks, run = ctypes.c_int64(0), ctypes.c_void_p()
     with torch.cuda.device(indptr.device):
-        _lib.check(lib.agcn_partition_device(indptr.data_ptr(), n_rows, None, 0, ctypes.byref(n_blocks), s.cuda_stream))
-        out = torch.empty((n_blocks.value, 4), dtype=torch.int32, device=indptr.device)
-        if n_blocks.value:
-            _lib.check(lib.agcn_partition_device(indptr.data_ptr(), n_rows, out.data_ptr(), n_blocks.value,
-                                                 ctypes.byref(n_blocks), s.cuda_stream))
+        _lib.check(lib.agcn_partition_begin(indptr.data_ptr(), n_rows, ctypes.byref(run), ctypes.byref(n_blocks), s.cuda_stream))
+        try:
+            out = torch.empty((n_blocks.value, 4), dtype=torch.int32, device=indptr.device)
+        except BaseException:
+            lib.agcn_partition_finish(run, None)
+            raise
+        _lib.check(lib.agcn_partition_finish(run, out.data_ptr() if n_blocks.value else None))
     return out

@@ -241,13 +241,14 @@ static int dist_set_graph(agcn_dist *d, const int *d_indptr, const int *d_indice
     // sliced exchange: one column range per slice; otherwise the caller's choice of equal ranges
     d->ranges = chunks > 1 ? chunks : column_ranges;
     if (d->ranges == 1) {
-        rc = partition_device(d->indptr, per, nullptr, 0, &d->n_blocks, s);
+        PartitionRun run;
+        rc = partition_begin(&run, d->indptr, per, s);
         if (rc != AGCN_OK) return rc;
-        if (d->n_blocks > 0) {
-            AGCN_CUDA(cudaMalloc(&d->block4, (size_t)d->n_blocks * 16));
-            rc = partition_device(d->indptr, per, d->block4, d->n_blocks, &d->n_blocks, s);
-            if (rc != AGCN_OK) return rc;
-        }
+        d->n_blocks = run.n_blocks;
+        const cudaError_t e = d->n_blocks > 0 ? cudaMalloc(&d->block4, (size_t)d->n_blocks * 16) : cudaSuccess;
+        rc = partition_finish(&run, d->block4);
+        AGCN_CUDA(e);
+        if (rc != AGCN_OK) return rc;
         return spmm_create(&d->plan, d->block4, d->n_blocks, d->idx, per, d->n_gathered, d->local_nnz, s);
     }
     // with a sliced exchange the product over a slice starts when that slice has arrived; with column

@@ -28,6 +28,16 @@ int env_int(const char *name, int dflt);
 
 // partition.cu
 int partition_device(const int *d_indptr, int64_t n_rows, int *d_block4, int64_t cap_blocks, int64_t *n_blocks, cudaStream_t s);
+// The same in two halves: begin counts (and waits for the stream), finish fills n_blocks tuples asynchronously
+// and gives the scratch back (d_block4 == nullptr: only that).
+struct PartitionRun {
+    const int *indptr = nullptr;
+    int64_t n_rows = 0, n_blocks = 0;
+    void *memory = nullptr;
+    cudaStream_t stream = nullptr;
+};
+int partition_begin(PartitionRun *run, const int *d_indptr, int64_t n_rows, cudaStream_t s);
+int partition_finish(PartitionRun *run, int *d_block4);
 
 // spmm.cu
 int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, const int *d_indices,

@@ -9,11 +9,15 @@
 //                          the tuple covers j = min(R(D), rows left in the run) rows
 //   D > 384             -> ceil(D / 384) tuples of <= 384 nonzeros each
 // with R(D), w(D) the pattern tables of block_level_partition.py:7-21 and the
-// fall-backs of :56-63.  So: (A) a max-scan finds run starts, (B) a sum-scan
-// of per-row tuple counts finds output offsets, (C) every row writes its own
-// tuples.  Each phase works on tiles of PART_TILE rows staged through shared
-// memory; the two cross-tile scans are single-block kernels.
+// fall-backs of :56-63.  Three launches over tiles of PART_TILE rows staged
+// through shared memory: (A) every tile describes itself -- its last run start,
+// its leading rows that belong to a run begun earlier, the tuples all other rows
+// open; (B) one thread block scans the descriptions, which closes the open runs,
+// and leaves every tile its incoming run start and its first output position;
+// (C) every row writes its own tuples.
+// Bound: launch latency up to some 100 000 rows, instruction issue above.
 #pragma once
+#include "../host_common.h"
 #include "primitives.cuh"
 
 namespace agcn {
@@ -24,6 +28,7 @@ constexpr int PART_ITEMS = 8;
 constexpr int PART_TILE = PART_BLOCK * PART_ITEMS;
 constexpr int PART_MAX_ROWS_PER_TUPLE = 12;
 constexpr int PART_HALO = PART_MAX_ROWS_PER_TUPLE + 1;   // rows looked at past a tile
+constexpr int PART_WORD_TOTAL = 0, PART_WORD_NEGATIVE = 1;    // host words
 
 // rows per tuple R(D) and nonzeros per virtual warp w(D), 1 <= D <= 384
 __device__ __forceinline__ int part_rows_per_tuple(int d)
@@ -35,6 +40,12 @@ __device__ __forceinline__ int part_warp_nz(int d)
     if (d >= 192) return 32;
     const int f = 12 / part_rows_per_tuple(d);
     return (d + f - 1) / f;
+}
+
+// x mod R(d), with the division by a constant in every case
+__device__ __forceinline__ unsigned part_mod_rows(unsigned x, int d)
+{
+    return d <= 32 ? x % 12u : d <= 64 ? x % 6u : d <= 96 ? x & 3u : d <= 128 ? x % 3u : d <= 191 ? x & 1u : 0u;
 }
 
 // Shared-memory view of indptr[tile_first - 1 .. tile_first + PART_TILE + PART_HALO]
@@ -74,88 +85,125 @@ __device__ __forceinline__ PartTile part_load_tile(const int *__restrict__ indpt
     return t;
 }
 
-// (A) per tile: index of the last row in the tile that starts a run (-1 if none)
-__global__ void __launch_bounds__(PART_BLOCK)
-part_run_heads_kernel(const int *__restrict__ indptr, int64_t n_rows, int *__restrict__ tile_last_head,
-                      int *__restrict__ err_flag)
-{
-    __shared__ int s_ip[PART_SMEM_INTS];
-    __shared__ int s_warp[PART_BLOCK / 32];
-    const PartTile t = part_load_tile(indptr, n_rows, s_ip);
-    int last = -1;
-    bool negative = false;
-#pragma unroll
-    for (int k = 0; k < PART_ITEMS; k++) {
-        const int64_t i = t.first + (int64_t)threadIdx.x * PART_ITEMS + k;
-        if (i < n_rows) {
-            const int d = t.deg(i);
-            negative |= d < 0;
-            if (i == 0 || d != t.deg(i - 1)) last = (int)i;
-        }
-    }
-    if (negative) atomicOr(err_flag, 1);
-    last = warp_reduce(last, OpMax());
-    if (lane_id() == 0) s_warp[warp_id()] = last;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int m = -1;
-        for (int w = 0; w < PART_BLOCK / 32; w++) m = m > s_warp[w] ? m : s_warp[w];
-        tile_last_head[blockIdx.x] = m;
-    }
-}
+// What a tile says about itself.
+struct PartTileInfo {
+    int last_head;    // last row of the tile that starts a run, -1 if none
+    int lead;         // rows before the tile's first run start, where their tuples depend on where that run began
+    int lead_deg;     // ... and their degree (1 .. 384; lead is 0 for any other degree)
+    int rest;         // tuples opened by all other rows
+};
 
 // Number of tuples each of this thread's PART_ITEMS rows opens.
-// incoming_head = start of the run that is open when the tile begins.
-__device__ __forceinline__ void part_row_counts(const PartTile &t, int incoming_head, int *s_scan,
-                                                int (&cnt)[PART_ITEMS])
+// incoming_head = start of the run that is open when the tile begins; -1: not known, rows of that run
+// that need it count in `lead` instead.  Returns the last run start of this thread's rows, -1 if none.
+__device__ __forceinline__ int part_row_counts(const PartTile &t, int incoming_head, int *s_scan, int (&cnt)[PART_ITEMS],
+                                               int &lead, int &lead_deg, bool &negative)
 {
     const int64_t my_first = t.first + (int64_t)threadIdx.x * PART_ITEMS;
     // last run head among this thread's rows, then an exclusive max-scan over the block
     int head_local = -1;
+    int prev = my_first > 0 && my_first < t.n_rows ? t.deg(my_first - 1) : -1;
+    int deg[PART_ITEMS];
+    unsigned heads = 0;
 #pragma unroll
     for (int k = 0; k < PART_ITEMS; k++) {
         const int64_t i = my_first + k;
-        if (i < t.n_rows && (i == 0 || t.deg(i) != t.deg(i - 1))) head_local = (int)i;
+        deg[k] = t.deg(i);
+        if (i < t.n_rows) {
+            negative |= deg[k] < 0;
+            if (i == 0 || deg[k] != prev) { head_local = (int)i; heads |= 1u << k; }
+        }
+        prev = deg[k];
     }
     int unused_total;
     int run_head = block_scan_exclusive<PART_BLOCK>(head_local, OpMax(), -1, unused_total, s_scan);
     run_head = run_head > incoming_head ? run_head : incoming_head;
+    lead = 0;
+    lead_deg = 0;
 #pragma unroll
     for (int k = 0; k < PART_ITEMS; k++) {
         const int64_t i = my_first + k;
         int c = 0;
         if (i < t.n_rows) {
-            const int d = t.deg(i);
-            if (i == 0 || d != t.deg(i - 1)) run_head = (int)i;
+            const int d = deg[k];
+            if (heads & (1u << k)) run_head = (int)i;
             if (d > PART_DEG_BOUND) c = (d + PART_DEG_BOUND - 1) / PART_DEG_BOUND;
-            else if (d >= 1) c = ((int)i - run_head) % part_rows_per_tuple(d) == 0 ? 1 : 0;
+            else if (d >= 1) {
+                if (run_head < 0) { lead++; lead_deg = d; }
+                else c = part_mod_rows((unsigned)((int)i - run_head), d) == 0 ? 1 : 0;
+            }
         }
         cnt[k] = c;
     }
+    return head_local;
 }
 
-// (B) per tile: number of tuples the tile's rows open
+// (A) the description of every tile
 __global__ void __launch_bounds__(PART_BLOCK)
-part_count_kernel(const int *__restrict__ indptr, int64_t n_rows, const int *__restrict__ tile_incoming_head,
-                  int64_t *__restrict__ tile_count)
+part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInfo *__restrict__ tiles, HostWords *out)
 {
     __shared__ int s_ip[PART_SMEM_INTS];
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
-    __shared__ int64_t s_sum[PART_BLOCK / 32];
+    __shared__ int s_red[4][PART_BLOCK / 32];
     const PartTile t = part_load_tile(indptr, n_rows, s_ip);
-    int cnt[PART_ITEMS];
-    part_row_counts(t, tile_incoming_head[blockIdx.x], s_scan, cnt);
-    int64_t sum = 0;
+    int cnt[PART_ITEMS], lead, lead_deg;
+    bool negative = false;
+    int head = part_row_counts(t, -1, s_scan, cnt, lead, lead_deg, negative);
+    if (negative) out->w[PART_WORD_NEGATIVE] = 1;
+    int rest = 0;
 #pragma unroll
-    for (int k = 0; k < PART_ITEMS; k++) sum += cnt[k];
-    sum = warp_reduce(sum, OpAdd());
-    if (lane_id() == 0) s_sum[warp_id()] = sum;
+    for (int k = 0; k < PART_ITEMS; k++) rest += cnt[k];
+    head = warp_reduce(head, OpMax());
+    lead = warp_reduce(lead, OpAdd());
+    lead_deg = warp_reduce(lead_deg, OpMax());
+    rest = warp_reduce(rest, OpAdd());
+    if (lane_id() == 0) { s_red[0][warp_id()] = head; s_red[1][warp_id()] = lead; s_red[2][warp_id()] = lead_deg; s_red[3][warp_id()] = rest; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        int64_t s = 0;
-        for (int w = 0; w < PART_BLOCK / 32; w++) s += s_sum[w];
-        tile_count[blockIdx.x] = s;
+        PartTileInfo info = {-1, 0, 0, 0};
+        for (int w = 0; w < PART_BLOCK / 32; w++) {
+            info.last_head = max(info.last_head, s_red[0][w]);
+            info.lead += s_red[1][w];
+            info.lead_deg = max(info.lead_deg, s_red[2][w]);
+            info.rest += s_red[3][w];
+        }
+        tiles[blockIdx.x] = info;
     }
+}
+
+// (B) one block: the run start that is open when every tile begins, and every tile's first output position.
+// 1024 tiles (two million rows) per step.
+constexpr int PART_SCAN_BLOCK = 1024;
+
+__global__ void __launch_bounds__(PART_SCAN_BLOCK)
+part_scan_kernel(const PartTileInfo *__restrict__ tiles, int64_t n_tiles, int *__restrict__ tile_head,
+                 int64_t *__restrict__ tile_offset, HostWords *out)
+{
+    __shared__ int s_head[PART_SCAN_BLOCK / 32 + 1];
+    __shared__ int64_t s_sum[PART_SCAN_BLOCK / 32 + 1];
+    int carry_head = -1;
+    int64_t carry = 0;
+    for (int64_t base = 0; base < n_tiles; base += PART_SCAN_BLOCK) {
+        const int64_t b = base + threadIdx.x;
+        PartTileInfo info = {-1, 0, 0, 0};
+        if (b < n_tiles) info = tiles[b];
+        int head_total;
+        int head = block_scan_exclusive<PART_SCAN_BLOCK>(info.last_head, OpMax(), -1, head_total, s_head);
+        head = max(head, carry_head);
+        int64_t count = info.rest;
+        if (info.lead > 0) {
+            // rows o .. o + lead - 1 of their run open a tuple where their number is a multiple of R
+            const int64_t o = b * PART_TILE - head;
+            const int r = part_rows_per_tuple(info.lead_deg);
+            count += (o + info.lead + r - 1) / r - (o + r - 1) / r;
+        }
+        int64_t total;
+        const int64_t ex = block_scan_exclusive<PART_SCAN_BLOCK>(count, OpAdd(), (int64_t)0, total, s_sum);
+        if (b < n_tiles) { tile_head[b] = head; tile_offset[b] = carry + ex; }
+        carry += total;
+        carry_head = max(carry_head, head_total);
+    }
+    if (threadIdx.x == 0) out->w[PART_WORD_TOTAL] = carry;
 }
 
 // (C) every row that opens tuples writes them at its scanned offset.  A row of degree D > 384 owns
@@ -175,8 +223,9 @@ part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const int *__re
     __shared__ int64_t s_heavy_out[PART_HEAVY_QUEUE];
     if (threadIdx.x == 0) s_heavy_n = 0;
     const PartTile t = part_load_tile(indptr, n_rows, s_ip);      // synchronises the block
-    int cnt[PART_ITEMS];
-    part_row_counts(t, tile_incoming_head[blockIdx.x], s_scan, cnt);
+    int cnt[PART_ITEMS], lead, lead_deg;
+    bool negative;
+    part_row_counts(t, tile_incoming_head[blockIdx.x], s_scan, cnt, lead, lead_deg, negative);
     int sum = 0;
 #pragma unroll
     for (int k = 0; k < PART_ITEMS; k++) sum += cnt[k];

@@ -4,59 +4,83 @@
 #include "internal.h"
 #include "kernels/partition_kernels.cuh"
 
-#include <cstddef>
 #include <mutex>
+#include <new>
+
+struct agcn_partition_run {
+    agcn::PartitionRun run;
+};
 
 namespace agcn {
 
-// Tile scratch of one partitioner call: one run-head index and one tuple count per PART_TILE rows,
-// the tuple total and an error word.  The regular entry point allocates it per call; the
+// Tile scratch of one partitioner call.  The regular entry points take it from the pool; the
 // allocation-free one points it at a fixed array in the library's device image.
 struct PartScratch {
+    PartTileInfo *info;
     int *tile_head;
-    int64_t *tile_count;
-    int64_t *total;
-    int *err;
+    int64_t *tile_offset;
 };
 
-// The pipeline both entry points run.  `who` names the entry point in error messages.
-static int partition_pipeline(const char *who, const int *d_indptr, int64_t n_rows, int *d_block4, int64_t cap_blocks,
-                              int64_t *n_blocks, const PartScratch &sc, cudaStream_t s)
+static PartScratch part_scratch(Carver &c, int64_t tiles)
+{
+    PartScratch sc;
+    sc.info = c.take<PartTileInfo>(tiles);
+    sc.tile_offset = c.take<int64_t>(tiles);
+    sc.tile_head = c.take<int>(tiles);
+    return sc;
+}
+
+static int partition_check(const char *who, const int *d_indptr, int64_t n_rows, const int *d_block4, const void *result)
+{
+    AGCN_REQUIRE(d_indptr != nullptr && result != nullptr, "%s: null pointer", who);
+    AGCN_REQUIRE(n_rows > 0, "%s: empty graph (n_rows = %lld); the reference script raises IndexError here", who, (long long)n_rows);
+    AGCN_REQUIRE(n_rows < (int64_t)INT32_MAX, "%s: n_rows = %lld does not fit the int32 row ids of .block4", who, (long long)n_rows);
+    AGCN_REQUIRE(d_block4 == nullptr || aligned16(d_block4), "%s: block4 output must be 16-byte aligned", who);
+    return AGCN_OK;
+}
+
+// Phases A and B: how many tuples there are and where every tile's begin.  Waits for the stream.
+// `who` names the entry point in error messages.
+static int partition_count(const char *who, const int *d_indptr, int64_t n_rows, int64_t *n_blocks, const PartScratch &sc, cudaStream_t s)
 {
     const int64_t tiles = ceil_div(n_rows, PART_TILE);
-    AGCN_CUDA(cudaMemsetAsync(sc.err, 0, sizeof(int), s));      // the one word that must start at zero
-    auto k_scan_max = single_block_scan_exclusive_kernel<int, OpMax>;
-    auto k_scan_add = single_block_scan_exclusive_kernel<int64_t, OpAdd>;
-    AGCN_KERNEL(part_run_heads_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.tile_head, sc.err);
-    AGCN_LAUNCH_CHECK("part_run_heads_kernel");
-    AGCN_KERNEL(k_scan_max, 1, 1024, s, sc.tile_head, tiles, -1, (int *)nullptr);
-    AGCN_LAUNCH_CHECK("single_block_scan_exclusive_kernel<max>");
-    AGCN_KERNEL(part_count_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, (const int *)sc.tile_head, sc.tile_count);
-    AGCN_LAUNCH_CHECK("part_count_kernel");
-    AGCN_KERNEL(k_scan_add, 1, 1024, s, sc.tile_count, tiles, (int64_t)0, sc.total);
-    AGCN_LAUNCH_CHECK("single_block_scan_exclusive_kernel<add>");
-
-    int64_t total = 0;
-    int err = 0;
-    AGCN_CUDA(cudaMemcpyAsync(&total, sc.total, sizeof(total), cudaMemcpyDeviceToHost, s));
-    AGCN_CUDA(cudaMemcpyAsync(&err, sc.err, sizeof(err), cudaMemcpyDeviceToHost, s));
-    AGCN_CUDA(cudaStreamSynchronize(s));
-    if (err != 0) {
+    AGCN_HOST_WORDS(words, s);
+    AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words.device());
+    AGCN_LAUNCH_CHECK("part_describe_kernel");
+    AGCN_KERNEL(part_scan_kernel, 1, PART_SCAN_BLOCK, s, (const PartTileInfo *)sc.info, tiles, sc.tile_head, sc.tile_offset, words.device());
+    AGCN_LAUNCH_CHECK("part_scan_kernel");
+    AGCN_CUDA(words.sync());
+    if (words[PART_WORD_NEGATIVE] != 0) {
         set_error("%s: indptr decreases somewhere (negative degree); "
                   "the reference script prints 'cur_degree number is wrong' and stops", who);
         return AGCN_ERR_RANGE;
     }
-    *n_blocks = total;
-    if (d_block4 == nullptr || cap_blocks == 0) return AGCN_OK;
-    if (cap_blocks < total) {
-        set_error("%s: %lld blocks needed, capacity %lld", who, (long long)total, (long long)cap_blocks);
+    *n_blocks = words[PART_WORD_TOTAL];
+    return AGCN_OK;
+}
+
+// Phase C, asynchronous.
+static int partition_emit(const int *d_indptr, int64_t n_rows, int64_t n_blocks, int *d_block4, const PartScratch &sc, cudaStream_t s)
+{
+    if (n_blocks == 0) return AGCN_OK;
+    AGCN_KERNEL(part_emit_kernel, (unsigned)ceil_div(n_rows, PART_TILE), PART_BLOCK, s, d_indptr, n_rows, (const int *)sc.tile_head,
+                (const int64_t *)sc.tile_offset, reinterpret_cast<int4 *>(d_block4));
+    AGCN_LAUNCH_CHECK("part_emit_kernel");
+    return AGCN_OK;
+}
+
+// Count and, given room, emit: what the one-call entry points do.
+static int partition_pipeline(const char *who, const int *d_indptr, int64_t n_rows, int *d_block4, int64_t cap_blocks,
+                              int64_t *n_blocks, const PartScratch &sc, cudaStream_t s)
+{
+    int rc = partition_count(who, d_indptr, n_rows, n_blocks, sc, s);
+    if (rc != AGCN_OK || d_block4 == nullptr || cap_blocks == 0) return rc;
+    if (cap_blocks < *n_blocks) {
+        set_error("%s: %lld blocks needed, capacity %lld", who, (long long)*n_blocks, (long long)cap_blocks);
         return AGCN_ERR_CAPACITY;
     }
-    if (total > 0) {
-        AGCN_KERNEL(part_emit_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, (const int *)sc.tile_head,
-                    (const int64_t *)sc.tile_count, reinterpret_cast<int4 *>(d_block4));
-        AGCN_LAUNCH_CHECK("part_emit_kernel");
-    }
+    rc = partition_emit(d_indptr, n_rows, *n_blocks, d_block4, sc, s);
+    if (rc != AGCN_OK) return rc;
     AGCN_CUDA(cudaStreamSynchronize(s));
     return AGCN_OK;
 }
@@ -64,23 +88,48 @@ static int partition_pipeline(const char *who, const int *d_indptr, int64_t n_ro
 int partition_device(const int *d_indptr, int64_t n_rows, int *d_block4, int64_t cap_blocks,
                      int64_t *n_blocks, cudaStream_t s)
 {
-    AGCN_REQUIRE(d_indptr != nullptr && n_blocks != nullptr, "agcn_partition: null pointer");
-    AGCN_REQUIRE(n_rows > 0, "agcn_partition: empty graph (n_rows = %lld); the reference script raises IndexError here",
-                 (long long)n_rows);
-    AGCN_REQUIRE(n_rows < (int64_t)INT32_MAX, "agcn_partition: n_rows = %lld does not fit the int32 row ids of .block4",
-                 (long long)n_rows);
-    AGCN_REQUIRE(d_block4 == nullptr || aligned16(d_block4), "agcn_partition: block4 output must be 16-byte aligned");
+    int rc = partition_check("agcn_partition", d_indptr, n_rows, d_block4, n_blocks);
+    if (rc != AGCN_OK) return rc;
     *n_blocks = 0;
-
     const int64_t tiles = ceil_div(n_rows, PART_TILE);
+    Carver size;
+    part_scratch(size, tiles);
     DeviceScratch scratch(s);
-    PartScratch sc;
-    AGCN_ALLOC(tile_head, scratch, int, tiles);
-    AGCN_ALLOC(tile_count, scratch, int64_t, tiles);
-    AGCN_ALLOC(d_total, scratch, int64_t, 1);
-    AGCN_ALLOC(d_err, scratch, int, 1);
-    sc.tile_head = tile_head; sc.tile_count = tile_count; sc.total = d_total; sc.err = d_err;
-    return partition_pipeline("agcn_partition", d_indptr, n_rows, d_block4, cap_blocks, n_blocks, sc, s);
+    AGCN_ALLOC(block, scratch, unsigned char, (int64_t)size.bytes());
+    Carver c(block);
+    return partition_pipeline("agcn_partition", d_indptr, n_rows, d_block4, cap_blocks, n_blocks, part_scratch(c, tiles), s);
+}
+
+int partition_begin(PartitionRun *run, const int *d_indptr, int64_t n_rows, cudaStream_t s)
+{
+    int rc = partition_check("agcn_partition", d_indptr, n_rows, nullptr, run);
+    if (rc != AGCN_OK) return rc;
+    const int64_t tiles = ceil_div(n_rows, PART_TILE);
+    Carver size;
+    part_scratch(size, tiles);
+    run->indptr = d_indptr; run->n_rows = n_rows; run->n_blocks = 0; run->stream = s;
+    const cudaError_t e = pool_alloc(&run->memory, size.bytes(), s);
+    if (e != cudaSuccess) {
+        set_error("agcn_partition: device allocation of %zu bytes: %s", size.bytes(), cudaGetErrorString(e));
+        return AGCN_ERR_CUDA;
+    }
+    Carver c(run->memory);
+    rc = partition_count("agcn_partition", d_indptr, n_rows, &run->n_blocks, part_scratch(c, tiles), s);
+    if (rc != AGCN_OK) { pool_free(run->memory, s); run->memory = nullptr; }
+    return rc;
+}
+
+int partition_finish(PartitionRun *run, int *d_block4)
+{
+    if (run->memory == nullptr) return AGCN_OK;
+    int rc = AGCN_OK;
+    if (d_block4 != nullptr) {
+        Carver c(run->memory);
+        rc = partition_emit(run->indptr, run->n_rows, run->n_blocks, d_block4, part_scratch(c, ceil_div(run->n_rows, PART_TILE)), run->stream);
+    }
+    pool_free(run->memory, run->stream);
+    run->memory = nullptr;
+    return rc;
 }
 
 }  // namespace agcn
@@ -92,6 +141,36 @@ extern "C" int agcn_partition_device(const int32_t *d_indptr, int64_t n_rows, in
     return agcn::partition_device(d_indptr, n_rows, d_block4, cap_blocks, n_blocks, static_cast<cudaStream_t>(stream));
 }
 
+// The two halves of a call whose output the caller allocates in between (agcn_partition_device does the
+// first half twice then: once to count and once to fill).
+extern "C" int agcn_partition_begin(const int32_t *d_indptr, int64_t n_rows, agcn_partition_run **run, int64_t *n_blocks, void *stream)
+{
+    using namespace agcn;
+    clear_error();
+    AGCN_REQUIRE(run != nullptr && n_blocks != nullptr, "agcn_partition_begin: null pointer");
+    *run = nullptr;
+    *n_blocks = 0;
+    agcn_partition_run *r = new (std::nothrow) agcn_partition_run;
+    AGCN_REQUIRE(r != nullptr, "agcn_partition_begin: out of host memory");
+    const int rc = partition_begin(&r->run, d_indptr, n_rows, static_cast<cudaStream_t>(stream));
+    if (rc != AGCN_OK) { delete r; return rc; }
+    *n_blocks = r->run.n_blocks;
+    *run = r;
+    return AGCN_OK;
+}
+
+extern "C" int agcn_partition_finish(agcn_partition_run *run, int32_t *d_block4)
+{
+    using namespace agcn;
+    clear_error();
+    AGCN_REQUIRE(run != nullptr, "agcn_partition_finish: null run");
+    const bool misaligned = d_block4 != nullptr && !aligned16(d_block4);
+    const int rc = partition_finish(&run->run, misaligned ? nullptr : d_block4);
+    delete run;
+    AGCN_REQUIRE(!misaligned, "agcn_partition_finish: block4 output must be 16-byte aligned");
+    return rc;
+}
+
 extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int32_t *h_block4,
                                    int64_t cap_blocks, int64_t *n_blocks)
 {
@@ -100,20 +179,28 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
     AGCN_REQUIRE(h_indptr != nullptr && n_blocks != nullptr, "agcn_partition_host: null pointer");
     AGCN_REQUIRE(n_rows > 0, "agcn_partition_host: empty graph (n_rows = %lld); the reference script raises IndexError here",
                  (long long)n_rows);
-    DeviceScratch scratch(nullptr);
+    *n_blocks = 0;
+    const cudaStream_t s = nullptr;
+    DeviceScratch scratch(s);
     AGCN_ALLOC(d_indptr, scratch, int, n_rows + 1);
-    AGCN_CUDA(cudaMemcpy(d_indptr, h_indptr, (size_t)(n_rows + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    int rc = partition_device(d_indptr, n_rows, nullptr, 0, n_blocks, nullptr);
-    if (rc != AGCN_OK || h_block4 == nullptr || cap_blocks == 0) return rc;
-    if (cap_blocks < *n_blocks) {
+    AGCN_CUDA(cudaMemcpyAsync(d_indptr, h_indptr, (size_t)(n_rows + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
+    PartitionRun run;
+    int rc = partition_begin(&run, d_indptr, n_rows, s);
+    if (rc != AGCN_OK) return rc;
+    *n_blocks = run.n_blocks;
+    const bool wanted = h_block4 != nullptr && cap_blocks != 0;
+    if (!wanted || run.n_blocks == 0 || cap_blocks < run.n_blocks) {
+        partition_finish(&run, nullptr);
+        if (!wanted || cap_blocks >= *n_blocks) return AGCN_OK;
         set_error("agcn_partition_host: %lld blocks needed, capacity %lld", (long long)*n_blocks, (long long)cap_blocks);
         return AGCN_ERR_CAPACITY;
     }
-    if (*n_blocks == 0) return AGCN_OK;
-    AGCN_ALLOC(d_block4, scratch, int, *n_blocks * 4);
-    rc = partition_device(d_indptr, n_rows, d_block4, *n_blocks, n_blocks, nullptr);
+    int *d_block4 = scratch.alloc<int>(run.n_blocks * 4);
+    rc = partition_finish(&run, d_block4);
+    if (d_block4 == nullptr) return AGCN_ERR_CUDA;
     if (rc != AGCN_OK) return rc;
-    AGCN_CUDA(cudaMemcpy(h_block4, d_block4, (size_t)*n_blocks * 16, cudaMemcpyDeviceToHost));
+    AGCN_CUDA(cudaMemcpyAsync(h_block4, d_block4, (size_t)*n_blocks * 16, cudaMemcpyDeviceToHost, s));
+    AGCN_CUDA(cudaStreamSynchronize(s));
     return AGCN_OK;
 }
 
@@ -125,10 +212,9 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
 // fails or steals from its pool), a latency-critical loop that cannot afford
 // the device-wide synchronisation cudaMalloc / cudaFree imply, or a plug-in
 // host that forbids allocation calls after start-up.  For them the tile
-// scratch of the partitioner (one run-head index and one tuple count per 2048
-// rows, plus the total and an error word) lives in a fixed array in the
+// scratch of the partitioner (28 bytes per 2048 rows) lives in a fixed array in the
 // library's device image instead of a per-call allocation.  Every GPU that
-// loads the library holds that array (about 96 KB) until the process exits,
+// loads the library holds that array (about 224 KB) until the process exits,
 // which is why it is sized for AGCN_PARTITION_NOALLOC_MAX_ROWS rows and no
 // more.
 //
@@ -136,9 +222,8 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
 // up once per device with cudaGetSymbolAddress, on the first call made with
 // that device current.  That first call should therefore happen before any
 // stream capture is started.  All calls on a device share the array and it
-// keeps what the previous call left: the error word is cleared at the start
-// of every call, everything else is overwritten before it is read.  Two calls
-// that overlap on the same GPU (different streams or threads) race on it.
+// keeps what the previous call left: everything is overwritten before it is
+// read.  Two calls that overlap on the same GPU (different streams or threads) race on it.
 // ---------------------------------------------------------------------------
 namespace agcn {
 
@@ -146,32 +231,27 @@ constexpr int64_t PART_NOALLOC_MAX_ROWS = AGCN_PARTITION_NOALLOC_MAX_ROWS;
 constexpr int64_t PART_NOALLOC_MAX_TILES = (PART_NOALLOC_MAX_ROWS + PART_TILE - 1) / PART_TILE;
 constexpr int PART_NOALLOC_MAX_DEVICES = 64;
 
-struct PartStaticScratch {
-    int64_t tile_count[PART_NOALLOC_MAX_TILES];
-    int64_t total;
-    int tile_head[PART_NOALLOC_MAX_TILES];
-    int err;
-};
+constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + sizeof(int64_t) + sizeof(int)) + 3 * 256;
 
 }  // namespace agcn
 
-static __device__ __align__(256) unsigned char g_part_static_scratch[sizeof(agcn::PartStaticScratch)];
+static __device__ __align__(256) unsigned char g_part_static_scratch[agcn::PART_STATIC_BYTES];
 
 namespace agcn {
 
 static std::mutex g_part_static_mutex;
-static PartStaticScratch *g_part_static_addr[PART_NOALLOC_MAX_DEVICES] = {};
+static void *g_part_static_addr[PART_NOALLOC_MAX_DEVICES] = {};
 
 // device address of the static scratch on the current device (looked up once per device)
-static int part_static_scratch(PartStaticScratch **out)
+static int part_static_scratch(void **out)
 {
     int dev = -1;
     AGCN_CUDA(cudaGetDevice(&dev));
     AGCN_REQUIRE(dev >= 0 && dev < PART_NOALLOC_MAX_DEVICES, "agcn_partition_device_noalloc: device ordinal %d not supported", dev);
     std::lock_guard<std::mutex> lock(g_part_static_mutex);
     if (g_part_static_addr[dev] == nullptr) {
-        PartStaticScratch *ptr = nullptr;
-        AGCN_CUDA(cudaGetSymbolAddress((void **)&ptr, g_part_static_scratch));
+        void *ptr = nullptr;
+        AGCN_CUDA(cudaGetSymbolAddress(&ptr, g_part_static_scratch));
         AGCN_REQUIRE(ptr != nullptr, "agcn_partition_device_noalloc: cudaGetSymbolAddress returned a null address");
         g_part_static_addr[dev] = ptr;
     }
@@ -190,17 +270,12 @@ static int partition_device_noalloc(const int *d_indptr, int64_t n_rows, int *d_
     AGCN_REQUIRE(d_block4 == nullptr || aligned16(d_block4), "agcn_partition_device_noalloc: block4 output must be 16-byte aligned");
     *n_blocks = 0;
 
-    PartStaticScratch *st = nullptr;
-    int rc = part_static_scratch(&st);
+    void *memory = nullptr;
+    int rc = part_static_scratch(&memory);
     if (rc != AGCN_OK) return rc;
-    // st is a device address: form member addresses by arithmetic only, never dereference it here
-    unsigned char *base = reinterpret_cast<unsigned char *>(st);
-    PartScratch sc;
-    sc.tile_count = reinterpret_cast<int64_t *>(base + offsetof(PartStaticScratch, tile_count));
-    sc.total = reinterpret_cast<int64_t *>(base + offsetof(PartStaticScratch, total));
-    sc.tile_head = reinterpret_cast<int *>(base + offsetof(PartStaticScratch, tile_head));
-    sc.err = reinterpret_cast<int *>(base + offsetof(PartStaticScratch, err));
-    return partition_pipeline("agcn_partition_device_noalloc", d_indptr, n_rows, d_block4, cap_blocks, n_blocks, sc, s);
+    Carver c(memory);
+    return partition_pipeline("agcn_partition_device_noalloc", d_indptr, n_rows, d_block4, cap_blocks, n_blocks,
+                              part_scratch(c, ceil_div(n_rows, PART_TILE)), s);
 }
 
 }  // namespace agcn

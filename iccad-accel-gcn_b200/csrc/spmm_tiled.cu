@@ -105,14 +105,14 @@ static int tiled_create(agcn_spmm_tiled **out, const int *d_indptr, const int *d
     for (int k = 0; k < n_ranges; k++) {
         const int *ip_k = indptr_t + (int64_t)k * per;
         const int64_t nnz_k = t->first[k + 1] - t->first[k];
-        int64_t nb = 0;
-        rc = partition_device(ip_k, n_rows, nullptr, 0, &nb, s);
+        PartitionRun run;
+        rc = partition_begin(&run, ip_k, n_rows, s);
         if (rc != AGCN_OK) return rc;
-        if (nb > 0) {
-            AGCN_CUDA(cudaMalloc(&t->block4[k], (size_t)nb * 16));
-            rc = partition_device(ip_k, n_rows, t->block4[k], nb, &nb, s);
-            if (rc != AGCN_OK) return rc;
-        }
+        const int64_t nb = run.n_blocks;
+        const cudaError_t e = nb > 0 ? cudaMalloc(&t->block4[k], (size_t)nb * 16) : cudaSuccess;
+        rc = partition_finish(&run, t->block4[k]);
+        AGCN_CUDA(e);
+        if (rc != AGCN_OK) return rc;
         t->n_blocks[k] = nb;
         rc = spmm_create(&t->plan[k], t->block4[k], nb, nnz_k > 0 ? t->idx + t->first[k] : nullptr, n_rows, n_cols, nnz_k, s);
         if (rc != AGCN_OK) return rc;

@@ -66,6 +66,13 @@ int agcn_partition_device(const int32_t *d_indptr, int64_t n_rows,
                           int32_t *d_block4, int64_t cap_blocks, int64_t *n_blocks,
                           void *stream);
 
+/* The same in two halves, for callers that allocate the output in between: begin counts (and waits for the
+ * stream), finish fills d_block4 [n_blocks x 4] behind what `stream` holds, without waiting, and ends the run
+ * (d_block4 == NULL only ends it).  d_indptr must stay unchanged until then. */
+typedef struct agcn_partition_run agcn_partition_run;
+int agcn_partition_begin(const int32_t *d_indptr, int64_t n_rows, agcn_partition_run **run, int64_t *n_blocks, void *stream);
+int agcn_partition_finish(agcn_partition_run *run, int32_t *d_block4);
+
 /* Same, host buffers in and out (what a ctypes replacement of the script
  * calls after np.fromfile, block_level_partition.py:31-34 / :105-106). */
 int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows,
@@ -77,7 +84,7 @@ int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows,
  * cannot take the device-wide synchronisation an allocation or free implies,
  * plug-in hosts that forbid allocation after start-up.  Same arguments, same
  * results and same error codes as agcn_partition_device, but the tile scratch
- * is a fixed array inside the library's device image (about 96 KB, resident on
+ * is a fixed array inside the library's device image (about 224 KB, resident on
  * every GPU that loads the library until the process exits) and the call makes
  * no cudaMalloc / cudaFree or other allocating call.
  *  - n_rows above AGCN_PARTITION_NOALLOC_MAX_ROWS is AGCN_ERR_INVALID.

@@ -108,3 +108,16 @@ def test_drop_in_script_same_files_as_the_reference(kat, tmp_path):
     for name in ("pubmed", "collab"):
         got = np.fromfile(tmp_path / "block_level_meta" / f"{name}.block4", dtype=np.int32)
         assert sha256_block4(got) == kat[name]["sha256"], name
+
+
+@pytest.mark.parametrize("run", [1, 2047, 2048, 2049, 6144, 5000])
+def test_runs_across_tiles_match_oracle(run):
+    # tiles of 2048 rows: a run that begins before a tile decides which of the tile's leading rows open a tuple
+    import torch
+    from accelgcn import partition
+    dev = require_cuda()
+    for degs in ([1, 40, 70, 100, 150, 300, 385], [0, 7], [33, 0, 33, 500]):
+        indptr = np.concatenate([[0], np.cumsum(np.repeat(degs, run))]).astype(np.int32)
+        want = oracle.partition(indptr)
+        assert np.array_equal(partition.block_level_partition(indptr), want)
+        assert np.array_equal(partition.block_level_partition_device(torch.from_numpy(indptr).to(dev)).cpu().numpy(), want)
