@@ -46,14 +46,6 @@ int exclusive_scan_i32_i64(const int *in, int64_t *out, int64_t n, int64_t *tile
 {
     return exclusive_scan<int, int64_t, int64_t>(in, out, n, tile_sums, total_out, s);
 }
-int exclusive_scan_u32_u32(const unsigned *in, unsigned *out, int64_t n, unsigned *tile_sums, cudaStream_t s)
-{
-    return exclusive_scan<unsigned, unsigned, unsigned>(in, out, n, tile_sums, (unsigned *)nullptr, s);
-}
-int exclusive_scan_u32_i32(const unsigned *in, int *out, int64_t n, int *tile_sums, cudaStream_t s)
-{
-    return exclusive_scan<unsigned, int, int>(in, out, n, tile_sums, (int *)nullptr, s);
-}
 
 }  // namespace agcn
 

@@ -127,11 +127,9 @@ private:
     type *var = (scratch).alloc<type>(count);                  \
     if (var == nullptr) return AGCN_ERR_CUDA
 
-// Exclusive prefix sums used by several entry points (defined in common.cu).
+// Exclusive prefix sum of a whole array (defined in common.cu).
 // tile_sums must hold ceil(n / 2048) elements.  total_out may be null.
 int exclusive_scan_i32_i64(const int *in, int64_t *out, int64_t n, int64_t *tile_sums, int64_t *total_out, cudaStream_t s);
-int exclusive_scan_u32_u32(const unsigned *in, unsigned *out, int64_t n, unsigned *tile_sums, cudaStream_t s);
-int exclusive_scan_u32_i32(const unsigned *in, int *out, int64_t n, int *tile_sums, cudaStream_t s);
 int64_t scan_tiles(int64_t n);
 
 }  // namespace agcn

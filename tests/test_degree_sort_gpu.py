@@ -116,3 +116,22 @@ def test_row_pointers_at_any_alignment():
         perm, nip, nix, _ = degree_sort.degree_sort_device(view, ix, None, relabel_cols=True)
         assert np.array_equal(perm.cpu().numpy(), want[0]), shift
         assert np.array_equal(nip.cpu().numpy(), want[1]) and np.array_equal(nix.cpu().numpy(), want[2]), shift
+
+
+@pytest.mark.parametrize("relabel", [False, True])
+@pytest.mark.parametrize("n,top", [(1, 5), (2047, 300), (2048, 3), (4095, 255), (4096, 256), (4097, 70_000), (12_289, 700), (70_001, 17_000_000)])
+def test_tile_edges_and_number_of_passes(n, top, relabel):
+    # rows around the sort tile (4096) and the row-pointer tile (2048); the largest degree decides how many of the
+    # four passes move anything (255 | 256, 65 536, 2^24), and puts rows across many tiles of the permute (2048 nonzeros)
+    from accelgcn import degree_sort
+    require_cuda()
+    rng = np.random.default_rng(n)
+    deg = rng.integers(0, min(top, 60) + 1, n)
+    deg[rng.integers(0, n)] = top
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    idx = rng.integers(0, n, int(indptr[-1]), dtype=np.int32)
+    val = rng.random(len(idx), dtype=np.float32)
+    got = degree_sort.degree_sort(indptr, idx, val, relabel_cols=relabel)
+    want = oracle.degree_sort(indptr, idx, val, relabel_cols=relabel)
+    for a, b, what in zip(got, want, ("perm", "indptr", "indices", "vals")):
+        assert np.array_equal(a, b), what
