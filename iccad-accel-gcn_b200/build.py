@@ -9,7 +9,7 @@ import subprocess
 import sys
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["common.cu", "memory.cu", "partition.cu", "degree_sort.cu", "spmm.cu", "spmm_tiled.cu", "host_spmm.cu", "gemm.cu", "layout.cu", "dist.cu", "probe.cu"]
+SOURCES = ["common.cu", "memory.cu", "host_copy.cu", "partition.cu", "degree_sort.cu", "spmm.cu", "spmm_tiled.cu", "host_spmm.cu", "gemm.cu", "layout.cu", "dist.cu", "probe.cu"]
 LIB = os.path.join(HERE, "lib", "libaccelgcn.so")
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared"]

@@ -1,6 +1,7 @@
 // C-ABI entry points of the degree sort (the ordering the reference assumes
 // of its <graph>.new_indptr / .new_indices inputs, main.cu:62-63).
 #include "host_common.h"
+#include "host_copy.h"
 #include "kernels/degree_sort_kernels.cuh"
 
 namespace agcn {
@@ -110,34 +111,33 @@ extern "C" int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_i
     const bool want_idx = h_new_indices != nullptr, want_val = h_new_vals != nullptr;
     AGCN_REQUIRE(!want_idx || (h_indices != nullptr && h_new_indptr != nullptr), "agcn_degree_sort_host: new_indices needs indices and new_indptr");
     AGCN_REQUIRE(!want_val || (h_vals != nullptr && want_idx), "agcn_degree_sort_host: new_vals needs vals and new_indices");
-    DeviceScratch scratch(nullptr);
-    AGCN_ALLOC(d_indptr, scratch, int, n_rows + 1);
-    AGCN_ALLOC(d_perm, scratch, int, n_rows);
-    AGCN_ALLOC(d_new_indptr, scratch, int, n_rows + 1);
-    int *d_indices = nullptr, *d_new_indices = nullptr;
+    const cudaStream_t s = nullptr;
+    DeviceScratch scratch(s);
+    unsigned char *block = nullptr;
+    int *d_indptr = nullptr, *d_perm = nullptr, *d_new_indptr = nullptr, *d_indices = nullptr, *d_new_indices = nullptr;
     float *d_vals = nullptr, *d_new_vals = nullptr;
-    AGCN_CUDA(cudaMemcpy(d_indptr, h_indptr, (size_t)(n_rows + 1) * sizeof(int), cudaMemcpyHostToDevice));
-    if (want_idx) {
-        d_indices = scratch.alloc<int>(nnz);
-        d_new_indices = scratch.alloc<int>(nnz);
-        if (d_indices == nullptr || d_new_indices == nullptr) return AGCN_ERR_CUDA;
-        AGCN_CUDA(cudaMemcpy(d_indices, h_indices, (size_t)nnz * sizeof(int), cudaMemcpyHostToDevice));
+    for (int round = 0; round < 2; round++) {
+        Carver c(block);
+        d_indptr = c.take<int>(n_rows + 1);
+        d_perm = c.take<int>(n_rows);
+        d_new_indptr = c.take<int>(n_rows + 1);
+        d_indices = want_idx ? c.take<int>(nnz) : nullptr;
+        d_new_indices = want_idx ? c.take<int>(nnz) : nullptr;
+        d_vals = want_val ? c.take<float>(nnz) : nullptr;
+        d_new_vals = want_val ? c.take<float>(nnz) : nullptr;
+        if (round == 0 && (block = scratch.alloc<unsigned char>((int64_t)c.bytes())) == nullptr) return AGCN_ERR_CUDA;
     }
-    if (want_val) {
-        d_vals = scratch.alloc<float>(nnz);
-        d_new_vals = scratch.alloc<float>(nnz);
-        if (d_vals == nullptr || d_new_vals == nullptr) return AGCN_ERR_CUDA;
-        AGCN_CUDA(cudaMemcpy(d_vals, h_vals, (size_t)nnz * sizeof(float), cudaMemcpyHostToDevice));
-    }
-    int rc = degree_sort_device(d_indptr, d_indices, d_vals, n_rows, nnz, relabel_cols, d_perm, d_new_indptr,
-                                d_new_indices, d_new_vals, nullptr);
+    const size_t row_bytes = (size_t)n_rows * sizeof(int), nz_bytes = (size_t)nnz * 4;
+    const HostSegment up[] = {{d_indptr, const_cast<int *>(h_indptr), row_bytes + sizeof(int)},
+                              {d_indices, const_cast<int *>(h_indices), want_idx ? nz_bytes : 0},
+                              {d_vals, const_cast<float *>(h_vals), want_val ? nz_bytes : 0}};
+    int rc = host_upload(up, 3, s);
     if (rc != AGCN_OK) return rc;
-    AGCN_CUDA(cudaMemcpy(h_perm, d_perm, (size_t)n_rows * sizeof(int), cudaMemcpyDeviceToHost));
-    if (h_new_indptr != nullptr)
-        AGCN_CUDA(cudaMemcpy(h_new_indptr, d_new_indptr, (size_t)(n_rows + 1) * sizeof(int), cudaMemcpyDeviceToHost));
-    if (want_idx && nnz > 0)
-        AGCN_CUDA(cudaMemcpy(h_new_indices, d_new_indices, (size_t)nnz * sizeof(int), cudaMemcpyDeviceToHost));
-    if (want_val && nnz > 0)
-        AGCN_CUDA(cudaMemcpy(h_new_vals, d_new_vals, (size_t)nnz * sizeof(float), cudaMemcpyDeviceToHost));
-    return AGCN_OK;
+    rc = degree_sort_device(d_indptr, d_indices, d_vals, n_rows, nnz, relabel_cols, d_perm, d_new_indptr, d_new_indices, d_new_vals, s);
+    if (rc != AGCN_OK) return rc;
+    const HostSegment down[] = {{d_perm, h_perm, row_bytes},
+                                {d_new_indptr, h_new_indptr, h_new_indptr != nullptr ? row_bytes + sizeof(int) : 0},
+                                {d_new_indices, h_new_indices, want_idx ? nz_bytes : 0},
+                                {d_new_vals, h_new_vals, want_val ? nz_bytes : 0}};
+    return host_download(down, 4, s);
 }

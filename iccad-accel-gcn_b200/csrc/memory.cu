@@ -6,6 +6,7 @@
 // of threads and streams, because the driver orders a block's next use after its last one.  What the pool
 // keeps between calls is bounded by POOL_KEEP_BYTES; agcn_release_scratch gives that back too.
 #include "host_common.h"
+#include "host_copy.h"
 
 #include <mutex>
 
@@ -114,5 +115,6 @@ extern "C" int agcn_release_scratch(void)
     AGCN_CUDA(pool_of_current_device(&pool));
     AGCN_CUDA(cudaDeviceSynchronize());
     AGCN_CUDA(cudaMemPoolTrimTo(pool, 0));
+    host_copy_release();
     return AGCN_OK;
 }

@@ -1,6 +1,7 @@
 // C-ABI entry points of the block-level partitioner
 // (replaces block_level_partition.py:38-106).
 #include "host_common.h"
+#include "host_copy.h"
 #include "internal.h"
 #include "kernels/partition_kernels.cuh"
 
@@ -183,9 +184,11 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
     const cudaStream_t s = nullptr;
     DeviceScratch scratch(s);
     AGCN_ALLOC(d_indptr, scratch, int, n_rows + 1);
-    AGCN_CUDA(cudaMemcpyAsync(d_indptr, h_indptr, (size_t)(n_rows + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
+    const HostSegment up = {d_indptr, const_cast<int *>(h_indptr), (size_t)(n_rows + 1) * sizeof(int)};
+    int rc = host_upload(&up, 1, s);
+    if (rc != AGCN_OK) return rc;
     PartitionRun run;
-    int rc = partition_begin(&run, d_indptr, n_rows, s);
+    rc = partition_begin(&run, d_indptr, n_rows, s);
     if (rc != AGCN_OK) return rc;
     *n_blocks = run.n_blocks;
     const bool wanted = h_block4 != nullptr && cap_blocks != 0;
@@ -199,9 +202,8 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
     rc = partition_finish(&run, d_block4);
     if (d_block4 == nullptr) return AGCN_ERR_CUDA;
     if (rc != AGCN_OK) return rc;
-    AGCN_CUDA(cudaMemcpyAsync(h_block4, d_block4, (size_t)*n_blocks * 16, cudaMemcpyDeviceToHost, s));
-    AGCN_CUDA(cudaStreamSynchronize(s));
-    return AGCN_OK;
+    const HostSegment down = {d_block4, h_block4, (size_t)*n_blocks * 16};
+    return host_download(&down, 1, s);
 }
 
 // ---------------------------------------------------------------------------
