@@ -488,7 +488,7 @@ extern "C" int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const 
     AGCN_CUDA(cudaMalloc(&f->d_status, 4 * sizeof(int)));
     AGCN_CUDA(cudaMemset(f->d_status, 0, 4 * sizeof(int)));
     for (cudaEvent_t &e : f->ev) AGCN_CUDA(cudaEventCreate(&e));
-    if (env_int("AGCN_GCN_FUSED", 0) != 0 && dist->plan != nullptr && dist->per > 0 && dist->n_blocks > 0) {
+    if (env_int("AGCN_GCN_FUSED", 0) != 0 && dist->plan != nullptr && dist->per > 0 && dist->n_blocks > 0 && !dist->plan->split) {
         // leading rows of at most 32 nonzeros (the block starts with its light rows in ascending degree), in whole tiles
         std::vector<int> h_indptr((size_t)dist->per + 1);
         AGCN_CUDA(cudaMemcpy(h_indptr.data(), dist->indptr, h_indptr.size() * sizeof(int), cudaMemcpyDeviceToHost));
@@ -496,7 +496,7 @@ extern "C" int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const 
         while (rows < dist->per && h_indptr[rows + 1] - h_indptr[rows] <= fused_layer_max_degree()) rows++;
         rows -= rows % 128;
         // the unit (8 tuples) that holds the first row left to the SpMM: first rows of every unit's first tuple
-        const int64_t n_units = ceil_div(dist->n_blocks, 8);
+        const int64_t n_units = dist->plan->n_units;
         std::vector<int> unit_row((size_t)n_units);
         AGCN_CUDA(cudaMemcpy2D(unit_row.data(), sizeof(int), dist->block4 + 1, 8 * 4 * sizeof(int), sizeof(int), (size_t)n_units,
                                cudaMemcpyDeviceToHost));

@@ -95,7 +95,7 @@ private:
 
 // Words in pinned host memory that kernels store results and error codes into (memory.cu).
 struct HostWords {
-    enum { COUNT = 6 };
+    enum { COUNT = 7 };
     int64_t w[COUNT];
 };
 

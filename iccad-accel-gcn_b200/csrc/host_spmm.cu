@@ -94,7 +94,8 @@ static int ctx_sync(agcn_host_ctx *c)
 // caller's host copy of .block4 (tuples tile [0, nnz) in order, so loc_begin is monotone).
 static void plan_parts(agcn_host_ctx *c, const int *h_block4, int want_parts)
 {
-    const int64_t n_units = ceil_div(c->n_blocks, HOST_SPMM_WARPS);
+    const int64_t n_units = c->plan->n_units;
+    if (c->plan->split) want_parts = 1;           // its units are not those of the caller's tuples (and it is small)
     c->part_unit.assign(1, 0);
     c->part_row.assign(1, 0);
     c->part_loc.assign(1, 0);

@@ -4,7 +4,9 @@
 
 struct agcn_spmm_plan {
     const int4 *block4 = nullptr;     // borrowed
-    int64_t n_blocks = 0, n_units = 0, n_rows = 0, n_cols = 0, nnz = 0;
+    const int4 *tuples = nullptr;     // what the kernels walk: block4, or the plan's own pieces of it (small plans)
+    bool split = false;
+    int64_t n_blocks = 0, n_tuples = 0, n_units = 0, n_rows = 0, n_cols = 0, nnz = 0;
     int device = -1;
     void *memory = nullptr;           // one pool block that holds the arrays below
     int2 *unit_carry = nullptr;       // [n_units]

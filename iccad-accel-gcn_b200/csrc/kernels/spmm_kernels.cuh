@@ -4,13 +4,14 @@
 // nonzeros; decode rules of spmm_accel.cu:18-34).
 //
 // Work decomposition.  A thread block ("unit") takes SPMM_WARPS consecutive
-// tuples, one per warp.  A warp first stages its tuple's (col, val) slice --
-// at most 384 pairs -- into shared memory with coalesced loads, then walks it.
+// tuples, one per warp.
+// A warp first stages its tuple's (col, val) slice -- at most 384 pairs -- into
+// shared memory with coalesced loads, then walks it.
 // The columns of one dense row are covered by a "slot" of S lanes, each lane
 // holding a float4 (the counterpart of the reference's combined warp,
 // spmm_accel.cu:36-53, with 16-byte instead of 4-byte lanes); a warp therefore
-// works on 32/S nonzeros at a time.  Rows of degree <= 32 are given one slot
-// each, longer rows are split over the slots of the warp and folded with
+// works on 32/S nonzeros at a time.  Rows of degree <= 32 are given whole to a
+// slot, longer rows are split over the slots of the warp and folded with
 // butterfly shuffles.  Accumulators live in registers.
 //
 // Heavy rows (degree > 384) span several tuples.  Their per-tuple partial sums
@@ -47,15 +48,17 @@ constexpr int SPMM_ZERO_ROWS_PER_BLOCK = 64;
 // and 2 x 6 / 2 x 7 by up to 30 % -- the gather wants occupancy more than per-warp depth.
 constexpr int SPMM_GATHER_BATCH = 4;
 constexpr int SPMM_MIN_BLOCKS = 40 / SPMM_WARPS;      // 40 resident warps per SM
-// Small launches (a few thread blocks per SM at most) cannot hide latency with occupancy: there each
-// warp walks its tuple alone, so the variant used for them trades registers for a deeper batch.
-constexpr int SPMM_SMALL_GATHER_BATCH = 16;
-constexpr int SPMM_SMALL_MIN_BLOCKS = 16 / SPMM_WARPS;
+// Small products (no more tuples than the GPU has room for warps) cannot hide latency with occupancy, and what they
+// wait for is the warp that walks 384 nonzeros alone.  Their plan cuts the tuples into pieces of fewer nonzeros
+// (plan_split_kernel), and the kernel keeps more gathers in flight per lane.
+constexpr int SPMM_SMALL_GATHER_BATCH = 8;
+constexpr int SPMM_SMALL_MIN_BLOCKS = 4;
 
 struct SpmmParams {
-    const int4 *block4;
-    int64_t n_blocks;
+    const int4 *tuples;       // the plan's: `.block4`, or its pieces
+    int64_t n_tuples;
     int64_t n_units;          // units of this launch (thread blocks beyond them zero-fill uncovered rows)
+    int light_every;          // order of the units: from the heavy end, but every light_every-th (0: none) from the light end
     int64_t unit_base;        // first unit of this launch: a product may be launched as several unit ranges
     const int *abort_flag;    // optional: a nonzero word makes every thread block return at once
     const int *idx;
@@ -177,6 +180,51 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
     return acc;
 }
 
+// `rows` consecutive rows of row_nz nonzeros each, whole rows for this lane: one stream of gathers, UNROLL in
+// flight across row boundaries.  (Row by row, rows of three nonzeros keep three gathers in flight and a slot with
+// six of them waits six times.)
+template <int UNROLL, bool PLAIN>
+__device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pairs, int rows, int row_nz, const float *__restrict__ x,
+                                             float *yr, int col, const L2Policies &pol)
+{
+    const int count = rows * row_nz;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    int left = row_nz;
+    auto take = [&](float a, const float4 &v) {
+        fma4(acc, a, v);
+        if (--left == 0) {
+            emit_row4<PLAIN>(p, yr, col, acc, p.relu, pol.stream);
+            acc = make_float4(0.f, 0.f, 0.f, 0.f);
+            left = row_nz;
+            yr += p.ldy;
+        }
+    };
+    int i = 0;
+    for (; i + UNROLL <= count; i += UNROLL) {
+        int2 q[UNROLL];
+        float4 v[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) q[u] = pairs[i + u];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)q[u].x * p.ldx, pol.keep);
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) take(__int_as_float(q[u].y), v[u]);
+    }
+    if (i < count) {
+        int2 q[UNROLL - 1];
+        float4 v[UNROLL - 1];
+#pragma unroll
+        for (int u = 0; u < UNROLL - 1; u++) {
+            const bool live = i + u < count;
+            q[u] = live ? pairs[i + u] : make_int2(0, 0);
+            v[u] = live ? ld_x4(x + (int64_t)q[u].x * p.ldx, pol.keep) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL - 1; u++)
+            if (i + u < count) take(__int_as_float(q[u].y), v[u]);
+    }
+}
+
 constexpr int SPMM_SCALAR_COLS = SPMM_PANEL / 32;   // columns per lane in scalar mode
 
 // Scalar mode: lane l owns columns l, l+32, ... (K = ceil(dim / 32) of them), every load instruction
@@ -288,7 +336,7 @@ spmm_units_kernel(const SpmmParams p)
     __shared__ int2 s_pair[SPMM_WARPS][SPMM_DEG_BOUND];
     __shared__ __align__(16) float s_part[SPMM_WARPS][SPMM_PANEL];
     __shared__ int s_row[SPMM_WARPS];
-    __shared__ int s_big[SPMM_WARPS];
+    __shared__ int s_big[SPMM_WARPS];               // the warp left a partial sum of row s_row in s_part
 
     constexpr bool VEC = S > 0;
     constexpr int LANES = VEC ? S : 32;
@@ -316,12 +364,14 @@ spmm_units_kernel(const SpmmParams p)
         return;
     }
 
-    const int64_t unit = p.unit_base + blockIdx.x;
+    const unsigned b = blockIdx.x, k = p.light_every, n = (unsigned)p.n_units;
+    const int64_t unit = p.unit_base + (k != 0 && b % k == k - 1 ? b / k : n - 1 - (k != 0 ? b - b / k : b));
     const int64_t e = unit * SPMM_WARPS + w;
-    const TupleView t = decode_tuple(p.block4, e, p.n_blocks);
+    const TupleView t = decode_tuple(p.tuples, e, p.n_tuples);
+    const bool big = t.valid && !t.small;
     const int total = t.n_rows * t.row_nz;
 
-    // stage the tuple's (col, val) slice
+    // stage the tuple's (col, val) pairs
     {
         const int *__restrict__ gi = p.idx + t.loc;
         const float *__restrict__ gv = p.val + t.loc;
@@ -331,17 +381,16 @@ spmm_units_kernel(const SpmmParams p)
     }
     __syncwarp();
 
-    const bool big = t.valid && !t.small;
     const int2 *pairs = s_pair[w];
 
     if (VEC) {
         const float *xc = p.x + col;
-        if (t.small && NS > 1 && t.row_nz <= 32) {
-            // one slot per row
-            for (int r = slot; r < t.n_rows; r += NS) {
-                const float4 acc = gather_vec4<BATCH>(pairs + r * t.row_nz, t.row_nz, 0, 1, xc, p.ldx, active, pol.keep);
-                if (active) emit_row4<PLAIN>(p, p.y + (int64_t)(t.row0 + r) * p.ldy, col, acc, p.relu, pol.stream);
-            }
+        if (t.small && t.row_nz <= 32) {
+            // whole rows for every slot, consecutive ones
+            const int each = (t.n_rows + NS - 1) / NS, r0 = slot * each;
+            const int rows = r0 < t.n_rows ? (r0 + each < t.n_rows ? each : t.n_rows - r0) : 0;
+            if (active)
+                gather_rows4<BATCH, PLAIN>(p, pairs + r0 * t.row_nz, rows, t.row_nz, xc, p.y + (int64_t)(t.row0 + r0) * p.ldy, col, pol);
         } else {
             // the slots of the warp share each row
             for (int r = 0; r < t.n_rows; r++) {
@@ -381,7 +430,7 @@ spmm_units_kernel(const SpmmParams p)
     if (w > 0 && s_big[w - 1] && s_row[w - 1] == t.row0) return;   // not the first tuple of its row here
     int w_end = w + 1;
     while (w_end < SPMM_WARPS && s_big[w_end] && s_row[w_end] == t.row0) w_end++;
-    const int64_t left = p.n_blocks - unit * SPMM_WARPS;
+    const int64_t left = p.n_tuples - unit * SPMM_WARPS;
     const int w_last = left < SPMM_WARPS ? (int)left - 1 : SPMM_WARPS - 1;
     const int2 uc = __ldg(p.unit_carry + unit);
     const bool enters = w == 0 && uc.x >= 0;            // the row began in an earlier unit
@@ -463,7 +512,7 @@ __device__ __forceinline__ bool tuple_is_big(const int4 &b) { return b.x > SPMM_
 __device__ __forceinline__ int tuple_rows(const int4 &b) { return tuple_is_big(b) ? 1 : (b.w & 0xffff); }
 
 // Error bits are single words of the host so that blocks can store to them without atomics.
-constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_ERR = 2;      // then one word per SPMM_ERR_* bit
+constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_ERR = 3;      // then one word per SPMM_ERR_* bit
 constexpr int PLAN_ERR_BITS = 4;
 constexpr int PLAN_BLOCK = 256;      // units per thread block, one per thread
 
@@ -498,6 +547,31 @@ __device__ __forceinline__ int tuple_errors(bool has_prev, const int4 &a, const 
     return err;
 }
 
+// How a tuple is cut into pieces of at most `most` nonzeros: whole rows where they fit, otherwise every row by itself.
+// A piece has the form of a tuple; one that is part of a row says so by a degree above the bound.
+struct TupleCut {
+    int pieces, rows_each, row_pieces, nz_each;
+};
+__device__ __forceinline__ TupleCut tuple_cut(const int4 &b, int most)
+{
+    const int rows = tuple_rows(b), row_nz = tuple_is_big(b) ? b.w : b.x;
+    TupleCut c;
+    if (row_nz <= most && !tuple_is_big(b)) {
+        const int fit = most / row_nz;
+        c.pieces = (rows + fit - 1) / fit;
+        c.rows_each = (rows + c.pieces - 1) / c.pieces;
+        c.pieces = (rows + c.rows_each - 1) / c.rows_each;
+        c.row_pieces = 0; c.nz_each = 0;
+    } else {
+        c.row_pieces = (row_nz + most - 1) / most;
+        c.nz_each = (row_nz + c.row_pieces - 1) / c.row_pieces;
+        c.row_pieces = (row_nz + c.nz_each - 1) / c.nz_each;
+        c.pieces = rows * c.row_pieces;
+        c.rows_each = 0;
+    }
+    return c;
+}
+
 // Does a heavy row enter unit u from the left / leave it to the right?
 __device__ __forceinline__ void unit_crossings(const int4 *__restrict__ block4, int64_t n_blocks, int64_t u,
                                                bool &enters, bool &leaves, bool &same_row, int &row_in, int &row_out)
@@ -521,12 +595,13 @@ __device__ __forceinline__ void unit_crossings(const int4 *__restrict__ block4, 
 // First pass over a `.block4` array: validates every tuple (and, in the blocks behind the tuple blocks,
 // every column id), and counts per PLAN_BLOCK units the rows no tuple covers and the carry slots.  One
 // launch and one read of 16 bytes per tuple and 4 per nonzero: bound by HBM for large graphs, by launch
-// latency for small ones.  ctl[0], ctl[1]: totals, ctl[2]: blocks done (zero at launch).
+// latency for small ones.  most > 0: also counts the pieces of at most that many nonzeros the tuples would be cut
+// into.  ctl[0..2]: totals, ctl[3]: blocks done (zero at launch).
 __global__ void __launch_bounds__(PLAN_BLOCK)
 plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int64_t n_rows, int64_t nnz,
                   const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned unit_grid,
-                  int64_t *__restrict__ tile_zero, int *__restrict__ tile_carry, unsigned long long *__restrict__ ctl,
-                  HostWords *out)
+                  int most, int64_t *__restrict__ tile_zero, int *__restrict__ tile_carry, int *__restrict__ tile_pieces,
+                  unsigned long long *__restrict__ ctl, HostWords *out)
 {
     if (blockIdx.x >= unit_grid) {
         const int64_t stride = (int64_t)(gridDim.x - unit_grid) * blockDim.x;
@@ -540,17 +615,19 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
         return;
     }
     __shared__ int64_t s_zero[PLAN_BLOCK / 32];
-    __shared__ int s_carry[PLAN_BLOCK / 32];
+    __shared__ int s_carry[PLAN_BLOCK / 32], s_pieces[PLAN_BLOCK / 32];
     const int64_t u = (int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x;
     int64_t zero = 0;
-    int carry = 0, err = 0;
+    int carry = 0, err = 0, pieces = 0;
     if (u < n_units || (n_units == 0 && u == 0)) {          // without any tuple, one thread counts the rows
         const int64_t e0 = u * SPMM_WARPS;
         const int64_t e1 = e0 + SPMM_WARPS < n_blocks ? e0 + SPMM_WARPS : n_blocks;
         int4 a = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
         for (int64_t e = e0; e < e1; e++) {
             const int4 b = block4[e];
-            err |= tuple_errors(e > 0, a, b, n_rows, nnz);
+            const int tuple_err = tuple_errors(e > 0, a, b, n_rows, nnz);
+            err |= tuple_err;
+            if (most > 0 && tuple_err == 0) pieces += tuple_cut(b, most).pieces;
             const int64_t g = tuple_gap(e > 0, a, b);
             zero += g > 0 ? g : 0;
             a = b;
@@ -566,20 +643,24 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
     if (err) plan_report(out, err);
     zero = warp_reduce(zero, OpAdd());
     carry = warp_reduce(carry, OpAdd());
-    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; }
+    pieces = warp_reduce(pieces, OpAdd());
+    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; s_pieces[warp_id()] = pieces; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        zero = 0; carry = 0;
-        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; }
+        zero = 0; carry = 0; pieces = 0;
+        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; pieces += s_pieces[w]; }
         tile_zero[blockIdx.x] = zero;
         tile_carry[blockIdx.x] = carry;
+        tile_pieces[blockIdx.x] = pieces;
         atomicAdd(ctl + 0, (unsigned long long)zero);
         atomicAdd(ctl + 1, (unsigned long long)carry);
+        atomicAdd(ctl + 2, (unsigned long long)pieces);
         __threadfence();
-        if (atomicAdd(ctl + 2, 1ull) == unit_grid - 1) {
+        if (atomicAdd(ctl + 3, 1ull) == unit_grid - 1) {
             __threadfence();
             out->w[PLAN_WORD_ZERO] = (int64_t)__ldcg(ctl + 0);
             out->w[PLAN_WORD_CARRY] = (int64_t)__ldcg(ctl + 1);
+            out->w[PLAN_WORD_PIECES] = (int64_t)__ldcg(ctl + 2);
         }
     }
 }
@@ -608,9 +689,37 @@ __device__ __forceinline__ int64_t tuple_lower_bound(const int4 *__restrict__ bl
     return lo;
 }
 
+// Writes the pieces of every tuple, in tuple order (small plans only: a handful of thread blocks).
+__global__ void __launch_bounds__(PLAN_BLOCK)
+plan_split_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int most, const int *__restrict__ tile_pieces, int4 *__restrict__ pieces)
+{
+    __shared__ int s_scan[PLAN_BLOCK / 32 + 1];
+    int before = 0, base, total;
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += PLAN_BLOCK) before += tile_pieces[k];
+    block_scan_exclusive<PLAN_BLOCK>(before, OpAdd(), 0, base, s_scan);
+    const int64_t e0 = ((int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x) * SPMM_WARPS;
+    int mine = 0;
+    for (int64_t e = e0; e < e0 + SPMM_WARPS && e < n_blocks; e++) mine += tuple_cut(block4[e], most).pieces;
+    int4 *out = pieces + base + block_scan_exclusive<PLAN_BLOCK>(mine, OpAdd(), 0, total, s_scan);
+    for (int64_t e = e0; e < e0 + SPMM_WARPS && e < n_blocks; e++) {
+        const int4 b = block4[e];
+        const TupleCut c = tuple_cut(b, most);
+        const int rows = tuple_rows(b), row_nz = tuple_is_big(b) ? b.w : b.x;
+        if (c.row_pieces == 0) {
+            for (int r = 0; r < rows; r += c.rows_each)
+                *out++ = make_int4(b.x, b.y + r, b.z + r * row_nz, rows - r < c.rows_each ? rows - r : c.rows_each);
+        } else {
+            for (int r = 0; r < rows; r++)
+                for (int k = 0; k < row_nz; k += c.nz_each)
+                    *out++ = make_int4(SPMM_DEG_BOUND + 1, b.y + r, b.z + r * row_nz + k, row_nz - k < c.nz_each ? row_nz - k : c.nz_each);
+        }
+    }
+}
+
 // Second pass: carry slots in unit order, and the list of rows no tuple covers.  A block adds up the counts
 // of the tiles before it itself (a few thousand words at most) -- no scan launches between the passes.
 // Gaps of many rows (the degree-0 rows of an ordered graph are one gap) are written by the whole block.
+// tile_zero == nullptr: the tuples are pieces nobody has counted; a block counts the units before its own (few).
 constexpr int PLAN_INLINE_GAP = 16, PLAN_GAP_QUEUE = 64;
 
 __global__ void __launch_bounds__(PLAN_BLOCK)
@@ -624,7 +733,19 @@ plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_
     __shared__ int s_gaps;
     if (threadIdx.x == 0) s_gaps = 0;
     int64_t zb = 0, cb = 0;
-    for (int64_t k = threadIdx.x; k < blockIdx.x; k += PLAN_BLOCK) { zb += tile_zero[k]; cb += tile_carry[k]; }
+    if (tile_zero != nullptr) {
+        for (int64_t k = threadIdx.x; k < blockIdx.x; k += PLAN_BLOCK) { zb += tile_zero[k]; cb += tile_carry[k]; }
+    } else {
+        for (int64_t k = threadIdx.x; k < (int64_t)blockIdx.x * PLAN_BLOCK; k += PLAN_BLOCK) {
+            bool en, lv, same;
+            int ri, ro;
+            unit_crossings(block4, n_blocks, k, en, lv, same, ri, ro);
+            cb += (en ? 1 : 0) + (lv ? 1 : 0) - (same ? 1 : 0);
+            if (zero_rows != nullptr)
+                for (int64_t e = k * SPMM_WARPS; e < (k + 1) * SPMM_WARPS; e++)
+                    zb += tuple_gap(e > 0, e > 0 ? block4[e - 1] : make_int4(0, 0, 0, 0), block4[e]);
+        }
+    }
     int64_t zero_base, carry_base, total;
     block_scan_exclusive<PLAN_BLOCK>(zb, OpAdd(), (int64_t)0, zero_base, s_scan64);
     block_scan_exclusive<PLAN_BLOCK>(cb, OpAdd(), (int64_t)0, carry_base, s_scan64);

@@ -27,6 +27,32 @@ void plan_free(agcn_spmm_plan *p)
     delete p;
 }
 
+// Nonzeros per piece when the tuples of a plan are to be cut into pieces, 0 when they are not.  A product ends with
+// its longest warp, so pieces are as small as they can be while the GPU still takes them in little more than one
+// wave (it holds 32 to 40 warps per SM); cutting in half pays up to about two waves, beyond that the extra warps
+// cost more than they balance.  us per product, uncut / cut, B200: 16 384 rows of 8 nonzeros (10 tuples per SM),
+// dim 60: 17.7 / 9.2, dim 128: 31 / 11; 40 000 rows of 10 (26), dim 128: 34 / 18; 100 000 rows of 8 (63), dim 128:
+// 50 / 33 -- but 100 000 rows of 25 (86), dim 32: 25 / 33.
+static int spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
+{
+    for (int most : {64, 96, 128, 192})
+        if (n_blocks + nnz / most - nnz / SPMM_DEG_BOUND <= (int64_t)(most < 192 ? 48 : 80) * sm_count) return most;
+    return 0;
+}
+
+// Order of the units, which are in ascending degree.  Starting at the heavy end leaves light units for the end of
+// the launch (500 000 rows of 12, dim 64: 159 -> 144 us).  Where nearly all tuples are full there is nothing to
+// balance, and units from both ends in turn are faster by 4-10 % (250 000 rows of 490, dim 32: 934 -> 872 us;
+// 20 000 rows of 400: 82 -> 72 us).  In between, with X in L2 and many waves, every fourth unit from the light end
+// is (500 000 skewed rows of 29, dim 32: 152 -> 146 us); with X beyond L2 it is not (5 M rows, dim 128: 5.59 -> 5.68 ms).
+static int spmm_light_every(const agcn_spmm_plan *p, int width)
+{
+    if (p->split) return 0;
+    if (p->nnz >= 250 * p->n_blocks) return 2;
+    const double x_bytes = (double)p->n_cols * width * 4.0;
+    return p->n_units > (int64_t)28 * p->sm_count && x_bytes <= 0.6 * p->l2_bytes ? 4 : 0;
+}
+
 // Two launches: the first pass counts and validates, the host sizes the plan's one pool block from its
 // answer, the second pass fills it.  (Six cudaMalloc / cudaFree pairs and nine launches before; a plan of
 // 16 384 rows took about 1 ms, most of it in the allocator.)
@@ -43,24 +69,29 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
     AGCN_REQUIRE(n_blocks < (int64_t)INT32_MAX, "agcn_spmm_create: too many blocks");
 
     const int4 *block4 = reinterpret_cast<const int4 *>(d_block4);
+    int device = 0, sm_count = 0, l2_bytes = 0;
+    AGCN_CUDA(cudaGetDevice(&device));
+    AGCN_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+    AGCN_CUDA(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, device));
     const int64_t n_units = ceil_div(n_blocks, SPMM_WARPS);
+    const int most = n_blocks > 0 ? env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count)) : 0;
     const int64_t tiles = n_units > 0 ? ceil_div(n_units, PLAN_BLOCK) : 1;
     DeviceScratch scratch(s);
     Carver size;
-    size.take<unsigned long long>(3); size.take<int64_t>(tiles); size.take<int>(tiles);
+    size.take<unsigned long long>(4); size.take<int64_t>(tiles); size.take<int>(tiles); size.take<int>(tiles);
     AGCN_ALLOC(block, scratch, unsigned char, (int64_t)size.bytes());
     Carver c(block);
-    unsigned long long *ctl = c.take<unsigned long long>(3);
+    unsigned long long *ctl = c.take<unsigned long long>(4);
     int64_t *tile_zero = c.take<int64_t>(tiles);
-    int *tile_carry = c.take<int>(tiles);
+    int *tile_carry = c.take<int>(tiles), *tile_pieces = c.take<int>(tiles);
     AGCN_HOST_WORDS(words, s);
-    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 3 * sizeof(*ctl), s));
+    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(*ctl), s));
     // 16 column ids per thread, at most 64 thread blocks per SM's worth of them
     const int64_t n_idx = d_indices != nullptr ? nnz : 0;
     const int64_t col_grid = n_idx > 0 ? ceil_div(n_idx, PLAN_BLOCK * 16) : 0;
     const unsigned grid = (unsigned)(tiles + (col_grid < 9472 ? col_grid : 9472));
     AGCN_KERNEL(plan_check_kernel, grid, PLAN_BLOCK, s, block4, n_blocks, n_units, n_rows, nnz, d_indices, n_idx, n_cols, (unsigned)tiles,
-                tile_zero, tile_carry, ctl, words.device());
+                most, tile_zero, tile_carry, tile_pieces, ctl, words.device());
     AGCN_LAUNCH_CHECK("plan_check_kernel");
     AGCN_CUDA(words.sync());
     int err = 0;
@@ -77,13 +108,19 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
     agcn_spmm_plan *p = new (std::nothrow) agcn_spmm_plan;
     AGCN_REQUIRE(p != nullptr, "agcn_spmm_create: out of host memory");
     struct Guard { agcn_spmm_plan *p; ~Guard() { plan_free(p); } } guard{p};       // frees the half-built plan on every early return
-    AGCN_CUDA(cudaGetDevice(&p->device));
-    p->block4 = block4; p->n_blocks = n_blocks; p->n_units = n_units;
+    p->device = device; p->sm_count = sm_count; p->l2_bytes = l2_bytes;
+    p->block4 = block4; p->n_blocks = n_blocks;
+    p->split = most > 0;
+    p->n_tuples = p->split ? words[PLAN_WORD_PIECES] : n_blocks;
+    p->n_units = ceil_div(p->n_tuples, SPMM_WARPS);
     p->n_rows = n_rows; p->n_cols = n_cols; p->nnz = nnz;
-    p->n_zero = words[PLAN_WORD_ZERO]; p->n_carry = words[PLAN_WORD_CARRY];
+    p->n_zero = words[PLAN_WORD_ZERO];
+    p->n_carry = p->split ? 2 * p->n_units : words[PLAN_WORD_CARRY];       // of pieces only a bound is known here
+    int4 *pieces = nullptr;
     for (int pass = 0; pass < 2; pass++) {
         Carver m(p->memory);
-        p->unit_carry = m.take<int2>(n_units);
+        pieces = p->split ? m.take<int4>(p->n_tuples) : nullptr;
+        p->unit_carry = m.take<int2>(p->n_units);
         p->carry_span = m.take<int2>(p->n_carry);
         p->carry_row = m.take<int>(p->n_carry);
         p->carry = m.take<unsigned char>((int64_t)spmm_carry_bytes(p->n_carry));
@@ -97,16 +134,23 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
     }
     if (p->n_carry > 0)
         AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(p->carry, p->n_carry), 0, (size_t)p->n_carry * SPMM_CARRY_PASSES * sizeof(int), s));
+    p->tuples = block4;
+    if (p->split) {
+        AGCN_KERNEL(plan_split_kernel, (unsigned)tiles, PLAN_BLOCK, s, block4, n_blocks, most, (const int *)tile_pieces, pieces);
+        AGCN_LAUNCH_CHECK("plan_split_kernel");
+        p->tuples = pieces;
+        tile_zero = nullptr;             // they were counted for the uncut tuples
+    }
     if (p->n_carry > 0 || p->n_zero > 0) {
-        AGCN_KERNEL(plan_assign_kernel, (unsigned)tiles, PLAN_BLOCK, s, block4, n_blocks, n_units, n_rows, (const int64_t *)tile_zero,
-                    (const int *)tile_carry, p->unit_carry, p->carry_span, p->carry_row, p->n_zero > 0 ? p->zero_rows : nullptr);
+        const int64_t assign_tiles = p->n_units > 0 ? ceil_div(p->n_units, PLAN_BLOCK) : 1;
+        AGCN_KERNEL(plan_assign_kernel, (unsigned)assign_tiles, PLAN_BLOCK, s, p->tuples, p->n_tuples, p->n_units, n_rows,
+                    (const int64_t *)tile_zero, (const int *)tile_carry, p->unit_carry, p->carry_span, p->carry_row,
+                    p->n_zero > 0 ? p->zero_rows : nullptr);
         AGCN_LAUNCH_CHECK("plan_assign_kernel");
     } else if (n_units > 0) {
         AGCN_CUDA(cudaMemsetAsync(p->unit_carry, 0xff, (size_t)n_units * sizeof(int2), s));      // no row crosses units
     }
     AGCN_CUDA(cudaStreamSynchronize(s));          // products may run on any stream
-    AGCN_CUDA(cudaDeviceGetAttribute(&p->l2_bytes, cudaDevAttrL2CacheSize, p->device));
-    AGCN_CUDA(cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device));
     p->panel_override = env_int("AGCN_SPMM_PANEL", 0);
     p->pad_unaligned = env_int("AGCN_SPMM_PAD", 1);
     guard.p = nullptr;
@@ -131,7 +175,7 @@ static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaS
     AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm);
 }
 
-// `small` launches always finish the rows that cross units themselves.
+// `small` launches (of a plan that is cut into pieces) always finish the rows that cross units themselves.
 template <int S>
 static void launch_units_for(const SpmmParams &prm, unsigned grid, bool small, bool plain, bool finish, cudaStream_t s)
 {
@@ -209,7 +253,6 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     const int64_t zero_blocks = !part.zero_fill || (accumulate && !activation) ? 0 : ceil_div(p->n_zero, SPMM_ZERO_ROWS_PER_BLOCK);
     const int64_t grid = (unit1 - unit0) + zero_blocks;
     AGCN_REQUIRE(grid < (int64_t)INT32_MAX, "agcn_spmm_run: grid too large");
-    const bool small = p->n_units <= (int64_t)SPMM_SMALL_MIN_BLOCKS * p->sm_count;
 
     // Column panels.  The gather re-reads a row of X once per nonzero of that column, so it runs
     // at L2 speed only while the X columns of a pass stay L2-resident.  When dim > 64 and the
@@ -231,7 +274,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     const bool whole = unit0 == 0 && unit1 == p->n_units;
     // Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM),
     // where a second launch costs more than blocks that wait for a counter; parts of a product always do that.
-    const bool carry_inside = !whole || p->n_units <= (int64_t)20 * p->sm_count;
+    const bool carry_inside = !whole || p->split || p->n_units <= (int64_t)20 * p->sm_count;
     // A carry slot holds SPMM_PANEL floats and every column pass uses its own columns (and arrival
     // counters) of it, so a product of up to SPMM_PANEL columns can be issued in parts whatever its
     // passes are -- with the same passes, hence the same bits, as a whole run.
@@ -242,8 +285,9 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     for (int col0 = 0; col0 < dim; col0 += panel) {
         const int width = dim - col0 < panel ? dim - col0 : panel;
         SpmmParams prm;
-        prm.block4 = p->block4; prm.n_blocks = p->n_blocks;
+        prm.tuples = p->tuples; prm.n_tuples = p->n_tuples;
         prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag;
+        prm.light_every = spmm_light_every(p, width);
         prm.idx = d_indices; prm.val = d_vals;
         prm.x = x_use + col0; prm.ldx = ldx_use;
         prm.y = d_y + col0; prm.ldy = ldy;
@@ -262,7 +306,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
         const bool plain = !accumulate && (vec ? y_vec : true);
         if (grid > 0) {
-            launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, small, plain, carry_inside, s);
+            launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, p->split, plain, carry_inside, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;
         }

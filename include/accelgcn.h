@@ -151,7 +151,8 @@ int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_indices, con
  * instead) and unaligned rows of Y get element-wise stores.  dim > 64 may run
  * as two 64-column passes when X is larger than L2 (environment variable
  * AGCN_SPMM_PANEL = columns per pass, read at plan creation, overrides that
- * choice).  A plan must not be run concurrently on two streams (the runs share
+ * choice).  Plans of few tuples hold a copy of them cut into pieces of 64 to 192
+ * nonzeros (AGCN_SPMM_PIECE = nonzeros per piece, 0 = uncut, overrides the choice).  A plan must not be run concurrently on two streams (the runs share
  * its scratch).
  * ---------------------------------------------------------------------- */
 typedef struct agcn_spmm_plan agcn_spmm_plan;

@@ -459,6 +459,18 @@ def test_forced_column_passes_on_small_graphs(cfg1, cfg4_small, panel, monkeypat
             case.check(x, case.run(x))
 
 
+@pytest.mark.parametrize("piece", [0, 7, 64, 100, 192])
+def test_tuples_cut_into_pieces(cfg1, cfg4_small, piece, monkeypatch):
+    # AGCN_SPMM_PIECE (read at plan creation): 0 = uncut, the form of large plans (heavy rows across units, light and
+    # heavy units in turn); pieces that do not divide a row, hold several rows, or make a row cross many units
+    monkeypatch.setenv("AGCN_SPMM_PIECE", str(piece))
+    holes = Case(1, 0.25, empty_rows=(0, 5, 1000, 1001, 1002, 4095))
+    for case in (cfg1, cfg4_small, holes):
+        for dim in (128, 61, 16):
+            x = case.x(dim)
+            case.check(x, case.run(x))
+
+
 def test_full_size_config3():
     # N = 2 400 000, ~6e7 nonzeros, dim 64: the whole product against the CPU oracle (fp64 accumulation)
     import torch
