@@ -7,9 +7,10 @@
 //  - uploads, kernels and downloads run on three streams chained by events;
 //  - a product is launched as several unit ranges (a unit = 8 consecutive tuples), and the rows a
 //    range completes are downloaded while the next range computes;
-//  - when the graph itself is part of the call (agcn_spmm_host_batch), column ids and values are
-//    uploaded in the same ranges and every range is multiplied -- for all products -- as soon as
-//    it has arrived, so the kernels and the downloads hide under the upload of A.
+//  - when the graph itself is part of the call (agcn_spmm_host_batch), column ids and values go up in
+//    the same ranges, between the X, in the order that makes most rows of Y ready per byte (upload_order),
+//    and every (range, product) pair is multiplied as soon as both are there, so the kernels and the
+//    downloads hide under the uploads.
 // One cudaMemcpyAsync per copy; pinned host memory gives full overlap (pageable memory works,
 // staged by the driver).
 #include "host_common.h"
@@ -29,8 +30,8 @@ struct agcn_host_ctx {
     cudaStream_t s_up = nullptr, s_run = nullptr, s_down = nullptr;
     void *graph[3] = {nullptr, nullptr, nullptr};     // block4, idx, val
     size_t graph_cap[3] = {0, 0, 0};
-    std::vector<void *> xbuf, ybuf, cbuf;             // per product of a batch: X, Y, carry scratch
-    std::vector<size_t> xcap, ycap, ccap;
+    std::vector<void *> xbuf, xpad, ybuf, cbuf;       // per product of a batch: X, its aligned copy, Y, carry scratch
+    std::vector<size_t> xcap, pcap, ycap, ccap;
     agcn_spmm_plan *plan = nullptr;                   // of the graph set last
     int64_t n_rows = 0, n_cols = 0, nnz = 0, n_blocks = 0;
     // unit ranges a product is issued in, with the first row / first nonzero of each boundary
@@ -68,12 +69,19 @@ static int ctx_chain(agcn_host_ctx *c, cudaStream_t from, cudaStream_t to)
     return AGCN_OK;
 }
 
-static int reserve(void **buf, size_t *cap, size_t bytes)
+// The buffers come from the library's pool: a context that is made anew finds the last one's memory there
+// (cudaMalloc of them took 3-10 ms).  All three streams use them, so the first use waits for the pool.
+static int reserve(agcn_host_ctx *c, void **buf, size_t *cap, size_t bytes)
 {
     if (bytes <= *cap) return AGCN_OK;
-    if (*buf != nullptr) AGCN_CUDA(cudaFree(*buf));
+    pool_free_waiting(*buf);
     *buf = nullptr; *cap = 0;
-    AGCN_CUDA(cudaMalloc(buf, bytes));
+    const cudaError_t e = pool_alloc(buf, bytes, c->s_run);
+    if (e != cudaSuccess) {
+        set_error("agcn_host_spmm: device allocation of %zu bytes: %s", bytes, cudaGetErrorString(e));
+        return AGCN_ERR_CUDA;
+    }
+    AGCN_CUDA(cudaStreamSynchronize(c->s_run));
     *cap = bytes;
     return AGCN_OK;
 }
@@ -94,8 +102,8 @@ static int ctx_sync(agcn_host_ctx *c)
 // caller's host copy of .block4 (tuples tile [0, nnz) in order, so loc_begin is monotone).
 static void plan_parts(agcn_host_ctx *c, const int *h_block4, int want_parts)
 {
-    const int64_t n_units = c->plan->n_units;
-    if (c->plan->split) want_parts = 1;           // its units are not those of the caller's tuples (and it is small)
+    const int64_t n_units = ceil_div(c->n_blocks, HOST_SPMM_WARPS);
+    if (spmm_plan_splits(c->n_blocks, c->nnz)) want_parts = 1;      // its units are not those of the caller's tuples (and it is small)
     c->part_unit.assign(1, 0);
     c->part_row.assign(1, 0);
     c->part_loc.assign(1, 0);
@@ -117,7 +125,7 @@ static void plan_parts(agcn_host_ctx *c, const int *h_block4, int want_parts)
         c->part_row.push_back(row);
         c->part_loc.push_back(loc);
     }
-    c->part_unit.push_back(n_units);
+    c->part_unit.push_back(-1);            // to the last unit, whatever the plan's are
     c->part_row.push_back(c->n_rows);
     c->part_loc.push_back(c->nnz);
 }
@@ -141,10 +149,10 @@ static int upload_block4(agcn_host_ctx *c, const int *h_block4, int64_t n_blocks
     c->n_rows = n_rows; c->n_cols = n_cols; c->nnz = nnz; c->n_blocks = n_blocks;
     const size_t bytes[3] = {(size_t)n_blocks * 16, (size_t)nnz * 4, (size_t)nnz * 4};
     for (int i = 0; i < 3; i++) {
-        int rc = reserve(&c->graph[i], &c->graph_cap[i], bytes[i] > 0 ? bytes[i] : 16);
+        int rc = reserve(c, &c->graph[i], &c->graph_cap[i], bytes[i] > 0 ? bytes[i] : 16);
         if (rc != AGCN_OK) return rc;
     }
-    if (c->d_abort == nullptr) AGCN_CUDA(cudaMalloc(&c->d_abort, sizeof(int)));
+    if (c->d_abort == nullptr) AGCN_CUDA(pool_alloc(reinterpret_cast<void **>(&c->d_abort), sizeof(int), c->s_run));
     AGCN_CUDA(cudaMemsetAsync(c->d_abort, 0, sizeof(int), c->s_run));
     if (n_blocks > 0) AGCN_CUDA(cudaMemcpyAsync(c->graph[0], h_block4, bytes[0], cudaMemcpyHostToDevice, c->s_up));
     return ctx_chain(c, c->s_up, c->s_run);
@@ -164,9 +172,9 @@ static int host_set_graph(agcn_host_ctx *c, const int *h_block4, int64_t n_block
     int rc = check_graph_args(c, h_block4, n_blocks, h_indices, h_vals, n_rows, n_cols, nnz);
     if (rc != AGCN_OK) return rc;
     // the column ids and values go up behind .block4 while the plan is being built from it
-    rc = reserve(&c->graph[1], &c->graph_cap[1], nnz > 0 ? (size_t)nnz * 4 : 16);
-    if (rc == AGCN_OK) rc = reserve(&c->graph[2], &c->graph_cap[2], nnz > 0 ? (size_t)nnz * 4 : 16);
-    if (rc == AGCN_OK) rc = reserve(&c->graph[0], &c->graph_cap[0], n_blocks > 0 ? (size_t)n_blocks * 16 : 16);
+    rc = reserve(c, &c->graph[1], &c->graph_cap[1], nnz > 0 ? (size_t)nnz * 4 : 16);
+    if (rc == AGCN_OK) rc = reserve(c, &c->graph[2], &c->graph_cap[2], nnz > 0 ? (size_t)nnz * 4 : 16);
+    if (rc == AGCN_OK) rc = reserve(c, &c->graph[0], &c->graph_cap[0], n_blocks > 0 ? (size_t)n_blocks * 16 : 16);
     if (rc != AGCN_OK) return rc;
     rc = upload_block4(c, h_block4, n_blocks, n_rows, n_cols, nnz);
     if (rc != AGCN_OK) return rc;
@@ -194,25 +202,48 @@ static int host_set_graph(agcn_host_ctx *c, const int *h_block4, int64_t n_block
     return AGCN_OK;
 }
 
-static int reserve_products(agcn_host_ctx *c, int n, const int *dims, bool per_product_carry)
+// A product of up to 128 columns can be issued in unit ranges, from rows of X that are 16-byte aligned: its own, or
+// a copy with the rows padded to a multiple of four floats.
+static bool can_issue_in_parts(int dim) { return dim <= HOST_SPMM_PANEL; }
+static bool needs_padding(int dim) { return dim % 4 != 0; }
+
+static int reserve_products(agcn_host_ctx *c, int n, const int *dims)
 {
     if ((int)c->xbuf.size() < n) {
-        c->xbuf.resize(n, nullptr); c->ybuf.resize(n, nullptr); c->cbuf.resize(n, nullptr);
-        c->xcap.resize(n, 0); c->ycap.resize(n, 0); c->ccap.resize(n, 0);
+        c->xbuf.resize(n, nullptr); c->xpad.resize(n, nullptr); c->ybuf.resize(n, nullptr); c->cbuf.resize(n, nullptr);
+        c->xcap.resize(n, 0); c->pcap.resize(n, 0); c->ycap.resize(n, 0); c->ccap.resize(n, 0);
     }
     for (int i = 0; i < n; i++) {
-        int rc = reserve(&c->xbuf[i], &c->xcap[i], (size_t)c->n_cols * dims[i] * 4);
-        if (rc == AGCN_OK) rc = reserve(&c->ybuf[i], &c->ycap[i], (size_t)c->n_rows * dims[i] * 4);
-        // products whose unit ranges interleave each keep their own partial sums of the heavy rows
-        if (rc == AGCN_OK && per_product_carry && c->plan->n_carry > 0) {
-            const int64_t n = c->plan->n_carry;
-            rc = reserve(&c->cbuf[i], &c->ccap[i], spmm_carry_bytes(n));
-            if (rc == AGCN_OK)
-                AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(c->cbuf[i], n), 0, (size_t)n * SPMM_CARRY_PASSES * sizeof(int), c->s_run));
-        }
+        int rc = reserve(c, &c->xbuf[i], &c->xcap[i], (size_t)c->n_cols * dims[i] * 4);
+        if (rc == AGCN_OK) rc = reserve(c, &c->ybuf[i], &c->ycap[i], (size_t)c->n_rows * dims[i] * 4);
+        if (rc == AGCN_OK && can_issue_in_parts(dims[i]) && needs_padding(dims[i]))
+            rc = reserve(c, &c->xpad[i], &c->pcap[i], (size_t)c->n_cols * ((dims[i] + 3) / 4) * 16);
         if (rc != AGCN_OK) return rc;
     }
     return AGCN_OK;
+}
+
+// Products whose unit ranges interleave each keep their own partial sums of the heavy rows.
+static int reserve_carries(agcn_host_ctx *c, int n)
+{
+    const int64_t slots = c->plan->n_carry;
+    for (int i = 0; i < n && slots > 0; i++) {
+        const int rc = reserve(c, &c->cbuf[i], &c->ccap[i], spmm_carry_bytes(slots));
+        if (rc != AGCN_OK) return rc;
+        AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(c->cbuf[i], slots), 0, (size_t)slots * SPMM_CARRY_PASSES * sizeof(int), c->s_run));
+    }
+    return AGCN_OK;
+}
+
+// X of product i has arrived: what the kernels gather from.
+static int product_operand(agcn_host_ctx *c, int i, int dim, const float **x, int64_t *ldx)
+{
+    *x = static_cast<const float *>(c->xbuf[i]);
+    *ldx = dim;
+    if (!needs_padding(dim)) return AGCN_OK;
+    *x = static_cast<const float *>(c->xpad[i]);
+    *ldx = (dim + 3) & ~3;
+    return spmm_pad_rows(static_cast<const float *>(c->xbuf[i]), dim, dim, static_cast<float *>(c->xpad[i]), c->n_cols, c->s_run);
 }
 
 // rows [lo, hi) of product i: device -> host, on the download stream, after what s_run holds now
@@ -224,8 +255,6 @@ static int download_rows(agcn_host_ctx *c, int i, float *h_y, int dim, int64_t l
     return AGCN_OK;
 }
 
-static bool can_issue_in_parts(int dim) { return dim <= HOST_SPMM_PANEL && dim % 4 == 0; }
-
 // Products on a graph that is already on the device: X_i up, product i in unit ranges, rows down as
 // they complete.
 static int host_products(agcn_host_ctx *c, int n, const float *const *h_x, float *const *h_y, const int *dims)
@@ -235,7 +264,7 @@ static int host_products(agcn_host_ctx *c, int n, const float *const *h_x, float
     for (int i = 0; i < n; i++)
         AGCN_REQUIRE(h_x[i] != nullptr && h_y[i] != nullptr && dims[i] >= 1, "agcn_host_spmm: null X or Y, or dim < 1");
     if (n == 0) return AGCN_OK;
-    int rc = reserve_products(c, n, dims, false);
+    int rc = reserve_products(c, n, dims);
     if (rc != AGCN_OK) return rc;
     const int *idx = static_cast<const int *>(c->graph[1]);
     const float *val = static_cast<const float *>(c->graph[2]);
@@ -258,11 +287,15 @@ static int host_products(agcn_host_ctx *c, int n, const float *const *h_x, float
             if (rc != AGCN_OK) { ctx_sync(c); return rc; }
             continue;
         }
+        const float *x = nullptr;
+        int64_t ldx = 0;
+        rc = product_operand(c, i, dim, &x, &ldx);
+        if (rc != AGCN_OK) { ctx_sync(c); return rc; }
         for (int k = 0; k < n_parts; k++) {
             SpmmLaunchPart part;
             part.unit0 = c->part_unit[k]; part.unit1 = c->part_unit[k + 1];
             part.zero_fill = k == 0;
-            rc = spmm_run_prepared(c->plan, idx, val, static_cast<const float *>(c->xbuf[i]), dim, true, y, dim, dim, c->s_run, 0, 0, part);
+            rc = spmm_run_prepared(c->plan, idx, val, x, ldx, true, y, dim, dim, c->s_run, 0, 0, part);
             if (rc == AGCN_OK) rc = ctx_chain(c, c->s_run, c->s_down);
             if (rc == AGCN_OK) rc = download_rows(c, i, h_y[i], dim, c->part_row[k], c->part_row[k + 1]);
             if (rc != AGCN_OK) { ctx_sync(c); return rc; }
@@ -271,8 +304,43 @@ static int host_products(agcn_host_ctx *c, int n, const float *const *h_x, float
     return ctx_sync(c);
 }
 
-// The graph and the products in one call: A is uploaded in unit ranges and every range is
-// multiplied for all products as soon as it is on the device.
+// The graph and the products in one call.  A row of Y can be computed, and start its way down, when its range of A
+// and its X are up, so the order of the uploads decides how long the link's other direction stays idle.
+struct UploadItem {
+    bool is_x;
+    int index;           // product, or range of A
+};
+
+// Greedy: next goes what makes most bytes of Y ready per byte sent.  Ranges begin with the light rows, which bring
+// many rows of Y per nonzero; the heavy ones, which bring few, go last and hide the downloads.  (All of X, then A in
+// order, for 500 000 skewed rows of 29 with 32 + 64 columns: the first row of Y starts down after 4.2 of 8.3 ms;
+// this way after 1.3 ms.)
+static std::vector<UploadItem> upload_order(const agcn_host_ctx *c, int n, const int *dims)
+{
+    const int n_parts = (int)c->part_row.size() - 1;
+    std::vector<UploadItem> order;
+    int x_done = 0, a_done = 0;
+    double cols = 0, rows = 0;
+    while (x_done < n || a_done < n_parts) {
+        double gain_x = -1, gain_a = -1;
+        // with no X (or no A) there yet, what the other would make ready counts
+        if (x_done < n) gain_x = (rows > 0 ? rows : c->n_rows) / (double)c->n_cols;
+        if (a_done < n_parts) {
+            const double r = (double)(c->part_row[a_done + 1] - c->part_row[a_done]);
+            const double bytes = 8.0 * (double)(c->part_loc[a_done + 1] - c->part_loc[a_done]) + 1;
+            gain_a = cols > 0 ? r * cols * 4 / bytes : 0;
+        }
+        if (gain_x >= gain_a) {
+            order.push_back({true, x_done});
+            cols += dims[x_done++];
+        } else {
+            order.push_back({false, a_done});
+            rows = (double)c->part_row[++a_done];
+        }
+    }
+    return order;
+}
+
 static int host_graph_and_products(agcn_host_ctx *c, const int *h_block4, int64_t n_blocks, const int *h_indices,
                                    const float *h_vals, int64_t n_rows, int64_t n_cols, int64_t nnz, int n,
                                    const float *const *h_x, float *const *h_y, const int *dims)
@@ -292,54 +360,69 @@ static int host_graph_and_products(agcn_host_ctx *c, const int *h_block4, int64_
     const auto host_t0 = std::chrono::steady_clock::now();
     c->timed = false;
     AGCN_CUDA(cudaEventRecord(c->t_up0, c->s_up));
-    // .block4 first, then every X behind it: the plan is built (on the host and on s_run) under those uploads
     rc = upload_block4(c, h_block4, n_blocks, n_rows, n_cols, nnz);
-    if (rc == AGCN_OK) rc = reserve_products(c, n, dims, false);
+    if (rc == AGCN_OK) rc = reserve_products(c, n, dims);
     if (rc != AGCN_OK) { ctx_sync(c); return rc; }
-    for (int i = 0; i < n; i++)
-        AGCN_CUDA(cudaMemcpyAsync(c->xbuf[i], h_x[i], (size_t)n_cols * dims[i] * 4, cudaMemcpyHostToDevice, c->s_up));
-    rc = build_plan(c);               // on the host and on s_run, under the uploads of X
-    if (rc == AGCN_OK) rc = reserve_products(c, n, dims, true);       // now that the number of carry slots is known
-    if (rc != AGCN_OK) { ctx_sync(c); return rc; }
-    const auto host_t1 = std::chrono::steady_clock::now();
-    // Column ids and values in ranges of about 32 MB: long enough for full PCIe speed, short enough
-    // that the first product starts early and the last download is short.  Every upload is enqueued
-    // before the first launch, so that the copy engine runs without a gap however long the host
-    // takes over the launches below.  (Enqueued ahead of the plan build they delay it: its small
-    // device-to-host copies then wait behind them.)
-    plan_parts(c, h_block4, (int)std::max<int64_t>(1, std::min<int64_t>(64, (nnz * 8) >> 25)));
-    const int n_parts = (int)c->part_unit.size() - 1;
+    // Column ids and values in ranges of a sixteenth, but of 4 to 32 MB: long enough for full PCIe speed, short enough
+    // that the first product starts early and the last download is short.  Every upload is enqueued before the
+    // plan is built and before the first launch, so that the copy engine runs without a gap however long the host
+    // takes over them.
+    const int64_t a_bytes = nnz * 8, range_bytes = std::max<int64_t>((int64_t)4 << 20, std::min<int64_t>((int64_t)32 << 20, a_bytes / 16));
+    plan_parts(c, h_block4, (int)std::max<int64_t>(1, std::min<int64_t>(64, a_bytes / range_bytes)));
+    const std::vector<UploadItem> order = upload_order(c, n, dims);
     int *idx = static_cast<int *>(c->graph[1]);
     float *val = static_cast<float *>(c->graph[2]);
-    std::vector<cudaEvent_t> part_up((size_t)n_parts);
-    for (int k = 0; k < n_parts; k++) {
-        const int64_t p0 = c->part_loc[k], p1 = c->part_loc[k + 1];
-        AGCN_CUDA(cudaMemcpyAsync(idx + p0, h_indices + p0, (size_t)(p1 - p0) * 4, cudaMemcpyHostToDevice, c->s_up));
-        AGCN_CUDA(cudaMemcpyAsync(val + p0, h_vals + p0, (size_t)(p1 - p0) * 4, cudaMemcpyHostToDevice, c->s_up));
-        rc = ctx_event(c, &part_up[k]);
+    std::vector<cudaEvent_t> arrived(order.size());
+    for (size_t o = 0; o < order.size(); o++) {
+        const int k = order[o].index;
+        if (order[o].is_x) {
+            AGCN_CUDA(cudaMemcpyAsync(c->xbuf[k], h_x[k], (size_t)n_cols * dims[k] * 4, cudaMemcpyHostToDevice, c->s_up));
+        } else {
+            const int64_t p0 = c->part_loc[k], p1 = c->part_loc[k + 1];
+            AGCN_CUDA(cudaMemcpyAsync(idx + p0, h_indices + p0, (size_t)(p1 - p0) * 4, cudaMemcpyHostToDevice, c->s_up));
+            AGCN_CUDA(cudaMemcpyAsync(val + p0, h_vals + p0, (size_t)(p1 - p0) * 4, cudaMemcpyHostToDevice, c->s_up));
+        }
+        rc = ctx_event(c, &arrived[o]);
         if (rc != AGCN_OK) { ctx_sync(c); return rc; }
-        AGCN_CUDA(cudaEventRecord(part_up[k], c->s_up));
+        AGCN_CUDA(cudaEventRecord(arrived[o], c->s_up));
     }
     AGCN_CUDA(cudaEventRecord(c->t_up1, c->s_up));
-    for (int k = 0; k < n_parts; k++) {
-        const int64_t p0 = c->part_loc[k], p1 = c->part_loc[k + 1];
-        AGCN_CUDA(cudaStreamWaitEvent(c->s_run, part_up[k], 0));
-        if (k == 0) AGCN_CUDA(cudaEventRecord(c->t_run0, c->s_run));
-        // a column id outside [0, n_cols) sets the abort word, and every kernel behind it returns at once
-        rc = spmm_check_cols(idx + p0, p1 - p0, n_cols, c->d_abort, c->s_run);
-        for (int i = 0; i < n && rc == AGCN_OK; i++) {
-            SpmmLaunchPart part;
-            part.unit0 = c->part_unit[k]; part.unit1 = c->part_unit[k + 1];
-            part.zero_fill = k == 0; part.abort_flag = c->d_abort;
-            part.carry = c->cbuf[i];
-            rc = spmm_run_prepared(c->plan, idx, val, static_cast<const float *>(c->xbuf[i]), dims[i], true,
-                                   static_cast<float *>(c->ybuf[i]), dims[i], dims[i], c->s_run, 0, 0, part);
+    rc = build_plan(c);               // on the host and on s_run, under the uploads
+    if (rc == AGCN_OK) rc = reserve_carries(c, n);
+    if (rc != AGCN_OK) { ctx_sync(c); return rc; }
+    const auto host_t1 = std::chrono::steady_clock::now();
+
+    int x_done = 0, a_done = 0;
+    std::vector<const float *> x((size_t)n, nullptr);
+    std::vector<int64_t> ldx((size_t)n, 0);
+    // product i over the ranges [k0, k1): one launch, and its rows down
+    auto multiply = [&](int i, int k0, int k1) {
+        SpmmLaunchPart part;
+        part.unit0 = c->part_unit[k0]; part.unit1 = c->part_unit[k1];
+        part.zero_fill = k0 == 0; part.abort_flag = c->d_abort;
+        part.carry = c->cbuf[i];
+        int r = spmm_run_prepared(c->plan, idx, val, x[i], ldx[i], true, static_cast<float *>(c->ybuf[i]), dims[i], dims[i], c->s_run, 0, 0, part);
+        if (r == AGCN_OK) r = ctx_chain(c, c->s_run, c->s_down);
+        return r != AGCN_OK ? r : download_rows(c, i, h_y[i], dims[i], c->part_row[k0], c->part_row[k1]);
+    };
+    for (size_t o = 0; o < order.size() && rc == AGCN_OK; o++) {
+        const int k = order[o].index;
+        AGCN_CUDA(cudaStreamWaitEvent(c->s_run, arrived[o], 0));
+        if (o == 0) AGCN_CUDA(cudaEventRecord(c->t_run0, c->s_run));
+        if (order[o].is_x) {
+            rc = product_operand(c, k, dims[k], &x[k], &ldx[k]);
+            // the ranges that are there already, in a few launches so that the first rows start down early
+            const int each = std::max(1, (a_done + 3) / 4);
+            for (int k0 = 0; k0 < a_done && rc == AGCN_OK; k0 += each) rc = multiply(k, k0, std::min(k0 + each, a_done));
+            x_done++;
+        } else {
+            // a column id outside [0, n_cols) sets the abort word, and every kernel behind it returns at once
+            rc = spmm_check_cols(idx + c->part_loc[k], c->part_loc[k + 1] - c->part_loc[k], n_cols, c->d_abort, c->s_run);
+            for (int i = 0; i < x_done && rc == AGCN_OK; i++) rc = multiply(i, k, k + 1);
+            a_done++;
         }
-        if (rc == AGCN_OK) rc = ctx_chain(c, c->s_run, c->s_down);
-        for (int i = 0; i < n && rc == AGCN_OK; i++)
-            rc = download_rows(c, i, h_y[i], dims[i], c->part_row[k], c->part_row[k + 1]);
-        if (rc != AGCN_OK) { ctx_sync(c); return rc; }
     }
+    if (rc != AGCN_OK) { ctx_sync(c); return rc; }
     AGCN_CUDA(cudaEventRecord(c->t_run1, c->s_run));
     AGCN_CUDA(cudaEventRecord(c->t_down1, c->s_down));
     c->host_plan_ms = std::chrono::duration<float, std::milli>(host_t1 - host_t0).count();
@@ -388,11 +471,10 @@ extern "C" int agcn_host_ctx_destroy(agcn_host_ctx *ctx)
     agcn::clear_error();
     if (ctx == nullptr) return AGCN_OK;
     agcn::plan_free(ctx->plan);
-    for (int i = 0; i < 3; i++) cudaFree(ctx->graph[i]);
-    for (void *p : ctx->xbuf) cudaFree(p);
-    for (void *p : ctx->ybuf) cudaFree(p);
-    for (void *p : ctx->cbuf) cudaFree(p);
-    cudaFree(ctx->d_abort);
+    for (int i = 0; i < 3; i++) agcn::pool_free_waiting(ctx->graph[i]);
+    for (const std::vector<void *> *v : {&ctx->xbuf, &ctx->xpad, &ctx->ybuf, &ctx->cbuf})
+        for (void *p : *v) agcn::pool_free_waiting(p);
+    agcn::pool_free_waiting(ctx->d_abort);
     for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
     for (cudaEvent_t e : {ctx->t_up0, ctx->t_up1, ctx->t_run0, ctx->t_run1, ctx->t_down1}) if (e) cudaEventDestroy(e);
     if (ctx->s_up) cudaStreamDestroy(ctx->s_up);

@@ -69,6 +69,10 @@ struct SpmmLaunchPart {
 int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *x_use, int64_t ldx_use,
                       bool x_vec, float *d_y, int64_t ldy, int dim, cudaStream_t s, int activation, int accumulate,
                       const SpmmLaunchPart &part);
+// Aligned copy of X: rows of dim floats padded with zeros to a multiple of four
+int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n_rows, cudaStream_t s);
+// Whether spmm_create would cut the tuples of a graph of that size on the current device
+bool spmm_plan_splits(int64_t n_blocks, int64_t nnz);
 int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag, cudaStream_t s);
 void plan_free(agcn_spmm_plan *p);
 

@@ -40,6 +40,18 @@ static int spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
     return 0;
 }
 
+static int spmm_piece_choice(int64_t n_blocks, int64_t nnz, int sm_count)
+{
+    return n_blocks > 0 ? env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count)) : 0;
+}
+
+bool spmm_plan_splits(int64_t n_blocks, int64_t nnz)
+{
+    int device = 0, sm_count = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return true;
+    return spmm_piece_choice(n_blocks, nnz, sm_count) > 0;
+}
+
 // Order of the units, which are in ascending degree.  Starting at the heavy end leaves light units for the end of
 // the launch (500 000 rows of 12, dim 64: 159 -> 144 us).  Where nearly all tuples are full there is nothing to
 // balance, and units from both ends in turn are faster by 4-10 % (250 000 rows of 490, dim 32: 934 -> 872 us;
@@ -74,7 +86,7 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
     AGCN_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
     AGCN_CUDA(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, device));
     const int64_t n_units = ceil_div(n_blocks, SPMM_WARPS);
-    const int most = n_blocks > 0 ? env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count)) : 0;
+    const int most = spmm_piece_choice(n_blocks, nnz, sm_count);
     const int64_t tiles = n_units > 0 ? ceil_div(n_units, PLAN_BLOCK) : 1;
     DeviceScratch scratch(s);
     Carver size;
@@ -194,6 +206,15 @@ static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, u
     else launch_units_for<32>(prm, grid, small, plain, finish, s);
 }
 
+int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n_rows, cudaStream_t s)
+{
+    const int ldp = (dim + 3) & ~3;
+    const int64_t quads = n_rows * (ldp >> 2);
+    AGCN_KERNEL(spmm_pad_rows_kernel, (unsigned)ceil_div(quads, 256), 256, s, d_x, ldx, dim, d_xp, ldp, n_rows);
+    AGCN_LAUNCH_CHECK("spmm_pad_rows_kernel");
+    return AGCN_OK;
+}
+
 // Rows of X that are not 16-byte aligned (dim % 4 != 0 with the reference's ld = dim, an odd
 // stride or base) would force 4-byte gathers: 1.2-1.6x the time of the 16-byte path.  Instead X
 // is copied once into plan-owned rows padded to a multiple of 4 floats (2 * n_cols * dim * 4
@@ -218,9 +239,8 @@ int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cu
         AGCN_CUDA(pool_alloc(reinterpret_cast<void **>(&p->x_pad), need, s));
         p->x_pad_bytes = need;
     }
-    const int64_t quads = p->n_cols * (ldp >> 2);
-    AGCN_KERNEL(spmm_pad_rows_kernel, (unsigned)ceil_div(quads, 256), 256, s, d_x, ldx, dim, p->x_pad, ldp, p->n_cols);
-    AGCN_LAUNCH_CHECK("spmm_pad_rows_kernel");
+    const int rc = spmm_pad_rows(d_x, ldx, dim, p->x_pad, p->n_cols, s);
+    if (rc != AGCN_OK) return rc;
     p->launches_last_run++;
     *x_use = p->x_pad;
     *ldx_use = ldp;
