@@ -7,6 +7,8 @@ or fails to load, importing a function from here raises.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
@@ -78,6 +80,7 @@ DIST_ID_BYTES = 128
 MAX_WORLD = 64
 
 _lib = None
+_call = None
 
 
 class AccelGcnError(RuntimeError):
@@ -107,6 +110,54 @@ def load():
             fn.restype, fn.argtypes = res, args
         _lib = lib
     return _lib
+
+
+def call():
+    """The native caller `call(address, *integers) -> int` (csrc/pycall.c): what the hot paths use in place of
+    ctypes.  No fallback: it is built with the library."""
+    global _call
+    if _call is None:
+        path = os.path.join(os.path.dirname(DEFAULT_LIB), "agcn_call.so")
+        if not os.path.exists(path):
+            raise FileNotFoundError(f"{path} not found: build it with `python iccad-accel-gcn_b200/build.py`")
+        loader = importlib.machinery.ExtensionFileLoader("agcn_call", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("agcn_call", loader))
+        loader.exec_module(module)
+        _call = module.call
+    return _call
+
+
+def address(name: str) -> int:
+    """Address of a library function, for `call`."""
+    return ctypes.cast(getattr(load(), name), ctypes.c_void_p).value
+
+
+def raw_stream(index: int) -> int:
+    """The cudaStream_t of the current stream of device `index` (torch.cuda.current_stream builds an object for it)."""
+    import torch
+    return torch._C._cuda_getCurrentRawStream(index)
+
+
+class _Here:
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *exc):
+        return False
+
+
+_HERE_ALREADY = _Here()
+
+
+def on_device(index: int):
+    """Makes device `index` current for a `with` block; nothing is done where it already is."""
+    import torch
+    return _HERE_ALREADY if torch._C._cuda_getDevice() == index else torch.cuda.device(index)
+
+
+def device_index(device) -> int:
+    import torch
+    return device.index if device.index is not None else torch.cuda.current_device()
 
 
 def check(code: int) -> None:

@@ -43,14 +43,15 @@ def degree_sort_device(indptr, indices, vals=None, relabel_cols: bool = True, st
     n_rows, nnz = indptr.numel() - 1, indices.numel()
     if n_rows <= 0:
         raise IndexError("empty graph")
-    s = stream if stream is not None else torch.cuda.current_stream(dev)
+    index = _lib.device_index(dev)
+    s = stream.cuda_stream if stream is not None else _lib.raw_stream(index)
     perm = torch.empty(n_rows, dtype=torch.int32, device=dev)
     new_indptr = torch.empty(n_rows + 1, dtype=torch.int32, device=dev)
     new_indices = torch.empty(nnz, dtype=torch.int32, device=dev)
     new_vals = None if vals is None else torch.empty(nnz, dtype=torch.float32, device=dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(index):
         _lib.check(lib.agcn_degree_sort_device(
             indptr.data_ptr(), indices.data_ptr(), None if vals is None else vals.data_ptr(), n_rows, nnz,
             int(bool(relabel_cols)), perm.data_ptr(), new_indptr.data_ptr(), new_indices.data_ptr(),
-            None if new_vals is None else new_vals.data_ptr(), s.cuda_stream))
+            None if new_vals is None else new_vals.data_ptr(), s))
     return perm, new_indptr, new_indices, new_vals

@@ -45,10 +45,11 @@ def block_level_partition_device(indptr, stream=None):
     n_rows = indptr.numel() - 1
     if n_rows <= 0:
         raise IndexError("empty graph")
-    s = stream if stream is not None else torch.cuda.current_stream(indptr.device)
+    dev = _lib.device_index(indptr.device)
+    s = stream.cuda_stream if stream is not None else _lib.raw_stream(dev)
     n_blocks, run = ctypes.c_int64(0), ctypes.c_void_p()
-    with torch.cuda.device(indptr.device):
-        _lib.check(lib.agcn_partition_begin(indptr.data_ptr(), n_rows, ctypes.byref(run), ctypes.byref(n_blocks), s.cuda_stream))
+    with _lib.on_device(dev):
+        _lib.check(lib.agcn_partition_begin(indptr.data_ptr(), n_rows, ctypes.byref(run), ctypes.byref(n_blocks), s))
         try:
             out = torch.empty((n_blocks.value, 4), dtype=torch.int32, device=indptr.device)
         except BaseException:

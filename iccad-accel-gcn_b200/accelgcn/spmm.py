@@ -28,31 +28,31 @@ class SpmmPlan:
         self._lib = lib
         self.block4 = block4            # keep alive: the plan borrows it
         self.device = block4.device
-        self._dev_index = block4.device.index if block4.device.index is not None else torch.cuda.current_device()
+        self._dev_index = _lib.device_index(block4.device)
         self.n_rows, self.n_cols = int(n_rows), int(n_cols)
         self.n_blocks = block4.numel() // 4
         self.nnz = int(indices.numel())
-        s = stream if stream is not None else torch.cuda.current_stream(self.device)
+        s = stream.cuda_stream if stream is not None else _lib.raw_stream(self._dev_index)
         h = ctypes.c_void_p()
-        with torch.cuda.device(self.device):
+        with _lib.on_device(self._dev_index):
             _lib.check(lib.agcn_spmm_create(ctypes.byref(h), block4.data_ptr(), self.n_blocks, indices.data_ptr(),
-                                            self.n_rows, self.n_cols, self.nnz, s.cuda_stream))
+                                            self.n_rows, self.n_cols, self.nnz, s))
         self._h = h
+        self._run = _lib.address("agcn_spmm_run_act")
+        self._call = _lib.call()
+        self._raw_stream = torch._C._cuda_getCurrentRawStream
 
     def run(self, indices, vals, x, y, dim: int | None = None, ldx: int | None = None, ldy: int | None = None,
             stream=None, relu: bool = False) -> None:
-        import torch
-        dim = int(x.shape[1] if dim is None else dim)
-        ldx = int(x.stride(0) if ldx is None and x.dim() == 2 else (dim if ldx is None else ldx))
-        ldy = int(y.stride(0) if ldy is None and y.dim() == 2 else (dim if ldy is None else ldy))
-        s = stream if stream is not None else torch.cuda.current_stream(self.device)
-        args = (self._h, indices.data_ptr(), vals.data_ptr(), x.data_ptr(), ldx, y.data_ptr(), ldy, dim,
-                1 if relu else 0, s.cuda_stream)
-        if torch.cuda.current_device() == self._dev_index:      # the usual case: no device switch needed
-            rc = self._lib.agcn_spmm_run_act(*args)
-        else:
-            with torch.cuda.device(self.device):
-                rc = self._lib.agcn_spmm_run_act(*args)
+        if dim is None:
+            dim = x.shape[1]
+        if ldx is None:
+            ldx = x.stride(0) if x.dim() == 2 else dim
+        if ldy is None:
+            ldy = y.stride(0) if y.dim() == 2 else dim
+        # the library makes the plan's device current where it is not
+        rc = self._call(self._run, self._h.value, indices.data_ptr(), vals.data_ptr(), x.data_ptr(), ldx, y.data_ptr(), ldy, dim,
+                        1 if relu else 0, stream.cuda_stream if stream is not None else self._raw_stream(self._dev_index))
         if rc != 0:
             _lib.check(rc)
 

@@ -1,4 +1,5 @@
-"""Builds lib/libaccelgcn.so from csrc/ with nvcc for sm_100a (cross-compiles without a GPU).
+"""Builds lib/libaccelgcn.so from csrc/ with nvcc for sm_100a (cross-compiles without a GPU), and the small
+extension module the Python layer calls it through.
 
     python iccad-accel-gcn_b200/build.py [--force] [--verbose]
 """
@@ -7,6 +8,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 SOURCES = ["common.cu", "memory.cu", "host_copy.cu", "partition.cu", "degree_sort.cu", "spmm.cu", "spmm_tiled.cu", "host_spmm.cu", "gemm.cu", "layout.cu", "dist.cu", "probe.cu"]
@@ -40,7 +42,20 @@ def build_harness(force: bool = False) -> str:
     return HARNESS
 
 
+CALL = os.path.join(HERE, "lib", "agcn_call.so")
+
+
+def build_call(force: bool = False) -> str:
+    """lib/agcn_call.so: the extension module through which the Python layer makes its hot calls."""
+    src = os.path.join(HERE, "csrc", "pycall.c")
+    if force or not os.path.exists(CALL) or os.path.getmtime(src) > os.path.getmtime(CALL):
+        os.makedirs(os.path.dirname(CALL), exist_ok=True)
+        subprocess.check_call(["gcc", "-O2", "-Wall", "-shared", "-fPIC", "-I" + sysconfig.get_paths()["include"], "-o", CALL, src])
+    return CALL
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_call(force)
     if not force and os.path.exists(LIB) and all(os.path.getmtime(f) <= os.path.getmtime(LIB) for f in _inputs()):
         return LIB
     os.makedirs(os.path.dirname(LIB), exist_ok=True)

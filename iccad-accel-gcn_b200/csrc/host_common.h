@@ -42,6 +42,21 @@ void clear_error();
         if (!(cond)) { ::agcn::set_error(__VA_ARGS__); return AGCN_ERR_INVALID; }                \
     } while (0)
 
+// Makes a device current for a scope; nothing is done where it already is.
+class DeviceOf {
+public:
+    explicit DeviceOf(int device)
+    {
+        if (cudaGetDevice(&before_) != cudaSuccess || before_ == device || device < 0) before_ = -1;
+        else cudaSetDevice(device);
+    }
+    ~DeviceOf() { if (before_ >= 0) cudaSetDevice(before_); }
+    DeviceOf(const DeviceOf &) = delete;
+    DeviceOf &operator=(const DeviceOf &) = delete;
+private:
+    int before_ = -1;
+};
+
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 

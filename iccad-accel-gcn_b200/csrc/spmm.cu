@@ -18,12 +18,11 @@ int env_int(const char *name, int dflt)
 void plan_free(agcn_spmm_plan *p)
 {
     if (p == nullptr) return;
-    int dev = p->device;
-    cudaGetDevice(&dev);
-    if (dev != p->device) cudaSetDevice(p->device);
-    pool_free_waiting(p->memory);
-    if (p->x_pad != nullptr) pool_free_waiting(p->x_pad);
-    if (dev != p->device) cudaSetDevice(dev);
+    {
+        const DeviceOf on(p->device);
+        pool_free_waiting(p->memory);
+        pool_free_waiting(p->x_pad);
+    }
     delete p;
 }
 
@@ -345,6 +344,7 @@ int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const
 {
     int rc = spmm_check_run_args(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, activation);
     if (rc != AGCN_OK) return rc;
+    const DeviceOf on(p->device);
     p->launches_last_run = 0;
     const float *x_use = nullptr;
     int64_t ldx_use = 0;
