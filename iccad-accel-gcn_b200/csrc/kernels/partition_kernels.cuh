@@ -14,7 +14,9 @@
 // its leading rows that belong to a run begun earlier, the tuples all other rows
 // open; (B) one thread block scans the descriptions, which closes the open runs,
 // and leaves every tile its incoming run start and its first output position;
-// (C) every row writes its own tuples.
+// (C) every row writes its own tuples.  Up to PART_DIRECT_TILES tiles (C) scans
+// the descriptions itself and writes to scratch before the count is known to the
+// host, which saves a launch and a wait.
 // Bound: launch latency up to some 100 000 rows, instruction issue above.
 #pragma once
 #include "../host_common.h"
@@ -95,20 +97,23 @@ struct PartTileInfo {
 
 // Number of tuples each of this thread's PART_ITEMS rows opens.
 // incoming_head = start of the run that is open when the tile begins; -1: not known, rows of that run
-// that need it count in `lead` instead.  Returns the last run start of this thread's rows, -1 if none.
-__device__ __forceinline__ int part_row_counts(const PartTile &t, int incoming_head, int *s_scan, int (&cnt)[PART_ITEMS],
-                                               int &lead, int &lead_deg, bool &negative)
+// that need it count in `lead` instead.  Returns the last run start of this thread's rows, -1 if none; `heads` has
+// a bit for every one of its rows that starts a run.
+__device__ __forceinline__ int part_row_counts(const PartTile &t, int incoming_head, int *s_scan, int (&deg)[PART_ITEMS],
+                                               int (&cnt)[PART_ITEMS], unsigned &heads, int &lead, int &lead_deg, bool &negative)
 {
     const int64_t my_first = t.first + (int64_t)threadIdx.x * PART_ITEMS;
     // last run head among this thread's rows, then an exclusive max-scan over the block
     int head_local = -1;
     int prev = my_first > 0 && my_first < t.n_rows ? t.deg(my_first - 1) : -1;
-    int deg[PART_ITEMS];
-    unsigned heads = 0;
+    heads = 0;
+    int at = t.ip(my_first);
 #pragma unroll
     for (int k = 0; k < PART_ITEMS; k++) {
         const int64_t i = my_first + k;
-        deg[k] = t.deg(i);
+        const int next = t.ip(i + 1);
+        deg[k] = next - at;
+        at = next;
         if (i < t.n_rows) {
             negative |= deg[k] < 0;
             if (i == 0 || deg[k] != prev) { head_local = (int)i; heads |= 1u << k; }
@@ -146,9 +151,10 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
     __shared__ int s_red[4][PART_BLOCK / 32];
     const PartTile t = part_load_tile(indptr, n_rows, s_ip);
-    int cnt[PART_ITEMS], lead, lead_deg;
+    int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
+    unsigned heads;
     bool negative = false;
-    int head = part_row_counts(t, -1, s_scan, cnt, lead, lead_deg, negative);
+    int head = part_row_counts(t, -1, s_scan, deg, cnt, heads, lead, lead_deg, negative);
     if (negative) out->w[PART_WORD_NEGATIVE] = 1;
     int rest = 0;
 #pragma unroll
@@ -171,6 +177,16 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
     }
 }
 
+// Tuples opened by the leading rows of tile b, once the start of their run is known.
+__device__ __forceinline__ int64_t part_lead_tuples(const PartTileInfo &info, int64_t b, int head)
+{
+    if (info.lead <= 0) return 0;
+    // rows o .. o + lead - 1 of their run open a tuple where their number is a multiple of R
+    const int64_t o = b * PART_TILE - head;
+    const int r = part_rows_per_tuple(info.lead_deg);
+    return (o + info.lead + r - 1) / r - (o + r - 1) / r;
+}
+
 // (B) one block: the run start that is open when every tile begins, and every tile's first output position.
 // 1024 tiles (two million rows) per step.
 constexpr int PART_SCAN_BLOCK = 1024;
@@ -190,13 +206,7 @@ part_scan_kernel(const PartTileInfo *__restrict__ tiles, int64_t n_tiles, int *_
         int head_total;
         int head = block_scan_exclusive<PART_SCAN_BLOCK>(info.last_head, OpMax(), -1, head_total, s_head);
         head = max(head, carry_head);
-        int64_t count = info.rest;
-        if (info.lead > 0) {
-            // rows o .. o + lead - 1 of their run open a tuple where their number is a multiple of R
-            const int64_t o = b * PART_TILE - head;
-            const int r = part_rows_per_tuple(info.lead_deg);
-            count += (o + info.lead + r - 1) / r - (o + r - 1) / r;
-        }
+        const int64_t count = info.rest + part_lead_tuples(info, b, head);
         int64_t total;
         const int64_t ex = block_scan_exclusive<PART_SCAN_BLOCK>(count, OpAdd(), (int64_t)0, total, s_sum);
         if (b < n_tiles) { tile_head[b] = head; tile_offset[b] = carry + ex; }
@@ -212,39 +222,81 @@ part_scan_kernel(const PartTileInfo *__restrict__ tiles, int64_t n_tiles, int *_
 constexpr int PART_INLINE_TUPLES = 8;
 constexpr int PART_HEAVY_QUEUE = 128;
 
+constexpr int PART_DIRECT_TILES = PART_BLOCK;      // half a million rows
+
+// tile_offset == nullptr: this block scans the descriptions of the (at most PART_DIRECT_TILES) tiles itself, and
+// the last one reports the total.  Nothing is written outside `cap` tuples (a
+// decreasing indptr, found by (A), may give any position here).
 __global__ void __launch_bounds__(PART_BLOCK)
-part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const int *__restrict__ tile_incoming_head,
-                 const int64_t *__restrict__ tile_offset, int4 *__restrict__ block4)
+part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileInfo *__restrict__ info,
+                 const int *__restrict__ tile_incoming_head, const int64_t *__restrict__ tile_offset, int64_t cap,
+                 int4 *__restrict__ block4, HostWords *report)
 {
     __shared__ int s_ip[PART_SMEM_INTS];
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
+    __shared__ int64_t s_scan64[PART_BLOCK / 32 + 1];
+    __shared__ unsigned char s_heads[PART_BLOCK + 2];      // a bit per row that starts a run (or lies past the end), a byte per thread
     __shared__ int s_heavy_n;
     __shared__ int s_heavy_row[PART_HEAVY_QUEUE], s_heavy_deg[PART_HEAVY_QUEUE], s_heavy_loc[PART_HEAVY_QUEUE];
     __shared__ int64_t s_heavy_out[PART_HEAVY_QUEUE];
     if (threadIdx.x == 0) s_heavy_n = 0;
+    int incoming;
+    int64_t first_out;
+    if (tile_offset != nullptr) {
+        incoming = tile_incoming_head[blockIdx.x];
+        first_out = tile_offset[blockIdx.x];
+    } else {
+        const int b = threadIdx.x;
+        PartTileInfo mine = {-1, 0, 0, 0};
+        if (b <= (int)blockIdx.x) mine = info[b];
+        int unused;
+        const int head = block_scan_exclusive<PART_BLOCK>(mine.last_head, OpMax(), -1, unused, s_scan);
+        const int64_t count = b <= (int)blockIdx.x ? mine.rest + part_lead_tuples(mine, b, head) : 0;
+        int64_t total;
+        const int64_t before = block_scan_exclusive<PART_BLOCK>(count, OpAdd(), (int64_t)0, total, s_scan64);
+        if (b == (int)blockIdx.x) { s_scan[0] = head; s_scan64[0] = before; }
+        __syncthreads();
+        incoming = s_scan[0];
+        first_out = s_scan64[0];
+        if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) report->w[PART_WORD_TOTAL] = total;
+    }
     const PartTile t = part_load_tile(indptr, n_rows, s_ip);      // synchronises the block
-    int cnt[PART_ITEMS], lead, lead_deg;
+    int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
+    unsigned heads;
     bool negative;
-    part_row_counts(t, tile_incoming_head[blockIdx.x], s_scan, cnt, lead, lead_deg, negative);
+    part_row_counts(t, incoming, s_scan, deg, cnt, heads, lead, lead_deg, negative);
+    const int64_t my_first = t.first + (int64_t)threadIdx.x * PART_ITEMS;
     int sum = 0;
 #pragma unroll
-    for (int k = 0; k < PART_ITEMS; k++) sum += cnt[k];
+    for (int k = 0; k < PART_ITEMS; k++) {
+        sum += cnt[k];
+        if (my_first + k >= n_rows) heads |= 1u << k;
+    }
+    s_heads[threadIdx.x] = (unsigned char)heads;
+    if (threadIdx.x < 2) {               // the rows a tuple of this tile may reach into
+        unsigned m = 0;
+        for (int k = 0; k < 8; k++) {
+            const int64_t i = t.first + PART_TILE + threadIdx.x * 8 + k;
+            if (i >= n_rows || threadIdx.x * 8 + k >= PART_MAX_ROWS_PER_TUPLE || t.deg(i) != t.deg(i - 1)) m |= 1u << k;
+        }
+        s_heads[PART_BLOCK + threadIdx.x] = (unsigned char)m;
+    }
     int tile_total;
-    const int ex = block_scan_exclusive<PART_BLOCK>(sum, OpAdd(), 0, tile_total, s_scan);
-    int64_t out = tile_offset[blockIdx.x] + ex;
+    const int ex = block_scan_exclusive<PART_BLOCK>(sum, OpAdd(), 0, tile_total, s_scan);      // synchronises: s_heads is complete
+    int64_t out = first_out + ex;
+    const unsigned window = s_heads[threadIdx.x] | s_heads[threadIdx.x + 1] << 8 | s_heads[threadIdx.x + 2] << 16;
     const int ip0 = indptr[0];
-    const int64_t my_first = t.first + (int64_t)threadIdx.x * PART_ITEMS;
 #pragma unroll
     for (int k = 0; k < PART_ITEMS; k++) {
         if (cnt[k] == 0) continue;
         const int64_t i = my_first + k;
-        const int d = t.deg(i);
+        const int d = deg[k];
         const int loc = t.ip(i) - ip0;
         if (d <= PART_DEG_BOUND) {
-            const int rows_max = part_rows_per_tuple(d);
-            int j = 1;
-            while (j < rows_max && t.deg(i + j) == d) j++;
-            block4[out] = make_int4(d, (int)i, loc, (part_warp_nz(d) << 16) + j);
+            // up to R(D) rows, as far as the run goes
+            const int run = __ffs((window >> (k + 1)) | 1u << (PART_MAX_ROWS_PER_TUPLE - 1));
+            const int j = min(part_rows_per_tuple(d), run);
+            if ((uint64_t)out < (uint64_t)cap) block4[out] = make_int4(d, (int)i, loc, (part_warp_nz(d) << 16) + j);
             out += 1;
         } else {
             int slot = PART_HEAVY_QUEUE;
@@ -252,7 +304,7 @@ part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const int *__re
             if (slot < PART_HEAVY_QUEUE) {
                 s_heavy_row[slot] = (int)i; s_heavy_deg[slot] = d; s_heavy_loc[slot] = loc; s_heavy_out[slot] = out;
             } else {
-                for (int c = 0; c < cnt[k]; c++) {
+                for (int c = 0; c < cnt[k] && (uint64_t)(out + c) < (uint64_t)cap; c++) {
                     const int done = c * PART_DEG_BOUND;
                     const int take = d - done < PART_DEG_BOUND ? d - done : PART_DEG_BOUND;
                     block4[out + c] = make_int4(d, (int)i, loc + done, take);
@@ -267,7 +319,7 @@ part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const int *__re
         const int d = s_heavy_deg[q], row = s_heavy_row[q], loc = s_heavy_loc[q];
         const int64_t o = s_heavy_out[q];
         const int n_tuples = (d + PART_DEG_BOUND - 1) / PART_DEG_BOUND;
-        for (int c = threadIdx.x; c < n_tuples; c += PART_BLOCK) {
+        for (int c = threadIdx.x; c < n_tuples && (uint64_t)(o + c) < (uint64_t)cap; c += PART_BLOCK) {
             const int done = c * PART_DEG_BOUND;
             const int take = d - done < PART_DEG_BOUND ? d - done : PART_DEG_BOUND;
             block4[o + c] = make_int4(d, row, loc + done, take);
