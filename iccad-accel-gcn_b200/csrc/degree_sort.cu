@@ -6,7 +6,7 @@
 
 namespace agcn {
 
-// A memset and five to eight launches, one synchronisation at the end (15 to 25 launches, eight allocations and
+// Two launches up to 65 536 rows, a memset and five to eight above; one synchronisation at the end (15 to 25 launches, eight allocations and
 // two synchronisations before: 0.9 ms for 16 384 rows, most of it in the allocator).
 static int degree_sort_device(const int *d_indptr, const int *d_indices, const float *d_vals,
                               int64_t n_rows, int64_t nnz, int relabel_cols,
@@ -30,6 +30,7 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
         passes = 1;
         while (passes < RADIX_PASSES && (nnz >> (passes * RADIX_BITS)) != 0) passes++;
     }
+    const bool small = n_rows <= SMALL_MAX_ROWS;
     DeviceScratch scratch(s);
     SortBuffers buf;
     SortControl *ctl = nullptr;
@@ -40,26 +41,33 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
     for (int round = 0; round < 2; round++) {
         Carver c(block);
         ctl = c.take<SortControl>(1);
-        final_state = c.take<unsigned long long>(final_tiles);
-        state = c.take<unsigned long long>(passes * tiles * RADIX_BINS);
+        final_state = c.take<unsigned long long>(small ? 0 : final_tiles);
+        state = c.take<unsigned long long>(small ? 0 : passes * tiles * RADIX_BINS);
         cleared = c.bytes();
-        for (int k = 0; k < 2; k++) { buf.keys[k] = c.take<unsigned>(n_rows); buf.rows[k] = c.take<int>(n_rows); }
+        for (int k = 0; k < 2; k++) { buf.keys[k] = c.take<unsigned>(small ? 0 : n_rows); buf.rows[k] = c.take<int>(small ? 0 : n_rows); }
         new_id = permute && relabel_cols ? c.take<int>(n_rows) : nullptr;
         tile_row = permute_tiles > 0 ? c.take<int>(permute_tiles) : nullptr;
         if (round == 0 && (block = scratch.alloc<unsigned char>((int64_t)c.bytes())) == nullptr) return AGCN_ERR_CUDA;
     }
     AGCN_HOST_WORDS(words, s);
-    AGCN_CUDA(cudaMemsetAsync(ctl, 0, cleared, s));
-    AGCN_KERNEL(degree_count_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, nnz, permute ? 1 : 0, ctl, words.device());
-    AGCN_LAUNCH_CHECK("degree_count_kernel");
-    for (int pass = 0; pass < passes; pass++) {
-        AGCN_KERNEL(radix_pass_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, pass, buf, ctl, state + pass * tiles * RADIX_BINS,
-                    words.device());
-        AGCN_LAUNCH_CHECK("radix_pass_kernel");
+    if (small) {
+        AGCN_CUDA(cudaFuncSetAttribute(sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_SMEM_BYTES));
+        sort_small_kernel<<<SMALL_CLUSTER, SMALL_BLOCK, SMALL_SMEM_BYTES, s>>>(d_indptr, (int)n_rows, (int)ceil_div(n_rows, SMALL_CLUSTER * SMALL_BLOCK), nnz,
+                                                                               permute ? 1 : 0, ctl, d_perm, d_new_indptr, new_id, tile_row, words.device());
+        AGCN_LAUNCH_CHECK("sort_small_kernel");
+    } else {
+        AGCN_CUDA(cudaMemsetAsync(ctl, 0, cleared, s));
+        AGCN_KERNEL(degree_count_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, nnz, permute ? 1 : 0, ctl, words.device());
+        AGCN_LAUNCH_CHECK("degree_count_kernel");
+        for (int pass = 0; pass < passes; pass++) {
+            AGCN_KERNEL(radix_pass_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, pass, buf, ctl, state + pass * tiles * RADIX_BINS,
+                        words.device());
+            AGCN_LAUNCH_CHECK("radix_pass_kernel");
+        }
+        AGCN_KERNEL(sort_finish_kernel, (unsigned)final_tiles, SORT_BLOCK, s, n_rows, passes, buf, ctl, final_state, d_perm, d_new_indptr,
+                    new_id, tile_row, words.device());
+        AGCN_LAUNCH_CHECK("sort_finish_kernel");
     }
-    AGCN_KERNEL(sort_finish_kernel, (unsigned)final_tiles, SORT_BLOCK, s, n_rows, passes, buf, ctl, final_state, d_perm, d_new_indptr,
-                new_id, tile_row, words.device());
-    AGCN_LAUNCH_CHECK("sort_finish_kernel");
     if (permute_tiles > 0) {
         AGCN_KERNEL(csr_permute_kernel, (unsigned)permute_tiles, PERMUTE_BLOCK, s, d_indptr, d_indices,
                     d_new_vals != nullptr ? d_vals : (const float *)nullptr, (const int *)d_perm, (const int *)d_new_indptr,

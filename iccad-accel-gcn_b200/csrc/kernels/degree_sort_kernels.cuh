@@ -16,6 +16,8 @@
 #include "../host_common.h"
 #include "primitives.cuh"
 
+#include <cooperative_groups.h>
+
 namespace agcn {
 
 constexpr int RADIX_BITS = 8;
@@ -56,24 +58,32 @@ __device__ __forceinline__ void chain_store(unsigned long long *p, unsigned long
     asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" :: "l"(p), "l"(v) : "memory");
 }
 
-// Sum of the values of all tiles before `tile`; `stride` words between tiles.  Publishes nothing.
+// Sum of the values of all tiles before `tile`; `stride` words between tiles.  Publishes nothing.  Eight
+// predecessors are read at a time: most have only their count to say when many tiles start together, and one by
+// one the walk is a chain of L2 latencies.
 __device__ __forceinline__ unsigned long long chain_look_back(const unsigned long long *state, int64_t tile, int64_t stride,
                                                               SortControl *ctl, HostWords *out)
 {
+    constexpr int AHEAD = 8;
     unsigned long long sum = 0;
-    for (int64_t t = tile - 1; t >= 0; t--) {
-        unsigned long long v = chain_load(state + t * stride);
-        for (int spin = 0; (v & ~CHAIN_VALUE) == 0; spin++) {
-            if (spin >= CHAIN_SPIN_LIMIT || *reinterpret_cast<volatile int *>(&ctl->bad) == SORT_BAD_TIMEOUT) {
-                ctl->bad = SORT_BAD_TIMEOUT;
-                out->w[SORT_WORD_TIMEOUT] = 1;
-                return sum;
+    for (int64_t t = tile - 1; t >= 0; t -= AHEAD) {
+        unsigned long long v[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) v[k] = t - k >= 0 ? chain_load(state + (t - k) * stride) : CHAIN_PREFIX;
+#pragma unroll
+        for (int k = 0; k < AHEAD; k++) {
+            for (int spin = 0; (v[k] & ~CHAIN_VALUE) == 0; spin++) {
+                if (spin >= CHAIN_SPIN_LIMIT || *reinterpret_cast<volatile int *>(&ctl->bad) == SORT_BAD_TIMEOUT) {
+                    ctl->bad = SORT_BAD_TIMEOUT;
+                    out->w[SORT_WORD_TIMEOUT] = 1;
+                    return sum;
+                }
+                if (spin > 16) __nanosleep(200);
+                v[k] = chain_load(state + (t - k) * stride);
             }
-            if (spin > 16) __nanosleep(200);
-            v = chain_load(state + t * stride);
+            sum += v[k] & CHAIN_VALUE;
+            if (v[k] & CHAIN_PREFIX) return sum;
         }
-        sum += v & CHAIN_VALUE;
-        if (v & CHAIN_PREFIX) break;
     }
     return sum;
 }
@@ -301,6 +311,155 @@ sort_finish_kernel(int64_t n, int passes, SortBuffers buf, SortControl *__restri
         const int j = k * SORT_BLOCK + threadIdx.x;
         if (base + j < n) new_indptr[base + j] = (int)s_deg[j + (j >> 5)];
     }
+}
+
+// The whole sort of a small graph in one cluster of eight thread blocks: keys stay in registers, a pass exchanges
+// them through the blocks' shared memory, and the results are those of the kernels above.  Five launches of a few
+// thread blocks each are a chain of launch, load and scan latencies: 16 384 rows took 56 us on the GPU, one thread
+// block of 16 rows per thread 35 us, this 17 us; 65 536 rows are as many as eight blocks hold.
+constexpr int SMALL_CLUSTER = 8;
+constexpr int SMALL_BLOCK = 1024;
+constexpr int SMALL_WARPS = SMALL_BLOCK / 32;
+constexpr int SMALL_ITEMS = 8;
+constexpr int SMALL_MAX_ROWS = SMALL_CLUSTER * SMALL_BLOCK * SMALL_ITEMS;
+constexpr int SMALL_SMEM_BYTES = SMALL_BLOCK * SMALL_ITEMS * 8 + SMALL_WARPS * RADIX_BINS * 2;
+
+// items = rows per thread: ceil(n / 8192), at most SMALL_ITEMS
+__global__ void __cluster_dims__(SMALL_CLUSTER, 1, 1) __launch_bounds__(SMALL_BLOCK, 1)
+sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz, int check_nnz, SortControl *__restrict__ ctl,
+                  int *__restrict__ perm, int *__restrict__ new_indptr, int *__restrict__ new_id, int *__restrict__ tile_row,
+                  HostWords *out)
+{
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    extern __shared__ unsigned s_small[];
+    unsigned *s_key = s_small;
+    int *s_row = reinterpret_cast<int *>(s_small + SMALL_BLOCK * SMALL_ITEMS);
+    unsigned short (*s_count)[RADIX_BINS] = reinterpret_cast<unsigned short (*)[RADIX_BINS]>(s_small + 2 * SMALL_BLOCK * SMALL_ITEMS);
+    __shared__ unsigned s_total[RADIX_BINS], s_base[RADIX_BINS], s_scan[SMALL_WARPS + 1];
+    __shared__ unsigned s_say[3];                // for the other blocks: largest degree, negative seen, sum of degrees
+    __shared__ unsigned s_get[SMALL_CLUSTER][2];
+    const int w = warp_id(), lane = lane_id(), block = (int)cluster.block_rank();
+    const int per_block = SMALL_BLOCK * items, first = block * per_block + w * 32 * items + lane;       // item k of this thread is row first + 32 k
+    if (threadIdx.x < 3) s_say[threadIdx.x] = 0;
+    __syncthreads();
+    unsigned key[SMALL_ITEMS], top = 0;
+    int row[SMALL_ITEMS];
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        const int i = first + k * 32;
+        row[k] = i;
+        key[k] = 0;
+        if (k < items && i < n) {
+            const int d = indptr[i + 1] - indptr[i];
+            if (d < 0) s_say[1] = 1;
+            else key[k] = (unsigned)d;
+        }
+        top = max(top, key[k]);
+    }
+    top = warp_reduce(top, OpMax());
+    if (lane == 0) atomicMax(&s_say[0], top);
+    cluster.sync();
+    if (threadIdx.x < 2 * SMALL_CLUSTER) s_get[threadIdx.x >> 1][threadIdx.x & 1] = *cluster.map_shared_rank(&s_say[threadIdx.x & 1], threadIdx.x >> 1);
+    __syncthreads();
+    bool negative = false;
+#pragma unroll
+    for (int b = 0; b < SMALL_CLUSTER; b++) { top = max(top, s_get[b][0]); negative |= s_get[b][1] != 0; }
+    const int64_t own = (int64_t)indptr[n] - (int64_t)indptr[0];
+    const bool bad = negative || (check_nnz && own != nnz);
+    if (block == 0 && threadIdx.x == 0) {
+        out->w[SORT_WORD_NNZ] = own;
+        if (negative) out->w[SORT_WORD_NEGATIVE] = 1;
+        ctl->bad = bad ? SORT_BAD_INPUT : 0;
+    }
+    for (int shift = 0; shift < 32 && (top >> shift) != 0; shift += RADIX_BITS) {
+        for (int b = threadIdx.x; b < SMALL_WARPS * RADIX_BINS / 2; b += SMALL_BLOCK) reinterpret_cast<unsigned *>(&s_count[0][0])[b] = 0;
+        __syncthreads();
+        unsigned short rank[SMALL_ITEMS];
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            if (k >= items) break;
+            const bool live = first + k * 32 < n;
+            const unsigned digit = live ? ((key[k] >> shift) & (RADIX_BINS - 1)) : (unsigned)RADIX_BINS;
+            const unsigned peers = __match_any_sync(FULL_MASK, digit);
+            const unsigned before = __popc(peers & ((1u << lane) - 1u));
+            unsigned seen = 0;
+            if (live) seen = s_count[w][digit];
+            __syncwarp();
+            if (live && before == 0) s_count[w][digit] = (unsigned short)(seen + __popc(peers));
+            __syncwarp();
+            rank[k] = (unsigned short)(seen + before);
+        }
+        __syncthreads();
+        if (threadIdx.x < RADIX_BINS) {
+            unsigned total = 0;
+#pragma unroll 8
+            for (int ww = 0; ww < SMALL_WARPS; ww++) {
+                const unsigned c = s_count[ww][threadIdx.x];
+                s_count[ww][threadIdx.x] = (unsigned short)total;
+                total += c;
+            }
+            s_total[threadIdx.x] = total;
+        }
+        cluster.sync();
+        unsigned all = 0, before = 0, unused;
+        if (threadIdx.x < RADIX_BINS) {
+#pragma unroll
+            for (int b = 0; b < SMALL_CLUSTER; b++) {
+                const unsigned c = *cluster.map_shared_rank(&s_total[threadIdx.x], b);
+                all += c;
+                before += b < block ? c : 0u;
+            }
+        }
+        const unsigned bin = block_scan_exclusive<SMALL_BLOCK>(all, OpAdd(), 0u, unused, s_scan);
+        if (threadIdx.x < RADIX_BINS) s_base[threadIdx.x] = bin + before;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            if (k < items && first + k * 32 < n) {
+                const unsigned digit = (key[k] >> shift) & (RADIX_BINS - 1);
+                const unsigned pos = s_base[digit] + s_count[w][digit] + rank[k], to = pos / (unsigned)per_block, at = pos - to * per_block;
+                *cluster.map_shared_rank(&s_key[at], to) = key[k];
+                *cluster.map_shared_rank(&s_row[at], to) = row[k];
+            }
+        }
+        cluster.sync();
+#pragma unroll
+        for (int k = 0; k < SMALL_ITEMS; k++) {
+            if (k < items && first + k * 32 < n) {
+                const int at = first - block * per_block + k * 32;
+                key[k] = s_key[at];
+                row[k] = s_row[at];
+            }
+        }
+    }
+    // row pointers: the warp's rows in order, 32 at a time (their sum fits 31 bits, or the input is bad)
+    unsigned sum = 0, total;
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) sum += warp_reduce(key[k], OpAdd());
+    const unsigned start = block_scan_exclusive<SMALL_BLOCK>(lane == 0 ? sum : 0u, OpAdd(), 0u, total, s_scan);
+    if (threadIdx.x == 0) s_say[2] = total;
+    cluster.sync();
+    if (threadIdx.x < SMALL_CLUSTER) s_get[threadIdx.x][0] = *cluster.map_shared_rank(&s_say[2], threadIdx.x);
+    __syncthreads();
+    unsigned e = __shfl_sync(FULL_MASK, start, 0);
+    for (int b = 0; b < block; b++) e += s_get[b][0];
+#pragma unroll
+    for (int k = 0; k < SMALL_ITEMS; k++) {
+        if (k >= items) break;
+        const int i = first + k * 32;
+        const unsigned incl = warp_scan_inclusive(key[k], OpAdd()), b = e + incl - key[k];
+        e += __shfl_sync(FULL_MASK, incl, 31);
+        if (i >= n) continue;
+        perm[i] = row[k];
+        if (new_id != nullptr) new_id[row[k]] = i;
+        if (new_indptr == nullptr) continue;
+        new_indptr[i] = (int)b;
+        if (i == n - 1) new_indptr[n] = (int)(b + key[k]);
+        if (tile_row != nullptr && !bad)
+            for (unsigned t = (b + PERMUTE_TILE - 1) / PERMUTE_TILE; t * PERMUTE_TILE < b + key[k]; t++) tile_row[t] = i;
+    }
+    cluster.sync();              // no block ends while another may read its shared memory
 }
 
 // CSR permute.  Each block produces PERMUTE_TILE consecutive output nonzeros.  The rows it touches (all

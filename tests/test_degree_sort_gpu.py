@@ -119,9 +119,10 @@ def test_row_pointers_at_any_alignment():
 
 
 @pytest.mark.parametrize("relabel", [False, True])
-@pytest.mark.parametrize("n,top", [(1, 5), (2047, 300), (2048, 3), (4095, 255), (4096, 256), (4097, 70_000), (12_289, 700), (70_001, 17_000_000)])
+@pytest.mark.parametrize("n,top", [(1, 5), (2047, 300), (2048, 3), (4095, 255), (4096, 256), (4097, 70_000), (8192, 300), (12_289, 700),
+                                   (65_536, 300), (65_537, 256), (69_632, 70_000), (70_001, 17_000_000)])
 def test_tile_edges_and_number_of_passes(n, top, relabel):
-    # rows around the sort tile (4096) and the row-pointer tile (2048); the largest degree decides how many of the
+    # rows around the cluster's 8192 per item and its end (65 536), the sort tile (4096) and the row-pointer tile (2048) above; the largest degree decides how many of the
     # four passes move anything (255 | 256, 65 536, 2^24), and puts rows across many tiles of the permute (2048 nonzeros)
     from accelgcn import degree_sort
     require_cuda()
