@@ -103,7 +103,7 @@ static int ctx_sync(agcn_host_ctx *c)
 static void plan_parts(agcn_host_ctx *c, const int *h_block4, int want_parts)
 {
     const int64_t n_units = ceil_div(c->n_blocks, HOST_SPMM_WARPS);
-    if (spmm_plan_splits(c->n_blocks, c->nnz)) want_parts = 1;      // its units are not those of the caller's tuples (and it is small)
+    if (spmm_plan_splits(c->n_blocks, c->n_rows, c->nnz)) want_parts = 1;      // its units are not those of the caller's tuples (and it is small)
     c->part_unit.assign(1, 0);
     c->part_row.assign(1, 0);
     c->part_loc.assign(1, 0);

@@ -36,6 +36,7 @@ struct PartitionRun {
     const int *indptr = nullptr;
     int64_t n_rows = 0, n_blocks = 0;
     void *memory = nullptr;
+    int4 *tuples = nullptr;        // in memory, where the graph was small enough to write them at once
     cudaStream_t stream = nullptr;
 };
 int partition_begin(PartitionRun *run, const int *d_indptr, int64_t n_rows, cudaStream_t s);
@@ -72,7 +73,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
 // Aligned copy of X: rows of dim floats padded with zeros to a multiple of four
 int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n_rows, cudaStream_t s);
 // Whether spmm_create would cut the tuples of a graph of that size on the current device
-bool spmm_plan_splits(int64_t n_blocks, int64_t nnz);
+bool spmm_plan_splits(int64_t n_blocks, int64_t n_rows, int64_t nnz);
 int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag, cudaStream_t s);
 void plan_free(agcn_spmm_plan *p);
 

@@ -592,42 +592,45 @@ __device__ __forceinline__ void unit_crossings(const int4 *__restrict__ block4, 
     same_row = enters && leaves && first.y == last.y;
 }
 
+// Column ids, by `blocks` thread blocks of which this is number `block`.
+__device__ __forceinline__ void plan_check_ids(const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned block, unsigned blocks, HostWords *out)
+{
+    const int64_t stride = (int64_t)blocks * blockDim.x;
+    bool bad = false;
+#pragma unroll 4
+    for (int64_t i = (int64_t)block * blockDim.x + threadIdx.x; i < n_idx; i += stride) {
+        const int c = __ldcs(idx + i);
+        bad |= c < 0 || c >= n_cols;
+    }
+    if (bad) plan_report(out, SPMM_ERR_COL);
+}
+
 // First pass over a `.block4` array: validates every tuple (and, in the blocks behind the tuple blocks,
 // every column id), and counts per PLAN_BLOCK units the rows no tuple covers and the carry slots.  One
 // launch and one read of 16 bytes per tuple and 4 per nonzero: bound by HBM for large graphs, by launch
-// latency for small ones.  most > 0: also counts the pieces of at most that many nonzeros the tuples would be cut
-// into.  ctl[0..2]: totals, ctl[3]: blocks done (zero at launch).
+// latency for small ones.  ctl[0], ctl[1]: totals, ctl[2]: blocks done (zero at launch).
 __global__ void __launch_bounds__(PLAN_BLOCK)
 plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int64_t n_rows, int64_t nnz,
                   const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned unit_grid,
-                  int most, int64_t *__restrict__ tile_zero, int *__restrict__ tile_carry, int *__restrict__ tile_pieces,
-                  unsigned long long *__restrict__ ctl, HostWords *out)
+                  int64_t *__restrict__ tile_zero, int *__restrict__ tile_carry, unsigned long long *__restrict__ ctl,
+                  HostWords *out)
 {
     if (blockIdx.x >= unit_grid) {
-        const int64_t stride = (int64_t)(gridDim.x - unit_grid) * blockDim.x;
-        bool bad = false;
-#pragma unroll 4
-        for (int64_t i = (int64_t)(blockIdx.x - unit_grid) * blockDim.x + threadIdx.x; i < n_idx; i += stride) {
-            const int c = __ldcs(idx + i);
-            bad |= c < 0 || c >= n_cols;
-        }
-        if (bad) plan_report(out, SPMM_ERR_COL);
+        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - unit_grid, gridDim.x - unit_grid, out);
         return;
     }
     __shared__ int64_t s_zero[PLAN_BLOCK / 32];
-    __shared__ int s_carry[PLAN_BLOCK / 32], s_pieces[PLAN_BLOCK / 32];
+    __shared__ int s_carry[PLAN_BLOCK / 32];
     const int64_t u = (int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x;
     int64_t zero = 0;
-    int carry = 0, err = 0, pieces = 0;
+    int carry = 0, err = 0;
     if (u < n_units || (n_units == 0 && u == 0)) {          // without any tuple, one thread counts the rows
         const int64_t e0 = u * SPMM_WARPS;
         const int64_t e1 = e0 + SPMM_WARPS < n_blocks ? e0 + SPMM_WARPS : n_blocks;
         int4 a = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
         for (int64_t e = e0; e < e1; e++) {
             const int4 b = block4[e];
-            const int tuple_err = tuple_errors(e > 0, a, b, n_rows, nnz);
-            err |= tuple_err;
-            if (most > 0 && tuple_err == 0) pieces += tuple_cut(b, most).pieces;
+            err |= tuple_errors(e > 0, a, b, n_rows, nnz);
             const int64_t g = tuple_gap(e > 0, a, b);
             zero += g > 0 ? g : 0;
             a = b;
@@ -643,24 +646,20 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
     if (err) plan_report(out, err);
     zero = warp_reduce(zero, OpAdd());
     carry = warp_reduce(carry, OpAdd());
-    pieces = warp_reduce(pieces, OpAdd());
-    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; s_pieces[warp_id()] = pieces; }
+    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        zero = 0; carry = 0; pieces = 0;
-        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; pieces += s_pieces[w]; }
+        zero = 0; carry = 0;
+        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; }
         tile_zero[blockIdx.x] = zero;
         tile_carry[blockIdx.x] = carry;
-        tile_pieces[blockIdx.x] = pieces;
         atomicAdd(ctl + 0, (unsigned long long)zero);
         atomicAdd(ctl + 1, (unsigned long long)carry);
-        atomicAdd(ctl + 2, (unsigned long long)pieces);
         __threadfence();
-        if (atomicAdd(ctl + 3, 1ull) == unit_grid - 1) {
+        if (atomicAdd(ctl + 2, 1ull) == unit_grid - 1) {
             __threadfence();
             out->w[PLAN_WORD_ZERO] = (int64_t)__ldcg(ctl + 0);
             out->w[PLAN_WORD_CARRY] = (int64_t)__ldcg(ctl + 1);
-            out->w[PLAN_WORD_PIECES] = (int64_t)__ldcg(ctl + 2);
         }
     }
 }
@@ -689,37 +688,9 @@ __device__ __forceinline__ int64_t tuple_lower_bound(const int4 *__restrict__ bl
     return lo;
 }
 
-// Writes the pieces of every tuple, in tuple order (small plans only: a handful of thread blocks).
-__global__ void __launch_bounds__(PLAN_BLOCK)
-plan_split_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int most, const int *__restrict__ tile_pieces, int4 *__restrict__ pieces)
-{
-    __shared__ int s_scan[PLAN_BLOCK / 32 + 1];
-    int before = 0, base, total;
-    for (int k = threadIdx.x; k < (int)blockIdx.x; k += PLAN_BLOCK) before += tile_pieces[k];
-    block_scan_exclusive<PLAN_BLOCK>(before, OpAdd(), 0, base, s_scan);
-    const int64_t e0 = ((int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x) * SPMM_WARPS;
-    int mine = 0;
-    for (int64_t e = e0; e < e0 + SPMM_WARPS && e < n_blocks; e++) mine += tuple_cut(block4[e], most).pieces;
-    int4 *out = pieces + base + block_scan_exclusive<PLAN_BLOCK>(mine, OpAdd(), 0, total, s_scan);
-    for (int64_t e = e0; e < e0 + SPMM_WARPS && e < n_blocks; e++) {
-        const int4 b = block4[e];
-        const TupleCut c = tuple_cut(b, most);
-        const int rows = tuple_rows(b), row_nz = tuple_is_big(b) ? b.w : b.x;
-        if (c.row_pieces == 0) {
-            for (int r = 0; r < rows; r += c.rows_each)
-                *out++ = make_int4(b.x, b.y + r, b.z + r * row_nz, rows - r < c.rows_each ? rows - r : c.rows_each);
-        } else {
-            for (int r = 0; r < rows; r++)
-                for (int k = 0; k < row_nz; k += c.nz_each)
-                    *out++ = make_int4(SPMM_DEG_BOUND + 1, b.y + r, b.z + r * row_nz + k, row_nz - k < c.nz_each ? row_nz - k : c.nz_each);
-        }
-    }
-}
-
 // Second pass: carry slots in unit order, and the list of rows no tuple covers.  A block adds up the counts
 // of the tiles before it itself (a few thousand words at most) -- no scan launches between the passes.
 // Gaps of many rows (the degree-0 rows of an ordered graph are one gap) are written by the whole block.
-// tile_zero == nullptr: the tuples are pieces nobody has counted; a block counts the units before its own (few).
 constexpr int PLAN_INLINE_GAP = 16, PLAN_GAP_QUEUE = 64;
 
 __global__ void __launch_bounds__(PLAN_BLOCK)
@@ -733,19 +704,7 @@ plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_
     __shared__ int s_gaps;
     if (threadIdx.x == 0) s_gaps = 0;
     int64_t zb = 0, cb = 0;
-    if (tile_zero != nullptr) {
-        for (int64_t k = threadIdx.x; k < blockIdx.x; k += PLAN_BLOCK) { zb += tile_zero[k]; cb += tile_carry[k]; }
-    } else {
-        for (int64_t k = threadIdx.x; k < (int64_t)blockIdx.x * PLAN_BLOCK; k += PLAN_BLOCK) {
-            bool en, lv, same;
-            int ri, ro;
-            unit_crossings(block4, n_blocks, k, en, lv, same, ri, ro);
-            cb += (en ? 1 : 0) + (lv ? 1 : 0) - (same ? 1 : 0);
-            if (zero_rows != nullptr)
-                for (int64_t e = k * SPMM_WARPS; e < (k + 1) * SPMM_WARPS; e++)
-                    zb += tuple_gap(e > 0, e > 0 ? block4[e - 1] : make_int4(0, 0, 0, 0), block4[e]);
-        }
-    }
+    for (int64_t k = threadIdx.x; k < blockIdx.x; k += PLAN_BLOCK) { zb += tile_zero[k]; cb += tile_carry[k]; }
     int64_t zero_base, carry_base, total;
     block_scan_exclusive<PLAN_BLOCK>(zb, OpAdd(), (int64_t)0, zero_base, s_scan64);
     block_scan_exclusive<PLAN_BLOCK>(cb, OpAdd(), (int64_t)0, carry_base, s_scan64);
@@ -803,6 +762,118 @@ plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_
     const int gaps = s_gaps < PLAN_GAP_QUEUE ? s_gaps : PLAN_GAP_QUEUE;
     for (int q = 0; q < gaps; q++)
         for (int64_t k = threadIdx.x; k < s_gap_len[q]; k += PLAN_BLOCK) zero_rows[s_gap_out[q] + k] = (int)(s_gap_row[q] + k);
+}
+
+// The whole plan of a small graph in one launch: block 0 validates the tuples, cuts them into pieces of at most
+// `most` nonzeros (cap_pieces of them fit), lists the rows no tuple covers and hands out the carry slots; the other
+// blocks check the column ids.  Every array has its final place already, sized by bounds the host knows, so the
+// host waits once.  (Two kernels with a wait between them before, the cutting 8 tuples per thread: a plan of 16 384
+// rows took 70 us; 26 now, 12 of them on the GPU.)  Bound by latency: a chain of scans over about ten tuples per thread.
+constexpr int PLAN_SMALL_BLOCK = 1024;
+
+__global__ void __launch_bounds__(PLAN_SMALL_BLOCK)
+plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows, int64_t nnz, const int *__restrict__ idx, int64_t n_idx,
+                  int64_t n_cols, int most, int4 *pieces, int cap_pieces, int2 *unit_carry, int2 *carry_span, int *carry_row, int *zero_rows,
+                  HostWords *out)
+{
+    if (blockIdx.x > 0) {
+        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - 1, gridDim.x - 1, out);
+        return;
+    }
+    __shared__ int s_scan[PLAN_SMALL_BLOCK / 32 + 1];
+    __shared__ int s_gap_out[PLAN_GAP_QUEUE], s_gap_row[PLAN_GAP_QUEUE], s_gap_len[PLAN_GAP_QUEUE];
+    __shared__ int s_gaps;
+    if (threadIdx.x == 0) s_gaps = 0;
+    const int each = (n_blocks + PLAN_SMALL_BLOCK - 1) / PLAN_SMALL_BLOCK;
+    const int e0 = min((int)threadIdx.x * each, n_blocks), e1 = min(e0 + each, n_blocks);
+    const int4 before = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
+    int4 a = before;
+    int err = 0, mine = 0;
+    int64_t zero = 0;
+    for (int e = e0; e < e1; e++) {
+        const int4 b = block4[e];
+        err |= tuple_errors(e > 0, a, b, n_rows, nnz);
+        if (err == 0) { mine += tuple_cut(b, most).pieces; zero += tuple_gap(e > 0, a, b); }
+        a = b;
+    }
+    const bool last = e0 < e1 && e1 == n_blocks;
+    if (last && err == 0) zero += n_rows - ((int64_t)a.y + tuple_rows(a));
+    if (err) plan_report(out, err);
+    if (__syncthreads_or(err)) return;
+    int n_pieces, n_zero;
+    int piece = block_scan_exclusive<PLAN_SMALL_BLOCK>(mine, OpAdd(), 0, n_pieces, s_scan);
+    int zero_out = block_scan_exclusive<PLAN_SMALL_BLOCK>((int)zero, OpAdd(), 0, n_zero, s_scan);
+    if (threadIdx.x == 0) { out->w[PLAN_WORD_ZERO] = n_zero; out->w[PLAN_WORD_PIECES] = n_pieces; }
+    if (n_pieces > cap_pieces) return;              // cannot be: valid tuples do not overlap
+    a = before;
+    for (int e = e0; e < e1; e++) {
+        const int4 b = block4[e];
+        const TupleCut c = tuple_cut(b, most);
+        const int rows = tuple_rows(b), row_nz = tuple_is_big(b) ? b.w : b.x;
+        if (c.row_pieces == 0) {
+            for (int r = 0; r < rows; r += c.rows_each)
+                pieces[piece++] = make_int4(b.x, b.y + r, b.z + r * row_nz, rows - r < c.rows_each ? rows - r : c.rows_each);
+        } else {
+            for (int r = 0; r < rows; r++)
+                for (int k = 0; k < row_nz; k += c.nz_each)
+                    pieces[piece++] = make_int4(SPMM_DEG_BOUND + 1, b.y + r, b.z + r * row_nz + k, row_nz - k < c.nz_each ? row_nz - k : c.nz_each);
+        }
+        a = b;
+    }
+    if (zero > 0) {
+        a = before;
+        for (int e = e0; e < e1 + (last ? 1 : 0); e++) {
+            const int4 b = e < e1 ? block4[e] : make_int4(0, 0, 0, 0);
+            const int first = e > 0 ? a.y + tuple_rows(a) : 0;
+            const int g = e < e1 ? (int)tuple_gap(e > 0, a, b) : (int)(n_rows - first);
+            int q = PLAN_GAP_QUEUE;
+            if (g > PLAN_INLINE_GAP) q = atomicAdd(&s_gaps, 1);
+            if (q < PLAN_GAP_QUEUE) { s_gap_out[q] = zero_out; s_gap_row[q] = first; s_gap_len[q] = g; }
+            else for (int k = 0; k < g; k++) zero_rows[zero_out + k] = first + k;
+            zero_out += g;
+            a = b;
+        }
+    }
+    __syncthreads();                // the pieces are there, and the queue of gaps
+    for (int q = 0; q < min(s_gaps, PLAN_GAP_QUEUE); q++)
+        for (int k = threadIdx.x; k < s_gap_len[q]; k += PLAN_SMALL_BLOCK) zero_rows[s_gap_out[q] + k] = s_gap_row[q] + k;
+
+    // Carry slots: a row that crosses units has one in every unit it touches, consecutive ones.  `chain` = first slot
+    // of the row that is open when a unit begins.
+    const int n_units = (n_pieces + SPMM_WARPS - 1) / SPMM_WARPS;
+    int slot_base = 0, chain_base = -1;
+    for (int u0 = 0; u0 < n_units; u0 += PLAN_SMALL_BLOCK) {
+        const int u = u0 + threadIdx.x;
+        bool en = false, lv = false;
+        int row_in = 0;
+        if (u < n_units) {
+            const int p0 = u * SPMM_WARPS, p1 = min(p0 + SPMM_WARPS, n_pieces);
+            const int4 head = __ldcg(pieces + p0), tail = __ldcg(pieces + p1 - 1);
+            row_in = head.y;
+            if (p0 > 0 && tuple_is_big(head)) {
+                const int4 x = __ldcg(pieces + p0 - 1);
+                en = tuple_is_big(x) && x.y == head.y;
+            }
+            if (p1 < n_pieces && tuple_is_big(tail)) {
+                const int4 x = __ldcg(pieces + p1);
+                lv = tuple_is_big(x) && x.y == tail.y;
+            }
+        }
+        const bool same = en && lv && u < n_units && __ldcg(pieces + min((u + 1) * SPMM_WARPS, n_pieces) - 1).y == row_in;
+        const bool opens = lv && !same;
+        int slots, chain_last;
+        const int slot = slot_base + block_scan_exclusive<PLAN_SMALL_BLOCK>((en ? 1 : 0) + (opens ? 1 : 0), OpAdd(), 0, slots, s_scan);
+        const int out_slot = slot + (en ? 1 : 0);
+        int chain = block_scan_exclusive<PLAN_SMALL_BLOCK>(opens ? out_slot : -1, OpMax(), -1, chain_last, s_scan);
+        chain = max(chain, chain_base);
+        if (u < n_units) {
+            unit_carry[u] = make_int2(en ? slot : -1, lv ? (same ? slot : out_slot) : -1);
+            if (en && !same)             // the row ends here: its slots are chain .. slot
+                for (int q = chain; q <= slot; q++) { carry_span[q] = make_int2(chain, slot - chain + 1); carry_row[q] = row_in; }
+        }
+        slot_base += slots;
+        chain_base = max(chain_base, chain_last);
+    }
 }
 
 }  // namespace agcn

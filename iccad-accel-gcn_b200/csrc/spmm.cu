@@ -39,16 +39,18 @@ static int spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
     return 0;
 }
 
-static int spmm_piece_choice(int64_t n_blocks, int64_t nnz, int sm_count)
+// A cut plan keeps room for a list of all rows: not where there are a great many without any nonzero.
+static int spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int sm_count)
 {
-    return n_blocks > 0 ? env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count)) : 0;
+    if (n_blocks == 0 || n_rows > ((int64_t)1 << 20)) return 0;
+    return env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count));
 }
 
-bool spmm_plan_splits(int64_t n_blocks, int64_t nnz)
+bool spmm_plan_splits(int64_t n_blocks, int64_t n_rows, int64_t nnz)
 {
     int device = 0, sm_count = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return true;
-    return spmm_piece_choice(n_blocks, nnz, sm_count) > 0;
+    return spmm_piece_choice(n_blocks, n_rows, nnz, sm_count) > 0;
 }
 
 // Order of the units, which are in ascending degree.  Starting at the heavy end leaves light units for the end of
@@ -64,73 +66,26 @@ static int spmm_light_every(const agcn_spmm_plan *p, int width)
     return p->n_units > (int64_t)28 * p->sm_count && x_bytes <= 0.6 * p->l2_bytes ? 4 : 0;
 }
 
-// Two launches: the first pass counts and validates, the host sizes the plan's one pool block from its
-// answer, the second pass fills it.  (Six cudaMalloc / cudaFree pairs and nine launches before; a plan of
-// 16 384 rows took about 1 ms, most of it in the allocator.)
-int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, const int *d_indices,
-                       int64_t n_rows, int64_t n_cols, int64_t nnz, cudaStream_t s)
+static int plan_errors(const HostWordsLease &words)
 {
-    AGCN_REQUIRE(out != nullptr, "agcn_spmm_create: null plan pointer");
-    *out = nullptr;
-    AGCN_REQUIRE(n_blocks >= 0 && (n_blocks == 0 || d_block4 != nullptr), "agcn_spmm_create: null block4");
-    AGCN_REQUIRE(aligned16(d_block4), "agcn_spmm_create: block4 must be 16-byte aligned");
-    AGCN_REQUIRE(n_rows > 0 && n_rows < (int64_t)INT32_MAX && n_cols > 0 && n_cols < (int64_t)INT32_MAX,
-                 "agcn_spmm_create: n_rows / n_cols out of range");
-    AGCN_REQUIRE(nnz >= 0 && nnz <= (int64_t)INT32_MAX, "agcn_spmm_create: nnz out of range");
-    AGCN_REQUIRE(n_blocks < (int64_t)INT32_MAX, "agcn_spmm_create: too many blocks");
-
-    const int4 *block4 = reinterpret_cast<const int4 *>(d_block4);
-    int device = 0, sm_count = 0, l2_bytes = 0;
-    AGCN_CUDA(cudaGetDevice(&device));
-    AGCN_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
-    AGCN_CUDA(cudaDeviceGetAttribute(&l2_bytes, cudaDevAttrL2CacheSize, device));
-    const int64_t n_units = ceil_div(n_blocks, SPMM_WARPS);
-    const int most = spmm_piece_choice(n_blocks, nnz, sm_count);
-    const int64_t tiles = n_units > 0 ? ceil_div(n_units, PLAN_BLOCK) : 1;
-    DeviceScratch scratch(s);
-    Carver size;
-    size.take<unsigned long long>(4); size.take<int64_t>(tiles); size.take<int>(tiles); size.take<int>(tiles);
-    AGCN_ALLOC(block, scratch, unsigned char, (int64_t)size.bytes());
-    Carver c(block);
-    unsigned long long *ctl = c.take<unsigned long long>(4);
-    int64_t *tile_zero = c.take<int64_t>(tiles);
-    int *tile_carry = c.take<int>(tiles), *tile_pieces = c.take<int>(tiles);
-    AGCN_HOST_WORDS(words, s);
-    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(*ctl), s));
-    // 16 column ids per thread, at most 64 thread blocks per SM's worth of them
-    const int64_t n_idx = d_indices != nullptr ? nnz : 0;
-    const int64_t col_grid = n_idx > 0 ? ceil_div(n_idx, PLAN_BLOCK * 16) : 0;
-    const unsigned grid = (unsigned)(tiles + (col_grid < 9472 ? col_grid : 9472));
-    AGCN_KERNEL(plan_check_kernel, grid, PLAN_BLOCK, s, block4, n_blocks, n_units, n_rows, nnz, d_indices, n_idx, n_cols, (unsigned)tiles,
-                most, tile_zero, tile_carry, tile_pieces, ctl, words.device());
-    AGCN_LAUNCH_CHECK("plan_check_kernel");
-    AGCN_CUDA(words.sync());
     int err = 0;
     for (int k = 0; k < PLAN_ERR_BITS; k++) err |= words[PLAN_WORD_ERR + k] != 0 ? 1 << k : 0;
-    if (err != 0) {
-        set_error("agcn_spmm_create: invalid input:%s%s%s%s",
-                  (err & SPMM_ERR_TUPLE) ? " malformed .block4 tuple;" : "",
-                  (err & SPMM_ERR_ROW) ? " tuple rows out of range or not ascending;" : "",
-                  (err & SPMM_ERR_LOC) ? " tuple nonzero range outside [0, nnz) or out of order;" : "",
-                  (err & SPMM_ERR_COL) ? " column index outside [0, n_cols);" : "");
-        return AGCN_ERR_RANGE;
-    }
+    if (err == 0) return AGCN_OK;
+    set_error("agcn_spmm_create: invalid input:%s%s%s%s",
+              (err & SPMM_ERR_TUPLE) ? " malformed .block4 tuple;" : "",
+              (err & SPMM_ERR_ROW) ? " tuple rows out of range or not ascending;" : "",
+              (err & SPMM_ERR_LOC) ? " tuple nonzero range outside [0, nnz) or out of order;" : "",
+              (err & SPMM_ERR_COL) ? " column index outside [0, n_cols);" : "");
+    return AGCN_ERR_RANGE;
+}
 
-    agcn_spmm_plan *p = new (std::nothrow) agcn_spmm_plan;
-    AGCN_REQUIRE(p != nullptr, "agcn_spmm_create: out of host memory");
-    struct Guard { agcn_spmm_plan *p; ~Guard() { plan_free(p); } } guard{p};       // frees the half-built plan on every early return
-    p->device = device; p->sm_count = sm_count; p->l2_bytes = l2_bytes;
-    p->block4 = block4; p->n_blocks = n_blocks;
-    p->split = most > 0;
-    p->n_tuples = p->split ? words[PLAN_WORD_PIECES] : n_blocks;
-    p->n_units = ceil_div(p->n_tuples, SPMM_WARPS);
-    p->n_rows = n_rows; p->n_cols = n_cols; p->nnz = nnz;
-    p->n_zero = words[PLAN_WORD_ZERO];
-    p->n_carry = p->split ? 2 * p->n_units : words[PLAN_WORD_CARRY];       // of pieces only a bound is known here
-    int4 *pieces = nullptr;
+// The plan's arrays, in one pool block: n_pieces tuples of its own (0: it walks the caller's), bookkeeping of its
+// units, n_carry slots, n_zero rows.
+static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int4 **pieces, cudaStream_t s)
+{
     for (int pass = 0; pass < 2; pass++) {
         Carver m(p->memory);
-        pieces = p->split ? m.take<int4>(p->n_tuples) : nullptr;
+        *pieces = m.take<int4>(n_pieces);
         p->unit_carry = m.take<int2>(p->n_units);
         p->carry_span = m.take<int2>(p->n_carry);
         p->carry_row = m.take<int>(p->n_carry);
@@ -145,23 +100,106 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
     }
     if (p->n_carry > 0)
         AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(p->carry, p->n_carry), 0, (size_t)p->n_carry * SPMM_CARRY_PASSES * sizeof(int), s));
-    p->tuples = block4;
-    if (p->split) {
-        AGCN_KERNEL(plan_split_kernel, (unsigned)tiles, PLAN_BLOCK, s, block4, n_blocks, most, (const int *)tile_pieces, pieces);
-        AGCN_LAUNCH_CHECK("plan_split_kernel");
-        p->tuples = pieces;
-        tile_zero = nullptr;             // they were counted for the uncut tuples
-    }
+    return AGCN_OK;
+}
+
+// One launch and one wait: the memory is sized by what the pieces can be at most (a piece that is not the last of
+// its tuple or row holds more than half of `most` nonzeros).
+static int plan_fill_small(agcn_spmm_plan *p, int most, const int *d_indices, int64_t n_idx, cudaStream_t s)
+{
+    const int64_t cap = p->n_blocks + 2 * p->nnz / most + 8;
+    AGCN_REQUIRE(cap < (int64_t)INT32_MAX / 4, "agcn_spmm_create: too many pieces");
+    p->split = true;
+    p->n_units = ceil_div(cap, SPMM_WARPS);
+    p->n_carry = 2 * p->n_units;
+    p->n_zero = p->n_rows;
+    int4 *pieces = nullptr;
+    int rc = plan_memory(p, cap, &pieces, s);
+    if (rc != AGCN_OK) return rc;
+    AGCN_HOST_WORDS(words, s);
+    const int64_t col_blocks = ceil_div(n_idx, PLAN_SMALL_BLOCK * 16);
+    AGCN_KERNEL(plan_small_kernel, (unsigned)(1 + (col_blocks < 2368 ? col_blocks : 2368)), PLAN_SMALL_BLOCK, s, p->block4, (int)p->n_blocks,
+                p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, most, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
+                p->zero_rows, words.device());
+    AGCN_LAUNCH_CHECK("plan_small_kernel");
+    AGCN_CUDA(words.sync());
+    rc = plan_errors(words);
+    if (rc != AGCN_OK) return rc;
+    AGCN_REQUIRE(words[PLAN_WORD_PIECES] <= cap, "agcn_spmm_create: more pieces than the tuples can have");
+    p->tuples = pieces;
+    p->n_tuples = words[PLAN_WORD_PIECES];
+    p->n_units = ceil_div(p->n_tuples, SPMM_WARPS);
+    p->n_zero = words[PLAN_WORD_ZERO];
+    return AGCN_OK;
+}
+
+// Two launches: the first pass counts and validates, the host sizes the plan's one pool block from its
+// answer, the second pass fills it.  (Six cudaMalloc / cudaFree pairs and nine launches before.)
+static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cudaStream_t s)
+{
+    p->tuples = p->block4;
+    p->n_tuples = p->n_blocks;
+    p->n_units = ceil_div(p->n_blocks, SPMM_WARPS);
+    const int64_t tiles = p->n_units > 0 ? ceil_div(p->n_units, PLAN_BLOCK) : 1;
+    DeviceScratch scratch(s);
+    Carver size;
+    size.take<unsigned long long>(3); size.take<int64_t>(tiles); size.take<int>(tiles);
+    AGCN_ALLOC(block, scratch, unsigned char, (int64_t)size.bytes());
+    Carver c(block);
+    unsigned long long *ctl = c.take<unsigned long long>(3);
+    int64_t *tile_zero = c.take<int64_t>(tiles);
+    int *tile_carry = c.take<int>(tiles);
+    AGCN_HOST_WORDS(words, s);
+    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 3 * sizeof(*ctl), s));
+    // 16 column ids per thread, at most 64 thread blocks per SM's worth of them
+    const int64_t col_grid = n_idx > 0 ? ceil_div(n_idx, PLAN_BLOCK * 16) : 0;
+    const unsigned grid = (unsigned)(tiles + (col_grid < 9472 ? col_grid : 9472));
+    AGCN_KERNEL(plan_check_kernel, grid, PLAN_BLOCK, s, p->block4, p->n_blocks, p->n_units, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols,
+                (unsigned)tiles, tile_zero, tile_carry, ctl, words.device());
+    AGCN_LAUNCH_CHECK("plan_check_kernel");
+    AGCN_CUDA(words.sync());
+    int rc = plan_errors(words);
+    if (rc != AGCN_OK) return rc;
+    p->n_zero = words[PLAN_WORD_ZERO];
+    p->n_carry = words[PLAN_WORD_CARRY];
+    int4 *pieces = nullptr;
+    rc = plan_memory(p, 0, &pieces, s);
+    if (rc != AGCN_OK) return rc;
     if (p->n_carry > 0 || p->n_zero > 0) {
-        const int64_t assign_tiles = p->n_units > 0 ? ceil_div(p->n_units, PLAN_BLOCK) : 1;
-        AGCN_KERNEL(plan_assign_kernel, (unsigned)assign_tiles, PLAN_BLOCK, s, p->tuples, p->n_tuples, p->n_units, n_rows,
-                    (const int64_t *)tile_zero, (const int *)tile_carry, p->unit_carry, p->carry_span, p->carry_row,
-                    p->n_zero > 0 ? p->zero_rows : nullptr);
+        AGCN_KERNEL(plan_assign_kernel, (unsigned)tiles, PLAN_BLOCK, s, p->tuples, p->n_tuples, p->n_units, p->n_rows, (const int64_t *)tile_zero,
+                    (const int *)tile_carry, p->unit_carry, p->carry_span, p->carry_row, p->n_zero > 0 ? p->zero_rows : nullptr);
         AGCN_LAUNCH_CHECK("plan_assign_kernel");
-    } else if (n_units > 0) {
-        AGCN_CUDA(cudaMemsetAsync(p->unit_carry, 0xff, (size_t)n_units * sizeof(int2), s));      // no row crosses units
+    } else if (p->n_units > 0) {
+        AGCN_CUDA(cudaMemsetAsync(p->unit_carry, 0xff, (size_t)p->n_units * sizeof(int2), s));      // no row crosses units
     }
     AGCN_CUDA(cudaStreamSynchronize(s));          // products may run on any stream
+    return AGCN_OK;
+}
+
+int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, const int *d_indices,
+                       int64_t n_rows, int64_t n_cols, int64_t nnz, cudaStream_t s)
+{
+    AGCN_REQUIRE(out != nullptr, "agcn_spmm_create: null plan pointer");
+    *out = nullptr;
+    AGCN_REQUIRE(n_blocks >= 0 && (n_blocks == 0 || d_block4 != nullptr), "agcn_spmm_create: null block4");
+    AGCN_REQUIRE(aligned16(d_block4), "agcn_spmm_create: block4 must be 16-byte aligned");
+    AGCN_REQUIRE(n_rows > 0 && n_rows < (int64_t)INT32_MAX && n_cols > 0 && n_cols < (int64_t)INT32_MAX,
+                 "agcn_spmm_create: n_rows / n_cols out of range");
+    AGCN_REQUIRE(nnz >= 0 && nnz <= (int64_t)INT32_MAX, "agcn_spmm_create: nnz out of range");
+    AGCN_REQUIRE(n_blocks < (int64_t)INT32_MAX, "agcn_spmm_create: too many blocks");
+
+    agcn_spmm_plan *p = new (std::nothrow) agcn_spmm_plan;
+    AGCN_REQUIRE(p != nullptr, "agcn_spmm_create: out of host memory");
+    struct Guard { agcn_spmm_plan *p; ~Guard() { plan_free(p); } } guard{p};       // frees the half-built plan on every early return
+    AGCN_CUDA(cudaGetDevice(&p->device));
+    AGCN_CUDA(cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device));
+    AGCN_CUDA(cudaDeviceGetAttribute(&p->l2_bytes, cudaDevAttrL2CacheSize, p->device));
+    p->block4 = reinterpret_cast<const int4 *>(d_block4);
+    p->n_blocks = n_blocks; p->n_rows = n_rows; p->n_cols = n_cols; p->nnz = nnz;
+    const int64_t n_idx = d_indices != nullptr ? nnz : 0;
+    const int most = spmm_piece_choice(n_blocks, n_rows, nnz, p->sm_count);
+    const int rc = most > 0 ? plan_fill_small(p, most, d_indices, n_idx, s) : plan_fill(p, d_indices, n_idx, s);
+    if (rc != AGCN_OK) return rc;
     p->panel_override = env_int("AGCN_SPMM_PANEL", 0);
     p->pad_unaligned = env_int("AGCN_SPMM_PAD", 1);
     guard.p = nullptr;
