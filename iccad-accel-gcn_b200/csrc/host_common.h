@@ -110,7 +110,7 @@ private:
 
 // Words in pinned host memory that kernels store results and error codes into (memory.cu).
 struct HostWords {
-    enum { COUNT = 7 };
+    enum { COUNT = 8 };
     int64_t w[COUNT];
 };
 

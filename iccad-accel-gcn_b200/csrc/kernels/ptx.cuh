@@ -18,13 +18,19 @@ namespace agcn {
 struct L2Policies {
     uint64_t keep;     // evict_last
     uint64_t stream;   // evict_first
+    int hot;           // first column whose row of X is to be kept
 };
+
+// Rows of X from column `hot` on are to stay in L2, the others are to leave first (HOT: X many times larger than L2).
+template <bool HOT>
+__device__ __forceinline__ uint64_t x_policy(const L2Policies &p, int column) { return !HOT || column >= p.hot ? p.keep : p.stream; }
 
 __device__ __forceinline__ L2Policies make_l2_policies()
 {
     L2Policies p;
     asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p.keep));
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p.stream));
+    p.hot = 0;
     return p;
 }
 

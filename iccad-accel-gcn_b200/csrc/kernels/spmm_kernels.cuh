@@ -44,15 +44,17 @@ constexpr int SPMM_THREADS = SPMM_WARPS * 32;
 constexpr int SPMM_PANEL = 128;        // dense columns covered by one launch
 constexpr int SPMM_ZERO_ROWS_PER_BLOCK = 64;
 // Gathers a lane keeps in flight, and thread blocks per SM the register budget is capped for.
-// Measured on B200: 4 in flight x 5 blocks (40 warps per SM, 48 registers) beats 8 x 3 by 10-20 %
-// and 2 x 6 / 2 x 7 by up to 30 % -- the gather wants occupancy more than per-warp depth.
-constexpr int SPMM_GATHER_BATCH = 4;
-constexpr int SPMM_MIN_BLOCKS = 40 / SPMM_WARPS;      // 40 resident warps per SM
+// Seven gathers at 4 blocks (32 warps per SM, 64 registers) are 1-8 % faster than four at 5 blocks (48 registers)
+// for widths up to 16 and above 32, six or eight 2-8 % slower than seven; at 17..32 columns, where a warp takes four
+// nonzeros at a time, the 40 warps are 2-5 % faster.  (2.4 M rows of 25, B200, us: dim 16 601 -> 555, dim 64 1490 ->
+// 1447, dim 128 2983 -> 2875; 700 000 rows of 15, dim 64: 235 -> 221.  More gathers at fewer blocks lose 5-30 %.)
+constexpr int SPMM_GATHER_BATCH = 7, SPMM_MIN_BLOCKS = 4;
+constexpr int SPMM_WIDE_GATHER_BATCH = 4, SPMM_WIDE_MIN_BLOCKS = 5;
 // Small products (no more tuples than the GPU has room for warps) cannot hide latency with occupancy, and what they
 // wait for is the warp that walks 384 nonzeros alone.  Their plan cuts the tuples into pieces of fewer nonzeros
-// (plan_split_kernel), and the kernel keeps more gathers in flight per lane.
-constexpr int SPMM_SMALL_GATHER_BATCH = 8;
-constexpr int SPMM_SMALL_MIN_BLOCKS = 4;
+// (plan_small_kernel), and where they fit two blocks per SM the kernel keeps more gathers in flight per lane
+// (16 384 rows of 8, dim 60: 9.0 -> 8.6 us).
+constexpr int SPMM_DEEP_GATHER_BATCH = 16, SPMM_DEEP_MIN_BLOCKS = 2;
 
 struct SpmmParams {
     const int4 *tuples;       // the plan's: `.block4`, or its pieces
@@ -75,6 +77,7 @@ struct SpmmParams {
                               // null: spmm_carry_kernel follows
     const int *zero_rows;     // rows no tuple covers
     int64_t n_zero_rows;
+    int hot_column;           // HOT kernels: rows of X from this column on are kept in L2; 0: no such choice
     int relu;                 // nonzero: Y = max(A * X, 0) (fused GCN activation)
     // The fields below are read only by the general (PLAIN = false) kernel flavour.
     int accumulate;           // nonzero: Y += A * X (later column ranges of a column-tiled product)
@@ -146,9 +149,9 @@ __device__ __forceinline__ void fma4(float4 &acc, float a, const float4 &v)
 }
 
 // UNROLL independent 16-byte loads are issued per lane before the first FMA needs one.
-template <int UNROLL>
+template <int UNROLL, bool HOT>
 __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int first, int step,
-                                              const float *__restrict__ x, int64_t ldx, bool active, uint64_t keep)
+                                              const float *__restrict__ x, int64_t ldx, bool active, const L2Policies &pol)
 {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (!active) return acc;
@@ -159,7 +162,7 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) p[u] = pairs[i + u * step];
 #pragma unroll
-        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)p[u].x * ldx, keep);
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)p[u].x * ldx, x_policy<HOT>(pol, p[u].x));
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) fma4(acc, __int_as_float(p[u].y), v[u]);
     }
@@ -171,7 +174,7 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
         for (int u = 0; u < UNROLL - 1; u++) {
             const bool live = i + u * step < count;
             p[u] = live ? pairs[i + u * step] : make_int2(0, 0);
-            v[u] = live ? ld_x4(x + (int64_t)p[u].x * ldx, keep) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = live ? ld_x4(x + (int64_t)p[u].x * ldx, x_policy<HOT>(pol, p[u].x)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < UNROLL - 1; u++)
@@ -183,7 +186,7 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
 // `rows` consecutive rows of row_nz nonzeros each, whole rows for this lane: one stream of gathers, UNROLL in
 // flight across row boundaries.  (Row by row, rows of three nonzeros keep three gathers in flight and a slot with
 // six of them waits six times.)
-template <int UNROLL, bool PLAIN>
+template <int UNROLL, bool PLAIN, bool HOT>
 __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pairs, int rows, int row_nz, const float *__restrict__ x,
                                              float *yr, int col, const L2Policies &pol)
 {
@@ -206,7 +209,7 @@ __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pa
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) q[u] = pairs[i + u];
 #pragma unroll
-        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)q[u].x * p.ldx, pol.keep);
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)q[u].x * p.ldx, x_policy<HOT>(pol, q[u].x));
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) take(__int_as_float(q[u].y), v[u]);
     }
@@ -217,7 +220,7 @@ __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pa
         for (int u = 0; u < UNROLL - 1; u++) {
             const bool live = i + u < count;
             q[u] = live ? pairs[i + u] : make_int2(0, 0);
-            v[u] = live ? ld_x4(x + (int64_t)q[u].x * p.ldx, pol.keep) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = live ? ld_x4(x + (int64_t)q[u].x * p.ldx, x_policy<HOT>(pol, q[u].x)) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < UNROLL - 1; u++)
@@ -328,8 +331,9 @@ __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 spa
 // FINISH: rows that cross units are finished here (in launches of few units);
 // a template parameter because the code costs registers the large launches
 // do not have (two more spills, 3 % of a product of 500 000 rows).
+// HOT: rows of X the L2 is to keep are told from the others.
 // ---------------------------------------------------------------------------
-template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH>
+template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT>
 __global__ void __launch_bounds__(SPMM_THREADS, MIN_BLOCKS)
 spmm_units_kernel(const SpmmParams p)
 {
@@ -345,7 +349,8 @@ spmm_units_kernel(const SpmmParams p)
     const int slot = lane / LANES, sl = lane % LANES;
     const int col = VEC ? sl * 4 : sl;
     const bool active = col < p.dim;
-    const L2Policies pol = make_l2_policies();
+    L2Policies pol = make_l2_policies();
+    if (HOT) pol.hot = p.hot_column;
 
     if (p.abort_flag != nullptr && *p.abort_flag != 0) return;     // input rejected by a check earlier in the stream
     if ((int64_t)blockIdx.x >= p.n_units) {
@@ -390,11 +395,11 @@ spmm_units_kernel(const SpmmParams p)
             const int each = (t.n_rows + NS - 1) / NS, r0 = slot * each;
             const int rows = r0 < t.n_rows ? (r0 + each < t.n_rows ? each : t.n_rows - r0) : 0;
             if (active)
-                gather_rows4<BATCH, PLAIN>(p, pairs + r0 * t.row_nz, rows, t.row_nz, xc, p.y + (int64_t)(t.row0 + r0) * p.ldy, col, pol);
+                gather_rows4<BATCH, PLAIN, HOT>(p, pairs + r0 * t.row_nz, rows, t.row_nz, xc, p.y + (int64_t)(t.row0 + r0) * p.ldy, col, pol);
         } else {
             // the slots of the warp share each row
             for (int r = 0; r < t.n_rows; r++) {
-                float4 acc = gather_vec4<BATCH>(pairs + r * t.row_nz, t.row_nz, slot, NS, xc, p.ldx, active, pol.keep);
+                float4 acc = gather_vec4<BATCH, HOT>(pairs + r * t.row_nz, t.row_nz, slot, NS, xc, p.ldx, active, pol);
 #pragma unroll
                 for (int off = LANES; off < 32; off <<= 1) {
                     acc.x += __shfl_xor_sync(FULL_MASK, acc.x, off);
@@ -512,8 +517,9 @@ __device__ __forceinline__ bool tuple_is_big(const int4 &b) { return b.x > SPMM_
 __device__ __forceinline__ int tuple_rows(const int4 &b) { return tuple_is_big(b) ? 1 : (b.w & 0xffff); }
 
 // Error bits are single words of the host so that blocks can store to them without atomics.
-constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_ERR = 3;      // then one word per SPMM_ERR_* bit
+constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_FULL = 3, PLAN_WORD_ERR = 4;      // then one word per SPMM_ERR_* bit
 constexpr int PLAN_ERR_BITS = 4;
+constexpr int PLAN_FULL_NZ = 256;
 constexpr int PLAN_BLOCK = 256;      // units per thread block, one per thread
 
 __device__ __forceinline__ void plan_report(HostWords *out, int err)
@@ -608,7 +614,8 @@ __device__ __forceinline__ void plan_check_ids(const int *__restrict__ idx, int6
 // First pass over a `.block4` array: validates every tuple (and, in the blocks behind the tuple blocks,
 // every column id), and counts per PLAN_BLOCK units the rows no tuple covers and the carry slots.  One
 // launch and one read of 16 bytes per tuple and 4 per nonzero: bound by HBM for large graphs, by launch
-// latency for small ones.  ctl[0], ctl[1]: totals, ctl[2]: blocks done (zero at launch).
+// latency for small ones.  ctl[0..2]: totals (the third: tuples of at least PLAN_FULL_NZ nonzeros), ctl[3]: blocks
+// done (zero at launch).
 __global__ void __launch_bounds__(PLAN_BLOCK)
 plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int64_t n_rows, int64_t nnz,
                   const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned unit_grid,
@@ -620,10 +627,10 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
         return;
     }
     __shared__ int64_t s_zero[PLAN_BLOCK / 32];
-    __shared__ int s_carry[PLAN_BLOCK / 32];
+    __shared__ int s_carry[PLAN_BLOCK / 32], s_full[PLAN_BLOCK / 32];
     const int64_t u = (int64_t)blockIdx.x * PLAN_BLOCK + threadIdx.x;
     int64_t zero = 0;
-    int carry = 0, err = 0;
+    int carry = 0, err = 0, full = 0;
     if (u < n_units || (n_units == 0 && u == 0)) {          // without any tuple, one thread counts the rows
         const int64_t e0 = u * SPMM_WARPS;
         const int64_t e1 = e0 + SPMM_WARPS < n_blocks ? e0 + SPMM_WARPS : n_blocks;
@@ -631,6 +638,7 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
         for (int64_t e = e0; e < e1; e++) {
             const int4 b = block4[e];
             err |= tuple_errors(e > 0, a, b, n_rows, nnz);
+            full += tuple_nz(b) >= PLAN_FULL_NZ;
             const int64_t g = tuple_gap(e > 0, a, b);
             zero += g > 0 ? g : 0;
             a = b;
@@ -646,20 +654,23 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
     if (err) plan_report(out, err);
     zero = warp_reduce(zero, OpAdd());
     carry = warp_reduce(carry, OpAdd());
-    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; }
+    full = warp_reduce(full, OpAdd());
+    if (lane_id() == 0) { s_zero[warp_id()] = zero; s_carry[warp_id()] = carry; s_full[warp_id()] = full; }
     __syncthreads();
     if (threadIdx.x == 0) {
-        zero = 0; carry = 0;
-        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; }
+        zero = 0; carry = 0; full = 0;
+        for (int w = 0; w < PLAN_BLOCK / 32; w++) { zero += s_zero[w]; carry += s_carry[w]; full += s_full[w]; }
         tile_zero[blockIdx.x] = zero;
         tile_carry[blockIdx.x] = carry;
         atomicAdd(ctl + 0, (unsigned long long)zero);
         atomicAdd(ctl + 1, (unsigned long long)carry);
+        atomicAdd(ctl + 2, (unsigned long long)full);
         __threadfence();
-        if (atomicAdd(ctl + 2, 1ull) == unit_grid - 1) {
+        if (atomicAdd(ctl + 3, 1ull) == unit_grid - 1) {
             __threadfence();
             out->w[PLAN_WORD_ZERO] = (int64_t)__ldcg(ctl + 0);
             out->w[PLAN_WORD_CARRY] = (int64_t)__ldcg(ctl + 1);
+            out->w[PLAN_WORD_FULL] = (int64_t)__ldcg(ctl + 2);
         }
     }
 }

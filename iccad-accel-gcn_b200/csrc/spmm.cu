@@ -46,6 +46,24 @@ static int spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int 
     return env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count));
 }
 
+// The thread blocks of full tuples take equally long and are started first: where they fill 5 blocks per SM once but
+// 4 blocks per SM not quite twice, the second round is a tail in which most of the GPU waits (100 000 skewed rows of
+// 20, 87 tuples per SM, dim 128: 62 us at 5 blocks, 77 at 4; 150 000 rows: 126 and 105).
+static bool spmm_wide_form(const agcn_spmm_plan *p)
+{
+    const int64_t full_units = p->n_full / SPMM_WARPS;
+    return full_units > (int64_t)SPMM_MIN_BLOCKS * p->sm_count && full_units <= (int64_t)SPMM_WIDE_MIN_BLOCKS * p->sm_count;
+}
+
+// Columns whose rows of X are to stay in L2 when X is many times larger: the last ones, which in a symmetric graph in
+// degree order are named most often.  45 % of L2 (each half of the GPU keeps its own copy of what it reads).
+// 0 = all alike: below 6x L2 that is as fast or faster.  (X / L2 = 9, 14, 19 at dim 128: -3, -4, -4.5 %.)
+static int64_t spmm_hot_column(const agcn_spmm_plan *p, int width)
+{
+    if ((double)p->n_cols * width * 4.0 < 6.0 * p->l2_bytes) return 0;
+    return p->n_cols - (int64_t)(0.45 * p->l2_bytes / (width * 4.0));
+}
+
 bool spmm_plan_splits(int64_t n_blocks, int64_t n_rows, int64_t nnz)
 {
     int device = 0, sm_count = 0;
@@ -143,14 +161,14 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     const int64_t tiles = p->n_units > 0 ? ceil_div(p->n_units, PLAN_BLOCK) : 1;
     DeviceScratch scratch(s);
     Carver size;
-    size.take<unsigned long long>(3); size.take<int64_t>(tiles); size.take<int>(tiles);
+    size.take<unsigned long long>(4); size.take<int64_t>(tiles); size.take<int>(tiles);
     AGCN_ALLOC(block, scratch, unsigned char, (int64_t)size.bytes());
     Carver c(block);
-    unsigned long long *ctl = c.take<unsigned long long>(3);
+    unsigned long long *ctl = c.take<unsigned long long>(4);
     int64_t *tile_zero = c.take<int64_t>(tiles);
     int *tile_carry = c.take<int>(tiles);
     AGCN_HOST_WORDS(words, s);
-    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 3 * sizeof(*ctl), s));
+    AGCN_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(*ctl), s));
     // 16 column ids per thread, at most 64 thread blocks per SM's worth of them
     const int64_t col_grid = n_idx > 0 ? ceil_div(n_idx, PLAN_BLOCK * 16) : 0;
     const unsigned grid = (unsigned)(tiles + (col_grid < 9472 ? col_grid : 9472));
@@ -162,6 +180,7 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     if (rc != AGCN_OK) return rc;
     p->n_zero = words[PLAN_WORD_ZERO];
     p->n_carry = words[PLAN_WORD_CARRY];
+    p->n_full = words[PLAN_WORD_FULL];
     int4 *pieces = nullptr;
     rc = plan_memory(p, 0, &pieces, s);
     if (rc != AGCN_OK) return rc;
@@ -217,30 +236,47 @@ int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag
     return AGCN_OK;
 }
 
-template <int S, int BATCH, int MIN_BLOCKS, bool FINISH>
+template <int S, int BATCH, int MIN_BLOCKS, bool FINISH, bool HOT = false>
 static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaStream_t s)
 {
-    auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH>;
+    auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH, HOT> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH, HOT>;
     AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm);
 }
 
-// `small` launches (of a plan that is cut into pieces) always finish the rows that cross units themselves.
+// Which of the kernel's forms a launch uses.
+struct SpmmForm {
+    bool plain;      // Y overwritten with 16-byte stores
+    bool finish;     // rows that cross units are finished in the launch
+    bool deep;       // few thread blocks, many gathers per lane
+    bool wide;       // more thread blocks per SM, fewer gathers per lane
+};
+
 template <int S>
-static void launch_units_for(const SpmmParams &prm, unsigned grid, bool small, bool plain, bool finish, cudaStream_t s)
+static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
 {
-    if (small) launch_units<S, SPMM_SMALL_GATHER_BATCH, SPMM_SMALL_MIN_BLOCKS, true>(prm, grid, plain, s);
-    else if (finish) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, true>(prm, grid, plain, s);
-    else launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, plain, s);
+    if (f.deep) { launch_units<S, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, true>(prm, grid, f.plain, s); return; }
+    // 17..32 columns, and the 4-byte mode, always take the 5-block form
+    constexpr bool ALWAYS_WIDE = S == 8 || S == 0;
+    if (f.finish) {
+        if (ALWAYS_WIDE || f.wide) launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, true>(prm, grid, f.plain, s);
+        else if constexpr (!ALWAYS_WIDE) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, true>(prm, grid, f.plain, s);
+    } else if constexpr (ALWAYS_WIDE) {
+        launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false>(prm, grid, f.plain, s);
+    } else if constexpr (S >= 16) {
+        if (prm.hot_column > 0) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true>(prm, grid, f.plain, s);
+        else launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, f.plain, s);
+    } else {
+        launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, f.plain, s);
+    }
 }
 
-static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, unsigned grid, bool small, bool plain, bool finish,
-                                   cudaStream_t s)
+static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
 {
-    if (!vec) launch_units_for<0>(prm, grid, small, plain, finish, s);
-    else if (width <= 16) launch_units_for<4>(prm, grid, small, plain, finish, s);
-    else if (width <= 32) launch_units_for<8>(prm, grid, small, plain, finish, s);
-    else if (width <= 64) launch_units_for<16>(prm, grid, small, plain, finish, s);
-    else launch_units_for<32>(prm, grid, small, plain, finish, s);
+    if (!vec) launch_units_for<0>(prm, grid, f, s);
+    else if (width <= 16) launch_units_for<4>(prm, grid, f, s);
+    else if (width <= 32) launch_units_for<8>(prm, grid, f, s);
+    else if (width <= 64) launch_units_for<16>(prm, grid, f, s);
+    else launch_units_for<32>(prm, grid, f, s);
 }
 
 int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n_rows, cudaStream_t s)
@@ -345,6 +381,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.tuples = p->tuples; prm.n_tuples = p->n_tuples;
         prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag;
         prm.light_every = spmm_light_every(p, width);
+        prm.hot_column = (int)spmm_hot_column(p, width);
         prm.idx = d_indices; prm.val = d_vals;
         prm.x = x_use + col0; prm.ldx = ldx_use;
         prm.y = d_y + col0; prm.ldy = ldy;
@@ -363,7 +400,8 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
         const bool plain = !accumulate && (vec ? y_vec : true);
         if (grid > 0) {
-            launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, p->split, plain, carry_inside, s);
+            const SpmmForm form = {plain, carry_inside, p->split && 3 * p->n_units <= (int64_t)8 * p->sm_count, spmm_wide_form(p)};
+            launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, form, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;
         }
