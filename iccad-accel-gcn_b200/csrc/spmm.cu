@@ -49,8 +49,11 @@ static int spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int 
 // The thread blocks of full tuples take equally long and are started first: where they fill 5 blocks per SM once but
 // 4 blocks per SM not quite twice, the second round is a tail in which most of the GPU waits (100 000 skewed rows of
 // 20, 87 tuples per SM, dim 128: 62 us at 5 blocks, 77 at 4; 150 000 rows: 126 and 105).
-static bool spmm_wide_form(const agcn_spmm_plan *p)
+// Also where all tuples are full and little more than half of a slot's 32 lanes have a column (139 000 rows of 456, dims
+// 68 and 80: 2 % faster, dim 96 already 3 % slower).
+static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
 {
+    if (p->nnz >= 250 * p->n_blocks && width > 64 && width <= 80) return true;
     const int64_t full_units = p->n_full / SPMM_WARPS;
     return full_units > (int64_t)SPMM_MIN_BLOCKS * p->sm_count && full_units <= (int64_t)SPMM_WIDE_MIN_BLOCKS * p->sm_count;
 }
@@ -263,7 +266,8 @@ static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmFor
     } else if constexpr (ALWAYS_WIDE) {
         launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false>(prm, grid, f.plain, s);
     } else if constexpr (S >= 16) {
-        if (prm.hot_column > 0) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true>(prm, grid, f.plain, s);
+        if (S == 32 && f.wide) launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false>(prm, grid, f.plain, s);
+        else if (prm.hot_column > 0) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true>(prm, grid, f.plain, s);
         else launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, f.plain, s);
     } else {
         launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, f.plain, s);
@@ -400,7 +404,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
         const bool plain = !accumulate && (vec ? y_vec : true);
         if (grid > 0) {
-            const SpmmForm form = {plain, carry_inside, p->split && 3 * p->n_units <= (int64_t)8 * p->sm_count, spmm_wide_form(p)};
+            const SpmmForm form = {plain, carry_inside, p->split && 3 * p->n_units <= (int64_t)8 * p->sm_count, spmm_wide_form(p, width)};
             launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, form, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;

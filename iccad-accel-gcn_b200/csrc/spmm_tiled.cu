@@ -204,10 +204,11 @@ extern "C" int agcn_spmm_tiled_info(const agcn_spmm_tiled *plan, int *n_ranges, 
 }
 
 // How many column ranges a product of this shape should be cut into (1 = do not tile).
-// A slab of X (range columns x dim x 4 bytes) should stay in L2 next to the streams of A and Y
-// passing through: about a third of L2 per slab.  Tiling pays only while every row keeps enough
-// nonzeros per range to amortise the extra pass over Y (read + write per range after the first):
-// a mean of 48 per row and range.
+// A slab of X (range columns x dim x 4 bytes) should stay in L2 next to the streams of A and Y passing through: half
+// of L2 per slab, as much as one half of the GPU keeps of what both read.  Tiling pays only while every row keeps
+// enough nonzeros per range to amortise the extra pass over Y (read + write per range after the first): a mean of 48
+// per row and range.  (A third of L2 per slab before: 250 000 rows of 490 at dim 128 in 3 ranges 3.33 ms, in 2 3.24;
+// at dim 112 3.10 and 2.97.)
 extern "C" int agcn_spmm_tiled_suggest(int64_t n_rows, int64_t n_cols, int64_t nnz, int dim)
 {
     int dev = 0, l2 = 0;
@@ -216,7 +217,7 @@ extern "C" int agcn_spmm_tiled_suggest(int64_t n_rows, int64_t n_cols, int64_t n
     if (n_rows <= 0 || n_cols <= 0 || dim <= 0) return 1;
     const double x_bytes = (double)n_cols * dim * 4.0;
     if (x_bytes <= 0.6 * l2) return 1;
-    int k = (int)((x_bytes + 0.35 * l2 - 1.0) / (0.35 * l2));
+    int k = (int)((x_bytes + 0.5 * l2 - 1.0) / (0.5 * l2));
     if (k > agcn::TILE_MAX_RANGES) k = agcn::TILE_MAX_RANGES;
     while (k > 1 && (double)nnz / (double)n_rows / k < 48.0) k--;
     return k;
