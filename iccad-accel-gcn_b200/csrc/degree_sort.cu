@@ -139,13 +139,13 @@ extern "C" int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_i
     const HostSegment up[] = {{d_indptr, const_cast<int *>(h_indptr), row_bytes + sizeof(int)},
                               {d_indices, const_cast<int *>(h_indices), want_idx ? nz_bytes : 0},
                               {d_vals, const_cast<float *>(h_vals), want_val ? nz_bytes : 0}};
-    int rc = host_upload(up, 3, s);
-    if (rc != AGCN_OK) return rc;
-    rc = degree_sort_device(d_indptr, d_indices, d_vals, n_rows, nnz, relabel_cols, d_perm, d_new_indptr, d_new_indices, d_new_vals, s);
-    if (rc != AGCN_OK) return rc;
     const HostSegment down[] = {{d_perm, h_perm, row_bytes},
                                 {d_new_indptr, h_new_indptr, h_new_indptr != nullptr ? row_bytes + sizeof(int) : 0},
                                 {d_new_indices, h_new_indices, want_idx ? nz_bytes : 0},
                                 {d_new_vals, h_new_vals, want_val ? nz_bytes : 0}};
+    int rc = host_upload(up, 3, s, down, 4);
+    if (rc != AGCN_OK) return rc;
+    rc = degree_sort_device(d_indptr, d_indices, d_vals, n_rows, nnz, relabel_cols, d_perm, d_new_indptr, d_new_indices, d_new_vals, s);
+    if (rc != AGCN_OK) return rc;
     return host_download(down, 4, s);
 }

@@ -17,6 +17,10 @@ namespace agcn {
 
 constexpr size_t STAGE_PIECE = (size_t)1 << 20;
 constexpr int STAGE_THREADS = 12;                  // the link needs about 6 at 8-10 GB/s each; fresh pages cost as much again
+// Threads beside these that only fault in the pages of the output arrays while the upload keeps the link busy: a
+// fresh array is zeroed by the kernel page by page at its first write, which took 2 ms of 120 MB of outputs.
+constexpr int TOUCH_THREADS = 4;
+constexpr size_t TOUCH_PIECE = (size_t)2 << 20;
 constexpr size_t STAGE_MIN_BYTES = (size_t)2 << 20;    // below this, starting threads costs more than it saves
 
 // The pinned buffers: 24 MiB, made at the first use, given back by agcn_release_scratch.  One call at a time
@@ -48,8 +52,10 @@ struct StageJob {
     bool up;
     cudaStream_t stream;
     int device;
-    std::atomic<size_t> next{0};
+    std::atomic<size_t> next{0}, next_touch{0};
     std::atomic<int> error{0};
+    const HostSegment *touch;
+    int n_touch;
     size_t first[HOST_SEGMENTS_MAX + 1];           // first piece of every segment
 
     // piece i: its segment, offset and size; false past the end
@@ -62,6 +68,26 @@ struct StageJob {
         *at = (i - first[k]) * STAGE_PIECE;
         *bytes = seg[k].bytes - *at < STAGE_PIECE ? seg[k].bytes - *at : STAGE_PIECE;
         return true;
+    }
+
+    // Faults in output pages, TOUCH_PIECE at a time, until none are left.  Their contents stay: an output may be
+    // the array that is being uploaded.
+    void touch_outputs()
+    {
+        for (;;) {
+            size_t i = next_touch.fetch_add(1);
+            const HostSegment *g = nullptr;
+            for (int k = 0; k < n_touch; k++) {
+                const size_t pieces = (touch[k].bytes + TOUCH_PIECE - 1) / TOUCH_PIECE;
+                if (i < pieces) { g = &touch[k]; break; }
+                i -= pieces;
+            }
+            if (g == nullptr) return;
+            unsigned char *p = static_cast<unsigned char *>(g->host) + i * TOUCH_PIECE;
+            const size_t bytes = g->bytes - i * TOUCH_PIECE < TOUCH_PIECE ? g->bytes - i * TOUCH_PIECE : TOUCH_PIECE;
+            for (size_t at = 0; at < bytes; at += 4096) __atomic_fetch_or(p + at, (unsigned char)0, __ATOMIC_RELAXED);
+            __atomic_fetch_or(p + bytes - 1, (unsigned char)0, __ATOMIC_RELAXED);
+        }
     }
 
     void work(unsigned char *buffers)
@@ -95,7 +121,7 @@ struct StageJob {
     }
 };
 
-static int host_copy(const HostSegment *seg, int n, bool up, cudaStream_t s)
+static int host_copy(const HostSegment *seg, int n, bool up, cudaStream_t s, const HostSegment *outputs, int n_outputs)
 {
     AGCN_REQUIRE(n >= 0 && n <= HOST_SEGMENTS_MAX, "host copy: too many segments");
     HostSegment staged[HOST_SEGMENTS_MAX];
@@ -119,7 +145,11 @@ static int host_copy(const HostSegment *seg, int n, bool up, cudaStream_t s)
         for (int i = 0; i < m; i++) AGCN_CUDA(copy_plain(staged[i], up, s));
         return AGCN_OK;
     }
+    HostSegment touch[HOST_SEGMENTS_MAX];
     StageJob job;
+    job.touch = touch; job.n_touch = 0;
+    for (int i = 0; i < n_outputs && i < HOST_SEGMENTS_MAX; i++)
+        if (outputs[i].bytes > 0 && !is_pinned(outputs[i].host)) touch[job.n_touch++] = outputs[i];
     job.seg = staged; job.n = m; job.up = up; job.stream = s;
     AGCN_CUDA(cudaGetDevice(&job.device));
     job.first[0] = 0;
@@ -127,26 +157,31 @@ static int host_copy(const HostSegment *seg, int n, bool up, cudaStream_t s)
     const unsigned cores = std::thread::hardware_concurrency();
     int threads = cores > 1 ? (int)(cores < STAGE_THREADS ? cores : STAGE_THREADS) : 1;
     if ((size_t)threads > job.first[m]) threads = (int)job.first[m];
-    std::thread pool[STAGE_THREADS];
-    int started = 1;                                // the calling thread is one of them
+    std::thread pool[STAGE_THREADS], touchers[TOUCH_THREADS];
+    int started = 1, touching = 0;                  // the calling thread is one of them
     try {
+        for (; job.n_touch > 0 && cores > TOUCH_THREADS && touching < TOUCH_THREADS; touching++) touchers[touching] = std::thread([&job] { job.touch_outputs(); });
         for (; started < threads; started++)
-            pool[started] = std::thread([&job, started] { job.work(g_stage.memory + (size_t)started * 2 * STAGE_PIECE); });
+            pool[started] = std::thread([&job, started] { job.work(g_stage.memory + (size_t)started * 2 * STAGE_PIECE); job.touch_outputs(); });
     } catch (const std::system_error &) {
         // fewer threads than asked for: the ones that run share the pieces
     }
     job.work(g_stage.memory);
     for (int t = 1; t < started; t++) pool[t].join();
+    for (int t = 0; t < touching; t++) touchers[t].join();
     const cudaError_t e = (cudaError_t)job.error.load();
     AGCN_CUDA(e);
     return AGCN_OK;
 }
 
-int host_upload(const HostSegment *seg, int n, cudaStream_t s) { return host_copy(seg, n, true, s); }
+int host_upload(const HostSegment *seg, int n, cudaStream_t s, const HostSegment *outputs, int n_outputs)
+{
+    return host_copy(seg, n, true, s, outputs, n_outputs);
+}
 
 int host_download(const HostSegment *seg, int n, cudaStream_t s)
 {
-    const int rc = host_copy(seg, n, false, s);
+    const int rc = host_copy(seg, n, false, s, nullptr, 0);
     if (rc != AGCN_OK) return rc;
     AGCN_CUDA(cudaStreamSynchronize(s));
     return AGCN_OK;
