@@ -65,6 +65,7 @@ inline int *spmm_carry_counters(void *carry, int64_t n_carry) { return reinterpr
 struct SpmmLaunchPart {
     int64_t unit0 = 0, unit1 = -1;      // units [unit0, unit1); -1 = to the end
     bool zero_fill = true;
+    bool after_pad = false;             // the launch before this one on the stream is the aligned copy of X
     const int *abort_flag = nullptr;    // optional device word: nonzero makes the kernels return at once
     void *carry = nullptr;              // optional carry scratch to use instead of the plan's (products in flight together)
 };

@@ -74,5 +74,10 @@ __device__ __forceinline__ void st_y1(float *p, float v, uint64_t policy)
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" :: "l"(p), "f"(v), "l"(policy) : "memory");
 }
 
+// Programmatic dependent launch: the launch after this one may start; this one's predecessor has finished and what
+// it wrote is visible.  Both do nothing in launches without that attribute.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 }  // namespace agcn
 #endif

@@ -78,6 +78,7 @@ struct SpmmParams {
     const int *zero_rows;     // rows no tuple covers
     int64_t n_zero_rows;
     int hot_column;           // HOT kernels: rows of X from this column on are kept in L2; 0: no such choice
+    int after_pad;            // host only: launched so that it overlaps the copy of X before it
     int relu;                 // nonzero: Y = max(A * X, 0) (fused GCN activation)
     // The fields below are read only by the general (PLAIN = false) kernel flavour.
     int accumulate;           // nonzero: Y += A * X (later column ranges of a column-tiled product)
@@ -387,6 +388,7 @@ spmm_units_kernel(const SpmmParams p)
     __syncwarp();
 
     const int2 *pairs = s_pair[w];
+    wait_for_predecessor();             // X may be the copy that the launch before this one makes
 
     if (VEC) {
         const float *xc = p.x + col;
@@ -487,22 +489,40 @@ spmm_carry_kernel(const SpmmParams p, const int *__restrict__ carry_row, int64_t
 
 // X[n_rows x dim] with row stride ldx  ->  XP[n_rows x ldp], ldp = dim rounded up to 4, tail zero:
 // the 16-byte-aligned copy of a dense operand whose rows are not (dim % 4 != 0 or an unaligned base).
-// One thread per 16 bytes written.
-__global__ void __launch_bounds__(256)
+// Every thread writes PAD_ITEMS times 16 bytes; a 64-bit division for each of them was as much work as the
+// memory traffic (500 000 x 61: 40 us).  It lets the product that follows begin at once: that one waits
+// before it reads X.
+constexpr int PAD_BLOCK = 256, PAD_ITEMS = 4;
+
+__global__ void __launch_bounds__(PAD_BLOCK)
 spmm_pad_rows_kernel(const float *__restrict__ x, int64_t ldx, int dim, float *__restrict__ xp, int ldp, int64_t n_rows)
 {
-    const int quads = ldp >> 2;
-    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_rows * quads) return;
-    const int64_t row = i / quads;
-    const int c = (int)(i - row * quads) * 4;
-    const float *src = x + row * ldx + c;
-    float4 v;
-    v.x = c + 0 < dim ? __ldg(src + 0) : 0.f;
-    v.y = c + 1 < dim ? __ldg(src + 1) : 0.f;
-    v.z = c + 2 < dim ? __ldg(src + 2) : 0.f;
-    v.w = c + 3 < dim ? __ldg(src + 3) : 0.f;
-    *reinterpret_cast<float4 *>(xp + row * ldp + c) = v;
+    launch_dependents();
+    const unsigned quads = (unsigned)ldp >> 2, per_quad = ((1u << 20) + quads - 1) / quads;      // n / quads = n * per_quad >> 20 for n * quads < 2^20
+    const int64_t first = (int64_t)blockIdx.x * (PAD_BLOCK * PAD_ITEMS);
+    const int64_t row0 = first / quads;
+    const unsigned rest = (unsigned)(first - row0 * quads);
+    float4 v[PAD_ITEMS];
+#pragma unroll
+    for (int k = 0; k < PAD_ITEMS; k++) {
+        const unsigned at = rest + k * PAD_BLOCK + threadIdx.x;
+        const unsigned r = quads <= 512 ? at * per_quad >> 20 : at / quads;
+        const int64_t row = row0 + r;
+        const int c = (int)(at - r * quads) * 4;
+        v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (row < n_rows) {
+            const float *src = x + row * ldx + c;
+            if (c + 0 < dim) v[k].x = __ldg(src + 0);
+            if (c + 1 < dim) v[k].y = __ldg(src + 1);
+            if (c + 2 < dim) v[k].z = __ldg(src + 2);
+            if (c + 3 < dim) v[k].w = __ldg(src + 3);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < PAD_ITEMS; k++) {
+        const int64_t at = first + k * PAD_BLOCK + threadIdx.x;
+        if (at < n_rows * quads) *reinterpret_cast<float4 *>(xp + at * 4) = v[k];
+    }
 }
 
 // ---------------------------------------------------------------------------

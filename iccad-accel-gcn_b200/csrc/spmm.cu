@@ -243,7 +243,18 @@ template <int S, int BATCH, int MIN_BLOCKS, bool FINISH, bool HOT = false>
 static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaStream_t s)
 {
     auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH, HOT> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH, HOT>;
-    AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm);
+    if (!prm.after_pad) {
+        AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm);
+        return;
+    }
+    // behind the copy of X: reads its tuples and nonzeros while that still runs
+    cudaLaunchAttribute early = {};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(SPMM_THREADS); cfg.stream = s;
+    cfg.attrs = &early; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k, prm);
 }
 
 // Which of the kernel's forms a launch uses.
@@ -286,8 +297,9 @@ static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, u
 int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n_rows, cudaStream_t s)
 {
     const int ldp = (dim + 3) & ~3;
-    const int64_t quads = n_rows * (ldp >> 2);
-    AGCN_KERNEL(spmm_pad_rows_kernel, (unsigned)ceil_div(quads, 256), 256, s, d_x, ldx, dim, d_xp, ldp, n_rows);
+    const int64_t blocks = ceil_div(n_rows * (ldp >> 2), PAD_BLOCK * PAD_ITEMS);
+    AGCN_REQUIRE(blocks < (int64_t)INT32_MAX, "agcn_spmm_run: operand too large to pad");
+    AGCN_KERNEL(spmm_pad_rows_kernel, (unsigned)blocks, PAD_BLOCK, s, d_x, ldx, dim, d_xp, ldp, n_rows);
     AGCN_LAUNCH_CHECK("spmm_pad_rows_kernel");
     return AGCN_OK;
 }
@@ -384,6 +396,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         SpmmParams prm;
         prm.tuples = p->tuples; prm.n_tuples = p->n_tuples;
         prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag;
+        prm.after_pad = part.after_pad && col0 == 0 ? 1 : 0;
         prm.light_every = spmm_light_every(p, width);
         prm.hot_column = (int)spmm_hot_column(p, width);
         prm.idx = d_indices; prm.val = d_vals;
@@ -431,7 +444,9 @@ int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const
     bool x_vec = false;
     rc = spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
     if (rc != AGCN_OK) return rc;
-    return spmm_run_prepared(p, d_indices, d_vals, x_use, ldx_use, x_vec, d_y, ldy, dim, s, activation, accumulate, SpmmLaunchPart());
+    SpmmLaunchPart part;
+    part.after_pad = x_use != d_x;
+    return spmm_run_prepared(p, d_indices, d_vals, x_use, ldx_use, x_vec, d_y, ldy, dim, s, activation, accumulate, part);
 }
 
 }  // namespace agcn
