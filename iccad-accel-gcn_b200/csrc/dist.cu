@@ -110,6 +110,7 @@ struct agcn_gcn2 {
     float *z = nullptr, *h1 = nullptr;        // [per x 128] each
     int *d_status = nullptr;                  // status words: the GEMM of each layer, the fused kernel, the GEMM of the other rows
     cudaEvent_t ev[8] = {};
+    bool alone = false;                       // the last run exchanged nothing and used events 0, 1, 3, 5, 7 only
     // AGCN_GCN_FUSED=1: the leading rows of the block (at most 32 nonzeros each) go through one kernel
     // from layer 1's gathered operand to layer 2's operand; the other rows through SpMM and GEMM as before
     float *z2 = nullptr;                      // [per x 128]: layer 2's operand
@@ -526,6 +527,24 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
     AGCN_REQUIRE(fwd != nullptr && d_x_block != nullptr && d_out_block != nullptr, "agcn_gcn2_forward_run: null argument");
     agcn_dist *d = fwd->dist;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (d->world == 1 && d->tiled == nullptr && fwd->fused_rows == 0) {
+        // nothing is exchanged: transform and product alternate on the stream, with one event between them
+        // (the waits and events of the exchange took 8 us of a forward over 16 384 rows)
+        fwd->alone = true;
+        d->launches_last_step = 0;
+        AGCN_CUDA(cudaEventRecord(fwd->ev[0], s));
+        for (int layer = 0; layer < 2; layer++) {
+            int rc = gemm_tf32_async(layer == 0 ? d_x_block : fwd->h1, 128, fwd->w[layer], fwd->z, 128, d->per, fwd->d_status + layer, s);
+            if (rc != AGCN_OK) return rc;
+            AGCN_CUDA(cudaEventRecord(fwd->ev[4 * layer + 1], s));
+            rc = spmm_run(d->plan, d->idx, d->val, fwd->z, 128, layer == 0 ? fwd->h1 : d_out_block, 128, 128, s, AGCN_ACT_RELU, 0);
+            if (rc != AGCN_OK) return rc;
+            AGCN_CUDA(cudaEventRecord(fwd->ev[4 * layer + 3], s));
+            d->launches_last_step = d->plan->launches_last_run;
+        }
+        return AGCN_OK;
+    }
+    fwd->alone = false;
     const float *h = d_x_block;
     const bool fused = fwd->fused_rows > 0;
     for (int layer = 0; layer < 2; layer++) {
@@ -587,7 +606,13 @@ extern "C" int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6)
                   status[0] != 0 ? 1 : 2);
         return AGCN_ERR_CUDA;
     }
-    if (ms6 != nullptr)
+    if (ms6 != nullptr && fwd->alone) {
+        for (int layer = 0; layer < 2; layer++) {
+            AGCN_CUDA(cudaEventElapsedTime(&ms6[3 * layer], fwd->ev[layer == 0 ? 0 : 3], fwd->ev[4 * layer + 1]));
+            ms6[3 * layer + 1] = 0.f;
+            AGCN_CUDA(cudaEventElapsedTime(&ms6[3 * layer + 2], fwd->ev[4 * layer + 1], fwd->ev[4 * layer + 3]));
+        }
+    } else if (ms6 != nullptr)
         for (int layer = 0; layer < 2; layer++)
             for (int k = 0; k < 3; k++)
                 AGCN_CUDA(cudaEventElapsedTime(&ms6[3 * layer + k], fwd->ev[4 * layer + k], fwd->ev[4 * layer + k + 1]));

@@ -38,7 +38,7 @@ static const char *gemm_status_text(int status)
 }
 
 // Checks the arguments, encodes the tensor map of H and launches.  Nothing is allocated and the
-// stream is not synchronised; *d_status (device, zeroed here on the stream) receives a GEMM_ERR_*
+// stream is not synchronised; *d_status (device, zeroed by the kernel) receives a GEMM_ERR_*
 // code if a pipeline wait runs out.
 static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
                             int k_dim, int n_dim, int *d_status, cudaStream_t s, uint32_t spin_limit, int skip_first_load)
@@ -50,8 +50,10 @@ static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, flo
     AGCN_REQUIRE(ldh >= GEMM_DIM && ldz >= GEMM_DIM && ldh % 4 == 0 && ldz % 4 == 0,
                  "agcn_gemm_tf32: row strides must be >= 128 and multiples of 4 floats");
     AGCN_REQUIRE(aligned16(d_h) && aligned16(d_z), "agcn_gemm_tf32: H and Z must be 16-byte aligned");
-    AGCN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
-    if (m_rows == 0) return AGCN_OK;
+    if (m_rows == 0) {
+        AGCN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
+        return AGCN_OK;
+    }
 
     EncodeTiledFn encode = nullptr;
     int rc = get_encode_fn(&encode);

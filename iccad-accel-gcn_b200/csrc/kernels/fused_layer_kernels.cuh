@@ -62,14 +62,7 @@ gcn_fused_layer_kernel(const int *__restrict__ indptr, const int *__restrict__ i
         *s_abort = 0;
         fence_barrier_init();
     }
-    // W[k][n] (row-major) -> B operand: row n holds its K values, 32 per 128-byte swizzled row
-    for (int i = threadIdx.x; i < GEMM_DIM * GEMM_DIM; i += FUSED_THREADS) {
-        const int k = i / GEMM_DIM, n = i % GEMM_DIM;
-        const int chunk = ((k % GEMM_KBLK) >> 2) ^ (n & 7);
-        const uint32_t off = (uint32_t)(k / GEMM_KBLK) * GEMM_STAGE_BYTES + (uint32_t)n * 128u + (uint32_t)chunk * 16u +
-                             (uint32_t)(k & 3) * 4u;
-        *reinterpret_cast<float *>(s_w + off) = w[i];
-    }
+    gemm_load_w<FUSED_THREADS>(w, s_w, threadIdx.x);
     fence_proxy_async();
     if (warp == 1) tmem_alloc(smem_u32(s_tmem_base), GEMM_TMEM_COLS);
     tc_fence_before();

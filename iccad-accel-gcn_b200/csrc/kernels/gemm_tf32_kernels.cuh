@@ -146,6 +146,32 @@ constexpr uint32_t GEMM_IDESC = (1u << 4)                 /* D format: f32 */
                               | ((uint32_t)(GEMM_DIM >> 3) << 17)      /* N / 8 */
                               | ((uint32_t)(GEMM_TILE_M >> 4) << 24);  /* M / 16 */
 
+// W[k][n] (row-major) -> B operand: row n holds its K values, 32 per 128-byte swizzled row.  A warp takes 8
+// consecutive n of 4 consecutive k at a time: 32 different banks, whole sectors.  (Lanes along n alone met on 8
+// banks and every load was waited for: 10 us of a 16 us product of 16 384 rows.)
+template <int THREADS>
+__device__ __forceinline__ void gemm_load_w(const float *__restrict__ w, uint8_t *s_w, int t)
+{
+    constexpr int BATCH = 16;
+    constexpr int WARPS = THREADS / 32;
+    const int lane = t & 31;
+    for (int i0 = t >> 5; i0 < GEMM_DIM * GEMM_DIM / 32; i0 += WARPS * BATCH) {
+        float v[BATCH];
+#pragma unroll
+        for (int u = 0; u < BATCH; u++) {
+            const int i = i0 + u * WARPS, k = (i >> 4) * 4 + (lane >> 3), n = (i & 15) * 8 + (lane & 7);
+            v[u] = i < GEMM_DIM * GEMM_DIM / 32 ? __ldg(w + k * GEMM_DIM + n) : 0.f;
+        }
+#pragma unroll
+        for (int u = 0; u < BATCH; u++) {
+            const int i = i0 + u * WARPS, k = (i >> 4) * 4 + (lane >> 3), n = (i & 15) * 8 + (lane & 7);
+            const int chunk = ((k % GEMM_KBLK) >> 2) ^ (n & 7);
+            const uint32_t off = (uint32_t)(k / GEMM_KBLK) * GEMM_STAGE_BYTES + (uint32_t)n * 128u + (uint32_t)chunk * 16u + (uint32_t)(k & 3) * 4u;
+            if (i < GEMM_DIM * GEMM_DIM / 32) *reinterpret_cast<float *>(s_w + off) = v[u];
+        }
+    }
+}
+
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__restrict__ w,
                      float *__restrict__ z, int64_t ldz, int64_t m_rows, int n_tiles, int *__restrict__ err_flag,
@@ -178,20 +204,19 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
         *s_never = 0;
         fence_barrier_init();
     }
-    // W[k][n] (row-major) -> B operand: row n holds its K values, 32 per 128-byte swizzled row
-    for (int i = threadIdx.x; i < GEMM_DIM * GEMM_DIM; i += GEMM_THREADS) {
-        const int k = i / GEMM_DIM, n = i % GEMM_DIM;
-        const int chunk = ((k % GEMM_KBLK) >> 2) ^ (n & 7);
-        const uint32_t off = (uint32_t)(k / GEMM_KBLK) * GEMM_STAGE_BYTES + (uint32_t)n * 128u + (uint32_t)chunk * 16u +
-                             (uint32_t)(k & 3) * 4u;
-        *reinterpret_cast<float *>(s_w + off) = w[i];
-    }
-    fence_proxy_async();                 // generic-proxy writes of W must be visible to the tensor core's reads
+    // (a memset of its own cost 2 us; nobody else writes the word for the thousands of polls a wait takes at least)
+    if (blockIdx.x == 0 && threadIdx.x == 0) *err_flag = 0;
     if (warp == 1) tmem_alloc(smem_u32(s_tmem_base), GEMM_TMEM_COLS);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *s_tmem_base;
+    if (warp != 0) {
+        // while the producer's first loads are under way
+        gemm_load_w<GEMM_THREADS - 32>(w, s_w, threadIdx.x - 32);
+        fence_proxy_async();             // generic-proxy writes of W must be visible to the tensor core's reads
+        asm volatile("bar.sync 1, %0;" :: "n"(GEMM_THREADS - 32) : "memory");
+    }
 
     const int my_tiles = n_tiles > (int)blockIdx.x ? (n_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
 
