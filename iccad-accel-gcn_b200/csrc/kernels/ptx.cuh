@@ -69,6 +69,10 @@ __device__ __forceinline__ void st_y4(float *p, const float4 &v, uint64_t policy
     asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
                  :: "l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(policy) : "memory");
 }
+__device__ __forceinline__ void st_y2(float *p, float a, float b, uint64_t policy)
+{
+    asm volatile("st.global.L2::cache_hint.v2.f32 [%0], {%1, %2}, %3;" :: "l"(p), "f"(a), "f"(b), "l"(policy) : "memory");
+}
 __device__ __forceinline__ void st_y1(float *p, float v, uint64_t policy)
 {
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" :: "l"(p), "f"(v), "l"(policy) : "memory");

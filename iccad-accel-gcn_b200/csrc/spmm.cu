@@ -46,16 +46,16 @@ static int spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int 
     return env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count));
 }
 
-// The thread blocks of full tuples take equally long and are started first: where they fill 5 blocks per SM once but
-// 4 blocks per SM not quite twice, the second round is a tail in which most of the GPU waits (100 000 skewed rows of
-// 20, 87 tuples per SM, dim 128: 62 us at 5 blocks, 77 at 4; 150 000 rows: 126 and 105).
+// The thread blocks of (half) full tuples take about equally long and are started first.  Where there are a few more
+// than 4 blocks per SM hold at once, the second round is a tail in which most of the GPU waits, and 5 blocks per SM
+// avoid it: dim 128, skewed rows, full blocks per SM and us at 4 / 5 blocks: 3.7: 52 / 57, 4.0: 78 / 63, 4.3: 79 / 63,
+// 4.5: 91 / 70, 4.9: 87 / 84, 5.1: 96 / 106, 6.1: 105 / 127.
 // Also where all tuples are full and little more than half of a slot's 32 lanes have a column (139 000 rows of 456, dims
 // 68 and 80: 2 % faster, dim 96 already 3 % slower).
 static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
 {
     if (p->nnz >= 250 * p->n_blocks && width > 64 && width <= 80) return true;
-    const int64_t full_units = p->n_full / SPMM_WARPS;
-    return full_units > (int64_t)SPMM_MIN_BLOCKS * p->sm_count && full_units <= (int64_t)SPMM_WIDE_MIN_BLOCKS * p->sm_count;
+    return p->n_full > (int64_t)SPMM_MIN_BLOCKS * SPMM_WARPS * p->sm_count && 10 * p->n_full <= (int64_t)49 * SPMM_WARPS * p->sm_count;
 }
 
 // Columns whose rows of X are to stay in L2 when X is many times larger: the last ones, which in a symmetric graph in
