@@ -110,7 +110,8 @@ struct agcn_gcn2 {
     float *z = nullptr, *h1 = nullptr;        // [per x 128] each
     int *d_status = nullptr;                  // status words: the GEMM of each layer, the fused kernel, the GEMM of the other rows
     cudaEvent_t ev[8] = {};
-    bool alone = false;                       // the last run exchanged nothing and used events 0, 1, 3, 5, 7 only
+    unsigned long long *d_stamps = nullptr;   // begin and end of the two transforms (ns), of a run that exchanged nothing
+    bool alone = false;                       // ... as the last one did: its events are 0 and 7
     // AGCN_GCN_FUSED=1: the leading rows of the block (at most 32 nonzeros each) go through one kernel
     // from layer 1's gathered operand to layer 2's operand; the other rows through SpMM and GEMM as before
     float *z2 = nullptr;                      // [per x 128]: layer 2's operand
@@ -351,7 +352,7 @@ static int dist_spmm_on_gathered(agcn_dist *d, const float *d_gathered, float *d
 static void gcn2_free(agcn_gcn2 *f)
 {
     if (f == nullptr) return;
-    cudaFree(f->z); cudaFree(f->h1); cudaFree(f->z2); cudaFree(f->d_status);
+    cudaFree(f->z); cudaFree(f->h1); cudaFree(f->z2); cudaFree(f->d_status); cudaFree(f->d_stamps);
     for (cudaEvent_t e : f->ev) if (e) cudaEventDestroy(e);
     delete f;
 }
@@ -487,6 +488,7 @@ extern "C" int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const 
     AGCN_CUDA(cudaMalloc(&f->z, bytes));
     AGCN_CUDA(cudaMalloc(&f->h1, bytes));
     AGCN_CUDA(cudaMalloc(&f->d_status, 4 * sizeof(int)));
+    AGCN_CUDA(cudaMalloc(&f->d_stamps, 4 * sizeof(unsigned long long)));
     AGCN_CUDA(cudaMemset(f->d_status, 0, 4 * sizeof(int)));
     for (cudaEvent_t &e : f->ev) AGCN_CUDA(cudaEventCreate(&e));
     if (env_int("AGCN_GCN_FUSED", 0) != 0 && dist->plan != nullptr && dist->per > 0 && dist->n_blocks > 0 && !dist->plan->split) {
@@ -528,20 +530,28 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
     agcn_dist *d = fwd->dist;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (d->world == 1 && d->tiled == nullptr && fwd->fused_rows == 0) {
-        // nothing is exchanged: transform and product alternate on the stream, with one event between them
-        // (the waits and events of the exchange took 8 us of a forward over 16 384 rows)
+        // Nothing is exchanged: transform and product alternate on the stream, each starting while the one before it
+        // ends.  The transforms note their own times: events between the kernels keep them apart (13 us of a forward
+        // over 16 384 rows).  (A product does not start before the transform's end: thread blocks that wait for it on SMs
+        // taken by the transform spread the heavy rows unevenly, 2 % of a forward over 5 M rows.)
         fwd->alone = true;
-        d->launches_last_step = 0;
+        const DeviceOf on(d->plan->device);
         AGCN_CUDA(cudaEventRecord(fwd->ev[0], s));
         for (int layer = 0; layer < 2; layer++) {
-            int rc = gemm_tf32_async(layer == 0 ? d_x_block : fwd->h1, 128, fwd->w[layer], fwd->z, 128, d->per, fwd->d_status + layer, s);
+            int rc = gemm_tf32_async(layer == 0 ? d_x_block : fwd->h1, 128, fwd->w[layer], fwd->z, 128, d->per, fwd->d_status + layer, s,
+                                     layer == 1, fwd->d_stamps + 2 * layer);
             if (rc != AGCN_OK) return rc;
-            AGCN_CUDA(cudaEventRecord(fwd->ev[4 * layer + 1], s));
-            rc = spmm_run(d->plan, d->idx, d->val, fwd->z, 128, layer == 0 ? fwd->h1 : d_out_block, 128, 128, s, AGCN_ACT_RELU, 0);
+            float *out = layer == 0 ? fwd->h1 : d_out_block;
+            rc = spmm_check_run_args(d->plan, d->idx, d->val, fwd->z, 128, out, 128, 128, AGCN_ACT_RELU);
             if (rc != AGCN_OK) return rc;
-            AGCN_CUDA(cudaEventRecord(fwd->ev[4 * layer + 3], s));
+            SpmmLaunchPart part;
+            part.early = d->per > 0;
+            d->plan->launches_last_run = 0;
+            rc = spmm_run_prepared(d->plan, d->idx, d->val, fwd->z, 128, true, out, 128, 128, s, AGCN_ACT_RELU, 0, part);
+            if (rc != AGCN_OK) return rc;
             d->launches_last_step = d->plan->launches_last_run;
         }
+        AGCN_CUDA(cudaEventRecord(fwd->ev[7], s));
         return AGCN_OK;
     }
     fwd->alone = false;
@@ -607,11 +617,15 @@ extern "C" int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6)
         return AGCN_ERR_CUDA;
     }
     if (ms6 != nullptr && fwd->alone) {
-        for (int layer = 0; layer < 2; layer++) {
-            AGCN_CUDA(cudaEventElapsedTime(&ms6[3 * layer], fwd->ev[layer == 0 ? 0 : 3], fwd->ev[4 * layer + 1]));
-            ms6[3 * layer + 1] = 0.f;
-            AGCN_CUDA(cudaEventElapsedTime(&ms6[3 * layer + 2], fwd->ev[4 * layer + 1], fwd->ev[4 * layer + 3]));
-        }
+        unsigned long long t[4];
+        float total = 0.f;
+        AGCN_CUDA(cudaMemcpy(t, fwd->d_stamps, sizeof(t), cudaMemcpyDeviceToHost));
+        AGCN_CUDA(cudaEventElapsedTime(&total, fwd->ev[0], fwd->ev[7]));
+        ms6[0] = (float)(t[1] - t[0]) * 1e-6f;
+        ms6[1] = ms6[4] = 0.f;
+        ms6[2] = (float)(t[2] - t[1]) * 1e-6f;
+        ms6[3] = (float)(t[3] - t[2]) * 1e-6f;
+        ms6[5] = total - (float)(t[3] - t[0]) * 1e-6f;
     } else if (ms6 != nullptr)
         for (int layer = 0; layer < 2; layer++)
             for (int k = 0; k < 3; k++)

@@ -41,7 +41,8 @@ static const char *gemm_status_text(int status)
 // stream is not synchronised; *d_status (device, zeroed by the kernel) receives a GEMM_ERR_*
 // code if a pipeline wait runs out.
 static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
-                            int k_dim, int n_dim, int *d_status, cudaStream_t s, uint32_t spin_limit, int skip_first_load)
+                            int k_dim, int n_dim, int *d_status, cudaStream_t s, uint32_t spin_limit, int skip_first_load,
+                            bool early = false, unsigned long long *d_stamp = nullptr)
 {
     AGCN_REQUIRE(d_h != nullptr && d_w != nullptr && d_z != nullptr && d_status != nullptr, "agcn_gemm_tf32: null pointer");
     AGCN_REQUIRE(k_dim == GEMM_DIM && n_dim == GEMM_DIM,
@@ -84,8 +85,8 @@ static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, flo
     }
     const int n_tiles = (int)ceil_div(m_rows, GEMM_TILE_M);
     const int grid = n_tiles < sm_count_of[dev] ? n_tiles : sm_count_of[dev];
-    gemm_tf32_128_kernel<<<grid, GEMM_THREADS, GEMM_SMEM_BYTES, s>>>(map, d_w, d_z, ldz, m_rows, n_tiles, d_status, spin_limit,
-                                                                      skip_first_load);
+    AGCN_CUDA(launch_early(early, gemm_tf32_128_kernel, (unsigned)grid, GEMM_THREADS, GEMM_SMEM_BYTES, s, map, d_w, d_z, ldz, m_rows, n_tiles, d_status,
+                           spin_limit, skip_first_load, d_stamp));
     AGCN_LAUNCH_CHECK("gemm_tf32_128_kernel");
     return AGCN_OK;
 }
@@ -123,9 +124,9 @@ static int gemm_tf32_sync(const float *d_h, int64_t ldh, const float *d_w, float
 }
 
 int gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
-                    int *d_status, cudaStream_t s)
+                    int *d_status, cudaStream_t s, bool early, unsigned long long *d_stamp)
 {
-    return gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, GEMM_DIM, GEMM_DIM, d_status, s, GEMM_SPIN_LIMIT, 0);
+    return gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, GEMM_DIM, GEMM_DIM, d_status, s, GEMM_SPIN_LIMIT, 0, early, d_stamp);
 }
 
 }  // namespace agcn

@@ -42,6 +42,20 @@ void clear_error();
         if (!(cond)) { ::agcn::set_error(__VA_ARGS__); return AGCN_ERR_INVALID; }                \
     } while (0)
 
+// Kernel launch that, if `early`, may start while the launch before it on the stream still runs (the kernel waits
+// for that one itself before it uses what it makes).
+template <typename... Params, typename... Args>
+inline cudaError_t launch_early(bool early, void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, Args... args)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(block); cfg.dynamicSmemBytes = smem; cfg.stream = s;
+    cfg.attrs = &attr; cfg.numAttrs = early ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // Makes a device current for a scope; nothing is done where it already is.
 class DeviceOf {
 public:

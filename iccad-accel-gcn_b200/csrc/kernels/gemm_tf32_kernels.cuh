@@ -24,6 +24,8 @@
 #include <cuda.h>
 #include <stdint.h>
 
+#include "ptx.cuh"
+
 namespace agcn {
 
 constexpr int GEMM_DIM = 128;                 // K and N of the product
@@ -175,8 +177,9 @@ __device__ __forceinline__ void gemm_load_w(const float *__restrict__ w, uint8_t
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__restrict__ w,
                      float *__restrict__ z, int64_t ldz, int64_t m_rows, int n_tiles, int *__restrict__ err_flag,
-                     uint32_t spin_limit, int skip_first_load)
+                     uint32_t spin_limit, int skip_first_load, unsigned long long *stamp)
 {
+    // stamp: null, or where the times (ns) of the first load and of the last thread block's end go.
     // spin_limit: polls a wait may take (GEMM_SPIN_LIMIT in normal use).  skip_first_load: self-test
     // of the failure path only -- the producer leaves out the first load of the thread block, so the
     // MMA issuer's wait for it runs out and the kernel must leave through the abort path.
@@ -205,7 +208,10 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
         fence_barrier_init();
     }
     // (a memset of its own cost 2 us; nobody else writes the word for the thousands of polls a wait takes at least)
-    if (blockIdx.x == 0 && threadIdx.x == 0) *err_flag = 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        *err_flag = 0;
+        if (stamp != nullptr) stamp[1] = 0;
+    }
     if (warp == 1) tmem_alloc(smem_u32(s_tmem_base), GEMM_TMEM_COLS);
     tc_fence_before();
     __syncthreads();
@@ -224,6 +230,8 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
         // ---- TMA producer ---------------------------------------------------------------------
         if (lane == 0) {
             uint32_t g = 0;      // K-blocks issued so far
+            wait_for_predecessor();          // H may be what the launch before this one makes
+            if (stamp != nullptr && blockIdx.x == 0) stamp[0] = global_time_ns();
             for (int it = 0; it < my_tiles && !*s_abort; it++) {
                 const int tile = (int)blockIdx.x + it * (int)gridDim.x;
                 for (int kb = 0; kb < GEMM_KBLKS; kb++, g++) {
@@ -320,6 +328,7 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
     // ---- teardown: everyone is done (or gave up); free the tensor memory ------------------------
     tc_fence_before();
     __syncthreads();
+    if (stamp != nullptr && threadIdx.x == 0) atomicMax(stamp + 1, global_time_ns());
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, GEMM_TMEM_COLS);

@@ -78,6 +78,13 @@ __device__ __forceinline__ void st_y1(float *p, float v, uint64_t policy)
     asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" :: "l"(p), "f"(v), "l"(policy) : "memory");
 }
 
+__device__ __forceinline__ unsigned long long global_time_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    return t;
+}
+
 // Programmatic dependent launch: the launch after this one may start; this one's predecessor has finished and what
 // it wrote is visible.  Both do nothing in launches without that attribute.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

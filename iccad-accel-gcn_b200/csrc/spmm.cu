@@ -243,18 +243,7 @@ template <int S, int BATCH, int MIN_BLOCKS, bool FINISH, bool HOT = false>
 static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaStream_t s)
 {
     auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH, HOT> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH, HOT>;
-    if (!prm.after_pad) {
-        AGCN_KERNEL(k, grid, SPMM_THREADS, s, prm);
-        return;
-    }
-    // behind the copy of X: reads its tuples and nonzeros while that still runs
-    cudaLaunchAttribute early = {};
-    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    early.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid); cfg.blockDim = dim3(SPMM_THREADS); cfg.stream = s;
-    cfg.attrs = &early; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k, prm);
+    launch_early(prm.early != 0, k, grid, SPMM_THREADS, 0, s, prm);
 }
 
 // Which of the kernel's forms a launch uses.
@@ -396,7 +385,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         SpmmParams prm;
         prm.tuples = p->tuples; prm.n_tuples = p->n_tuples;
         prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag;
-        prm.after_pad = part.after_pad && col0 == 0 ? 1 : 0;
+        prm.early = part.early && col0 == 0 ? 1 : 0;
         prm.light_every = spmm_light_every(p, width);
         prm.hot_column = (int)spmm_hot_column(p, width);
         prm.idx = d_indices; prm.val = d_vals;
@@ -445,7 +434,7 @@ int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const
     rc = spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
     if (rc != AGCN_OK) return rc;
     SpmmLaunchPart part;
-    part.after_pad = x_use != d_x;
+    part.early = x_use != d_x;          // behind the copy of X
     return spmm_run_prepared(p, d_indices, d_vals, x_use, ldx_use, x_vec, d_y, ldy, dim, s, activation, accumulate, part);
 }
 
