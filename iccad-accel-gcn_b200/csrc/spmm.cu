@@ -27,16 +27,23 @@ void plan_free(agcn_spmm_plan *p)
 }
 
 // Nonzeros per piece when the tuples of a plan are to be cut into pieces, 0 when they are not.  A product ends with
-// its longest warp, so pieces are as small as they can be while the GPU still takes them in little more than one
-// wave (it holds 32 to 40 warps per SM); cutting in half pays up to about two waves, beyond that the extra warps
-// cost more than they balance.  us per product, uncut / cut, B200: 16 384 rows of 8 nonzeros (10 tuples per SM),
-// dim 60: 17.7 / 9.2, dim 128: 31 / 11; 40 000 rows of 10 (26), dim 128: 34 / 18; 100 000 rows of 8 (63), dim 128:
-// 50 / 33 -- but 100 000 rows of 25 (86), dim 32: 25 / 33.
+// its longest warp, so pieces are as small as the nonzeros that an SM has to go through allow; beyond 7 500 of them
+// (20 full tuples; the SM holds 32 to 40 warps) the extra warps cost more than they balance, unless there are few
+// tuples for them.  us per product, uncut / 192 / 128 / 64, B200, nonzeros per SM in brackets:
+// 16 384 rows of 8 [900], dim 60: 17.7 / 9.4 / 8.3 / 7.3;  80 000 rows of 4 [2 100], dim 64: - / 12.4 / 11.2 / 10.3;
+// 80 000 of 7 [3 900]: - / 15.1 / 13.5 / 15.2, dim 128: - / 25 / 23 / 25;  135 000 of 4 [3 400]: 50 / 34 / 31 / -;
+// 165 000 of 6 [6 300], dim 32: 17.4 / 13.4 / 14.2 / -, dim 128: 54 / 45 / 47 / -;  200 000 of 6 [7 700], dim 64:
+// 29.2 / 30.0 / 31.4 / -;  100 000 of 25 [17 000], dim 32: 25 / 33 / - / -.
+// Beyond 80 tuples per SM one thread block takes so long to cut them that a plan used once loses (150 000 rows of 5:
+// 236 -> 244 us from the graph to Y).
 static int spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
 {
-    for (int most : {64, 96, 128, 192})
-        if (n_blocks + nnz / most - nnz / SPMM_DEG_BOUND <= (int64_t)(most < 192 ? 48 : 80) * sm_count) return most;
-    return 0;
+    const int64_t per_sm = nnz / sm_count;
+    if (n_blocks > (int64_t)80 * sm_count) return 0;
+    if (per_sm <= 1900) return 64;
+    if (per_sm <= 2700) return 96;
+    if (per_sm <= 4000) return 128;
+    return per_sm <= 7500 || n_blocks + nnz / SPMM_DEG_BOUND <= (int64_t)80 * sm_count ? 192 : 0;
 }
 
 // A cut plan keeps room for a list of all rows: not where there are a great many without any nonzero.
