@@ -43,7 +43,7 @@ const char *agcn_last_error(void);
 int agcn_version(void);
 
 /* Scratch memory comes from a stream-ordered pool of the library, one per device, which keeps at most
- * 512 MB between calls.  This returns what the current device's pool keeps (it waits for the device). */
+ * 2 GB between calls.  This returns what the current device's pool keeps (it waits for the device). */
 int agcn_release_scratch(void);
 
 /* ------------------------------------------------------------------------
