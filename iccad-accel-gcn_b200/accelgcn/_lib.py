@@ -7,6 +7,7 @@ or fails to load, importing a function from here raises.
 from __future__ import annotations
 
 import ctypes
+import functools
 import importlib.machinery
 import importlib.util
 import os
@@ -127,6 +128,7 @@ def call():
     return _call
 
 
+@functools.lru_cache(maxsize=None)
 def address(name: str) -> int:
     """Address of a library function, for `call`."""
     return ctypes.cast(getattr(load(), name), ctypes.c_void_p).value

@@ -69,10 +69,10 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
         AGCN_LAUNCH_CHECK("sort_finish_kernel");
     }
     if (permute_tiles > 0) {
-        AGCN_KERNEL(csr_permute_kernel, (unsigned)permute_tiles, PERMUTE_BLOCK, s, d_indptr, d_indices,
-                    d_new_vals != nullptr ? d_vals : (const float *)nullptr, (const int *)d_perm, (const int *)d_new_indptr,
-                    (const int *)new_id, (const int *)tile_row, n_rows, nnz, d_new_indices, d_new_vals, (const SortControl *)ctl,
-                    words.device());
+        AGCN_CUDA(launch_early(true, csr_permute_kernel, (unsigned)permute_tiles, PERMUTE_BLOCK, 0, s, d_indptr, d_indices,
+                               d_new_vals != nullptr ? d_vals : (const float *)nullptr, (const int *)d_perm, (const int *)d_new_indptr,
+                               (const int *)new_id, (const int *)tile_row, n_rows, nnz, d_new_indices, d_new_vals, (const SortControl *)ctl,
+                               words.device()));
         AGCN_LAUNCH_CHECK("csr_permute_kernel");
     }
     AGCN_CUDA(words.sync());

@@ -15,6 +15,7 @@
 #pragma once
 #include "../host_common.h"
 #include "primitives.cuh"
+#include "ptx.cuh"
 
 #include <cooperative_groups.h>
 
@@ -332,6 +333,7 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
 {
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
+    launch_dependents();         // the permute takes its place on the SMs that this leaves idle
     extern __shared__ unsigned s_small[];
     unsigned *s_key = s_small;
     int *s_row = reinterpret_cast<int *>(s_small + SMALL_BLOCK * SMALL_ITEMS);
@@ -469,16 +471,17 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
 // Bound by the 4-byte lookups (a 32-byte sector of L2 each) and HBM.
 __global__ void __launch_bounds__(PERMUTE_BLOCK)
 csr_permute_kernel(const int *__restrict__ old_indptr, const int *__restrict__ old_indices,
-                   const float *__restrict__ old_vals, const int *__restrict__ perm,
-                   const int *__restrict__ new_indptr, const int *__restrict__ new_id, const int *__restrict__ tile_row,
-                   int64_t n_rows, int64_t nnz, int *__restrict__ new_indices, float *__restrict__ new_vals,
-                   const SortControl *__restrict__ ctl, HostWords *out)
+                   const float *__restrict__ old_vals, const int *perm, const int *new_indptr, const int *new_id,
+                   const int *tile_row, int64_t n_rows, int64_t nnz, int *__restrict__ new_indices, float *__restrict__ new_vals,
+                   const SortControl *ctl, HostWords *out)
 {
+    // (what the sort makes is not __restrict__: no load of it may move above the wait)
     constexpr int WORDS = PERMUTE_TILE / 32;
     __shared__ int s_delta[PERMUTE_TILE + 1];     // per row of the tile: old start - new start
     __shared__ unsigned s_bits[WORDS];
     __shared__ int s_rank[WORDS];                 // marks before a word
     static_assert(WORDS <= PERMUTE_BLOCK && WORDS == 64, "one warp scans the words, two per lane");
+    wait_for_predecessor();      // launched early: the order of the rows is there
     if (ctl->bad != 0) return;
     const int64_t p0 = (int64_t)blockIdx.x * PERMUTE_TILE;
     const int count = (int)(nnz - p0 < PERMUTE_TILE ? nnz - p0 : PERMUTE_TILE);

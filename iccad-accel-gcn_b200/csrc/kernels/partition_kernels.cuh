@@ -21,6 +21,7 @@
 #pragma once
 #include "../host_common.h"
 #include "primitives.cuh"
+#include "ptx.cuh"
 
 namespace agcn {
 
@@ -150,6 +151,7 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
     __shared__ int s_ip[PART_SMEM_INTS];
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
     __shared__ int s_red[4][PART_BLOCK / 32];
+    launch_dependents();
     const PartTile t = part_load_tile(indptr, n_rows, s_ip);
     int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
     unsigned heads;
@@ -228,7 +230,7 @@ constexpr int PART_DIRECT_TILES = PART_BLOCK;      // half a million rows
 // the last one reports the total.  Nothing is written outside `cap` tuples (a
 // decreasing indptr, found by (A), may give any position here).
 __global__ void __launch_bounds__(PART_BLOCK)
-part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileInfo *__restrict__ info,
+part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileInfo *info,      // not __restrict__: read after the wait
                  const int *__restrict__ tile_incoming_head, const int64_t *__restrict__ tile_offset, int64_t cap,
                  int4 *__restrict__ block4, HostWords *report)
 {
@@ -240,6 +242,8 @@ part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileI
     __shared__ int s_heavy_row[PART_HEAVY_QUEUE], s_heavy_deg[PART_HEAVY_QUEUE], s_heavy_loc[PART_HEAVY_QUEUE];
     __shared__ int64_t s_heavy_out[PART_HEAVY_QUEUE];
     if (threadIdx.x == 0) s_heavy_n = 0;
+    const PartTile t = part_load_tile(indptr, n_rows, s_ip);      // synchronises the block
+    wait_for_predecessor();      // launched early behind (A), which has nothing to do with indptr but read it
     int incoming;
     int64_t first_out;
     if (tile_offset != nullptr) {
@@ -258,9 +262,9 @@ part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileI
         __syncthreads();
         incoming = s_scan[0];
         first_out = s_scan64[0];
+        __syncthreads();         // s_scan is used again
         if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) report->w[PART_WORD_TOTAL] = total;
     }
-    const PartTile t = part_load_tile(indptr, n_rows, s_ip);      // synchronises the block
     int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
     unsigned heads;
     bool negative;

@@ -73,8 +73,8 @@ static int partition_direct(const char *who, const int *d_indptr, int64_t n_rows
     AGCN_HOST_WORDS(words, s);
     AGCN_KERNEL(part_describe_kernel, tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words.device());
     AGCN_LAUNCH_CHECK("part_describe_kernel");
-    AGCN_KERNEL(part_emit_kernel, tiles, PART_BLOCK, s, d_indptr, n_rows, (const PartTileInfo *)sc.info, (const int *)nullptr,
-                (const int64_t *)nullptr, cap, tuples, words.device());
+    AGCN_CUDA(launch_early(true, part_emit_kernel, tiles, PART_BLOCK, 0, s, d_indptr, n_rows, (const PartTileInfo *)sc.info, (const int *)nullptr,
+                           (const int64_t *)nullptr, cap, tuples, words.device()));
     AGCN_LAUNCH_CHECK("part_emit_kernel");
     return partition_answer(who, words, n_blocks);
 }
