@@ -60,12 +60,12 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
         AGCN_KERNEL(degree_count_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, nnz, permute ? 1 : 0, ctl, words.device());
         AGCN_LAUNCH_CHECK("degree_count_kernel");
         for (int pass = 0; pass < passes; pass++) {
-            AGCN_KERNEL(radix_pass_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, pass, buf, ctl, state + pass * tiles * RADIX_BINS,
-                        words.device());
+            AGCN_CUDA(launch_early(true, radix_pass_kernel, (unsigned)tiles, SORT_BLOCK, 0, s, d_indptr, n_rows, pass, buf, ctl,
+                                   state + pass * tiles * RADIX_BINS, words.device()));
             AGCN_LAUNCH_CHECK("radix_pass_kernel");
         }
-        AGCN_KERNEL(sort_finish_kernel, (unsigned)final_tiles, SORT_BLOCK, s, n_rows, passes, buf, ctl, final_state, d_perm, d_new_indptr,
-                    new_id, tile_row, words.device());
+        AGCN_CUDA(launch_early(true, sort_finish_kernel, (unsigned)final_tiles, SORT_BLOCK, 0, s, n_rows, passes, buf, ctl, final_state, d_perm,
+                               d_new_indptr, new_id, tile_row, words.device()));
         AGCN_LAUNCH_CHECK("sort_finish_kernel");
     }
     if (permute_tiles > 0) {

@@ -94,6 +94,7 @@ __global__ void __launch_bounds__(SORT_BLOCK)
 degree_count_kernel(const int *__restrict__ indptr, int64_t n_rows, int64_t nnz, int check_nnz, SortControl *__restrict__ ctl, HostWords *out)
 {
     __shared__ unsigned s_hist[RADIX_PASSES][RADIX_BINS];
+    launch_dependents();
     for (int b = threadIdx.x; b < RADIX_PASSES * RADIX_BINS; b += SORT_BLOCK) (&s_hist[0][0])[b] = 0;
     __syncthreads();
     const int64_t base = (int64_t)blockIdx.x * SORT_TILE;
@@ -159,6 +160,8 @@ radix_pass_kernel(const int *__restrict__ indptr, int64_t n, int pass, SortBuffe
     __shared__ unsigned s_scan[SORT_WARPS + 1];
     __shared__ unsigned s_first[RADIX_BINS];
     __shared__ unsigned s_tile;
+    wait_for_predecessor();      // every kernel of the sort is launched early behind the one before it
+    launch_dependents();
     if (pass > 0 && ctl->hist[pass][0] == (unsigned)n) return;     // every digit is zero: nothing moves
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctl->next_tile[pass], 1u);
     for (int b = threadIdx.x; b < SORT_WARPS * RADIX_BINS / 2; b += SORT_BLOCK) reinterpret_cast<unsigned *>(&s_count[0][0])[b] = 0;
@@ -259,6 +262,8 @@ sort_finish_kernel(int64_t n, int passes, SortBuffers buf, SortControl *__restri
     __shared__ int64_t s_deg[FINAL_TILE + FINAL_TILE / 32];
     __shared__ unsigned s_tile;
     __shared__ unsigned long long s_before;
+    wait_for_predecessor();
+    launch_dependents();
     if (threadIdx.x == 0) s_tile = atomicAdd(&ctl->next_tile[RADIX_PASSES], 1u);
     __syncthreads();
     const int64_t tile = s_tile, base = tile * FINAL_TILE;

@@ -194,11 +194,12 @@ __device__ __forceinline__ int64_t part_lead_tuples(const PartTileInfo &info, in
 constexpr int PART_SCAN_BLOCK = 1024;
 
 __global__ void __launch_bounds__(PART_SCAN_BLOCK)
-part_scan_kernel(const PartTileInfo *__restrict__ tiles, int64_t n_tiles, int *__restrict__ tile_head,
+part_scan_kernel(const PartTileInfo *tiles, int64_t n_tiles, int *__restrict__ tile_head,
                  int64_t *__restrict__ tile_offset, HostWords *out)
 {
     __shared__ int s_head[PART_SCAN_BLOCK / 32 + 1];
     __shared__ int64_t s_sum[PART_SCAN_BLOCK / 32 + 1];
+    wait_for_predecessor();      // launched early behind (A)
     int carry_head = -1;
     int64_t carry = 0;
     for (int64_t base = 0; base < n_tiles; base += PART_SCAN_BLOCK) {

@@ -60,7 +60,8 @@ static int partition_count(const char *who, const int *d_indptr, int64_t n_rows,
     AGCN_HOST_WORDS(words, s);
     AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words.device());
     AGCN_LAUNCH_CHECK("part_describe_kernel");
-    AGCN_KERNEL(part_scan_kernel, 1, PART_SCAN_BLOCK, s, (const PartTileInfo *)sc.info, tiles, sc.tile_head, sc.tile_offset, words.device());
+    AGCN_CUDA(launch_early(true, part_scan_kernel, 1, PART_SCAN_BLOCK, 0, s, (const PartTileInfo *)sc.info, tiles, sc.tile_head, sc.tile_offset,
+                           words.device()));
     AGCN_LAUNCH_CHECK("part_scan_kernel");
     return partition_answer(who, words, n_blocks);
 }
