@@ -37,7 +37,11 @@ def block_level_partition(indptr) -> np.ndarray:
 
 
 def block_level_partition_device(indptr, stream=None):
-    """Device tensor in (torch int32 CUDA tensor [n_rows+1]), device tensor out [n_blocks, 4]."""
+    """Device tensor in (torch int32 CUDA tensor [n_rows+1]), device tensor out [n_blocks, 4].
+
+    On the current stream the tuples are written behind what that stream holds, like the result of any torch
+    operation.  With another `stream` they are complete when the call returns: neither tensor is known to torch's
+    allocator as in use there, and the caller may go on with them anywhere."""
     import torch
     lib = _lib.load()
     if not (indptr.is_cuda and indptr.dtype == torch.int32 and indptr.is_contiguous()):
@@ -46,7 +50,8 @@ def block_level_partition_device(indptr, stream=None):
     if n_rows <= 0:
         raise IndexError("empty graph")
     dev = _lib.device_index(indptr.device)
-    s = stream.cuda_stream if stream is not None else _lib.raw_stream(dev)
+    current = _lib.raw_stream(dev)
+    s = stream.cuda_stream if stream is not None else current
     n_blocks, run = ctypes.c_int64(0), ctypes.c_void_p()
     with _lib.on_device(dev):
         _lib.check(lib.agcn_partition_begin(indptr.data_ptr(), n_rows, ctypes.byref(run), ctypes.byref(n_blocks), s))
@@ -56,4 +61,6 @@ def block_level_partition_device(indptr, stream=None):
             lib.agcn_partition_finish(run, None)
             raise
         _lib.check(lib.agcn_partition_finish(run, out.data_ptr() if n_blocks.value else None))
+        if s != current:
+            stream.synchronize()
     return out

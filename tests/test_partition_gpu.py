@@ -122,3 +122,25 @@ def test_runs_across_tiles_match_oracle(run):
         want = oracle.partition(indptr)
         assert np.array_equal(partition.block_level_partition(indptr), want)
         assert np.array_equal(partition.block_level_partition_device(torch.from_numpy(indptr).to(dev)).cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("n", [5_000, 700_000])
+def test_on_another_stream_the_tuples_are_complete_on_return(n):
+    # one-pass form (up to 256 tiles of 2048 rows) and the form whose last kernel still reads the row pointers: with a
+    # stream that is not the current one the caller goes on elsewhere, here while that stream is kept busy
+    import torch
+    from accelgcn import partition
+    dev = require_cuda()
+    indptr = np.concatenate([[0], np.cumsum(np.sort(np.random.default_rng(n).integers(0, 60, n)))]).astype(np.int32)
+    want = oracle.partition(indptr)
+    side = torch.cuda.Stream(dev)
+    busy = torch.zeros(1 << 26, device=dev)
+    for _ in range(4):
+        d_ip = torch.from_numpy(indptr).to(dev)
+        torch.cuda.synchronize()
+        out = partition.block_level_partition_device(d_ip, stream=side)
+        assert side.query()                       # nothing of the call is left on that stream
+        d_ip.zero_()                              # the row pointers are the caller's again
+        assert np.array_equal(out.cpu().numpy(), want)
+        with torch.cuda.stream(side):
+            busy.add_(1)
