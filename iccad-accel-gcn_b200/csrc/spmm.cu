@@ -387,8 +387,11 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     AGCN_REQUIRE(panel >= 1 && panel <= SPMM_PANEL, "agcn_spmm_run: AGCN_SPMM_PANEL must be 1..%d", SPMM_PANEL);
     if (x_vec && panel % 4 != 0) panel = (panel + 3) & ~3;         // keep every panel's first column 16-byte aligned
     if (panel > SPMM_PANEL) panel = SPMM_PANEL;
-    for (int col0 = 0; col0 < dim; col0 += panel) {
-        const int width = dim - col0 < panel ? dim - col0 : panel;
+    for (int col0 = 0, width = 0; col0 < dim; col0 += width) {
+        // a pass ends where the carry slot does: behind the last slot lie the arrival counters
+        const int slot_left = SPMM_PANEL - col0 % SPMM_PANEL;
+        width = dim - col0 < panel ? dim - col0 : panel;
+        if (width > slot_left) width = slot_left;
         SpmmParams prm;
         prm.tuples = p->tuples; prm.n_tuples = p->n_tuples;
         prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag;

@@ -459,6 +459,27 @@ def test_forced_column_passes_on_small_graphs(cfg1, cfg4_small, panel, monkeypat
             case.check(x, case.run(x))
 
 
+@pytest.mark.parametrize("panel", [48, 96, 100])
+@pytest.mark.parametrize("dim", [192, 256, 301])
+def test_column_passes_that_do_not_divide_a_carry_slot(cfg4_small, panel, dim, monkeypatch):
+    # a slot holds 128 columns of a row that crosses units, and the arrival counters follow the last slot: a pass
+    # that went on past its slot left counters that are not zero, and the plan's next product a row unwritten
+    import torch
+    from accelgcn import spmm
+    monkeypatch.setenv("AGCN_SPMM_PANEL", str(panel))
+    monkeypatch.setenv("AGCN_SPMM_PIECE", "0")
+    c = cfg4_small
+    plan = spmm.SpmmPlan(c.t["block4"], c.t["idx"], c.n, c.n)
+    assert plan.info()["n_carry"] > 0
+    x = c.x(dim)
+    xt = torch.from_numpy(x).to(c.dev)
+    for _ in range(3):
+        y = torch.full((c.n, dim), float("nan"), device=c.dev)
+        plan.run(c.t["idx"], c.t["val"], xt, y)
+        c.check(x, y.cpu().numpy())
+    plan.close()
+
+
 @pytest.mark.parametrize("piece", [0, 7, 64, 100, 192])
 def test_tuples_cut_into_pieces(cfg1, cfg4_small, piece, monkeypatch):
     # AGCN_SPMM_PIECE (read at plan creation): 0 = uncut, the form of large plans (heavy rows across units, light and
