@@ -77,8 +77,8 @@ inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // Stream-ordered memory of the current device's pool (memory.cu).
 cudaError_t pool_alloc(void **out, size_t bytes, cudaStream_t s);
 void pool_free(void *p, cudaStream_t s);
-// for blocks that work on any stream may still use: waits for the device, as cudaFree does
-void pool_free_waiting(void *p);
+// for blocks that work on any stream may still use: waits for `device`, whose pool the block is from, as cudaFree does
+cudaError_t pool_free_waiting(void *p, int device);
 
 // Pool memory for the length of a call, used and given back on one stream.
 class DeviceScratch {

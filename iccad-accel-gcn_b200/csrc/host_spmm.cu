@@ -27,6 +27,7 @@ constexpr int HOST_SPMM_PANEL = 128;                  // widest product that can
 }
 
 struct agcn_host_ctx {
+    int device = -1;                                  // streams and buffers are this device's; every call makes it current
     cudaStream_t s_up = nullptr, s_run = nullptr, s_down = nullptr;
     void *graph[3] = {nullptr, nullptr, nullptr};     // block4, idx, val
     size_t graph_cap[3] = {0, 0, 0};
@@ -74,8 +75,9 @@ static int ctx_chain(agcn_host_ctx *c, cudaStream_t from, cudaStream_t to)
 static int reserve(agcn_host_ctx *c, void **buf, size_t *cap, size_t bytes)
 {
     if (bytes <= *cap) return AGCN_OK;
-    pool_free_waiting(*buf);
+    const cudaError_t freed = pool_free_waiting(*buf, c->device);
     *buf = nullptr; *cap = 0;
+    AGCN_CUDA(freed);
     const cudaError_t e = pool_alloc(buf, bytes, c->s_run);
     if (e != cudaSuccess) {
         set_error("agcn_host_spmm: device allocation of %zu bytes: %s", bytes, cudaGetErrorString(e));
@@ -452,7 +454,8 @@ extern "C" int agcn_host_ctx_create(agcn_host_ctx **ctx)
     *ctx = nullptr;
     agcn_host_ctx *c = new (std::nothrow) agcn_host_ctx;
     AGCN_REQUIRE(c != nullptr, "agcn_host_ctx_create: out of host memory");
-    cudaError_t e = cudaStreamCreateWithFlags(&c->s_up, cudaStreamNonBlocking);
+    cudaError_t e = cudaGetDevice(&c->device);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->s_up, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->s_run, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->s_down, cudaStreamNonBlocking);
     for (cudaEvent_t *ev : {&c->t_up0, &c->t_up1, &c->t_run0, &c->t_run1, &c->t_down1})
@@ -468,19 +471,27 @@ extern "C" int agcn_host_ctx_create(agcn_host_ctx **ctx)
 
 extern "C" int agcn_host_ctx_destroy(agcn_host_ctx *ctx)
 {
-    agcn::clear_error();
+    using namespace agcn;
+    clear_error();
     if (ctx == nullptr) return AGCN_OK;
-    agcn::plan_free(ctx->plan);
-    for (int i = 0; i < 3; i++) agcn::pool_free_waiting(ctx->graph[i]);
+    const DeviceOf on(ctx->device);
+    cudaError_t failed = cudaSuccess;
+    auto release = [&](void *p) {
+        const cudaError_t e = pool_free_waiting(p, ctx->device);
+        if (failed == cudaSuccess) failed = e;
+    };
+    plan_free(ctx->plan);
+    for (int i = 0; i < 3; i++) release(ctx->graph[i]);
     for (const std::vector<void *> *v : {&ctx->xbuf, &ctx->xpad, &ctx->ybuf, &ctx->cbuf})
-        for (void *p : *v) agcn::pool_free_waiting(p);
-    agcn::pool_free_waiting(ctx->d_abort);
+        for (void *p : *v) release(p);
+    release(ctx->d_abort);
     for (cudaEvent_t e : ctx->events) cudaEventDestroy(e);
     for (cudaEvent_t e : {ctx->t_up0, ctx->t_up1, ctx->t_run0, ctx->t_run1, ctx->t_down1}) if (e) cudaEventDestroy(e);
     if (ctx->s_up) cudaStreamDestroy(ctx->s_up);
     if (ctx->s_run) cudaStreamDestroy(ctx->s_run);
     if (ctx->s_down) cudaStreamDestroy(ctx->s_down);
     delete ctx;
+    AGCN_CUDA(failed);
     return AGCN_OK;
 }
 
@@ -489,12 +500,14 @@ extern "C" int agcn_host_set_graph(agcn_host_ctx *ctx, const int32_t *h_block4, 
                                    int64_t n_rows, int64_t n_cols, int64_t nnz)
 {
     agcn::clear_error();
+    const agcn::DeviceOf on(ctx != nullptr ? ctx->device : -1);
     return agcn::host_set_graph(ctx, h_block4, n_blocks, h_indices, h_vals, n_rows, n_cols, nnz);
 }
 
 extern "C" int agcn_host_spmm(agcn_host_ctx *ctx, const float *h_x, float *h_y, int dim)
 {
     agcn::clear_error();
+    const agcn::DeviceOf on(ctx != nullptr ? ctx->device : -1);
     return agcn::host_products(ctx, 1, &h_x, &h_y, &dim);
 }
 
@@ -502,6 +515,7 @@ extern "C" int agcn_host_spmm_batch(agcn_host_ctx *ctx, int n_products, const fl
                                     const int *dims)
 {
     agcn::clear_error();
+    const agcn::DeviceOf on(ctx != nullptr ? ctx->device : -1);
     return agcn::host_products(ctx, n_products, h_x, h_y, dims);
 }
 
@@ -510,6 +524,7 @@ extern "C" int agcn_spmm_host(agcn_host_ctx *ctx, const int32_t *h_block4, int64
                               int64_t n_rows, int64_t n_cols, int64_t nnz, int dim)
 {
     agcn::clear_error();
+    const agcn::DeviceOf on(ctx != nullptr ? ctx->device : -1);
     return agcn::host_graph_and_products(ctx, h_block4, n_blocks, h_indices, h_vals, n_rows, n_cols, nnz, 1, &h_x, &h_y, &dim);
 }
 
@@ -519,6 +534,7 @@ extern "C" int agcn_spmm_host_batch(agcn_host_ctx *ctx, const int32_t *h_block4,
                                     int n_products, const float *const *h_x, float *const *h_y, const int *dims)
 {
     agcn::clear_error();
+    const agcn::DeviceOf on(ctx != nullptr ? ctx->device : -1);
     return agcn::host_graph_and_products(ctx, h_block4, n_blocks, h_indices, h_vals, n_rows, n_cols, nnz, n_products, h_x, h_y, dims);
 }
 

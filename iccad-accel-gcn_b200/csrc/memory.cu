@@ -58,11 +58,13 @@ void pool_free(void *p, cudaStream_t s)
     if (p != nullptr) cudaFreeAsync(p, s);
 }
 
-void pool_free_waiting(void *p)
+cudaError_t pool_free_waiting(void *p, int device)
 {
-    if (p == nullptr) return;
-    cudaDeviceSynchronize();             // what cudaFree did: whoever still uses the block is done
-    cudaFreeAsync(p, cudaStreamPerThread);
+    if (p == nullptr) return cudaSuccess;
+    const DeviceOf on(device);           // the wait and the per-thread stream are those of the current device
+    const cudaError_t waited = cudaDeviceSynchronize();      // what cudaFree did: whoever still uses the block is done
+    const cudaError_t freed = cudaFreeAsync(p, cudaStreamPerThread);
+    return waited != cudaSuccess ? waited : freed;
 }
 
 // ---------------------------------------------------------------------------

@@ -18,11 +18,8 @@ int env_int(const char *name, int dflt)
 void plan_free(agcn_spmm_plan *p)
 {
     if (p == nullptr) return;
-    {
-        const DeviceOf on(p->device);
-        pool_free_waiting(p->memory);
-        pool_free_waiting(p->x_pad);
-    }
+    pool_free_waiting(p->memory, p->device);
+    pool_free_waiting(p->x_pad, p->device);
     delete p;
 }
 
@@ -319,7 +316,7 @@ int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cu
     const size_t need = (size_t)p->n_cols * ldp * sizeof(float);
     if (need > p->x_pad_bytes) {
         // growing the scratch synchronises the device once per plan and width; steady state allocates nothing
-        pool_free_waiting(p->x_pad);
+        AGCN_CUDA(pool_free_waiting(p->x_pad, p->device));
         p->x_pad = nullptr; p->x_pad_bytes = 0;
         AGCN_CUDA(pool_alloc(reinterpret_cast<void **>(&p->x_pad), need, s));
         p->x_pad_bytes = need;

@@ -13,7 +13,8 @@
  *    thread's last failure.  The caller owns every buffer it passes in; the
  *    library owns only plan-internal scratch.
  *  - All entry points run on the CUDA device that is current in the calling
- *    thread.  There is no CPU fallback: without a usable device the calls
+ *    thread; a plan and a host context stay on the one they were created on,
+ *    whichever is current when they are used or destroyed.  There is no CPU fallback: without a usable device the calls
  *    fail with AGCN_ERR_CUDA.
  *  - Reference citations are file:line in xiexi51/ICCAD-Accel-GCN.
  */
