@@ -74,7 +74,8 @@ private:
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// Stream-ordered memory of the current device's pool (memory.cu).
+// Stream-ordered memory of the current device's pool (memory.cu).  Refused (cudaErrorStreamCaptureUnsupported) while
+// `s` is being captured: the block would belong to the graph.
 cudaError_t pool_alloc(void **out, size_t bytes, cudaStream_t s);
 void pool_free(void *p, cudaStream_t s);
 // for blocks that work on any stream may still use: waits for `device`, whose pool the block is from, as cudaFree does

@@ -23,6 +23,7 @@ struct agcn_spmm_plan {
     int pad_unaligned = 1;            // AGCN_SPMM_PAD at creation: copy unaligned X into 16-byte-aligned rows
     float *x_pad = nullptr;           // [n_cols][dim rounded up to 4], grown on demand
     size_t x_pad_bytes = 0;
+    bool x_pad_malloc = false;        // from cudaMalloc, not from the pool
 };
 
 namespace agcn {

@@ -49,7 +49,11 @@ cudaError_t pool_alloc(void **out, size_t bytes, cudaStream_t s)
 {
     *out = nullptr;
     cudaMemPool_t pool = nullptr;
-    cudaError_t e = pool_of_current_device(&pool);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e != cudaSuccess) return e;
+    if (capture != cudaStreamCaptureStatusNone) return cudaErrorStreamCaptureUnsupported;
+    e = pool_of_current_device(&pool);
     return e != cudaSuccess ? e : cudaMallocFromPoolAsync(out, bytes > 0 ? bytes : 16, pool, s);
 }
 

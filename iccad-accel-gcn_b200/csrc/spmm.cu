@@ -15,11 +15,18 @@ int env_int(const char *name, int dflt)
     return v != nullptr && *v ? atoi(v) : dflt;
 }
 
+static cudaError_t pad_free(agcn_spmm_plan *p)
+{
+    float *x_pad = p->x_pad;
+    p->x_pad = nullptr; p->x_pad_bytes = 0;
+    return p->x_pad_malloc ? cudaFree(x_pad) : pool_free_waiting(x_pad, p->device);
+}
+
 void plan_free(agcn_spmm_plan *p)
 {
     if (p == nullptr) return;
     pool_free_waiting(p->memory, p->device);
-    pool_free_waiting(p->x_pad, p->device);
+    pad_free(p);
     delete p;
 }
 
@@ -316,9 +323,18 @@ int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cu
     const size_t need = (size_t)p->n_cols * ldp * sizeof(float);
     if (need > p->x_pad_bytes) {
         // growing the scratch synchronises the device once per plan and width; steady state allocates nothing
-        AGCN_CUDA(pool_free_waiting(p->x_pad, p->device));
-        p->x_pad = nullptr; p->x_pad_bytes = 0;
-        AGCN_CUDA(pool_alloc(reinterpret_cast<void **>(&p->x_pad), need, s));
+        // (Under stream capture a pool block would be the graph's own and gone outside of it; cudaMalloc is refused
+        // there, or in relaxed capture gives memory that outlives the graph.)
+        AGCN_CUDA(pad_free(p));
+        cudaError_t e = pool_alloc(reinterpret_cast<void **>(&p->x_pad), need, s);
+        p->x_pad_malloc = e == cudaErrorStreamCaptureUnsupported;
+        if (p->x_pad_malloc) e = cudaMalloc(reinterpret_cast<void **>(&p->x_pad), need);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            p->x_pad = nullptr;
+            set_error("agcn_spmm_run: %zu bytes for the aligned copy of X: %s", need, cudaGetErrorString(e));
+            return AGCN_ERR_CUDA;
+        }
         p->x_pad_bytes = need;
     }
     const int rc = spmm_pad_rows(d_x, ldx, dim, p->x_pad, p->n_cols, s);

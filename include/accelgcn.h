@@ -148,7 +148,8 @@ int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_indices, con
  * main.cu:12,137).  Rows of X are gathered 16 bytes per lane; when they are not
  * 16-byte aligned (dim % 4 != 0 with ld = dim, an odd stride or base) X is first
  * copied into plan-owned aligned rows (grown on demand: the first such call of
- * a width allocates; AGCN_SPMM_PAD=0 at plan creation selects 4-byte gathers
+ * a width allocates, so make it before a stream capture, and the widest one
+ * before the first capture: growing moves the rows; AGCN_SPMM_PAD=0 at plan creation selects 4-byte gathers
  * instead) and unaligned rows of Y get element-wise stores.  dim > 64 may run
  * as two 64-column passes when X is larger than L2 (environment variable
  * AGCN_SPMM_PANEL = columns per pass, read at plan creation, overrides that

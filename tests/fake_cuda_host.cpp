@@ -23,6 +23,7 @@ std::map<cudaStream_t, int> g_stream_device;
 int g_syncs[2] = {0, 0};                                 // device-wide waits
 int g_wrong_device = 0;                                  // frees, allocations or copies on a stream of another device
 int g_fail_free = 0;
+bool g_capturing = false;
 
 int stream_device(cudaStream_t s)
 {
@@ -71,6 +72,11 @@ cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned)
     *s = reinterpret_cast<cudaStream_t>(std::malloc(8));
     std::lock_guard<std::mutex> l(g_mutex);
     g_stream_device[*s] = t_device;
+    return cudaSuccess;
+}
+cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *st)
+{
+    *st = g_capturing ? cudaStreamCaptureStatusActive : cudaStreamCaptureStatusNone;
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
@@ -156,10 +162,25 @@ static void context_device()
     g_fail_free = 0;
 }
 
+// A block allocated on a stream that is being captured would be the graph's: none is handed out.
+static void pool_under_capture()
+{
+    void *p = nullptr;
+    cudaSetDevice(0);
+    g_capturing = true;
+    CHECK(agcn::pool_alloc(&p, 64, nullptr) == cudaErrorStreamCaptureUnsupported);
+    CHECK(p == nullptr && g_block_device.empty());
+    g_capturing = false;
+    CHECK(agcn::pool_alloc(&p, 64, nullptr) == cudaSuccess && p != nullptr);
+    agcn::pool_free(p, nullptr);
+    CHECK(g_block_device.empty());
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "context_device") context_device();
+    else if (what == "pool_under_capture") pool_under_capture();
     else { std::printf("unknown scenario\n"); return 2; }
     std::printf("%d failures\n", failures);
     return failures != 0;

@@ -548,6 +548,45 @@ def test_unaligned_widths_padded_copy_equals_scalar_path(cfg4_small, dim, monkey
     assert spmm_close(y_pad, y_scalar, row_abs_scale(cfg4_small.indptr, cfg4_small.val, x)).all()
 
 
+def test_first_unaligned_width_under_stream_capture(cfg4_small):
+    # the aligned copy of X is made at a width's first call.  Captured in the default mode that call is refused, as any
+    # allocation is; in relaxed mode its memory outlives the graph, so that products outside of it can use it too
+    import ctypes
+    import torch
+    from accelgcn import spmm
+    from accelgcn._lib import AccelGcnError
+    c, dim = cfg4_small, 61
+    rt = ctypes.CDLL(next(line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line))
+    x = c.x(dim)
+    xt = torch.from_numpy(x).to(c.dev)
+    y = torch.empty((c.n, dim), device=c.dev)
+    side = torch.cuda.Stream(c.dev)
+    stream, graph, exe = ctypes.c_void_p(side.cuda_stream), ctypes.c_void_p(), ctypes.c_void_p()
+    plan = spmm.SpmmPlan(c.t["block4"], c.t["idx"], c.n, c.n)
+    torch.cuda.synchronize()
+    assert rt.cudaStreamBeginCapture(stream, 0) == 0                  # cudaStreamCaptureModeGlobal
+    with pytest.raises(AccelGcnError):
+        plan.run(c.t["idx"], c.t["val"], xt, y, stream=side)
+    rt.cudaStreamEndCapture(stream, ctypes.byref(graph))
+    rt.cudaGetLastError()
+    assert rt.cudaStreamBeginCapture(stream, 2) == 0                  # cudaStreamCaptureModeRelaxed
+    plan.run(c.t["idx"], c.t["val"], xt, y, stream=side)
+    assert rt.cudaStreamEndCapture(stream, ctypes.byref(graph)) == 0
+    assert rt.cudaGraphInstantiate(ctypes.byref(exe), graph, ctypes.c_ulonglong(0)) == 0
+    plan.run(c.t["idx"], c.t["val"], xt, y)                           # the graph has not run
+    c.check(x, y.cpu().numpy())
+    for _ in range(2):
+        y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        assert rt.cudaGraphLaunch(exe, stream) == 0
+        side.synchronize()
+        c.check(x, y.cpu().numpy())
+    assert rt.cudaGraphExecDestroy(exe) == 0 and rt.cudaGraphDestroy(graph) == 0
+    plan.run(c.t["idx"], c.t["val"], xt, y)
+    c.check(x, y.cpu().numpy())
+    plan.close()
+
+
 @pytest.mark.parametrize("case_name", ["cfg1", "cfg4_small"])
 def test_column_tiled_small(case_name, request):
     # tiled plan with several range layouts (one of them empty), ReLU, an unaligned width and the
