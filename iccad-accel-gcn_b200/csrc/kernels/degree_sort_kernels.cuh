@@ -169,10 +169,11 @@ radix_pass_kernel(const int *__restrict__ indptr, int64_t n, int pass, SortBuffe
     const int64_t tile = s_tile;
     const int done = sort_passes_done(ctl, pass, n);
     const bool odd = (done & 1) != 0;           // pass k of those that move something writes buffer k mod 2
-    const unsigned *__restrict__ keys_in = odd ? buf.keys[0] : buf.keys[1];
-    const int *__restrict__ rows_in = odd ? buf.rows[0] : buf.rows[1];
-    unsigned *__restrict__ keys_out = odd ? buf.keys[1] : buf.keys[0];
-    int *__restrict__ rows_out = odd ? buf.rows[1] : buf.rows[0];
+    // (not __restrict__: the pass before may still be writing them when this kernel starts)
+    const unsigned *keys_in = odd ? buf.keys[0] : buf.keys[1];
+    const int *rows_in = odd ? buf.rows[0] : buf.rows[1];
+    unsigned *keys_out = odd ? buf.keys[1] : buf.keys[0];
+    int *rows_out = odd ? buf.rows[1] : buf.rows[0];
 
     const int w = warp_id(), lane = lane_id(), shift = pass * RADIX_BITS;
     const int64_t warp_base = tile * SORT_TILE + (int64_t)w * SORT_WARP_KEYS;
@@ -268,8 +269,8 @@ sort_finish_kernel(int64_t n, int passes, SortBuffers buf, SortControl *__restri
     __syncthreads();
     const int64_t tile = s_tile, base = tile * FINAL_TILE;
     const bool odd = (sort_passes_done(ctl, passes, n) & 1) != 0;
-    const int *__restrict__ rows = odd ? buf.rows[0] : buf.rows[1];
-    const unsigned *__restrict__ keys = odd ? buf.keys[0] : buf.keys[1];
+    const int *rows = odd ? buf.rows[0] : buf.rows[1];          // written by the kernel before: not __restrict__
+    const unsigned *keys = odd ? buf.keys[0] : buf.keys[1];
 #pragma unroll
     for (int k = 0; k < FINAL_ITEMS; k++) {
         const int j = k * SORT_BLOCK + threadIdx.x;
@@ -533,7 +534,7 @@ csr_permute_kernel(const int *__restrict__ old_indptr, const int *__restrict__ o
             if (c[k] < 0 || c[k] >= n_rows) { bad = true; c[k] = 0; }
         if (bad) out->w[SORT_WORD_COLUMN] = 1;
 #pragma unroll
-        for (int k = 0; k < PERMUTE_ITEMS; k++) c[k] = __ldg(new_id + c[k]);
+        for (int k = 0; k < PERMUTE_ITEMS; k++) c[k] = new_id[c[k]];
     }
 #pragma unroll
     for (int k = 0; k < PERMUTE_ITEMS; k++)

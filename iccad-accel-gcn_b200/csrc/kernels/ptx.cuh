@@ -34,18 +34,20 @@ __device__ __forceinline__ L2Policies make_l2_policies()
     return p;
 }
 
-// dense operand X: read-only path, 16 bytes per lane, keep in L2
+// dense operand X: 16 bytes per lane, keep in L2.  Not the read-only path (.nc): the launch before may still be
+// making X while the reader is already resident and waits for it.  (A load needs a column id, staged in shared memory
+// and read behind that wait, for its address: it cannot move above it.)
 __device__ __forceinline__ float4 ld_x4(const float *p, uint64_t policy)
 {
     float4 v;
-    asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+    asm("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(policy));
     return v;
 }
 __device__ __forceinline__ float ld_x1(const float *p, uint64_t policy)
 {
     float v;
-    asm("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+    asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
     return v;
 }
 

@@ -136,3 +136,23 @@ def test_tile_edges_and_number_of_passes(n, top, relabel):
     want = oracle.degree_sort(indptr, idx, val, relabel_cols=relabel)
     for a, b, what in zip(got, want, ("perm", "indptr", "indices", "vals")):
         assert np.array_equal(a, b), what
+
+
+@pytest.mark.parametrize("n", [50_000, 200_000])
+def test_two_graphs_in_turn_in_the_same_scratch(n):
+    # the permute is resident while the kernel before it writes the new names it looks up, into the memory in which
+    # the last call had other names
+    import torch
+    from accelgcn import degree_sort
+    dev = require_cuda()
+    graphs, want = [], []
+    for seed in (1, 2):
+        rng = np.random.default_rng(seed)
+        indptr = np.concatenate([[0], np.cumsum(rng.integers(0, 12, n))]).astype(np.int32)
+        idx = rng.integers(0, n, int(indptr[-1]), dtype=np.int32)
+        graphs.append([torch.from_numpy(a).to(dev) for a in (indptr, idx)])
+        want.append(oracle.degree_sort(indptr, idx, None, relabel_cols=True))
+    for k in range(12):
+        got = degree_sort.degree_sort_device(*graphs[k % 2], None, relabel_cols=True)
+        for a, b in zip(got[:3], want[k % 2][:3]):
+            assert np.array_equal(a.cpu().numpy(), b)

@@ -548,6 +548,27 @@ def test_unaligned_widths_padded_copy_equals_scalar_path(cfg4_small, dim, monkey
     assert spmm_close(y_pad, y_scalar, row_abs_scale(cfg4_small.indptr, cfg4_small.val, x)).all()
 
 
+def test_product_that_starts_under_the_copy_of_x_reads_the_new_x(cfg1, cfg4_small):
+    # with unaligned rows the product is resident while the copy of X it reads is still being written: X changes from
+    # run to run, and every run must equal, bit for bit, the product of the same X in aligned rows
+    import torch
+    from accelgcn import spmm
+    for c in (cfg1, cfg4_small):
+        plan = spmm.SpmmPlan(c.t["block4"], c.t["idx"], c.n, c.n)
+        aligned = torch.zeros((c.n, 64), device=c.dev)
+        y, want = torch.empty((c.n, 61), device=c.dev), torch.empty((c.n, 64), device=c.dev)
+        x = torch.from_numpy(c.x(61)).to(c.dev)
+        bad = torch.zeros((), dtype=torch.int64, device=c.dev)
+        for _ in range(20):
+            x.mul_(-1.0).add_(0.25)
+            aligned[:, :61] = x
+            plan.run(c.t["idx"], c.t["val"], aligned, want)
+            plan.run(c.t["idx"], c.t["val"], x, y)
+            bad += (y != want[:, :61]).sum()
+        assert int(bad) == 0
+        plan.close()
+
+
 def test_first_unaligned_width_under_stream_capture(cfg4_small):
     # the aligned copy of X is made at a width's first call.  Captured in the default mode that call is refused, as any
     # allocation is; in relaxed mode its memory outlives the graph, so that products outside of it can use it too
