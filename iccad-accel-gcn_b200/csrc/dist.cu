@@ -490,6 +490,8 @@ extern "C" int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const 
     AGCN_CUDA(cudaMalloc(&f->d_status, 4 * sizeof(int)));
     AGCN_CUDA(cudaMalloc(&f->d_stamps, 4 * sizeof(unsigned long long)));
     AGCN_CUDA(cudaMemset(f->d_status, 0, 4 * sizeof(int)));
+    AGCN_CUDA(cudaMemset(f->d_stamps, 0, 4 * sizeof(unsigned long long)));
+    AGCN_CUDA(cudaStreamSynchronize(nullptr));           // a forward's stream need not wait for the default one
     for (cudaEvent_t &e : f->ev) AGCN_CUDA(cudaEventCreate(&e));
     if (env_int("AGCN_GCN_FUSED", 0) != 0 && dist->plan != nullptr && dist->per > 0 && dist->n_blocks > 0 && !dist->plan->split) {
         // leading rows of at most 32 nonzeros (the block starts with its light rows in ascending degree), in whole tiles
@@ -532,14 +534,15 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
     if (d->world == 1 && d->tiled == nullptr && fwd->fused_rows == 0) {
         // Nothing is exchanged: transform and product alternate on the stream, each starting while the one before it
         // ends.  The transforms note their own times: events between the kernels keep them apart (13 us of a forward
-        // over 16 384 rows).  (A product does not start before the transform's end: thread blocks that wait for it on SMs
+        // over 16 384 rows), and so would a memset of their status words (which keep what they hold until it is read).  (A
+        // product does not start before the transform's end: thread blocks that wait for it on SMs
         // taken by the transform spread the heavy rows unevenly, 2 % of a forward over 5 M rows.)
         fwd->alone = true;
         const DeviceOf on(d->plan->device);
         AGCN_CUDA(cudaEventRecord(fwd->ev[0], s));
         for (int layer = 0; layer < 2; layer++) {
             int rc = gemm_tf32_async(layer == 0 ? d_x_block : fwd->h1, 128, fwd->w[layer], fwd->z, 128, d->per, fwd->d_status + layer, s,
-                                     layer == 1, fwd->d_stamps + 2 * layer);
+                                     true, layer == 1, fwd->d_stamps + 2 * layer);
             if (rc != AGCN_OK) return rc;
             float *out = layer == 0 ? fwd->h1 : d_out_block;
             rc = spmm_check_run_args(d->plan, d->idx, d->val, fwd->z, 128, out, 128, 128, AGCN_ACT_RELU);
@@ -600,8 +603,8 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
     return AGCN_OK;
 }
 
-// After the stream of the last run has been synchronised: the status of its GEMMs (a pipeline wait
-// that ran out gives AGCN_ERR_CUDA) and, optionally, six times in milliseconds -- per layer the
+// After the stream of the last run has been synchronised: the status of the GEMMs (a pipeline wait
+// that ran out in a run since the last call gives AGCN_ERR_CUDA) and, optionally, six times in milliseconds -- per layer the
 // dense transform, the wait for the first slice of the exchange, and the SpMM (which includes the
 // waits for later slices).
 extern "C" int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6)
@@ -612,6 +615,8 @@ extern "C" int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6)
     int status[4] = {0, 0, 0, 0};
     AGCN_CUDA(cudaMemcpy(status, fwd->d_status, sizeof(status), cudaMemcpyDeviceToHost));
     if (status[0] != 0 || status[1] != 0 || status[2] != 0 || status[3] != 0) {
+        AGCN_CUDA(cudaMemset(fwd->d_status, 0, sizeof(status)));           // reported once
+        AGCN_CUDA(cudaStreamSynchronize(nullptr));
         set_error("agcn_gcn2_forward: a pipeline wait of the dense transform ran out (layer %d); the output is incomplete",
                   status[0] != 0 ? 1 : 2);
         return AGCN_ERR_CUDA;

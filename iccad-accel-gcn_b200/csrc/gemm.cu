@@ -38,11 +38,12 @@ static const char *gemm_status_text(int status)
 }
 
 // Checks the arguments, encodes the tensor map of H and launches.  Nothing is allocated and the
-// stream is not synchronised; *d_status (device, zeroed by the kernel) receives a GEMM_ERR_*
-// code if a pipeline wait runs out.
+// stream is not synchronised; *d_status (device) receives a GEMM_ERR_* code if a pipeline wait runs
+// out.  It is zeroed on the stream, or with keep_status left as it is: then it was zero before, or
+// holds an earlier launch's code that nobody has read yet.
 static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
                             int k_dim, int n_dim, int *d_status, cudaStream_t s, uint32_t spin_limit, int skip_first_load,
-                            bool early = false, unsigned long long *d_stamp = nullptr)
+                            bool keep_status = false, bool early = false, unsigned long long *d_stamp = nullptr)
 {
     AGCN_REQUIRE(d_h != nullptr && d_w != nullptr && d_z != nullptr && d_status != nullptr, "agcn_gemm_tf32: null pointer");
     AGCN_REQUIRE(k_dim == GEMM_DIM && n_dim == GEMM_DIM,
@@ -51,10 +52,8 @@ static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, flo
     AGCN_REQUIRE(ldh >= GEMM_DIM && ldz >= GEMM_DIM && ldh % 4 == 0 && ldz % 4 == 0,
                  "agcn_gemm_tf32: row strides must be >= 128 and multiples of 4 floats");
     AGCN_REQUIRE(aligned16(d_h) && aligned16(d_z), "agcn_gemm_tf32: H and Z must be 16-byte aligned");
-    if (m_rows == 0) {
-        AGCN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
-        return AGCN_OK;
-    }
+    if (!keep_status) AGCN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
+    if (m_rows == 0) return AGCN_OK;
 
     EncodeTiledFn encode = nullptr;
     int rc = get_encode_fn(&encode);
@@ -124,9 +123,9 @@ static int gemm_tf32_sync(const float *d_h, int64_t ldh, const float *d_w, float
 }
 
 int gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
-                    int *d_status, cudaStream_t s, bool early, unsigned long long *d_stamp)
+                    int *d_status, cudaStream_t s, bool keep_status, bool early, unsigned long long *d_stamp)
 {
-    return gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, GEMM_DIM, GEMM_DIM, d_status, s, GEMM_SPIN_LIMIT, 0, early, d_stamp);
+    return gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, GEMM_DIM, GEMM_DIM, d_status, s, GEMM_SPIN_LIMIT, 0, keep_status, early, d_stamp);
 }
 
 }  // namespace agcn

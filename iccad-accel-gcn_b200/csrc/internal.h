@@ -81,10 +81,11 @@ int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag
 void plan_free(agcn_spmm_plan *p);
 
 
-// gemm.cu: Z = H * W (128 x 128, TF32) enqueued on `s`; nothing allocated, nothing synchronised.  early: the launch
-// before it on the stream makes H; d_stamp: when it began and ended, in ns (both optional)
+// gemm.cu: Z = H * W (128 x 128, TF32) enqueued on `s`; nothing allocated, nothing synchronised.  keep_status: *d_status
+// is not zeroed first; early: the launch before it on the stream makes H; d_stamp: when it began and ended, in ns, the
+// end zero before the first launch (all optional)
 int gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
-                    int *d_status, cudaStream_t s, bool early = false, unsigned long long *d_stamp = nullptr);
+                    int *d_status, cudaStream_t s, bool keep_status = false, bool early = false, unsigned long long *d_stamp = nullptr);
 // Z2[r] = relu(A[r, :] * Z1) * W for the first m_rows rows of a CSR block, all of at most
 // fused_layer_max_degree() nonzeros (gemm.cu)
 int fused_layer_async(const int *d_indptr, const int *d_indices, const float *d_vals, const float *d_z_in, const float *d_w,

@@ -179,7 +179,8 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
                      float *__restrict__ z, int64_t ldz, int64_t m_rows, int n_tiles, int *__restrict__ err_flag,
                      uint32_t spin_limit, int skip_first_load, unsigned long long *stamp)
 {
-    // stamp: null, or where the times (ns) of the first load and of the last thread block's end go.
+    // err_flag: zero before the launch.  stamp: null, or where the times (ns) of the first load and of the last thread
+    // block's end go; the latter only grows and starts at zero.
     // spin_limit: polls a wait may take (GEMM_SPIN_LIMIT in normal use).  skip_first_load: self-test
     // of the failure path only -- the producer leaves out the first load of the thread block, so the
     // MMA issuer's wait for it runs out and the kernel must leave through the abort path.
@@ -206,11 +207,6 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
         *s_abort = 0;
         *s_never = 0;
         fence_barrier_init();
-    }
-    // (a memset of its own cost 2 us; nobody else writes the word for the thousands of polls a wait takes at least)
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        *err_flag = 0;
-        if (stamp != nullptr) stamp[1] = 0;
     }
     if (warp == 1) tmem_alloc(smem_u32(s_tmem_base), GEMM_TMEM_COLS);
     tc_fence_before();

@@ -402,7 +402,7 @@ int agcn_dist_gathered(const agcn_dist *dist, int slot, const float **d_gathered
  * its operator exists for.  W1 / W2 are borrowed [128 x 128] device arrays.
  * run enqueues one forward on `stream` and returns; after synchronising that
  * stream, agcn_gcn2_forward_status reports a dense transform whose bounded wait
- * ran out (AGCN_ERR_CUDA) and, if ms6 is not NULL, six times in milliseconds:
+ * ran out (AGCN_ERR_CUDA; on one GPU in any run since the last call) and, if ms6 is not NULL, six times in milliseconds:
  * per layer the transform, the wait for the exchange's first slice, the SpMM.
  * ---------------------------------------------------------------------- */
 typedef struct agcn_gcn2 agcn_gcn2;

@@ -110,6 +110,44 @@ def test_gemm_bounded_wait_runs_out_and_the_next_call_succeeds():
         _check_gemm(h.cpu().numpy(), w.cpu().numpy(), z2.cpu().numpy())
 
 
+@pytest.mark.parametrize("m", [1, 128 * 5, 128 * 300])
+def test_gemm_error_of_any_thread_block_is_reported_every_time(m):
+    # the status word is zeroed on the stream and not by a thread block of the launch that may report into it
+    import torch
+    from accelgcn import gemm, synth, _lib
+    dev = require_cuda()
+    h, w = synth.features(m, 128, 4, dev), synth.glorot(128, 128, 5, 9, dev)
+    z = torch.zeros((m, 128), device=dev)
+    for _ in range(10):
+        assert gemm.selftest_timeout(h, w, z) == _lib.ERR_CUDA
+    want = gemm.gemm_tf32(h, w)
+    status = torch.full((1,), 5, dtype=torch.int32, device=dev)          # what an earlier launch left is gone too
+    gemm.gemm_tf32_async(h, w, z, status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and torch.equal(z, want)
+
+
+def test_forward_times_of_the_last_of_several_runs():
+    # the transforms note their own begin and end; the end only grows and is never cleared by a run
+    import torch
+    from accelgcn import synth, degree_sort, sharded, gcn
+    dev = require_cuda()
+    g = synth.make_config(5, dev, 0.0005)
+    _, ip, ix, v = degree_sort.degree_sort_device(g.indptr, g.indices, g.vals)
+    sh = sharded.ShardedSpmm(ip, ix, v, 0, 1)
+    fwd = gcn.GcnForward(sh, [synth.glorot(128, 128, 1005, k, dev) for k in (8, 9)])
+    x = sh.to_block(synth.features(g.n, 128, 1005, dev))
+    for runs in (1, 3, 2):
+        for _ in range(runs):
+            fwd.forward(x)
+        torch.cuda.synchronize()
+        times = fwd.status(timings=True)
+        # one run of 25 000 nodes is well below a millisecond; times that span several runs or none are not
+        assert all(t >= 0 for layer in times for t in layer) and all(layer[0] > 0 and layer[2] > 0 for layer in times)
+        assert sum(t for layer in times for t in layer) < 5.0
+    fwd.close(); sh.close()
+
+
 def _forward_reference(ip_h, ix_h, v_h, x_h, w1_h, w2_h):
     """CPU forward: fp32 storage, dense transform in fp64 row blocks, SpMM with fp64 accumulation (oracle)."""
     from oracle import oracle
