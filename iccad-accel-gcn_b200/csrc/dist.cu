@@ -505,10 +505,12 @@ extern "C" int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const 
         std::vector<int> unit_row((size_t)n_units);
         AGCN_CUDA(cudaMemcpy2D(unit_row.data(), sizeof(int), dist->block4 + 1, 8 * 4 * sizeof(int), sizeof(int), (size_t)n_units,
                                cudaMemcpyDeviceToHost));
-        int64_t lo = 0, hi = n_units;                    // first unit whose first row is > rows
+        // first unit that begins at or behind that row (a heavy row begins several): the one before it holds the row's
+        // beginning.  From inside the row its partial sums would not all arrive, now or in the next product.
+        int64_t lo = 0, hi = n_units;
         while (lo < hi) {
             const int64_t mid = lo + (hi - lo) / 2;
-            if (unit_row[mid] <= rows) lo = mid + 1; else hi = mid;
+            if (unit_row[mid] < rows) lo = mid + 1; else hi = mid;
         }
         if (rows >= 128 * 64 && lo > 0) {
             f->fused_rows = rows;

@@ -268,12 +268,59 @@ def test_fused_layer_matches_fp64(m, n_cols):
     assert np.all(np.abs(got - ref) <= 2e-3 * scale + 1e-5), float(np.max(np.abs(got - ref) / (scale + 1e-30)))
 
 
+def _captured_nodes(forward, x):
+    """Operations one forward enqueues: kernels, memsets and event records of a captured run."""
+    import ctypes
+    import torch
+    rt = ctypes.CDLL(next(line.split()[-1] for line in open("/proc/self/maps") if "libcudart" in line))
+    side, graph, n = torch.cuda.Stream(), ctypes.c_void_p(), ctypes.c_size_t(0)
+    out = torch.empty_like(x)
+    torch.cuda.synchronize()
+    assert rt.cudaStreamBeginCapture(ctypes.c_void_p(side.cuda_stream), 2) == 0
+    forward.forward(x, out=out, stream=side)
+    assert rt.cudaStreamEndCapture(ctypes.c_void_p(side.cuda_stream), ctypes.byref(graph)) == 0
+    assert rt.cudaGraphGetNodes(graph, None, ctypes.byref(n)) == 0 and rt.cudaGraphDestroy(graph) == 0
+    return n.value
+
+
+def test_fused_layer_boundary_in_front_of_a_row_of_several_units(monkeypatch):
+    # the first row left to the SpMM spans several units (27 tuples): it is multiplied from its first unit on, and its
+    # arrival counter is zero again for the products that follow
+    import torch
+    from accelgcn import synth, sharded, gcn
+    dev = require_cuda()
+    monkeypatch.setenv("AGCN_SPMM_PIECE", "0")
+    light, heavy = 128 * 80, 3
+    n = light + heavy
+    rng = np.random.default_rng(3)
+    deg = np.concatenate([np.full(light, 8), np.full(heavy, n)])
+    ip = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(dev)
+    ix = torch.from_numpy(np.concatenate([rng.integers(0, n, light * 8), np.tile(np.arange(n), heavy)]).astype(np.int32)).to(dev)
+    v = torch.from_numpy((rng.random(int(deg.sum())) / np.repeat(deg, deg)).astype(np.float32)).to(dev)
+    sh = sharded.ShardedSpmm(ip, ix, v, 0, 1)
+    x = sh.to_block(synth.features(n, 128, 7, dev))
+    w = [synth.glorot(128, 128, 7, k, dev) for k in (1, 2)]
+    plain = gcn.GcnForward(sh, w)
+    want = plain.forward(x).clone()
+    monkeypatch.setenv("AGCN_GCN_FUSED", "1")
+    fused = gcn.GcnForward(sh, w)
+    scale = float(want.abs().max())
+    assert _captured_nodes(fused, x) > _captured_nodes(plain, x)
+    for _ in range(3):
+        got = fused.forward(x, out=torch.full_like(x, float("nan")))
+        assert float((got - want).abs().max()) <= 2e-3 * scale
+        assert torch.equal(plain.forward(x, out=torch.full_like(x, float("nan"))), want)
+    fused.status(); plain.status()
+    fused.close(); plain.close(); sh.close()
+
+
 def test_forward_with_fused_layer_boundary(monkeypatch):
     # AGCN_GCN_FUSED=1: the light rows of the block take the fused kernel between the layers, the others
     # SpMM + GEMM; the result must agree with the plain forward (same arithmetic, another summation order)
     import torch
     from accelgcn import synth, degree_sort, sharded, gcn
     dev = require_cuda()
+    monkeypatch.setenv("AGCN_SPMM_PIECE", "0")             # plans whose tuples are cut do without the fused kernel
     g = synth.make_config(5, dev, 0.002)
     _, ip, ix, v = degree_sort.degree_sort_device(g.indptr, g.indices, g.vals)
     x = synth.features(g.n, 128, 1005, dev)
@@ -284,14 +331,14 @@ def test_forward_with_fused_layer_boundary(monkeypatch):
     want = plain.forward(xb).clone()
     torch.cuda.synchronize()
     plain.status()
+    plain_nodes = _captured_nodes(plain, xb)
     plain.close()
     monkeypatch.setenv("AGCN_GCN_FUSED", "1")
     fused = gcn.GcnForward(sh, [w1, w2])
     got = fused.forward(xb)
     torch.cuda.synchronize()
     fused.status()
-    deg = (ip[1:] - ip[:-1])
-    assert int((deg <= 32).sum()) >= 128 * 64              # the fused path is really taken at this size
+    assert _captured_nodes(fused, xb) > plain_nodes        # the fused path is really taken at this size
     scale = float(want.abs().max())
     assert float((got - want).abs().max()) <= 2e-3 * scale
     fused.close(); sh.close()
