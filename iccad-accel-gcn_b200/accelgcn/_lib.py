@@ -40,6 +40,7 @@ PROTOTYPES = {
     "agcn_gemm_tf32": (_int, [_vp, _i64, _vp, _vp, _i64, _i64, _int, _int, _vp]),
     "agcn_spmm_plan_info": (_int, [_vp, ctypes.POINTER(_i64), ctypes.POINTER(_i64), ctypes.POINTER(_i64),
                                   ctypes.POINTER(_int)]),
+    "agcn_spmm_plan_hot_column": (_int, [_vp, _int, ctypes.POINTER(_i64)]),
     "agcn_host_ctx_create": (_int, [ctypes.POINTER(_vp)]),
     "agcn_host_ctx_destroy": (_int, [_vp]),
     "agcn_host_set_graph": (_int, [_vp, _vp, _i64, _vp, _vp, _i64, _i64, _i64]),

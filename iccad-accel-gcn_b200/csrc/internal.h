@@ -20,6 +20,7 @@ struct agcn_spmm_plan {
     int l2_bytes = 0, sm_count = 0;   // of the device the plan was created on
     int panel_override = 0;           // AGCN_SPMM_PANEL at creation (0 = choose automatically)
     bool never_split = false;         // set for the ranges of a column-tiled product
+    bool hot_tail = false;            // the last rows of X are named so often that L2 is better kept for them (uncut plans)
     int pad_unaligned = 1;            // AGCN_SPMM_PAD at creation: copy unaligned X into 16-byte-aligned rows
     float *x_pad = nullptr;           // [n_cols][dim rounded up to 4], grown on demand
     size_t x_pad_bytes = 0;
@@ -49,6 +50,8 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
                 int64_t n_rows, int64_t n_cols, int64_t nnz, cudaStream_t s);
 int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *d_x, int64_t ldx,
              float *d_y, int64_t ldy, int dim, cudaStream_t s, int activation = 0, int accumulate = 0);
+// First row of X that a pass of `width` columns keeps in L2 before the others; 0: all rows alike
+int64_t spmm_hot_column(const agcn_spmm_plan *p, int width);
 int spmm_check_run_args(const agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *d_x, int64_t ldx,
                         const float *d_y, int64_t ldy, int dim, int activation);
 int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cudaStream_t s,

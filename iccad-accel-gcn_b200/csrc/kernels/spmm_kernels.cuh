@@ -551,7 +551,9 @@ __device__ __forceinline__ bool tuple_is_big(const int4 &b) { return b.x > SPMM_
 __device__ __forceinline__ int tuple_rows(const int4 &b) { return tuple_is_big(b) ? 1 : (b.w & 0xffff); }
 
 // Error bits are single words of the host so that blocks can store to them without atomics.
-constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_FULL = 3, PLAN_WORD_ERR = 4;      // then one word per SPMM_ERR_* bit
+constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_FULL = 3;
+constexpr int PLAN_WORD_TAIL = PLAN_WORD_PIECES;            // uncut plans, which have no pieces
+constexpr int PLAN_WORD_ERR = 4;      // then one word per SPMM_ERR_* bit
 constexpr int PLAN_ERR_BITS = 4;
 constexpr int PLAN_FULL_NZ = 192;
 constexpr int PLAN_BLOCK = 256;      // units per thread block, one per thread
@@ -645,19 +647,44 @@ __device__ __forceinline__ void plan_check_ids(const int *__restrict__ idx, int6
     if (bad) plan_report(out, SPMM_ERR_COL);
 }
 
+// How many of PLAN_SAMPLES column ids, one from every PLAN_SAMPLES-th part of the nonzeros, are at least `first` (anywhere
+// in its part: at even distances it could always be the last, largest id of a row).  By one thread block.
+constexpr int PLAN_SAMPLE_ITEMS = 16, PLAN_SAMPLES = PLAN_BLOCK * PLAN_SAMPLE_ITEMS;
+
+__device__ __forceinline__ void plan_tail_share(const int *__restrict__ idx, int64_t n_idx, int64_t first, HostWords *out)
+{
+    const int64_t part = n_idx / PLAN_SAMPLES;
+    int count = 0;
+#pragma unroll
+    for (int k = 0; k < PLAN_SAMPLE_ITEMS; k++) {
+        const unsigned n = k * PLAN_BLOCK + threadIdx.x;
+        const int64_t within = part * (int64_t)(n * 2654435769u >> 8) >> 24;
+        count += n_idx > 0 && __ldg(idx + n * part + within) >= first;
+    }
+    __shared__ int s_sum;
+    if (threadIdx.x == 0) s_sum = 0;
+    __syncthreads();
+    count = warp_reduce(count, OpAdd());
+    if (lane_id() == 0) atomicAdd(&s_sum, count);
+    __syncthreads();
+    if (threadIdx.x == 0) out->w[PLAN_WORD_TAIL] = s_sum;
+}
+
 // First pass over a `.block4` array: validates every tuple (and, in the blocks behind the tuple blocks,
 // every column id), and counts per PLAN_BLOCK units the rows no tuple covers and the carry slots.  One
 // launch and one read of 16 bytes per tuple and 4 per nonzero: bound by HBM for large graphs, by launch
 // latency for small ones.  ctl[0..2]: totals (the third: tuples of at least PLAN_FULL_NZ nonzeros), ctl[3]: blocks
-// done (zero at launch).
+// done (zero at launch).  tail_first >= 0: the first block behind the tuple blocks samples the column ids from there on.
 __global__ void __launch_bounds__(PLAN_BLOCK)
 plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_units, int64_t n_rows, int64_t nnz,
-                  const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned unit_grid,
+                  const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned unit_grid, int64_t tail_first,
                   int64_t *__restrict__ tile_zero, int *__restrict__ tile_carry, unsigned long long *__restrict__ ctl,
                   HostWords *out)
 {
     if (blockIdx.x >= unit_grid) {
-        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - unit_grid, gridDim.x - unit_grid, out);
+        const unsigned asked = tail_first >= 0 ? 1 : 0;
+        if (blockIdx.x - unit_grid < asked) plan_tail_share(idx, n_idx, tail_first, out);
+        else plan_check_ids(idx, n_idx, n_cols, blockIdx.x - unit_grid - asked, gridDim.x - unit_grid - asked, out);
         return;
     }
     __shared__ int64_t s_zero[PLAN_BLOCK / 32];

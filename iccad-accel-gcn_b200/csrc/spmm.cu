@@ -69,13 +69,22 @@ static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
     return p->n_full > (int64_t)SPMM_MIN_BLOCKS * SPMM_WARPS * p->sm_count && 10 * p->n_full <= (int64_t)49 * SPMM_WARPS * p->sm_count;
 }
 
-// Columns whose rows of X are to stay in L2 when X is many times larger: the last ones, which in a symmetric graph in
-// degree order are named most often.  45 % of L2 (each half of the GPU keeps its own copy of what it reads).
-// 0 = all alike: below 6x L2 that is as fast or faster.  (X / L2 = 9, 14, 19 at dim 128: -3, -4, -4.5 %.)
-static int64_t spmm_hot_column(const agcn_spmm_plan *p, int width)
+// Columns whose rows of X are to stay in L2 when X is many times larger: the last ones, 45 % of L2 (each half of the
+// GPU keeps its own copy of what it reads), where they are named often enough: in a symmetric graph with columns in
+// degree order they are.  0 = all alike.  Dim 128, time with / without:
+// degree order, X / L2 = 9, 19: window named by 50, 42 % of the nonzeros: -3, -3 %; dim 64..96, X / L2 = 4.6, 5.8,
+// 6.2, 6.9: +0.7, +0.5, +0.2, +0.2 %, hence the 6x;
+// popular rows anywhere: window named by 3, 13, 23, 32, 42, 52 %: +18, +9, +3, -0.2, -2, -3 %, hence the share of a
+// third; uniform columns: 5, 14, 24, 33, 43 %: +4, -3, -8, -12, -13 %;
+// row blocks of 2, 4, 8 ranks, whose last rows are the middle of the degree order: 14, 6, 5 %: +7, +12, +11 %.
+constexpr double SPMM_HOT_X = 6.0, SPMM_HOT_L2 = 0.45, SPMM_HOT_SHARE = 0.33;
+
+static int64_t hot_rows(const agcn_spmm_plan *p, int width) { return (int64_t)(SPMM_HOT_L2 * p->l2_bytes / (width * 4.0)); }
+
+int64_t spmm_hot_column(const agcn_spmm_plan *p, int width)
 {
-    if ((double)p->n_cols * width * 4.0 < 6.0 * p->l2_bytes) return 0;
-    return p->n_cols - (int64_t)(0.45 * p->l2_bytes / (width * 4.0));
+    if (!p->hot_tail || (double)p->n_cols * width * 4.0 < SPMM_HOT_X * p->l2_bytes) return 0;
+    return p->n_cols - hot_rows(p, width);
 }
 
 bool spmm_plan_splits(int64_t n_blocks, int64_t n_rows, int64_t nnz)
@@ -185,9 +194,11 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     AGCN_CUDA(cudaMemsetAsync(ctl, 0, 4 * sizeof(*ctl), s));
     // 16 column ids per thread, at most 64 thread blocks per SM's worth of them
     const int64_t col_grid = n_idx > 0 ? ceil_div(n_idx, PLAN_BLOCK * 16) : 0;
-    const unsigned grid = (unsigned)(tiles + (col_grid < 9472 ? col_grid : 9472));
+    // the widest pass has the narrowest window: where that one is named often enough, so are the others
+    const bool ask_tail = n_idx > 0 && (double)p->n_cols * SPMM_PANEL * 4.0 >= SPMM_HOT_X * p->l2_bytes;
+    const unsigned grid = (unsigned)(tiles + (ask_tail ? 1 : 0) + (col_grid < 9472 ? col_grid : 9472));
     AGCN_KERNEL(plan_check_kernel, grid, PLAN_BLOCK, s, p->block4, p->n_blocks, p->n_units, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols,
-                (unsigned)tiles, tile_zero, tile_carry, ctl, words.device());
+                (unsigned)tiles, ask_tail ? p->n_cols - hot_rows(p, SPMM_PANEL) : (int64_t)-1, tile_zero, tile_carry, ctl, words.device());
     AGCN_LAUNCH_CHECK("plan_check_kernel");
     AGCN_CUDA(words.sync());
     int rc = plan_errors(words);
@@ -195,6 +206,7 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     p->n_zero = words[PLAN_WORD_ZERO];
     p->n_carry = words[PLAN_WORD_CARRY];
     p->n_full = words[PLAN_WORD_FULL];
+    p->hot_tail = ask_tail && (double)words[PLAN_WORD_TAIL] >= SPMM_HOT_SHARE * PLAN_SAMPLES;
     int4 *pieces = nullptr;
     rc = plan_memory(p, 0, &pieces, s);
     if (rc != AGCN_OK) return rc;
@@ -501,5 +513,13 @@ extern "C" int agcn_spmm_plan_info(const agcn_spmm_plan *plan, int64_t *n_units,
     if (n_carry) *n_carry = plan->n_carry;
     if (n_zero_rows) *n_zero_rows = plan->n_zero;
     if (launches_last_run) *launches_last_run = plan->launches_last_run;
+    return AGCN_OK;
+}
+
+extern "C" int agcn_spmm_plan_hot_column(const agcn_spmm_plan *plan, int width, int64_t *column)
+{
+    agcn::clear_error();
+    AGCN_REQUIRE(plan != nullptr && column != nullptr && width >= 1 && width <= agcn::SPMM_PANEL, "agcn_spmm_plan_hot_column: null argument, or width outside 1..128");
+    *column = agcn::spmm_hot_column(plan, width);
     return AGCN_OK;
 }

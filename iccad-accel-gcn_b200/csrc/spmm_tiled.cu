@@ -116,7 +116,8 @@ static int tiled_create(agcn_spmm_tiled **out, const int *d_indptr, const int *d
         t->n_blocks[k] = nb;
         rc = spmm_create(&t->plan[k], t->block4[k], nb, nnz_k > 0 ? t->idx + t->first[k] : nullptr, n_rows, n_cols, nnz_k, s);
         if (rc != AGCN_OK) return rc;
-        t->plan[k]->never_split = true;      // a range's slab stays in L2 by construction: no column passes
+        t->plan[k]->never_split = true;      // a range's slab stays in L2 by construction: no column passes,
+        t->plan[k]->hot_tail = false;        // and no row of it before another
     }
     guard.t = nullptr;
     *out = t;

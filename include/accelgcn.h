@@ -181,6 +181,11 @@ int agcn_spmm_destroy(agcn_spmm_plan *plan);
 int agcn_spmm_plan_info(const agcn_spmm_plan *plan, int64_t *n_units, int64_t *n_carry,
                         int64_t *n_zero_rows, int *launches_last_run);
 
+/* Where X is several times larger than L2 and a third or more of the nonzeros name its last rows (a graph in degree
+ * order with renamed columns), those rows are kept in L2 before the others.  *column receives the first of them for a
+ * pass of `width` (1..128) columns, 0 where all rows are treated alike (for reporting). */
+int agcn_spmm_plan_hot_column(const agcn_spmm_plan *plan, int width, int64_t *column);
+
 /* ------------------------------------------------------------------------
  * Column-tiled SpMM.  No counterpart in the reference, whose kernel gathers X
  * un-tiled (spmm_accel.cu:55-78).  The gather runs at L2 speed only while the

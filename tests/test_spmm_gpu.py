@@ -548,6 +548,45 @@ def test_unaligned_widths_padded_copy_equals_scalar_path(cfg4_small, dim, monkey
     assert spmm_close(y_pad, y_scalar, row_abs_scale(cfg4_small.indptr, cfg4_small.val, x)).all()
 
 
+def test_rows_of_x_kept_in_l2_are_rows_that_are_named_often():
+    # the last rows of an X many times larger than L2 go before the others only where the nonzeros name them: not in a
+    # matrix with columns in any order, not below 6x L2, not where the plan has not seen the column ids
+    import ctypes
+    import torch
+    from accelgcn import spmm, partition, _lib
+    dev = require_cuda()
+    lib = _lib.load()
+    l2 = torch.cuda.get_device_properties(dev).L2_cache_size
+    n, mean = 2_400_000, 12
+    window = int(0.45 * l2 / 512)
+    indptr = torch.arange(0, (n + 1) * mean, mean, dtype=torch.int32, device=dev)
+    block4 = partition.block_level_partition_device(indptr)
+    gen = torch.Generator(device=dev).manual_seed(1)
+    anywhere = torch.randint(0, n, (n * mean,), device=dev, generator=gen, dtype=torch.int32)
+
+    def hot(ids, width, n_cols=n, known=True):
+        col, h = ctypes.c_int64(-1), ctypes.c_void_p()
+        _lib.check(lib.agcn_spmm_create(ctypes.byref(h), block4.data_ptr(), block4.shape[0], ids.data_ptr() if known else None, n, n_cols,
+                                        n * mean, None))
+        _lib.check(lib.agcn_spmm_plan_hot_column(h, width, ctypes.byref(col)))
+        _lib.check(lib.agcn_spmm_destroy(h))
+        return col.value
+
+    assert hot(anywhere, 128) == 0
+    for share, want in ((0.25, False), (0.42, True), (0.9, True)):
+        # by row, as sorted rows have it: the last ids of a row are the largest
+        tail = torch.rand((n, mean), device=dev, generator=gen) < share
+        ids = torch.where(tail, (n - window + torch.randint(0, window, (n, mean), device=dev, generator=gen)).int(), anywhere.view(n, mean))
+        ids = ids.sort(dim=1).values.contiguous()
+        assert (hot(ids, 128) > 0) == want, share
+        if want:
+            assert hot(ids, 128) == n - window and 0 < hot(ids, 100) < n - window
+            assert hot(ids, 64) == 0 or n * 64 * 4 >= 6 * l2          # the threshold is in bytes of the pass
+            assert hot(ids, 128, known=False) == 0
+            assert hot(ids, 128, n_cols=2 ** 31 - 2) == 0             # then the last rows are others
+        del ids, tail
+
+
 def test_product_that_starts_under_the_copy_of_x_reads_the_new_x(cfg1, cfg4_small):
     # with unaligned rows the product is resident while the copy of X it reads is still being written: X changes from
     # run to run, and every run must equal, bit for bit, the product of the same X in aligned rows
