@@ -129,6 +129,8 @@ struct HostWords {
     int64_t w[COUNT];
 };
 
+int host_words_chunks();          // how many pinned chunks of them there are
+
 class HostWordsLease {
 public:
     explicit HostWordsLease(cudaStream_t s);

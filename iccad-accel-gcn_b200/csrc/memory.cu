@@ -72,17 +72,21 @@ cudaError_t pool_free_waiting(void *p, int device)
 }
 
 // ---------------------------------------------------------------------------
-// Host words: pinned, mapped, 64 bytes each, kept in a free list.  A kernel stores its result or error
+// Host words: pinned, mapped, 128 bytes each with their link, kept in a free list.  A kernel stores its result or error
 // code straight into one and the host reads it after the stream synchronisation it needs anyway, in place
 // of a device word, a memset and a device-to-host copy.
 // ---------------------------------------------------------------------------
-constexpr int HOST_WORDS_PER_CHUNK = 64;      // one 4 KiB page; more chunks only if more calls run at once
+constexpr int HOST_WORDS_PER_CHUNK = 64;      // 8 KiB; more chunks only if more calls run at once
 
 struct HostWordsNode {
     HostWords words;
     HostWordsNode *next;
     char pad[64 - (sizeof(HostWords) + sizeof(HostWordsNode *)) % 64];
 };
+static_assert(sizeof(HostWordsNode) == 128, "as the comments say");
+
+static int g_words_chunks = 0;
+int host_words_chunks() { return g_words_chunks; }
 
 static std::mutex g_words_mutex;
 static HostWordsNode *g_words_free = nullptr;
@@ -93,6 +97,7 @@ HostWordsLease::HostWordsLease(cudaStream_t s) : s_(s)
     if (g_words_free == nullptr) {
         void *chunk = nullptr;
         if (cudaHostAlloc(&chunk, HOST_WORDS_PER_CHUNK * sizeof(HostWordsNode), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return;
+        g_words_chunks++;
         HostWordsNode *n = static_cast<HostWordsNode *>(chunk);
         for (int i = 0; i < HOST_WORDS_PER_CHUNK; i++) { n[i].next = g_words_free; g_words_free = &n[i]; }
     }

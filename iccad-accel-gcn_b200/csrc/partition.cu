@@ -20,6 +20,7 @@ struct PartScratch {
     PartTileInfo *info;
     int *tile_head;
     int64_t *tile_offset;
+    HostWords *words = nullptr;    // on the device: where the answer is stored instead of in leased host words
 };
 
 static PartScratch part_scratch(Carver &c, int64_t tiles)
@@ -40,30 +41,45 @@ static int partition_check(const char *who, const int *d_indptr, int64_t n_rows,
     return AGCN_OK;
 }
 
-static int partition_answer(const char *who, HostWordsLease &words, int64_t *n_blocks)
+static int partition_answer(const char *who, int64_t negative, int64_t total, int64_t *n_blocks)
 {
-    AGCN_CUDA(words.sync());
-    if (words[PART_WORD_NEGATIVE] != 0) {
+    if (negative != 0) {
         set_error("%s: indptr decreases somewhere (negative degree); "
                   "the reference script prints 'cur_degree number is wrong' and stops", who);
         return AGCN_ERR_RANGE;
     }
-    *n_blocks = words[PART_WORD_TOTAL];
+    *n_blocks = total;
     return AGCN_OK;
 }
 
 // Phases A and B: how many tuples there are and where every tile's begin.  Waits for the stream.
 // `who` names the entry point in error messages.
-static int partition_count(const char *who, const int *d_indptr, int64_t n_rows, int64_t *n_blocks, const PartScratch &sc, cudaStream_t s)
+static int partition_launch_count(const int *d_indptr, int64_t n_rows, const PartScratch &sc, HostWords *words, cudaStream_t s)
 {
     const int64_t tiles = ceil_div(n_rows, PART_TILE);
-    AGCN_HOST_WORDS(words, s);
-    AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words.device());
+    AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words);
     AGCN_LAUNCH_CHECK("part_describe_kernel");
-    AGCN_CUDA(launch_early(true, part_scan_kernel, 1, PART_SCAN_BLOCK, 0, s, (const PartTileInfo *)sc.info, tiles, sc.tile_head, sc.tile_offset,
-                           words.device()));
+    AGCN_CUDA(launch_early(true, part_scan_kernel, 1, PART_SCAN_BLOCK, 0, s, (const PartTileInfo *)sc.info, tiles, sc.tile_head, sc.tile_offset, words));
     AGCN_LAUNCH_CHECK("part_scan_kernel");
-    return partition_answer(who, words, n_blocks);
+    return AGCN_OK;
+}
+
+static int partition_count(const char *who, const int *d_indptr, int64_t n_rows, int64_t *n_blocks, const PartScratch &sc, cudaStream_t s)
+{
+    if (sc.words != nullptr) {
+        HostWords words;
+        AGCN_CUDA(cudaMemsetAsync(sc.words, 0, sizeof(words), s));
+        const int rc = partition_launch_count(d_indptr, n_rows, sc, sc.words, s);
+        if (rc != AGCN_OK) return rc;
+        AGCN_CUDA(cudaMemcpyAsync(&words, sc.words, sizeof(words), cudaMemcpyDeviceToHost, s));
+        AGCN_CUDA(cudaStreamSynchronize(s));
+        return partition_answer(who, words.w[PART_WORD_NEGATIVE], words.w[PART_WORD_TOTAL], n_blocks);
+    }
+    AGCN_HOST_WORDS(words, s);
+    const int rc = partition_launch_count(d_indptr, n_rows, sc, words.device(), s);
+    if (rc != AGCN_OK) return rc;
+    AGCN_CUDA(words.sync());
+    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
 }
 
 // Phases A and C of a graph of few tiles, into scratch of `cap` tuples; *n_blocks may come out larger than that.
@@ -77,7 +93,8 @@ static int partition_direct(const char *who, const int *d_indptr, int64_t n_rows
     AGCN_CUDA(launch_early(true, part_emit_kernel, tiles, PART_BLOCK, 0, s, d_indptr, n_rows, (const PartTileInfo *)sc.info, (const int *)nullptr,
                            (const int64_t *)nullptr, cap, tuples, words.device()));
     AGCN_LAUNCH_CHECK("part_emit_kernel");
-    return partition_answer(who, words, n_blocks);
+    AGCN_CUDA(words.sync());
+    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
 }
 
 // Phase C, asynchronous.
@@ -253,8 +270,9 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
 // fails or steals from its pool), a latency-critical loop that cannot afford
 // the device-wide synchronisation cudaMalloc / cudaFree imply, or a plug-in
 // host that forbids allocation calls after start-up.  For them the tile
-// scratch of the partitioner (28 bytes per 2048 rows) lives in a fixed array in the
-// library's device image instead of a per-call allocation.  Every GPU that
+// scratch of the partitioner (28 bytes per 2048 rows) and its result words live in a
+// fixed array in the library's device image instead of a per-call allocation or leased
+// host words (which are pinned when there are none free).  Every GPU that
 // loads the library holds that array (about 224 KB) until the process exits,
 // which is why it is sized for AGCN_PARTITION_NOALLOC_MAX_ROWS rows and no
 // more.
@@ -272,7 +290,7 @@ constexpr int64_t PART_NOALLOC_MAX_ROWS = AGCN_PARTITION_NOALLOC_MAX_ROWS;
 constexpr int64_t PART_NOALLOC_MAX_TILES = (PART_NOALLOC_MAX_ROWS + PART_TILE - 1) / PART_TILE;
 constexpr int PART_NOALLOC_MAX_DEVICES = 64;
 
-constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + sizeof(int64_t) + sizeof(int)) + 3 * 256;
+constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + sizeof(int64_t) + sizeof(int)) + 3 * 256 + 256;
 
 }  // namespace agcn
 
@@ -315,8 +333,10 @@ static int partition_device_noalloc(const int *d_indptr, int64_t n_rows, int *d_
     int rc = part_static_scratch(&memory);
     if (rc != AGCN_OK) return rc;
     Carver c(memory);
-    return partition_pipeline("agcn_partition_device_noalloc", d_indptr, n_rows, d_block4, cap_blocks, n_blocks,
-                              part_scratch(c, ceil_div(n_rows, PART_TILE)), s);
+    HostWords *words = c.take<HostWords>(1);
+    PartScratch sc = part_scratch(c, ceil_div(n_rows, PART_TILE));
+    sc.words = words;
+    return partition_pipeline("agcn_partition_device_noalloc", d_indptr, n_rows, d_block4, cap_blocks, n_blocks, sc, s);
 }
 
 }  // namespace agcn

@@ -110,3 +110,28 @@ def test_noalloc_partition_leaves_free_device_memory_unchanged():
         assert torch.cuda.mem_get_info(dev)[0] == free_before
     torch.cuda.synchronize()
     assert torch.cuda.mem_get_info(dev)[0] == free_before
+
+
+def test_noalloc_partition_pins_no_host_memory():
+    # in a process of its own: the other entry points store their results in pinned words, which are allocated when
+    # none is free; this one may not
+    import subprocess
+    import sys
+    from conftest import PKG
+    require_cuda()
+    program = """
+import ctypes, sys, torch
+sys.path.insert(0, sys.argv[1])
+from accelgcn import _lib
+lib = _lib.load()
+chunks = lib["_ZN4agcn17host_words_chunksEv"]
+ip = torch.arange(0, 4 * 5001, 4, dtype=torch.int32, device="cuda")
+out = torch.empty((5000, 4), dtype=torch.int32, device="cuda")
+n = ctypes.c_int64(0)
+for _ in range(2):
+    _lib.check(lib.agcn_partition_device_noalloc(ip.data_ptr(), 5000, out.data_ptr(), 5000, ctypes.byref(n), None))
+    assert n.value == (5000 + 11) // 12 and chunks() == 0
+_lib.check(lib.agcn_partition_device(ip.data_ptr(), 5000, out.data_ptr(), 5000, ctypes.byref(n), None))
+assert chunks() == 1
+"""
+    subprocess.run([sys.executable, "-c", program, PKG], check=True, timeout=300)
