@@ -115,12 +115,13 @@ extern "C" int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_i
     using namespace agcn;
     clear_error();
     AGCN_REQUIRE(h_indptr != nullptr && h_perm != nullptr, "agcn_degree_sort_host: null indptr or perm");
-    AGCN_REQUIRE(n_rows > 0 && nnz >= 0, "agcn_degree_sort_host: bad sizes");
+    AGCN_REQUIRE(n_rows > 0 && n_rows < (int64_t)INT32_MAX && nnz >= 0 && nnz <= (int64_t)INT32_MAX, "agcn_degree_sort_host: bad sizes");
     const bool want_idx = h_new_indices != nullptr, want_val = h_new_vals != nullptr;
     AGCN_REQUIRE(!want_idx || (h_indices != nullptr && h_new_indptr != nullptr), "agcn_degree_sort_host: new_indices needs indices and new_indptr");
     AGCN_REQUIRE(!want_val || (h_vals != nullptr && want_idx), "agcn_degree_sort_host: new_vals needs vals and new_indices");
     const cudaStream_t s = nullptr;
     DeviceScratch scratch(s);
+    const WaitOnExit drain(s);
     unsigned char *block = nullptr;
     int *d_indptr = nullptr, *d_perm = nullptr, *d_new_indptr = nullptr, *d_indices = nullptr, *d_new_indices = nullptr;
     float *d_vals = nullptr, *d_new_vals = nullptr;

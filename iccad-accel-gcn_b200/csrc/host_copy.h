@@ -11,10 +11,22 @@ struct HostSegment {
 };
 constexpr int HOST_SEGMENTS_MAX = 4;
 
-// Host arrays may be reused when these return; the device side is ordered on `s`.  Downloads are complete.
+// Pageable arrays may be reused when host_upload returns, pinned ones when `s` has been waited for (WaitOnExit); the
+// device side is ordered on `s`.  Downloads are complete.
 // `outputs`: arrays a later host_download fills, whose pages may be faulted in meanwhile.
 int host_upload(const HostSegment *seg, int n, cudaStream_t s, const HostSegment *outputs = nullptr, int n_outputs = 0);
 int host_download(const HostSegment *seg, int n, cudaStream_t s);
+// Waits for `s` when a call that uploads ends, however it ends: the caller's arrays are the caller's again.
+class WaitOnExit {
+public:
+    explicit WaitOnExit(cudaStream_t s) : s_(s) {}
+    ~WaitOnExit() { cudaStreamSynchronize(s_); }
+    WaitOnExit(const WaitOnExit &) = delete;
+    WaitOnExit &operator=(const WaitOnExit &) = delete;
+private:
+    cudaStream_t s_;
+};
+
 // gives the pinned buffers back
 void host_copy_release();
 

@@ -236,9 +236,11 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
     AGCN_REQUIRE(h_indptr != nullptr && n_blocks != nullptr, "agcn_partition_host: null pointer");
     AGCN_REQUIRE(n_rows > 0, "agcn_partition_host: empty graph (n_rows = %lld); the reference script raises IndexError here",
                  (long long)n_rows);
+    AGCN_REQUIRE(n_rows < (int64_t)INT32_MAX, "agcn_partition_host: n_rows = %lld does not fit the int32 row ids of .block4", (long long)n_rows);
     *n_blocks = 0;
     const cudaStream_t s = nullptr;
     DeviceScratch scratch(s);
+    const WaitOnExit drain(s);
     AGCN_ALLOC(d_indptr, scratch, int, n_rows + 1);
     const HostSegment up = {d_indptr, const_cast<int *>(h_indptr), (size_t)(n_rows + 1) * sizeof(int)};
     int rc = host_upload(&up, 1, s);

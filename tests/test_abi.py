@@ -53,6 +53,11 @@ def test_argument_errors_need_no_gpu():
     ip = np.zeros(1, dtype=np.int32)
     assert lib.agcn_partition_host(ip.ctypes.data, 0, None, 0, ctypes.byref(n)) == _lib.ERR_INVALID
     assert b"empty graph" in lib.agcn_last_error()
+    perm = np.zeros(1, dtype=np.int32)
+    for big in (2 ** 31 - 1, 2 ** 40):                 # sizes that no array of these has: found before one is read
+        assert lib.agcn_partition_host(ip.ctypes.data, big, None, 0, ctypes.byref(n)) == _lib.ERR_INVALID
+        assert lib.agcn_degree_sort_host(ip.ctypes.data, None, None, big, 0, 0, perm.ctypes.data, None, None, None) == _lib.ERR_INVALID
+    assert lib.agcn_degree_sort_host(ip.ctypes.data, None, None, 1, 2 ** 31, 0, perm.ctypes.data, None, None, None) == _lib.ERR_INVALID
     assert lib.agcn_spmm_run(None, None, None, None, 0, None, 0, 4, None) == _lib.ERR_INVALID
 
 
