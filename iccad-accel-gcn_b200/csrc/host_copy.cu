@@ -9,8 +9,8 @@
 
 #include <atomic>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
 #include <thread>
 
 namespace agcn {
@@ -163,13 +163,14 @@ static int host_copy(const HostSegment *seg, int n, bool up, cudaStream_t s, con
         for (; job.n_touch > 0 && cores > TOUCH_THREADS && touching < TOUCH_THREADS; touching++) touchers[touching] = std::thread([&job] { job.touch_outputs(); });
         for (; started < threads; started++)
             pool[started] = std::thread([&job, started] { job.work(g_stage.memory + (size_t)started * 2 * STAGE_PIECE); job.touch_outputs(); });
-    } catch (const std::system_error &) {
-        // fewer threads than asked for: the ones that run share the pieces
+    } catch (const std::exception &) {
+        // fewer threads than asked for (no thread or no memory for one): the ones that run share the pieces
     }
     job.work(g_stage.memory);
     for (int t = 1; t < started; t++) pool[t].join();
     for (int t = 0; t < touching; t++) touchers[t].join();
     const cudaError_t e = (cudaError_t)job.error.load();
+    if (e != cudaSuccess) cudaStreamSynchronize(s);      // copies of other threads may still use the buffers the next call gets
     AGCN_CUDA(e);
     return AGCN_OK;
 }

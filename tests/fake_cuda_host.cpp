@@ -9,7 +9,9 @@
 #include <cstring>
 #include <map>
 #include <mutex>
+#include <new>
 #include <string>
+#include <vector>
 
 static int failures = 0;
 #define CHECK(cond) do { if (!(cond)) { std::printf("%s:%d: %s\n", __FILE__, __LINE__, #cond); failures++; } } while (0)
@@ -24,6 +26,9 @@ int g_syncs[2] = {0, 0};                                 // device-wide waits
 int g_wrong_device = 0;                                  // frees, allocations or copies on a stream of another device
 int g_fail_free = 0;
 bool g_capturing = false;
+std::atomic<int> g_copies{0}, g_copies_waited_for{0};    // copies issued; how many of them the last stream wait covered
+int g_fail_copy = 0;                                     // number of the copy that fails
+thread_local int t_news_left = -1;                       // allocations of this thread until one fails
 
 int stream_device(cudaStream_t s)
 {
@@ -80,7 +85,7 @@ cudaError_t cudaStreamIsCapturing(cudaStream_t, cudaStreamCaptureStatus *st)
     return cudaSuccess;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
-cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+cudaError_t cudaStreamSynchronize(cudaStream_t) { g_copies_waited_for = g_copies.load(); return cudaSuccess; }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
 cudaError_t cudaEventCreate(cudaEvent_t *e) { return event_of(e); }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t *e, unsigned) { return event_of(e); }
@@ -89,8 +94,22 @@ cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t s) { if (stream_device(s) 
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
 cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t, cudaEvent_t) { *ms = 0.f; return cudaSuccess; }
 cudaError_t cudaMemsetAsync(void *p, int v, size_t n, cudaStream_t) { std::memset(p, v, n); return cudaSuccess; }
-cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t) { std::memcpy(d, s, n); return cudaSuccess; }
+cudaError_t cudaMemcpyAsync(void *d, const void *s, size_t n, cudaMemcpyKind, cudaStream_t)
+{
+    if (++g_copies == g_fail_copy) return cudaErrorUnknown;
+    std::memcpy(d, s, n);
+    return cudaSuccess;
 }
+}
+
+// ---- allocations that fail ---------------------------------------------------------------------
+void *operator new(size_t bytes)
+{
+    if (t_news_left >= 0 && t_news_left-- == 0) throw std::bad_alloc();
+    return std::malloc(bytes > 0 ? bytes : 1);
+}
+void operator delete(void *p) noexcept { std::free(p); }
+void operator delete(void *p, size_t) noexcept { std::free(p); }
 
 // ---- what the sources under test call in the others --------------------------------------------
 namespace agcn {
@@ -176,11 +195,42 @@ static void pool_under_capture()
     CHECK(g_block_device.empty());
 }
 
+// A copy that fails on one of several threads: the call fails, and by then nothing uses the shared buffers any more.
+static void staged_copy_fails()
+{
+    std::vector<unsigned char> src(64 << 20, 7), dst(64 << 20, 0);
+    const agcn::HostSegment seg = {dst.data(), src.data(), src.size()};
+    for (const int k : {1, 9, 40}) {
+        g_copies = 0; g_copies_waited_for = 0; g_fail_copy = k;
+        CHECK(agcn::host_upload(&seg, 1, nullptr) == AGCN_ERR_CUDA);
+        CHECK(g_copies >= k && g_copies_waited_for == g_copies);
+    }
+    g_fail_copy = 0;
+    CHECK(agcn::host_upload(&seg, 1, nullptr) == AGCN_OK);
+    CHECK(src == dst);
+}
+
+// No memory for the k-th thread: the call goes on with those that run, and no exception leaves it.
+static void staged_copy_without_threads()
+{
+    std::vector<unsigned char> src(64 << 20, 9), dst(64 << 20), out(8 << 20, 1);
+    const agcn::HostSegment seg = {dst.data(), src.data(), src.size()}, touched = {dst.data(), out.data(), out.size()};
+    for (int k = 0; k < 18; k++) {
+        std::memset(dst.data(), 0, dst.size());
+        t_news_left = k;
+        const int rc = agcn::host_upload(&seg, 1, nullptr, &touched, 1);
+        t_news_left = -1;
+        CHECK(rc == AGCN_OK && src == dst && out[12345] == 1);
+    }
+}
+
 int main(int argc, char **argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
     if (what == "context_device") context_device();
     else if (what == "pool_under_capture") pool_under_capture();
+    else if (what == "staged_copy_fails") staged_copy_fails();
+    else if (what == "staged_copy_without_threads") staged_copy_without_threads();
     else { std::printf("unknown scenario\n"); return 2; }
     std::printf("%d failures\n", failures);
     return failures != 0;

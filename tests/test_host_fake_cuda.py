@@ -18,7 +18,7 @@ def program(tmp_path_factory):
     return exe
 
 
-@pytest.mark.parametrize("scenario", ["context_device", "pool_under_capture"])
+@pytest.mark.parametrize("scenario", ["context_device", "pool_under_capture", "staged_copy_fails", "staged_copy_without_threads"])
 def test_scenario(program, scenario):
     out = subprocess.run([program, scenario], capture_output=True, text=True, timeout=120)
     assert out.returncode == 0, out.stdout + out.stderr
