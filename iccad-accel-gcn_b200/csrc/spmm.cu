@@ -61,6 +61,9 @@ static int spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int 
 // than 4 blocks per SM hold at once, the second round is a tail in which most of the GPU waits, and 5 blocks per SM
 // avoid it: dim 128, skewed rows, full blocks per SM and us at 4 / 5 blocks: 3.7: 52 / 57, 4.0: 78 / 63, 4.3: 79 / 63,
 // 4.5: 91 / 70, 4.9: 87 / 84, 5.1: 96 / 106, 6.1: 105 / 127.
+// Narrower passes gain as much or lose nothing, full blocks per SM and time at 5 / 4 blocks: 4.6 skewed, dim 16, 48, 64:
+// -10, -19, -19 %; 4.7 power law: -4, 0, 0 %; 4.8 skewed: -7, -9, -11 %; 4.9 skewed: -3, -3, -5 % (dim 96, 128: +2, +1 %);
+// 5.3 dense: +3, -2, -1 %; 5.7 skewed: +21, +18, +20 %; 5.8 dense: +12, +9, +10 %.
 // Also where all tuples are full and little more than half of a slot's 32 lanes have a column (139 000 rows of 456, dims
 // 68 and 80: 2 % faster, dim 96 already 3 % slower).
 static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
@@ -77,13 +80,14 @@ static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
 // popular rows anywhere: window named by 3, 13, 23, 32, 42, 52 %: +18, +9, +3, -0.2, -2, -3 %, hence the share of a
 // third; uniform columns: 5, 14, 24, 33, 43 %: +4, -3, -8, -12, -13 %;
 // row blocks of 2, 4, 8 ranks, whose last rows are the middle of the degree order: 14, 6, 5 %: +7, +12, +11 %.
+// (Passes of up to 32 columns were not measured and have no such kernel.)
 constexpr double SPMM_HOT_X = 6.0, SPMM_HOT_L2 = 0.45, SPMM_HOT_SHARE = 0.33;
 
 static int64_t hot_rows(const agcn_spmm_plan *p, int width) { return (int64_t)(SPMM_HOT_L2 * p->l2_bytes / (width * 4.0)); }
 
 int64_t spmm_hot_column(const agcn_spmm_plan *p, int width)
 {
-    if (!p->hot_tail || (double)p->n_cols * width * 4.0 < SPMM_HOT_X * p->l2_bytes) return 0;
+    if (!p->hot_tail || width <= 32 || (double)p->n_cols * width * 4.0 < SPMM_HOT_X * p->l2_bytes) return 0;
     return p->n_cols - hot_rows(p, width);
 }
 
@@ -286,13 +290,18 @@ static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmFor
     if (f.finish) {
         if (ALWAYS_WIDE || f.wide) launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, true>(prm, grid, f.plain, s);
         else if constexpr (!ALWAYS_WIDE) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, true>(prm, grid, f.plain, s);
-    } else if constexpr (ALWAYS_WIDE) {
+        return;
+    }
+    if constexpr (ALWAYS_WIDE) {
         launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false>(prm, grid, f.plain, s);
-    } else if constexpr (S >= 16) {
-        if (S == 32 && f.wide) launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false>(prm, grid, f.plain, s);
-        else if (prm.hot_column > 0) launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true>(prm, grid, f.plain, s);
-        else launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, f.plain, s);
     } else {
+        // launches of many blocks: the 5-block form above 64 columns only (constexpr: no other one is built)
+        if constexpr (S == 32) {
+            if (f.wide) { launch_units<S, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false>(prm, grid, f.plain, s); return; }
+        }
+        if constexpr (S >= 16) {
+            if (prm.hot_column > 0) { launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true>(prm, grid, f.plain, s); return; }
+        }
         launch_units<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false>(prm, grid, f.plain, s);
     }
 }

@@ -584,6 +584,10 @@ def test_rows_of_x_kept_in_l2_are_rows_that_are_named_often():
             assert hot(ids, 64) == 0 or n * 64 * 4 >= 6 * l2          # the threshold is in bytes of the pass
             assert hot(ids, 128, known=False) == 0
             assert hot(ids, 128, n_cols=2 ** 31 - 2) == 0             # then the last rows are others
+            # five times the columns, named at their end: passes of more than 32 columns have the kernel for it
+            far = torch.where(ids >= n - window, ids + 4 * n, ids)
+            assert 0 < hot(far, 64, n_cols=5 * n) < 5 * n and hot(far, 32, n_cols=5 * n) == 0
+            del far
         del ids, tail
 
 
