@@ -11,6 +11,7 @@ import functools
 import importlib.machinery
 import importlib.util
 import os
+import sysconfig
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 DEFAULT_LIB = os.path.join(os.path.dirname(_HERE), "lib", "libaccelgcn.so")
@@ -119,9 +120,9 @@ def call():
     ctypes.  No fallback: it is built with the library."""
     global _call
     if _call is None:
-        path = os.path.join(os.path.dirname(DEFAULT_LIB), "agcn_call.so")
+        path = os.path.join(os.path.dirname(DEFAULT_LIB), "agcn_call" + sysconfig.get_config_var("EXT_SUFFIX"))
         if not os.path.exists(path):
-            raise FileNotFoundError(f"{path} not found: build it with `python iccad-accel-gcn_b200/build.py`")
+            raise FileNotFoundError(f"{path} not found: build it with `python iccad-accel-gcn_b200/build.py` under this Python")
         loader = importlib.machinery.ExtensionFileLoader("agcn_call", path)
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("agcn_call", loader))
         loader.exec_module(module)

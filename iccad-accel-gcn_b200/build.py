@@ -42,11 +42,12 @@ def build_harness(force: bool = False) -> str:
     return HARNESS
 
 
-CALL = os.path.join(HERE, "lib", "agcn_call.so")
+# named for the interpreter it is built for, like any extension module: another one does not find it
+CALL = os.path.join(HERE, "lib", "agcn_call" + sysconfig.get_config_var("EXT_SUFFIX"))
 
 
 def build_call(force: bool = False) -> str:
-    """lib/agcn_call.so: the extension module through which the Python layer makes its hot calls."""
+    """The extension module through which the Python layer makes its hot calls."""
     src = os.path.join(HERE, "csrc", "pycall.c")
     if force or not os.path.exists(CALL) or os.path.getmtime(src) > os.path.getmtime(CALL):
         os.makedirs(os.path.dirname(CALL), exist_ok=True)

@@ -69,6 +69,19 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
         _lib.load()
 
 
+def test_native_caller_is_the_one_built_for_this_python(monkeypatch):
+    # a library folder built under another Python version holds a module of another name, which is not loaded
+    from accelgcn import _lib
+    _build()
+    monkeypatch.setattr(_lib, "_call", None)
+    lib = _lib.load()
+    assert _lib.call()(_lib.address("agcn_version")) == lib.agcn_version()
+    monkeypatch.setattr(_lib, "_call", None)
+    monkeypatch.setattr(_lib.sysconfig, "get_config_var", lambda name: ".cpython-399-x86_64-linux-gnu.so")
+    with pytest.raises(FileNotFoundError):
+        _lib.call()
+
+
 def test_host_partition_raises_on_empty_graph_like_the_script():
     from accelgcn import partition
     with pytest.raises(IndexError):
