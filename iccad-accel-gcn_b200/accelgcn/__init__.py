@@ -13,4 +13,4 @@ of libaccelgcn.so (include/accelgcn.h).
 PyTorch appears here only as the owner of device memory and streams (and of the
 process group in `sharded`); all compute is in the shared library.
 """
-from ._lib import AccelGcnError, load, lib_path  # noqa: F401
+from ._lib import AccelGcnError, load, lib_path, release_scratch  # noqa: F401

@@ -164,6 +164,12 @@ def device_index(device) -> int:
     return device.index if device.index is not None else torch.cuda.current_device()
 
 
+def release_scratch() -> None:
+    """Gives back what the library keeps between calls: the current device's scratch pool (up to 2 GB, which torch's
+    allocator does not see) and the pinned pieces of the host copies.  Waits for the device."""
+    check(load().agcn_release_scratch())
+
+
 def check(code: int) -> None:
     if code != OK:
         raise AccelGcnError(code, load().agcn_last_error().decode("utf-8", "replace"))

@@ -138,6 +138,24 @@ def test_tile_edges_and_number_of_passes(n, top, relabel):
         assert np.array_equal(a, b), what
 
 
+def test_release_scratch_gives_the_pool_back():
+    # between calls the library keeps scratch that no other allocator of the process can use
+    import torch
+    import accelgcn
+    from accelgcn import degree_sort
+    dev = require_cuda()
+    n = 4_000_000                                     # about 0.1 GB of scratch
+    indptr = torch.arange(0, 2 * (n + 1), 2, dtype=torch.int32, device=dev)
+    idx = torch.zeros(2 * n, dtype=torch.int32, device=dev)
+    keep = degree_sort.degree_sort_device(indptr, idx, None, relabel_cols=True)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info(dev)[0]
+    accelgcn.release_scratch()
+    assert torch.cuda.mem_get_info(dev)[0] >= before + 8 * n
+    again = degree_sort.degree_sort_device(indptr, idx, None, relabel_cols=True)      # and takes new scratch when it needs some
+    assert all(torch.equal(a, b) for a, b in zip(keep[:3], again[:3]))
+
+
 @pytest.mark.parametrize("n", [50_000, 200_000])
 def test_two_graphs_in_turn_in_the_same_scratch(n):
     # the permute is resident while the kernel before it writes the new names it looks up, into the memory in which
