@@ -44,12 +44,9 @@ class SpmmPlan:
 
     def run(self, indices, vals, x, y, dim: int | None = None, ldx: int | None = None, ldy: int | None = None,
             stream=None, relu: bool = False) -> None:
-        if dim is None:
-            dim = x.shape[1]
-        if ldx is None:
-            ldx = x.stride(0) if x.dim() == 2 else dim
-        if ldy is None:
-            ldy = y.stride(0) if y.dim() == 2 else dim
+        dim = x.shape[1] if dim is None else int(dim)
+        ldx = (x.stride(0) if x.dim() == 2 else dim) if ldx is None else int(ldx)
+        ldy = (y.stride(0) if y.dim() == 2 else dim) if ldy is None else int(ldy)
         # the library makes the plan's device current where it is not
         rc = self._call(self._run, self._h.value, indices.data_ptr(), vals.data_ptr(), x.data_ptr(), ldx, y.data_ptr(), ldy, dim,
                         1 if relu else 0, stream.cuda_stream if stream is not None else self._raw_stream(self._dev_index))

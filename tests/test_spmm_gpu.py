@@ -548,6 +548,21 @@ def test_unaligned_widths_padded_copy_equals_scalar_path(cfg4_small, dim, monkey
     assert spmm_close(y_pad, y_scalar, row_abs_scale(cfg4_small.indptr, cfg4_small.val, x)).all()
 
 
+def test_widths_and_strides_of_any_number_type(cfg1):
+    # what int() takes, as the call did before it went through the native caller
+    import torch
+    from accelgcn import spmm
+    c = cfg1
+    x = torch.from_numpy(c.x(32)).to(c.dev)
+    plan = spmm.SpmmPlan(c.t["block4"], c.t["idx"], c.n, c.n)
+    want, y = torch.empty((c.n, 32), device=c.dev), torch.empty((c.n, 32), device=c.dev)
+    plan.run(c.t["idx"], c.t["val"], x, want)
+    for number in (int, float, np.int32, np.float64, torch.tensor):
+        plan.run(c.t["idx"], c.t["val"], x, y.zero_(), dim=number(32), ldx=number(32), ldy=number(32))
+        assert torch.equal(y, want)
+    plan.close()
+
+
 def test_rows_of_x_kept_in_l2_are_rows_that_are_named_often():
     # the last rows of an X many times larger than L2 go before the others only where the nonzeros name them: not in a
     # matrix with columns in any order, not below 6x L2, not where the plan has not seen the column ids
