@@ -6,7 +6,7 @@
 
 namespace agcn {
 
-// Two launches up to 65 536 rows, a memset and five to eight above; one synchronisation at the end (15 to 25 launches, eight allocations and
+// Two launches up to 65 536 rows, a memset and four to seven above; one synchronisation at the end (15 to 25 launches, eight allocations and
 // two synchronisations before: 0.9 ms for 16 384 rows, most of it in the allocator).
 static int degree_sort_device(const int *d_indptr, const int *d_indices, const float *d_vals,
                               int64_t n_rows, int64_t nnz, int relabel_cols,

@@ -355,7 +355,7 @@ static int host_graph_and_products(agcn_host_ctx *c, const int *h_block4, int64_
         AGCN_REQUIRE(h_x[i] != nullptr && h_y[i] != nullptr && dims[i] >= 1, "agcn_spmm_host_batch: null X or Y, or dim < 1");
         stream_a = stream_a && can_issue_in_parts(dims[i]);
     }
-    if (!stream_a) {         // widths the unit-range launch does not take: graph first, then the products
+    if (!stream_a) {         // a width above 128 (or an empty graph): graph first, then the products
         rc = host_set_graph(c, h_block4, n_blocks, h_indices, h_vals, n_rows, n_cols, nnz);
         return rc != AGCN_OK ? rc : host_products(c, n, h_x, h_y, dims);
     }

@@ -68,7 +68,7 @@ extern "C" int agcn_probe_gather_bandwidth(int64_t table_rows, int row_floats, i
     AGCN_CUDA(cudaEventCreate(&e0));
     AGCN_CUDA(cudaEventCreate(&e1));
     // resident_blocks > 0: unused dynamic shared memory sized so that only that many thread blocks fit
-    // on an SM (the SpMM keeps 5); 0 = whatever the registers allow
+    // on an SM (the SpMM keeps 4); 0 = whatever the registers allow
     const size_t smem = resident_blocks == 0 ? 0 : (size_t)(220 * 1024 / resident_blocks) & ~(size_t)1023;
     if (smem > 48 * 1024) {
         AGCN_CUDA(cudaFuncSetAttribute(probe_gather_kernel<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));

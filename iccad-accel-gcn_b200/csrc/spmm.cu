@@ -329,7 +329,7 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
 // stride or base) would force 4-byte gathers: 1.2-1.6x the time of the 16-byte path.  Instead X
 // is copied once into plan-owned rows padded to a multiple of 4 floats (2 * n_cols * dim * 4
 // bytes of streaming traffic against nnz * dim * 4 bytes of gather) and the 16-byte path runs
-// on the copy; Y keeps the caller's layout and gets element-wise stores where it is unaligned.
+// on the copy; Y keeps the caller's layout and gets stores as wide as each row's alignment allows.
 // On return *x_use / *ldx_use name the operand to gather from and *x_vec says whether its rows
 // are 16-byte aligned.
 int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cudaStream_t s,

@@ -150,7 +150,7 @@ int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_indices, con
  * copied into plan-owned aligned rows (grown on demand: the first such call of
  * a width allocates, so make it before a stream capture, and the widest one
  * before the first capture: growing moves the rows; AGCN_SPMM_PAD=0 at plan creation selects 4-byte gathers
- * instead) and unaligned rows of Y get element-wise stores.  dim > 64 may run
+ * instead) and unaligned rows of Y get stores as wide as each row's alignment allows.  dim > 64 may run
  * as two 64-column passes when X is larger than L2 (environment variable
  * AGCN_SPMM_PANEL = columns per pass, read at plan creation, overrides that
  * choice).  Plans of few tuples hold a copy of them cut into pieces of 64 to 192
@@ -303,8 +303,8 @@ int agcn_spmm_host(agcn_host_ctx *ctx, const int32_t *h_block4, int64_t n_blocks
 /* agcn_host_set_graph + agcn_host_spmm_batch in one call, for a harness that hands over the
  * graph with every step.  Column ids and values go up in ranges of tuples, and every range is
  * multiplied for all products as soon as it has arrived, so kernels and downloads hide under
- * the upload of A (dims that are multiples of 4 up to 128; other widths upload first, then
- * multiply).  A column id outside [0, n_cols) is found by a check that runs ahead of each
+ * the upload of A (dims up to 128; with a wider one among them the graph is set first, then all
+ * are multiplied).  A column id outside [0, n_cols) is found by a check that runs ahead of each
  * range's kernels and stops them: the call returns AGCN_ERR_RANGE and the Y_i are undefined. */
 int agcn_spmm_host_batch(agcn_host_ctx *ctx, const int32_t *h_block4, int64_t n_blocks,
                          const int32_t *h_indices, const float *h_vals,
@@ -312,7 +312,7 @@ int agcn_spmm_host_batch(agcn_host_ctx *ctx, const int32_t *h_block4, int64_t n_
                          int n_products, const float *const *h_x, float *const *h_y, const int *dims);
 
 /* Where the time of the last agcn_spmm_host_batch call on this context went (the streamed form:
- * every width a multiple of 4 up to 128), in milliseconds from the start of its uploads:
+ * every width up to 128), in milliseconds from the start of its uploads:
  * ms6[0] last byte of A uploaded, [1] first kernel started, [2] last kernel finished, [3] last
  * byte of Y downloaded; host side: [4] until the plan was built, [5] until all was enqueued. */
 int agcn_host_last_timing(agcn_host_ctx *ctx, float *ms6);
@@ -426,7 +426,7 @@ int agcn_gcn2_forward_destroy(agcn_gcn2 *fwd);
  * is a power of two.
  * ---------------------------------------------------------------------- */
 int agcn_probe_gather_bandwidth(int64_t table_rows, int row_floats, int64_t total_rows, int iters,
-                                int resident_blocks /* per SM; 0 = no limit, the SpMM keeps 5 */,
+                                int resident_blocks /* per SM; 0 = no limit, the SpMM keeps 4 */,
                                 double *gb_per_s);
 
 #ifdef __cplusplus

@@ -704,13 +704,13 @@ def test_host_batch_and_streamed_graph(cfg1, cfg4_small):
         h = spmm.HostSpmm()
         dims = [32, 64, 128, 60, 33]
         xs = [np.ascontiguousarray(c.x(d)) for d in dims]
-        ys = h.step_batch(c.block4, c.idx, c.val, xs[:4], c.n)              # streamed (all widths multiples of 4)
+        ys = h.step_batch(c.block4, c.idx, c.val, xs[:4], c.n)              # streamed, in one range: these plans are cut
         for x, y in zip(xs[:4], ys):
             c.check(x, y)
         t = h.last_timing()                                                  # where the time of that call went
         assert 0 <= t["first_kernel_started"] <= t["last_kernel_finished"] <= t["last_y_downloaded"] + 1e-3
         assert t["a_uploaded"] > 0 and t["host_all_enqueued"] >= t["host_plan_built"] > 0
-        ys_all = h.step_batch(c.block4, c.idx, c.val, xs, c.n)              # 33 columns: upload first, then multiply
+        ys_all = h.step_batch(c.block4, c.idx, c.val, xs, c.n)              # 33 columns: through an aligned copy of X
         for x, y in zip(xs, ys_all):
             c.check(x, y)
         h.set_graph(c.block4, c.idx, c.val, c.n, c.n)
@@ -747,6 +747,18 @@ def test_streamed_graph_in_several_ranges_and_malformed_block4():
     c = Case(2, 0.2)
     assert len(c.idx) * 8 >> 25 >= 4
     h = spmm.HostSpmm()
+    # widths that are no multiple of 4 go through an aligned copy of X per product, made when that X has arrived; the
+    # products' ranges interleave and every one keeps its own partial sums
+    odd = [np.ascontiguousarray(c.x(d)) for d in (33, 64, 61)]
+    want = [c.run(x) for x in odd]
+    c.check(odd[2], want[2])
+    for y, w in zip(h.step_batch(c.block4, c.idx, c.val, odd, c.n), want):
+        assert np.array_equal(y, w)
+    t = h.last_timing()                                   # of the streamed form, whatever the widths: an error after another
+    assert 0 <= t["first_kernel_started"] <= t["last_kernel_finished"]
+    h.set_graph(c.block4, c.idx, c.val, c.n, c.n)
+    for y, w in zip(h.run_batch(odd), want):
+        assert np.array_equal(y, w)
     xs = [np.ascontiguousarray(c.x(d)) for d in (32, 64)]
     ys = h.step_batch(c.block4, c.idx, c.val, xs, c.n)
     for x, y in zip(xs, ys):
