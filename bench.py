@@ -58,9 +58,9 @@ WORKLOADS["replicas"] = (0, 1.0, (64,))
 METRIC, UNIT = "spmm_gflops", "GFLOP/s"
 FALLBACK_HBM_GBS = 6650.0
 # (workload, dim, kernel variant) -> dram__bytes_read + dram__bytes_write per product, from the ncu captures
-# summarised under profiles/ (same command as the default run)
-NCU_TRAFFIC_BYTES = {("cfg2", 128, "column-tiled"): 1.770e9, ("cfg2", 128, "two 64-column passes"): 3.971e9,
-                     ("cfg3", 64, "one pass"): 9.524e9}
+# summarised under profiles/ (single products on the same graphs; column-tiled: two ranges)
+NCU_TRAFFIC_BYTES = {("cfg2", 128, "column-tiled"): 2.208e9, ("cfg2", 128, "two 64-column passes"): 3.881e9,
+                     ("cfg3", 64, "one pass"): 9.356e9}
 
 
 def hbm_peak():
@@ -284,8 +284,9 @@ def reference_arm(args, rank, world):
 
 # ----------------------------------------------------------------------------------------
 def gather_peaks(dims):
-    """Measured ceiling of the gather itself: GB/s of whole-row reads from an L2-resident table (32 MB)
-    with the SpMM's access shape, per row width (agcn_probe_gather_bandwidth)."""
+    """Measured rate of the gather itself: GB/s of whole-row reads from an L2-resident table (32 MB) with the
+    SpMM's access shape, per row width (agcn_probe_gather_bandwidth).  Rows in random order: a lower bound of
+    what products reach whose column ids ascend within a row."""
     import ctypes
     from accelgcn import _lib
     lib = _lib.load()
@@ -295,7 +296,7 @@ def gather_peaks(dims):
             continue
         rows = (32 << 20) // (4 * d)             # a 32 MB table: a power-of-two number of rows
         best = 0.0
-        for resident in (5, 0):            # the SpMM's residency, and whatever the registers allow
+        for resident in (4, 0):            # the SpMM's residency, and whatever the registers allow
             gbs = ctypes.c_double(0.0)
             _lib.check(lib.agcn_probe_gather_bandwidth(rows, d, (2 << 30) // (4 * d), 5, resident, ctypes.byref(gbs)))
             best = max(best, gbs.value)

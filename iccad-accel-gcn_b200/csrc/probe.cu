@@ -1,7 +1,8 @@
 // Measurement aid: how fast can this GPU gather whole rows of a dense table that stays in L2?
 // The SpMM (spmm_accel.cu:55-78 in the reference) moves nnz * dim * 4 bytes of X through the
-// L2 -> SM path for 4 * dim * N bytes from HBM, so on dense graphs its ceiling is this gather rate,
-// not the HBM bandwidth.  The probe issues the same access shape as the SpMM's float4 mode -- a
+// L2 -> SM path for 4 * dim * N bytes from HBM, so on dense graphs it is bound by the gather, not by
+// the HBM bandwidth.  (Rows come in random order here and ascend within a row there, so products
+// can be faster: a measured rate, not a ceiling.)  The probe issues the same access shape as the SpMM's float4 mode -- a
 // slot of dim/4 lanes reads one row with 16-byte loads, four independent rows in flight per lane,
 // 256 threads per block at a residency the caller chooses, the same L2 policy -- with row numbers
 // from a counter-based hash instead of a column array and a plain add instead of the FMA, so what
