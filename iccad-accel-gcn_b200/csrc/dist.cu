@@ -550,7 +550,7 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
             rc = spmm_check_run_args(d->plan, d->idx, d->val, fwd->z, 128, out, 128, 128, AGCN_ACT_RELU);
             if (rc != AGCN_OK) return rc;
             SpmmLaunchPart part;
-            part.early = d->per > 0;
+            if (d->per > 0) part.early = SpmmLaunchPart::ONLY_X;
             d->plan->launches_last_run = 0;
             rc = spmm_run_prepared(d->plan, d->idx, d->val, fwd->z, 128, true, out, 128, 128, s, AGCN_ACT_RELU, 0, part);
             if (rc != AGCN_OK) return rc;

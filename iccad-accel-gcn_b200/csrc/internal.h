@@ -69,7 +69,9 @@ inline int *spmm_carry_counters(void *carry, int64_t n_carry) { return reinterpr
 struct SpmmLaunchPart {
     int64_t unit0 = 0, unit1 = -1;      // units [unit0, unit1); -1 = to the end
     bool zero_fill = true;
-    bool early = false;                 // the launch before this one on the stream makes X (it alone): start while it runs
+    // Start while the launch before this one on the stream still runs: ONLY_X: that one makes X and nothing else that
+    // is read here, and was itself launched behind all it follows; ANY: it may be any operation.
+    enum Early { NO, ONLY_X, ANY } early = NO;
     const int *abort_flag = nullptr;    // optional device word: nonzero makes the kernels return at once
     void *carry = nullptr;              // optional carry scratch to use instead of the plan's (products in flight together)
 };

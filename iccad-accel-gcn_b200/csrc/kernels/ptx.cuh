@@ -51,17 +51,18 @@ __device__ __forceinline__ float ld_x1(const float *p, uint64_t policy)
     return v;
 }
 
-// sparse operand (col ids / values): streamed once per launch
+// sparse operand (col ids / values): streamed once per launch.  Not .nc and volatile: where the launch before may be
+// anything it may also be what makes them, and no load of them moves above the wait for it.
 __device__ __forceinline__ int ld_a(const int *p, uint64_t policy)
 {
     int v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy));
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.s32 %0, [%1], %2;" : "=r"(v) : "l"(p), "l"(policy));
     return v;
 }
 __device__ __forceinline__ float ld_a(const float *p, uint64_t policy)
 {
     float v;
-    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+    asm volatile("ld.global.L1::no_allocate.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
     return v;
 }
 

@@ -78,7 +78,8 @@ struct SpmmParams {
     const int *zero_rows;     // rows no tuple covers
     int64_t n_zero_rows;
     int hot_column;           // HOT kernels: rows of X from this column on are kept in L2; 0: no such choice
-    int early;                // host only: launched so that it overlaps the kernel before it, which makes X
+    int early;                // host only: launched so that it overlaps the kernel before it
+    int wait_first;           // ... which may be any kernel: idx and val, too, are read behind the wait for it
     int relu;                 // nonzero: Y = max(A * X, 0) (fused GCN activation)
     // The fields below are read only by the general (PLAIN = false) kernel flavour.
     int accumulate;           // nonzero: Y += A * X (later column ranges of a column-tiled product)
@@ -365,7 +366,7 @@ spmm_units_kernel(const SpmmParams p)
     L2Policies pol = make_l2_policies();
     if (HOT) pol.hot = p.hot_column;
 
-    launch_dependents();        // a dense transform of this product's result may lay out its weights meanwhile
+    if (!p.wait_first) launch_dependents();     // a dense transform of this product's result may lay out its weights meanwhile
     if (p.abort_flag != nullptr && *p.abort_flag != 0) return;     // input rejected by a check earlier in the stream
     if ((int64_t)blockIdx.x >= p.n_units) {
         wait_for_predecessor();
@@ -390,6 +391,10 @@ spmm_units_kernel(const SpmmParams p)
     const TupleView t = decode_tuple(p.tuples, e, p.n_tuples);
     const bool big = t.valid && !t.small;
     const int total = t.n_rows * t.row_nz;
+    if (p.wait_first) {                 // tuples are the plan's and do not change
+        wait_for_predecessor();
+        launch_dependents();            // not above the wait: then whoever comes next finds that one finished, too
+    }
 
     // stage the tuple's (col, val) pairs
     {

@@ -666,6 +666,52 @@ def test_first_unaligned_width_under_stream_capture(cfg4_small):
     plan.close()
 
 
+@pytest.mark.parametrize("case_name,dim", [("cfg1", 16), ("cfg1", 60), ("cfg4_small", 64), ("cfg4_small", 128), ("cfg4_small", 61)])
+def test_products_behind_work_of_any_kind(case_name, dim, request):
+    # a product is launched while the operation before it still runs, whatever that is: kernels and copies that make its
+    # column ids, values and X right before, products whose result it multiplies, streams that join; also captured
+    import torch
+    from accelgcn import spmm
+    c = request.getfixturevalue(case_name)
+    idx0, val0, x0 = c.t["idx"], c.t["val"], torch.from_numpy(c.x(dim)).to(c.dev)
+    plan = spmm.SpmmPlan(c.t["block4"], idx0, c.n, c.n)
+    idx, val, x = torch.zeros_like(idx0), torch.empty_like(val0), torch.empty_like(x0)
+    y, z = torch.empty_like(x0), torch.empty_like(x0)
+    side = torch.cuda.Stream(c.dev)
+
+    def steps(between):
+        x.copy_(x0); between()
+        for k in range(6):
+            idx.zero_(); val.fill_(float("nan")); between()
+            idx.copy_(idx0); torch.mul(val0, 0.5 + 0.125 * k, out=val); between()
+            plan.run(idx, val, x, y); between()
+            plan.run(idx, val, y, z, relu=True); between()
+            plan.run(idx, val, z, x); between()
+            x.add_(x0); between()
+            side.wait_stream(torch.cuda.current_stream()); between()
+            plan.run(idx, val, x, y, stream=side); between()
+            torch.cuda.current_stream().wait_stream(side); between()
+            plan.run(idx, val, y, z); between()
+            torch.nn.functional.normalize(z, dim=1, out=x); between()
+        return x
+
+    plan.run(idx0, val0, x0, y)                      # the aligned copy of X is made outside of the capture
+    want = steps(torch.cuda.synchronize).clone()
+    assert bool(torch.isfinite(want).all()) and float(want.abs().max()) > 0
+    for _ in range(10):
+        assert torch.equal(steps(lambda: None), want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        steps(lambda: None)
+    for _ in range(3):
+        x.fill_(float("nan"))
+        graph.replay()
+        assert torch.equal(x, want)
+    torch.cuda.synchronize()
+    plan.close()
+
+
 @pytest.mark.parametrize("case_name", ["cfg1", "cfg4_small"])
 def test_column_tiled_small(case_name, request):
     # tiled plan with several range layouts (one of them empty), ReLU, an unaligned width and the
