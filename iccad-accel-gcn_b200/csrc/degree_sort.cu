@@ -6,7 +6,7 @@
 
 namespace agcn {
 
-// Two launches up to 65 536 rows, a memset and four to seven above; one synchronisation at the end (15 to 25 launches, eight allocations and
+// Two launches up to 65 536 rows, a memset and five to eight above; one synchronisation at the end (15 to 25 launches, eight allocations and
 // two synchronisations before: 0.9 ms for 16 384 rows, most of it in the allocator).
 static int degree_sort_device(const int *d_indptr, const int *d_indices, const float *d_vals,
                               int64_t n_rows, int64_t nnz, int relabel_cols,
@@ -34,45 +34,51 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
     DeviceScratch scratch(s);
     SortBuffers buf;
     SortControl *ctl = nullptr;
-    unsigned long long *state = nullptr, *final_state = nullptr;
-    int *new_id = nullptr, *tile_row = nullptr;
+    unsigned long long *final_state = nullptr;
+    SortCounts counts = {nullptr, tiles, ceil_div(tiles, COUNT_GROUP), ceil_div(tiles, COUNT_SUPER)};
+    PermuteMap map = {nullptr, nullptr, nullptr};
     size_t cleared = 0;
     void *block = nullptr;
     for (int round = 0; round < 2; round++) {
         Carver c(block);
         ctl = c.take<SortControl>(1);
         final_state = c.take<unsigned long long>(small ? 0 : final_tiles);
-        state = c.take<unsigned long long>(small ? 0 : passes * tiles * RADIX_BINS);
+        counts.rows = c.take<unsigned>(small ? 0 : passes * (counts.tiles + counts.groups + counts.supers) * RADIX_BINS);
         cleared = c.bytes();
         for (int k = 0; k < 2; k++) { buf.keys[k] = c.take<unsigned>(small ? 0 : n_rows); buf.rows[k] = c.take<int>(small ? 0 : n_rows); }
-        new_id = permute && relabel_cols ? c.take<int>(n_rows) : nullptr;
-        tile_row = permute_tiles > 0 ? c.take<int>(permute_tiles) : nullptr;
+        map.new_id = permute && relabel_cols ? c.take<int>(n_rows) : nullptr;
+        map.delta = permute_tiles > 0 ? c.take<int>(n_rows) : nullptr;
+        map.tile_row = permute_tiles > 0 ? c.take<int>(permute_tiles) : nullptr;
         if (round == 0 && (block = scratch.alloc<unsigned char>((int64_t)c.bytes())) == nullptr) return AGCN_ERR_CUDA;
     }
     AGCN_HOST_WORDS(words, s);
     if (small) {
         AGCN_CUDA(cudaFuncSetAttribute(sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_SMEM_BYTES));
         sort_small_kernel<<<SMALL_CLUSTER, SMALL_BLOCK, SMALL_SMEM_BYTES, s>>>(d_indptr, (int)n_rows, (int)ceil_div(n_rows, SMALL_CLUSTER * SMALL_BLOCK), nnz,
-                                                                               permute ? 1 : 0, ctl, d_perm, d_new_indptr, new_id, tile_row, words.device());
+                                                                               permute ? 1 : 0, ctl, d_perm, d_new_indptr, map, words.device());
         AGCN_LAUNCH_CHECK("sort_small_kernel");
     } else {
         AGCN_CUDA(cudaMemsetAsync(ctl, 0, cleared, s));
-        AGCN_KERNEL(degree_count_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, nnz, permute ? 1 : 0, ctl, words.device());
+        AGCN_KERNEL(degree_count_kernel, (unsigned)tiles, SORT_BLOCK, s, d_indptr, n_rows, nnz, permute ? 1 : 0, counts, ctl, words.device());
         AGCN_LAUNCH_CHECK("degree_count_kernel");
         for (int pass = 0; pass < passes; pass++) {
-            AGCN_CUDA(launch_early(true, radix_pass_kernel, (unsigned)tiles, SORT_BLOCK, 0, s, d_indptr, n_rows, pass, buf, ctl,
-                                   state + pass * tiles * RADIX_BINS, words.device()));
+            AGCN_CUDA(launch_early(true, radix_pass_kernel, (unsigned)tiles, RADIX_BLOCK, 0, s, d_indptr, (int)n_rows, pass, passes, buf,
+                                   (const SortControl *)ctl, counts));
             AGCN_LAUNCH_CHECK("radix_pass_kernel");
         }
-        AGCN_CUDA(launch_early(true, sort_finish_kernel, (unsigned)final_tiles, SORT_BLOCK, 0, s, n_rows, passes, buf, ctl, final_state, d_perm,
-                               d_new_indptr, new_id, tile_row, words.device()));
+        AGCN_CUDA(launch_early(true, sort_finish_kernel, (unsigned)final_tiles, SORT_BLOCK, 0, s, d_indptr, n_rows, passes, buf, ctl, final_state, d_perm,
+                               d_new_indptr, map, words.device()));
         AGCN_LAUNCH_CHECK("sort_finish_kernel");
+        if (permute_tiles > 0) {
+            AGCN_CUDA(launch_early(true, tile_rows_kernel, (unsigned)ceil_div(permute_tiles, SORT_BLOCK), SORT_BLOCK, 0, s, (const int *)d_new_indptr,
+                                   (int)n_rows, (int)permute_tiles, (const SortControl *)ctl, map.tile_row));
+            AGCN_LAUNCH_CHECK("tile_rows_kernel");
+        }
     }
     if (permute_tiles > 0) {
-        AGCN_CUDA(launch_early(true, csr_permute_kernel, (unsigned)permute_tiles, PERMUTE_BLOCK, 0, s, d_indptr, d_indices,
-                               d_new_vals != nullptr ? d_vals : (const float *)nullptr, (const int *)d_perm, (const int *)d_new_indptr,
-                               (const int *)new_id, (const int *)tile_row, n_rows, nnz, d_new_indices, d_new_vals, (const SortControl *)ctl,
-                               words.device()));
+        AGCN_CUDA(launch_early(true, csr_permute_kernel, (unsigned)(ceil_div(permute_tiles, PERMUTE_WARPS) * (d_new_vals != nullptr ? 2 : 1)), PERMUTE_BLOCK, 0, s, d_indices,
+                               d_new_vals != nullptr ? d_vals : (const float *)nullptr, (const int *)d_new_indptr, map, n_rows, nnz, d_new_indices,
+                               d_new_vals, (const SortControl *)ctl, words.device()));
         AGCN_LAUNCH_CHECK("csr_permute_kernel");
     }
     AGCN_CUDA(words.sync());

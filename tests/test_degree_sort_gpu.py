@@ -138,6 +138,42 @@ def test_tile_edges_and_number_of_passes(n, top, relabel):
         assert np.array_equal(a, b), what
 
 
+@pytest.mark.parametrize("n", [65_536 + 1, 65_536 * 2, 2_097_152, 2_101_249, 4_300_000])
+@pytest.mark.parametrize("kind", ["low", "high", "mixed"])
+def test_counters_of_tiles_groups_and_groups_of_groups(n, kind):
+    # a tile of 4096 rows adds up counters of tiles, of groups of 16 and of 512 of them: sizes around their edges, with all
+    # second digits zero (not counted), none zero, and some
+    from accelgcn import degree_sort
+    require_cuda()
+    rng = np.random.default_rng(n)
+    deg = rng.integers(0, 3, n)
+    if kind == "high":
+        deg = 256 + rng.integers(0, 200, n) if n < 200_000 else 256 * rng.integers(1, 3, n)
+    if kind == "mixed":
+        some = rng.random(n) < 0.05
+        deg[some] = rng.integers(0, 2_000, int(some.sum()))
+    indptr = np.concatenate([[0], np.cumsum(deg)])
+    assert indptr[-1] < 2**31
+    indptr = indptr.astype(np.int32)
+    if kind == "high":                                   # the order alone: a perm for row pointers without the matrix
+        import torch
+        from accelgcn import _lib
+        dev = torch.device("cuda")
+        t, perm, nip = torch.from_numpy(indptr).to(dev), torch.empty(n, dtype=torch.int32, device=dev), torch.empty(n + 1, dtype=torch.int32, device=dev)
+        _lib.check(_lib.load().agcn_degree_sort_device(t.data_ptr(), None, None, n, 0, 0, perm.data_ptr(), nip.data_ptr(), None, None, None))
+        perm, nip = perm.cpu().numpy(), nip.cpu().numpy()
+    else:
+        idx = rng.integers(0, n, int(indptr[-1]), dtype=np.int32)
+        perm, nip, nix, _ = degree_sort.degree_sort(indptr, idx, None, relabel_cols=True)
+    want = np.argsort(deg, kind="stable")
+    assert np.array_equal(perm, want)
+    assert np.array_equal(nip, np.concatenate([[0], np.cumsum(deg[want])]))
+    if kind != "high":
+        inv = np.empty(n, dtype=np.int32); inv[want] = np.arange(n, dtype=np.int32)
+        start = np.repeat(indptr[want] - nip[:-1], deg[want])
+        assert np.array_equal(nix, inv[idx[start + np.arange(len(idx))]])
+
+
 def test_release_scratch_gives_the_pool_back():
     # between calls the library keeps scratch that no other allocator of the process can use
     import torch
