@@ -73,17 +73,24 @@ struct PartTile {
 constexpr int PART_TILE_INTS = PART_TILE + PART_HALO + 2;                  // row pointers a tile looks at
 constexpr int PART_SMEM_INTS = PART_TILE_INTS + PART_TILE_INTS / 32 + 1;   // the same, padded
 
-__device__ __forceinline__ PartTile part_load_tile(const int *__restrict__ indptr, int64_t n_rows, int *s_ip)
+// All loads of a thread are in flight together (one by one, nine L2 or HBM latencies were half of the kernel's time).
+__device__ __forceinline__ PartTile part_load_tile(const int *__restrict__ indptr, int64_t n_rows, int64_t tile, int *s_ip)
 {
+    constexpr int LOADS = (PART_TILE_INTS + PART_BLOCK - 1) / PART_BLOCK;
     PartTile t;
     t.s_ip = s_ip;
-    t.first = (int64_t)blockIdx.x * PART_TILE;
+    t.first = tile * PART_TILE;
     t.n_rows = n_rows;
-    for (int k = threadIdx.x; k < PART_TILE_INTS; k += PART_BLOCK) {
-        int64_t i = t.first - 1 + k;
+    int v[LOADS];
+#pragma unroll
+    for (int k = 0; k < LOADS; k++) {
+        int64_t i = t.first - 1 + k * PART_BLOCK + threadIdx.x;
         i = i < 0 ? 0 : (i > n_rows ? n_rows : i);
-        s_ip[part_pad(k)] = indptr[i];
+        v[k] = indptr[i];
     }
+#pragma unroll
+    for (int k = 0; k < LOADS; k++)
+        if (k * PART_BLOCK + (int)threadIdx.x < PART_TILE_INTS) s_ip[part_pad(k * PART_BLOCK + threadIdx.x)] = v[k];
     __syncthreads();
     return t;
 }
@@ -152,7 +159,7 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
     __shared__ int s_red[4][PART_BLOCK / 32];
     launch_dependents();
-    const PartTile t = part_load_tile(indptr, n_rows, s_ip);
+    const PartTile t = part_load_tile(indptr, n_rows, blockIdx.x, s_ip);
     int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
     unsigned heads;
     bool negative = false;
@@ -219,116 +226,158 @@ part_scan_kernel(const PartTileInfo *tiles, int64_t n_tiles, int *__restrict__ t
     if (threadIdx.x == 0) out->w[PART_WORD_TOTAL] = carry;
 }
 
-// (C) every row that opens tuples writes them at its scanned offset.  A row of degree D > 384 owns
-// ceil(D / 384) tuples -- thousands for a hub row -- so rows with more than PART_INLINE_TUPLES are
-// queued in shared memory and written by the whole block together instead of by their one thread.
-constexpr int PART_INLINE_TUPLES = 8;
-constexpr int PART_HEAVY_QUEUE = 128;
+// (C) every row that opens tuples writes them at its scanned offset.  A row of degree D > 384 owns ceil(D / 384) of
+// them, so the tiles of a graph's hub rows have many times the tuples of the others: tuples are then dealt out one per
+// thread, which looks its row up in the scanned offsets, and a tile of more than PART_CHUNK is shared by the blocks
+// before the tile blocks, PART_CHUNK output positions each.  (Row by row the last of 1172 tiles, 2.4 M rows of 25,
+// kept the kernel for 44 us; 21 now.)
+constexpr int PART_CHUNK = 4096;
 
 constexpr int PART_DIRECT_TILES = PART_BLOCK;      // half a million rows
 
-// tile_offset == nullptr: this block scans the descriptions of the (at most PART_DIRECT_TILES) tiles itself, and
-// the last one reports the total.  Nothing is written outside `cap` tuples (a
-// decreasing indptr, found by (A), may give any position here).
-__global__ void __launch_bounds__(PART_BLOCK)
-part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileInfo *info,      // not __restrict__: read after the wait
-                 const int *__restrict__ tile_incoming_head, const int64_t *__restrict__ tile_offset, int64_t cap,
-                 int4 *__restrict__ block4, HostWords *report)
+// The tuples of one tile that lie at output positions [lo, hi), hi <= first_out + their number.
+struct PartEmitShared {
+    int ip[PART_SMEM_INTS];
+    int scan[PART_BLOCK / 32 + 1];
+    int pos[PART_TILE];                        // tuples of the tile before each of its rows
+    unsigned char heads[PART_BLOCK + 2];       // a bit per row that starts a run (or lies past the end), a byte per thread
+};
+
+// Tuple c of row i (row r of its tile)
+__device__ __forceinline__ int4 part_tuple(const PartEmitShared &sh, int64_t i, int r, int d, int loc, int c)
 {
-    __shared__ int s_ip[PART_SMEM_INTS];
-    __shared__ int s_scan[PART_BLOCK / 32 + 1];
-    __shared__ int64_t s_scan64[PART_BLOCK / 32 + 1];
-    __shared__ unsigned char s_heads[PART_BLOCK + 2];      // a bit per row that starts a run (or lies past the end), a byte per thread
-    __shared__ int s_heavy_n;
-    __shared__ int s_heavy_row[PART_HEAVY_QUEUE], s_heavy_deg[PART_HEAVY_QUEUE], s_heavy_loc[PART_HEAVY_QUEUE];
-    __shared__ int64_t s_heavy_out[PART_HEAVY_QUEUE];
-    if (threadIdx.x == 0) s_heavy_n = 0;
-    const PartTile t = part_load_tile(indptr, n_rows, s_ip);      // synchronises the block
-    wait_for_predecessor();      // launched early behind (A), which has nothing to do with indptr but read it
-    int incoming;
-    int64_t first_out;
-    if (tile_offset != nullptr) {
-        incoming = tile_incoming_head[blockIdx.x];
-        first_out = tile_offset[blockIdx.x];
-    } else {
-        const int b = threadIdx.x;
-        PartTileInfo mine = {-1, 0, 0, 0};
-        if (b <= (int)blockIdx.x) mine = info[b];
-        int unused;
-        const int head = block_scan_exclusive<PART_BLOCK>(mine.last_head, OpMax(), -1, unused, s_scan);
-        const int64_t count = b <= (int)blockIdx.x ? mine.rest + part_lead_tuples(mine, b, head) : 0;
-        int64_t total;
-        const int64_t before = block_scan_exclusive<PART_BLOCK>(count, OpAdd(), (int64_t)0, total, s_scan64);
-        if (b == (int)blockIdx.x) { s_scan[0] = head; s_scan64[0] = before; }
-        __syncthreads();
-        incoming = s_scan[0];
-        first_out = s_scan64[0];
-        __syncthreads();         // s_scan is used again
-        if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) report->w[PART_WORD_TOTAL] = total;
+    if (d > PART_DEG_BOUND) {
+        const int done = c * PART_DEG_BOUND;
+        return make_int4(d, (int)i, loc + done, d - done < PART_DEG_BOUND ? d - done : PART_DEG_BOUND);
     }
+    // up to R(D) rows, as far as the run goes
+    const int at = r >> 3;
+    const unsigned window = sh.heads[at] | sh.heads[at + 1] << 8 | sh.heads[at + 2] << 16;
+    const int run = __ffs((window >> ((r & 7) + 1)) | 1u << (PART_MAX_ROWS_PER_TUPLE - 1));
+    return make_int4(d, (int)i, loc, (part_warp_nz(d) << 16) + min(part_rows_per_tuple(d), run));
+}
+
+__device__ __forceinline__ void part_emit_tile(const PartTile &t, PartEmitShared &sh, int incoming, int64_t first_out, int64_t lo, int64_t hi,
+                                               int64_t cap, int ip0, int4 *__restrict__ block4)
+{
+    static_assert(PART_ITEMS == 8, "a byte of run starts per thread");
     int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
     unsigned heads;
     bool negative;
-    part_row_counts(t, incoming, s_scan, deg, cnt, heads, lead, lead_deg, negative);
+    part_row_counts(t, incoming, sh.scan, deg, cnt, heads, lead, lead_deg, negative);
     const int64_t my_first = t.first + (int64_t)threadIdx.x * PART_ITEMS;
     int sum = 0;
+    bool several = false;
 #pragma unroll
     for (int k = 0; k < PART_ITEMS; k++) {
         sum += cnt[k];
-        if (my_first + k >= n_rows) heads |= 1u << k;
+        several |= cnt[k] > 1;
+        if (my_first + k >= t.n_rows) heads |= 1u << k;
     }
-    s_heads[threadIdx.x] = (unsigned char)heads;
+    sh.heads[threadIdx.x] = (unsigned char)heads;
     if (threadIdx.x < 2) {               // the rows a tuple of this tile may reach into
         unsigned m = 0;
         for (int k = 0; k < 8; k++) {
             const int64_t i = t.first + PART_TILE + threadIdx.x * 8 + k;
-            if (i >= n_rows || threadIdx.x * 8 + k >= PART_MAX_ROWS_PER_TUPLE || t.deg(i) != t.deg(i - 1)) m |= 1u << k;
+            if (i >= t.n_rows || threadIdx.x * 8 + k >= PART_MAX_ROWS_PER_TUPLE || t.deg(i) != t.deg(i - 1)) m |= 1u << k;
         }
-        s_heads[PART_BLOCK + threadIdx.x] = (unsigned char)m;
+        sh.heads[PART_BLOCK + threadIdx.x] = (unsigned char)m;
     }
     int tile_total;
-    const int ex = block_scan_exclusive<PART_BLOCK>(sum, OpAdd(), 0, tile_total, s_scan);      // synchronises: s_heads is complete
-    int64_t out = first_out + ex;
-    const unsigned window = s_heads[threadIdx.x] | s_heads[threadIdx.x + 1] << 8 | s_heads[threadIdx.x + 2] << 16;
-    const int ip0 = indptr[0];
+    int at = block_scan_exclusive<PART_BLOCK>(sum, OpAdd(), 0, tile_total, sh.scan);      // synchronises: heads is complete
+    if (!__syncthreads_or(several)) {
 #pragma unroll
-    for (int k = 0; k < PART_ITEMS; k++) {
-        if (cnt[k] == 0) continue;
-        const int64_t i = my_first + k;
-        const int d = deg[k];
-        const int loc = t.ip(i) - ip0;
-        if (d <= PART_DEG_BOUND) {
-            // up to R(D) rows, as far as the run goes
-            const int run = __ffs((window >> (k + 1)) | 1u << (PART_MAX_ROWS_PER_TUPLE - 1));
-            const int j = min(part_rows_per_tuple(d), run);
-            if ((uint64_t)out < (uint64_t)cap) block4[out] = make_int4(d, (int)i, loc, (part_warp_nz(d) << 16) + j);
-            out += 1;
-        } else {
-            int slot = PART_HEAVY_QUEUE;
-            if (cnt[k] > PART_INLINE_TUPLES) slot = atomicAdd(&s_heavy_n, 1);
-            if (slot < PART_HEAVY_QUEUE) {
-                s_heavy_row[slot] = (int)i; s_heavy_deg[slot] = d; s_heavy_loc[slot] = loc; s_heavy_out[slot] = out;
-            } else {
-                for (int c = 0; c < cnt[k] && (uint64_t)(out + c) < (uint64_t)cap; c++) {
-                    const int done = c * PART_DEG_BOUND;
-                    const int take = d - done < PART_DEG_BOUND ? d - done : PART_DEG_BOUND;
-                    block4[out + c] = make_int4(d, (int)i, loc + done, take);
-                }
-            }
-            out += cnt[k];
+        for (int k = 0; k < PART_ITEMS; k++) {
+            if (cnt[k] == 0) continue;
+            const int64_t out = first_out + at++;
+            if (out >= lo && out < hi && (uint64_t)out < (uint64_t)cap)
+                block4[out] = part_tuple(sh, my_first + k, threadIdx.x * PART_ITEMS + k, deg[k], t.ip(my_first + k) - ip0, 0);
         }
+        return;
     }
+#pragma unroll
+    for (int k = 0; k < PART_ITEMS; k++) { sh.pos[threadIdx.x * PART_ITEMS + k] = at; at += cnt[k]; }
     __syncthreads();
-    const int n_heavy = s_heavy_n < PART_HEAVY_QUEUE ? s_heavy_n : PART_HEAVY_QUEUE;
-    for (int q = 0; q < n_heavy; q++) {
-        const int d = s_heavy_deg[q], row = s_heavy_row[q], loc = s_heavy_loc[q];
-        const int64_t o = s_heavy_out[q];
-        const int n_tuples = (d + PART_DEG_BOUND - 1) / PART_DEG_BOUND;
-        for (int c = threadIdx.x; c < n_tuples && (uint64_t)(o + c) < (uint64_t)cap; c += PART_BLOCK) {
-            const int done = c * PART_DEG_BOUND;
-            const int take = d - done < PART_DEG_BOUND ? d - done : PART_DEG_BOUND;
-            block4[o + c] = make_int4(d, row, loc + done, take);
+    const int64_t end = first_out + tile_total < hi ? first_out + tile_total : hi;
+    for (int64_t out = (first_out > lo ? first_out : lo) + threadIdx.x; out < end; out += PART_BLOCK) {
+        const int o = (int)(out - first_out);
+        int r = 0;                       // the last row with no more than o tuples before it
+#pragma unroll
+        for (int step = PART_TILE / 2; step > 0; step >>= 1)
+            if (sh.pos[r + step] <= o) r += step;
+        const int64_t i = t.first + r;
+        if ((uint64_t)out < (uint64_t)cap) block4[out] = part_tuple(sh, i, r, t.deg(i), t.ip(i) - ip0, o - sh.pos[r]);
+    }
+}
+
+// tile_offset == nullptr: this block scans the descriptions of the (at most PART_DIRECT_TILES) tiles itself, and
+// the last tile's reports the total; otherwise there are `cap` tuples.  Nothing is written outside `cap` tuples (a
+// decreasing indptr, found by (A), may give any position here).  The first `chunks` blocks: PART_CHUNK output positions
+// each; the others: a tile each.
+__global__ void __launch_bounds__(PART_BLOCK, 4)
+part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileInfo *info,      // not __restrict__: read after the wait
+                 const int *__restrict__ tile_incoming_head, const int64_t *__restrict__ tile_offset, int tiles, int chunks, int64_t cap,
+                 int4 *__restrict__ block4, HostWords *report)
+{
+    __shared__ PartEmitShared sh;
+    __shared__ int64_t s_scan64[PART_BLOCK / 32 + 1];
+    __shared__ int64_t s_offset[PART_DIRECT_TILES + 1];
+    __shared__ int s_head[PART_DIRECT_TILES];
+    __shared__ int s_list[2], s_listed;
+    const int of_tile = (int)blockIdx.x - chunks;
+    PartTile t;
+    if (of_tile >= 0) t = part_load_tile(indptr, n_rows, of_tile, sh.ip);
+    const int ip0 = indptr[0];
+    wait_for_predecessor();      // launched early behind (A), which has nothing to do with indptr but read it
+    const bool direct = tile_offset == nullptr;
+    if (direct) {
+        const int b = threadIdx.x;
+        PartTileInfo mine = {-1, 0, 0, 0};
+        if (b < tiles) mine = info[b];
+        int unused;
+        const int head = block_scan_exclusive<PART_BLOCK>(mine.last_head, OpMax(), -1, unused, sh.scan);
+        const int64_t count = b < tiles ? mine.rest + part_lead_tuples(mine, b, head) : 0;
+        int64_t total;
+        s_offset[b] = block_scan_exclusive<PART_BLOCK>(count, OpAdd(), (int64_t)0, total, s_scan64);
+        s_head[b] = head;
+        if (b == 0) s_offset[PART_DIRECT_TILES] = total;
+        __syncthreads();
+        if (of_tile == 0 && b == 0) report->w[PART_WORD_TOTAL] = total;
+    }
+    auto offset = [&](int b) { return direct ? s_offset[b < tiles ? b : PART_DIRECT_TILES] : (b < tiles ? tile_offset[b] : cap); };
+    auto head_of = [&](int b) { return direct ? s_head[b] : tile_incoming_head[b]; };
+    if (of_tile >= 0) {
+        const int64_t first_out = offset(of_tile), end = offset(of_tile + 1);
+        if (end - first_out <= PART_CHUNK) part_emit_tile(t, sh, head_of(of_tile), first_out, first_out, end, cap, ip0, block4);
+        return;
+    }
+    // tiles of more than PART_CHUNK tuples that reach into this block's positions: two at most
+    const int64_t lo = (int64_t)blockIdx.x * PART_CHUNK, hi = lo + PART_CHUNK;
+    auto tiles_before = [&](int64_t x) {           // how many tiles begin before position x: a step by all threads leaves 1/256
+        int a = 0, z = tiles;
+        while (a < z) {
+            const int step = (z - a + PART_BLOCK - 1) / PART_BLOCK, mine = a + (int)threadIdx.x * step;
+            const int before = __syncthreads_count(mine < z && offset(mine) < x);      // samples a, a + step, ... that begin before x
+            if (before == 0) return a;
+            z = min(z, a + before * step);
+            a = a + (before - 1) * step + 1;
         }
+        return a;
+    };
+    const int b1 = tiles_before(hi), b0 = tiles_before(lo + 1);
+    if (threadIdx.x == 0) s_listed = 0;
+    __syncthreads();
+    for (int b = (b0 > 0 ? b0 - 1 : 0) + threadIdx.x; b < b1; b += PART_BLOCK)
+        if (offset(b + 1) - offset(b) > PART_CHUNK) {
+            const int q = atomicAdd(&s_listed, 1);
+            if (q < 2) s_list[q] = b;
+        }
+    __syncthreads();
+    for (int q = 0; q < min(s_listed, 2); q++) {
+        const int b = s_list[q];
+        __syncthreads();                 // the tile before is done with
+        t = part_load_tile(indptr, n_rows, b, sh.ip);
+        part_emit_tile(t, sh, head_of(b), offset(b), lo, hi, cap, ip0, block4);
     }
 }
 

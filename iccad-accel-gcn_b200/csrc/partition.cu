@@ -90,8 +90,9 @@ static int partition_direct(const char *who, const int *d_indptr, int64_t n_rows
     AGCN_HOST_WORDS(words, s);
     AGCN_KERNEL(part_describe_kernel, tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words.device());
     AGCN_LAUNCH_CHECK("part_describe_kernel");
-    AGCN_CUDA(launch_early(true, part_emit_kernel, tiles, PART_BLOCK, 0, s, d_indptr, n_rows, (const PartTileInfo *)sc.info, (const int *)nullptr,
-                           (const int64_t *)nullptr, cap, tuples, words.device()));
+    const unsigned chunks = (unsigned)ceil_div(cap, PART_CHUNK);
+    AGCN_CUDA(launch_early(true, part_emit_kernel, chunks + tiles, PART_BLOCK, 0, s, d_indptr, n_rows, (const PartTileInfo *)sc.info, (const int *)nullptr,
+                           (const int64_t *)nullptr, (int)tiles, (int)chunks, cap, tuples, words.device()));
     AGCN_LAUNCH_CHECK("part_emit_kernel");
     AGCN_CUDA(words.sync());
     return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
@@ -101,8 +102,9 @@ static int partition_direct(const char *who, const int *d_indptr, int64_t n_rows
 static int partition_emit(const int *d_indptr, int64_t n_rows, int64_t n_blocks, int *d_block4, const PartScratch &sc, cudaStream_t s)
 {
     if (n_blocks == 0) return AGCN_OK;
-    AGCN_KERNEL(part_emit_kernel, (unsigned)ceil_div(n_rows, PART_TILE), PART_BLOCK, s, d_indptr, n_rows, (const PartTileInfo *)nullptr,
-                (const int *)sc.tile_head, (const int64_t *)sc.tile_offset, n_blocks, reinterpret_cast<int4 *>(d_block4), (HostWords *)nullptr);
+    const int64_t tiles = ceil_div(n_rows, PART_TILE), chunks = ceil_div(n_blocks, PART_CHUNK);
+    AGCN_KERNEL(part_emit_kernel, (unsigned)(chunks + tiles), PART_BLOCK, s, d_indptr, n_rows, (const PartTileInfo *)nullptr,
+                (const int *)sc.tile_head, (const int64_t *)sc.tile_offset, (int)tiles, (int)chunks, n_blocks, reinterpret_cast<int4 *>(d_block4), (HostWords *)nullptr);
     AGCN_LAUNCH_CHECK("part_emit_kernel");
     return AGCN_OK;
 }

@@ -124,6 +124,29 @@ def test_runs_across_tiles_match_oracle(run):
         assert np.array_equal(partition.block_level_partition_device(torch.from_numpy(indptr).to(dev)).cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("rows", [3_000, 600_000])
+@pytest.mark.parametrize("total", [4095, 4096, 4097, 8192, 30_000])
+def test_tiles_of_many_tuples_match_oracle(rows, total):
+    # a tile (2048 rows) of more than 4096 tuples is written by several blocks, 4096 output positions each: hub rows that
+    # make up `total` tuples between rows of one and of none, at the start, at the end and in neighbouring tiles; both the
+    # form that counts and writes in one go (up to 524 288 rows) and the other
+    # (the first tile has exactly `total` of them)
+    import torch
+    from accelgcn import partition
+    dev = require_cuda()
+    rng = np.random.default_rng(total)
+    deg = rng.choice([0, 1, 5, 40, 200, 384], rows)
+    for first in (0, 2047, rows - 900):
+        hubs = 1 + rng.multinomial(total - 700, rng.dirichlet(np.ones(700)))
+        deg[first:first + 700] = hubs * 384 - rng.integers(0, 300, 700)
+    deg[700:2048] = 0
+    deg[4096:8192] = 0                                  # tiles without any tuple
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    want = oracle.partition(indptr)
+    assert np.array_equal(partition.block_level_partition(indptr), want)
+    assert np.array_equal(partition.block_level_partition_device(torch.from_numpy(indptr).to(dev)).cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("n", [5_000, 700_000])
 def test_on_another_stream_the_tuples_are_complete_on_return(n):
     # one-pass form (up to 256 tiles of 2048 rows) and the form whose last kernel still reads the row pointers: with a
