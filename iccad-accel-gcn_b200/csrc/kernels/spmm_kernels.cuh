@@ -639,17 +639,31 @@ __device__ __forceinline__ void unit_crossings(const int4 *__restrict__ block4, 
     same_row = enters && leaves && first.y == last.y;
 }
 
+// Is any of the column ids idx[0 .. n_idx) outside [0, n_cols)?  The part of thread `first` of `stride`.  16 bytes per
+// load (one id per load and 64-bit comparisons: 54 us for 6e7 ids, of which HBM needs 37) but for the ends that are not
+// aligned.
+__device__ __forceinline__ bool ids_outside(const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, int64_t first, int64_t stride)
+{
+    const unsigned n = (unsigned)n_cols;                       // below 2^31: negative ids compare as larger ones
+    int64_t head = (int64_t)((16 - (reinterpret_cast<uintptr_t>(idx) & 15)) & 15) / 4;
+    if (head > n_idx) head = n_idx;
+    const int4 *quads = reinterpret_cast<const int4 *>(idx + head);
+    const int64_t n_quads = (n_idx - head) / 4, tail = head + n_quads * 4;
+    bool bad = false;
+#pragma unroll 4
+    for (int64_t i = first; i < n_quads; i += stride) {
+        const int4 c = __ldcs(quads + i);
+        bad |= (unsigned)c.x >= n || (unsigned)c.y >= n || (unsigned)c.z >= n || (unsigned)c.w >= n;
+    }
+    if (first < head) bad |= (unsigned)idx[first] >= n;        // at most three ids at either end; there are as many threads
+    if (first < n_idx - tail) bad |= (unsigned)idx[tail + first] >= n;
+    return bad;
+}
+
 // Column ids, by `blocks` thread blocks of which this is number `block`.
 __device__ __forceinline__ void plan_check_ids(const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned block, unsigned blocks, HostWords *out)
 {
-    const int64_t stride = (int64_t)blocks * blockDim.x;
-    bool bad = false;
-#pragma unroll 4
-    for (int64_t i = (int64_t)block * blockDim.x + threadIdx.x; i < n_idx; i += stride) {
-        const int c = __ldcs(idx + i);
-        bad |= c < 0 || c >= n_cols;
-    }
-    if (bad) plan_report(out, SPMM_ERR_COL);
+    if (ids_outside(idx, n_idx, n_cols, (int64_t)block * blockDim.x + threadIdx.x, (int64_t)blocks * blockDim.x)) plan_report(out, SPMM_ERR_COL);
 }
 
 // How many of PLAN_SAMPLES column ids, one from every PLAN_SAMPLES-th part of the nonzeros, are at least `first` (anywhere
@@ -745,24 +759,28 @@ plan_check_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_u
 __global__ void __launch_bounds__(256)
 plan_check_cols_kernel(const int *__restrict__ idx, int64_t nnz, int64_t n_cols, int *__restrict__ err_flag)
 {
-    const int64_t stride = (int64_t)gridDim.x * blockDim.x;
-    bool bad = false;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nnz; i += stride) {
-        const int c = idx[i];
-        bad |= c < 0 || c >= n_cols;
-    }
-    if (bad) atomicOr(err_flag, SPMM_ERR_COL);
+    if (ids_outside(idx, nnz, n_cols, (int64_t)blockIdx.x * blockDim.x + threadIdx.x, (int64_t)gridDim.x * blockDim.x)) atomicOr(err_flag, SPMM_ERR_COL);
 }
 
-// first tuple whose row is >= row (tuples are in ascending row order)
-__device__ __forceinline__ int64_t tuple_lower_bound(const int4 *__restrict__ block4, int64_t n_blocks, int64_t row)
+// First and last tuple of the row that tuple e belongs to (tuples are in ascending row order).  In steps that double,
+// then halve: a row of few tuples is two or three loads away, where a search of all tuples is a chain of 18.
+__device__ __forceinline__ int64_t tuple_row_first(const int4 *__restrict__ block4, int64_t e)
 {
-    int64_t lo = 0, hi = n_blocks;
-    while (lo < hi) {
-        const int64_t mid = lo + ((hi - lo) >> 1);
-        if ((int64_t)block4[mid].y < row) lo = mid + 1; else hi = mid;
-    }
-    return lo;
+    const int row = block4[e].y;
+    int64_t step = 1;
+    while (e - step >= 0 && block4[e - step].y == row) { e -= step; step *= 2; }
+    for (step >>= 1; step > 0; step >>= 1)
+        if (e - step >= 0 && block4[e - step].y == row) e -= step;
+    return e;
+}
+__device__ __forceinline__ int64_t tuple_row_last(const int4 *__restrict__ block4, int64_t n_blocks, int64_t e)
+{
+    const int row = block4[e].y;
+    int64_t step = 1;
+    while (e + step < n_blocks && block4[e + step].y == row) { e += step; step *= 2; }
+    for (step >>= 1; step > 0; step >>= 1)
+        if (e + step < n_blocks && block4[e + step].y == row) e += step;
+    return e;
 }
 
 // Second pass: carry slots in unit order, and the list of rows no tuple covers.  A block adds up the counts
@@ -814,8 +832,9 @@ plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_
             const int s = side == 0 ? uc.x : uc.y;
             if (s < 0 || (side == 1 && same)) continue;
             const int row = side == 0 ? ri : ro;
-            const int64_t u0 = tuple_lower_bound(block4, n_blocks, row) / SPMM_WARPS;
-            const int64_t u1 = (tuple_lower_bound(block4, n_blocks, (int64_t)row + 1) - 1) / SPMM_WARPS;
+            const int64_t e = side == 0 ? e0 : e1 - 1;
+            const int64_t u0 = tuple_row_first(block4, e) / SPMM_WARPS;
+            const int64_t u1 = tuple_row_last(block4, n_blocks, e) / SPMM_WARPS;
             carry_span[s] = make_int2(s - (int)(u - u0), (int)(u1 - u0 + 1));
             carry_row[s] = row;
         }
