@@ -39,7 +39,6 @@ struct PartitionRun {
     const int *indptr = nullptr;
     int64_t n_rows = 0, n_blocks = 0;
     void *memory = nullptr;
-    int4 *tuples = nullptr;        // in memory, where the graph was small enough to write them at once
     cudaStream_t stream = nullptr;
 };
 int partition_begin(PartitionRun *run, const int *d_indptr, int64_t n_rows, cudaStream_t s);

@@ -14,9 +14,8 @@
 // its leading rows that belong to a run begun earlier, the tuples all other rows
 // open; (B) one thread block scans the descriptions, which closes the open runs,
 // and leaves every tile its incoming run start and its first output position;
-// (C) every row writes its own tuples.  Up to PART_DIRECT_TILES tiles (C) scans
-// the descriptions itself and writes to scratch before the count is known to the
-// host, which saves a launch and a wait.
+// (C) every row writes its own tuples.  The host waits between (B) and (C), for
+// the number of tuples it has to find room for, and not behind (C).
 // Bound: launch latency up to some 100 000 rows, instruction issue above.
 #pragma once
 #include "../host_common.h"
@@ -233,8 +232,6 @@ part_scan_kernel(const PartTileInfo *tiles, int64_t n_tiles, int *__restrict__ t
 // kept the kernel for 44 us; 21 now.)
 constexpr int PART_CHUNK = 4096;
 
-constexpr int PART_DIRECT_TILES = PART_BLOCK;      // half a million rows
-
 // The tuples of one tile that lie at output positions [lo, hi), hi <= first_out + their number.
 struct PartEmitShared {
     int ip[PART_SMEM_INTS];
@@ -310,45 +307,21 @@ __device__ __forceinline__ void part_emit_tile(const PartTile &t, PartEmitShared
     }
 }
 
-// tile_offset == nullptr: this block scans the descriptions of the (at most PART_DIRECT_TILES) tiles itself, and
-// the last tile's reports the total; otherwise there are `cap` tuples.  Nothing is written outside `cap` tuples (a
-// decreasing indptr, found by (A), may give any position here).  The first `chunks` blocks: PART_CHUNK output positions
-// each; the others: a tile each.
+// `cap` is the number of tuples; nothing is written outside of them, whatever became of indptr since they were counted.
+// The first `chunks` blocks: PART_CHUNK output positions each; the others: a tile each.
 __global__ void __launch_bounds__(PART_BLOCK, 4)
-part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileInfo *info,      // not __restrict__: read after the wait
-                 const int *__restrict__ tile_incoming_head, const int64_t *__restrict__ tile_offset, int tiles, int chunks, int64_t cap,
-                 int4 *__restrict__ block4, HostWords *report)
+part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const int *__restrict__ tile_incoming_head, const int64_t *__restrict__ tile_offset,
+                 int tiles, int chunks, int64_t cap, int4 *__restrict__ block4)
 {
     __shared__ PartEmitShared sh;
-    __shared__ int64_t s_scan64[PART_BLOCK / 32 + 1];
-    __shared__ int64_t s_offset[PART_DIRECT_TILES + 1];
-    __shared__ int s_head[PART_DIRECT_TILES];
     __shared__ int s_list[2], s_listed;
     const int of_tile = (int)blockIdx.x - chunks;
-    PartTile t;
-    if (of_tile >= 0) t = part_load_tile(indptr, n_rows, of_tile, sh.ip);
     const int ip0 = indptr[0];
-    wait_for_predecessor();      // launched early behind (A), which has nothing to do with indptr but read it
-    const bool direct = tile_offset == nullptr;
-    if (direct) {
-        const int b = threadIdx.x;
-        PartTileInfo mine = {-1, 0, 0, 0};
-        if (b < tiles) mine = info[b];
-        int unused;
-        const int head = block_scan_exclusive<PART_BLOCK>(mine.last_head, OpMax(), -1, unused, sh.scan);
-        const int64_t count = b < tiles ? mine.rest + part_lead_tuples(mine, b, head) : 0;
-        int64_t total;
-        s_offset[b] = block_scan_exclusive<PART_BLOCK>(count, OpAdd(), (int64_t)0, total, s_scan64);
-        s_head[b] = head;
-        if (b == 0) s_offset[PART_DIRECT_TILES] = total;
-        __syncthreads();
-        if (of_tile == 0 && b == 0) report->w[PART_WORD_TOTAL] = total;
-    }
-    auto offset = [&](int b) { return direct ? s_offset[b < tiles ? b : PART_DIRECT_TILES] : (b < tiles ? tile_offset[b] : cap); };
-    auto head_of = [&](int b) { return direct ? s_head[b] : tile_incoming_head[b]; };
+    auto offset = [&](int b) { return b < tiles ? tile_offset[b] : cap; };
     if (of_tile >= 0) {
         const int64_t first_out = offset(of_tile), end = offset(of_tile + 1);
-        if (end - first_out <= PART_CHUNK) part_emit_tile(t, sh, head_of(of_tile), first_out, first_out, end, cap, ip0, block4);
+        if (end - first_out <= PART_CHUNK)
+            part_emit_tile(part_load_tile(indptr, n_rows, of_tile, sh.ip), sh, tile_incoming_head[of_tile], first_out, first_out, end, cap, ip0, block4);
         return;
     }
     // tiles of more than PART_CHUNK tuples that reach into this block's positions: two at most
@@ -376,8 +349,7 @@ part_emit_kernel(const int *__restrict__ indptr, int64_t n_rows, const PartTileI
     for (int q = 0; q < min(s_listed, 2); q++) {
         const int b = s_list[q];
         __syncthreads();                 // the tile before is done with
-        t = part_load_tile(indptr, n_rows, b, sh.ip);
-        part_emit_tile(t, sh, head_of(b), offset(b), lo, hi, cap, ip0, block4);
+        part_emit_tile(part_load_tile(indptr, n_rows, b, sh.ip), sh, tile_incoming_head[b], offset(b), lo, hi, cap, ip0, block4);
     }
 }
 

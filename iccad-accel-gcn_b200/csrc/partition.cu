@@ -82,29 +82,13 @@ static int partition_count(const char *who, const int *d_indptr, int64_t n_rows,
     return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
 }
 
-// Phases A and C of a graph of few tiles, into scratch of `cap` tuples; *n_blocks may come out larger than that.
-static int partition_direct(const char *who, const int *d_indptr, int64_t n_rows, int64_t *n_blocks, const PartScratch &sc, int4 *tuples,
-                            int64_t cap, cudaStream_t s)
-{
-    const unsigned tiles = (unsigned)ceil_div(n_rows, PART_TILE);
-    AGCN_HOST_WORDS(words, s);
-    AGCN_KERNEL(part_describe_kernel, tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words.device());
-    AGCN_LAUNCH_CHECK("part_describe_kernel");
-    const unsigned chunks = (unsigned)ceil_div(cap, PART_CHUNK);
-    AGCN_CUDA(launch_early(true, part_emit_kernel, chunks + tiles, PART_BLOCK, 0, s, d_indptr, n_rows, (const PartTileInfo *)sc.info, (const int *)nullptr,
-                           (const int64_t *)nullptr, (int)tiles, (int)chunks, cap, tuples, words.device()));
-    AGCN_LAUNCH_CHECK("part_emit_kernel");
-    AGCN_CUDA(words.sync());
-    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
-}
-
 // Phase C, asynchronous.
 static int partition_emit(const int *d_indptr, int64_t n_rows, int64_t n_blocks, int *d_block4, const PartScratch &sc, cudaStream_t s)
 {
     if (n_blocks == 0) return AGCN_OK;
     const int64_t tiles = ceil_div(n_rows, PART_TILE), chunks = ceil_div(n_blocks, PART_CHUNK);
-    AGCN_KERNEL(part_emit_kernel, (unsigned)(chunks + tiles), PART_BLOCK, s, d_indptr, n_rows, (const PartTileInfo *)nullptr,
-                (const int *)sc.tile_head, (const int64_t *)sc.tile_offset, (int)tiles, (int)chunks, n_blocks, reinterpret_cast<int4 *>(d_block4), (HostWords *)nullptr);
+    AGCN_KERNEL(part_emit_kernel, (unsigned)(chunks + tiles), PART_BLOCK, s, d_indptr, n_rows, (const int *)sc.tile_head,
+                (const int64_t *)sc.tile_offset, (int)tiles, (int)chunks, n_blocks, reinterpret_cast<int4 *>(d_block4));
     AGCN_LAUNCH_CHECK("part_emit_kernel");
     return AGCN_OK;
 }
@@ -140,17 +124,13 @@ int partition_device(const int *d_indptr, int64_t n_rows, int *d_block4, int64_t
     return partition_pipeline("agcn_partition", d_indptr, n_rows, d_block4, cap_blocks, n_blocks, part_scratch(c, tiles), s);
 }
 
-// Room for the tuples of a graph of few tiles: two per row, twice what an ordered graph of 384 nonzeros per row has.
-static int64_t partition_direct_cap(int64_t n_rows) { return n_rows <= (int64_t)PART_DIRECT_TILES * PART_TILE ? 2 * n_rows + 1024 : 0; }
-
 int partition_begin(PartitionRun *run, const int *d_indptr, int64_t n_rows, cudaStream_t s)
 {
     int rc = partition_check("agcn_partition", d_indptr, n_rows, nullptr, run);
     if (rc != AGCN_OK) return rc;
-    const int64_t tiles = ceil_div(n_rows, PART_TILE), cap = partition_direct_cap(n_rows);
+    const int64_t tiles = ceil_div(n_rows, PART_TILE);
     Carver size;
     part_scratch(size, tiles);
-    size.take<int4>(cap);
     run->indptr = d_indptr; run->n_rows = n_rows; run->n_blocks = 0; run->stream = s;
     const cudaError_t e = pool_alloc(&run->memory, size.bytes(), s);
     if (e != cudaSuccess) {
@@ -158,15 +138,7 @@ int partition_begin(PartitionRun *run, const int *d_indptr, int64_t n_rows, cuda
         return AGCN_ERR_CUDA;
     }
     Carver c(run->memory);
-    const PartScratch sc = part_scratch(c, tiles);
-    int4 *tuples = c.take<int4>(cap);
-    if (cap > 0) {
-        rc = partition_direct("agcn_partition", d_indptr, n_rows, &run->n_blocks, sc, tuples, cap, s);
-        run->tuples = rc == AGCN_OK && run->n_blocks <= cap ? tuples : nullptr;
-        if (rc == AGCN_OK && run->tuples == nullptr) rc = partition_count("agcn_partition", d_indptr, n_rows, &run->n_blocks, sc, s);
-    } else {
-        rc = partition_count("agcn_partition", d_indptr, n_rows, &run->n_blocks, sc, s);
-    }
+    rc = partition_count("agcn_partition", d_indptr, n_rows, &run->n_blocks, part_scratch(c, tiles), s);
     if (rc != AGCN_OK) { pool_free(run->memory, s); run->memory = nullptr; }
     return rc;
 }
@@ -176,15 +148,8 @@ int partition_finish(PartitionRun *run, int *d_block4)
     if (run->memory == nullptr) return AGCN_OK;
     int rc = AGCN_OK;
     if (d_block4 != nullptr && run->n_blocks > 0) {
-        if (run->tuples != nullptr) {
-            if (cudaMemcpyAsync(d_block4, run->tuples, (size_t)run->n_blocks * sizeof(int4), cudaMemcpyDeviceToDevice, run->stream) != cudaSuccess) {
-                set_error("agcn_partition: copy of the tuples: %s", cudaGetErrorString(cudaGetLastError()));
-                rc = AGCN_ERR_CUDA;
-            }
-        } else {
-            Carver c(run->memory);
-            rc = partition_emit(run->indptr, run->n_rows, run->n_blocks, d_block4, part_scratch(c, ceil_div(run->n_rows, PART_TILE)), run->stream);
-        }
+        Carver c(run->memory);
+        rc = partition_emit(run->indptr, run->n_rows, run->n_blocks, d_block4, part_scratch(c, ceil_div(run->n_rows, PART_TILE)), run->stream);
     }
     pool_free(run->memory, run->stream);
     run->memory = nullptr;
