@@ -861,8 +861,8 @@ plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_
 }
 
 // The whole plan of a small graph in one launch: block 0 validates the tuples, cuts them into pieces of at most
-// `most` nonzeros (cap_pieces of them fit), lists the rows no tuple covers and hands out the carry slots; the other
-// blocks check the column ids.  Every array has its final place already, sized by bounds the host knows, so the
+// `most` nonzeros (cap_pieces of them fit), lists the rows no tuple covers and hands out the carry slots; the next
+// clear_blocks zero the arrival counters of the slots, the other blocks check the column ids.  Every array has its final place already, sized by bounds the host knows, so the
 // host waits once.  (Two kernels with a wait between them before, the cutting 8 tuples per thread: a plan of 16 384
 // rows took 70 us; 26 now, 12 of them on the GPU.)  Bound by latency: a chain of scans over about ten tuples per thread.
 constexpr int PLAN_SMALL_BLOCK = 1024;
@@ -870,10 +870,14 @@ constexpr int PLAN_SMALL_BLOCK = 1024;
 __global__ void __launch_bounds__(PLAN_SMALL_BLOCK)
 plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows, int64_t nnz, const int *__restrict__ idx, int64_t n_idx,
                   int64_t n_cols, int most, int4 *pieces, int cap_pieces, int2 *unit_carry, int2 *carry_span, int *carry_row, int *zero_rows,
-                  HostWords *out)
+                  int *counters, int n_counters, unsigned clear_blocks, HostWords *out)
 {
+    if (blockIdx.x > clear_blocks) {
+        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - 1 - clear_blocks, gridDim.x - 1 - clear_blocks, out);
+        return;
+    }
     if (blockIdx.x > 0) {
-        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - 1, gridDim.x - 1, out);
+        for (int k = (blockIdx.x - 1) * PLAN_SMALL_BLOCK + threadIdx.x; k < n_counters; k += clear_blocks * PLAN_SMALL_BLOCK) counters[k] = 0;
         return;
     }
     __shared__ int s_scan[PLAN_SMALL_BLOCK / 32 + 1];

@@ -143,8 +143,6 @@ static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int4 **pieces, cudaS
             return AGCN_ERR_CUDA;
         }
     }
-    if (p->n_carry > 0)
-        AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(p->carry, p->n_carry), 0, (size_t)p->n_carry * SPMM_CARRY_PASSES * sizeof(int), s));
     return AGCN_OK;
 }
 
@@ -162,10 +160,11 @@ static int plan_fill_small(agcn_spmm_plan *p, int most, const int *d_indices, in
     int rc = plan_memory(p, cap, &pieces, s);
     if (rc != AGCN_OK) return rc;
     AGCN_HOST_WORDS(words, s);
-    const int64_t col_blocks = ceil_div(n_idx, PLAN_SMALL_BLOCK * 16);
-    AGCN_KERNEL(plan_small_kernel, (unsigned)(1 + (col_blocks < 2368 ? col_blocks : 2368)), PLAN_SMALL_BLOCK, s, p->block4, (int)p->n_blocks,
-                p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, most, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
-                p->zero_rows, words.device());
+    const int64_t col_blocks = ceil_div(n_idx, PLAN_SMALL_BLOCK * 16), counters = p->n_carry * SPMM_CARRY_PASSES;
+    const int64_t clear_blocks = ceil_div(counters, PLAN_SMALL_BLOCK * 16);
+    AGCN_KERNEL(plan_small_kernel, (unsigned)(1 + clear_blocks + (col_blocks < 2368 ? col_blocks : 2368)), PLAN_SMALL_BLOCK, s, p->block4,
+                (int)p->n_blocks, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, most, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
+                p->zero_rows, spmm_carry_counters(p->carry, p->n_carry), (int)counters, (unsigned)clear_blocks, words.device());
     AGCN_LAUNCH_CHECK("plan_small_kernel");
     AGCN_CUDA(words.sync());
     rc = plan_errors(words);
@@ -214,6 +213,8 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     int4 *pieces = nullptr;
     rc = plan_memory(p, 0, &pieces, s);
     if (rc != AGCN_OK) return rc;
+    if (p->n_carry > 0)
+        AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(p->carry, p->n_carry), 0, (size_t)p->n_carry * SPMM_CARRY_PASSES * sizeof(int), s));
     if (p->n_carry > 0 || p->n_zero > 0) {
         AGCN_KERNEL(plan_assign_kernel, (unsigned)tiles, PLAN_BLOCK, s, p->tuples, p->n_tuples, p->n_units, p->n_rows, (const int64_t *)tile_zero,
                     (const int *)tile_carry, p->unit_carry, p->carry_span, p->carry_row, p->n_zero > 0 ? p->zero_rows : nullptr);
