@@ -491,20 +491,9 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
     }
     top = warp_reduce(top, OpMax());
     if (lane == 0) atomicMax(&s_say[0], top);
-    cluster.sync();
-    if (threadIdx.x < 2 * SMALL_CLUSTER) s_get[threadIdx.x >> 1][threadIdx.x & 1] = *cluster.map_shared_rank(&s_say[threadIdx.x & 1], threadIdx.x >> 1);
-    __syncthreads();
-    bool negative = false;
-#pragma unroll
-    for (int b = 0; b < SMALL_CLUSTER; b++) { top = max(top, s_get[b][0]); negative |= s_get[b][1] != 0; }
-    const int64_t own = (int64_t)indptr[n] - (int64_t)indptr[0];
-    const bool bad = negative || (check_nnz && own != nnz);
-    if (block == 0 && threadIdx.x == 0) {
-        out->w[SORT_WORD_NNZ] = own;
-        if (negative) out->w[SORT_WORD_NEGATIVE] = 1;
-        ctl->bad = bad ? SORT_BAD_INPUT : 0;
-    }
-    for (int shift = 0; shift < 32 && (top >> shift) != 0; shift += RADIX_BITS) {
+    bool bad = false;
+    // the first pass says with its counts which other ones move anything
+    for (int shift = 0; shift == 0 || (shift < 32 && (top >> shift) != 0); shift += RADIX_BITS) {
         for (int b = threadIdx.x; b < SMALL_WARPS * RADIX_BINS / 2; b += SMALL_BLOCK) reinterpret_cast<unsigned *>(&s_count[0][0])[b] = 0;
         __syncthreads();
         unsigned short rank[SMALL_ITEMS];
@@ -534,6 +523,8 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
             s_total[threadIdx.x] = total;
         }
         cluster.sync();
+        if (shift == 0 && threadIdx.x < 2 * SMALL_CLUSTER)
+            s_get[threadIdx.x >> 1][threadIdx.x & 1] = *cluster.map_shared_rank(&s_say[threadIdx.x & 1], threadIdx.x >> 1);
         unsigned all = 0, before = 0, unused;
         if (threadIdx.x < RADIX_BINS) {
 #pragma unroll
@@ -546,6 +537,18 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
         const unsigned bin = block_scan_exclusive<SMALL_BLOCK>(all, OpAdd(), 0u, unused, s_scan);
         if (threadIdx.x < RADIX_BINS) s_base[threadIdx.x] = bin + before;
         __syncthreads();
+        if (shift == 0) {
+            bool negative = false;
+#pragma unroll
+            for (int b = 0; b < SMALL_CLUSTER; b++) { top = max(top, s_get[b][0]); negative |= s_get[b][1] != 0; }
+            const int64_t own = (int64_t)indptr[n] - (int64_t)indptr[0];
+            bad = negative || (check_nnz && own != nnz);
+            if (block == 0 && threadIdx.x == 0) {
+                out->w[SORT_WORD_NNZ] = own;
+                if (negative) out->w[SORT_WORD_NEGATIVE] = 1;
+                ctl->bad = bad ? SORT_BAD_INPUT : 0;
+            }
+        }
 #pragma unroll
         for (int k = 0; k < SMALL_ITEMS; k++) {
             if (k < items && first + k * 32 < n) {
@@ -574,6 +577,7 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
     cluster.sync();
     if (threadIdx.x < SMALL_CLUSTER) s_get[threadIdx.x][0] = *cluster.map_shared_rank(&s_say[2], threadIdx.x);
     __syncthreads();
+    cluster.barrier_arrive();    // this block reads no other one's shared memory any more
     unsigned e = __shfl_sync(FULL_MASK, start, 0);
     for (int b = 0; b < block; b++) e += s_get[b][0];
 #pragma unroll
@@ -592,7 +596,7 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
         if (map.tile_row != nullptr && !bad)
             for (unsigned t = (b + PERMUTE_TILE - 1) / PERMUTE_TILE; t * PERMUTE_TILE < b + key[k]; t++) map.tile_row[t] = i;
     }
-    cluster.sync();              // no block ends while another may read its shared memory
+    cluster.barrier_wait();      // no block ends while another may read its shared memory
 }
 
 // CSR permute.  Each warp produces PERMUTE_TILE consecutive column ids or values by itself.  The rows it touches (all
