@@ -33,17 +33,25 @@ void plan_free(agcn_spmm_plan *p)
 // Nonzeros per piece when the tuples of a plan are to be cut into pieces, 0 when they are not.  A product ends with
 // its longest warp, so pieces are as small as the nonzeros that an SM has to go through allow; beyond 7 500 of them
 // (20 full tuples; the SM holds 32 to 40 warps) the extra warps cost more than they balance, unless there are few
-// tuples for them.  us per product, uncut / 192 / 128 / 64, B200, nonzeros per SM in brackets:
+// tuples for them.  us per product (before launches overlapped), uncut / 192 / 128 / 64, B200, nonzeros per SM in brackets:
 // 16 384 rows of 8 [900], dim 60: 17.7 / 9.4 / 8.3 / 7.3;  80 000 rows of 4 [2 100], dim 64: - / 12.4 / 11.2 / 10.3;
 // 80 000 of 7 [3 900]: - / 15.1 / 13.5 / 15.2, dim 128: - / 25 / 23 / 25;  135 000 of 4 [3 400]: 50 / 34 / 31 / -;
 // 165 000 of 6 [6 300], dim 32: 17.4 / 13.4 / 14.2 / -, dim 128: 54 / 45 / 47 / -;  200 000 of 6 [7 700], dim 64:
 // 29.2 / 30.0 / 31.4 / -;  100 000 of 25 [17 000], dim 32: 25 / 33 / - / -.
+// Few nonzeros: as small as leaves the blocks two per SM in one wave (the form with 16 gathers in flight per lane).
+// 32 / 64 / 96, nonzeros per SM in brackets: 2 048 rows of 4 [70], dim 60, 128: 4.9 / 5.5 / 4.8, 5.2 / 5.9 / 6.7;  4 096 of 10
+// [300]: 5.8 / 6.1 / 6.6, 6.2 / 7.0 / 7.8;  8 192 of 8 [500]: 6.4 / 6.8 / 7.1, 7.1 / 7.5 / 8.7;  16 384 of 4 [550]: 6.8 / 6.8 / 7.2,
+// 7.2 / 7.6 / 8.9, dim 16: 5.9 / 5.5 / 5.8;  16 384 of 8 [1 000]: 8.2 / 7.6 / 8.0, 9.0 / 9.7 / 9.7, dim 16: 6.2 / 5.9 / 6.1;  8 192 of
+// 20 [1 160]: 8.2 / 8.7 / 7.8, 10.5 / 10.8 / 9.4;  16 384 of 14 [1 660]: 9.6 / 9.3 / 10.0, 12.8 / 11.6 / 13.5.
 // Beyond 80 tuples per SM one thread block takes so long to cut them that a plan used once loses (150 000 rows of 5:
 // 236 -> 244 us from the graph to Y).
 static int spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
 {
     const int64_t per_sm = nnz / sm_count;
     if (n_blocks > (int64_t)80 * sm_count) return 0;
+    if (per_sm <= 500) return 32;
+    if (per_sm <= 1050) return 64;
+    if (per_sm <= 1575) return 96;
     if (per_sm <= 1900) return 64;
     if (per_sm <= 2700) return 96;
     if (per_sm <= 4000) return 128;
