@@ -53,9 +53,10 @@ static int degree_sort_device(const int *d_indptr, const int *d_indices, const f
     }
     AGCN_HOST_WORDS(words, s);
     if (small) {
-        AGCN_CUDA(cudaFuncSetAttribute(sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMALL_SMEM_BYTES));
-        sort_small_kernel<<<SMALL_CLUSTER, SMALL_BLOCK, SMALL_SMEM_BYTES, s>>>(d_indptr, (int)n_rows, (int)ceil_div(n_rows, SMALL_CLUSTER * SMALL_BLOCK), nnz,
-                                                                               permute ? 1 : 0, ctl, d_perm, d_new_indptr, map, words.device());
+        const int items = (int)ceil_div(n_rows, SMALL_CLUSTER * SMALL_BLOCK), smem = small_smem_bytes(items);
+        if (smem > 40 << 10) AGCN_CUDA(cudaFuncSetAttribute(sort_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, small_smem_bytes(SMALL_ITEMS)));
+        sort_small_kernel<<<SMALL_CLUSTER, SMALL_BLOCK, smem, s>>>(d_indptr, (int)n_rows, items, nnz, permute ? 1 : 0, ctl, d_perm, d_new_indptr, map,
+                                                                   words.device());
         AGCN_LAUNCH_CHECK("sort_small_kernel");
     } else {
         AGCN_CUDA(cudaMemsetAsync(ctl, 0, cleared, s));

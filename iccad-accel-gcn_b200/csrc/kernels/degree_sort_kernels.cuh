@@ -454,7 +454,7 @@ constexpr int SMALL_BLOCK = 1024;
 constexpr int SMALL_WARPS = SMALL_BLOCK / 32;
 constexpr int SMALL_ITEMS = 8;
 constexpr int SMALL_MAX_ROWS = SMALL_CLUSTER * SMALL_BLOCK * SMALL_ITEMS;
-constexpr int SMALL_SMEM_BYTES = SMALL_BLOCK * SMALL_ITEMS * 8 + SMALL_WARPS * RADIX_BINS * 2;
+constexpr int small_smem_bytes(int items) { return SMALL_BLOCK * items * 8 + SMALL_WARPS * RADIX_BINS * 2; }
 
 // items = rows per thread: ceil(n / 8192), at most SMALL_ITEMS
 __global__ void __cluster_dims__(SMALL_CLUSTER, 1, 1) __launch_bounds__(SMALL_BLOCK, 1)
@@ -464,15 +464,15 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
     namespace cg = cooperative_groups;
     cg::cluster_group cluster = cg::this_cluster();
     launch_dependents();         // the permute takes its place on the SMs that this leaves idle
-    extern __shared__ unsigned s_small[];
-    unsigned *s_key = s_small;
-    int *s_row = reinterpret_cast<int *>(s_small + SMALL_BLOCK * SMALL_ITEMS);
-    unsigned short (*s_count)[RADIX_BINS] = reinterpret_cast<unsigned short (*)[RADIX_BINS]>(s_small + 2 * SMALL_BLOCK * SMALL_ITEMS);
     __shared__ unsigned s_total[RADIX_BINS], s_base[RADIX_BINS], s_scan[SMALL_WARPS + 1];
     __shared__ unsigned s_say[3];                // for the other blocks: largest degree, negative seen, sum of degrees
     __shared__ unsigned s_get[SMALL_CLUSTER][2];
     const int w = warp_id(), lane = lane_id(), block = (int)cluster.block_rank();
     const int per_block = SMALL_BLOCK * items, first = block * per_block + w * 32 * items + lane;       // item k of this thread is row first + 32 k
+    extern __shared__ unsigned s_small[];        // small_smem_bytes(items): no more than there are rows, or the SM changes its carve-out
+    unsigned *s_key = s_small;
+    int *s_row = reinterpret_cast<int *>(s_small + per_block);
+    unsigned short (*s_count)[RADIX_BINS] = reinterpret_cast<unsigned short (*)[RADIX_BINS]>(s_small + 2 * per_block);
     if (threadIdx.x < 3) s_say[threadIdx.x] = 0;
     __syncthreads();
     unsigned key[SMALL_ITEMS], top = 0;

@@ -9,12 +9,12 @@
 //                          the tuple covers j = min(R(D), rows left in the run) rows
 //   D > 384             -> ceil(D / 384) tuples of <= 384 nonzeros each
 // with R(D), w(D) the pattern tables of block_level_partition.py:7-21 and the
-// fall-backs of :56-63.  Three launches over tiles of PART_TILE rows staged
+// fall-backs of :56-63.  Two launches over tiles of PART_TILE rows staged
 // through shared memory: (A) every tile describes itself -- its last run start,
 // its leading rows that belong to a run begun earlier, the tuples all other rows
-// open; (B) one thread block scans the descriptions, which closes the open runs,
-// and leaves every tile its incoming run start and its first output position;
-// (C) every row writes its own tuples.  The host waits between (B) and (C), for
+// open -- and (B) the last thread block scans the descriptions, which closes the
+// open runs, and leaves every tile its incoming run start and its first output
+// position; (C) every row writes its own tuples.  The host waits between (B) and (C), for
 // the number of tuples it has to find room for, and not behind (C).
 // Bound: launch latency up to some 100 000 rows, instruction issue above.
 #pragma once
@@ -30,7 +30,10 @@ constexpr int PART_ITEMS = 8;
 constexpr int PART_TILE = PART_BLOCK * PART_ITEMS;
 constexpr int PART_MAX_ROWS_PER_TUPLE = 12;
 constexpr int PART_HALO = PART_MAX_ROWS_PER_TUPLE + 1;   // rows looked at past a tile
-constexpr int PART_WORD_TOTAL = 0, PART_WORD_NEGATIVE = 1;    // host words
+constexpr int PART_WORD_TOTAL = 0, PART_WORD_NEGATIVE = 1, PART_WORD_TIMEOUT = 2;    // host words
+// Polls before the last block gives up on a tile's description (each backs off; well over a second): the other blocks
+// wait for nothing, so the limit is there for a bug, not for load.
+constexpr int PART_SPIN_LIMIT = 1 << 22;
 
 // rows per tuple R(D) and nonzeros per virtual warp w(D), 1 <= D <= 384
 __device__ __forceinline__ int part_rows_per_tuple(int d)
@@ -150,14 +153,43 @@ __device__ __forceinline__ int part_row_counts(const PartTile &t, int incoming_h
     return head_local;
 }
 
-// (A) the description of every tile
+// Tuples opened by the leading rows of tile b, once the start of their run is known.
+__device__ __forceinline__ int64_t part_lead_tuples(const PartTileInfo &info, int64_t b, int head)
+{
+    if (info.lead <= 0) return 0;
+    // rows o .. o + lead - 1 of their run open a tuple where their number is a multiple of R
+    const int64_t o = b * PART_TILE - head;
+    const int r = part_rows_per_tuple(info.lead_deg);
+    return (o + info.lead + r - 1) / r - (o + r - 1) / r;
+}
+
+// Says that tile b's description is there: the call's own number, which memory that held other calls' cannot hold.
+__device__ __forceinline__ void part_say(unsigned long long *tag, unsigned long long call)
+{
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" :: "l"(tag), "l"(call) : "memory");
+}
+__device__ __forceinline__ bool part_said(const unsigned long long *tag, unsigned long long call)
+{
+    for (int spin = 0; spin < PART_SPIN_LIMIT; spin++) {
+        unsigned long long v;
+        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(tag) : "memory");
+        if (v == call) return true;
+        if (spin > 16) __nanosleep(200);
+    }
+    return false;
+}
+
+// (A) the description of every tile, and (B) by the last block (the others are running or done when it starts) the run
+// start that is open when every tile begins and every tile's first output position.  (As a launch of its own, one
+// block, (B) cost the host 3 us and the GPU 6 more.)
 __global__ void __launch_bounds__(PART_BLOCK)
-part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInfo *__restrict__ tiles, HostWords *out)
+part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInfo *tiles, unsigned long long *tags, unsigned long long call,
+                     int *__restrict__ tile_head, int64_t *__restrict__ tile_offset, HostWords *out)
 {
     __shared__ int s_ip[PART_SMEM_INTS];
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
+    __shared__ int64_t s_scan64[PART_BLOCK / 32 + 1];
     __shared__ int s_red[4][PART_BLOCK / 32];
-    launch_dependents();
     const PartTile t = part_load_tile(indptr, n_rows, blockIdx.x, s_ip);
     int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
     unsigned heads;
@@ -182,46 +214,30 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
             info.rest += s_red[3][w];
         }
         tiles[blockIdx.x] = info;
+        part_say(tags + blockIdx.x, call);
     }
-}
-
-// Tuples opened by the leading rows of tile b, once the start of their run is known.
-__device__ __forceinline__ int64_t part_lead_tuples(const PartTileInfo &info, int64_t b, int head)
-{
-    if (info.lead <= 0) return 0;
-    // rows o .. o + lead - 1 of their run open a tuple where their number is a multiple of R
-    const int64_t o = b * PART_TILE - head;
-    const int r = part_rows_per_tuple(info.lead_deg);
-    return (o + info.lead + r - 1) / r - (o + r - 1) / r;
-}
-
-// (B) one block: the run start that is open when every tile begins, and every tile's first output position.
-// 1024 tiles (two million rows) per step.
-constexpr int PART_SCAN_BLOCK = 1024;
-
-__global__ void __launch_bounds__(PART_SCAN_BLOCK)
-part_scan_kernel(const PartTileInfo *tiles, int64_t n_tiles, int *__restrict__ tile_head,
-                 int64_t *__restrict__ tile_offset, HostWords *out)
-{
-    __shared__ int s_head[PART_SCAN_BLOCK / 32 + 1];
-    __shared__ int64_t s_sum[PART_SCAN_BLOCK / 32 + 1];
-    wait_for_predecessor();      // launched early behind (A)
+    if (blockIdx.x + 1 < gridDim.x) return;
     int carry_head = -1;
     int64_t carry = 0;
-    for (int64_t base = 0; base < n_tiles; base += PART_SCAN_BLOCK) {
+    bool all = true;
+    for (int64_t base = 0; base < gridDim.x; base += PART_BLOCK) {
         const int64_t b = base + threadIdx.x;
         PartTileInfo info = {-1, 0, 0, 0};
-        if (b < n_tiles) info = tiles[b];
+        if (b < gridDim.x) {
+            if (all && part_said(tags + b, call)) info = tiles[b];
+            else all = false;
+        }
         int head_total;
-        int head = block_scan_exclusive<PART_SCAN_BLOCK>(info.last_head, OpMax(), -1, head_total, s_head);
-        head = max(head, carry_head);
-        const int64_t count = info.rest + part_lead_tuples(info, b, head);
+        int head_in = block_scan_exclusive<PART_BLOCK>(info.last_head, OpMax(), -1, head_total, s_scan);
+        head_in = max(head_in, carry_head);
+        const int64_t count = info.rest + part_lead_tuples(info, b, head_in);
         int64_t total;
-        const int64_t ex = block_scan_exclusive<PART_SCAN_BLOCK>(count, OpAdd(), (int64_t)0, total, s_sum);
-        if (b < n_tiles) { tile_head[b] = head; tile_offset[b] = carry + ex; }
+        const int64_t ex = block_scan_exclusive<PART_BLOCK>(count, OpAdd(), (int64_t)0, total, s_scan64);
+        if (b < gridDim.x) { tile_head[b] = head_in; tile_offset[b] = carry + ex; }
         carry += total;
         carry_head = max(carry_head, head_total);
     }
+    if (!all) out->w[PART_WORD_TIMEOUT] = 1;
     if (threadIdx.x == 0) out->w[PART_WORD_TOTAL] = carry;
 }
 

@@ -5,6 +5,7 @@
 #include "internal.h"
 #include "kernels/partition_kernels.cuh"
 
+#include <atomic>
 #include <mutex>
 #include <new>
 
@@ -18,6 +19,7 @@ namespace agcn {
 // allocation-free one points it at a fixed array in the library's device image.
 struct PartScratch {
     PartTileInfo *info;
+    unsigned long long *tags;
     int *tile_head;
     int64_t *tile_offset;
     HostWords *words = nullptr;    // on the device: where the answer is stored instead of in leased host words
@@ -27,6 +29,7 @@ static PartScratch part_scratch(Carver &c, int64_t tiles)
 {
     PartScratch sc;
     sc.info = c.take<PartTileInfo>(tiles);
+    sc.tags = c.take<unsigned long long>(tiles);
     sc.tile_offset = c.take<int64_t>(tiles);
     sc.tile_head = c.take<int>(tiles);
     return sc;
@@ -41,8 +44,12 @@ static int partition_check(const char *who, const int *d_indptr, int64_t n_rows,
     return AGCN_OK;
 }
 
-static int partition_answer(const char *who, int64_t negative, int64_t total, int64_t *n_blocks)
+static int partition_answer(const char *who, int64_t negative, int64_t timeout, int64_t total, int64_t *n_blocks)
 {
+    if (timeout != 0) {
+        set_error("%s: a wait between tiles ran out", who);
+        return AGCN_ERR_CUDA;
+    }
     if (negative != 0) {
         set_error("%s: indptr decreases somewhere (negative degree); "
                   "the reference script prints 'cur_degree number is wrong' and stops", who);
@@ -52,15 +59,18 @@ static int partition_answer(const char *who, int64_t negative, int64_t total, in
     return AGCN_OK;
 }
 
+// High bits of a call's number: what other uses of the scratch do not leave behind (no float, id or offset looks so).
+constexpr unsigned long long PART_CALL_MARK = 0x7ff4a9c3ull << 32;
+
 // Phases A and B: how many tuples there are and where every tile's begin.  Waits for the stream.
 // `who` names the entry point in error messages.
 static int partition_launch_count(const int *d_indptr, int64_t n_rows, const PartScratch &sc, HostWords *words, cudaStream_t s)
 {
     const int64_t tiles = ceil_div(n_rows, PART_TILE);
-    AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, words);
+    static std::atomic<unsigned long long> calls{0};       // numbers the calls of the process
+    AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, sc.tags, PART_CALL_MARK + ++calls, sc.tile_head,
+                sc.tile_offset, words);
     AGCN_LAUNCH_CHECK("part_describe_kernel");
-    AGCN_CUDA(launch_early(true, part_scan_kernel, 1, PART_SCAN_BLOCK, 0, s, (const PartTileInfo *)sc.info, tiles, sc.tile_head, sc.tile_offset, words));
-    AGCN_LAUNCH_CHECK("part_scan_kernel");
     return AGCN_OK;
 }
 
@@ -73,13 +83,13 @@ static int partition_count(const char *who, const int *d_indptr, int64_t n_rows,
         if (rc != AGCN_OK) return rc;
         AGCN_CUDA(cudaMemcpyAsync(&words, sc.words, sizeof(words), cudaMemcpyDeviceToHost, s));
         AGCN_CUDA(cudaStreamSynchronize(s));
-        return partition_answer(who, words.w[PART_WORD_NEGATIVE], words.w[PART_WORD_TOTAL], n_blocks);
+        return partition_answer(who, words.w[PART_WORD_NEGATIVE], words.w[PART_WORD_TIMEOUT], words.w[PART_WORD_TOTAL], n_blocks);
     }
     AGCN_HOST_WORDS(words, s);
     const int rc = partition_launch_count(d_indptr, n_rows, sc, words.device(), s);
     if (rc != AGCN_OK) return rc;
     AGCN_CUDA(words.sync());
-    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
+    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TIMEOUT], words[PART_WORD_TOTAL], n_blocks);
 }
 
 // Phase C, asynchronous.
@@ -239,10 +249,10 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
 // fails or steals from its pool), a latency-critical loop that cannot afford
 // the device-wide synchronisation cudaMalloc / cudaFree imply, or a plug-in
 // host that forbids allocation calls after start-up.  For them the tile
-// scratch of the partitioner (28 bytes per 2048 rows) and its result words live in a
+// scratch of the partitioner (36 bytes per 2048 rows) and its result words live in a
 // fixed array in the library's device image instead of a per-call allocation or leased
 // host words (which are pinned when there are none free).  Every GPU that
-// loads the library holds that array (about 224 KB) until the process exits,
+// loads the library holds that array (about 288 KB) until the process exits,
 // which is why it is sized for AGCN_PARTITION_NOALLOC_MAX_ROWS rows and no
 // more.
 //
@@ -259,7 +269,7 @@ constexpr int64_t PART_NOALLOC_MAX_ROWS = AGCN_PARTITION_NOALLOC_MAX_ROWS;
 constexpr int64_t PART_NOALLOC_MAX_TILES = (PART_NOALLOC_MAX_ROWS + PART_TILE - 1) / PART_TILE;
 constexpr int PART_NOALLOC_MAX_DEVICES = 64;
 
-constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + sizeof(int64_t) + sizeof(int)) + 3 * 256 + 256;
+constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + 2 * sizeof(int64_t) + sizeof(int)) + 4 * 256 + 256;
 
 }  // namespace agcn
 
