@@ -35,23 +35,22 @@ def degree_sort(indptr, indices, vals=None, relabel_cols: bool = True):
 def degree_sort_device(indptr, indices, vals=None, relabel_cols: bool = True, stream=None):
     """torch CUDA tensors (int32 / float32).  Same return convention, on the device."""
     import torch
-    lib = _lib.load()
     for t, dt in ((indptr, torch.int32), (indices, torch.int32)) + (((vals, torch.float32),) if vals is not None else ()):
         if not (t.is_cuda and t.dtype == dt and t.is_contiguous()):
             raise TypeError("degree_sort_device needs contiguous CUDA tensors (int32 indptr/indices, float32 vals)")
-    dev = indptr.device
     n_rows, nnz = indptr.numel() - 1, indices.numel()
     if n_rows <= 0:
         raise IndexError("empty graph")
-    index = _lib.device_index(dev)
+    index = _lib.device_index(indptr.device)
     s = stream.cuda_stream if stream is not None else _lib.raw_stream(index)
-    perm = torch.empty(n_rows, dtype=torch.int32, device=dev)
-    new_indptr = torch.empty(n_rows + 1, dtype=torch.int32, device=dev)
-    new_indices = torch.empty(nnz, dtype=torch.int32, device=dev)
-    new_vals = None if vals is None else torch.empty(nnz, dtype=torch.float32, device=dev)
+    perm = indptr.new_empty(n_rows)
+    new_indptr = indptr.new_empty(n_rows + 1)
+    new_indices = indptr.new_empty(nnz)
+    new_vals = None if vals is None else indptr.new_empty(nnz, dtype=torch.float32)
     with _lib.on_device(index):
-        _lib.check(lib.agcn_degree_sort_device(
+        _lib.check(_lib.call()(
+            _lib.address("agcn_degree_sort_device"),
             indptr.data_ptr(), indices.data_ptr(), None if vals is None else vals.data_ptr(), n_rows, nnz,
-            int(bool(relabel_cols)), perm.data_ptr(), new_indptr.data_ptr(), new_indices.data_ptr(),
+            1 if relabel_cols else 0, perm.data_ptr(), new_indptr.data_ptr(), new_indices.data_ptr(),
             None if new_vals is None else new_vals.data_ptr(), s))
     return perm, new_indptr, new_indices, new_vals

@@ -43,7 +43,6 @@ def block_level_partition_device(indptr, stream=None):
     operation.  With another `stream` they are complete when the call returns: neither tensor is known to torch's
     allocator as in use there, and the caller may go on with them anywhere."""
     import torch
-    lib = _lib.load()
     if not (indptr.is_cuda and indptr.dtype == torch.int32 and indptr.is_contiguous()):
         raise TypeError("indptr must be a contiguous int32 CUDA tensor")
     n_rows = indptr.numel() - 1
@@ -52,15 +51,17 @@ def block_level_partition_device(indptr, stream=None):
     dev = _lib.device_index(indptr.device)
     current = _lib.raw_stream(dev)
     s = stream.cuda_stream if stream is not None else current
-    n_blocks, run = ctypes.c_int64(0), ctypes.c_void_p()
+    call, answer = _lib.call(), (ctypes.c_int64 * 2)()             # the run, the number of tuples
+    at = ctypes.addressof(answer)
     with _lib.on_device(dev):
-        _lib.check(lib.agcn_partition_begin(indptr.data_ptr(), n_rows, ctypes.byref(run), ctypes.byref(n_blocks), s))
+        _lib.check(call(_lib.address("agcn_partition_begin"), indptr.data_ptr(), n_rows, at, at + 8, s))
+        run, n_blocks = answer
         try:
-            out = torch.empty((n_blocks.value, 4), dtype=torch.int32, device=indptr.device)
+            out = indptr.new_empty((n_blocks, 4))
         except BaseException:
-            lib.agcn_partition_finish(run, None)
+            call(_lib.address("agcn_partition_finish"), run, None)
             raise
-        _lib.check(lib.agcn_partition_finish(run, out.data_ptr() if n_blocks.value else None))
+        _lib.check(call(_lib.address("agcn_partition_finish"), run, out.data_ptr() if n_blocks else None))
         if s != current:
             stream.synchronize()
     return out

@@ -22,10 +22,9 @@ class SpmmPlan:
 
     def __init__(self, block4, indices, n_rows: int, n_cols: int, stream=None):
         import torch
-        lib = _lib.load()
         if not (block4.is_cuda and block4.dtype == torch.int32 and block4.is_contiguous()):
             raise TypeError("block4 must be a contiguous int32 CUDA tensor")
-        self._lib = lib
+        self._lib = _lib.load()
         self.block4 = block4            # keep alive: the plan borrows it
         self.device = block4.device
         self._dev_index = _lib.device_index(block4.device)
@@ -34,12 +33,12 @@ class SpmmPlan:
         self.nnz = int(indices.numel())
         s = stream.cuda_stream if stream is not None else _lib.raw_stream(self._dev_index)
         h = ctypes.c_void_p()
+        self._call = _lib.call()
         with _lib.on_device(self._dev_index):
-            _lib.check(lib.agcn_spmm_create(ctypes.byref(h), block4.data_ptr(), self.n_blocks, indices.data_ptr(),
-                                            self.n_rows, self.n_cols, self.nnz, s))
+            _lib.check(self._call(_lib.address("agcn_spmm_create"), ctypes.addressof(h), block4.data_ptr(), self.n_blocks, indices.data_ptr(),
+                                  self.n_rows, self.n_cols, self.nnz, s))
         self._h = h
         self._run = _lib.address("agcn_spmm_run_act")
-        self._call = _lib.call()
         self._raw_stream = torch._C._cuda_getCurrentRawStream
 
     def run(self, indices, vals, x, y, dim: int | None = None, ldx: int | None = None, ldy: int | None = None,
