@@ -500,6 +500,8 @@ __global__ void __launch_bounds__(SPMM_THREADS)
 spmm_carry_kernel(const SpmmParams p, const int *__restrict__ carry_row, int64_t n_carry)
 {
     const int64_t s = (int64_t)blockIdx.x * SPMM_WARPS + warp_id();
+    wait_for_predecessor();         // launched early behind the units
+    launch_dependents();
     if (s >= n_carry) return;
     const int2 span = p.carry_span[s];
     if (span.x != s) return;
@@ -514,9 +516,10 @@ spmm_carry_kernel(const SpmmParams p, const int *__restrict__ carry_row, int64_t
 constexpr int PAD_BLOCK = 256, PAD_ITEMS = 4;
 
 __global__ void __launch_bounds__(PAD_BLOCK)
-spmm_pad_rows_kernel(const float *__restrict__ x, int64_t ldx, int dim, float *__restrict__ xp, int ldp, int64_t n_rows)
+spmm_pad_rows_kernel(const float *x, int64_t ldx, int dim, float *xp, int ldp, int64_t n_rows)      // not __restrict__: X is read behind the wait
 {
-    launch_dependents();
+    wait_for_predecessor();         // launched early behind whatever makes X
+    launch_dependents();            // not above the wait: the product reads column ids and values before it waits for this kernel
     const unsigned quads = (unsigned)ldp >> 2, per_quad = ((1u << 20) + quads - 1) / quads;      // n / quads = n * per_quad >> 20 for n * quads < 2^20
     const int64_t first = (int64_t)blockIdx.x * (PAD_BLOCK * PAD_ITEMS);
     const int64_t row0 = first / quads;
@@ -531,10 +534,10 @@ spmm_pad_rows_kernel(const float *__restrict__ x, int64_t ldx, int dim, float *_
         v[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (row < n_rows) {
             const float *src = x + row * ldx + c;
-            if (c + 0 < dim) v[k].x = __ldg(src + 0);
-            if (c + 1 < dim) v[k].y = __ldg(src + 1);
-            if (c + 2 < dim) v[k].z = __ldg(src + 2);
-            if (c + 3 < dim) v[k].w = __ldg(src + 3);
+            if (c + 0 < dim) v[k].x = src[0];
+            if (c + 1 < dim) v[k].y = src[1];
+            if (c + 2 < dim) v[k].z = src[2];
+            if (c + 3 < dim) v[k].w = src[3];
         }
     }
 #pragma unroll

@@ -329,7 +329,7 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
     const int ldp = (dim + 3) & ~3;
     const int64_t blocks = ceil_div(n_rows * (ldp >> 2), PAD_BLOCK * PAD_ITEMS);
     AGCN_REQUIRE(blocks < (int64_t)INT32_MAX, "agcn_spmm_run: operand too large to pad");
-    AGCN_KERNEL(spmm_pad_rows_kernel, (unsigned)blocks, PAD_BLOCK, s, d_x, ldx, dim, d_xp, ldp, n_rows);
+    AGCN_CUDA(launch_early(true, spmm_pad_rows_kernel, (unsigned)blocks, PAD_BLOCK, 0, s, d_x, ldx, dim, d_xp, ldp, n_rows));
     AGCN_LAUNCH_CHECK("spmm_pad_rows_kernel");
     return AGCN_OK;
 }
@@ -468,7 +468,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         }
         if (p->n_carry > 0 && !carry_inside) {
             auto k = vec ? spmm_carry_kernel<true> : spmm_carry_kernel<false>;
-            AGCN_KERNEL(k, (unsigned)ceil_div(p->n_carry, SPMM_WARPS), SPMM_THREADS, s, prm, (const int *)p->carry_row, p->n_carry);
+            AGCN_CUDA(launch_early(true, k, (unsigned)ceil_div(p->n_carry, SPMM_WARPS), SPMM_THREADS, 0, s, prm, (const int *)p->carry_row, p->n_carry));
             AGCN_LAUNCH_CHECK("spmm_carry_kernel");
             p->launches_last_run++;
         }
