@@ -19,6 +19,7 @@ struct L2Policies {
     uint64_t keep;     // evict_last
     uint64_t stream;   // evict_first
     int hot;           // first column whose row of X is to be kept
+    int cols;          // how many columns this lane has, where rows of X are read 4 bytes at a time
 };
 
 // Rows of X from column `hot` on are to stay in L2, the others are to leave first (HOT: X many times larger than L2).
@@ -30,7 +31,7 @@ __device__ __forceinline__ L2Policies make_l2_policies()
     L2Policies p;
     asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p.keep));
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p.stream));
-    p.hot = 0;
+    p.hot = 0; p.cols = 4;
     return p;
 }
 
@@ -48,6 +49,19 @@ __device__ __forceinline__ float ld_x1(const float *p, uint64_t policy)
 {
     float v;
     asm("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(policy));
+    return v;
+}
+
+// Four columns of row `column` of X for this lane: the 16 bytes at p, or (LOOSE lanes per row: rows of any alignment)
+// p[0], p[LOOSE], p[2 LOOSE], p[3 LOOSE] as far as the row goes.
+template <bool HOT, int LOOSE>
+__device__ __forceinline__ float4 ld_x(const float *p, const L2Policies &pol, int column)
+{
+    if (LOOSE == 0) return ld_x4(p, x_policy<HOT>(pol, column));
+    float4 v = make_float4(ld_x1(p, pol.keep), 0.f, 0.f, 0.f);
+    if (pol.cols > 1) v.y = ld_x1(p + LOOSE, pol.keep);
+    if (pol.cols > 2) v.z = ld_x1(p + 2 * LOOSE, pol.keep);
+    if (pol.cols > 3) v.w = ld_x1(p + 3 * LOOSE, pol.keep);
     return v;
 }
 

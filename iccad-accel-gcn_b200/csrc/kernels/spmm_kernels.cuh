@@ -115,13 +115,21 @@ __device__ __forceinline__ float4 relu4(const float4 &v, int on)
 }
 __device__ __forceinline__ float relu1(float v, int on) { return on ? fmaxf(v, 0.f) : v; }
 
-// Writes columns col .. col+3 of one result row.  PLAIN: one 16-byte store.  Otherwise the row may
+// LOOSE: lanes that share a row which have columns LOOSE apart, yr + col being the first one's place.
+// Otherwise writes columns col .. col+3 of one result row.  PLAIN: one 16-byte store.  Otherwise the row may
 // be unaligned or end inside the four columns (dim not a multiple of 4: narrower stores), and
 // the product may be added to what the row holds (column-tiled products).
-template <bool PLAIN>
+template <bool PLAIN, int LOOSE = 0>
 __device__ __forceinline__ void emit_row4(const SpmmParams &p, float *yr, int col, float4 v, int act, uint64_t policy)
 {
-    if (PLAIN) {
+    if (LOOSE > 0) {
+        const float e[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            float *d = yr + col + k * LOOSE;
+            if (col + k * LOOSE < p.dim_store) st_y1(d, relu1(p.accumulate ? e[k] + *d : e[k], act), policy);
+        }
+    } else if (PLAIN) {
         st_y4(yr + col, relu4(v, act), policy);
     } else if (p.y_vec) {
         if (p.accumulate) {
@@ -163,7 +171,7 @@ __device__ __forceinline__ void fma4(float4 &acc, float a, const float4 &v)
 }
 
 // UNROLL independent 16-byte loads are issued per lane before the first FMA needs one.
-template <int UNROLL, bool HOT>
+template <int UNROLL, bool HOT, int LOOSE>
 __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int first, int step,
                                               const float *__restrict__ x, int64_t ldx, bool active, const L2Policies &pol)
 {
@@ -176,7 +184,7 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) p[u] = pairs[i + u * step];
 #pragma unroll
-        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)p[u].x * ldx, x_policy<HOT>(pol, p[u].x));
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_x<HOT, LOOSE>(x + (int64_t)p[u].x * ldx, pol, p[u].x);
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) fma4(acc, __int_as_float(p[u].y), v[u]);
     }
@@ -188,7 +196,7 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
         for (int u = 0; u < UNROLL - 1; u++) {
             const bool live = i + u * step < count;
             p[u] = live ? pairs[i + u * step] : make_int2(0, 0);
-            v[u] = live ? ld_x4(x + (int64_t)p[u].x * ldx, x_policy<HOT>(pol, p[u].x)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = live ? ld_x<HOT, LOOSE>(x + (int64_t)p[u].x * ldx, pol, p[u].x) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < UNROLL - 1; u++)
@@ -200,7 +208,7 @@ __device__ __forceinline__ float4 gather_vec4(const int2 *pairs, int count, int 
 // `rows` consecutive rows of row_nz nonzeros each, whole rows for this lane: one stream of gathers, UNROLL in
 // flight across row boundaries.  (Row by row, rows of three nonzeros keep three gathers in flight and a slot with
 // six of them waits six times.)
-template <int UNROLL, bool PLAIN, bool HOT>
+template <int UNROLL, bool PLAIN, bool HOT, int LOOSE>
 __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pairs, int rows, int row_nz, const float *__restrict__ x,
                                              float *yr, int col, const L2Policies &pol)
 {
@@ -210,7 +218,7 @@ __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pa
     auto take = [&](float a, const float4 &v) {
         fma4(acc, a, v);
         if (--left == 0) {
-            emit_row4<PLAIN>(p, yr, col, acc, p.relu, pol.stream);
+            emit_row4<PLAIN, LOOSE>(p, yr, col, acc, p.relu, pol.stream);
             acc = make_float4(0.f, 0.f, 0.f, 0.f);
             left = row_nz;
             yr += p.ldy;
@@ -223,7 +231,7 @@ __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pa
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) q[u] = pairs[i + u];
 #pragma unroll
-        for (int u = 0; u < UNROLL; u++) v[u] = ld_x4(x + (int64_t)q[u].x * p.ldx, x_policy<HOT>(pol, q[u].x));
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_x<HOT, LOOSE>(x + (int64_t)q[u].x * p.ldx, pol, q[u].x);
 #pragma unroll
         for (int u = 0; u < UNROLL; u++) take(__int_as_float(q[u].y), v[u]);
     }
@@ -234,7 +242,7 @@ __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pa
         for (int u = 0; u < UNROLL - 1; u++) {
             const bool live = i + u < count;
             q[u] = live ? pairs[i + u] : make_int2(0, 0);
-            v[u] = live ? ld_x4(x + (int64_t)q[u].x * p.ldx, x_policy<HOT>(pol, q[u].x)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[u] = live ? ld_x<HOT, LOOSE>(x + (int64_t)q[u].x * p.ldx, pol, q[u].x) : make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll
         for (int u = 0; u < UNROLL - 1; u++)
@@ -313,21 +321,22 @@ __device__ __forceinline__ float sum_parts1(const float (*part)[SPMM_PANEL], int
 }
 
 // Stores a row whose partials lie in carry slots span.x .. span.x + span.y - 1, adding them in slot order.
-// VEC: `first` is the first of the four columns of this lane; otherwise the lane takes columns first, first + 32, ...
-template <bool VEC, bool PLAIN>
+// VEC: `first` is the place of the first of the four columns of this lane (SPMM_PANEL: it has none); otherwise the lane
+// takes columns first, first + 32, ...
+template <bool VEC, bool PLAIN, int LOOSE = 0>
 __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 span, int row, int first, uint64_t policy)
 {
     const float *parts = p.carry + (int64_t)span.x * SPMM_PANEL;
     float *yr = p.y + (int64_t)row * p.ldy;
     if (VEC) {
-        if (first >= p.dim) return;
+        if (first >= (LOOSE > 0 ? SPMM_PANEL : p.dim)) return;
         float4 sum = __ldcg(reinterpret_cast<const float4 *>(parts + first));
 #pragma unroll 8
         for (int q = 1; q < span.y; q++) {
             const float4 v = __ldcg(reinterpret_cast<const float4 *>(parts + (int64_t)q * SPMM_PANEL + first));
             sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
         }
-        emit_row4<PLAIN>(p, yr, first, sum, p.relu, policy);
+        emit_row4<PLAIN, LOOSE>(p, yr, LOOSE > 0 ? first / 4 : first, sum, p.relu, policy);
     } else {
         for (int c = first; c < p.dim; c += 32) {
             float sum = __ldcg(parts + c);
@@ -346,8 +355,10 @@ __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 spa
 // a template parameter because the code costs registers the large launches
 // do not have (two more spills, 3 % of a product of 500 000 rows).
 // HOT: rows of X the L2 is to keep are told from the others.
+// ANY_ROWS: as float4 mode, with the same additions in the same order, but rows of X and Y of any alignment: lane l of a
+// slot has columns l, l + S, l + 2 S, l + 3 S (consecutive ones cost four times the wavefronts).
 // ---------------------------------------------------------------------------
-template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT>
+template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT, bool ANY_ROWS>
 __global__ void __launch_bounds__(SPMM_THREADS, MIN_BLOCKS)
 spmm_units_kernel(const SpmmParams p)
 {
@@ -361,10 +372,13 @@ spmm_units_kernel(const SpmmParams p)
     constexpr int NS = 32 / LANES;          // nonzeros a warp works on at a time
     const int w = warp_id(), lane = lane_id();
     const int slot = lane / LANES, sl = lane % LANES;
-    const int col = VEC ? sl * 4 : sl;
-    const bool active = col < p.dim;
+    constexpr int LOOSE = ANY_ROWS ? S : 0;
+    const int col = VEC ? sl * 4 : sl;              // place of the lane's sums among the partials
+    const int ycol = ANY_ROWS ? sl : col;           // and of the first of them in a row of X and Y
+    const bool active = ycol < (ANY_ROWS ? p.dim_store : p.dim);
     L2Policies pol = make_l2_policies();
     if (HOT) pol.hot = p.hot_column;
+    if (ANY_ROWS) pol.cols = (p.dim_store - sl + S - 1) / S;
 
     if (!p.wait_first) launch_dependents();     // a dense transform of this product's result may lay out its weights meanwhile
     if (p.abort_flag != nullptr && *p.abort_flag != 0) return;     // input rejected by a check earlier in the stream
@@ -377,7 +391,7 @@ spmm_units_kernel(const SpmmParams p)
             if (zb + k >= p.n_zero_rows) break;
             float *yr = p.y + (int64_t)p.zero_rows[zb + k] * p.ldy;
             if (VEC) {
-                if (active) emit_row4<PLAIN>(p, yr, col, make_float4(0.f, 0.f, 0.f, 0.f), p.relu, pol.stream);
+                if (active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, make_float4(0.f, 0.f, 0.f, 0.f), p.relu, pol.stream);
             } else {
                 for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, 0.f, p.relu, pol.stream);
             }
@@ -410,17 +424,17 @@ spmm_units_kernel(const SpmmParams p)
     wait_for_predecessor();             // X may be what the launch before this one makes
 
     if (VEC) {
-        const float *xc = p.x + col;
+        const float *xc = p.x + ycol;
         if (t.small && t.row_nz <= 32) {
             // whole rows for every slot, consecutive ones
             const int each = (t.n_rows + NS - 1) / NS, r0 = slot * each;
             const int rows = r0 < t.n_rows ? (r0 + each < t.n_rows ? each : t.n_rows - r0) : 0;
             if (active)
-                gather_rows4<BATCH, PLAIN, HOT>(p, pairs + r0 * t.row_nz, rows, t.row_nz, xc, p.y + (int64_t)(t.row0 + r0) * p.ldy, col, pol);
+                gather_rows4<BATCH, PLAIN, HOT, LOOSE>(p, pairs + r0 * t.row_nz, rows, t.row_nz, xc, p.y + (int64_t)(t.row0 + r0) * p.ldy, ycol, pol);
         } else {
             // the slots of the warp share each row
             for (int r = 0; r < t.n_rows; r++) {
-                float4 acc = gather_vec4<BATCH, HOT>(pairs + r * t.row_nz, t.row_nz, slot, NS, xc, p.ldx, active, pol);
+                float4 acc = gather_vec4<BATCH, HOT, LOOSE>(pairs + r * t.row_nz, t.row_nz, slot, NS, xc, p.ldx, active, pol);
 #pragma unroll
                 for (int off = LANES; off < 32; off <<= 1) {
                     acc.x += __shfl_xor_sync(FULL_MASK, acc.x, off);
@@ -429,7 +443,7 @@ spmm_units_kernel(const SpmmParams p)
                     acc.w += __shfl_xor_sync(FULL_MASK, acc.w, off);
                 }
                 if (slot == 0 && active) {
-                    if (t.small) emit_row4<PLAIN>(p, p.y + (int64_t)(t.row0 + r) * p.ldy, col, acc, p.relu, pol.stream);
+                    if (t.small) emit_row4<PLAIN, LOOSE>(p, p.y + (int64_t)(t.row0 + r) * p.ldy, ycol, acc, p.relu, pol.stream);
                     else *reinterpret_cast<float4 *>(&s_part[w][col]) = acc;
                 }
             }
@@ -465,7 +479,7 @@ spmm_units_kernel(const SpmmParams p)
     float *yr = p.y + (int64_t)t.row0 * p.ldy;
     if (!partial) {
         if (VEC) {
-            if (slot == 0 && active) emit_row4<PLAIN>(p, yr, col, sum_parts4(s_part, w, w_end, col), p.relu, pol.stream);
+            if (slot == 0 && active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, sum_parts4(s_part, w, w_end, col), p.relu, pol.stream);
         } else {
             for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, sum_parts1(s_part, w, w_end, c), p.relu, pol.stream);
         }
@@ -489,7 +503,7 @@ spmm_units_kernel(const SpmmParams p)
     if (arrived != span.y - 1) return;
     if (lane == 0) p.carry_count[span.x] = 0;       // ready for the next product
     __threadfence();
-    finish_carried_row<VEC, PLAIN>(p, span, t.row0, VEC ? (slot == 0 && active ? col : SPMM_PANEL) : lane, pol.stream);
+    finish_carried_row<VEC, PLAIN, LOOSE>(p, span, t.row0, VEC ? (slot == 0 && active ? col : SPMM_PANEL) : lane, pol.stream);
 }
 
 // Adds the carried partials of every row that crosses unit boundaries.  One warp per carry slot; the warp of

@@ -278,7 +278,7 @@ int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag
 template <int S, int BATCH, int MIN_BLOCKS, bool FINISH, bool HOT = false>
 static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaStream_t s)
 {
-    auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH, HOT> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH, HOT>;
+    auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH, HOT, false> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH, HOT, false>;
     launch_early(prm.early != 0, k, grid, SPMM_THREADS, 0, s, prm);
 }
 
@@ -288,11 +288,20 @@ struct SpmmForm {
     bool finish;     // rows that cross units are finished in the launch
     bool deep;       // few thread blocks, many gathers per lane
     bool wide;       // more thread blocks per SM, fewer gathers per lane
+    bool loose;      // rows of X of any alignment (deep launches only)
 };
 
 template <int S>
 static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
 {
+    if constexpr (S > 0) {
+        if (f.loose) {
+            auto k = f.deep ? spmm_units_kernel<S, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, false, true, false, true>
+                            : spmm_units_kernel<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true, false, true>;
+            launch_early(prm.early != 0, k, grid, SPMM_THREADS, 0, s, prm);
+            return;
+        }
+    }
     if (f.deep) { launch_units<S, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, true>(prm, grid, f.plain, s); return; }
     // 17..32 columns, and the 4-byte mode, always take the 5-block form
     constexpr bool ALWAYS_WIDE = S == 8 || S == 0;
@@ -334,6 +343,8 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
     return AGCN_OK;
 }
 
+static bool x_rows_aligned(const float *d_x, int64_t ldx, int dim) { return dim % 4 == 0 && ldx % 4 == 0 && aligned16(d_x); }
+
 // Rows of X that are not 16-byte aligned (dim % 4 != 0 with the reference's ld = dim, an odd
 // stride or base) would force 4-byte gathers: 1.2-1.6x the time of the 16-byte path.  Instead X
 // is copied once into plan-owned rows padded to a multiple of 4 floats (2 * n_cols * dim * 4
@@ -341,10 +352,27 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
 // on the copy; Y keeps the caller's layout and gets stores as wide as each row's alignment allows.
 // On return *x_use / *ldx_use name the operand to gather from and *x_vec says whether its rows
 // are 16-byte aligned.
+static bool spmm_deep(const agcn_spmm_plan *p) { return p->split && 3 * p->n_units <= (int64_t)8 * p->sm_count; }
+
+// Small products gather 4 bytes at a time from X as it is instead, with the additions of the 16-byte path in its order:
+// to a chain of latencies the copy adds a kernel, and where a row of X is named a few times the copy of it is a good part
+// of the work.  us with the copy / without, nonzeros per SM and per row of X in brackets, dims 17, 61, 127:
+// 2 048 rows of 4 [70, 5]: 7.9 / 6.7 (17);  500 dense rows of 100 [340, 100]: 7.7 / 7.1, 7.9 / 7.1, 9.2 / 7.3;
+// 16 384 of 8 [1 000, 9]: 10.1 / 7.8, 14.1 / 11.0, 19.2 / 15.4;  30 000 of 12 [2 600, 13]: 13.2 / 10.6, 16.0 / 14.6, 24.1 / 22.6;
+// 80 000 of 4 [2 700, 5]: - , 20.4 / 14.3, 37.0 / 26.8;  but
+// 1 000 dense of 150 [1 000, 150]: 9.5 / 9.5, 11.4 / 11.9, 14.2 / 15.6;  30 000 skewed of 16 [3 200, 16]: 14.9 / 12.2, 16.6 / 17.6,
+// 26.7 / 26.7;  100 000 skewed of 10 [6 800, 10]: 17.8 / 20.7, 29.7 / 32.4, 62.0 / 64.8.
+// (Its sums take 4 S places of a carry slot where the columns may be fewer: forced passes might not leave them.)
+static bool spmm_loose(const agcn_spmm_plan *p)
+{
+    if (!p->pad_unaligned || p->panel_override != 0 || !p->split) return false;
+    return (spmm_deep(p) && p->nnz <= (int64_t)500 * p->sm_count) || (p->nnz <= 13 * p->n_cols && p->nnz <= (int64_t)2700 * p->sm_count);
+}
+
 int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cudaStream_t s,
                    const float **x_use, int64_t *ldx_use, bool *x_vec)
 {
-    const bool x_aligned = dim % 4 == 0 && ldx % 4 == 0 && aligned16(d_x);
+    const bool x_aligned = x_rows_aligned(d_x, ldx, dim);
     *x_use = d_x;
     *ldx_use = ldx;
     *x_vec = x_aligned;
@@ -428,7 +456,8 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     // passes are -- with the same passes, hence the same bits, as a whole run.
     if (!whole) AGCN_REQUIRE(dim <= SPMM_PANEL, "agcn_spmm_run: a product issued in unit ranges is limited to %d columns", SPMM_PANEL);
     AGCN_REQUIRE(panel >= 1 && panel <= SPMM_PANEL, "agcn_spmm_run: AGCN_SPMM_PANEL must be 1..%d", SPMM_PANEL);
-    if (x_vec && panel % 4 != 0) panel = (panel + 3) & ~3;         // keep every panel's first column 16-byte aligned
+    const bool loose = !x_vec && whole && spmm_loose(p);
+    if ((x_vec || loose) && panel % 4 != 0) panel = (panel + 3) & ~3;         // keep every panel's first column 16-byte aligned
     if (panel > SPMM_PANEL) panel = SPMM_PANEL;
     for (int col0 = 0, width = 0; col0 < dim; col0 += width) {
         // a pass ends where the carry slot does: behind the last slot lie the arrival counters
@@ -454,14 +483,14 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.zero_rows = p->zero_rows; prm.n_zero_rows = p->n_zero;
         prm.relu = activation;
         prm.accumulate = accumulate;
-        const bool vec = x_vec && aligned16(prm.x);
+        const bool vec = loose || (x_vec && aligned16(prm.x));
         const bool y_vec = width % 4 == 0 && ldy % 4 == 0 && aligned16(prm.y);
         prm.y_vec = y_vec ? 1 : 0;
         prm.dim_store = width;
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
-        const bool plain = !accumulate && (vec ? y_vec : true);
+        const bool plain = !accumulate && !loose && (vec ? y_vec : true);
         if (grid > 0) {
-            const SpmmForm form = {plain, carry_inside, p->split && 3 * p->n_units <= (int64_t)8 * p->sm_count, spmm_wide_form(p, width)};
+            const SpmmForm form = {plain, carry_inside, spmm_deep(p), spmm_wide_form(p, width), loose};
             launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, form, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;
@@ -483,10 +512,10 @@ int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const
     if (rc != AGCN_OK) return rc;
     const DeviceOf on(p->device);
     p->launches_last_run = 0;
-    const float *x_use = nullptr;
-    int64_t ldx_use = 0;
-    bool x_vec = false;
-    rc = spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
+    const float *x_use = d_x;
+    int64_t ldx_use = ldx;
+    bool x_vec = x_rows_aligned(d_x, ldx, dim);
+    rc = spmm_loose(p) ? AGCN_OK : spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
     if (rc != AGCN_OK) return rc;
     SpmmLaunchPart part;
     // A product is launched while the operation before it still runs and waits for it on the GPU, so that launch, first

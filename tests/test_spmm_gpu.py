@@ -712,6 +712,41 @@ def test_products_behind_work_of_any_kind(case_name, dim, request):
     plan.close()
 
 
+@pytest.mark.parametrize("dim", [1, 2, 3, 5, 15, 16, 17, 31, 33, 60, 61, 63, 64, 65, 97, 127, 128, 129, 150, 259])
+@pytest.mark.parametrize("kind", ["few", "pieces", "hubs"])
+def test_small_products_from_rows_of_any_alignment(kind, dim):
+    # small products read unaligned rows of X as they are: bit for bit what the copied, aligned rows give, whatever X holds,
+    # for the launches with many and with few gathers per lane, rows that cross thread blocks, rows without nonzeros
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    rng = np.random.default_rng(dim)
+    n, deg = {"few": (700, lambda: rng.integers(0, 30, 700)), "pieces": (30_000, lambda: rng.integers(0, 20, 30_000)),
+              "hubs": (20_000, lambda: np.concatenate([rng.integers(0, 3, 19_990), [700, 900, 1_500, 2_000, 2_500, 3_100, 4_000, 6_000, 9_000, 20_000]]))}[kind]
+    deg = np.sort(deg())
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(dev)
+    nnz = int(deg.sum())
+    idx = torch.from_numpy(rng.integers(0, n, nnz, dtype=np.int32)).to(dev)
+    val = torch.from_numpy(rng.standard_normal(nnz).astype(np.float32)).to(dev)
+    plan = spmm.SpmmPlan(partition.block_level_partition_device(indptr), idx, n, n)
+    wide = (dim + 3) // 4 * 4
+    xs = torch.from_numpy(rng.standard_normal((n, dim)).astype(np.float32)).to(dev)
+    xs[5, 0], xs[6, dim - 1], xs[7, dim // 2] = float("inf"), float("-inf"), float("nan")
+    for relu in (False, True):
+        aligned, want = torch.zeros((n, wide), device=dev), torch.full((n, wide), 7.0, device=dev)
+        aligned[:, :dim] = xs
+        plan.run(idx, val, aligned, want, relu=relu)
+        for shift, ldx, ldy in ((0, dim, dim), (1, dim, dim + 1), (3, dim + 2, wide), (2, wide + 1, dim)):
+            x = torch.full((n * ldx + shift,), float("nan"), device=dev)[shift:]
+            y = torch.full((n * ldy + shift,), 7.0, device=dev)[shift:]
+            x.view(n, ldx)[:, :dim] = xs
+            plan.run(idx, val, x, y, dim=dim, ldx=ldx, ldy=ldy, relu=relu)
+            got = y.view(n, ldy)
+            assert torch.equal(got[:, :dim].nan_to_num(3.0, 4.0, 5.0), want[:, :dim].nan_to_num(3.0, 4.0, 5.0)), (relu, shift, ldx, ldy)
+            assert bool((got[:, dim:] == 7.0).all())
+    plan.close()
+
+
 @pytest.mark.parametrize("case_name", ["cfg1", "cfg4_small"])
 def test_column_tiled_small(case_name, request):
     # tiled plan with several range layouts (one of them empty), ReLU, an unaligned width and the
