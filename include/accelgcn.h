@@ -147,13 +147,13 @@ int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_indices, con
  * run to run.  Any dim >= 1 (the reference harness sweeps every dim 16..128,
  * main.cu:12,137).  Rows of X are gathered 16 bytes per lane; when they are not
  * 16-byte aligned (dim % 4 != 0 with ld = dim, an odd stride or base) X is first
- * copied into plan-owned aligned rows (grown on demand: the first such call of
+ * copied (by small products: read as it is, with the same result) into plan-owned aligned rows (grown on demand: the first such call of
  * a width allocates, so make it before a stream capture, and the widest one
  * before the first capture: growing moves the rows; AGCN_SPMM_PAD=0 at plan creation selects 4-byte gathers
  * instead) and unaligned rows of Y get stores as wide as each row's alignment allows.  dim > 64 may run
  * as two 64-column passes when X is larger than L2 (environment variable
  * AGCN_SPMM_PANEL = columns per pass, read at plan creation, overrides that
- * choice).  Plans of few tuples hold a copy of them cut into pieces of 64 to 192
+ * choice).  Plans of few tuples hold a copy of them cut into pieces of 32 to 192
  * nonzeros (AGCN_SPMM_PIECE = nonzeros per piece, 0 = uncut, overrides the choice).  A plan must not be run concurrently on two streams (the runs share
  * its scratch).
  * ---------------------------------------------------------------------- */

@@ -138,6 +138,22 @@ def test_tile_edges_and_number_of_passes(n, top, relabel):
         assert np.array_equal(a, b), what
 
 
+@pytest.mark.parametrize("items", [1, 2, 3, 4, 5, 8])
+def test_rows_per_thread_of_the_cluster_sort(items):
+    # the cluster's shared memory is sized by the rows per thread (above three of them it needs more than the default)
+    from accelgcn import degree_sort
+    require_cuda()
+    for n in (8192 * (items - 1) + 1, 8192 * items):
+        rng = np.random.default_rng(n)
+        deg = rng.integers(0, 5, n)
+        deg[rng.integers(0, n, 20)] = rng.integers(250, 3_000, 20)
+        indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+        idx = rng.integers(0, n, int(indptr[-1]), dtype=np.int32)
+        got = degree_sort.degree_sort(indptr, idx, None, relabel_cols=True)
+        for a, b, what in zip(got, oracle.degree_sort(indptr, idx, None, relabel_cols=True), ("perm", "indptr", "indices")):
+            assert np.array_equal(a, b), (n, what)
+
+
 @pytest.mark.parametrize("n", [65_536 + 1, 65_536 * 2, 2_097_152, 2_101_249, 4_300_000])
 @pytest.mark.parametrize("kind", ["low", "high", "mixed"])
 def test_counters_of_tiles_groups_and_groups_of_groups(n, kind):
