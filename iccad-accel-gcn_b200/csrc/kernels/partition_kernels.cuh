@@ -12,9 +12,9 @@
 // fall-backs of :56-63.  Two launches over tiles of PART_TILE rows staged
 // through shared memory: (A) every tile describes itself -- its last run start,
 // its leading rows that belong to a run begun earlier, the tuples all other rows
-// open -- and (B) the last thread block scans the descriptions, which closes the
-// open runs, and leaves every tile its incoming run start and its first output
-// position; (C) every row writes its own tuples.  The host waits between (B) and (C), for
+// open -- and (B) the thread block that is done last scans the descriptions, which
+// closes the open runs, and leaves every tile its incoming run start and its first
+// output position; (C) every row writes its own tuples.  The host waits between (B) and (C), for
 // the number of tuples it has to find room for, and not behind (C).
 // Bound: launch latency up to some 100 000 rows, instruction issue above.
 #pragma once
@@ -30,10 +30,7 @@ constexpr int PART_ITEMS = 8;
 constexpr int PART_TILE = PART_BLOCK * PART_ITEMS;
 constexpr int PART_MAX_ROWS_PER_TUPLE = 12;
 constexpr int PART_HALO = PART_MAX_ROWS_PER_TUPLE + 1;   // rows looked at past a tile
-constexpr int PART_WORD_TOTAL = 0, PART_WORD_NEGATIVE = 1, PART_WORD_TIMEOUT = 2;    // host words
-// Polls before the last block gives up on a tile's description (each backs off; well over a second): the other blocks
-// wait for nothing, so the limit is there for a bug, not for load.
-constexpr int PART_SPIN_LIMIT = 1 << 22;
+constexpr int PART_WORD_TOTAL = 0, PART_WORD_NEGATIVE = 1;    // host words
 
 // rows per tuple R(D) and nonzeros per virtual warp w(D), 1 <= D <= 384
 __device__ __forceinline__ int part_rows_per_tuple(int d)
@@ -98,7 +95,7 @@ __device__ __forceinline__ PartTile part_load_tile(const int *__restrict__ indpt
 }
 
 // What a tile says about itself.
-struct PartTileInfo {
+struct PartTileInfo {         // read as an int4
     int last_head;    // last row of the tile that starts a run, -1 if none
     int lead;         // rows before the tile's first run start, where their tuples depend on where that run began
     int lead_deg;     // ... and their degree (1 .. 384; lead is 0 for any other degree)
@@ -163,33 +160,23 @@ __device__ __forceinline__ int64_t part_lead_tuples(const PartTileInfo &info, in
     return (o + info.lead + r - 1) / r - (o + r - 1) / r;
 }
 
-// Says that tile b's description is there: the call's own number, which memory that held other calls' cannot hold.
-__device__ __forceinline__ void part_say(unsigned long long *tag, unsigned long long call)
-{
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" :: "l"(tag), "l"(call) : "memory");
-}
-__device__ __forceinline__ bool part_said(const unsigned long long *tag, unsigned long long call)
-{
-    for (int spin = 0; spin < PART_SPIN_LIMIT; spin++) {
-        unsigned long long v;
-        asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(tag) : "memory");
-        if (v == call) return true;
-        if (spin > 16) __nanosleep(200);
-    }
-    return false;
-}
+// How many thread blocks of a call have described their tile: a counter for each of the calls under way (partition.cu
+// hands them out).  Zero when the library is loaded, and after every call: the block that arrives last resets it.
+constexpr int PART_COUNTERS = 64;
+static __device__ unsigned g_part_arrived[PART_COUNTERS];
 
-// (A) the description of every tile, and (B) by the last block (the others are running or done when it starts) the run
-// start that is open when every tile begins and every tile's first output position.  (As a launch of its own, one
-// block, (B) cost the host 3 us and the GPU 6 more.)
+// (A) the description of every tile, and (B) by the block that arrives last, whichever that is, the run start that is
+// open when every tile begins and every tile's first output position.  (As a launch of its own, one block, (B) cost the
+// host 3 us and the GPU 6 more.)  `own`: a zeroed word to count arrivals in; null: counter number `counter` does.
 __global__ void __launch_bounds__(PART_BLOCK)
-part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInfo *tiles, unsigned long long *tags, unsigned long long call,
-                     int *__restrict__ tile_head, int64_t *__restrict__ tile_offset, HostWords *out)
+part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInfo *tiles, unsigned *own, int counter, int *__restrict__ tile_head,
+                     int64_t *__restrict__ tile_offset, HostWords *out)
 {
     __shared__ int s_ip[PART_SMEM_INTS];
     __shared__ int s_scan[PART_BLOCK / 32 + 1];
     __shared__ int64_t s_scan64[PART_BLOCK / 32 + 1];
     __shared__ int s_red[4][PART_BLOCK / 32];
+    __shared__ bool s_last;
     const PartTile t = part_load_tile(indptr, n_rows, blockIdx.x, s_ip);
     int deg[PART_ITEMS], cnt[PART_ITEMS], lead, lead_deg;
     unsigned heads;
@@ -214,18 +201,22 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
             info.rest += s_red[3][w];
         }
         tiles[blockIdx.x] = info;
-        part_say(tags + blockIdx.x, call);
+        unsigned *arrived = own != nullptr ? own : g_part_arrived + counter;
+        __threadfence();
+        s_last = atomicAdd(arrived, 1u) == gridDim.x - 1;
+        if (s_last) *arrived = 0;
     }
-    if (blockIdx.x + 1 < gridDim.x) return;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();                 // all descriptions are there
     int carry_head = -1;
     int64_t carry = 0;
-    bool all = true;
     for (int64_t base = 0; base < gridDim.x; base += PART_BLOCK) {
         const int64_t b = base + threadIdx.x;
         PartTileInfo info = {-1, 0, 0, 0};
         if (b < gridDim.x) {
-            if (all && part_said(tags + b, call)) info = tiles[b];
-            else all = false;
+            const int4 v = __ldcg(reinterpret_cast<const int4 *>(tiles) + b);
+            info = {v.x, v.y, v.z, v.w};
         }
         int head_total;
         int head_in = block_scan_exclusive<PART_BLOCK>(info.last_head, OpMax(), -1, head_total, s_scan);
@@ -237,7 +228,6 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
         carry += total;
         carry_head = max(carry_head, head_total);
     }
-    if (!all) out->w[PART_WORD_TIMEOUT] = 1;
     if (threadIdx.x == 0) out->w[PART_WORD_TOTAL] = carry;
 }
 

@@ -19,7 +19,7 @@ namespace agcn {
 // allocation-free one points it at a fixed array in the library's device image.
 struct PartScratch {
     PartTileInfo *info;
-    unsigned long long *tags;
+    unsigned *arrived;             // for calls that find no counter free
     int *tile_head;
     int64_t *tile_offset;
     HostWords *words = nullptr;    // on the device: where the answer is stored instead of in leased host words
@@ -29,7 +29,7 @@ static PartScratch part_scratch(Carver &c, int64_t tiles)
 {
     PartScratch sc;
     sc.info = c.take<PartTileInfo>(tiles);
-    sc.tags = c.take<unsigned long long>(tiles);
+    sc.arrived = c.take<unsigned>(1);
     sc.tile_offset = c.take<int64_t>(tiles);
     sc.tile_head = c.take<int>(tiles);
     return sc;
@@ -44,12 +44,8 @@ static int partition_check(const char *who, const int *d_indptr, int64_t n_rows,
     return AGCN_OK;
 }
 
-static int partition_answer(const char *who, int64_t negative, int64_t timeout, int64_t total, int64_t *n_blocks)
+static int partition_answer(const char *who, int64_t negative, int64_t total, int64_t *n_blocks)
 {
-    if (timeout != 0) {
-        set_error("%s: a wait between tiles ran out", who);
-        return AGCN_ERR_CUDA;
-    }
     if (negative != 0) {
         set_error("%s: indptr decreases somewhere (negative degree); "
                   "the reference script prints 'cur_degree number is wrong' and stops", who);
@@ -59,37 +55,63 @@ static int partition_answer(const char *who, int64_t negative, int64_t timeout, 
     return AGCN_OK;
 }
 
-// High bits of a call's number: what other uses of the scratch do not leave behind (no float, id or offset looks so).
-constexpr unsigned long long PART_CALL_MARK = 0x7ff4a9c3ull << 32;
+// The arrival counter of one call, its own until the call has waited for its kernel.  All zero when they are handed out:
+// the kernel leaves its counter so, and one whose kernel is not known to have ended is not handed out again.
+class ArrivalCounter {
+public:
+    ArrivalCounter()
+    {
+        uint64_t free = free_.load();
+        while (free != 0 && !free_.compare_exchange_weak(free, free & (free - 1))) {}
+        number_ = free != 0 ? __builtin_ctzll(free) : -1;
+    }
+    ~ArrivalCounter() { if (number_ >= 0 && !launched_) free_.fetch_or((uint64_t)1 << number_); }
+    ArrivalCounter(const ArrivalCounter &) = delete;
+    ArrivalCounter &operator=(const ArrivalCounter &) = delete;
+    int number() const { return number_; }          // -1: none was free
+    void launched() { launched_ = true; }
+    void ended() { launched_ = false; }
+private:
+    static_assert(PART_COUNTERS == 64, "a bit of free_ each");
+    static std::atomic<uint64_t> free_;
+    int number_;
+    bool launched_ = false;
+};
+std::atomic<uint64_t> ArrivalCounter::free_{~(uint64_t)0};
 
-// Phases A and B: how many tuples there are and where every tile's begin.  Waits for the stream.
-// `who` names the entry point in error messages.
-static int partition_launch_count(const int *d_indptr, int64_t n_rows, const PartScratch &sc, HostWords *words, cudaStream_t s)
+// Phases A and B: how many tuples there are and where every tile's begin.  `who` names the entry point in error messages.
+static int partition_launch_count(const int *d_indptr, int64_t n_rows, const PartScratch &sc, unsigned *own, int counter, HostWords *words,
+                                  cudaStream_t s)
 {
-    const int64_t tiles = ceil_div(n_rows, PART_TILE);
-    static std::atomic<unsigned long long> calls{0};       // numbers the calls of the process
-    AGCN_KERNEL(part_describe_kernel, (unsigned)tiles, PART_BLOCK, s, d_indptr, n_rows, sc.info, sc.tags, PART_CALL_MARK + ++calls, sc.tile_head,
+    AGCN_KERNEL(part_describe_kernel, (unsigned)ceil_div(n_rows, PART_TILE), PART_BLOCK, s, d_indptr, n_rows, sc.info, own, counter, sc.tile_head,
                 sc.tile_offset, words);
     AGCN_LAUNCH_CHECK("part_describe_kernel");
     return AGCN_OK;
 }
 
+// The same, and the wait for the stream.
 static int partition_count(const char *who, const int *d_indptr, int64_t n_rows, int64_t *n_blocks, const PartScratch &sc, cudaStream_t s)
 {
     if (sc.words != nullptr) {
         HostWords words;
         AGCN_CUDA(cudaMemsetAsync(sc.words, 0, sizeof(words), s));
-        const int rc = partition_launch_count(d_indptr, n_rows, sc, sc.words, s);
+        unsigned *arrived = reinterpret_cast<unsigned *>(&sc.words->w[HostWords::COUNT - 1]);      // zeroed with the words
+        const int rc = partition_launch_count(d_indptr, n_rows, sc, arrived, 0, sc.words, s);
         if (rc != AGCN_OK) return rc;
         AGCN_CUDA(cudaMemcpyAsync(&words, sc.words, sizeof(words), cudaMemcpyDeviceToHost, s));
         AGCN_CUDA(cudaStreamSynchronize(s));
-        return partition_answer(who, words.w[PART_WORD_NEGATIVE], words.w[PART_WORD_TIMEOUT], words.w[PART_WORD_TOTAL], n_blocks);
+        return partition_answer(who, words.w[PART_WORD_NEGATIVE], words.w[PART_WORD_TOTAL], n_blocks);
     }
+    ArrivalCounter counter;            // given back after the words, which wait for a kernel that an early return leaves running
+    const bool none = counter.number() < 0;
+    if (none) AGCN_CUDA(cudaMemsetAsync(sc.arrived, 0, sizeof(unsigned), s));
     AGCN_HOST_WORDS(words, s);
-    const int rc = partition_launch_count(d_indptr, n_rows, sc, words.device(), s);
+    const int rc = partition_launch_count(d_indptr, n_rows, sc, none ? sc.arrived : nullptr, counter.number(), words.device(), s);
     if (rc != AGCN_OK) return rc;
+    counter.launched();
     AGCN_CUDA(words.sync());
-    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TIMEOUT], words[PART_WORD_TOTAL], n_blocks);
+    counter.ended();
+    return partition_answer(who, words[PART_WORD_NEGATIVE], words[PART_WORD_TOTAL], n_blocks);
 }
 
 // Phase C, asynchronous.
@@ -249,10 +271,10 @@ extern "C" int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows, int3
 // fails or steals from its pool), a latency-critical loop that cannot afford
 // the device-wide synchronisation cudaMalloc / cudaFree imply, or a plug-in
 // host that forbids allocation calls after start-up.  For them the tile
-// scratch of the partitioner (36 bytes per 2048 rows) and its result words live in a
+// scratch of the partitioner (28 bytes per 2048 rows) and its result words live in a
 // fixed array in the library's device image instead of a per-call allocation or leased
 // host words (which are pinned when there are none free).  Every GPU that
-// loads the library holds that array (about 288 KB) until the process exits,
+// loads the library holds that array (about 224 KB) until the process exits,
 // which is why it is sized for AGCN_PARTITION_NOALLOC_MAX_ROWS rows and no
 // more.
 //
@@ -269,7 +291,7 @@ constexpr int64_t PART_NOALLOC_MAX_ROWS = AGCN_PARTITION_NOALLOC_MAX_ROWS;
 constexpr int64_t PART_NOALLOC_MAX_TILES = (PART_NOALLOC_MAX_ROWS + PART_TILE - 1) / PART_TILE;
 constexpr int PART_NOALLOC_MAX_DEVICES = 64;
 
-constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + 2 * sizeof(int64_t) + sizeof(int)) + 4 * 256 + 256;
+constexpr size_t PART_STATIC_BYTES = (size_t)PART_NOALLOC_MAX_TILES * (sizeof(PartTileInfo) + sizeof(int64_t) + sizeof(int)) + 3 * 256 + 2 * 256;
 
 }  // namespace agcn
 

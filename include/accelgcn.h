@@ -85,7 +85,7 @@ int agcn_partition_host(const int32_t *h_indptr, int64_t n_rows,
  * cannot take the device-wide synchronisation an allocation or free implies,
  * plug-in hosts that forbid allocation after start-up.  Same arguments, same
  * results and same error codes as agcn_partition_device, but the tile scratch
- * is a fixed array inside the library's device image (about 288 KB, resident on
+ * is a fixed array inside the library's device image (about 224 KB, resident on
  * every GPU that loads the library until the process exits) and the call makes
  * no cudaMalloc / cudaFree or other allocating call.
  *  - n_rows above AGCN_PARTITION_NOALLOC_MAX_ROWS is AGCN_ERR_INVALID.

@@ -167,3 +167,77 @@ def test_on_another_stream_the_tuples_are_complete_on_return(n):
         assert np.array_equal(out.cpu().numpy(), want)
         with torch.cuda.stream(side):
             busy.add_(1)
+
+
+def test_count_does_not_depend_on_what_the_scratch_held():
+    # the scratch is pool memory, never cleared: here, before every call, the pool's block of that size is filled (as the
+    # row pointers of a call that is refused) with descriptions of 300 tiles and marks that say that they are there, as a
+    # kernel that looked for marks in this memory left and expected them.  Own process: the marks count its calls.  Of the
+    # row pointers the last tile's are in L2, so that it is described before the others.
+    import subprocess, sys
+    from conftest import PKG
+    require_cuda()
+    code = """
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import torch
+from accelgcn import _lib
+lib = _lib.load()
+tiles, rows = 300, 2048 * 300
+d_ip = torch.arange(rows + 1, dtype=torch.int32, device="cuda")
+flush = torch.empty(1 << 26, device="cuda")
+n = ctypes.c_int64(0)
+for k in range(60):
+    held = np.zeros(2816, dtype=np.int32)
+    held[:4 * tiles].reshape(tiles, 4)[:] = (-1, 0, 0, 1_000_000)          # last run start, two of leading rows, tuples
+    held[1216:1216 + 2 * tiles].reshape(tiles, 2)[:] = (2 * k + 2, 0x7ff4a9c3)
+    assert lib.agcn_partition_host(held.ctypes.data, len(held) - 1, None, 0, ctypes.byref(n)) == _lib.ERR_RANGE
+    flush.zero_()
+    d_ip[-5000:].sum()
+    torch.cuda.synchronize()
+    _lib.check(lib.agcn_partition_device(d_ip.data_ptr(), rows, None, 0, ctypes.byref(n), None))
+    assert n.value == rows // 12, (k, n.value)
+"""
+    out = subprocess.run([sys.executable, "-c", code, PKG], capture_output=True, text=True, timeout=300)
+    assert out.returncode == 0, out.stderr[-2000:]
+
+
+def test_many_calls_at_once():
+    # 70 calls under way together, six more than there are arrival counters: each on a stream of its own that is kept
+    # busy until all have been started; twice, so that counters are used again
+    import threading
+    import torch
+    from accelgcn import _lib
+    dev = require_cuda()
+    lib = _lib.load()
+    rng = np.random.default_rng(5)
+    sizes = [int(n) for n in rng.integers(1, 40_000, 70)]
+    ips = [np.concatenate([[0], np.cumsum(rng.integers(0, 500, n))]).astype(np.int32) for n in sizes]
+    want = [oracle.partition(ip) for ip in ips]
+    d_ips = [torch.from_numpy(ip).to(dev) for ip in ips]
+    outs = [torch.full((len(w) + 1, 4), -7, dtype=torch.int32, device=dev) for w in want]
+    streams = [torch.cuda.Stream(dev) for _ in sizes]
+    answers = [None] * len(sizes)
+
+    def one(k):
+        n = ctypes.c_int64(0)
+        rc = lib.agcn_partition_device(d_ips[k].data_ptr(), sizes[k], outs[k].data_ptr(), len(want[k]), ctypes.byref(n), streams[k].cuda_stream)
+        answers[k] = (rc, n.value)
+
+    for _ in range(2):
+        for o in outs:
+            o.fill_(-7)
+        torch.cuda.synchronize()
+        for s in streams:
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(100_000_000)
+        threads = [threading.Thread(target=one, args=(k,)) for k in range(len(sizes))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for k, w in enumerate(want):
+            assert answers[k] == (0, len(w)), k
+            got = outs[k].cpu().numpy()
+            assert np.array_equal(got[:-1], w) and (got[-1] == -7).all(), k
