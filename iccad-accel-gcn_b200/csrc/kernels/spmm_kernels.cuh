@@ -887,14 +887,15 @@ constexpr int PLAN_SMALL_BLOCK = 1024;
 __global__ void __launch_bounds__(PLAN_SMALL_BLOCK)
 plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows, int64_t nnz, const int *__restrict__ idx, int64_t n_idx,
                   int64_t n_cols, int most, int4 *pieces, int cap_pieces, int2 *unit_carry, int2 *carry_span, int *carry_row, int *zero_rows,
-                  int *counters, int n_counters, unsigned clear_blocks, HostWords *out)
+                  int *counters, int64_t n_counters, unsigned clear_blocks, HostWords *out)
 {
     if (blockIdx.x > clear_blocks) {
         plan_check_ids(idx, n_idx, n_cols, blockIdx.x - 1 - clear_blocks, gridDim.x - 1 - clear_blocks, out);
         return;
     }
     if (blockIdx.x > 0) {
-        for (int k = (blockIdx.x - 1) * PLAN_SMALL_BLOCK + threadIdx.x; k < n_counters; k += clear_blocks * PLAN_SMALL_BLOCK) counters[k] = 0;
+        // 32 for every slot there may be: past 2^31 of them where the pieces are forced to be few nonzeros each
+        for (int64_t k = (int64_t)(blockIdx.x - 1) * PLAN_SMALL_BLOCK + threadIdx.x; k < n_counters; k += (int64_t)clear_blocks * PLAN_SMALL_BLOCK) counters[k] = 0;
         return;
     }
     __shared__ int s_scan[PLAN_SMALL_BLOCK / 32 + 1];

@@ -172,7 +172,7 @@ static int plan_fill_small(agcn_spmm_plan *p, int most, const int *d_indices, in
     const int64_t clear_blocks = ceil_div(counters, PLAN_SMALL_BLOCK * 16);
     AGCN_KERNEL(plan_small_kernel, (unsigned)(1 + clear_blocks + (col_blocks < 2368 ? col_blocks : 2368)), PLAN_SMALL_BLOCK, s, p->block4,
                 (int)p->n_blocks, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, most, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
-                p->zero_rows, spmm_carry_counters(p->carry, p->n_carry), (int)counters, (unsigned)clear_blocks, words.device());
+                p->zero_rows, spmm_carry_counters(p->carry, p->n_carry), counters, (unsigned)clear_blocks, words.device());
     AGCN_LAUNCH_CHECK("plan_small_kernel");
     AGCN_CUDA(words.sync());
     rc = plan_errors(words);

@@ -124,3 +124,13 @@ def test_synthetic_graphs_are_seeded_and_well_formed():
     assert g4.vals.min() > 0 and g4.vals.max() <= 1 and g4.info["max_degree"] > 384
     x = synth.features(100, 60, 1001, "cpu")
     assert x.shape == (100, 60) and x.min() >= -1 and x.max() < 1
+
+
+def test_arrival_counters_of_a_plan_travel_as_64_bits():
+    # a plan has 32 arrival counters per carry slot, more than 2^31 from 2^28 pieces on (pieces forced to one nonzero,
+    # 1.3e8 nonzeros, 43 GB on the GPU: not a test's size).  As an int their number was negative and none was cleared.
+    import subprocess
+    names = subprocess.run(["nm", "-C", _build()], capture_output=True, text=True, check=True).stdout
+    (args,) = re.findall(r" T agcn::plan_small_kernel\((.*)\)$", names, flags=re.M)
+    counters, number, blocks, words = [a.strip() for a in args.split(",")][-4:]
+    assert (counters, number, blocks, words) == ("int*", "long", "unsigned int", "agcn::HostWords*")
