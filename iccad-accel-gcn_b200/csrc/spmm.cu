@@ -440,14 +440,16 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     // Passes stay multiples of 32 columns so that every row segment is whole 128-byte lines.
     // AGCN_SPMM_PANEL (read when the plan is created) overrides the choice.  (A product whose A is
     // column-tiled -- agcn_spmm_tiled_* -- keeps its X slab in L2 by construction and never splits.)
+    const bool whole = unit0 == 0 && unit1 == p->n_units;
+    const bool loose = !x_vec && whole && spmm_loose(p);
+    const int64_t ldx_panel = loose ? (dim + 3) & ~3 : ldx_use;         // the passes, hence the sums, that the aligned copy would get
     int panel = SPMM_PANEL;
-    if (dim > 64 && dim % 32 == 0 && ldx_use % 32 == 0 && !accumulate && !p->never_split) {
+    if (dim > 64 && dim % 32 == 0 && ldx_panel % 32 == 0 && !accumulate && !p->never_split) {
         const int full = dim < SPMM_PANEL ? dim : SPMM_PANEL;
         const double x_bytes = (double)p->n_cols * full * 4.0;
         if (x_bytes > 0.75 * (double)p->l2_bytes && x_bytes <= 4.0 * (double)p->l2_bytes) panel = 64;
     }
     if (p->panel_override > 0) panel = p->panel_override;
-    const bool whole = unit0 == 0 && unit1 == p->n_units;
     // Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM),
     // where a second launch costs more than blocks that wait for a counter; parts of a product always do that.
     const bool carry_inside = !whole || p->split || p->n_units <= (int64_t)20 * p->sm_count;
@@ -456,7 +458,6 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     // passes are -- with the same passes, hence the same bits, as a whole run.
     if (!whole) AGCN_REQUIRE(dim <= SPMM_PANEL, "agcn_spmm_run: a product issued in unit ranges is limited to %d columns", SPMM_PANEL);
     AGCN_REQUIRE(panel >= 1 && panel <= SPMM_PANEL, "agcn_spmm_run: AGCN_SPMM_PANEL must be 1..%d", SPMM_PANEL);
-    const bool loose = !x_vec && whole && spmm_loose(p);
     if ((x_vec || loose) && panel % 4 != 0) panel = (panel + 3) & ~3;         // keep every panel's first column 16-byte aligned
     if (panel > SPMM_PANEL) panel = SPMM_PANEL;
     for (int col0 = 0, width = 0; col0 < dim; col0 += width) {

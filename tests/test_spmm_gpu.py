@@ -741,9 +741,37 @@ def test_small_products_from_rows_of_any_alignment(kind, dim):
             y = torch.full((n * ldy + shift,), 7.0, device=dev)[shift:]
             x.view(n, ldx)[:, :dim] = xs
             plan.run(idx, val, x, y, dim=dim, ldx=ldx, ldy=ldy, relu=relu)
+            assert plan.info()["launches_last_run"] == (dim + 127) // 128            # one a pass, none for a copy
             got = y.view(n, ldy)
             assert torch.equal(got[:, :dim].nan_to_num(3.0, 4.0, 5.0), want[:, :dim].nan_to_num(3.0, 4.0, 5.0)), (relu, shift, ldx, ldy)
             assert bool((got[:, dim:] == 7.0).all())
+    plan.close()
+
+
+def test_unaligned_rows_of_a_large_operand_get_the_passes_of_the_copy():
+    # few rows, an X larger than L2: a product of 128 columns runs as two passes of 64 (other slots, another order of the
+    # additions in rows of more than 32 nonzeros), also from rows that are not aligned and not copied
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    rng = np.random.default_rng(3)
+    n, cols, dim = 1_000, 260_000, 128
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(np.sort(rng.integers(0, 300, n)))]).astype(np.int32)).to(dev)
+    nnz = int(indptr[-1])
+    idx = torch.from_numpy(rng.integers(0, cols, nnz, dtype=np.int32)).to(dev)
+    val = torch.from_numpy(rng.standard_normal(nnz).astype(np.float32)).to(dev)
+    plan = spmm.SpmmPlan(partition.block_level_partition_device(indptr), idx, n, cols)
+    xs = torch.randn(cols, dim, device=dev, generator=torch.Generator(dev).manual_seed(1))
+    want = torch.empty((n, dim), device=dev)
+    plan.run(idx, val, xs, want)
+    assert plan.info()["launches_last_run"] == 2
+    for ldx, shift in ((129, 0), (128, 1), (131, 2)):
+        x = torch.full((cols * ldx + shift,), float("nan"), device=dev)[shift:]
+        x.view(cols, ldx)[:, :dim] = xs
+        got = torch.empty((n, dim), device=dev)
+        plan.run(idx, val, x, got, dim=dim, ldx=ldx, ldy=dim)
+        assert plan.info()["launches_last_run"] == 2                 # no copy
+        assert torch.equal(got, want), (ldx, shift)
     plan.close()
 
 
