@@ -154,6 +154,25 @@ def test_rows_per_thread_of_the_cluster_sort(items):
             assert np.array_equal(a, b), (n, what)
 
 
+@pytest.mark.parametrize("n", [3, 40, 8_192, 20_000])
+@pytest.mark.parametrize("long", [4 * 256, 4 * 256 + 1, 5 * 256, 32 * 256, 33 * 256 + 7, 3_000_000])
+def test_rows_that_begin_many_tiles_of_the_permute(n, long):
+    # the cluster sort marks where every 256th nonzero belongs: rows of up to four such places by their thread, longer ones
+    # by the warp, one or several of them side by side, before and behind each other
+    from accelgcn import degree_sort
+    require_cuda()
+    rng = np.random.default_rng(n + long)
+    deg = rng.integers(0, 300, n)
+    deg[rng.permutation(n)[:1 + min(n, 40) // 8]] = long
+    deg[n // 2] = long + 1
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    idx = rng.integers(0, n, int(indptr[-1]), dtype=np.int32)
+    val = rng.standard_normal(len(idx)).astype(np.float32)
+    got = degree_sort.degree_sort(indptr, idx, val, relabel_cols=True)
+    for a, b, what in zip(got, oracle.degree_sort(indptr, idx, val, relabel_cols=True), ("perm", "indptr", "indices", "vals")):
+        assert np.array_equal(a, b), what
+
+
 @pytest.mark.parametrize("n", [65_536 + 1, 65_536 * 2, 2_097_152, 2_101_249, 4_300_000])
 @pytest.mark.parametrize("kind", ["low", "high", "mixed"])
 def test_counters_of_tiles_groups_and_groups_of_groups(n, kind):
