@@ -877,8 +877,15 @@ plan_assign_kernel(const int4 *__restrict__ block4, int64_t n_blocks, int64_t n_
         for (int64_t k = threadIdx.x; k < s_gap_len[q]; k += PLAN_BLOCK) zero_rows[s_gap_out[q] + k] = (int)(s_gap_row[q] + k);
 }
 
-// The whole plan of a small graph in one launch: block 0 validates the tuples, cuts them into pieces of at most
-// `most` nonzeros (cap_pieces of them fit), lists the rows no tuple covers and hands out the carry slots; the next
+// How the tuples of a small graph are cut: into pieces of at most `most` nonzeros where that makes no more than `fit` of
+// them (`fit_uneven` where the rows are of very different lengths), else of at most `otherwise`.
+struct PieceChoice {
+    int most, otherwise;
+    int fit, fit_uneven;
+};
+
+// The whole plan of a small graph in one launch: block 0 validates the tuples, cuts them into pieces
+// (cap_pieces of them fit), lists the rows no tuple covers and hands out the carry slots; the next
 // clear_blocks zero the arrival counters of the slots, the other blocks check the column ids.  Every array has its final place already, sized by bounds the host knows, so the
 // host waits once.  (Two kernels with a wait between them before, the cutting 8 tuples per thread: a plan of 16 384
 // rows took 70 us; 26 now, 12 of them on the GPU.)  Bound by latency: a chain of scans over about ten tuples per thread.
@@ -886,7 +893,7 @@ constexpr int PLAN_SMALL_BLOCK = 1024;
 
 __global__ void __launch_bounds__(PLAN_SMALL_BLOCK)
 plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows, int64_t nnz, const int *__restrict__ idx, int64_t n_idx,
-                  int64_t n_cols, int most, int4 *pieces, int cap_pieces, int2 *unit_carry, int2 *carry_span, int *carry_row, int *zero_rows,
+                  int64_t n_cols, const PieceChoice choice, int4 *pieces, int cap_pieces, int2 *unit_carry, int2 *carry_span, int *carry_row, int *zero_rows,
                   int *counters, int64_t n_counters, unsigned clear_blocks, HostWords *out)
 {
     if (blockIdx.x > clear_blocks) {
@@ -902,11 +909,12 @@ plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows,
     __shared__ int s_gap_out[PLAN_GAP_QUEUE], s_gap_row[PLAN_GAP_QUEUE], s_gap_len[PLAN_GAP_QUEUE];
     __shared__ int s_gaps;
     if (threadIdx.x == 0) s_gaps = 0;
+    const int longest = block4[n_blocks - 1].x;            // of rows in degree order
     const int each = (n_blocks + PLAN_SMALL_BLOCK - 1) / PLAN_SMALL_BLOCK;
     const int e0 = min((int)threadIdx.x * each, n_blocks), e1 = min(e0 + each, n_blocks);
     const int4 before = e0 > 0 ? block4[e0 - 1] : make_int4(0, 0, 0, 0);
     int4 a = before;
-    int err = 0, mine = 0;
+    int err = 0, mine = 0, most = choice.most;
     int64_t zero = 0;
     for (int e = e0; e < e1; e++) {
         const int4 b = block4[e];
@@ -920,6 +928,16 @@ plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows,
     if (__syncthreads_or(err)) return;
     int n_pieces, n_zero;
     int piece = block_scan_exclusive<PLAN_SMALL_BLOCK>(mine, OpAdd(), 0, n_pieces, s_scan);
+    if (choice.otherwise != most) {
+        // rows of an even graph that are longer than a piece would cross thread blocks all of them: three of them fit a piece
+        const bool uneven = longest > 2 * most && longest * n_rows > 4 * nnz;
+        if (n_pieces > (uneven ? choice.fit_uneven : choice.fit) || (!uneven && 3 * nnz > most * n_rows)) {
+            most = choice.otherwise;
+            mine = 0;
+            for (int e = e0; e < e1; e++) mine += tuple_cut(block4[e], most).pieces;
+            piece = block_scan_exclusive<PLAN_SMALL_BLOCK>(mine, OpAdd(), 0, n_pieces, s_scan);
+        }
+    }
     int zero_out = block_scan_exclusive<PLAN_SMALL_BLOCK>((int)zero, OpAdd(), 0, n_zero, s_scan);
     if (threadIdx.x == 0) { out->w[PLAN_WORD_ZERO] = n_zero; out->w[PLAN_WORD_PIECES] = n_pieces; }
     if (n_pieces > cap_pieces) return;              // cannot be: valid tuples do not overlap

@@ -30,6 +30,9 @@ void plan_free(agcn_spmm_plan *p)
     delete p;
 }
 
+// Up to this many thread blocks a cut plan's products keep 16 gathers in flight per lane.
+static int spmm_deep_units(int sm_count) { return 8 * sm_count / 3; }
+
 // Nonzeros per piece when the tuples of a plan are to be cut into pieces, 0 when they are not.  A product ends with
 // its longest warp, so pieces are as small as the nonzeros that an SM has to go through allow; beyond 7 500 of them
 // (20 full tuples; the SM holds 32 to 40 warps) the extra warps cost more than they balance, unless there are few
@@ -38,31 +41,42 @@ void plan_free(agcn_spmm_plan *p)
 // 80 000 of 7 [3 900]: - / 15.1 / 13.5 / 15.2, dim 128: - / 25 / 23 / 25;  135 000 of 4 [3 400]: 50 / 34 / 31 / -;
 // 165 000 of 6 [6 300], dim 32: 17.4 / 13.4 / 14.2 / -, dim 128: 54 / 45 / 47 / -;  200 000 of 6 [7 700], dim 64:
 // 29.2 / 30.0 / 31.4 / -;  100 000 of 25 [17 000], dim 32: 25 / 33 / - / -.
-// Few nonzeros: as small as leaves the blocks two per SM in one wave (the form with 16 gathers in flight per lane).
-// 32 / 64 / 96, nonzeros per SM in brackets: 2 048 rows of 4 [70], dim 60, 128: 4.9 / 5.5 / 4.8, 5.2 / 5.9 / 6.7;  4 096 of 10
-// [300]: 5.8 / 6.1 / 6.6, 6.2 / 7.0 / 7.8;  8 192 of 8 [500]: 6.4 / 6.8 / 7.1, 7.1 / 7.5 / 8.7;  16 384 of 4 [550]: 6.8 / 6.8 / 7.2,
-// 7.2 / 7.6 / 8.9, dim 16: 5.9 / 5.5 / 5.8;  16 384 of 8 [1 000]: 8.2 / 7.6 / 8.0, 9.0 / 9.7 / 9.7, dim 16: 6.2 / 5.9 / 6.1;  8 192 of
-// 20 [1 160]: 8.2 / 8.7 / 7.8, 10.5 / 10.8 / 9.4;  16 384 of 14 [1 660]: 9.6 / 9.3 / 10.0, 12.8 / 11.6 / 13.5.
+// Two ranges (pieces of 64 leave SMs idle; they are just too many for two blocks per SM) have a second size, which the
+// kernel that cuts takes where its thread blocks fit: the form with 16 gathers
+// in flight has two per SM, and a second wave of equal blocks is as long as the first.  Blocks of graphs with hub rows are
+// not equal, the heavy ones go first, and up to 8/3 per SM are faster in that form.  Rows of an even graph that do not
+// fit a piece would have to meet across blocks, all of them, which costs more than short warps give.  us, one size / 64,
+// nonzeros per SM in brackets, dim 60 unless stated:
+// 32, taken: 8 192 rows of 8 [440]: 3.4 / 4.9;  power law, 2 048 of 14 [200], dim 60, 128: 5.6 / 6.3, 5.7 / 6.8;  4 500 of 4
+// [130], dim 16: 5.4 / 4.9;  not taken: rows of 20 [140], dim 32: 5.3 / 3.7;  of 100 [340], dim 16: 4.9 / 3.3;
+// 96, taken: 8 192 of 20 [1 110], 256 blocks: 6.3 / 9.6;  power law, 20 000 of 8 [1 140], 348: 8.1 / 9.2, 9 500 of 20 [1 360],
+// 338, dim 128 (the largest loss): 13.6 / 11.1;  skewed, 20 000 of 10 [1 300], 392: 9.1 / 10.9;  not taken: 1 000 of 200 [1 350],
+// 375: 12.2 / 6.6;  16 384 of 14 [1 550], 342: 10.4 / 6.3;  30 000 of 6 [1 220], 313, dim 32: 7.4 / 4.4;  4 096 of 40 [1 110], 256:
+// 6.2 / 4.9.
 // Beyond 80 tuples per SM one thread block takes so long to cut them that a plan used once loses (150 000 rows of 5:
 // 236 -> 244 us from the graph to Y).
-static int spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
+static PieceChoice spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
 {
     const int64_t per_sm = nnz / sm_count;
-    if (n_blocks > (int64_t)80 * sm_count) return 0;
-    if (per_sm <= 500) return 32;
-    if (per_sm <= 1050) return 64;
-    if (per_sm <= 1575) return 96;
-    if (per_sm <= 1900) return 64;
-    if (per_sm <= 2700) return 96;
-    if (per_sm <= 4000) return 128;
-    return per_sm <= 7500 || n_blocks + nnz / SPMM_DEG_BOUND <= (int64_t)80 * sm_count ? 192 : 0;
+    const auto always = [](int most) { return PieceChoice{most, most, 0, 0}; };
+    const auto where_it_fits = [&](int most) {
+        return PieceChoice{most, 64, SPMM_WARPS * SPMM_DEEP_MIN_BLOCKS * sm_count, SPMM_WARPS * spmm_deep_units(sm_count)};
+    };
+    if (n_blocks > (int64_t)80 * sm_count) return always(0);
+    if (per_sm <= 500) return where_it_fits(32);
+    if (per_sm > 1050 && per_sm <= 1575) return where_it_fits(96);
+    if (per_sm <= 1900) return always(64);
+    if (per_sm <= 2700) return always(96);
+    if (per_sm <= 4000) return always(128);
+    return always(per_sm <= 7500 || n_blocks + nnz / SPMM_DEG_BOUND <= (int64_t)80 * sm_count ? 192 : 0);
 }
 
 // A cut plan keeps room for a list of all rows: not where there are a great many without any nonzero.
-static int spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int sm_count)
+static PieceChoice spmm_piece_choice(int64_t n_blocks, int64_t n_rows, int64_t nnz, int sm_count)
 {
-    if (n_blocks == 0 || n_rows > ((int64_t)1 << 20)) return 0;
-    return env_int("AGCN_SPMM_PIECE", spmm_piece(n_blocks, nnz, sm_count));
+    if (n_blocks == 0 || n_rows > ((int64_t)1 << 20)) return PieceChoice{0, 0, 0, 0};
+    const int forced = env_int("AGCN_SPMM_PIECE", INT32_MIN);
+    return forced != INT32_MIN ? PieceChoice{forced, forced, 0, 0} : spmm_piece(n_blocks, nnz, sm_count);
 }
 
 // The thread blocks of (half) full tuples take about equally long and are started first.  Where there are a few more
@@ -103,7 +117,7 @@ bool spmm_plan_splits(int64_t n_blocks, int64_t n_rows, int64_t nnz)
 {
     int device = 0, sm_count = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) return true;
-    return spmm_piece_choice(n_blocks, n_rows, nnz, sm_count) > 0;
+    return spmm_piece_choice(n_blocks, n_rows, nnz, sm_count).most > 0;
 }
 
 // Order of the units, which are in ascending degree.  Starting at the heavy end leaves light units for the end of
@@ -155,10 +169,10 @@ static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int4 **pieces, cudaS
 }
 
 // One launch and one wait: the memory is sized by what the pieces can be at most (a piece that is not the last of
-// its tuple or row holds more than half of `most` nonzeros).
-static int plan_fill_small(agcn_spmm_plan *p, int most, const int *d_indices, int64_t n_idx, cudaStream_t s)
+// its tuple or row holds more than half of the nonzeros that a piece may have).
+static int plan_fill_small(agcn_spmm_plan *p, const PieceChoice &choice, const int *d_indices, int64_t n_idx, cudaStream_t s)
 {
-    const int64_t cap = p->n_blocks + 2 * p->nnz / most + 8;
+    const int64_t cap = p->n_blocks + 2 * p->nnz / (choice.most < choice.otherwise ? choice.most : choice.otherwise) + 8;
     AGCN_REQUIRE(cap < (int64_t)INT32_MAX / 4, "agcn_spmm_create: too many pieces");
     p->split = true;
     p->n_units = ceil_div(cap, SPMM_WARPS);
@@ -171,7 +185,7 @@ static int plan_fill_small(agcn_spmm_plan *p, int most, const int *d_indices, in
     const int64_t col_blocks = ceil_div(n_idx, PLAN_SMALL_BLOCK * 16), counters = p->n_carry * SPMM_CARRY_PASSES;
     const int64_t clear_blocks = ceil_div(counters, PLAN_SMALL_BLOCK * 16);
     AGCN_KERNEL(plan_small_kernel, (unsigned)(1 + clear_blocks + (col_blocks < 2368 ? col_blocks : 2368)), PLAN_SMALL_BLOCK, s, p->block4,
-                (int)p->n_blocks, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, most, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
+                (int)p->n_blocks, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, choice, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
                 p->zero_rows, spmm_carry_counters(p->carry, p->n_carry), counters, (unsigned)clear_blocks, words.device());
     AGCN_LAUNCH_CHECK("plan_small_kernel");
     AGCN_CUDA(words.sync());
@@ -255,8 +269,8 @@ int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, con
     p->block4 = reinterpret_cast<const int4 *>(d_block4);
     p->n_blocks = n_blocks; p->n_rows = n_rows; p->n_cols = n_cols; p->nnz = nnz;
     const int64_t n_idx = d_indices != nullptr ? nnz : 0;
-    const int most = spmm_piece_choice(n_blocks, n_rows, nnz, p->sm_count);
-    const int rc = most > 0 ? plan_fill_small(p, most, d_indices, n_idx, s) : plan_fill(p, d_indices, n_idx, s);
+    const PieceChoice choice = spmm_piece_choice(n_blocks, n_rows, nnz, p->sm_count);
+    const int rc = choice.most > 0 ? plan_fill_small(p, choice, d_indices, n_idx, s) : plan_fill(p, d_indices, n_idx, s);
     if (rc != AGCN_OK) return rc;
     p->panel_override = env_int("AGCN_SPMM_PANEL", 0);
     p->pad_unaligned = env_int("AGCN_SPMM_PAD", 1);
@@ -352,7 +366,7 @@ static bool x_rows_aligned(const float *d_x, int64_t ldx, int dim) { return dim 
 // on the copy; Y keeps the caller's layout and gets stores as wide as each row's alignment allows.
 // On return *x_use / *ldx_use name the operand to gather from and *x_vec says whether its rows
 // are 16-byte aligned.
-static bool spmm_deep(const agcn_spmm_plan *p) { return p->split && 3 * p->n_units <= (int64_t)8 * p->sm_count; }
+static bool spmm_deep(const agcn_spmm_plan *p) { return p->split && p->n_units <= spmm_deep_units(p->sm_count); }
 
 // Small products gather 4 bytes at a time from X as it is instead, with the additions of the 16-byte path in its order:
 // to a chain of latencies the copy adds a kernel, and where a row of X is named a few times the copy of it is a good part

@@ -748,6 +748,48 @@ def test_small_products_from_rows_of_any_alignment(kind, dim):
     plan.close()
 
 
+@pytest.mark.parametrize("rows,degree,hub,piece", [(8_192, 8, 0, 32), (9_000, 8, 0, 32), (9_268, 8, 0, 32), (9_269, 8, 0, 64), (3_000, 10, 0, 32), (3_000, 11, 0, 64),
+                                                   (3_000, 11, 64, 64), (3_000, 11, 65, 32), (10_000, 4, 0, 32), (2_500, 20, 0, 64), (2_500, 20, 79, 64), (2_500, 20, 81, 32), (2_500, 20, 700, 32),
+                                                   (9_472, 20, 0, 96), (9_476, 20, 0, 64), (9_476, 20, 2_000, 96), (11_500, 20, 2_000, 96),
+                                                   (4_096, 40, 0, 64), (4_096, 40, 1_000, 96), (16_384, 14, 0, 64), (16_384, 8, 0, 64), (16_384, 16, 0, 64)])
+def test_pieces_of_small_plans(rows, degree, hub, piece):
+    # how the plan of a small graph is cut is chosen by the number of pieces: where they leave two thread blocks (of 8) per
+    # SM, 8/3 with a last row of two pieces and of four times the mean, and rows of an even graph fit a piece three times
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
+        pytest.skip("sizes are those of 148 SMs")
+    deg = np.full(rows, degree)
+    if hub:
+        deg[-1] = hub
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    block4 = oracle.partition(indptr)
+
+    def pieces(most):
+        n = 0
+        for d, _, _, info in block4:
+            r, nz = (info & 0xFFFF, d) if d <= 384 else (1, info)
+            if nz <= most and d <= 384:
+                each = -(-r // -(-r // (most // nz)))
+                n += -(-r // each)
+            else:
+                n += r * -(-nz // -(-nz // -(-nz // most)))
+        return n
+
+    rng = np.random.default_rng(rows)
+    idx = rng.integers(0, rows, int(indptr[-1]), dtype=np.int32)
+    val = rng.standard_normal(len(idx)).astype(np.float32)
+    x = rng.standard_normal((rows, 33)).astype(np.float32)
+    d_idx, d_val, d_x = (torch.from_numpy(a).to(dev) for a in (idx, val, x))
+    y = torch.full((rows, 33), float("nan"), device=dev)
+    plan = spmm.SpmmPlan(torch.from_numpy(block4).to(dev), d_idx, rows, rows)
+    assert plan.info()["n_units"] == -(-pieces(piece) // 8)
+    plan.run(d_idx, d_val, d_x, y)
+    assert spmm_close(y.cpu().numpy(), oracle.spmm_csr(indptr, idx, val, x), row_abs_scale(indptr, val, x)).all()
+    plan.close()
+
+
 def test_unaligned_rows_of_a_large_operand_get_the_passes_of_the_copy():
     # few rows, an X larger than L2: a product of 128 columns runs as two passes of 64 (other slots, another order of the
     # additions in rows of more than 32 nonzeros), also from rows that are not aligned and not copied
