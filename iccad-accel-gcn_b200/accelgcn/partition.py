@@ -40,7 +40,9 @@ def block_level_partition_device(indptr, stream=None):
     """Device tensor in (torch int32 CUDA tensor [n_rows+1]), device tensor out [n_blocks, 4].
 
     On the current stream the tuples are written behind what that stream holds, like the result of any torch
-    operation.  With another `stream` they are complete when the call returns: neither tensor is known to torch's
+    operation, and indptr is read there after the call has returned, whatever its size: an indptr that another
+    stream overwrites, or that torch's allocator holds for another stream (record_stream), has to wait for this one.
+    With another `stream` they are complete when the call returns: neither tensor is known to torch's
     allocator as in use there, and the caller may go on with them anywhere."""
     import torch
     if not (indptr.is_cuda and indptr.dtype == torch.int32 and indptr.is_contiguous()):

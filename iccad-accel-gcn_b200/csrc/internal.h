@@ -33,8 +33,8 @@ int env_int(const char *name, int dflt);
 
 // partition.cu
 int partition_device(const int *d_indptr, int64_t n_rows, int *d_block4, int64_t cap_blocks, int64_t *n_blocks, cudaStream_t s);
-// The same in two halves: begin counts (and waits for the stream), finish fills n_blocks tuples asynchronously
-// and gives the scratch back (d_block4 == nullptr: only that).
+// The same in two halves: begin counts (and waits for the stream), finish fills n_blocks tuples asynchronously, from the
+// row pointers, and gives the scratch back (d_block4 == nullptr: only that).
 struct PartitionRun {
     const int *indptr = nullptr;
     int64_t n_rows = 0, n_blocks = 0;

@@ -69,7 +69,9 @@ int agcn_partition_device(const int32_t *d_indptr, int64_t n_rows,
 
 /* The same in two halves, for callers that allocate the output in between: begin counts (and waits for the
  * stream), finish fills d_block4 [n_blocks x 4] behind what `stream` holds, without waiting, and ends the run
- * (d_block4 == NULL only ends it).  d_indptr must stay unchanged until then. */
+ * (d_block4 == NULL only ends it).  What finish puts on `stream` reads d_indptr, for graphs of any size: it must stay
+ * valid and unchanged until the stream has got that far, not only until finish returns (work behind it on the same
+ * stream may overwrite or free it). */
 typedef struct agcn_partition_run agcn_partition_run;
 int agcn_partition_begin(const int32_t *d_indptr, int64_t n_rows, agcn_partition_run **run, int64_t *n_blocks, void *stream);
 int agcn_partition_finish(agcn_partition_run *run, int32_t *d_block4);

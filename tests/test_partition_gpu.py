@@ -116,7 +116,7 @@ def test_runs_across_tiles_match_oracle(run):
     import torch
     from accelgcn import partition
     dev = require_cuda()
-    # the last: more tuples than the scratch of the one-pass form holds (two per row and 1024), so it counts again
+    # the last: 391 thousand tuples in the run's rows, many tiles of more than 4096
     for degs in ([1, 40, 70, 100, 150, 300, 385], [0, 7], [33, 0, 33, 500], [2, 150_000_000 // run, 3]):
         indptr = np.concatenate([[0], np.cumsum(np.repeat(degs, run))]).astype(np.int32)
         want = oracle.partition(indptr)
@@ -128,9 +128,8 @@ def test_runs_across_tiles_match_oracle(run):
 @pytest.mark.parametrize("total", [4095, 4096, 4097, 8192, 30_000])
 def test_tiles_of_many_tuples_match_oracle(rows, total):
     # a tile (2048 rows) of more than 4096 tuples is written by several blocks, 4096 output positions each: hub rows that
-    # make up `total` tuples between rows of one and of none, at the start, at the end and in neighbouring tiles; both the
-    # form that counts and writes in one go (up to 524 288 rows) and the other
-    # (the first tile has exactly `total` of them)
+    # make up `total` tuples between rows of one and of none, at the start, at the end and in neighbouring tiles; few tiles,
+    # and more than the 256 that the scan of the tiles takes at a time (the first tile has exactly `total` tuples)
     import torch
     from accelgcn import partition
     dev = require_cuda()
@@ -149,8 +148,8 @@ def test_tiles_of_many_tuples_match_oracle(rows, total):
 
 @pytest.mark.parametrize("n", [5_000, 700_000])
 def test_on_another_stream_the_tuples_are_complete_on_return(n):
-    # one-pass form (up to 256 tiles of 2048 rows) and the form whose last kernel still reads the row pointers: with a
-    # stream that is not the current one the caller goes on elsewhere, here while that stream is kept busy
+    # with a stream that is not the current one the caller goes on elsewhere, here while that stream is kept busy; few tiles
+    # of 2048 rows, and more than the 256 that their scan takes at a time
     import torch
     from accelgcn import partition
     dev = require_cuda()
@@ -167,6 +166,25 @@ def test_on_another_stream_the_tuples_are_complete_on_return(n):
         assert np.array_equal(out.cpu().numpy(), want)
         with torch.cuda.stream(side):
             busy.add_(1)
+
+
+@pytest.mark.parametrize("n", [5_000, 2_048 * 256, 2_048 * 256 + 1, 700_000])
+def test_row_pointers_may_be_overwritten_behind_the_call_on_its_stream(n):
+    # the tuples are written behind the call, from the row pointers; work behind it on the same stream comes later.  The
+    # scan of the tiles takes 256 at a time: one round of it, exactly, and a second one of a single row
+    import torch
+    from accelgcn import partition
+    dev = require_cuda()
+    indptr = np.concatenate([[0], np.cumsum(np.sort(np.random.default_rng(n).integers(0, 60, n)))]).astype(np.int32)
+    want = oracle.partition(indptr)
+    src = torch.from_numpy(indptr).to(dev)
+    for _ in range(4):
+        d_ip = src.clone()
+        out = partition.block_level_partition_device(d_ip)
+        d_ip.fill_(7)
+        del d_ip
+        torch.full((n + 1,), -1, dtype=torch.int32, device=dev)          # takes the block that was just given back
+        assert np.array_equal(out.cpu().numpy(), want)
 
 
 def test_count_does_not_depend_on_what_the_scratch_held():
