@@ -748,6 +748,31 @@ def test_small_products_from_rows_of_any_alignment(kind, dim):
     plan.close()
 
 
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+@pytest.mark.parametrize("nnz", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 4_099, 6_000_001])
+def test_a_column_id_outside_is_found_wherever_it_is(nnz, shift):
+    # ids are checked 16 bytes at a time but for the ends that are not aligned: one bad id at either end, next to them and
+    # inside, of arrays that begin at any of the four places of 16 bytes; small plans, and (6e6 nonzeros, uncut) large ones
+    import torch
+    from accelgcn import spmm, AccelGcnError
+    dev = require_cuda()
+    cols = 1_000
+    deg = [min(384, nnz - at) for at in range(0, nnz, 384)]
+    block4 = torch.from_numpy(oracle.partition(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32))).to(dev)
+    room = torch.full((nnz + 8,), -1, dtype=torch.int32, device=dev)         # what lies around them is not looked at
+    idx = room[shift:shift + nnz]
+    idx.copy_(torch.arange(nnz, device=dev) % cols)
+    idx[-1] = cols - 1
+    spmm.SpmmPlan(block4, idx, len(deg), cols).close()
+    for at in sorted({k for k in (0, 1, 2, 3, 4, nnz // 2, nnz - 5, nnz - 4, nnz - 3, nnz - 2, nnz - 1) if 0 <= k < nnz}):
+        was = int(idx[at])
+        for bad in (cols, -1, 2**31 - 1, -2**31):
+            idx[at] = bad
+            with pytest.raises(AccelGcnError, match="column index"):
+                spmm.SpmmPlan(block4, idx, len(deg), cols)
+        idx[at] = was
+
+
 @pytest.mark.parametrize("rows,degree,hub,piece", [(8_192, 8, 0, 32), (9_000, 8, 0, 32), (9_268, 8, 0, 32), (9_269, 8, 0, 64), (3_000, 10, 0, 32), (3_000, 11, 0, 64),
                                                    (3_000, 11, 64, 64), (3_000, 11, 65, 32), (10_000, 4, 0, 32), (2_500, 20, 0, 64), (2_500, 20, 79, 64), (2_500, 20, 81, 32), (2_500, 20, 700, 32),
                                                    (9_472, 20, 0, 96), (9_476, 20, 0, 64), (9_476, 20, 2_000, 96), (11_500, 20, 2_000, 96),
