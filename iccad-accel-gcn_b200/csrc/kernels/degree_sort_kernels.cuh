@@ -454,7 +454,7 @@ constexpr int SMALL_BLOCK = 1024;
 constexpr int SMALL_WARPS = SMALL_BLOCK / 32;
 constexpr int SMALL_ITEMS = 8;
 constexpr int SMALL_MAX_ROWS = SMALL_CLUSTER * SMALL_BLOCK * SMALL_ITEMS;
-constexpr unsigned SMALL_MARKS = 4;                  // tiles of a row that its thread marks by itself
+constexpr unsigned SMALL_MARKS = 64;                 // tiles of a row that its thread marks by itself
 constexpr int small_smem_bytes(int items) { return SMALL_BLOCK * items * 8 + SMALL_WARPS * RADIX_BINS * 2; }
 
 // items = rows per thread: ceil(n / 8192), at most SMALL_ITEMS
@@ -588,9 +588,10 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
         const int i = first + k * 32;
         const unsigned incl = warp_scan_inclusive(key[k], OpAdd()), b = e + incl - key[k];
         e += __shfl_sync(FULL_MASK, incl, 31);
-        // the tiles that begin in the row (none past the end: no nonzeros).  Those of a row of many are dealt out to the
-        // warp: by one thread a hub row of 1e7 nonzeros made the sort of 60 000 rows of 25 take 313 us instead of 131, 300 rows
-        // of 30 000 90 instead of 74.
+        // the tiles that begin in the row (none past the end: no nonzeros).  Those of a row of a great many are dealt out to the
+        // warp, row after row: by one thread a hub row of 1e7 nonzeros made the sort of 60 000 rows of 25 take 313 us instead
+        // of 131, 300 rows of 30 000 90 instead of 74.  (From 4 tiles on, or the tiles of 32 rows at once and a search for
+        // whose each is, power-law graphs of up to 16 000 nonzeros per row lost up to 15 and 7 us of 190.)
         unsigned t = (b + PERMUTE_TILE - 1) / PERMUTE_TILE;
         const unsigned t_end = mark ? (b + key[k] + PERMUTE_TILE - 1) / PERMUTE_TILE : t;
         for (unsigned many = __ballot_sync(FULL_MASK, t_end - t > SMALL_MARKS); many != 0; many &= many - 1) {

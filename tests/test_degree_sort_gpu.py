@@ -155,9 +155,9 @@ def test_rows_per_thread_of_the_cluster_sort(items):
 
 
 @pytest.mark.parametrize("n", [3, 40, 8_192, 20_000])
-@pytest.mark.parametrize("long", [4 * 256, 4 * 256 + 1, 5 * 256, 32 * 256, 33 * 256 + 7, 3_000_000])
+@pytest.mark.parametrize("long", [2 * 256, 64 * 256, 64 * 256 + 1, 65 * 256, 96 * 256, 97 * 256 + 7, 3_000_000])
 def test_rows_that_begin_many_tiles_of_the_permute(n, long):
-    # the cluster sort marks where every 256th nonzero belongs: rows of up to four such places by their thread, longer ones
+    # the cluster sort marks where every 256th nonzero belongs: rows of up to 64 such places by their thread, longer ones
     # by the warp, one or several of them side by side, before and behind each other
     from accelgcn import degree_sort
     require_cuda()
