@@ -60,7 +60,8 @@ static PieceChoice spmm_piece(int64_t n_blocks, int64_t nnz, int sm_count)
     const int64_t per_sm = nnz / sm_count;
     const auto always = [](int most) { return PieceChoice{most, most, 0, 0}; };
     const auto where_it_fits = [&](int most) {
-        return PieceChoice{most, 64, SPMM_WARPS * SPMM_DEEP_MIN_BLOCKS * sm_count, SPMM_WARPS * spmm_deep_units(sm_count)};
+        const PieceChoice c = {most, 64, SPMM_WARPS * SPMM_DEEP_MIN_BLOCKS * sm_count, SPMM_WARPS * spmm_deep_units(sm_count)};
+        return n_blocks > c.fit_uneven || nnz > (int64_t)most * c.fit_uneven ? always(64) : c;       // more pieces than fit for certain
     };
     if (n_blocks > (int64_t)80 * sm_count) return always(0);
     if (per_sm <= 500) return where_it_fits(32);
