@@ -581,33 +581,38 @@ sort_small_kernel(const int *__restrict__ indptr, int n, int items, int64_t nnz,
     cluster.barrier_arrive();    // this block reads no other one's shared memory any more
     unsigned e = __shfl_sync(FULL_MASK, start, 0);
     for (int b = 0; b < block; b++) e += s_get[b][0];
-    const bool mark = map.tile_row != nullptr && !bad;
+    const bool mark = map.tile_row != nullptr && !bad, hubs = top > SMALL_MARKS * PERMUTE_TILE;
 #pragma unroll
     for (int k = 0; k < SMALL_ITEMS; k++) {
         if (k >= items) break;
         const int i = first + k * 32;
         const unsigned incl = warp_scan_inclusive(key[k], OpAdd()), b = e + incl - key[k];
         e += __shfl_sync(FULL_MASK, incl, 31);
+        if (i < n) {
+            perm[i] = row[k];
+            if (map.new_id != nullptr) map.new_id[row[k]] = i;
+            if (new_indptr != nullptr) {
+                new_indptr[i] = (int)b;
+                if (map.delta != nullptr) map.delta[i] = indptr[row[k]] - indptr[0] - (int)b;
+                if (i == n - 1) new_indptr[n] = (int)(b + key[k]);
+            }
+        }
+        if (!mark) continue;
         // the tiles that begin in the row (none past the end: no nonzeros).  Those of a row of a great many are dealt out to the
         // warp, row after row: by one thread a hub row of 1e7 nonzeros made the sort of 60 000 rows of 25 take 313 us instead
         // of 131, 300 rows of 30 000 90 instead of 74.  (From 4 tiles on, or the tiles of 32 rows at once and a search for
         // whose each is, power-law graphs of up to 16 000 nonzeros per row lost up to 15 and 7 us of 190.)
         unsigned t = (b + PERMUTE_TILE - 1) / PERMUTE_TILE;
-        const unsigned t_end = mark ? (b + key[k] + PERMUTE_TILE - 1) / PERMUTE_TILE : t;
-        for (unsigned many = __ballot_sync(FULL_MASK, t_end - t > SMALL_MARKS); many != 0; many &= many - 1) {
-            const int from = __ffs(many) - 1;
-            const unsigned last = __shfl_sync(FULL_MASK, t_end, from);
-            for (unsigned q = __shfl_sync(FULL_MASK, t, from) + lane; q < last; q += 32) map.tile_row[q] = i - lane + from;
+        const unsigned t_end = (b + key[k] + PERMUTE_TILE - 1) / PERMUTE_TILE;
+        if (hubs) {
+            for (unsigned many = __ballot_sync(FULL_MASK, t_end - t > SMALL_MARKS); many != 0; many &= many - 1) {
+                const int from = __ffs(many) - 1;
+                const unsigned last = __shfl_sync(FULL_MASK, t_end, from);
+                for (unsigned q = __shfl_sync(FULL_MASK, t, from) + lane; q < last; q += 32) map.tile_row[q] = i - lane + from;
+            }
+            if (t_end - t > SMALL_MARKS) continue;
         }
-        if (t_end - t <= SMALL_MARKS)
-            for (; t < t_end; t++) map.tile_row[t] = i;
-        if (i >= n) continue;
-        perm[i] = row[k];
-        if (map.new_id != nullptr) map.new_id[row[k]] = i;
-        if (new_indptr == nullptr) continue;
-        new_indptr[i] = (int)b;
-        if (map.delta != nullptr) map.delta[i] = indptr[row[k]] - indptr[0] - (int)b;
-        if (i == n - 1) new_indptr[n] = (int)(b + key[k]);
+        for (; t < t_end; t++) map.tile_row[t] = i;
     }
     cluster.barrier_wait();      // no block ends while another may read its shared memory
 }
