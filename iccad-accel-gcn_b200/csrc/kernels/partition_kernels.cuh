@@ -16,7 +16,8 @@
 // closes the open runs, and leaves every tile its incoming run start and its first
 // output position; (C) every row writes its own tuples.  The host waits between (B) and (C), for
 // the number of tuples it has to find room for, and not behind (C).
-// Bound: launch latency up to some 100 000 rows, instruction issue above.
+// Bound: launches and the wait up to some 100 000 rows; above, instruction issue and a tile's chain of loads, scans and
+// stores (2.4 M rows of 25: 16 and 19 us, of which HBM needs 4).
 #pragma once
 #include "../host_common.h"
 #include "primitives.cuh"
@@ -235,7 +236,7 @@ part_describe_kernel(const int *__restrict__ indptr, int64_t n_rows, PartTileInf
 // them, so the tiles of a graph's hub rows have many times the tuples of the others: tuples are then dealt out one per
 // thread, which looks its row up in the scanned offsets, and a tile of more than PART_CHUNK is shared by the blocks
 // before the tile blocks, PART_CHUNK output positions each.  (Row by row the last of 1172 tiles, 2.4 M rows of 25,
-// kept the kernel for 44 us; 21 now.)
+// kept the kernel for 44 us; 19 now.)
 constexpr int PART_CHUNK = 4096;
 
 // The tuples of one tile that lie at output positions [lo, hi), hi <= first_out + their number.

@@ -378,7 +378,7 @@ spmm_units_kernel(const SpmmParams p)
     const bool active = ycol < (ANY_ROWS ? p.dim_store : p.dim);
     L2Policies pol = make_l2_policies();
     if (HOT) pol.hot = p.hot_column;
-    if (ANY_ROWS) pol.cols = (p.dim_store - sl + S - 1) / S;
+    if constexpr (ANY_ROWS) pol.cols = (p.dim_store - sl + S - 1) / S;
 
     if (!p.wait_first) launch_dependents();     // a dense transform of this product's result may lay out its weights meanwhile
     if (p.abort_flag != nullptr && *p.abort_flag != 0) return;     // input rejected by a check earlier in the stream

@@ -303,7 +303,7 @@ struct SpmmForm {
     bool finish;     // rows that cross units are finished in the launch
     bool deep;       // few thread blocks, many gathers per lane
     bool wide;       // more thread blocks per SM, fewer gathers per lane
-    bool loose;      // rows of X of any alignment (deep launches only)
+    bool loose;      // rows of X of any alignment, 4 bytes at a time (cut plans: spmm_loose)
 };
 
 template <int S>
@@ -353,6 +353,9 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
     const int ldp = (dim + 3) & ~3;
     const int64_t blocks = ceil_div(n_rows * (ldp >> 2), PAD_BLOCK * PAD_ITEMS);
     AGCN_REQUIRE(blocks < (int64_t)INT32_MAX, "agcn_spmm_run: operand too large to pad");
+    // Early: it is resident when the operation before it ends.  135 small graphs, dims 17 to 127, not early / early: in a
+    // stream 1.02 on average, up to 1.4 (4 096 rows of 40, dim 17: 8.3 / 5.8 us), 500 000 of 12, dim 17: 84.1 / 81.0;  in a
+    // replayed graph, where launches are closer, 0.97, at worst 16.9 / 18.8 (100 000 of 10, dim 17).
     AGCN_CUDA(launch_early(true, spmm_pad_rows_kernel, (unsigned)blocks, PAD_BLOCK, 0, s, d_x, ldx, dim, d_xp, ldp, n_rows));
     AGCN_LAUNCH_CHECK("spmm_pad_rows_kernel");
     return AGCN_OK;
@@ -360,13 +363,6 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
 
 static bool x_rows_aligned(const float *d_x, int64_t ldx, int dim) { return dim % 4 == 0 && ldx % 4 == 0 && aligned16(d_x); }
 
-// Rows of X that are not 16-byte aligned (dim % 4 != 0 with the reference's ld = dim, an odd
-// stride or base) would force 4-byte gathers: 1.2-1.6x the time of the 16-byte path.  Instead X
-// is copied once into plan-owned rows padded to a multiple of 4 floats (2 * n_cols * dim * 4
-// bytes of streaming traffic against nnz * dim * 4 bytes of gather) and the 16-byte path runs
-// on the copy; Y keeps the caller's layout and gets stores as wide as each row's alignment allows.
-// On return *x_use / *ldx_use name the operand to gather from and *x_vec says whether its rows
-// are 16-byte aligned.
 static bool spmm_deep(const agcn_spmm_plan *p) { return p->split && p->n_units <= spmm_deep_units(p->sm_count); }
 
 // Small products gather 4 bytes at a time from X as it is instead, with the additions of the 16-byte path in its order:
@@ -377,6 +373,9 @@ static bool spmm_deep(const agcn_spmm_plan *p) { return p->split && p->n_units <
 // 80 000 of 4 [2 700, 5]: - , 20.4 / 14.3, 37.0 / 26.8;  but
 // 1 000 dense of 150 [1 000, 150]: 9.5 / 9.5, 11.4 / 11.9, 14.2 / 15.6;  30 000 skewed of 16 [3 200, 16]: 14.9 / 12.2, 16.6 / 17.6,
 // 26.7 / 26.7;  100 000 skewed of 10 [6 800, 10]: 17.8 / 20.7, 29.7 / 32.4, 62.0 / 64.8.
+// The widths turn the balance both ways (rows named 13 to 16 times gain at 17 columns and lose at 61), so the limits leave
+// gains: they are where no width of the graphs above loses.  Over 68 graphs inside them, dims 17, 61, 127: 0.82 of the time
+// with the copy; slower: 30 000 rows of exactly 12 and 16 384 of exactly 10, dim 17 (12 and 7 %), 500 of 100, dim 127 (3 to 7 %).
 // (Its sums take 4 S places of a carry slot where the columns may be fewer: forced passes might not leave them.)
 static bool spmm_loose(const agcn_spmm_plan *p)
 {
@@ -384,6 +383,13 @@ static bool spmm_loose(const agcn_spmm_plan *p)
     return (spmm_deep(p) && p->nnz <= (int64_t)500 * p->sm_count) || (p->nnz <= 13 * p->n_cols && p->nnz <= (int64_t)2700 * p->sm_count);
 }
 
+// Rows of X that are not 16-byte aligned (dim % 4 != 0 with the reference's ld = dim, an odd
+// stride or base) would force 4-byte gathers: 1.2-1.6x the time of the 16-byte path.  Instead X
+// is copied once into plan-owned rows padded to a multiple of 4 floats (2 * n_cols * dim * 4
+// bytes of streaming traffic against nnz * dim * 4 bytes of gather) and the 16-byte path runs
+// on the copy; Y keeps the caller's layout and gets stores as wide as each row's alignment allows.
+// On return *x_use / *ldx_use name the operand to gather from and *x_vec says whether its rows
+// are 16-byte aligned.
 int spmm_prepare_x(agcn_spmm_plan *p, const float *d_x, int64_t ldx, int dim, cudaStream_t s,
                    const float **x_use, int64_t *ldx_use, bool *x_vec)
 {
