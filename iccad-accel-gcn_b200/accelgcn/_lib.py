@@ -57,6 +57,7 @@ PROTOTYPES = {
     "agcn_spmm_tiled_info": (_int, [_vp, ctypes.POINTER(_int), ctypes.POINTER(_i64), _vp, ctypes.POINTER(_int)]),
     "agcn_spmm_tiled_suggest": (_int, [_i64, _i64, _i64, _int]),
     "agcn_gemm_tf32_async": (_int, [_vp, _i64, _vp, _vp, _i64, _i64, _int, _int, _vp, _vp]),
+    "agcn_gemm_tf32_pair_async": (_int, [_vp, _vp, _vp, _vp, _i64, _vp, _vp]),
     "agcn_gemm_tf32_selftest_timeout": (_int, [_vp, _i64, _vp, _vp, _i64, _i64, _vp]),
     "agcn_gcn_fused_layer": (_int, [_vp, _vp, _vp, _vp, _vp, _vp, _i64, _i64, _vp, _vp]),
     "agcn_balanced_blocks": (_int, [_vp, _i64, _int, _vp, ctypes.POINTER(_i64)]),
@@ -76,6 +77,7 @@ PROTOTYPES = {
     "agcn_gcn2_forward_create": (_int, [ctypes.POINTER(_vp), _vp, _vp, _vp]),
     "agcn_gcn2_forward_run": (_int, [_vp, _vp, _vp, _vp]),
     "agcn_gcn2_forward_status": (_int, [_vp, _vp]),
+    "agcn_gcn2_forward_launches": (_int, [_vp, ctypes.POINTER(_int)]),
     "agcn_gcn2_forward_destroy": (_int, [_vp]),
     "agcn_probe_gather_bandwidth": (_int, [_i64, _int, _i64, _int, _int, ctypes.POINTER(ctypes.c_double)]),
 }

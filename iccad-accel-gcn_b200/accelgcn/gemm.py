@@ -36,6 +36,23 @@ def gemm_tf32_async(h, w, out, status, stream=None):
     return out
 
 
+def gemm_tf32_pair_async(p, w1, w2, out, status, stream=None):
+    """out = relu(p @ w1) @ w2 in one kernel (agcn_gemm_tf32_pair_async): contiguous fp32 CUDA tensors, p and out [m, 128],
+    both weights [128, 128].  `status` as in gemm_tf32_async."""
+    import torch
+    lib = _lib.load()
+    for t in (p, w1, w2, out):
+        if not (t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() and t.dim() == 2 and t.shape[1] == 128):
+            raise TypeError("gemm_tf32_pair_async needs contiguous float32 CUDA tensors of 128 columns")
+    if w1.shape[0] != 128 or w2.shape[0] != 128 or p.shape != out.shape:
+        raise ValueError("gemm_tf32_pair_async: weights must be [128, 128], out as p")
+    s = stream if stream is not None else torch.cuda.current_stream(p.device)
+    with torch.cuda.device(p.device):
+        _lib.check(lib.agcn_gemm_tf32_pair_async(p.data_ptr(), w1.data_ptr(), w2.data_ptr(), out.data_ptr(), p.shape[0],
+                                                 status.data_ptr(), s.cuda_stream))
+    return out
+
+
 def selftest_timeout(h, w, out, stream=None) -> int:
     """Runs the kernel's failure path on purpose (agcn_gemm_tf32_selftest_timeout) and returns the
     status code of the call: ERR_CUDA when the starved wait ran out and the kernel left cleanly."""

@@ -112,6 +112,8 @@ struct agcn_gcn2 {
     cudaEvent_t ev[8] = {};
     unsigned long long *d_stamps = nullptr;   // begin and end of the two transforms (ns), of a run that exchanged nothing
     bool alone = false;                       // ... as the last one did: its events are 0 and 7
+    bool paired = false;                      // ... with both transforms in one kernel, the first pair of the stamps
+    int launches = 0;                         // kernels of the last run
     // AGCN_GCN_FUSED=1: the leading rows of the block (at most 32 nonzeros each) go through one kernel
     // from layer 1's gathered operand to layer 2's operand; the other rows through SpMM and GEMM as before
     float *z2 = nullptr;                      // [per x 128]: layer 2's operand
@@ -523,6 +525,14 @@ extern "C" int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const 
     return AGCN_OK;
 }
 
+// From this many rows on, a forward that exchanges nothing applies A to X before W1, so that the two transforms follow one
+// another and are one kernel: A (X W1) = (A X) W1.  One pass over the activations less (1 KiB of HBM traffic per row) and one
+// launch less.  us per forward, transforms apart / together, B200, 128 features, power law: 30 000 rows of 12: 59.0 / 52.8;
+// 60 000 of 12: 97.8 / 83.9; 100 000 of 20: 184.6 / 166.8; 400 000 of 20: 769 / 697; 1 M of 12: 1 554 / 1 365; 2.5 M of 20:
+// 5 621 / 5 164.  16 384 of 8 would gain as well (46.4 / 41.1): smaller forwards are left with the bits of agcn_gemm_tf32 and
+// agcn_spmm_run_act called in turn.
+constexpr int64_t GCN_PAIR_ROWS = 32768;
+
 // Enqueues one forward on `stream` and returns without waiting.  d_x_block / d_out_block are this
 // rank's rows [rows_per_block x 128] (padding rows zero).  Per layer: Z = H * W on the tensor
 // cores, all-gather of Z on the communication stream (slice by slice), relu(A_block * Z).
@@ -534,32 +544,47 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
     agcn_dist *d = fwd->dist;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (d->world == 1 && d->tiled == nullptr && fwd->fused_rows == 0) {
-        // Nothing is exchanged: transform and product alternate on the stream, each starting while the one before it
+        // Nothing is exchanged: transforms and products alternate on the stream, each starting while the one before it
         // ends.  The transforms note their own times: events between the kernels keep them apart (13 us of a forward
         // over 16 384 rows), and so would a memset of their status words (which keep what they hold until it is read).  (A
         // product does not start before the transform's end: thread blocks that wait for it on SMs
         // taken by the transform spread the heavy rows unevenly, 2 % of a forward over 5 M rows.)
         fwd->alone = true;
+        fwd->paired = d->per >= GCN_PAIR_ROWS;
+        fwd->launches = 0;
         const DeviceOf on(d->plan->device);
-        AGCN_CUDA(cudaEventRecord(fwd->ev[0], s));
-        for (int layer = 0; layer < 2; layer++) {
-            int rc = gemm_tf32_async(layer == 0 ? d_x_block : fwd->h1, 128, fwd->w[layer], fwd->z, 128, d->per, fwd->d_status + layer, s,
-                                     true, layer == 1, fwd->d_stamps + 2 * layer);
-            if (rc != AGCN_OK) return rc;
-            float *out = layer == 0 ? fwd->h1 : d_out_block;
-            rc = spmm_check_run_args(d->plan, d->idx, d->val, fwd->z, 128, out, 128, 128, AGCN_ACT_RELU);
+        const auto product = [&](const float *x, float *y, int activation, SpmmLaunchPart::Early early) {
+            int rc = spmm_check_run_args(d->plan, d->idx, d->val, x, 128, y, 128, 128, activation);
             if (rc != AGCN_OK) return rc;
             SpmmLaunchPart part;
-            if (d->per > 0) part.early = SpmmLaunchPart::ONLY_X;
+            part.early = early;
             d->plan->launches_last_run = 0;
-            rc = spmm_run_prepared(d->plan, d->idx, d->val, fwd->z, 128, true, out, 128, 128, s, AGCN_ACT_RELU, 0, part);
-            if (rc != AGCN_OK) return rc;
+            rc = spmm_run_prepared(d->plan, d->idx, d->val, x, 128, true, y, 128, 128, s, activation, 0, part);
             d->launches_last_step = d->plan->launches_last_run;
+            fwd->launches += d->launches_last_step + 1;           // and the transform before it
+            return rc;
+        };
+        const auto made_here = d->per > 0 ? SpmmLaunchPart::ONLY_X : SpmmLaunchPart::NO;
+        AGCN_CUDA(cudaEventRecord(fwd->ev[0], s));
+        int rc = AGCN_OK;
+        if (fwd->paired) {
+            AGCN_REQUIRE(aligned16(d_x_block), "agcn_gcn2_forward_run: X must be 16-byte aligned");
+            rc = product(d_x_block, fwd->h1, AGCN_ACT_NONE, SpmmLaunchPart::ANY);
+            if (rc == AGCN_OK) rc = gemm_pair_async(fwd->h1, fwd->w[0], fwd->w[1], fwd->z, d->per, fwd->d_status, s, fwd->d_stamps);
+            if (rc == AGCN_OK) rc = product(fwd->z, d_out_block, AGCN_ACT_RELU, made_here);
+            fwd->launches--;                                      // two products, one transform
         }
+        for (int layer = 0; layer < 2 && !fwd->paired && rc == AGCN_OK; layer++) {
+            rc = gemm_tf32_async(layer == 0 ? d_x_block : fwd->h1, 128, fwd->w[layer], fwd->z, 128, d->per, fwd->d_status + layer, s,
+                                 true, layer == 1, fwd->d_stamps + 2 * layer);
+            if (rc == AGCN_OK) rc = product(fwd->z, layer == 0 ? fwd->h1 : d_out_block, AGCN_ACT_RELU, made_here);
+        }
+        if (rc != AGCN_OK) return rc;
         AGCN_CUDA(cudaEventRecord(fwd->ev[7], s));
         return AGCN_OK;
     }
     fwd->alone = false;
+    fwd->launches = 0;
     const float *h = d_x_block;
     const bool fused = fwd->fused_rows > 0;
     for (int layer = 0; layer < 2; layer++) {
@@ -586,6 +611,7 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
             rc = spmm_run_prepared(d->plan, d->idx, d->val, zg, 128, true, fwd->h1, 128, 128, s, AGCN_ACT_RELU, 0, part);
             if (rc != AGCN_OK) return rc;
             d->launches_last_step = d->plan->launches_last_run + 2;
+            fwd->launches += d->launches_last_step + 1;
             AGCN_CUDA(cudaEventRecord(d->ev_consumed[0], s));
             rc = gemm_tf32_async(fwd->h1 + fwd->fused_rows * 128, 128, fwd->w[1], fwd->z2 + fwd->fused_rows * 128, 128,
                                  d->per - fwd->fused_rows, fwd->d_status + 3, s);
@@ -600,6 +626,7 @@ extern "C" int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, flo
         rc = dist_spmm_gathered(d, 0, out, 128, AGCN_ACT_RELU, s);
         if (rc != AGCN_OK) return rc;
         AGCN_CUDA(cudaEventRecord(fwd->ev[4 * layer + 3], s));
+        fwd->launches += d->launches_last_step + (fused ? 0 : 1);
         h = out;
     }
     return AGCN_OK;
@@ -628,6 +655,13 @@ extern "C" int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6)
         float total = 0.f;
         AGCN_CUDA(cudaMemcpy(t, fwd->d_stamps, sizeof(t), cudaMemcpyDeviceToHost));
         AGCN_CUDA(cudaEventElapsedTime(&total, fwd->ev[0], fwd->ev[7]));
+        if (fwd->paired) {
+            const float transforms = (float)(t[1] - t[0]) * 1e-6f;
+            ms6[0] = ms6[3] = 0.5f * transforms;
+            ms6[1] = ms6[4] = 0.f;
+            ms6[2] = ms6[5] = 0.5f * (total - transforms);
+            return AGCN_OK;
+        }
         ms6[0] = (float)(t[1] - t[0]) * 1e-6f;
         ms6[1] = ms6[4] = 0.f;
         ms6[2] = (float)(t[2] - t[1]) * 1e-6f;
@@ -637,6 +671,14 @@ extern "C" int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6)
         for (int layer = 0; layer < 2; layer++)
             for (int k = 0; k < 3; k++)
                 AGCN_CUDA(cudaEventElapsedTime(&ms6[3 * layer + k], fwd->ev[4 * layer + k], fwd->ev[4 * layer + k + 1]));
+    return AGCN_OK;
+}
+
+extern "C" int agcn_gcn2_forward_launches(const agcn_gcn2 *fwd, int *launches)
+{
+    agcn::clear_error();
+    AGCN_REQUIRE(fwd != nullptr && launches != nullptr, "agcn_gcn2_forward_launches: null argument");
+    *launches = fwd->launches;
     return AGCN_OK;
 }
 

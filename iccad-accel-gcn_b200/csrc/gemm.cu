@@ -3,6 +3,7 @@
 // GCN layer around that SpMM.
 #include "host_common.h"
 #include "internal.h"
+#include "kernels/gemm_pair_kernels.cuh"
 #include "kernels/gemm_tf32_kernels.cuh"
 #include "kernels/fused_layer_kernels.cuh"
 
@@ -37,6 +38,26 @@ static const char *gemm_status_text(int status)
     return status == GEMM_ERR_TIMEOUT_PRODUCER ? "TMA producer" : status == GEMM_ERR_TIMEOUT_MMA ? "MMA issuer" : "epilogue";
 }
 
+// Tensor map of an operand's rows: boxes of GEMM_TILE_M rows x GEMM_KBLK floats
+static int gemm_map_rows(CUtensorMap *map, const float *d_h, int64_t ldh, int64_t m_rows)
+{
+    EncodeTiledFn encode = nullptr;
+    const int rc = get_encode_fn(&encode);
+    if (rc != AGCN_OK) return rc;
+    const cuuint64_t dims[2] = {(cuuint64_t)GEMM_DIM, (cuuint64_t)m_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)ldh * 4};
+    const cuuint32_t box[2] = {GEMM_KBLK, GEMM_TILE_M};
+    const cuuint32_t elem[2] = {1, 1};
+    const CUresult cr = encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(d_h), dims, strides, box, elem,
+                               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (cr != CUDA_SUCCESS) {
+        set_error("agcn_gemm_tf32: cuTensorMapEncodeTiled failed (%d)", (int)cr);
+        return AGCN_ERR_CUDA;
+    }
+    return AGCN_OK;
+}
+
 // Checks the arguments, encodes the tensor map of H and launches.  Nothing is allocated and the
 // stream is not synchronised; *d_status (device) receives a GEMM_ERR_* code if a pipeline wait runs
 // out.  It is zeroed on the stream, or with keep_status left as it is: then it was zero before, or
@@ -55,21 +76,9 @@ static int gemm_tf32_launch(const float *d_h, int64_t ldh, const float *d_w, flo
     if (!keep_status) AGCN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
     if (m_rows == 0) return AGCN_OK;
 
-    EncodeTiledFn encode = nullptr;
-    int rc = get_encode_fn(&encode);
-    if (rc != AGCN_OK) return rc;
     CUtensorMap map;
-    const cuuint64_t dims[2] = {(cuuint64_t)GEMM_DIM, (cuuint64_t)m_rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ldh * 4};
-    const cuuint32_t box[2] = {GEMM_KBLK, GEMM_TILE_M};
-    const cuuint32_t elem[2] = {1, 1};
-    CUresult cr = encode(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, const_cast<float *>(d_h), dims, strides, box, elem,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    if (cr != CUDA_SUCCESS) {
-        set_error("agcn_gemm_tf32: cuTensorMapEncodeTiled failed (%d)", (int)cr);
-        return AGCN_ERR_CUDA;
-    }
+    const int rc = gemm_map_rows(&map, d_h, ldh, m_rows);
+    if (rc != AGCN_OK) return rc;
 
     // per-device facts, looked up once
     static int sm_count_of[64] = {};
@@ -128,6 +137,36 @@ int gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z,
     return gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, GEMM_DIM, GEMM_DIM, d_status, s, GEMM_SPIN_LIMIT, 0, keep_status, early, d_stamp);
 }
 
+// keep_status, early, d_stamp: as for gemm_tf32_launch
+static int gemm_pair_launch(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, int *d_status, cudaStream_t s,
+                            bool keep_status, bool early, unsigned long long *d_stamp)
+{
+    AGCN_REQUIRE(d_p != nullptr && d_w1 != nullptr && d_w2 != nullptr && d_z != nullptr && d_status != nullptr, "agcn_gemm_tf32_pair: null pointer");
+    AGCN_REQUIRE(m_rows >= 0 && m_rows < ((int64_t)1 << 31) * GEMM_TILE_M / 2, "agcn_gemm_tf32_pair: row count out of range");
+    AGCN_REQUIRE(aligned16(d_p) && aligned16(d_z), "agcn_gemm_tf32_pair: P and Z must be 16-byte aligned");
+    if (!keep_status) AGCN_CUDA(cudaMemsetAsync(d_status, 0, sizeof(int), s));
+    if (m_rows == 0) return AGCN_OK;
+    CUtensorMap map;
+    const int rc = gemm_map_rows(&map, d_p, GEMM_DIM, m_rows);
+    if (rc != AGCN_OK) return rc;
+    int dev = 0, sm_count = 0;
+    AGCN_CUDA(cudaGetDevice(&dev));
+    AGCN_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
+    AGCN_CUDA(cudaFuncSetAttribute(gemm_tf32_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES));
+    const int n_tiles = (int)ceil_div(m_rows, GEMM_TILE_M);
+    const int grid = n_tiles < sm_count ? n_tiles : sm_count;
+    AGCN_CUDA(launch_early(early, gemm_tf32_pair_kernel, (unsigned)grid, PAIR_THREADS, PAIR_SMEM_BYTES, s, map, d_w1, d_w2, d_z, m_rows, n_tiles,
+                           d_status, GEMM_SPIN_LIMIT, d_stamp));
+    AGCN_LAUNCH_CHECK("gemm_tf32_pair_kernel");
+    return AGCN_OK;
+}
+
+int gemm_pair_async(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, int *d_status, cudaStream_t s,
+                    unsigned long long *d_stamp)
+{
+    return gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, s, true, true, d_stamp);
+}
+
 }  // namespace agcn
 
 extern "C" int agcn_gemm_tf32(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz,
@@ -144,6 +183,13 @@ extern "C" int agcn_gemm_tf32_async(const float *d_h, int64_t ldh, const float *
     agcn::clear_error();
     return agcn::gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, k_dim, n_dim, d_status, static_cast<cudaStream_t>(stream),
                                   agcn::GEMM_SPIN_LIMIT, 0);
+}
+
+extern "C" int agcn_gemm_tf32_pair_async(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows,
+                                         int32_t *d_status, void *stream)
+{
+    agcn::clear_error();
+    return agcn::gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, static_cast<cudaStream_t>(stream), false, false, nullptr);
 }
 
 extern "C" int agcn_gemm_tf32_selftest_timeout(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz,

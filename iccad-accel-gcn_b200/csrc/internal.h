@@ -90,6 +90,10 @@ void plan_free(agcn_spmm_plan *p);
 // end zero before the first launch (all optional)
 int gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
                     int *d_status, cudaStream_t s, bool keep_status = false, bool early = false, unsigned long long *d_stamp = nullptr);
+// Z = relu(P * W1) * W2, all of 128 columns, started while the launch before it, which makes P, still runs; *d_status is not
+// zeroed, and d_stamp is as above
+int gemm_pair_async(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, int *d_status, cudaStream_t s,
+                    unsigned long long *d_stamp);
 // Z2[r] = relu(A[r, :] * Z1) * W for the first m_rows rows of a CSR block, all of at most
 // fused_layer_max_degree() nonzeros (gemm.cu)
 int fused_layer_async(const int *d_indptr, const int *d_indices, const float *d_vals, const float *d_z_in, const float *d_w,

@@ -174,6 +174,24 @@ __device__ __forceinline__ void gemm_load_w(const float *__restrict__ w, uint8_t
     }
 }
 
+// 32 columns of 32 accumulator rows (v: a lane's row, from column 32 c) -> rows row0 .. of Z, as far as there are any
+__device__ __forceinline__ void gemm_store_patch(const float (&v)[32], float *patch, int lane, float *__restrict__ z, int64_t ldz, int64_t row0,
+                                                 int64_t m_rows, int c)
+{
+    // lane = row of the patch; write the row, then read the patch back 4 rows x 128 bytes at a time
+#pragma unroll
+    for (int j = 0; j < 8; j++)
+        *reinterpret_cast<float4 *>(patch + lane * GEMM_PATCH_STRIDE + j * 4) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int j = 0; j < 8; j++) {
+        const int r = j * 4 + (lane >> 3);
+        const float4 o = *reinterpret_cast<const float4 *>(patch + r * GEMM_PATCH_STRIDE + (lane & 7) * 4);
+        if (row0 + r < m_rows) *reinterpret_cast<float4 *>(z + (row0 + r) * ldz + c * 32 + (lane & 7) * 4) = o;
+    }
+    __syncwarp();
+}
+
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__restrict__ w,
                      float *__restrict__ z, int64_t ldz, int64_t m_rows, int n_tiles, int *__restrict__ err_flag,
@@ -301,19 +319,7 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
             for (int c = 0; c < GEMM_DIM / 32; c++) {
                 float v[32];
                 tmem_ld_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + acc * GEMM_DIM + c * 32, v);
-                // lane = row of the patch; write the row, then read the patch back 4 rows x 128 bytes at a time
-#pragma unroll
-                for (int j = 0; j < 8; j++)
-                    *reinterpret_cast<float4 *>(patch + lane * GEMM_PATCH_STRIDE + j * 4) = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
-                __syncwarp();
-#pragma unroll
-                for (int j = 0; j < 8; j++) {
-                    const int r = j * 4 + (lane >> 3);
-                    const float4 o = *reinterpret_cast<const float4 *>(patch + r * GEMM_PATCH_STRIDE + (lane & 7) * 4);
-                    if (row0 + r < m_rows)
-                        *reinterpret_cast<float4 *>(z + (row0 + r) * ldz + c * 32 + (lane & 7) * 4) = o;
-                }
-                __syncwarp();
+                gemm_store_patch(v, patch, lane, z, ldz, row0, m_rows, c);
             }
             tc_fence_before();
             __syncwarp();

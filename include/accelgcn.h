@@ -242,6 +242,12 @@ int agcn_gemm_tf32(const float *d_h, int64_t ldh, const float *d_w, float *d_z, 
 int agcn_gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz,
                          int64_t m_rows, int k_dim, int n_dim, int32_t *d_status, void *stream);
 
+/* Two of them with the activation between, Z = relu(P * W1) * W2, in one kernel: relu(P * W1) never leaves the SM.  P and Z
+ * are [m_rows x 128], contiguous, 16-byte aligned and do not overlap; both weights are 128 x 128.  Asynchronous, *d_status
+ * as in agcn_gemm_tf32_async. */
+int agcn_gemm_tf32_pair_async(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows,
+                              int32_t *d_status, void *stream);
+
 /* Self-test of the kernel's failure path (no other use): runs the product with a spin limit of
  * well under a millisecond and with the first load of every thread block left out, so that one
  * pipeline wait must run out.  The kernel leaves through its abort path (tensor memory freed,
@@ -411,12 +417,16 @@ int agcn_dist_gathered(const agcn_dist *dist, int slot, const float **d_gathered
  * stream, agcn_gcn2_forward_status reports a dense transform whose bounded wait
  * ran out (AGCN_ERR_CUDA; on one GPU in any run since the last call) and, if ms6 is not NULL, six times in milliseconds:
  * per layer the transform, the wait for the exchange's first slice, the SpMM.
+ * Where nothing is exchanged, from 32 768 rows on, A is applied to X before W1 (A (X W1) =
+ * (A X) W1) and both transforms are one kernel (agcn_gemm_tf32_pair_async): its time is then given by halves to
+ * the two layers, and so is that of the two products.  agcn_gcn2_forward_launches: kernels the last run launched.
  * ---------------------------------------------------------------------- */
 typedef struct agcn_gcn2 agcn_gcn2;
 
 int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const float *d_w1, const float *d_w2);
 int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, float *d_out_block, void *stream);
 int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6);
+int agcn_gcn2_forward_launches(const agcn_gcn2 *fwd, int *launches);
 int agcn_gcn2_forward_destroy(agcn_gcn2 *fwd);
 
 /* ------------------------------------------------------------------------

@@ -31,6 +31,31 @@ def test_gemm_tf32_matches_fp64(m):
     _check_gemm(h.cpu().numpy(), w.cpu().numpy(), z.cpu().numpy())
 
 
+@pytest.mark.parametrize("m", [1, 127, 128, 129, 128 * 148 + 5, 128 * 148 * 2, 128 * 148 * 5 + 77])
+def test_pair_of_transforms_matches_fp64(m):
+    # relu(P W1) W2 in one kernel, thread blocks with one to six tiles: their two accumulators of either product take turns.
+    # P, W1 and W2 are cut to TF32 (2^-10 each), the activations rounded (2^-11); relu does not stretch an error
+    import torch
+    from accelgcn import gemm, synth
+    dev = require_cuda()
+    p = synth.features(m, 128, 17 + m, dev)
+    w1, w2 = synth.glorot(128, 128, 5, 8, dev), synth.glorot(128, 128, 5, 9, dev)
+    z = torch.full((m + 2, 128), float("nan"), device=dev)
+    status = torch.full((1,), 9, dtype=torch.int32, device=dev)
+    gemm.gemm_tf32_pair_async(p, w1, w2, z[:m], status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0 and bool(torch.isnan(z[m:]).all())
+    p64, w1_64, w2_64 = p.double(), w1.double(), w2.double()
+    h = (p64 @ w1_64).clamp_(min=0)
+    bound = 2e-3 * (p64.abs() @ w1_64.abs()) @ w2_64.abs() + 1.5e-3 * h @ w2_64.abs() + 1e-6
+    assert bool(((z[:m].double() - h @ w2_64).abs() <= bound).all())
+    # values that TF32 holds, through the identity twice: exact
+    p = torch.randint(-512, 512, (m, 128), device=dev).float() / 64.0
+    eye = torch.eye(128, device=dev)
+    gemm.gemm_tf32_pair_async(p, eye, eye, z[:m], status)
+    assert torch.equal(z[:m], p.clamp(min=0)) and int(status.item()) == 0
+
+
 def test_gemm_identity_and_strided_rows():
     import torch
     from accelgcn import gemm, synth
