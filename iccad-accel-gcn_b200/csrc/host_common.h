@@ -72,6 +72,7 @@ private:
 };
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+inline bool aligned32(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 31u) == 0; }
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
 // Stream-ordered memory of the current device's pool (memory.cu).  Refused (cudaErrorStreamCaptureUnsupported) while

@@ -45,6 +45,12 @@ __device__ __forceinline__ float4 ld_x4(const float *p, uint64_t policy)
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p), "l"(policy));
     return v;
 }
+// the same, 32 bytes per lane
+__device__ __forceinline__ void ld_x8(const float *p, uint64_t policy, float4 &a, float4 &b)
+{
+    asm("ld.global.L2::cache_hint.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8], %9;"
+        : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w) : "l"(p), "l"(policy));
+}
 __device__ __forceinline__ float ld_x1(const float *p, uint64_t policy)
 {
     float v;
@@ -85,6 +91,11 @@ __device__ __forceinline__ void st_y4(float *p, const float4 &v, uint64_t policy
 {
     asm volatile("st.global.L2::cache_hint.v4.f32 [%0], {%1, %2, %3, %4}, %5;"
                  :: "l"(p), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w), "l"(policy) : "memory");
+}
+__device__ __forceinline__ void st_y8(float *p, const float4 &a, const float4 &b, uint64_t policy)
+{
+    asm volatile("st.global.L2::cache_hint.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8}, %9;"
+                 :: "l"(p), "f"(a.x), "f"(a.y), "f"(a.z), "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w), "l"(policy) : "memory");
 }
 __device__ __forceinline__ void st_y2(float *p, float a, float b, uint64_t policy)
 {

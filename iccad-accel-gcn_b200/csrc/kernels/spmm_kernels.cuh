@@ -50,6 +50,8 @@ constexpr int SPMM_ZERO_ROWS_PER_BLOCK = 64;
 // 1447, dim 128 2983 -> 2875; 700 000 rows of 15, dim 64: 235 -> 221.  More gathers at fewer blocks lose 5-30 %.)
 constexpr int SPMM_GATHER_BATCH = 7, SPMM_MIN_BLOCKS = 4;
 constexpr int SPMM_WIDE_GATHER_BATCH = 4, SPMM_WIDE_MIN_BLOCKS = 5;
+// With 32-byte loads: large launches, others, others with five blocks per SM (three, six gathers: 1-9 %, 14 % slower)
+constexpr int SPMM_OCTET_BATCH = 4, SPMM_OCTET_FEW = 3;
 // Small products (no more tuples than the GPU has room for warps) cannot hide latency with occupancy, and what they
 // wait for is the warp that walks 384 nonzeros alone.  Their plan cuts the tuples into pieces of fewer nonzeros
 // (plan_small_kernel), and where they fit two blocks per SM the kernel keeps more gathers in flight per lane
@@ -250,6 +252,111 @@ __device__ __forceinline__ void gather_rows4(const SpmmParams &p, const int2 *pa
     }
 }
 
+// The same with 8 columns per lane, 32 bytes per load.  (Functions of their own: written as one for either width they
+// cost the 16-byte forms registers, and small products 1-5 %.)
+struct Octet {
+    float4 a, b;
+};
+__device__ __forceinline__ Octet zero_octet() { return {make_float4(0.f, 0.f, 0.f, 0.f), make_float4(0.f, 0.f, 0.f, 0.f)}; }
+__device__ __forceinline__ void fma8(Octet &acc, float a, const Octet &v) { fma4(acc.a, a, v.a); fma4(acc.b, a, v.b); }
+template <bool HOT>
+__device__ __forceinline__ Octet ld_octet(const float *p, const L2Policies &pol, int column)
+{
+    Octet v;
+    ld_x8(p, x_policy<HOT>(pol, column), v.a, v.b);
+    return v;
+}
+template <bool PLAIN>
+__device__ __forceinline__ void emit_row8(const SpmmParams &p, float *yr, int col, const Octet &v, uint64_t policy)
+{
+    if (PLAIN) st_y8(yr + col, relu4(v.a, p.relu), relu4(v.b, p.relu), policy);
+    else { emit_row4<false>(p, yr, col, v.a, p.relu, policy); emit_row4<false>(p, yr, col + 4, v.b, p.relu, policy); }
+}
+
+template <int UNROLL, bool HOT>
+__device__ __forceinline__ Octet gather_vec8(const int2 *pairs, int count, int first, int step, const float *__restrict__ x, int64_t ldx, bool active,
+                                             const L2Policies &pol)
+{
+    Octet acc = zero_octet();
+    if (!active) return acc;
+    int i = first;
+    for (; i + (UNROLL - 1) * step < count; i += UNROLL * step) {
+        int2 p[UNROLL];
+        Octet v[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) p[u] = pairs[i + u * step];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_octet<HOT>(x + (int64_t)p[u].x * ldx, pol, p[u].x);
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) fma8(acc, __int_as_float(p[u].y), v[u]);
+    }
+    if (i < count) {
+        int2 p[UNROLL - 1];
+        Octet v[UNROLL - 1];
+#pragma unroll
+        for (int u = 0; u < UNROLL - 1; u++) {
+            const bool live = i + u * step < count;
+            p[u] = live ? pairs[i + u * step] : make_int2(0, 0);
+            v[u] = live ? ld_octet<HOT>(x + (int64_t)p[u].x * ldx, pol, p[u].x) : zero_octet();
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL - 1; u++)
+            if (i + u * step < count) fma8(acc, __int_as_float(p[u].y), v[u]);
+    }
+    return acc;
+}
+
+template <int UNROLL, bool PLAIN, bool HOT>
+__device__ __forceinline__ void gather_rows8(const SpmmParams &p, const int2 *pairs, int rows, int row_nz, const float *__restrict__ x, float *yr, int col,
+                                             const L2Policies &pol)
+{
+    const int count = rows * row_nz;
+    Octet acc = zero_octet();
+    int left = row_nz;
+    auto take = [&](float a, const Octet &v) {
+        fma8(acc, a, v);
+        if (--left == 0) {
+            emit_row8<PLAIN>(p, yr, col, acc, pol.stream);
+            acc = zero_octet();
+            left = row_nz;
+            yr += p.ldy;
+        }
+    };
+    int i = 0;
+    for (; i + UNROLL <= count; i += UNROLL) {
+        int2 q[UNROLL];
+        Octet v[UNROLL];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) q[u] = pairs[i + u];
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) v[u] = ld_octet<HOT>(x + (int64_t)q[u].x * p.ldx, pol, q[u].x);
+#pragma unroll
+        for (int u = 0; u < UNROLL; u++) take(__int_as_float(q[u].y), v[u]);
+    }
+    if (i < count) {
+        int2 q[UNROLL - 1];
+        Octet v[UNROLL - 1];
+#pragma unroll
+        for (int u = 0; u < UNROLL - 1; u++) {
+            const bool live = i + u < count;
+            q[u] = live ? pairs[i + u] : make_int2(0, 0);
+            v[u] = live ? ld_octet<HOT>(x + (int64_t)q[u].x * p.ldx, pol, q[u].x) : zero_octet();
+        }
+#pragma unroll
+        for (int u = 0; u < UNROLL - 1; u++)
+            if (i + u < count) take(__int_as_float(q[u].y), v[u]);
+    }
+}
+
+__device__ __forceinline__ float4 fold4(float4 v, int off)
+{
+    v.x += __shfl_xor_sync(FULL_MASK, v.x, off);
+    v.y += __shfl_xor_sync(FULL_MASK, v.y, off);
+    v.z += __shfl_xor_sync(FULL_MASK, v.z, off);
+    v.w += __shfl_xor_sync(FULL_MASK, v.w, off);
+    return v;
+}
+
 constexpr int SPMM_SCALAR_COLS = SPMM_PANEL / 32;   // columns per lane in scalar mode
 
 // Scalar mode: lane l owns columns l, l+32, ... (K = ceil(dim / 32) of them), every load instruction
@@ -351,6 +458,8 @@ __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 spa
 // main kernel.  S = lanes per slot in float4 mode (4, 8, 16 or 32; needs
 // dim % 4 == 0, dim <= 4*S and 16-byte aligned rows); S = 0 is the scalar
 // mode for every other dim (lane l owns columns l, l+32, l+64, l+96).
+// Q = columns per lane / 4: with 2, a lane has 8 columns (S = 8 or 16 for up to 64 or 128 of them), loaded 32 bytes at a time:
+// rows of X on 32-byte boundaries, dim % 8 == 0; for what products, see spmm_octets.
 // FINISH: rows that cross units are finished here (in launches of few units);
 // a template parameter because the code costs registers the large launches
 // do not have (two more spills, 3 % of a product of 500 000 rows).
@@ -358,7 +467,7 @@ __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 spa
 // ANY_ROWS: as float4 mode, with the same additions in the same order, but rows of X and Y of any alignment: lane l of a
 // slot has columns l, l + S, l + 2 S, l + 3 S (consecutive ones cost four times the wavefronts).
 // ---------------------------------------------------------------------------
-template <int S, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT, bool ANY_ROWS>
+template <int S, int Q, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT, bool ANY_ROWS>
 __global__ void __launch_bounds__(SPMM_THREADS, MIN_BLOCKS)
 spmm_units_kernel(const SpmmParams p)
 {
@@ -373,7 +482,7 @@ spmm_units_kernel(const SpmmParams p)
     const int w = warp_id(), lane = lane_id();
     const int slot = lane / LANES, sl = lane % LANES;
     constexpr int LOOSE = ANY_ROWS ? S : 0;
-    const int col = VEC ? sl * 4 : sl;              // place of the lane's sums among the partials
+    const int col = VEC ? sl * 4 * Q : sl;              // place of the lane's sums among the partials
     const int ycol = ANY_ROWS ? sl : col;           // and of the first of them in a row of X and Y
     const bool active = ycol < (ANY_ROWS ? p.dim_store : p.dim);
     L2Policies pol = make_l2_policies();
@@ -391,7 +500,9 @@ spmm_units_kernel(const SpmmParams p)
             if (zb + k >= p.n_zero_rows) break;
             float *yr = p.y + (int64_t)p.zero_rows[zb + k] * p.ldy;
             if (VEC) {
-                if (active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, make_float4(0.f, 0.f, 0.f, 0.f), p.relu, pol.stream);
+                if constexpr (Q == 2) {
+                    if (active) emit_row8<PLAIN>(p, yr, ycol, zero_octet(), pol.stream);
+                } else if (active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, make_float4(0.f, 0.f, 0.f, 0.f), p.relu, pol.stream);
             } else {
                 for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, 0.f, p.relu, pol.stream);
             }
@@ -423,7 +534,27 @@ spmm_units_kernel(const SpmmParams p)
     const int2 *pairs = s_pair[w];
     wait_for_predecessor();             // X may be what the launch before this one makes
 
-    if (VEC) {
+    if constexpr (Q == 2) {
+        const float *xc = p.x + ycol;
+        if (t.small && t.row_nz <= 32) {
+            const int each = (t.n_rows + NS - 1) / NS, r0 = slot * each;
+            const int rows = r0 < t.n_rows ? (r0 + each < t.n_rows ? each : t.n_rows - r0) : 0;
+            if (active) gather_rows8<BATCH, PLAIN, HOT>(p, pairs + r0 * t.row_nz, rows, t.row_nz, xc, p.y + (int64_t)(t.row0 + r0) * p.ldy, ycol, pol);
+        } else {
+            for (int r = 0; r < t.n_rows; r++) {
+                Octet acc = gather_vec8<BATCH, HOT>(pairs + r * t.row_nz, t.row_nz, slot, NS, xc, p.ldx, active, pol);
+#pragma unroll
+                for (int off = LANES; off < 32; off <<= 1) { acc.a = fold4(acc.a, off); acc.b = fold4(acc.b, off); }
+                if (slot == 0 && active) {
+                    if (t.small) emit_row8<PLAIN>(p, p.y + (int64_t)(t.row0 + r) * p.ldy, ycol, acc, pol.stream);
+                    else {
+                        *reinterpret_cast<float4 *>(&s_part[w][col]) = acc.a;
+                        *reinterpret_cast<float4 *>(&s_part[w][col + 4]) = acc.b;
+                    }
+                }
+            }
+        }
+    } else if (VEC) {
         const float *xc = p.x + ycol;
         if (t.small && t.row_nz <= 32) {
             // whole rows for every slot, consecutive ones
@@ -479,7 +610,9 @@ spmm_units_kernel(const SpmmParams p)
     float *yr = p.y + (int64_t)t.row0 * p.ldy;
     if (!partial) {
         if (VEC) {
-            if (slot == 0 && active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, sum_parts4(s_part, w, w_end, col), p.relu, pol.stream);
+            if constexpr (Q == 2) {
+                if (slot == 0 && active) emit_row8<PLAIN>(p, yr, ycol, {sum_parts4(s_part, w, w_end, col), sum_parts4(s_part, w, w_end, col + 4)}, pol.stream);
+            } else if (slot == 0 && active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, sum_parts4(s_part, w, w_end, col), p.relu, pol.stream);
         } else {
             for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, sum_parts1(s_part, w, w_end, c), p.relu, pol.stream);
         }
@@ -489,6 +622,8 @@ spmm_units_kernel(const SpmmParams p)
     float *mine = p.carry + (int64_t)my_slot * SPMM_PANEL;
     if (VEC) {
         if (slot == 0 && active) *reinterpret_cast<float4 *>(mine + col) = sum_parts4(s_part, w, w_end, col);
+        if constexpr (Q == 2)
+            if (slot == 0 && active) *reinterpret_cast<float4 *>(mine + col + 4) = sum_parts4(s_part, w, w_end, col + 4);
     } else {
         for (int c = lane; c < p.dim; c += 32) mine[c] = sum_parts1(s_part, w, w_end, c);
     }
@@ -504,6 +639,7 @@ spmm_units_kernel(const SpmmParams p)
     if (lane == 0) p.carry_count[span.x] = 0;       // ready for the next product
     __threadfence();
     finish_carried_row<VEC, PLAIN, LOOSE>(p, span, t.row0, VEC ? (slot == 0 && active ? col : SPMM_PANEL) : lane, pol.stream);
+    if constexpr (Q == 2) finish_carried_row<VEC, PLAIN, LOOSE>(p, span, t.row0, slot == 0 && active ? col + 4 : SPMM_PANEL, pol.stream);
 }
 
 // Adds the carried partials of every row that crosses unit boundaries.  One warp per carry slot; the warp of

@@ -106,6 +106,29 @@ static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
 // (Passes of up to 32 columns were not measured and have no such kernel.)
 constexpr double SPMM_HOT_X = 6.0, SPMM_HOT_L2 = 0.45, SPMM_HOT_SHARE = 0.33;
 
+// Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM), where a second
+// launch costs more than blocks that wait for a counter.
+static bool spmm_many_units(const agcn_spmm_plan *p) { return !p->split && p->n_units > (int64_t)20 * p->sm_count; }
+
+// Whether a pass of `width` columns (a multiple of 8) loads rows of X 32 bytes per lane: half the load instructions, two rows
+// with each where they have 65 to 128 columns, and more bytes in flight.  It gains where the 16-byte lanes of a slot are not
+// all used or, beyond 64 columns, where the gather comes from L2; rows of 64 and 128 columns otherwise keep HBM or the ports
+// of L2 as busy 16 bytes at a time.  It never gains up to 32 columns (4-25 % slower).  (A rule on plan and width alone: the
+// additions inside a row of more than 32 nonzeros come in another order, and a product issued in parts has the whole one's bits.)
+// Time with / without, B200.  More than 20 units per SM, 250 000 dense rows of 490, 500 000 skewed of 30, 500 000 power law of
+// 12, 2.4 M of 25, 1 M of 8: dim 40: .96 .95 .97 .98 .96;  48: .97 .97 .97 .98 .97;  56: .98 1.02 .99 - .99;  64: 1.00 1.01 .96
+// 1.00 .98;  72: .88 .94 .93 .95 .94;  80: .85 .96 .93 - .94;  88: .91 1.00 - - -;  96: .92 1.02 1.01 .94 1.02;  112: .95 1.00
+// .97 - .98;  128: .98 1.02 1.00 1.02 .98.
+// Fewer, 60 000 dense of 150, 150 000 power law of 10, 200 000 of 20, 100 000 skewed of 20 (in the form of five blocks): 40:
+// .98 .99 1.02 .97;  64: 1.00 .99 1.00 1.05;  72: .96 .96 .96 .93;  80: .96 .97 - .95;  96: .97 .97 - .98;  112: .99 .98 - 1.05;
+// 128: .99 .97 .99 1.04.
+static bool spmm_octets(const agcn_spmm_plan *p, int width)
+{
+    if (p->split || p->panel_override != 0 || width <= 32) return false;
+    if (spmm_many_units(p)) return width <= 48 || (width > 64 && (width <= 88 || p->nnz >= 250 * p->n_blocks));
+    return width > 64 && (width <= 96 || !spmm_wide_form(p, width));
+}
+
 static int64_t hot_rows(const agcn_spmm_plan *p, int width) { return (int64_t)(SPMM_HOT_L2 * p->l2_bytes / (width * 4.0)); }
 
 int64_t spmm_hot_column(const agcn_spmm_plan *p, int width)
@@ -290,10 +313,10 @@ int spmm_check_cols(const int *d_idx, int64_t count, int64_t n_cols, int *d_flag
     return AGCN_OK;
 }
 
-template <int S, int BATCH, int MIN_BLOCKS, bool FINISH, bool HOT = false>
+template <int S, int BATCH, int MIN_BLOCKS, bool FINISH, bool HOT = false, int Q = 1>
 static void launch_units(const SpmmParams &prm, unsigned grid, bool plain, cudaStream_t s)
 {
-    auto k = plain ? spmm_units_kernel<S, BATCH, MIN_BLOCKS, true, FINISH, HOT, false> : spmm_units_kernel<S, BATCH, MIN_BLOCKS, false, FINISH, HOT, false>;
+    auto k = plain ? spmm_units_kernel<S, Q, BATCH, MIN_BLOCKS, true, FINISH, HOT, false> : spmm_units_kernel<S, Q, BATCH, MIN_BLOCKS, false, FINISH, HOT, false>;
     launch_early(prm.early != 0, k, grid, SPMM_THREADS, 0, s, prm);
 }
 
@@ -304,15 +327,31 @@ struct SpmmForm {
     bool deep;       // few thread blocks, many gathers per lane
     bool wide;       // more thread blocks per SM, fewer gathers per lane
     bool loose;      // rows of X of any alignment, 4 bytes at a time (cut plans: spmm_loose)
+    bool octets;     // 32-byte loads (spmm_octets), of a plan of many units or not
+    bool many;
 };
+
+// S = lanes of 8 columns
+template <int S>
+static void launch_octets(const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
+{
+    if (f.many) {
+        if (f.finish) launch_units<S, SPMM_OCTET_BATCH, SPMM_MIN_BLOCKS, true, false, 2>(prm, grid, f.plain, s);
+        else if (prm.hot_column > 0) launch_units<S, SPMM_OCTET_BATCH, SPMM_MIN_BLOCKS, false, true, 2>(prm, grid, f.plain, s);
+        else launch_units<S, SPMM_OCTET_BATCH, SPMM_MIN_BLOCKS, false, false, 2>(prm, grid, f.plain, s);
+    } else if constexpr (S == 16) {                      // (spmm_octets: none of up to 64 columns)
+        if (f.wide) launch_units<S, SPMM_OCTET_FEW, SPMM_WIDE_MIN_BLOCKS, true, false, 2>(prm, grid, f.plain, s);
+        else launch_units<S, SPMM_OCTET_FEW, SPMM_MIN_BLOCKS, true, false, 2>(prm, grid, f.plain, s);
+    }
+}
 
 template <int S>
 static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
 {
     if constexpr (S > 0) {
         if (f.loose) {
-            auto k = f.deep ? spmm_units_kernel<S, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, false, true, false, true>
-                            : spmm_units_kernel<S, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true, false, true>;
+            auto k = f.deep ? spmm_units_kernel<S, 1, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, false, true, false, true>
+                            : spmm_units_kernel<S, 1, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true, false, true>;
             launch_early(prm.early != 0, k, grid, SPMM_THREADS, 0, s, prm);
             return;
         }
@@ -341,7 +380,8 @@ static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmFor
 
 static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
 {
-    if (!vec) launch_units_for<0>(prm, grid, f, s);
+    if (f.octets) width <= 64 ? launch_octets<8>(prm, grid, f, s) : launch_octets<16>(prm, grid, f, s);
+    else if (!vec) launch_units_for<0>(prm, grid, f, s);
     else if (width <= 16) launch_units_for<4>(prm, grid, f, s);
     else if (width <= 32) launch_units_for<8>(prm, grid, f, s);
     else if (width <= 64) launch_units_for<16>(prm, grid, f, s);
@@ -471,9 +511,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         if (x_bytes > 0.75 * (double)p->l2_bytes && x_bytes <= 4.0 * (double)p->l2_bytes) panel = 64;
     }
     if (p->panel_override > 0) panel = p->panel_override;
-    // Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM),
-    // where a second launch costs more than blocks that wait for a counter; parts of a product always do that.
-    const bool carry_inside = !whole || p->split || p->n_units <= (int64_t)20 * p->sm_count;
+    const bool carry_inside = !whole || !spmm_many_units(p);        // parts of a product always finish their rows
     // A carry slot holds SPMM_PANEL floats and every column pass uses its own columns (and arrival
     // counters) of it, so a product of up to SPMM_PANEL columns can be issued in parts whatever its
     // passes are -- with the same passes, hence the same bits, as a whole run.
@@ -510,9 +548,10 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.y_vec = y_vec ? 1 : 0;
         prm.dim_store = width;
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
-        const bool plain = !accumulate && !loose && (vec ? y_vec : true);
+        const bool octets = vec && !loose && prm.dim % 8 == 0 && ldx_use % 8 == 0 && aligned32(prm.x) && spmm_octets(p, prm.dim);
+        const bool plain = !accumulate && !loose && (vec ? y_vec : true) && (!octets || (width % 8 == 0 && ldy % 8 == 0 && aligned32(prm.y)));
         if (grid > 0) {
-            const SpmmForm form = {plain, carry_inside, spmm_deep(p), spmm_wide_form(p, width), loose};
+            const SpmmForm form = {plain, carry_inside, spmm_deep(p), spmm_wide_form(p, width), loose, octets, spmm_many_units(p)};
             launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, form, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;

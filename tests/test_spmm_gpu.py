@@ -748,6 +748,54 @@ def test_small_products_from_rows_of_any_alignment(kind, dim):
     plan.close()
 
 
+@pytest.fixture(scope="module", params=["many", "dense", "few"])
+def uncut(request):
+    # graphs whose tuples are not cut: more than 20 thread blocks per SM of light rows, of full tuples, and fewer
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    rng = np.random.default_rng(5)
+    deg = {"many": lambda: np.concatenate([rng.integers(0, 4, 290_000), rng.integers(33, 90, 500), [400, 3_000, 20_000]]),
+           "dense": lambda: np.concatenate([rng.integers(380, 385, 23_800), [500, 5_000]]),
+           "few": lambda: np.concatenate([rng.integers(0, 5, 150_000), rng.integers(33, 200, 300), [385, 900, 7_000]])}[request.param]()
+    deg = np.sort(deg)
+    n, cols = len(deg), 30_000
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    idx = rng.integers(0, cols, int(indptr[-1]), dtype=np.int32)
+    val = rng.standard_normal(len(idx)).astype(np.float32)
+    d_idx, d_val = torch.from_numpy(idx).to(dev), torch.from_numpy(val).to(dev)
+    plan = spmm.SpmmPlan(partition.block_level_partition_device(torch.from_numpy(indptr).to(dev)), d_idx, n, cols)
+    yield dict(dev=dev, n=n, cols=cols, indptr=indptr, idx=idx, val=val, d_idx=d_idx, d_val=d_val, plan=plan)
+    plan.close()
+
+
+@pytest.mark.parametrize("dim", [33, 40, 48, 49, 56, 65, 68, 72, 81, 88, 89, 96, 104, 127, 128, 136])
+def test_rows_of_x_32_bytes_at_a_time(uncut, dim):
+    # uncut plans load whole eights of columns where rows of X allow it: all layouts of X and Y that do and do not, widths on
+    # both sides of the rule's lines, the copy of an unaligned X in rows of eights, rows that cross thread blocks, rows without
+    # nonzeros; an infinity and a NaN stay in their column
+    import torch
+    g = uncut
+    n, cols, eights = g["n"], g["cols"], (dim + 7) // 8 * 8
+    xs = np.random.default_rng(dim).standard_normal((cols, dim)).astype(np.float32)
+    ref = oracle.spmm_csr(g["indptr"], g["idx"], g["val"], xs)
+    scale = row_abs_scale(g["indptr"], g["val"], xs)
+    touched = np.unique(np.repeat(np.arange(n), np.diff(g["indptr"]))[(g["idx"] == 7) | (g["idx"] == 9)])
+    for shift, ldx, ldy, relu in ((0, dim, dim, False), (8, eights, eights, True), (4, eights, eights + 4, False), (0, eights + 4, eights, True), (1, dim, dim + 1, False)):
+        x = torch.full((cols * ldx + shift,), float("nan"), device=g["dev"])[shift:]
+        y = torch.full((n * ldy + shift,), 7.0, device=g["dev"])[shift:]
+        x.view(cols, ldx)[:, :dim] = torch.from_numpy(xs).to(g["dev"])
+        g["plan"].run(g["d_idx"], g["d_val"], x, y, dim=dim, ldx=ldx, ldy=ldy, relu=relu)
+        got = y.view(n, ldy).cpu().numpy()
+        assert spmm_close(got[:, :dim], np.maximum(ref, 0) if relu else ref, scale).all(), (shift, ldx, ldy)
+        assert (got[:, dim:] == 7.0).all()
+        x.view(cols, ldx)[7, dim - 1], x.view(cols, ldx)[9, 0] = float("inf"), float("nan")
+        g["plan"].run(g["d_idx"], g["d_val"], x, y, dim=dim, ldx=ldx, ldy=ldy)
+        odd = ~torch.isfinite(y.view(n, ldy)).cpu().numpy()
+        assert not odd[:, 1:dim - 1].any() and not odd[:, dim:].any()
+        assert np.array_equal(np.flatnonzero(odd.any(axis=1)), touched)
+
+
 @pytest.mark.parametrize("shift", [0, 1, 2, 3])
 @pytest.mark.parametrize("nnz", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 4_099, 6_000_001])
 def test_a_column_id_outside_is_found_wherever_it_is(nnz, shift):
