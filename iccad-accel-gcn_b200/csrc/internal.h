@@ -15,6 +15,7 @@ struct agcn_spmm_plan {
     void *carry = nullptr;            // spmm_carry_bytes(n_carry): partial sums and arrival counters
     int *zero_rows = nullptr;         // [n_zero]
     int64_t n_carry = 0, n_zero = 0;
+    int64_t longest = 0;              // degree of the last tuple (cut plans)
     int64_t n_full = 0;               // tuples of at least 192 nonzeros (uncut plans)
     int launches_last_run = 0;
     int l2_bytes = 0, sm_count = 0;   // of the device the plan was created on

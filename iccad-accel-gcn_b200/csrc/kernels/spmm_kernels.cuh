@@ -57,6 +57,8 @@ constexpr int SPMM_OCTET_BATCH = 4, SPMM_OCTET_FEW = 3;
 // (plan_small_kernel), and where they fit two blocks per SM the kernel keeps more gathers in flight per lane
 // (16 384 rows of 8, dim 60: 9.0 -> 8.6 us).
 constexpr int SPMM_DEEP_GATHER_BATCH = 16, SPMM_DEEP_MIN_BLOCKS = 2;
+// Between those and the others: three blocks per SM (spmm_few_form).
+constexpr int SPMM_THREE_GATHER_BATCH = 8, SPMM_THREE_MIN_BLOCKS = 3;
 
 struct SpmmParams {
     const int4 *tuples;       // the plan's: `.block4`, or its pieces
@@ -711,6 +713,7 @@ __device__ __forceinline__ int tuple_rows(const int4 &b) { return tuple_is_big(b
 // Error bits are single words of the host so that blocks can store to them without atomics.
 constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_FULL = 3;
 constexpr int PLAN_WORD_TAIL = PLAN_WORD_PIECES;            // uncut plans, which have no pieces
+constexpr int PLAN_WORD_LONGEST = PLAN_WORD_FULL;           // cut plans, which do not count full tuples
 constexpr int PLAN_WORD_ERR = 4;      // then one word per SPMM_ERR_* bit
 constexpr int PLAN_ERR_BITS = 4;
 constexpr int PLAN_FULL_NZ = 192;
@@ -1075,7 +1078,7 @@ plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows,
         }
     }
     int zero_out = block_scan_exclusive<PLAN_SMALL_BLOCK>((int)zero, OpAdd(), 0, n_zero, s_scan);
-    if (threadIdx.x == 0) { out->w[PLAN_WORD_ZERO] = n_zero; out->w[PLAN_WORD_PIECES] = n_pieces; }
+    if (threadIdx.x == 0) { out->w[PLAN_WORD_ZERO] = n_zero; out->w[PLAN_WORD_PIECES] = n_pieces; out->w[PLAN_WORD_LONGEST] = longest; }
     if (n_pieces > cap_pieces) return;              // cannot be: valid tuples do not overlap
     a = before;
     for (int e = e0; e < e1; e++) {

@@ -748,6 +748,36 @@ def test_small_products_from_rows_of_any_alignment(kind, dim):
     plan.close()
 
 
+@pytest.mark.parametrize("hub", [0, 3_000])
+@pytest.mark.parametrize("units", [394, 395, 444, 445, 592, 593, 932, 933])
+def test_products_of_few_thread_blocks(units, hub, monkeypatch):
+    # both sides of the lines between the forms of launches of few thread blocks, on graphs with and without a hub row; every slot width
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    if torch.cuda.get_device_properties(dev).multi_processor_count != 148:
+        pytest.skip("sizes are those of 148 SMs")
+    monkeypatch.setenv("AGCN_SPMM_PIECE", "64")
+    rng = np.random.default_rng(units)
+    # tuples of 12 rows of 16: three pieces; a unit is eight pieces, the hub row 47 of them
+    pieces = units * 8 - (-(-hub // 64) if hub else 0)
+    deg = np.full(pieces // 3 * 12 + pieces % 3 * 4, 16)
+    deg = np.append(deg, hub) if hub else deg
+    indptr = np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)
+    n, cols = len(deg), 4_000
+    idx = rng.integers(0, cols, int(indptr[-1]), dtype=np.int32)
+    val = rng.standard_normal(len(idx)).astype(np.float32)
+    d_idx, d_val = torch.from_numpy(idx).to(dev), torch.from_numpy(val).to(dev)
+    plan = spmm.SpmmPlan(partition.block_level_partition_device(torch.from_numpy(indptr).to(dev)), d_idx, n, cols)
+    assert plan.info()["n_units"] == units
+    for dim in (16, 20, 32, 64, 100, 128):
+        x = rng.standard_normal((cols, dim)).astype(np.float32)
+        y = torch.full((n, dim), float("nan"), device=dev)
+        plan.run(d_idx, d_val, torch.from_numpy(x).to(dev), y)
+        assert spmm_close(y.cpu().numpy(), oracle.spmm_csr(indptr, idx, val, x), row_abs_scale(indptr, val, x)).all(), dim
+    plan.close()
+
+
 @pytest.fixture(scope="module", params=["many", "dense", "few"])
 def uncut(request):
     # graphs whose tuples are not cut: more than 20 thread blocks per SM of light rows, of full tuples, and fewer
