@@ -129,11 +129,13 @@ def spmm(block4, indices, vals, x, n_rows: int | None = None, out=None):
     import torch
     n_rows = int(x.shape[0] if n_rows is None else n_rows)
     y = out if out is not None else torch.empty((n_rows, x.shape[1]), dtype=torch.float32, device=x.device)
-    plan = SpmmPlan(block4, indices, n_rows, x.shape[0])
-    try:
-        plan.run(indices, vals, x, y)
-    finally:
-        plan.close()         # waits for the device
+    if not (block4.is_cuda and block4.dtype == torch.int32 and block4.is_contiguous()):
+        raise TypeError("block4 must be a contiguous int32 CUDA tensor")
+    dim, index = x.shape[1], _lib.device_index(block4.device)
+    with _lib.on_device(index):
+        _lib.check(_lib.call()(_lib.address("agcn_spmm_once"), block4.data_ptr(), block4.numel() // 4, indices.data_ptr(), vals.data_ptr(), n_rows,
+                               x.shape[0], indices.numel(), x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0) if y.dim() == 2 else dim, dim,
+                               _lib.raw_stream(index)))
     return y
 
 

@@ -15,6 +15,7 @@ struct agcn_spmm_plan {
     void *carry = nullptr;            // spmm_carry_bytes(n_carry): partial sums and arrival counters
     int *zero_rows = nullptr;         // [n_zero]
     int64_t n_carry = 0, n_zero = 0;
+    int64_t likely_units = 0;         // about how many units there are, where n_units is only a bound
     int64_t longest = 0;              // degree of the last tuple (cut plans)
     int64_t n_full = 0;               // tuples of at least 192 nonzeros (uncut plans)
     int launches_last_run = 0;
@@ -72,6 +73,7 @@ struct SpmmLaunchPart {
     // Start while the launch before this one on the stream still runs: ONLY_X: that one makes X and nothing else that
     // is read here, and was itself launched behind all it follows; ANY: it may be any operation.
     enum Early { NO, ONLY_X, ANY } early = NO;
+    const int *made = nullptr;          // with abort_flag: of a plan whose kernel was launched before, its numbers (SpmmParams::made)
     const int *abort_flag = nullptr;    // optional device word: nonzero makes the kernels return at once
     void *carry = nullptr;              // optional carry scratch to use instead of the plan's (products in flight together)
 };

@@ -34,6 +34,8 @@
 
 namespace agcn {
 
+constexpr int PLAN_MADE_UNITS = 0, PLAN_MADE_ZERO = 1, PLAN_MADE_WORDS = 2;
+
 constexpr int SPMM_DEG_BOUND = 384;    // format constant of .block4 (spmm_accel.cu:11)
 // tuples per unit, one per warp (4, 6 and 12 were measured within 2 % of 8; override to experiment)
 #ifndef AGCN_SPMM_WARPS
@@ -82,6 +84,8 @@ struct SpmmParams {
     const int *zero_rows;     // rows no tuple covers
     int64_t n_zero_rows;
     int hot_column;           // HOT kernels: rows of X from this column on are kept in L2; 0: no such choice
+    const int *made;          // ONCE kernels: where the plan kernel before this launch left its numbers of units and of rows without a
+                              // tuple (PLAN_MADE_*), of which n_units and n_zero_rows are the most there can be
     int early;                // host only: launched so that it overlaps the kernel before it
     int wait_first;           // ... which may be any kernel: idx and val, too, are read behind the wait for it
     int relu;                 // nonzero: Y = max(A * X, 0) (fused GCN activation)
@@ -460,6 +464,7 @@ __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 spa
 // main kernel.  S = lanes per slot in float4 mode (4, 8, 16 or 32; needs
 // dim % 4 == 0, dim <= 4*S and 16-byte aligned rows); S = 0 is the scalar
 // mode for every other dim (lane l owns columns l, l+32, l+64, l+96).
+// ONCE: the plan's kernel was launched before, and only it knows how many units and rows without a tuple there are (p.made).
 // Q = columns per lane / 4: with 2, a lane has 8 columns (S = 8 or 16 for up to 64 or 128 of them), loaded 32 bytes at a time:
 // rows of X on 32-byte boundaries, dim % 8 == 0; for what products, see spmm_octets.
 // FINISH: rows that cross units are finished here (in launches of few units);
@@ -469,7 +474,7 @@ __device__ __forceinline__ void finish_carried_row(const SpmmParams &p, int2 spa
 // ANY_ROWS: as float4 mode, with the same additions in the same order, but rows of X and Y of any alignment: lane l of a
 // slot has columns l, l + S, l + 2 S, l + 3 S (consecutive ones cost four times the wavefronts).
 // ---------------------------------------------------------------------------
-template <int S, int Q, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT, bool ANY_ROWS>
+template <int S, int Q, int BATCH, int MIN_BLOCKS, bool PLAIN, bool FINISH, bool HOT, bool ANY_ROWS, bool ONCE = false>
 __global__ void __launch_bounds__(SPMM_THREADS, MIN_BLOCKS)
 spmm_units_kernel(const SpmmParams p)
 {
@@ -491,28 +496,36 @@ spmm_units_kernel(const SpmmParams p)
     if (HOT) pol.hot = p.hot_column;
     if constexpr (ANY_ROWS) pol.cols = (p.dim_store - sl + S - 1) / S;
 
+    if constexpr (ONCE) wait_for_predecessor();                // launched early behind the plan's kernel, or the copy of X behind it
     if (!p.wait_first) launch_dependents();     // a dense transform of this product's result may lay out its weights meanwhile
     if (p.abort_flag != nullptr && *p.abort_flag != 0) return;     // input rejected by a check earlier in the stream
+    if constexpr (ONCE) {
+        if ((int64_t)blockIdx.x < p.n_units && blockIdx.x >= (unsigned)p.made[PLAN_MADE_UNITS]) return;
+    }
     if ((int64_t)blockIdx.x >= p.n_units) {
         wait_for_predecessor();
         // zero-fill rows that no tuple covers
         // (when accumulating, these rows keep their value and only the activation is applied)
-        const int64_t zb = ((int64_t)blockIdx.x - p.n_units) * SPMM_ZERO_ROWS_PER_BLOCK;
-        for (int k = w * NS + slot; k < SPMM_ZERO_ROWS_PER_BLOCK; k += SPMM_WARPS * NS) {
-            if (zb + k >= p.n_zero_rows) break;
-            float *yr = p.y + (int64_t)p.zero_rows[zb + k] * p.ldy;
-            if (VEC) {
-                if constexpr (Q == 2) {
-                    if (active) emit_row8<PLAIN>(p, yr, ycol, zero_octet(), pol.stream);
-                } else if (active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, make_float4(0.f, 0.f, 0.f, 0.f), p.relu, pol.stream);
-            } else {
-                for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, 0.f, p.relu, pol.stream);
+        int64_t zb = ((int64_t)blockIdx.x - p.n_units) * SPMM_ZERO_ROWS_PER_BLOCK;
+        const int64_t n_zero_rows = ONCE ? (int64_t)p.made[PLAN_MADE_ZERO] : p.n_zero_rows;
+        do {
+            for (int k = w * NS + slot; k < SPMM_ZERO_ROWS_PER_BLOCK; k += SPMM_WARPS * NS) {
+                if (zb + k >= n_zero_rows) break;
+                float *yr = p.y + (int64_t)p.zero_rows[zb + k] * p.ldy;
+                if (VEC) {
+                    if constexpr (Q == 2) {
+                        if (active) emit_row8<PLAIN>(p, yr, ycol, zero_octet(), pol.stream);
+                    } else if (active) emit_row4<PLAIN, LOOSE>(p, yr, ycol, make_float4(0.f, 0.f, 0.f, 0.f), p.relu, pol.stream);
+                } else {
+                    for (int c = lane; c < p.dim; c += 32) emit_row1<PLAIN>(p, yr + c, 0.f, p.relu, pol.stream);
+                }
             }
-        }
+            zb += ((int64_t)gridDim.x - p.n_units) * SPMM_ZERO_ROWS_PER_BLOCK;       // ONCE: as many blocks as there may be rows would be a great many
+        } while (ONCE && zb < n_zero_rows);
         return;
     }
 
-    const unsigned b = blockIdx.x, k = p.light_every, n = (unsigned)p.n_units;
+    const unsigned b = blockIdx.x, k = p.light_every, n = ONCE ? (unsigned)p.made[PLAN_MADE_UNITS] : (unsigned)p.n_units;
     const int64_t unit = p.unit_base + (k != 0 && b % k == k - 1 ? b / k : n - 1 - (k != 0 ? b - b / k : b));
     const int64_t e = unit * SPMM_WARPS + w;
     const TupleView t = decode_tuple(p.tuples, e, p.n_tuples);
@@ -719,8 +732,9 @@ constexpr int PLAN_ERR_BITS = 4;
 constexpr int PLAN_FULL_NZ = 192;
 constexpr int PLAN_BLOCK = 256;      // units per thread block, one per thread
 
-__device__ __forceinline__ void plan_report(HostWords *out, int err)
+__device__ __forceinline__ void plan_report(HostWords *out, int err, int *bad = nullptr)
 {
+    if (bad != nullptr) *bad = 1;
 #pragma unroll
     for (int k = 0; k < PLAN_ERR_BITS; k++)
         if (err & (1 << k)) out->w[PLAN_WORD_ERR + k] = 1;
@@ -817,9 +831,10 @@ __device__ __forceinline__ bool ids_outside(const int *__restrict__ idx, int64_t
 }
 
 // Column ids, by `blocks` thread blocks of which this is number `block`.
-__device__ __forceinline__ void plan_check_ids(const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned block, unsigned blocks, HostWords *out)
+__device__ __forceinline__ void plan_check_ids(const int *__restrict__ idx, int64_t n_idx, int64_t n_cols, unsigned block, unsigned blocks, HostWords *out,
+                                               int *bad = nullptr)
 {
-    if (ids_outside(idx, n_idx, n_cols, (int64_t)block * blockDim.x + threadIdx.x, (int64_t)blocks * blockDim.x)) plan_report(out, SPMM_ERR_COL);
+    if (ids_outside(idx, n_idx, n_cols, (int64_t)block * blockDim.x + threadIdx.x, (int64_t)blocks * blockDim.x)) plan_report(out, SPMM_ERR_COL, bad);
 }
 
 // How many of PLAN_SAMPLES column ids, one from every PLAN_SAMPLES-th part of the nonzeros, are at least `first` (anywhere
@@ -1033,10 +1048,12 @@ constexpr int PLAN_SMALL_BLOCK = 1024;
 __global__ void __launch_bounds__(PLAN_SMALL_BLOCK)
 plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows, int64_t nnz, const int *__restrict__ idx, int64_t n_idx,
                   int64_t n_cols, const PieceChoice choice, int4 *pieces, int cap_pieces, int2 *unit_carry, int2 *carry_span, int *carry_row, int *zero_rows,
-                  int *counters, int64_t n_counters, unsigned clear_blocks, HostWords *out)
+                  int *made, int *bad, int *counters, int64_t n_counters, unsigned clear_blocks, HostWords *out)
 {
+    // made, bad: null, or for a product launched behind this kernel: the numbers it needs, and a word that is zero unless something is wrong
+    launch_dependents();
     if (blockIdx.x > clear_blocks) {
-        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - 1 - clear_blocks, gridDim.x - 1 - clear_blocks, out);
+        plan_check_ids(idx, n_idx, n_cols, blockIdx.x - 1 - clear_blocks, gridDim.x - 1 - clear_blocks, out, bad);
         return;
     }
     if (blockIdx.x > 0) {
@@ -1063,7 +1080,7 @@ plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows,
     }
     const bool last = e0 < e1 && e1 == n_blocks;
     if (last && err == 0) zero += n_rows - ((int64_t)a.y + tuple_rows(a));
-    if (err) plan_report(out, err);
+    if (err) plan_report(out, err, bad);
     if (__syncthreads_or(err)) return;
     int n_pieces, n_zero;
     int piece = block_scan_exclusive<PLAN_SMALL_BLOCK>(mine, OpAdd(), 0, n_pieces, s_scan);
@@ -1079,7 +1096,16 @@ plan_small_kernel(const int4 *__restrict__ block4, int n_blocks, int64_t n_rows,
     }
     int zero_out = block_scan_exclusive<PLAN_SMALL_BLOCK>((int)zero, OpAdd(), 0, n_zero, s_scan);
     if (threadIdx.x == 0) { out->w[PLAN_WORD_ZERO] = n_zero; out->w[PLAN_WORD_PIECES] = n_pieces; out->w[PLAN_WORD_LONGEST] = longest; }
-    if (n_pieces > cap_pieces) return;              // cannot be: valid tuples do not overlap
+    if (n_pieces > cap_pieces) {                    // cannot be: valid tuples do not overlap
+        if (threadIdx.x == 0 && bad != nullptr) *bad = 1;
+        return;
+    }
+    if (made != nullptr) {
+        if (threadIdx.x == 0) { made[PLAN_MADE_UNITS] = (n_pieces + SPMM_WARPS - 1) / SPMM_WARPS; made[PLAN_MADE_ZERO] = n_zero; }
+        // the product counts on cap_pieces of them: the last unit's missing ones are empty
+        const int at = n_pieces + threadIdx.x;
+        if (threadIdx.x < SPMM_WARPS && at < cap_pieces) pieces[at] = make_int4(0, 0, 0, 0);
+    }
     a = before;
     for (int e = e0; e < e1; e++) {
         const int4 b = block4[e];

@@ -4,6 +4,7 @@
 #include "internal.h"
 #include "kernels/spmm_kernels.cuh"
 
+#include <atomic>
 #include <cstdlib>
 #include <new>
 
@@ -171,8 +172,8 @@ static int plan_errors(const HostWordsLease &words)
 }
 
 // The plan's arrays, in one pool block: n_pieces tuples of its own (0: it walks the caller's), bookkeeping of its
-// units, n_carry slots, n_zero rows.
-static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int4 **pieces, cudaStream_t s)
+// units, n_carry slots, n_zero rows, n_numbers words for the plan kernel to leave numbers in.
+static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int64_t n_numbers, int4 **pieces, int **numbers, cudaStream_t s)
 {
     for (int pass = 0; pass < 2; pass++) {
         Carver m(p->memory);
@@ -182,6 +183,7 @@ static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int4 **pieces, cudaS
         p->carry_row = m.take<int>(p->n_carry);
         p->carry = m.take<unsigned char>((int64_t)spmm_carry_bytes(p->n_carry));
         p->zero_rows = m.take<int>(p->n_zero);
+        *numbers = m.take<int>(n_numbers);
         if (pass == 1 || m.bytes() == 0) break;
         const cudaError_t e = pool_alloc(&p->memory, m.bytes(), s);
         if (e != cudaSuccess) {
@@ -192,31 +194,44 @@ static int plan_memory(agcn_spmm_plan *p, int64_t n_pieces, int4 **pieces, cudaS
     return AGCN_OK;
 }
 
-// One launch and one wait: the memory is sized by what the pieces can be at most (a piece that is not the last of
-// its tuple or row holds more than half of the nonzeros that a piece may have).
-static int plan_fill_small(agcn_spmm_plan *p, const PieceChoice &choice, const int *d_indices, int64_t n_idx, cudaStream_t s)
+// One launch: the memory is sized by what the pieces can be at most (a piece that is not the last of its tuple or row
+// holds more than half of the nonzeros that a piece may have).  made, bad: as for the kernel.
+static int plan_launch_small(agcn_spmm_plan *p, const PieceChoice &choice, const int *d_indices, int64_t n_idx, int *bad, const int **made,
+                             HostWordsLease &words, cudaStream_t s)
 {
     const int64_t cap = p->n_blocks + 2 * p->nnz / (choice.most < choice.otherwise ? choice.most : choice.otherwise) + 8;
     AGCN_REQUIRE(cap < (int64_t)INT32_MAX / 4, "agcn_spmm_create: too many pieces");
     p->split = true;
+    p->n_tuples = cap;
     p->n_units = ceil_div(cap, SPMM_WARPS);
     p->n_carry = 2 * p->n_units;
     p->n_zero = p->n_rows;
     int4 *pieces = nullptr;
-    int rc = plan_memory(p, cap, &pieces, s);
+    int *numbers = nullptr;
+    const int rc = plan_memory(p, cap, made != nullptr ? PLAN_MADE_WORDS : 0, &pieces, &numbers, s);
     if (rc != AGCN_OK) return rc;
-    AGCN_HOST_WORDS(words, s);
+    if (made != nullptr) *made = numbers;
+    p->tuples = pieces;
     const int64_t col_blocks = ceil_div(n_idx, PLAN_SMALL_BLOCK * 16), counters = p->n_carry * SPMM_CARRY_PASSES;
     const int64_t clear_blocks = ceil_div(counters, PLAN_SMALL_BLOCK * 16);
     AGCN_KERNEL(plan_small_kernel, (unsigned)(1 + clear_blocks + (col_blocks < 2368 ? col_blocks : 2368)), PLAN_SMALL_BLOCK, s, p->block4,
                 (int)p->n_blocks, p->n_rows, p->nnz, d_indices, n_idx, p->n_cols, choice, pieces, (int)cap, p->unit_carry, p->carry_span, p->carry_row,
-                p->zero_rows, spmm_carry_counters(p->carry, p->n_carry), counters, (unsigned)clear_blocks, words.device());
+                p->zero_rows, made != nullptr ? numbers : nullptr, bad, spmm_carry_counters(p->carry, p->n_carry), counters, (unsigned)clear_blocks,
+                words.device());
     AGCN_LAUNCH_CHECK("plan_small_kernel");
+    return AGCN_OK;
+}
+
+// The same, and one wait.
+static int plan_fill_small(agcn_spmm_plan *p, const PieceChoice &choice, const int *d_indices, int64_t n_idx, cudaStream_t s)
+{
+    AGCN_HOST_WORDS(words, s);
+    int rc = plan_launch_small(p, choice, d_indices, n_idx, nullptr, nullptr, words, s);
+    if (rc != AGCN_OK) return rc;
     AGCN_CUDA(words.sync());
     rc = plan_errors(words);
     if (rc != AGCN_OK) return rc;
-    AGCN_REQUIRE(words[PLAN_WORD_PIECES] <= cap, "agcn_spmm_create: more pieces than the tuples can have");
-    p->tuples = pieces;
+    AGCN_REQUIRE(words[PLAN_WORD_PIECES] <= p->n_tuples, "agcn_spmm_create: more pieces than the tuples can have");
     p->n_tuples = words[PLAN_WORD_PIECES];
     p->n_units = ceil_div(p->n_tuples, SPMM_WARPS);
     p->n_zero = words[PLAN_WORD_ZERO];
@@ -258,7 +273,8 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     p->n_full = words[PLAN_WORD_FULL];
     p->hot_tail = ask_tail && (double)words[PLAN_WORD_TAIL] >= SPMM_HOT_SHARE * PLAN_SAMPLES;
     int4 *pieces = nullptr;
-    rc = plan_memory(p, 0, &pieces, s);
+    int *numbers = nullptr;
+    rc = plan_memory(p, 0, 0, &pieces, &numbers, s);
     if (rc != AGCN_OK) return rc;
     if (p->n_carry > 0)
         AGCN_CUDA(cudaMemsetAsync(spmm_carry_counters(p->carry, p->n_carry), 0, (size_t)p->n_carry * SPMM_CARRY_PASSES * sizeof(int), s));
@@ -273,32 +289,47 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
     return AGCN_OK;
 }
 
-int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, const int *d_indices,
-                       int64_t n_rows, int64_t n_cols, int64_t nnz, cudaStream_t s)
+static int spmm_check_graph(const int *d_block4, int64_t n_blocks, int64_t n_rows, int64_t n_cols, int64_t nnz)
 {
-    AGCN_REQUIRE(out != nullptr, "agcn_spmm_create: null plan pointer");
-    *out = nullptr;
     AGCN_REQUIRE(n_blocks >= 0 && (n_blocks == 0 || d_block4 != nullptr), "agcn_spmm_create: null block4");
     AGCN_REQUIRE(aligned16(d_block4), "agcn_spmm_create: block4 must be 16-byte aligned");
     AGCN_REQUIRE(n_rows > 0 && n_rows < (int64_t)INT32_MAX && n_cols > 0 && n_cols < (int64_t)INT32_MAX,
                  "agcn_spmm_create: n_rows / n_cols out of range");
     AGCN_REQUIRE(nnz >= 0 && nnz <= (int64_t)INT32_MAX, "agcn_spmm_create: nnz out of range");
     AGCN_REQUIRE(n_blocks < (int64_t)INT32_MAX, "agcn_spmm_create: too many blocks");
+    return AGCN_OK;
+}
 
-    agcn_spmm_plan *p = new (std::nothrow) agcn_spmm_plan;
-    AGCN_REQUIRE(p != nullptr, "agcn_spmm_create: out of host memory");
-    struct Guard { agcn_spmm_plan *p; ~Guard() { plan_free(p); } } guard{p};       // frees the half-built plan on every early return
+// What a plan knows before it looks at the tuples.
+static int spmm_begin(agcn_spmm_plan *p, const int *d_block4, int64_t n_blocks, int64_t n_rows, int64_t n_cols, int64_t nnz)
+{
     AGCN_CUDA(cudaGetDevice(&p->device));
     AGCN_CUDA(cudaDeviceGetAttribute(&p->sm_count, cudaDevAttrMultiProcessorCount, p->device));
     AGCN_CUDA(cudaDeviceGetAttribute(&p->l2_bytes, cudaDevAttrL2CacheSize, p->device));
     p->block4 = reinterpret_cast<const int4 *>(d_block4);
     p->n_blocks = n_blocks; p->n_rows = n_rows; p->n_cols = n_cols; p->nnz = nnz;
-    const int64_t n_idx = d_indices != nullptr ? nnz : 0;
-    const PieceChoice choice = spmm_piece_choice(n_blocks, n_rows, nnz, p->sm_count);
-    const int rc = choice.most > 0 ? plan_fill_small(p, choice, d_indices, n_idx, s) : plan_fill(p, d_indices, n_idx, s);
-    if (rc != AGCN_OK) return rc;
     p->panel_override = env_int("AGCN_SPMM_PANEL", 0);
     p->pad_unaligned = env_int("AGCN_SPMM_PAD", 1);
+    return AGCN_OK;
+}
+
+int spmm_create(agcn_spmm_plan **out, const int *d_block4, int64_t n_blocks, const int *d_indices,
+                       int64_t n_rows, int64_t n_cols, int64_t nnz, cudaStream_t s)
+{
+    AGCN_REQUIRE(out != nullptr, "agcn_spmm_create: null plan pointer");
+    *out = nullptr;
+    int rc = spmm_check_graph(d_block4, n_blocks, n_rows, n_cols, nnz);
+    if (rc != AGCN_OK) return rc;
+
+    agcn_spmm_plan *p = new (std::nothrow) agcn_spmm_plan;
+    AGCN_REQUIRE(p != nullptr, "agcn_spmm_create: out of host memory");
+    struct Guard { agcn_spmm_plan *p; ~Guard() { plan_free(p); } } guard{p};       // frees the half-built plan on every early return
+    rc = spmm_begin(p, d_block4, n_blocks, n_rows, n_cols, nnz);
+    if (rc != AGCN_OK) return rc;
+    const int64_t n_idx = d_indices != nullptr ? nnz : 0;
+    const PieceChoice choice = spmm_piece_choice(n_blocks, n_rows, nnz, p->sm_count);
+    rc = choice.most > 0 ? plan_fill_small(p, choice, d_indices, n_idx, s) : plan_fill(p, d_indices, n_idx, s);
+    if (rc != AGCN_OK) return rc;
     guard.p = nullptr;
     *out = p;
     return AGCN_OK;
@@ -386,9 +417,28 @@ static void launch_units_for(const SpmmParams &prm, unsigned grid, const SpmmFor
     }
 }
 
+// Behind the plan's kernel (ONCE): the general flavour, deep or not, whatever the widths and blocks.
+template <int S>
+static void launch_once(const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
+{
+    auto go = [&](auto k) { launch_early(prm.early != 0, k, grid, SPMM_THREADS, 0, s, prm); };
+    if constexpr (S == 0) go(spmm_units_kernel<0, 1, SPMM_WIDE_GATHER_BATCH, SPMM_WIDE_MIN_BLOCKS, false, true, false, false, true>);
+    else if (f.loose) {
+        if (f.deep) go(spmm_units_kernel<S, 1, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, false, true, false, true, true>);
+        else go(spmm_units_kernel<S, 1, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true, false, true, true>);
+    } else if (f.deep) go(spmm_units_kernel<S, 1, SPMM_DEEP_GATHER_BATCH, SPMM_DEEP_MIN_BLOCKS, false, true, false, false, true>);
+    else go(spmm_units_kernel<S, 1, SPMM_GATHER_BATCH, SPMM_MIN_BLOCKS, false, true, false, false, true>);
+}
+
 static void launch_units_for_width(int width, bool vec, const SpmmParams &prm, unsigned grid, const SpmmForm &f, cudaStream_t s)
 {
-    if (f.octets) width <= 64 ? launch_octets<8>(prm, grid, f, s) : launch_octets<16>(prm, grid, f, s);
+    if (prm.made != nullptr) {
+        if (!vec) launch_once<0>(prm, grid, f, s);
+        else if (width <= 16) launch_once<4>(prm, grid, f, s);
+        else if (width <= 32) launch_once<8>(prm, grid, f, s);
+        else if (width <= 64) launch_once<16>(prm, grid, f, s);
+        else launch_once<32>(prm, grid, f, s);
+    } else if (f.octets) width <= 64 ? launch_octets<8>(prm, grid, f, s) : launch_octets<16>(prm, grid, f, s);
     else if (!vec) launch_units_for<0>(prm, grid, f, s);
     else if (width <= 16) launch_units_for<4>(prm, grid, f, s);
     else if (width <= 32) launch_units_for<8>(prm, grid, f, s);
@@ -433,7 +483,10 @@ static int spmm_few_form(const agcn_spmm_plan *p)
     return p->n_units <= 4 * sm || (uneven && 10 * p->n_units <= 63 * sm) ? 4 : 0;
 }
 
-static bool spmm_deep(const agcn_spmm_plan *p) { return p->split && p->n_units <= spmm_deep_units(p->sm_count); }
+static bool spmm_deep(const agcn_spmm_plan *p)
+{
+    return p->split && (p->likely_units > 0 ? p->likely_units : p->n_units) <= spmm_deep_units(p->sm_count);
+}
 
 // Small products gather 4 bytes at a time from X as it is instead, with the additions of the 16-byte path in its order:
 // to a chain of latencies the copy adds a kernel, and where a row of X is named a few times the copy of it is a good part
@@ -517,7 +570,8 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     const int64_t unit0 = part.unit0, unit1 = part.unit1 < 0 ? p->n_units : part.unit1;
     AGCN_REQUIRE(unit0 >= 0 && unit0 <= unit1 && unit1 <= p->n_units, "agcn_spmm_run: unit range outside the plan");
     // rows no tuple covers: zero-filled -- or, when accumulating, left alone unless an activation is due
-    const int64_t zero_blocks = !part.zero_fill || (accumulate && !activation) ? 0 : ceil_div(p->n_zero, SPMM_ZERO_ROWS_PER_BLOCK);
+    int64_t zero_blocks = !part.zero_fill || (accumulate && !activation) ? 0 : ceil_div(p->n_zero, SPMM_ZERO_ROWS_PER_BLOCK);
+    if (part.made != nullptr && zero_blocks > 2 * p->sm_count) zero_blocks = 2 * p->sm_count;         // n_zero is all rows then; the blocks take turns
     const int64_t grid = (unit1 - unit0) + zero_blocks;
     AGCN_REQUIRE(grid < (int64_t)INT32_MAX, "agcn_spmm_run: grid too large");
 
@@ -556,7 +610,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         if (width > slot_left) width = slot_left;
         SpmmParams prm;
         prm.tuples = p->tuples; prm.n_tuples = p->n_tuples;
-        prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag;
+        prm.n_units = unit1 - unit0; prm.unit_base = unit0; prm.abort_flag = part.abort_flag; prm.made = part.made;
         // a later pass follows the one before it, which waits for what came before
         prm.early = part.early == SpmmLaunchPart::ANY || (part.early == SpmmLaunchPart::ONLY_X && col0 == 0) ? 1 : 0;
         prm.wait_first = part.early == SpmmLaunchPart::ANY ? 1 : 0;
@@ -596,24 +650,119 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     return AGCN_OK;
 }
 
-int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *d_x, int64_t ldx,
-             float *d_y, int64_t ldy, int dim, cudaStream_t s, int activation, int accumulate)
+// made, bad: null, or of a plan whose kernel was launched before on the stream: SpmmLaunchPart::made and abort_flag
+static int spmm_run_whole(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *d_x, int64_t ldx,
+                          float *d_y, int64_t ldy, int dim, cudaStream_t s, int activation, int accumulate, const int *made, const int *bad)
 {
-    int rc = spmm_check_run_args(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, activation);
-    if (rc != AGCN_OK) return rc;
-    const DeviceOf on(p->device);
     p->launches_last_run = 0;
     const float *x_use = d_x;
     int64_t ldx_use = ldx;
     bool x_vec = x_rows_aligned(d_x, ldx, dim);
-    rc = spmm_loose(p) ? AGCN_OK : spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
+    const int rc = spmm_loose(p) ? AGCN_OK : spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
     if (rc != AGCN_OK) return rc;
     SpmmLaunchPart part;
     // A product is launched while the operation before it still runs and waits for it on the GPU, so that launch, first
     // instructions and tuples are no longer paid one after the other by a row of small products.  us per call, B200, before
     // and after: 2 048 rows of 4, dim 16: 6.1, 4.6; 16 384 rows of 8, dim 60: 10.2, 7.4; from 300 us on no difference.
     part.early = x_use != d_x ? SpmmLaunchPart::ONLY_X : SpmmLaunchPart::ANY;       // behind the copy of X, or the caller's work
+    part.made = made;
+    part.abort_flag = bad;
     return spmm_run_prepared(p, d_indices, d_vals, x_use, ldx_use, x_vec, d_y, ldy, dim, s, activation, accumulate, part);
+}
+
+int spmm_run(agcn_spmm_plan *p, const int *d_indices, const float *d_vals, const float *d_x, int64_t ldx,
+             float *d_y, int64_t ldy, int dim, cudaStream_t s, int activation, int accumulate)
+{
+    const int rc = spmm_check_run_args(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, activation);
+    if (rc != AGCN_OK) return rc;
+    const DeviceOf on(p->device);
+    return spmm_run_whole(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, s, activation, accumulate, nullptr, nullptr);
+}
+
+// The words that say "something is wrong" to products launched behind the plan of their graph: one for each of the calls
+// under way, zero when the library is loaded and when they are handed out.
+constexpr int PLAN_BAD_WORDS = 64;
+static __device__ int g_plan_bad[PLAN_BAD_WORDS];
+static std::atomic<uint64_t> g_plan_bad_free{~(uint64_t)0};
+
+class BadWord {
+public:
+    BadWord()
+    {
+        uint64_t free = g_plan_bad_free.load();
+        while (free != 0 && !g_plan_bad_free.compare_exchange_weak(free, free & (free - 1))) {}
+        number_ = free != 0 ? __builtin_ctzll(free) : -1;
+    }
+    ~BadWord() { if (number_ >= 0 && zero_) g_plan_bad_free.fetch_or((uint64_t)1 << number_); }     // else it stays out of use
+    BadWord(const BadWord &) = delete;
+    BadWord &operator=(const BadWord &) = delete;
+    bool none() const { return number_ < 0; }
+    cudaError_t address(int **out) const
+    {
+        void *base = nullptr;
+        const cudaError_t e = cudaGetSymbolAddress(&base, g_plan_bad);
+        *out = e == cudaSuccess ? static_cast<int *>(base) + number_ : nullptr;
+        return e;
+    }
+    void launched() { zero_ = false; }
+    void zero() { zero_ = true; }
+private:
+    int number_;
+    bool zero_ = true;
+};
+
+// Plan, product and the end of the plan in one call, which returns when Y is there (or untouched, and something was wrong).
+// The product of a small graph is launched behind the plan's kernel, without a wait between them: it finds on the device how many
+// thread blocks it has (PLAN_MADE_*), and whether anything is wrong.  (As create, run and destroy: a wait for the plan, one
+// for the device, and the launch of the product between.  From the graph, degree sort and partitioner included, to Y, us, B200, before / so:
+// 2 048 rows of 4: 114 / 102;  16 384 of 8: 122 / 112;  60 000 of 8: 176 / 160;  140 000 of 6: 181 / 177.)
+static int spmm_once(const int *d_block4, int64_t n_blocks, const int *d_indices, const float *d_vals, int64_t n_rows, int64_t n_cols, int64_t nnz,
+                     const float *d_x, int64_t ldx, float *d_y, int64_t ldy, int dim, cudaStream_t s)
+{
+    int rc = spmm_check_graph(d_block4, n_blocks, n_rows, n_cols, nnz);
+    if (rc != AGCN_OK) return rc;
+    agcn_spmm_plan plan;
+    rc = spmm_begin(&plan, d_block4, n_blocks, n_rows, n_cols, nnz);
+    if (rc != AGCN_OK) return rc;
+    const PieceChoice choice = spmm_piece_choice(n_blocks, n_rows, nnz, plan.sm_count);
+    BadWord word;
+    if (choice.most <= 0 || word.none()) {
+        agcn_spmm_plan *p = nullptr;
+        rc = spmm_create(&p, d_block4, n_blocks, d_indices, n_rows, n_cols, nnz, s);
+        if (rc == AGCN_OK) rc = spmm_run(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, s);
+        plan_free(p);
+        return rc;
+    }
+    int *bad = nullptr;
+    AGCN_CUDA(word.address(&bad));
+    // what is wrong with the graph is said before what is wrong with the operands
+    const int run_rc = spmm_check_run_args(&plan, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, 0);
+    struct Memory {
+        agcn_spmm_plan *p;
+        cudaStream_t s;
+        ~Memory() { pool_free(p->memory, s); if (p->x_pad_malloc) cudaFree(p->x_pad); else pool_free(p->x_pad, s); }
+    } memory{&plan, s};
+    AGCN_HOST_WORDS(words, s);
+    const int *made = nullptr;
+    rc = plan_launch_small(&plan, choice, d_indices, d_indices != nullptr ? nnz : 0, bad, &made, words, s);
+    if (rc != AGCN_OK) return rc;
+    word.launched();
+    if (run_rc == AGCN_OK) {
+        // the bound on the number of pieces says nothing of how many gathers pay: about three quarters of a piece's nonzeros are there
+        const int64_t likely = ceil_div(4 * nnz, 3 * (int64_t)choice.most);
+        plan.likely_units = ceil_div(choice.otherwise != choice.most && likely > choice.fit ? ceil_div(4 * nnz, 3 * (int64_t)choice.otherwise) : likely, SPMM_WARPS);
+        rc = spmm_run_whole(&plan, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, s, 0, 0, made, bad);
+    }
+    AGCN_CUDA(words.sync());
+    const int plan_rc = plan_errors(words);
+    if (plan_rc != AGCN_OK) {
+        AGCN_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
+        AGCN_CUDA(cudaStreamSynchronize(s));
+    }
+    word.zero();
+    if (plan_rc != AGCN_OK) return plan_rc;
+    if (run_rc != AGCN_OK) return spmm_check_run_args(&plan, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, 0);
+    return rc;
 }
 
 }  // namespace agcn
@@ -638,6 +787,13 @@ extern "C" int agcn_spmm_run_act(agcn_spmm_plan *plan, const int32_t *d_indices,
 {
     agcn::clear_error();
     return agcn::spmm_run(plan, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, static_cast<cudaStream_t>(stream), activation);
+}
+
+extern "C" int agcn_spmm_once(const int32_t *d_block4, int64_t n_blocks, const int32_t *d_indices, const float *d_vals, int64_t n_rows,
+                              int64_t n_cols, int64_t nnz, const float *d_x, int64_t ldx, float *d_y, int64_t ldy, int dim, void *stream)
+{
+    agcn::clear_error();
+    return agcn::spmm_once(d_block4, n_blocks, d_indices, d_vals, n_rows, n_cols, nnz, d_x, ldx, d_y, ldy, dim, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int agcn_spmm_destroy(agcn_spmm_plan *plan)

@@ -178,6 +178,11 @@ int agcn_spmm_run_act(agcn_spmm_plan *plan, const int32_t *d_indices, const floa
 
 int agcn_spmm_destroy(agcn_spmm_plan *plan);
 
+/* agcn_spmm_create, agcn_spmm_run and agcn_spmm_destroy for a graph that is multiplied once: the same checks and the same
+ * result, with one wait.  Returns when Y is complete; where something is wrong with the graph, Y is as it was. */
+int agcn_spmm_once(const int32_t *d_block4, int64_t n_blocks, const int32_t *d_indices, const float *d_vals, int64_t n_rows, int64_t n_cols,
+                   int64_t nnz, const float *d_x, int64_t ldx, float *d_y, int64_t ldy, int dim, void *stream);
+
 /* Number of kernel launches the last agcn_spmm_run on this plan issued, and
  * the sizes of its internal scratch (for reporting). */
 int agcn_spmm_plan_info(const agcn_spmm_plan *plan, int64_t *n_units, int64_t *n_carry,

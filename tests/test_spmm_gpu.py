@@ -748,6 +748,46 @@ def test_small_products_from_rows_of_any_alignment(kind, dim):
     plan.close()
 
 
+@pytest.mark.parametrize("kind", ["one row", "few", "pieces", "hubs", "mostly empty", "uncut"])
+def test_product_of_a_graph_that_is_used_once(kind):
+    # plan and product behind one another without a wait: the bits of a kept plan's product, whatever the number of pieces,
+    # rows without nonzeros (more than their thread blocks take at a time), rows that cross thread blocks, unaligned widths
+    import torch
+    from accelgcn import partition, spmm, AccelGcnError
+    dev = require_cuda()
+    rng = np.random.default_rng(len(kind))
+    deg = {"one row": lambda: [5], "few": lambda: rng.integers(0, 30, 700), "pieces": lambda: rng.integers(0, 20, 30_000),
+           "hubs": lambda: np.concatenate([rng.integers(0, 3, 19_990), [700, 900, 1_500, 4_000, 6_000, 9_000, 20_000]]),
+           "mostly empty": lambda: np.concatenate([np.zeros(300_000, int), rng.integers(1, 9, 2_000)]), "uncut": lambda: rng.integers(1, 5, 160_000)}[kind]()
+    indptr = np.concatenate([[0], np.cumsum(np.sort(deg))]).astype(np.int32)
+    n, cols, nnz = len(deg), 5_000, int(indptr[-1])
+    idx = torch.from_numpy(rng.integers(0, cols, nnz, dtype=np.int32)).to(dev)
+    val = torch.from_numpy(rng.standard_normal(nnz).astype(np.float32)).to(dev)
+    block4 = partition.block_level_partition_device(torch.from_numpy(indptr).to(dev))
+    plan = spmm.SpmmPlan(block4, idx, n, cols)
+    for dim in (1, 16, 61, 64, 100, 128, 150):
+        x = torch.from_numpy(rng.standard_normal((cols, dim)).astype(np.float32)).to(dev)
+        want, got = torch.full((n, dim), 7.0, device=dev), torch.full((n, dim), 8.0, device=dev)
+        plan.run(idx, val, x, want)
+        for _ in range(3):
+            assert spmm.spmm(block4, idx, val, x, n, out=got.fill_(8.0)) is got
+            assert torch.equal(got, want), dim
+    plan.close()
+    # refused as by a plan, Y as it was; and the next product is right again
+    for bad in (cols, -1):
+        was, idx[nnz // 2] = int(idx[nnz // 2]), bad
+        with pytest.raises(AccelGcnError, match="column index"):
+            spmm.spmm(block4, idx, val, x, n, out=got.fill_(9.0))
+        assert bool((got == 9.0).all())
+        idx[nnz // 2] = was
+    wrong = block4.clone()
+    wrong[-1, 1] = n
+    with pytest.raises(AccelGcnError, match="rows out of range"):
+        spmm.spmm(wrong, idx, val, x, n, out=got)
+    assert bool((got == 9.0).all())
+    assert torch.equal(spmm.spmm(block4, idx, val, x, n, out=got), want)
+
+
 @pytest.mark.parametrize("hub", [0, 3_000])
 @pytest.mark.parametrize("units", [394, 395, 444, 445, 592, 593, 932, 933])
 def test_products_of_few_thread_blocks(units, hub, monkeypatch):
