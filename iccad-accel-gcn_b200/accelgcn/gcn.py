@@ -3,7 +3,8 @@ the Python face of agcn_gcn2_forward_*.
 
 Per layer and per rank:  Z_block = H_block @ W  (tcgen05 TF32 GEMM on the rows this rank owns),
 all-gather of Z (NCCL, slice by slice), H'_block = relu(A_block @ Z) (the SpMM with its fused
-ReLU).  On one GPU and from 32 768 rows on: A @ X, both transforms in one kernel, relu(A @ Z).  The reference stops at the SpMM; the layers are the workload its operator exists for.
+ReLU).  On one GPU and from 32 768 rows on: A @ X, both transforms in one kernel, relu(A @ Z).
+The reference stops at the SpMM; the layers are the workload its operator exists for.
 Everything is enqueued by the library on the caller's stream; this class owns only the handle.
 """
 from __future__ import annotations

@@ -232,6 +232,33 @@ def test_two_layer_gcn_forward_matches_fp64(world, slices):
         sh.close()
 
 
+@pytest.mark.parametrize("n,launches", [(32_767, 4), (32_768, 3)])
+def test_forward_on_both_sides_of_the_line(n, launches):
+    # from 32 768 rows on A is applied to X before W1 and one kernel makes both transforms: the same function, TF32 in the transforms
+    import torch
+    from accelgcn import synth, sharded, gcn
+    dev = require_cuda()
+    gen = torch.Generator(dev).manual_seed(n)
+    ip = torch.arange(0, 5 * n + 1, 5, dtype=torch.int32, device=dev)
+    ix = torch.randint(0, n, (5 * n,), dtype=torch.int32, device=dev, generator=gen)
+    v = torch.rand(5 * n, device=dev, generator=gen)
+    x = synth.features(n, 128, 3, dev)
+    w = [synth.glorot(128, 128, 3, k, dev) for k in (8, 9)]
+    sh = sharded.ShardedSpmm(ip, ix, v, 0, 1)
+    fwd = gcn.GcnForward(sh, w)
+    out = fwd.forward(sh.to_block(x))
+    torch.cuda.synchronize()
+    times = fwd.status(timings=True)
+    assert fwd.launches() == launches and all(layer[0] > 0 and layer[2] > 0 for layer in times)
+
+    def times_a(h):
+        return (h[ix.long()] * v.double()[:, None]).view(n, 5, 128).sum(dim=1)
+
+    ref = times_a(times_a(x.double() @ w[0].double()).clamp_(min=0) @ w[1].double()).clamp_(min=0)
+    assert float((out.double() - ref).abs().max()) <= 4e-3 * float(ref.max())
+    fwd.close(); sh.close()
+
+
 def test_two_layer_gcn_forward_at_five_million_nodes():
     # configuration 5 at a tenth of its size (N = 5 000 000, ~1.07e8 nonzeros, 128 features): the whole
     # native forward against the CPU forward.  Tolerance: TF32 keeps 10 mantissa bits per operand of
