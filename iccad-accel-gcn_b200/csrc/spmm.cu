@@ -500,9 +500,24 @@ static bool spmm_deep(const agcn_spmm_plan *p)
 // gains: they are where no width of the graphs above loses.  Over 68 graphs inside them, dims 17, 61, 127: 0.82 of the time
 // with the copy; slower: 30 000 rows of exactly 12 and 16 384 of exactly 10, dim 17 (12 and 7 %), 500 of 100, dim 127 (3 to 7 %).
 // (Its sums take 4 S places of a carry slot where the columns may be fewer: forced passes might not leave them.)
-static bool spmm_loose(const agcn_spmm_plan *p)
+// Large products of an X whose rows are named a few times and that is a good part of L2 or more do, too: there the copy is two
+// passes of HBM over X, and the gather reads rows of the copy as often from HBM as it would those of X.  Time without the copy /
+// with, nonzeros per row of X and X of 61 columns / L2 in brackets, dims 30, 39, 54, 61, 78, 99, 127:
+// power law, 1.5 M of 4 [3.9, 2.8]: .86 .80 .78 .80 .78 .76 .76;  500 000 of 5 [4.9, 0.9]: .84 .80 .81 .81 .82 .79 .78;  2.4 M of 7 [6.8, 4.4]: .98 .90 .91 .96
+// .88 .87 .92;  900 000 of 8 [7.8, 1.7]: .99 .91 .91 .94 .91 .90 .93;  350 000 of 8 [7.7, 0.65]: .95 .88 .88 .89 .91 .88 .87;  skewed, 500 000 of
+// 8 [7.8, 0.9]: 1.16 .94 .93 .98 .91 .88 .91;  300 000 of 6 [5.9, 0.55]: - - .92 .96 .88 .88 .87;  not taken: power law, 160 000 of 6 [5.7, 0.30]: 1.03
+// - .94 .89 1.02 .90 .87;  2 M of 10 [9.8, 3.7]: 1.04 - .97 1.03 .96 .95 .98;  500 000 of 12 [11.6, 0.9]: 1.06 - .98 1.00 .99 .98 1.00;  500 000 of 18
+// [17.3, 0.9]: 1.18 - 1.06 1.10 1.07 1.07 1.09.
+constexpr double SPMM_LOOSE_L2 = 0.4;
+
+static bool spmm_loose(const agcn_spmm_plan *p, int dim)
 {
-    if (!p->pad_unaligned || p->panel_override != 0 || !p->split) return false;
+    if (!p->pad_unaligned || p->panel_override != 0) return false;
+    if (!p->split) {
+        // rows of whole eights keep the order of additions that the same columns have where they are aligned
+        if (dim > SPMM_PANEL || p->nnz > (dim > 32 ? 8 : 6) * p->n_cols || (double)p->n_cols * dim * 4.0 < SPMM_LOOSE_L2 * p->l2_bytes) return false;
+        return dim % 8 != 0 || !spmm_octets(p, dim);
+    }
     return (spmm_deep(p) && p->nnz <= (int64_t)500 * p->sm_count) || (p->nnz <= 13 * p->n_cols && p->nnz <= (int64_t)2700 * p->sm_count);
 }
 
@@ -586,7 +601,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
     // AGCN_SPMM_PANEL (read when the plan is created) overrides the choice.  (A product whose A is
     // column-tiled -- agcn_spmm_tiled_* -- keeps its X slab in L2 by construction and never splits.)
     const bool whole = unit0 == 0 && unit1 == p->n_units;
-    const bool loose = !x_vec && whole && spmm_loose(p);
+    const bool loose = !x_vec && whole && spmm_loose(p, dim);
     const int64_t ldx_panel = loose ? (dim + 3) & ~3 : ldx_use;         // the passes, hence the sums, that the aligned copy would get
     int panel = SPMM_PANEL;
     if (dim > 64 && dim % 32 == 0 && ldx_panel % 32 == 0 && !accumulate && !p->never_split) {
@@ -595,7 +610,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         if (x_bytes > 0.75 * (double)p->l2_bytes && x_bytes <= 4.0 * (double)p->l2_bytes) panel = 64;
     }
     if (p->panel_override > 0) panel = p->panel_override;
-    const bool carry_inside = !whole || !spmm_many_units(p);        // parts of a product always finish their rows
+    const bool carry_inside = !whole || loose || !spmm_many_units(p);        // parts of a product, and that form, always finish their rows
     // A carry slot holds SPMM_PANEL floats and every column pass uses its own columns (and arrival
     // counters) of it, so a product of up to SPMM_PANEL columns can be issued in parts whatever its
     // passes are -- with the same passes, hence the same bits, as a whole run.
@@ -632,7 +647,9 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.y_vec = y_vec ? 1 : 0;
         prm.dim_store = width;
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
-        const bool octets = vec && !loose && prm.dim % 8 == 0 && ldx_use % 8 == 0 && aligned32(prm.x) && spmm_octets(p, prm.dim);
+        // (not for the copy of an X that a whole product reads as it is: one issued in parts has the same bits)
+        const bool octets = vec && !loose && prm.dim % 8 == 0 && ldx_use % 8 == 0 && aligned32(prm.x) && spmm_octets(p, prm.dim) &&
+                            (dim % 4 == 0 || p->never_split || !spmm_loose(p, dim));
         const bool plain = !accumulate && !loose && (vec ? y_vec : true) && (!octets || (width % 8 == 0 && ldy % 8 == 0 && aligned32(prm.y)));
         if (grid > 0) {
             const SpmmForm form = {plain, carry_inside, spmm_deep(p), spmm_wide_form(p, width), loose, spmm_few_form(p), octets, spmm_many_units(p)};
@@ -658,7 +675,7 @@ static int spmm_run_whole(agcn_spmm_plan *p, const int *d_indices, const float *
     const float *x_use = d_x;
     int64_t ldx_use = ldx;
     bool x_vec = x_rows_aligned(d_x, ldx, dim);
-    const int rc = spmm_loose(p) ? AGCN_OK : spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
+    const int rc = spmm_loose(p, dim) ? AGCN_OK : spmm_prepare_x(p, d_x, ldx, dim, s, &x_use, &ldx_use, &x_vec);
     if (rc != AGCN_OK) return rc;
     SpmmLaunchPart part;
     // A product is launched while the operation before it still runs and waits for it on the GPU, so that launch, first

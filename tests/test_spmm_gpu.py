@@ -866,6 +866,51 @@ def test_rows_of_x_32_bytes_at_a_time(uncut, dim):
         assert np.array_equal(np.flatnonzero(odd.any(axis=1)), touched)
 
 
+@pytest.mark.parametrize("dim", [33, 36, 61, 99, 123])
+def test_large_products_of_an_x_that_is_named_a_few_times(dim):
+    # an X of 0.4 of L2 or more with up to eight nonzeros per row is read as it is, whatever its alignment, also by uncut plans:
+    # one launch, and bit for bit what the same columns in aligned rows give; rows that cross thread blocks, rows without nonzeros.
+    # (Not 127 columns: an aligned 128 of such an X goes in two passes of 64, whose additions come in another order.)
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    gen = torch.Generator(dev).manual_seed(dim)
+    rng = np.random.default_rng(dim)
+    deg = np.sort(np.concatenate([rng.integers(0, 6, 400_000), rng.integers(33, 300, 400), [385, 4_000, 30_000]]))
+    n = len(deg)
+    cols = int(0.42 * torch.cuda.get_device_properties(dev).L2_cache_size / (4 * 33)) + 7
+    indptr = torch.from_numpy(np.concatenate([[0], np.cumsum(deg)]).astype(np.int32)).to(dev)
+    nnz = int(deg.sum())
+    idx = torch.randint(0, cols, (nnz,), device=dev, generator=gen, dtype=torch.int32)
+    val = torch.randn(nnz, device=dev, generator=gen)
+    plan = spmm.SpmmPlan(partition.block_level_partition_device(indptr), idx, n, cols)
+    wide = (dim + 3) // 4 * 4
+    aligned = torch.zeros((cols, wide), device=dev)
+    aligned[:, :dim] = torch.randn(cols, dim, device=dev, generator=gen)
+    aligned[3, 0], aligned[5, dim - 1] = float("inf"), float("nan")
+    want = torch.empty((n, wide), device=dev)
+    plan.run(idx, val, aligned, want, relu=True)
+    plan.run(idx, val, aligned, want)
+    for shift, ldx, ldy in ((1, dim, dim), (0, dim + 1, wide), (3, wide + 2, dim + 1)):
+        x = torch.full((cols * ldx + shift,), float("nan"), device=dev)[shift:]
+        x.view(cols, ldx)[:, :dim] = aligned[:, :dim]
+        y = torch.full((n * ldy,), 7.0, device=dev)
+        for _ in range(2):                  # the arrival counters are zero again
+            plan.run(idx, val, x, y, dim=dim, ldx=ldx, ldy=ldy)
+            assert plan.info()["launches_last_run"] == 1
+        got = y.view(n, ldy)
+        assert torch.equal(got[:, :dim].nan_to_num(3.0, 4.0, 5.0), want[:, :dim].nan_to_num(3.0, 4.0, 5.0)), (shift, ldx, ldy)
+        assert bool((got[:, dim:] == 7.0).all())
+    # and against the definition, in 64 bits
+    rows = torch.repeat_interleave(torch.arange(n, device=dev), indptr.diff().long())
+    finite = aligned[:, :dim].nan_to_num(0.0, 0.0, 0.0).contiguous()
+    plan.run(idx, val, finite, y, dim=dim, ldx=dim, ldy=ldy)
+    ref = torch.zeros((n, dim), device=dev, dtype=torch.float64).index_add_(0, rows, val.double()[:, None] * finite.double()[idx.long()])
+    scale = torch.zeros(n, device=dev, dtype=torch.float64).index_add_(0, rows, val.double().abs()) * float(finite.abs().max())
+    assert spmm_close(y.view(n, ldy)[:, :dim].cpu().numpy(), ref.cpu().numpy(), scale.cpu().numpy()).all()
+    plan.close()
+
+
 @pytest.mark.parametrize("shift", [0, 1, 2, 3])
 @pytest.mark.parametrize("nnz", [1, 2, 3, 4, 5, 6, 7, 8, 9, 11, 4_099, 6_000_001])
 def test_a_column_id_outside_is_found_wherever_it_is(nnz, shift):
