@@ -358,7 +358,7 @@ struct SpmmForm {
     bool finish;     // rows that cross units are finished in the launch
     bool deep;       // few thread blocks, many gathers per lane
     bool wide;       // more thread blocks per SM, fewer gathers per lane
-    bool loose;      // rows of X of any alignment, 4 bytes at a time (cut plans: spmm_loose)
+    bool loose;      // rows of X of any alignment, 4 bytes at a time (spmm_loose)
     int few;         // thread blocks per SM of a launch of few, more than the deep ones: 3, 4 (17 to 32 columns) or 0: as ever
     bool octets;     // 32-byte loads (spmm_octets), of a plan of many units or not
     bool many;
