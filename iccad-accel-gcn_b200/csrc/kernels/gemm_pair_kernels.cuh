@@ -55,12 +55,13 @@ __device__ __forceinline__ void tmem_st_32x32(uint32_t taddr, const float (&v)[3
 }
 __device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// The nearest TF32 number, ties away from zero
+// The nearest TF32 number to a v >= 0, ties upwards; above the largest one v itself, which the tensor core cuts (a finite number
+// does not become infinite)
 __device__ __forceinline__ float to_tf32(float v)
 {
     uint32_t r;
     asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(v));
-    return __uint_as_float(r);
+    return v < 0x1.ffep127f ? __uint_as_float(r) : v;
 }
 
 __global__ void __launch_bounds__(PAIR_THREADS, 1)

@@ -54,6 +54,13 @@ def test_pair_of_transforms_matches_fp64(m):
     eye = torch.eye(128, device=dev)
     gemm.gemm_tf32_pair_async(p, eye, eye, z[:m], status)
     assert torch.equal(z[:m], p.clamp(min=0)) and int(status.item()) == 0
+    # an activation above the largest TF32 number, which the nearest one would be infinity for: cut
+    p.zero_()
+    w1 = eye.clone()
+    w1[1, 0] = 1.0
+    p[m - 1, 0], p[m - 1, 1] = float.fromhex("0x1.ffcp127"), float.fromhex("0x1.8p116")
+    gemm.gemm_tf32_pair_async(p, w1, eye, z[:m], status)
+    assert float(z[m - 1, 0]) == float.fromhex("0x1.ffcp127") and bool(torch.isfinite(z[:m]).all())
 
 
 def test_gemm_identity_and_strided_rows():
