@@ -3,6 +3,7 @@
 #include "host_common.h"
 #include "internal.h"
 #include "kernels/spmm_kernels.cuh"
+#include "spmm_rules.h"
 
 #include <atomic>
 #include <cstdlib>
@@ -461,26 +462,9 @@ int spmm_pad_rows(const float *d_x, int64_t ldx, int dim, float *d_xp, int64_t n
 
 static bool x_rows_aligned(const float *d_x, int64_t ldx, int dim) { return dim % 4 == 0 && ldx % 4 == 0 && aligned16(d_x); }
 
-// Cut plans of more thread blocks than the deep form takes, by how many the SMs hold at once.  Blocks of even graphs take
-// equally long, so what counts is that they are one round: up to three per SM eight gathers a lane with 80 registers
-// beat seven with 64.  Where there are hub rows, whose full pieces go first, and rows short enough that a piece holds several,
-// blocks get lighter towards the end: nothing waits for a last round, and three per SM gain up to four per SM.  17 to 32 columns, with
-// four gathers at five blocks otherwise, gain with seven at four blocks as far as four per SM, with hub rows 6.3.
-// Time with three per SM / before, dims 16, 32, 64, 128, blocks per SM in brackets: even rows 40 000 of 10, 20 000 of 20, 10 000 of
-// 60, 14 000 of 30 [2.8-3.0]: .92 .73 .86 .79, .92 .73 .87 .81, .94 .74 .85 .83, .83 .75 .88 .82;  power law, 16 384 of 9, 18 000 of
-// 8 [2.8], 25 000 of 7, 28 000 of 6 [3.5], 35 000 of 5 [3.9]: .94 .89 .92 .91, .96 .88 .94 .92, .87 .88 .86 .88, .93 .90 .90 .90, .97 .91 .92
-// .90;  skewed, 12 000 of 20, 20 000 of 11 [3.8]: .92 .90 .95 1.05, .95 .93 .93 .88;  not taken: dense, 3 500 of 110, 4 000 of 110
-// [3.5, 4.0]: 1.10 1.05 1.16 1.22, 1.18 1.09 1.20 1.14;  power law, 16 384 of 20, 30 000 of 14 [3.9, 4.3]: .96 .88 1.09 1.21, .97 .86 1.05 1.10.
-// 17 to 32 columns, four blocks / five: even, 25 000 of 25, 50 000 of 8 [3.5]: .87, .89;  dense, 7 000 of 100 [4.0]: .88;  power law,
-// 30 000 of 20 [4.2], 40 000 of 14 [4.6], 50 000 of 10 [5.8]: .88, .89, .92;  skewed, 25 000 of 30 [4.8], 40 000 of 15 [6.3]: .86, .90;
-// not taken: even, 30 000 of 12 [4.2]: 1.23;  dense, 5 000 of 100 [4.6]: 1.14;  skewed, 60 000 of 20 [9.0]: 1.10.
-static int spmm_few_form(const agcn_spmm_plan *p)
+static int spmm_few_form(const agcn_spmm_plan *p, int width)
 {
-    if (!p->split) return 0;
-    const bool uneven = p->longest * p->n_rows > 4 * p->nnz && p->nnz < 32 * p->n_rows;
-    const int64_t sm = p->sm_count;
-    if (p->n_units <= 3 * sm || (uneven && p->n_units <= 4 * sm)) return 3;
-    return p->n_units <= 4 * sm || (uneven && 10 * p->n_units <= 63 * sm) ? 4 : 0;
+    return p->split ? spmm_few_form(CutPlan{p->n_units, p->n_rows, p->nnz, p->longest, p->sm_count}, width) : 0;
 }
 
 static bool spmm_deep(const agcn_spmm_plan *p)
@@ -652,7 +636,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
                             (dim % 4 == 0 || p->never_split || !spmm_loose(p, dim));
         const bool plain = !accumulate && !loose && (vec ? y_vec : true) && (!octets || (width % 8 == 0 && ldy % 8 == 0 && aligned32(prm.y)));
         if (grid > 0) {
-            const SpmmForm form = {plain, carry_inside, spmm_deep(p), spmm_wide_form(p, width), loose, spmm_few_form(p), octets, spmm_many_units(p)};
+            const SpmmForm form = {plain, carry_inside, spmm_deep(p), spmm_wide_form(p, width), loose, spmm_few_form(p, width), octets, spmm_many_units(p)};
             launch_units_for_width(prm.dim, vec, prm, (unsigned)grid, form, s);
             AGCN_LAUNCH_CHECK("spmm_units_kernel");
             p->launches_last_run++;

@@ -1,0 +1,53 @@
+// Rules of the SpMM's dispatch that need nothing but a plan's numbers.
+#pragma once
+#include <stdint.h>
+
+namespace agcn {
+
+// What a rule may ask of a cut plan.
+struct CutPlan {
+    int64_t n_units, n_rows, nnz;
+    int64_t longest;          // nonzeros of the longest row
+    int sm_count;
+};
+
+// Thread blocks per SM, 3 or 4, of the form that a product of few thread blocks takes at `width` columns; 0: as any product.
+//
+// Cut plans of more thread blocks than the deep form takes, by how many the SMs hold at once.  Blocks of even graphs take
+// equally long, so what counts is that they are one round: up to three per SM eight gathers a lane with 80 registers
+// beat seven with 64.  Where there are hub rows, whose full pieces go first, and rows short enough that a piece holds several,
+// blocks get lighter towards the end.  Up to four per SM a second round of light blocks then costs little, the less the
+// longer the longest row is, compared with the others, and the more rows of X a warp reads at a time: always up to 32 columns,
+// where the longest row has 190 times the average up to 64, 290 times beyond (pieces of 128 lose at any width: none).
+// 17 to 32 columns, with four gathers at five blocks otherwise, gain with seven at four blocks as far as four per SM, with hub
+// rows 6.3.
+// Time with three per SM / without, B200, blocks per SM and the longest row as multiple of the average in brackets.
+// Up to three, dims 16, 32, 64, 128: even rows 40 000 of 10, 20 000 of 20, 10 000 of 60, 14 000 of 30 [2.8-3.0]: .92 .73 .86 .79, .92
+// .73 .87 .81, .94 .74 .85 .83, .83 .75 .88 .82;  power law, 16 384 of 9 [2.8]: .95 .94 .91 .91.
+// Three to four, dims 16, 32, 36, 60, 64, 100, 128; taken at all of them: power law, 25 000 of 7 [3.5, 479], 28 000 of 6 [3.5, 544],
+// 35 000 of 5 [3.9, 652], 30 000 of 9 [3.8, 464], 25 000 of 12 [3.9, 301], 24 000 of 12 [3.7, 292]: .94 .90 .91 .90 .89 .88 .90, .92 .85 .86 .86 .90 .84 .90, .93
+// .90 .86 .86 .90 .84 .90, .96 .90 .90 .89 .90 .86 .90, .96 .91 .89 .88 .94 .95 1.01, .96 .89 .89 .88 .90 .92 .99;  skewed, 20 000 of 11 [3.8, 342],
+// 22 000 of 14 [4.0, 295]: .97 .96 .92 .93 .94 .90 .90, .93 .93 .89 .88 .88 .85 .84.
+// Taken up to 64: power law, 20 000 of 10 [3.7, 280], 20 000 of 14 [3.5, 217], 18 000 of 12 [4.0, 225], 20 000 of 15 [3.7, 200]: .90 .89 .89 .90 .93 .97
+// 1.04, .94 .88 .88 .89 .90 .90 .96, .95 .92 .90 .91 .95 1.04 1.14, .95 .89 .93 .96 1.00 1.03 1.08;  skewed, 20 000 of 16 [4.0, 237]: .94 .91 .89 .88
+// .90 .84 .84.
+// Taken up to 32: power law, 16 384 of 20 [3.9, 128], 14 000 of 22 [3.7, 103], 18 000 of 18 [3.9, 152], 20 000 of 16 [3.9, 188]: .94 .93 1.01 1.02
+// 1.07 1.10 1.16, .95 .94 1.01 1.02 1.07 1.11 1.16, .97 .96 1.04 1.07 1.09 1.13 1.20, .95 .92 .97 1.03 1.07 1.08 1.14;  skewed, 12 000 of 20 [3.8, 114], 16 000 of 22
+// [4.0, 138]: .92 .91 .91 .92 .95 1.00 1.05, .95 .89 .92 .94 .99 1.03 1.06.
+// Not taken: pieces of 128, power law, 16 384 of 25 [3.8, 103], 18 000 of 22 [3.7, 128]: 1.04 1.05 1.10 1.12 1.15 1.20 1.24, 1.01 1.01 1.09 1.09 1.13 1.17 1.22;
+// above four, power law, 25 000 of 14 [4.4]: 1.00 .97 1.06 1.08 1.12 1.17 1.21;  dense, 3 500 of 110, 4 000 of 110 [3.5, 4.0], dims 16, 32, 64, 128: 1.10 1.05
+// 1.16 1.22, 1.18 1.09 1.20 1.14.
+// 17 to 32 columns, four blocks / five: even, 25 000 of 25, 50 000 of 8 [3.5]: .87, .89;  dense, 7 000 of 100 [4.0]: .88;  power law,
+// 16 384 of 25 [3.8], 30 000 of 20 [4.2], 40 000 of 14 [4.6], 50 000 of 10 [5.8]: .90, .88, .89, .92;  skewed, 25 000 of 30 [4.8], 40 000 of 15 [6.3]: .86,
+// .90;  not taken: even, 30 000 of 12 [4.2]: 1.23;  dense, 5 000 of 100 [4.6]: 1.14;  skewed, 60 000 of 20 [9.0]: 1.10.
+inline int spmm_few_form(const CutPlan &p, int width)
+{
+    const int64_t sm = p.sm_count;
+    const bool uneven = p.longest * p.n_rows > 4 * p.nnz && p.nnz < 32 * p.n_rows;
+    if (p.n_units <= 3 * sm) return 3;
+    const int64_t times = width <= 32 ? 0 : width <= 64 ? 190 : 290;
+    if (uneven && p.n_units <= 4 * sm && p.nnz <= 2700 * sm && p.longest * p.n_rows >= times * p.nnz) return 3;
+    return p.n_units <= 4 * sm || (uneven && 10 * p.n_units <= 63 * sm) ? 4 : 0;
+}
+
+}  // namespace agcn

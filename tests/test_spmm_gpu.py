@@ -788,7 +788,7 @@ def test_product_of_a_graph_that_is_used_once(kind):
     assert torch.equal(spmm.spmm(block4, idx, val, x, n, out=got), want)
 
 
-@pytest.mark.parametrize("hub", [0, 3_000])
+@pytest.mark.parametrize("hub", [0, 3_000, 6_000])
 @pytest.mark.parametrize("units", [394, 395, 444, 445, 592, 593, 932, 933])
 def test_products_of_few_thread_blocks(units, hub, monkeypatch):
     # both sides of the lines between the forms of launches of few thread blocks, on graphs with and without a hub row; every slot width
@@ -799,7 +799,7 @@ def test_products_of_few_thread_blocks(units, hub, monkeypatch):
         pytest.skip("sizes are those of 148 SMs")
     monkeypatch.setenv("AGCN_SPMM_PIECE", "64")
     rng = np.random.default_rng(units)
-    # tuples of 12 rows of 16: three pieces; a unit is eight pieces, the hub row 47 of them
+    # tuples of 12 rows of 16: three pieces; a unit is eight pieces, the hub row 47 or 94 of them
     pieces = units * 8 - (-(-hub // 64) if hub else 0)
     deg = np.full(pieces // 3 * 12 + pieces % 3 * 4, 16)
     deg = np.append(deg, hub) if hub else deg
