@@ -100,11 +100,21 @@ struct TupleView {
     bool valid, small;
 };
 
-__device__ __forceinline__ TupleView decode_tuple(const int4 *__restrict__ block4, int64_t e, int64_t n_blocks)
+// What the plan's kernel wrote.  A product launched behind that kernel (ONCE) is resident while it is written: such data
+// must not be read as read-only, not even behind the wait.
+template <bool ONCE, typename T>
+__device__ __forceinline__ T ld_plan(const T *p)
+{
+    if constexpr (ONCE) return *p;
+    else return __ldg(p);
+}
+
+template <bool ONCE>
+__device__ __forceinline__ TupleView decode_tuple(const int4 *tuples, int64_t e, int64_t n_tuples)
 {
     TupleView t;
-    t.valid = e < n_blocks;
-    const int4 b = t.valid ? __ldg(block4 + e) : make_int4(0, 0, 0, 0);
+    t.valid = e < n_tuples;
+    const int4 b = t.valid ? ld_plan<ONCE>(tuples + e) : make_int4(0, 0, 0, 0);
     t.small = b.x <= SPMM_DEG_BOUND;
     t.row0 = b.y;
     t.loc = b.z;
@@ -528,7 +538,7 @@ spmm_units_kernel(const SpmmParams p)
     const unsigned b = blockIdx.x, k = p.light_every, n = ONCE ? (unsigned)p.made[PLAN_MADE_UNITS] : (unsigned)p.n_units;
     const int64_t unit = p.unit_base + (k != 0 && b % k == k - 1 ? b / k : n - 1 - (k != 0 ? b - b / k : b));
     const int64_t e = unit * SPMM_WARPS + w;
-    const TupleView t = decode_tuple(p.tuples, e, p.n_tuples);
+    const TupleView t = decode_tuple<ONCE>(p.tuples, e, p.n_tuples);
     const bool big = t.valid && !t.small;
     const int total = t.n_rows * t.row_nz;
     if (p.wait_first) {                 // tuples are the plan's and do not change
@@ -618,7 +628,7 @@ spmm_units_kernel(const SpmmParams p)
     while (w_end < SPMM_WARPS && s_big[w_end] && s_row[w_end] == t.row0) w_end++;
     const int64_t left = p.n_tuples - unit * SPMM_WARPS;
     const int w_last = left < SPMM_WARPS ? (int)left - 1 : SPMM_WARPS - 1;
-    const int2 uc = __ldg(p.unit_carry + unit);
+    const int2 uc = ld_plan<ONCE>(p.unit_carry + unit);
     const bool enters = w == 0 && uc.x >= 0;            // the row began in an earlier unit
     const bool leaves = w_end - 1 == w_last && uc.y >= 0;   // the row goes on in the next unit
     const bool partial = enters || leaves;     // other units hold the rest of the row
@@ -644,7 +654,7 @@ spmm_units_kernel(const SpmmParams p)
     }
     if (!FINISH) return;                            // spmm_carry_kernel follows
     // the row's last unit to arrive adds the partials
-    const int2 span = __ldg(p.carry_span + my_slot);
+    const int2 span = ld_plan<ONCE>(p.carry_span + my_slot);
     __threadfence();
     __syncwarp();
     int arrived = 0;

@@ -788,6 +788,42 @@ def test_product_of_a_graph_that_is_used_once(kind):
     assert torch.equal(spmm.spmm(block4, idx, val, x, n, out=got), want)
 
 
+def _once_graph(deg, cols, seed, dev):
+    # a graph in degree order with its operands, and what a kept plan gives for it
+    import torch
+    from accelgcn import partition, spmm
+    rng = np.random.default_rng(seed)
+    indptr = np.concatenate([[0], np.cumsum(np.sort(deg))]).astype(np.int32)
+    n, nnz = len(deg), int(indptr[-1])
+    idx = torch.from_numpy(rng.integers(0, cols, nnz, dtype=np.int32)).to(dev)
+    val = torch.from_numpy(rng.standard_normal(nnz).astype(np.float32)).to(dev)
+    x = torch.from_numpy(rng.standard_normal((cols, 61 if seed % 2 else 64)).astype(np.float32)).to(dev)
+    block4 = partition.block_level_partition_device(torch.from_numpy(indptr).to(dev))
+    want = torch.full((n, x.shape[1]), 7.0, device=dev)
+    plan = spmm.SpmmPlan(block4, idx, n, cols)
+    plan.run(idx, val, x, want)
+    torch.cuda.synchronize()
+    plan.close()
+    return block4, idx, val, x, want
+
+
+def test_graphs_that_are_used_once_in_turn_in_the_same_memory():
+    # the product is resident while the plan's kernel writes the tuples and carry slots that it reads, into the memory in which the
+    # last graph had other ones: every row one further on, or other degrees altogether; rows that cross thread blocks in all of them
+    import torch
+    from accelgcn import spmm
+    dev = require_cuda()
+    rng = np.random.default_rng(3)
+    hubs = [700, 2_000, 5_000, 9_000]
+    deg = np.concatenate([rng.integers(1, 20, 9_000), hubs])
+    graphs = [_once_graph(np.append(deg, [0] * zeros), 4_000, 10 + zeros, dev) for zeros in (0, 1, 2)]
+    graphs += [_once_graph(np.concatenate([rng.integers(0, 20, 9_000), hubs[::2]]), 4_000, 21, dev)]
+    for k in range(80):
+        block4, idx, val, x, want = graphs[k % len(graphs)]
+        y = spmm.spmm(block4, idx, val, x, len(want), out=torch.full_like(want, 8.0))
+        assert torch.equal(y, want), k
+
+
 @pytest.mark.parametrize("hub", [0, 3_000, 6_000])
 @pytest.mark.parametrize("units", [394, 395, 444, 445, 592, 593, 932, 933])
 def test_products_of_few_thread_blocks(units, hub, monkeypatch):
