@@ -31,6 +31,7 @@
 #include "../host_common.h"
 #include "primitives.cuh"
 #include "ptx.cuh"
+#include "../spmm_rules.h"
 
 namespace agcn {
 
@@ -725,20 +726,9 @@ spmm_pad_rows_kernel(const float *x, int64_t ldx, int dim, float *xp, int ldp, i
 // ---------------------------------------------------------------------------
 // plan: built once per `.block4` array
 // ---------------------------------------------------------------------------
-constexpr int SPMM_ERR_TUPLE = 1;     // malformed tuple (degree, row count or chunk length)
-constexpr int SPMM_ERR_ROW = 2;       // rows out of range, overlapping or not ascending
-constexpr int SPMM_ERR_LOC = 4;       // nonzero range outside [0, nnz)
-constexpr int SPMM_ERR_COL = 8;       // column index outside [0, n_cols)
-
 __device__ __forceinline__ bool tuple_is_big(const int4 &b) { return b.x > SPMM_DEG_BOUND; }
 __device__ __forceinline__ int tuple_rows(const int4 &b) { return tuple_is_big(b) ? 1 : (b.w & 0xffff); }
 
-// Error bits are single words of the host so that blocks can store to them without atomics.
-constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_FULL = 3;
-constexpr int PLAN_WORD_TAIL = PLAN_WORD_PIECES;            // uncut plans, which have no pieces
-constexpr int PLAN_WORD_LONGEST = PLAN_WORD_FULL;           // cut plans, which do not count full tuples
-constexpr int PLAN_WORD_ERR = 4;      // then one word per SPMM_ERR_* bit
-constexpr int PLAN_ERR_BITS = 4;
 constexpr int PLAN_FULL_NZ = 192;
 constexpr int PLAN_BLOCK = 256;      // units per thread block, one per thread
 

@@ -159,11 +159,12 @@ static int spmm_light_every(const agcn_spmm_plan *p, int width)
     return p->n_units > (int64_t)28 * p->sm_count && x_bytes <= 0.6 * p->l2_bytes ? 4 : 0;
 }
 
-static int plan_errors(const HostWordsLease &words)
+// most_pieces: as for plan_faults
+static int plan_errors(const HostWordsLease &words, int64_t most_pieces)
 {
-    int err = 0;
-    for (int k = 0; k < PLAN_ERR_BITS; k++) err |= words[PLAN_WORD_ERR + k] != 0 ? 1 << k : 0;
+    const int err = plan_faults(words, most_pieces);
     if (err == 0) return AGCN_OK;
+    AGCN_REQUIRE((err & SPMM_ERR_PIECES) == 0, "agcn_spmm_create: more pieces than the tuples can have");
     set_error("agcn_spmm_create: invalid input:%s%s%s%s",
               (err & SPMM_ERR_TUPLE) ? " malformed .block4 tuple;" : "",
               (err & SPMM_ERR_ROW) ? " tuple rows out of range or not ascending;" : "",
@@ -230,9 +231,8 @@ static int plan_fill_small(agcn_spmm_plan *p, const PieceChoice &choice, const i
     int rc = plan_launch_small(p, choice, d_indices, n_idx, nullptr, nullptr, words, s);
     if (rc != AGCN_OK) return rc;
     AGCN_CUDA(words.sync());
-    rc = plan_errors(words);
+    rc = plan_errors(words, p->n_tuples);
     if (rc != AGCN_OK) return rc;
-    AGCN_REQUIRE(words[PLAN_WORD_PIECES] <= p->n_tuples, "agcn_spmm_create: more pieces than the tuples can have");
     p->n_tuples = words[PLAN_WORD_PIECES];
     p->n_units = ceil_div(p->n_tuples, SPMM_WARPS);
     p->n_zero = words[PLAN_WORD_ZERO];
@@ -267,7 +267,7 @@ static int plan_fill(agcn_spmm_plan *p, const int *d_indices, int64_t n_idx, cud
                 (unsigned)tiles, ask_tail ? p->n_cols - hot_rows(p, SPMM_PANEL) : (int64_t)-1, tile_zero, tile_carry, ctl, words.device());
     AGCN_LAUNCH_CHECK("plan_check_kernel");
     AGCN_CUDA(words.sync());
-    int rc = plan_errors(words);
+    int rc = plan_errors(words, INT64_MAX);
     if (rc != AGCN_OK) return rc;
     p->n_zero = words[PLAN_WORD_ZERO];
     p->n_carry = words[PLAN_WORD_CARRY];
@@ -755,7 +755,7 @@ static int spmm_once(const int *d_block4, int64_t n_blocks, const int *d_indices
         rc = spmm_run_whole(&plan, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, s, 0, 0, made, bad);
     }
     AGCN_CUDA(words.sync());
-    const int plan_rc = plan_errors(words);
+    const int plan_rc = plan_errors(words, plan.n_tuples);        // whatever sets *bad is an error here, too: the word is handed out again
     if (plan_rc != AGCN_OK) {
         AGCN_CUDA(cudaMemsetAsync(bad, 0, sizeof(int), s));
         AGCN_CUDA(cudaStreamSynchronize(s));

@@ -1,8 +1,30 @@
-// Rules of the SpMM's dispatch that need nothing but a plan's numbers.
+// What the host decides from a plan's numbers alone: whether they are sound, and which form of the kernel a product takes.
 #pragma once
 #include <stdint.h>
 
 namespace agcn {
+
+constexpr int SPMM_ERR_TUPLE = 1;     // malformed tuple (degree, row count or chunk length)
+constexpr int SPMM_ERR_ROW = 2;       // rows out of range, overlapping or not ascending
+constexpr int SPMM_ERR_LOC = 4;       // nonzero range outside [0, nnz)
+constexpr int SPMM_ERR_COL = 8;       // column index outside [0, n_cols)
+
+// Error bits are single words of the host so that blocks can store to them without atomics.
+constexpr int PLAN_WORD_ZERO = 0, PLAN_WORD_CARRY = 1, PLAN_WORD_PIECES = 2, PLAN_WORD_FULL = 3;
+constexpr int PLAN_WORD_TAIL = PLAN_WORD_PIECES;            // uncut plans, which have no pieces
+constexpr int PLAN_WORD_LONGEST = PLAN_WORD_FULL;           // cut plans, which do not count full tuples
+constexpr int PLAN_WORD_ERR = 4;      // then one word per SPMM_ERR_* bit
+constexpr int PLAN_ERR_BITS = 4;
+constexpr int SPMM_ERR_PIECES = 1 << PLAN_ERR_BITS;         // has no word: more pieces than there is room for
+
+// SPMM_ERR_* of what the plan's kernel left in the host's words (most_pieces: INT64_MAX for plans that are not cut).
+template <typename Words>
+int plan_faults(const Words &words, int64_t most_pieces)
+{
+    int err = 0;
+    for (int k = 0; k < PLAN_ERR_BITS; k++) err |= words[PLAN_WORD_ERR + k] != 0 ? 1 << k : 0;
+    return err == 0 && words[PLAN_WORD_PIECES] > most_pieces ? SPMM_ERR_PIECES : err;
+}
 
 // What a rule may ask of a cut plan.
 struct CutPlan {

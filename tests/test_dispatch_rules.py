@@ -1,4 +1,4 @@
-"""The dispatch rules that need only a plan's numbers (csrc/spmm_rules.h), on the graphs that were timed for them."""
+"""The decisions that need only a plan's numbers (csrc/spmm_rules.h), on the graphs that were timed for them."""
 import ctypes
 import os
 import subprocess
@@ -16,11 +16,13 @@ def rules(tmp_path_factory):
     src = d / "rules.cpp"
     src.write_text("""#include "spmm_rules.h"
 extern "C" int few_form(int64_t units, int64_t rows, int64_t nnz, int64_t longest, int sm, int width) { return agcn::spmm_few_form({units, rows, nnz, longest, sm}, width); }
+extern "C" int faults(const int64_t *words, int64_t most) { return agcn::plan_faults(words, most); }
 """)
     lib = str(d / "librules.so")
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I" + os.path.join(PKG, "csrc"), str(src), "-o", lib])
     dll = ctypes.CDLL(lib)
     dll.few_form.argtypes = [ctypes.c_int64] * 4 + [ctypes.c_int, ctypes.c_int]
+    dll.faults.argtypes = [ctypes.POINTER(ctypes.c_int64), ctypes.c_int64]
     return dll
 
 
@@ -55,3 +57,10 @@ def test_three_blocks_per_sm_where_they_were_measured_faster(rules, graph):
     for width in (16, 20, 32, 33, 60, 64, 65, 100, 128):
         form = rules.few_form(units, rows, nnz, longest, SM, width)
         assert form == (3 if width <= widest else 4), width
+
+
+@pytest.mark.parametrize("words,most,faults", [
+    ((5, 0, 800, 40, 0, 0, 0, 0), 800, 0), ((5, 0, 801, 40, 0, 0, 0, 0), 800, 16),          # pieces that do not fit are an error by themselves
+    ((5, 0, 801, 40, 0, 0, 0, 0), 2**63 - 1, 0), ((0, 0, 0, 0, 0, 0, 0, 1), 800, 8), ((0, 0, 900, 0, 1, 0, 1, 0), 800, 5)])
+def test_what_the_plan_kernel_reports(rules, words, most, faults):
+    assert rules.faults((ctypes.c_int64 * 8)(*words), most) == faults

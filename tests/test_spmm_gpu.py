@@ -824,6 +824,49 @@ def test_graphs_that_are_used_once_in_turn_in_the_same_memory():
         assert torch.equal(y, want), k
 
 
+def test_many_graphs_that_are_used_once_at_the_same_time():
+    # 70 calls under way together, six more than there are words that say "something is wrong" (those are products of a plan made first): each
+    # on a stream of its own that is kept busy until all have been started.  Every seventh names a column that is not there
+    import threading
+    import torch
+    from accelgcn import spmm, AccelGcnError
+    dev = require_cuda()
+    rng = np.random.default_rng(4)
+    graphs = [_once_graph(np.concatenate([rng.integers(0, 20, 500 + 37 * k), [900 + 10 * k]]), 1_000, k, dev) for k in range(70)]
+    for k in range(0, 70, 7):
+        graphs[k][1][k] = 1_000
+    outs = [torch.empty_like(g[4]) for g in graphs]
+    streams = [torch.cuda.Stream(dev) for _ in graphs]
+    said = [None] * len(graphs)
+
+    def one(k):
+        block4, idx, val, x, want = graphs[k]
+        try:
+            with torch.cuda.stream(streams[k]):
+                spmm.spmm(block4, idx, val, x, len(want), out=outs[k])
+            said[k] = ""
+        except AccelGcnError as e:
+            said[k] = str(e)
+
+    for _ in range(2):
+        for o in outs:
+            o.fill_(8.0)
+        torch.cuda.synchronize()
+        for s in streams:
+            with torch.cuda.stream(s):
+                torch.cuda._sleep(100_000_000)
+        threads = [threading.Thread(target=one, args=(k,)) for k in range(len(graphs))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        for k, g in enumerate(graphs):
+            if k % 7 == 0:
+                assert "column index" in said[k] and bool((outs[k] == 8.0).all()), k
+            else:
+                assert said[k] == "" and torch.equal(outs[k], g[4]), k
+
+
 @pytest.mark.parametrize("hub", [0, 3_000, 6_000])
 @pytest.mark.parametrize("units", [394, 395, 444, 445, 592, 593, 932, 933])
 def test_products_of_few_thread_blocks(units, hub, monkeypatch):
