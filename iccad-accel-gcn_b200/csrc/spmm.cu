@@ -32,6 +32,13 @@ void plan_free(agcn_spmm_plan *p)
     delete p;
 }
 
+// The same memory, of a plan that has only been used on `s`: in that stream's order, without a wait for the device.
+static void plan_give_back(agcn_spmm_plan *p, cudaStream_t s)
+{
+    pool_free(p->memory, s);
+    if (p->x_pad_malloc) cudaFree(p->x_pad); else pool_free(p->x_pad, s);
+}
+
 // Up to this many thread blocks a cut plan's products keep 16 gathers in flight per lane.
 static int spmm_deep_units(int sm_count) { return 8 * sm_count / 3; }
 
@@ -712,8 +719,8 @@ private:
     bool zero_ = true;
 };
 
-// Plan, product and the end of the plan in one call, which returns when Y is there (or untouched, and something was wrong).
-// The product of a small graph is launched behind the plan's kernel, without a wait between them: it finds on the device how many
+// Plan, product and the end of the plan in one call, which returns when Y is there (or untouched, and something was wrong); it waits
+// for its own stream only.  The product of a small graph is launched behind the plan's kernel, without a wait between them: it finds on the device how many
 // thread blocks it has (PLAN_MADE_*), and whether anything is wrong.  (As create, run and destroy: a wait for the plan, one
 // for the device, and the launch of the product between.  From the graph, degree sort and partitioner included, to Y, us, B200, before / so:
 // 2 048 rows of 4: 114 / 102;  16 384 of 8: 122 / 112;  60 000 of 8: 176 / 160;  140 000 of 6: 181 / 177.)
@@ -730,8 +737,12 @@ static int spmm_once(const int *d_block4, int64_t n_blocks, const int *d_indices
     if (choice.most <= 0 || word.none()) {
         agcn_spmm_plan *p = nullptr;
         rc = spmm_create(&p, d_block4, n_blocks, d_indices, n_rows, n_cols, nnz, s);
-        if (rc == AGCN_OK) rc = spmm_run(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, s);
-        plan_free(p);
+        if (rc != AGCN_OK) return rc;
+        rc = spmm_run(p, d_indices, d_vals, d_x, ldx, d_y, ldy, dim, s);
+        const cudaError_t waited = cudaStreamSynchronize(s);
+        plan_give_back(p, s);
+        delete p;
+        if (rc == AGCN_OK) AGCN_CUDA(waited);
         return rc;
     }
     int *bad = nullptr;
@@ -741,7 +752,7 @@ static int spmm_once(const int *d_block4, int64_t n_blocks, const int *d_indices
     struct Memory {
         agcn_spmm_plan *p;
         cudaStream_t s;
-        ~Memory() { pool_free(p->memory, s); if (p->x_pad_malloc) cudaFree(p->x_pad); else pool_free(p->x_pad, s); }
+        ~Memory() { plan_give_back(p, s); }
     } memory{&plan, s};
     AGCN_HOST_WORDS(words, s);
     const int *made = nullptr;

@@ -788,6 +788,35 @@ def test_product_of_a_graph_that_is_used_once(kind):
     assert torch.equal(spmm.spmm(block4, idx, val, x, n, out=got), want)
 
 
+@pytest.mark.parametrize("rows", [3_000, 160_000])
+def test_a_graph_that_is_used_once_waits_for_its_own_stream_only(rows):
+    # cut and uncut plans: Y is there when the call returns, while another stream is still busy
+    import torch
+    from accelgcn import partition, spmm
+    dev = require_cuda()
+    rng = np.random.default_rng(rows)
+    indptr = np.concatenate([[0], np.cumsum(np.sort(rng.integers(1, 5, rows)))]).astype(np.int32)
+    idx = torch.from_numpy(rng.integers(0, 500, int(indptr[-1]), dtype=np.int32)).to(dev)
+    val, x = torch.rand(len(idx), device=dev), torch.rand(500, 61, device=dev)
+    block4 = partition.block_level_partition_device(torch.from_numpy(indptr).to(dev))
+    want, got = (torch.full((rows, 61), 7.0, device=dev) for _ in range(2))
+    spmm.spmm(block4, idx, val, x, rows, out=want)
+    host = torch.empty((rows, 61), pin_memory=True)
+    busy, mine, done = torch.cuda.Stream(dev), torch.cuda.Stream(dev), torch.cuda.Event()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(busy):
+        torch.cuda._sleep(2_000_000_000)            # a second or so
+        done.record()
+    with torch.cuda.stream(mine):
+        spmm.spmm(block4, idx, val, x, rows, out=got)
+        assert mine.query() and not done.query()
+        host.copy_(got, non_blocking=True)
+        mine.synchronize()
+    assert not done.query()
+    torch.cuda.synchronize()
+    assert torch.equal(host, want.cpu())
+
+
 def _once_graph(deg, cols, seed, dev):
     # a graph in degree order with its operands, and what a kept plan gives for it
     import torch
