@@ -901,7 +901,7 @@ def ours_gcn(args, rank, world, local_rank):
     flops_step = 2 * (2.0 * nnz * 128 + 2.0 * n * 128 * 128)
     value = flops_step * args.steps / (total_ms / 1e3) / 1e9
     per_layer = {"gemm": gemm_ms, "wait_for_first_exchanged_slice": gather_ms, "spmm_relu_incl_later_slices": spmm_ms,
-                 "exchange_slices": shard.slices,
+                 "exchange_slices": shard.slices, "mean_of_both_layers": True,
                  "exchanged_bytes_in_per_rank_per_layer": 4 * 128 * per * (world - 1),
                  "limiting_phase": max((("gemm", gemm_ms), ("exchange", gather_ms), ("spmm", spmm_ms)), key=lambda kv: kv[1])[0]}
 
@@ -945,10 +945,6 @@ def ours_gcn(args, rank, world, local_rank):
         return
 
     peak, peak_src = hbm_peak()
-    # kernels that transform: one a layer, or one for both (which reads P and writes Z once, in gemm_ms of either layer)
-    transforms = fwd.launches() - 2 * shard.info()["launches_last_step"]
-    gemm_bytes = 2 * 4 * 128 * per + 4 * 128 * 128 * (3 - transforms)    # H read + Z written (+ W)
-    gemm_launch_ms = gemm_ms * (3 - transforms)
     spmm_bytes = min_bytes(int(shard.local_nnz), int(shard.n_blocks), per, shard.n_gathered, 128)
     line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": total_ms / args.steps, "higher_is_better": True,
@@ -963,9 +959,7 @@ def ours_gcn(args, rank, world, local_rank):
                          "frac": spmm_bytes / spmm_ms / 1e6 / peak, "traffic": None, "peak_source": peak_src,
                          "kernel": "spmm_units_kernel dim=128 (+ReLU), per rank",
                          "algorithmic_bytes_per_launch": spmm_bytes,
-                         "gemm": {"kernel": "gemm_tf32_128_kernel" if transforms == 2 else "gemm_tf32_pair_kernel",
-                                  "achieved": gemm_bytes / gemm_launch_ms / 1e6,
-                                  "frac": gemm_bytes / gemm_launch_ms / 1e6 / peak, "algorithmic_bytes_per_launch": gemm_bytes}},
+                         "gemm": transform_roofline(fwd.paired(), max(p[0], p[3]), per, peak)},
             "clocks": clocks,
             "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": 4 * 128 * per, "d2h_bytes_per_step": 4 * 128 * per,
                     "steps": e2e_steps, "bit_identical_to_resident_run": same},
@@ -987,6 +981,15 @@ def ours_gcn(args, rank, world, local_rank):
     else:
         dist.destroy_process_group()
     print(json.dumps(line), flush=True)
+
+
+def transform_roofline(paired, ms_per_layer, rows, peak):
+    """The dense transform's part of the roofline: one kernel a layer (the slower one: AGCN_GCN_FUSED=1 leaves the second few
+    rows), or (paired) one for both, whose time is given by halves to the layers and which reads its operand and writes its result once."""
+    layers = 2 if paired else 1
+    n_bytes, ms = 2 * 4 * 128 * rows + 4 * 128 * 128 * layers, ms_per_layer * layers
+    return {"kernel": "gemm_tf32_pair_kernel" if paired else "gemm_tf32_128_kernel", "achieved": n_bytes / ms / 1e6,
+            "frac": n_bytes / ms / 1e6 / peak, "algorithmic_bytes_per_launch": n_bytes}
 
 
 def gcn_sampled_check(ip, ix, v, x_rows, w1, w2, out_block, block_rows, dev, n_sample=48):

@@ -58,6 +58,12 @@ class GcnForward:
         _lib.check(self._lib.agcn_gcn2_forward_launches(self._h, ctypes.byref(n)))
         return n.value
 
+    def paired(self) -> bool:
+        """Whether one kernel made both transforms of the last forward."""
+        n = ctypes.c_int()
+        _lib.check(self._lib.agcn_gcn2_forward_paired(self._h, ctypes.byref(n)))
+        return n.value != 0
+
     def close(self):
         if getattr(self, "_h", None) is not None and self._h.value:
             self._lib.agcn_gcn2_forward_destroy(self._h)

@@ -682,6 +682,14 @@ extern "C" int agcn_gcn2_forward_launches(const agcn_gcn2 *fwd, int *launches)
     return AGCN_OK;
 }
 
+extern "C" int agcn_gcn2_forward_paired(const agcn_gcn2 *fwd, int *paired)
+{
+    agcn::clear_error();
+    AGCN_REQUIRE(fwd != nullptr && paired != nullptr, "agcn_gcn2_forward_paired: null argument");
+    *paired = fwd->alone && fwd->paired ? 1 : 0;
+    return AGCN_OK;
+}
+
 extern "C" int agcn_gcn2_forward_destroy(agcn_gcn2 *fwd)
 {
     agcn::clear_error();

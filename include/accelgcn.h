@@ -425,7 +425,8 @@ int agcn_dist_gathered(const agcn_dist *dist, int slot, const float **d_gathered
  * per layer the transform, the wait for the exchange's first slice, the SpMM.
  * Where nothing is exchanged, from 32 768 rows on, A is applied to X before W1 (A (X W1) =
  * (A X) W1) and both transforms are one kernel (agcn_gemm_tf32_pair_async): its time is then given by halves to
- * the two layers, and so is that of the two products.  agcn_gcn2_forward_launches: kernels the last run launched.
+ * the two layers, and so is that of the two products.  agcn_gcn2_forward_launches: kernels the last run launched;
+ * agcn_gcn2_forward_paired: 1 if one kernel made both transforms of it, else 0.
  * ---------------------------------------------------------------------- */
 typedef struct agcn_gcn2 agcn_gcn2;
 
@@ -433,6 +434,7 @@ int agcn_gcn2_forward_create(agcn_gcn2 **fwd, agcn_dist *dist, const float *d_w1
 int agcn_gcn2_forward_run(agcn_gcn2 *fwd, const float *d_x_block, float *d_out_block, void *stream);
 int agcn_gcn2_forward_status(agcn_gcn2 *fwd, float *ms6);
 int agcn_gcn2_forward_launches(const agcn_gcn2 *fwd, int *launches);
+int agcn_gcn2_forward_paired(const agcn_gcn2 *fwd, int *paired);
 int agcn_gcn2_forward_destroy(agcn_gcn2 *fwd);
 
 /* ------------------------------------------------------------------------

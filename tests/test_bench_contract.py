@@ -29,3 +29,13 @@ def test_other_ranks_of_the_reference_arm_exit_quietly():
                           "--gpus", "2"], capture_output=True, text=True, timeout=120,
                          env={**os.environ, "RANK": "1", "WORLD_SIZE": "2", "LOCAL_RANK": "1", "CUDA_VISIBLE_DEVICES": ""})
     assert out.returncode == 0 and out.stdout.strip() == ""
+
+
+def test_roofline_of_the_transforms():
+    sys.path.insert(0, ROOT)
+    import bench
+    rows = 1_000_000
+    apart, paired = (bench.transform_roofline(p, 0.25, rows, 6000.0) for p in (False, True))
+    assert apart["kernel"] == "gemm_tf32_128_kernel" and paired["kernel"] == "gemm_tf32_pair_kernel"
+    assert apart["algorithmic_bytes_per_launch"] == 1024 * rows + 65536 and paired["algorithmic_bytes_per_launch"] == 1024 * rows + 131072
+    assert abs(apart["achieved"] - (1024 * rows + 65536) / 0.25e6) < 1e-6 and abs(paired["achieved"] - (1024 * rows + 131072) / 0.5e6) < 1e-6

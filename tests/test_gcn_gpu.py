@@ -256,7 +256,7 @@ def test_forward_on_both_sides_of_the_line(n, launches):
     out = fwd.forward(sh.to_block(x))
     torch.cuda.synchronize()
     times = fwd.status(timings=True)
-    assert fwd.launches() == launches and all(layer[0] > 0 and layer[2] > 0 for layer in times)
+    assert fwd.launches() == launches and fwd.paired() == (launches == 3) and all(layer[0] > 0 and layer[2] > 0 for layer in times)
 
     def times_a(h):
         return (h[ix.long()] * v.double()[:, None]).view(n, 5, 128).sum(dim=1)
@@ -390,13 +390,14 @@ def test_forward_with_fused_layer_boundary(monkeypatch):
     want = plain.forward(xb).clone()
     torch.cuda.synchronize()
     plain.status()
-    plain_nodes = _captured_nodes(plain, xb)
+    plain_nodes, plain_paired = _captured_nodes(plain, xb), plain.paired()
     plain.close()
     monkeypatch.setenv("AGCN_GCN_FUSED", "1")
     fused = gcn.GcnForward(sh, [w1, w2])
     got = fused.forward(xb)
     torch.cuda.synchronize()
     fused.status()
+    assert plain_paired == (g.n >= 32_768) and not fused.paired()
     assert _captured_nodes(fused, xb) > plain_nodes        # the fused path is really taken at this size
     scale = float(want.abs().max())
     assert float((got - want).abs().max()) <= 2e-3 * scale
