@@ -122,8 +122,10 @@ static bool spmm_many_units(const agcn_spmm_plan *p) { return !p->split && p->n_
 // Whether a pass of `width` columns (a multiple of 8) loads rows of X 32 bytes per lane: half the load instructions, two rows
 // with each where they have 65 to 128 columns, and more bytes in flight.  It gains where the 16-byte lanes of a slot are not
 // all used or, beyond 64 columns, where the gather comes from L2; rows of 64 and 128 columns otherwise keep HBM or the ports
-// of L2 as busy 16 bytes at a time.  It never gains up to 32 columns (4-25 % slower).  (A rule on plan and width alone: the
-// additions inside a row of more than 32 nonzeros come in another order, and a product issued in parts has the whole one's bits.)
+// of L2 as busy 16 bytes at a time.  It never gains up to 32 columns (4-25 % slower), and gains although its forms spill 12 to 24
+// bytes of registers (three gathers at four blocks do not: 1-9 % slower).  The additions inside a row of more than 32 nonzeros come in
+// another order.  This is the rule on plan and width; rows of X have to begin on 32-byte boundaries as well (spmm_run_prepared), so
+// the same values in rows that do and in rows that do not can give other bits.  A product issued in parts has the whole one's.
 // Time with / without, B200.  More than 20 units per SM, 250 000 dense rows of 490, 500 000 skewed of 30, 500 000 power law of
 // 12, 2.4 M of 25, 1 M of 8: dim 40: .96 .95 .97 .98 .96;  48: .97 .97 .97 .98 .97;  56: .98 1.02 .99 - .99;  64: 1.00 1.01 .96
 // 1.00 .98;  72: .88 .94 .93 .95 .94;  80: .85 .96 .93 - .94;  88: .91 1.00 - - -;  96: .92 1.02 1.01 .94 1.02;  112: .95 1.00

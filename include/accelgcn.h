@@ -146,10 +146,12 @@ int agcn_degree_sort_host(const int32_t *h_indptr, const int32_t *h_indices, con
  * Unlike the reference kernel, which accumulates into Y with atomicAdd for
  * rows of degree >= 33 and never writes rows of degree 0 (:82-98), run
  * overwrites all of Y and does not read it; results are bit-identical from
- * run to run.  Any dim >= 1 (the reference harness sweeps every dim 16..128,
+ * run to run.  (Between layouts of X they need not be: rows of more than 32
+ * nonzeros may be summed in another order where rows of X do not begin on
+ * 32-byte boundaries.)  Any dim >= 1 (the reference harness sweeps every dim 16..128,
  * main.cu:12,137).  Rows of X are gathered 16 bytes per lane; when they are not
  * 16-byte aligned (dim % 4 != 0 with ld = dim, an odd stride or base) X is first
- * copied (by small products: read as it is, with the same result) into plan-owned aligned rows (grown on demand: the first such call of
+ * copied (by small products and of an X that is named a few times: read as it is, with the same result) into plan-owned aligned rows (grown on demand: the first such call of
  * a width allocates, so make it before a stream capture, and the widest one
  * before the first capture: growing moves the rows; AGCN_SPMM_PAD=0 at plan creation selects 4-byte gathers
  * instead) and unaligned rows of Y get stores as wide as each row's alignment allows.  dim > 64 may run

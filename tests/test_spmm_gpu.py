@@ -974,6 +974,31 @@ def test_rows_of_x_32_bytes_at_a_time(uncut, dim):
         assert np.array_equal(np.flatnonzero(odd.any(axis=1)), touched)
 
 
+@pytest.mark.parametrize("dim", [40, 48, 64, 72, 88, 96, 128])
+def test_bits_by_where_rows_of_x_begin(uncut, dim):
+    # rows of X on 32-byte boundaries, and unaligned ones that are copied onto such, give one result whatever their stride; rows on
+    # other 16-byte boundaries give one, too; rows of up to 32 nonzeros are the same in both
+    import torch
+    g = uncut
+    n, cols = g["n"], g["cols"]
+    xs = torch.from_numpy(np.random.default_rng(dim).standard_normal((cols, dim)).astype(np.float32)).to(g["dev"])
+
+    def product(shift, ldx):
+        x = torch.full((cols * ldx + shift,), float("nan"), device=g["dev"])[shift:]
+        x.view(cols, ldx)[:, :dim] = xs
+        y = torch.empty((n, dim), device=g["dev"])
+        g["plan"].run(g["d_idx"], g["d_val"], x, y, dim=dim, ldx=ldx, ldy=dim)
+        return y
+
+    eights, quads = product(0, dim), product(4, dim)
+    for shift, ldx in ((8, dim), (0, dim + 8), (1, dim), (2, dim + 1)):
+        assert torch.equal(product(shift, ldx), eights), (shift, ldx)
+    for shift, ldx in ((0, dim + 4), (12, dim), (4, dim + 8)):
+        assert torch.equal(product(shift, ldx), quads), (shift, ldx)
+    short = torch.from_numpy(np.diff(g["indptr"]) <= 32).to(g["dev"])
+    assert torch.equal(eights[short], quads[short])
+
+
 @pytest.mark.parametrize("dim", [33, 36, 61, 99, 123])
 def test_large_products_of_an_x_that_is_named_a_few_times(dim):
     # an X of 0.4 of L2 or more with up to eight nonzeros per row is read as it is, whatever its alignment, also by uncut plans:
