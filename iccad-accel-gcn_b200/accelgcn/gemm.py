@@ -64,6 +64,14 @@ def selftest_timeout(h, w, out, stream=None) -> int:
                                                    h.shape[0], s.cuda_stream)
 
 
+def pair_selftest_timeout(p, w1, w2, out, stream=None) -> int:
+    """The same for the pair of transforms (agcn_gemm_tf32_pair_selftest_timeout)."""
+    import torch
+    s = stream if stream is not None else torch.cuda.current_stream(p.device)
+    with torch.cuda.device(p.device):
+        return _lib.load().agcn_gemm_tf32_pair_selftest_timeout(p.data_ptr(), w1.data_ptr(), w2.data_ptr(), out.data_ptr(), p.shape[0], s.cuda_stream)
+
+
 def gcn_fused_layer(indptr, indices, vals, z_in, w, m_rows, out=None, status=None, stream=None):
     """Z2[r] = relu(A[r, :] @ Z1) @ W for the first m_rows rows of a CSR matrix, all of at most 32
     nonzeros (agcn_gcn_fused_layer): the activations stay in shared memory between the gather and the

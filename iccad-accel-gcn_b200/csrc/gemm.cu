@@ -113,14 +113,9 @@ static int gemm_status_word(int **out)
     return AGCN_OK;
 }
 
-static int gemm_tf32_sync(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
-                          int k_dim, int n_dim, cudaStream_t s, uint32_t spin_limit, int skip_first_load)
+// Waits for the stream and says what a launch on it has left in the status word.
+static int gemm_status_read(const int *d_status, cudaStream_t s)
 {
-    int *d_status = nullptr;
-    int rc = gemm_status_word(&d_status);
-    if (rc != AGCN_OK) return rc;
-    rc = gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, k_dim, n_dim, d_status, s, spin_limit, skip_first_load);
-    if (rc != AGCN_OK) return rc;
     int status = 0;
     AGCN_CUDA(cudaMemcpyAsync(&status, d_status, sizeof(int), cudaMemcpyDeviceToHost, s));
     AGCN_CUDA(cudaStreamSynchronize(s));
@@ -131,15 +126,25 @@ static int gemm_tf32_sync(const float *d_h, int64_t ldh, const float *d_w, float
     return AGCN_OK;
 }
 
+static int gemm_tf32_sync(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
+                          int k_dim, int n_dim, cudaStream_t s, uint32_t spin_limit, int skip_first_load)
+{
+    int *d_status = nullptr;
+    int rc = gemm_status_word(&d_status);
+    if (rc != AGCN_OK) return rc;
+    rc = gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, k_dim, n_dim, d_status, s, spin_limit, skip_first_load);
+    return rc != AGCN_OK ? rc : gemm_status_read(d_status, s);
+}
+
 int gemm_tf32_async(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz, int64_t m_rows,
                     int *d_status, cudaStream_t s, bool keep_status, bool early, unsigned long long *d_stamp)
 {
     return gemm_tf32_launch(d_h, ldh, d_w, d_z, ldz, m_rows, GEMM_DIM, GEMM_DIM, d_status, s, GEMM_SPIN_LIMIT, 0, keep_status, early, d_stamp);
 }
 
-// keep_status, early, d_stamp: as for gemm_tf32_launch
+// spin_limit, skip_first_load, keep_status, early, d_stamp: as for gemm_tf32_launch
 static int gemm_pair_launch(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, int *d_status, cudaStream_t s,
-                            bool keep_status, bool early, unsigned long long *d_stamp)
+                            uint32_t spin_limit, int skip_first_load, bool keep_status = false, bool early = false, unsigned long long *d_stamp = nullptr)
 {
     AGCN_REQUIRE(d_p != nullptr && d_w1 != nullptr && d_w2 != nullptr && d_z != nullptr && d_status != nullptr, "agcn_gemm_tf32_pair: null pointer");
     AGCN_REQUIRE(m_rows >= 0 && m_rows < ((int64_t)1 << 31) * GEMM_TILE_M / 2, "agcn_gemm_tf32_pair: row count out of range");
@@ -156,7 +161,7 @@ static int gemm_pair_launch(const float *d_p, const float *d_w1, const float *d_
     const int n_tiles = (int)ceil_div(m_rows, GEMM_TILE_M);
     const int grid = n_tiles < sm_count ? n_tiles : sm_count;
     AGCN_CUDA(launch_early(early, gemm_tf32_pair_kernel, (unsigned)grid, PAIR_THREADS, PAIR_SMEM_BYTES, s, map, d_w1, d_w2, d_z, m_rows, n_tiles,
-                           d_status, GEMM_SPIN_LIMIT, d_stamp));
+                           d_status, spin_limit, skip_first_load, d_stamp));
     AGCN_LAUNCH_CHECK("gemm_tf32_pair_kernel");
     return AGCN_OK;
 }
@@ -164,7 +169,7 @@ static int gemm_pair_launch(const float *d_p, const float *d_w1, const float *d_
 int gemm_pair_async(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, int *d_status, cudaStream_t s,
                     unsigned long long *d_stamp)
 {
-    return gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, s, true, true, d_stamp);
+    return gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, s, GEMM_SPIN_LIMIT, 0, true, true, d_stamp);
 }
 
 }  // namespace agcn
@@ -189,7 +194,8 @@ extern "C" int agcn_gemm_tf32_pair_async(const float *d_p, const float *d_w1, co
                                          int32_t *d_status, void *stream)
 {
     agcn::clear_error();
-    return agcn::gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, static_cast<cudaStream_t>(stream), false, false, nullptr);
+    return agcn::gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, static_cast<cudaStream_t>(stream),
+                                  agcn::GEMM_SPIN_LIMIT, 0);
 }
 
 extern "C" int agcn_gemm_tf32_selftest_timeout(const float *d_h, int64_t ldh, const float *d_w, float *d_z, int64_t ldz,
@@ -199,6 +205,17 @@ extern "C" int agcn_gemm_tf32_selftest_timeout(const float *d_h, int64_t ldh, co
     // 4096 polls of about 100 ns: the starved wait gives up after well under a millisecond
     return agcn::gemm_tf32_sync(d_h, ldh, d_w, d_z, ldz, m_rows, agcn::GEMM_DIM, agcn::GEMM_DIM,
                                 static_cast<cudaStream_t>(stream), 4096u, 1);
+}
+
+extern "C" int agcn_gemm_tf32_pair_selftest_timeout(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, void *stream)
+{
+    agcn::clear_error();
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    int *d_status = nullptr;
+    int rc = agcn::gemm_status_word(&d_status);
+    if (rc != AGCN_OK) return rc;
+    rc = agcn::gemm_pair_launch(d_p, d_w1, d_w2, d_z, m_rows, d_status, s, 4096u, 1);
+    return rc != AGCN_OK ? rc : agcn::gemm_status_read(d_status, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -108,10 +108,10 @@ gcn_fused_layer_kernel(const int *__restrict__ indptr, const int *__restrict__ i
         // ---- epilogue warps -------------------------------------------------------------------
         const int q = warp & 3;                                // TMEM lane quarter this warp may read
         float *patch = s_patch + (warp - 2) * (GEMM_PATCH_BYTES / 4);
-        for (int it = 0; it < my_tiles && !*s_abort; it++) {
+        for (int it = 0; it < my_tiles; it++) {
             const int tile = (int)blockIdx.x + it * (int)gridDim.x;
             const uint32_t acc = it & 1, acc_ph = (it >> 1) & 1;
-            if (!mbar_wait(smem_u32(&bar_acc_full[acc]), acc_ph, s_abort, spin_limit)) {
+            if (!mbar_wait_warp(smem_u32(&bar_acc_full[acc]), acc_ph, s_abort, spin_limit)) {
                 if (!*s_abort) { atomicExch(err_flag, GEMM_ERR_TIMEOUT_EPILOGUE); *s_abort = 1; }
                 break;
             }

@@ -66,9 +66,9 @@ __device__ __forceinline__ float to_tf32(float v)
 
 __global__ void __launch_bounds__(PAIR_THREADS, 1)
 gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap map_p, const float *__restrict__ w1, const float *__restrict__ w2, float *__restrict__ z,
-                      int64_t m_rows, int n_tiles, int *__restrict__ err_flag, uint32_t spin_limit, unsigned long long *stamp)
+                      int64_t m_rows, int n_tiles, int *__restrict__ err_flag, uint32_t spin_limit, int skip_first_load, unsigned long long *stamp)
 {
-    // err_flag, spin_limit, stamp: as in gemm_tf32_128_kernel
+    // err_flag, spin_limit, skip_first_load, stamp: as in gemm_tf32_128_kernel
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
     uint8_t *s_w1 = smem, *s_w2 = smem + GEMM_W_BYTES;             // 64 KiB each, K-major, swizzled
@@ -130,6 +130,7 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap map_p, const float *__
                 for (int kb = 0; kb < GEMM_KBLKS; kb++, g++) {
                     const uint32_t s = g % PAIR_STAGES, ph = (g / PAIR_STAGES) & 1;
                     if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, s_abort, spin_limit)) { give_up(GEMM_ERR_TIMEOUT_PRODUCER); break; }
+                    if (skip_first_load && g == 0) continue;      // self-test: this stage never fills
                     mbar_arrive_expect_tx(smem_u32(&bar_full[s]), GEMM_STAGE_BYTES);
                     tma_load_2d(smem_u32(s_ring + s * GEMM_STAGE_BYTES), &map_p, kb * GEMM_KBLK, tile * GEMM_TILE_M, smem_u32(&bar_full[s]));
                 }
@@ -190,9 +191,9 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap map_p, const float *__
     } else if (warp < 2 + GEMM_EPI_WARPS) {
         // ---- the activation ---------------------------------------------------------------------
         const uint32_t quarter = (uint32_t)((warp & 3) * 32) << 16;                 // TMEM lane quarter this warp may use
-        for (int it = 0; it < my_tiles && !*s_abort; it++) {
+        for (int it = 0; it < my_tiles; it++) {
             const uint32_t b = it & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_sum_full[b]), (it >> 1) & 1, s_abort, spin_limit))) { give_up(GEMM_ERR_TIMEOUT_EPILOGUE); break; }
+            if (!mbar_wait_warp(smem_u32(&bar_sum_full[b]), (it >> 1) & 1, s_abort, spin_limit)) { give_up(GEMM_ERR_TIMEOUT_EPILOGUE); break; }
             tc_fence_after();
 #pragma unroll 1
             for (int c = 0; c < GEMM_DIM / 32; c++) {
@@ -212,10 +213,10 @@ gemm_tf32_pair_kernel(const __grid_constant__ CUtensorMap map_p, const float *__
         // ---- epilogue: as in gemm_tf32_128_kernel -----------------------------------------------
         const int q = warp & 3;
         float *patch = s_patch + (warp - 2 - GEMM_EPI_WARPS) * (GEMM_PATCH_BYTES / 4);
-        for (int it = 0; it < my_tiles && !*s_abort; it++) {
+        for (int it = 0; it < my_tiles; it++) {
             const int tile = (int)blockIdx.x + it * (int)gridDim.x;
             const uint32_t b = it & 1;
-            if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(&bar_acc_full[b]), (it >> 1) & 1, s_abort, spin_limit))) { give_up(GEMM_ERR_TIMEOUT_EPILOGUE); break; }
+            if (!mbar_wait_warp(smem_u32(&bar_acc_full[b]), (it >> 1) & 1, s_abort, spin_limit)) { give_up(GEMM_ERR_TIMEOUT_EPILOGUE); break; }
             tc_fence_after();
             const int64_t row0 = (int64_t)tile * GEMM_TILE_M + q * 32;
 #pragma unroll 1

@@ -78,6 +78,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
     return false;
 }
+// The same by all lanes of a warp, with one answer for all of them: they go on, or leave, together (what follows are votes,
+// loads from tensor memory and synchronisations of whole warps).  Between such waits no lane looks at the abort flag by itself.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int *abort_flag, uint32_t spin_limit)
+{
+    return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, spin_limit)) != 0;
+}
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -306,10 +312,10 @@ gemm_tf32_128_kernel(const __grid_constant__ CUtensorMap map_h, const float *__r
         // ---- epilogue warps -------------------------------------------------------------------
         const int q = warp & 3;                                // TMEM lane quarter this warp may read
         float *patch = s_patch + (warp - 2) * (GEMM_PATCH_BYTES / 4);
-        for (int it = 0; it < my_tiles && !*s_abort; it++) {
+        for (int it = 0; it < my_tiles; it++) {
             const int tile = (int)blockIdx.x + it * (int)gridDim.x;
             const uint32_t acc = it & 1, acc_ph = (it >> 1) & 1;
-            if (!mbar_wait(smem_u32(&bar_acc_full[acc]), acc_ph, s_abort, spin_limit)) {
+            if (!mbar_wait_warp(smem_u32(&bar_acc_full[acc]), acc_ph, s_abort, spin_limit)) {
                 if (!*s_abort) { atomicExch(err_flag, GEMM_ERR_TIMEOUT_EPILOGUE); *s_abort = 1; }
                 break;
             }

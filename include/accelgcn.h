@@ -263,6 +263,8 @@ int agcn_gemm_tf32_pair_async(const float *d_p, const float *d_w1, const float *
  * run out.  The device stays usable: the next agcn_gemm_tf32 must succeed. */
 int agcn_gemm_tf32_selftest_timeout(const float *d_h, int64_t ldh, const float *d_w, float *d_z,
                                     int64_t ldz, int64_t m_rows, void *stream);
+/* The same of agcn_gemm_tf32_pair_async. */
+int agcn_gemm_tf32_pair_selftest_timeout(const float *d_p, const float *d_w1, const float *d_w2, float *d_z, int64_t m_rows, void *stream);
 
 /* One GCN layer boundary in one kernel, for rows of at most 32 nonzeros (no counterpart in the
  * reference, which stops at the SpMM, spmm_accel.cu:104-108):

@@ -142,6 +142,25 @@ def test_gemm_bounded_wait_runs_out_and_the_next_call_succeeds():
         _check_gemm(h.cpu().numpy(), w.cpu().numpy(), z2.cpu().numpy())
 
 
+@pytest.mark.parametrize("m", [1, 128 * 5, 128 * 700 + 9])
+def test_bounded_wait_of_the_pair_of_transforms_runs_out_and_the_next_call_succeeds(m):
+    # the same for the kernel that makes both, thread blocks with one tile and with several: all its warps leave, whichever of
+    # them gives up first
+    import torch
+    from accelgcn import gemm, synth, _lib
+    dev = require_cuda()
+    p, z = synth.features(m, 128, 4, dev), torch.zeros((m, 128), device=dev)
+    w1, w2 = (synth.glorot(128, 128, 5, k, dev) for k in (8, 9))
+    status = torch.full((1,), 9, dtype=torch.int32, device=dev)
+    want = torch.empty_like(z)
+    gemm.gemm_tf32_pair_async(p, w1, w2, want, status)
+    for _ in range(5):
+        assert gemm.pair_selftest_timeout(p, w1, w2, z) == _lib.ERR_CUDA and b"ran out" in _lib.load().agcn_last_error()
+        gemm.gemm_tf32_pair_async(p, w1, w2, z, status)
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0 and torch.equal(z, want)
+
+
 @pytest.mark.parametrize("m", [1, 128 * 5, 128 * 300])
 def test_gemm_error_of_any_thread_block_is_reported_every_time(m):
     # the status word is zeroed on the stream and not by a thread block of the launch that may report into it
