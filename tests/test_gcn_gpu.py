@@ -285,6 +285,39 @@ def test_forward_on_both_sides_of_the_line(n, launches):
     fwd.close(); sh.close()
 
 
+@pytest.mark.parametrize("n,mean", [(32_768, 8), (40_000, 20), (250_000, 12)])
+def test_paired_forward_is_its_three_calls_in_turn(n, mean):
+    # plans that cut their tuples and plans that do not, hub rows, W written right before the forward: the bits of A X,
+    # agcn_gemm_tf32_pair_async and relu(A Z) called one after the other, from run to run and with the result in place of X
+    import torch
+    from accelgcn import synth, sharded, gcn, gemm, degree_sort, partition, spmm
+    dev = require_cuda()
+    g = synth.chung_lu("powerlaw", n, synth.power_law_weights(n, 2.2, float(mean), n / 4), n * mean, 1, dev)
+    _, ip, ix, v = degree_sort.degree_sort_device(g.indptr, g.indices, g.vals, relabel_cols=True)
+    x = synth.features(n, 128, 3, dev)
+    w1, w2 = (synth.glorot(128, 128, 3, k, dev) for k in (8, 9))
+    plan = spmm.SpmmPlan(partition.block_level_partition_device(ip), ix, n, n)
+    p, z, want = (torch.full_like(x, float("nan")) for _ in range(3))
+    status = torch.full((1,), 9, dtype=torch.int32, device=dev)
+    plan.run(ix, v, x, p)
+    gemm.gemm_tf32_pair_async(p, w1, w2, z, status)
+    plan.run(ix, v, z, want, relu=True)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    plan.close()
+    sh = sharded.ShardedSpmm(ip, ix, v, 0, 1)
+    late = [torch.zeros_like(w1), torch.zeros_like(w2)]
+    fwd = gcn.GcnForward(sh, late)
+    block = sh.to_block(x)
+    for _ in range(3):
+        for t, w in zip(late, (w1, w2)):
+            t.fill_(float("nan"))
+            t.copy_(w)
+        assert torch.equal(fwd.forward(block)[:n], want) and fwd.paired()
+    assert torch.equal(fwd.forward(block, out=block)[:n], want)
+    fwd.status(); fwd.close(); sh.close()
+
+
 def test_two_layer_gcn_forward_at_five_million_nodes():
     # configuration 5 at a tenth of its size (N = 5 000 000, ~1.07e8 nonzeros, 128 features): the whole
     # native forward against the CPU forward.  Tolerance: TF32 keeps 10 mantissa bits per operand of
