@@ -115,29 +115,14 @@ static bool spmm_wide_form(const agcn_spmm_plan *p, int width)
 // (Passes of up to 32 columns were not measured and have no such kernel.)
 constexpr double SPMM_HOT_X = 6.0, SPMM_HOT_L2 = 0.45, SPMM_HOT_SHARE = 0.33;
 
-// Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM), where a second
-// launch costs more than blocks that wait for a counter.
-static bool spmm_many_units(const agcn_spmm_plan *p) { return !p->split && p->n_units > (int64_t)20 * p->sm_count; }
-
-// Whether a pass of `width` columns (a multiple of 8) loads rows of X 32 bytes per lane: half the load instructions, two rows
-// with each where they have 65 to 128 columns, and more bytes in flight.  It gains where the 16-byte lanes of a slot are not
-// all used or, beyond 64 columns, where the gather comes from L2; rows of 64 and 128 columns otherwise keep HBM or the ports
-// of L2 as busy 16 bytes at a time.  It never gains up to 32 columns (4-25 % slower), and gains although its forms spill 12 to 24
-// bytes of registers (three gathers at four blocks do not: 1-9 % slower).  The additions inside a row of more than 32 nonzeros come in
-// another order.  This is the rule on plan and width; rows of X have to begin on 32-byte boundaries as well (spmm_run_prepared), so
-// the same values in rows that do and in rows that do not can give other bits.  A product issued in parts has the whole one's.
-// Time with / without, B200.  More than 20 units per SM, 250 000 dense rows of 490, 500 000 skewed of 30, 500 000 power law of
-// 12, 2.4 M of 25, 1 M of 8: dim 40: .96 .95 .97 .98 .96;  48: .97 .97 .97 .98 .97;  56: .98 1.02 .99 - .99;  64: 1.00 1.01 .96
-// 1.00 .98;  72: .88 .94 .93 .95 .94;  80: .85 .96 .93 - .94;  88: .91 1.00 - - -;  96: .92 1.02 1.01 .94 1.02;  112: .95 1.00
-// .97 - .98;  128: .98 1.02 1.00 1.02 .98.
-// Fewer, 60 000 dense of 150, 150 000 power law of 10, 200 000 of 20, 100 000 skewed of 20 (in the form of five blocks): 40:
-// .98 .99 1.02 .97;  64: 1.00 .99 1.00 1.05;  72: .96 .96 .96 .93;  80: .96 .97 - .95;  96: .97 .97 - .98;  112: .99 .98 - 1.05;
-// 128: .99 .97 .99 1.04.
-static bool spmm_octets(const agcn_spmm_plan *p, int width)
+static UncutPlan spmm_uncut(const agcn_spmm_plan *p, int width)
 {
-    if (p->split || p->panel_override != 0 || width <= 32) return false;
-    if (spmm_many_units(p)) return width <= 48 || (width > 64 && (width <= 88 || p->nnz >= 250 * p->n_blocks));
-    return width > 64 && (width <= 96 || !spmm_wide_form(p, width));
+    return UncutPlan{p->n_units, p->n_blocks, p->nnz, spmm_wide_form(p, width), p->sm_count};
+}
+static bool spmm_many_units(const agcn_spmm_plan *p) { return !p->split && spmm_many_units(p->n_units, p->sm_count); }
+static bool spmm_octets(const agcn_spmm_plan *p, int width, int columns)
+{
+    return !p->split && p->panel_override == 0 && spmm_octets(spmm_uncut(p, width), width, columns);
 }
 
 static int64_t hot_rows(const agcn_spmm_plan *p, int width) { return (int64_t)(SPMM_HOT_L2 * p->l2_bytes / (width * 4.0)); }
@@ -509,7 +494,7 @@ static bool spmm_loose(const agcn_spmm_plan *p, int dim)
     if (!p->split) {
         // rows of whole eights keep the order of additions that the same columns have where they are aligned
         if (dim > SPMM_PANEL || p->nnz > (dim > 32 ? 8 : 6) * p->n_cols || (double)p->n_cols * dim * 4.0 < SPMM_LOOSE_L2 * p->l2_bytes) return false;
-        return dim % 8 != 0 || !spmm_octets(p, dim);
+        return dim % 8 != 0 || !spmm_octets(p, dim, dim);
     }
     return (spmm_deep(p) && p->nnz <= (int64_t)500 * p->sm_count) || (p->nnz <= 13 * p->n_cols && p->nnz <= (int64_t)2700 * p->sm_count);
 }
@@ -641,7 +626,7 @@ int spmm_run_prepared(agcn_spmm_plan *p, const int *d_indices, const float *d_va
         prm.dim_store = width;
         prm.dim = vec ? (width + 3) & ~3 : width;       // columns gathered (the padded copy holds zeros past dim)
         // (not for the copy of an X that a whole product reads as it is: one issued in parts has the same bits)
-        const bool octets = vec && !loose && prm.dim % 8 == 0 && ldx_use % 8 == 0 && aligned32(prm.x) && spmm_octets(p, prm.dim) &&
+        const bool octets = vec && !loose && prm.dim % 8 == 0 && ldx_use % 8 == 0 && aligned32(prm.x) && spmm_octets(p, prm.dim, width) &&
                             (dim % 4 == 0 || p->never_split || !spmm_loose(p, dim));
         const bool plain = !accumulate && !loose && (vec ? y_vec : true) && (!octets || (width % 8 == 0 && ldy % 8 == 0 && aligned32(prm.y)));
         if (grid > 0) {

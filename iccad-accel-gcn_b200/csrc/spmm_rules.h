@@ -26,6 +26,52 @@ int plan_faults(const Words &words, int64_t most_pieces)
     return err == 0 && words[PLAN_WORD_PIECES] > most_pieces ? SPMM_ERR_PIECES : err;
 }
 
+// What a rule may ask of an uncut plan.
+struct UncutPlan {
+    int64_t n_units, n_blocks, nnz;
+    bool wide;                // 16-byte loads would take the form of five blocks per SM at this width (spmm_wide_form)
+    int sm_count;
+};
+
+// Rows that cross units are finished inside the launch while it is a few waves of thread blocks (5 per SM), where a second
+// launch costs more than blocks that wait for a counter.
+inline bool spmm_many_units(int64_t n_units, int sm_count) { return n_units > (int64_t)20 * sm_count; }
+
+// Whether a pass that gathers `width` columns (a multiple of 8) and stores `columns` of them loads rows of X 32 bytes per lane:
+// half the load instructions, two rows with each where they have 65 to 128 columns, and more bytes in flight.  It gains where the 16-byte lanes of a slot are not
+// all used or, beyond 64 columns, where the gather comes from L2; rows of 64 and 128 columns otherwise keep HBM or the ports
+// of L2 as busy 16 bytes at a time.  It never gains up to 32 columns (4-25 % slower), and gains although its forms spill 12 to 24
+// bytes of registers (three gathers at four blocks do not: 1-9 % slower).  The additions inside a row of more than 32 nonzeros come in
+// another order.  This is the rule on plan and width; rows of X have to begin on 32-byte boundaries as well (spmm_run_prepared), so
+// the same values in rows that do and in rows that do not can give other bits.  A product issued in parts has the whole one's.
+// Time with / without, B200.  More than 20 units per SM, 250 000 dense rows of 490, 500 000 skewed of 30, 500 000 power law of
+// 12, 2.4 M of 25, 1 M of 8: dim 40: .96 .95 .97 .98 .96;  48: .97 .97 .97 .98 .97;  56: .98 1.02 .99 - .99;  64: 1.00 1.01 .96
+// 1.00 .98;  72: .88 .94 .93 .95 .94;  80: .85 .96 .93 - .94;  88: .91 1.00 - - -;  96: .92 1.02 1.01 .94 1.02;  112: .95 1.00
+// .97 - .98;  128: .98 1.02 1.00 1.02 .98.  Dense, up to 48 columns, not taken up to 40 units per SM, [26] 60 000 of 150, [30] 100 000 of 100, [33] 30 000
+// of 400, [34] 40 000 of 300, dims 37, 40, 45, 48: 1.01 1.00 1.02 1.00, 1.00 .99 1.01 1.00, 1.02 1.01 1.02 1.01, 1.00 1.00 1.01 1.00;  taken, [43] 60 000 of 250: .99
+// .98 1.00 .99.  (The largest loss that is left: 300 000 power law of 15 [26], dims 40, 45, 48: 1.02 1.02 1.00.)
+// Fewer, 60 000 dense of 150, 150 000 power law of 10, 200 000 of 20, 100 000 skewed of 20 (in the form of five blocks): 40:
+// .98 .99 1.02 .97;  64: 1.00 .99 1.00 1.05;  72: .96 .96 .96 .93;  80: .96 .97 - .95;  96: .97 .97 - .98;  112: .99 .98 - 1.05;
+// 128: .99 .97 .99 1.04.  Dense, not taken up to 11.5 units per SM (the last round of blocks is a good part of them), [6.7] 13 000 of 180, [7.9] 10 000 of
+// 250, [9.6] 8 000 of 400, [10.8] 9 000 of 400, dims 72, 88, 96, 112, 128: 1.06 1.05 1.06 1.04 1.03, 1.04 1.04 1.04 1.03 1.02, 1.05 1.05 1.06 1.05 1.03, 1.02 1.03 1.04
+// 1.03 1.01;  taken, [14] 20 000 of 250, [18] 60 000 of 100: .97 .98 .98 .98 .98, .96 .95 .96 .98 .98.
+// Fewer and not dense: 97 to 128 columns that are no multiple of 4, whose rows of Y are stored element by element, not taken, 90 000 power law of
+// 12, 120 000 of 10, 150 000 of 20, 80 000 skewed of 20, 150 000 of 12, dims 103, 109, 119, 127: 1.04 1.07 1.08 1.09, 1.03 1.06 1.07 1.08, 1.01 1.03 1.04 1.05, 1.02 1.05
+// 1.07 1.07, 1.01 1.04 1.05 1.08;  such up to 96, taken, the same, dims 69, 77, 85, 93: .95 .98 1.01 1.00, .94 .97 1.00 1.01, .97 .98 .99 .99, .88 .91 .94 .97, .92 .94
+// .96 .98.  (Left: 60 000 skewed of 25, dims 112, 120, 128: 1.00 1.01 1.02, and rows of Y that are unaligned by base or stride alone, which the rule does
+// not look at, so that bits do not depend on Y.)
+inline bool spmm_octets(const UncutPlan &p, int width, int columns)
+{
+    const bool dense = p.nnz >= 250 * p.n_blocks;
+    if (width <= 32) return false;
+    if (spmm_many_units(p.n_units, p.sm_count)) {
+        if (width <= 48) return !dense || p.n_units > (int64_t)40 * p.sm_count;
+        return width > 64 && (width <= 88 || dense);
+    }
+    if (width <= 64 || (dense && 2 * p.n_units <= (int64_t)23 * p.sm_count)) return false;
+    return width <= 96 || (!p.wide && (dense || columns % 4 == 0));
+}
+
 // What a rule may ask of a cut plan.
 struct CutPlan {
     int64_t n_units, n_rows, nnz;

@@ -16,12 +16,14 @@ def rules(tmp_path_factory):
     src = d / "rules.cpp"
     src.write_text("""#include "spmm_rules.h"
 extern "C" int few_form(int64_t units, int64_t rows, int64_t nnz, int64_t longest, int sm, int width) { return agcn::spmm_few_form({units, rows, nnz, longest, sm}, width); }
+extern "C" int octets(int64_t units, int64_t nnz, int wide, int sm, int width, int columns) { return agcn::spmm_octets({units, 8 * units, nnz, wide != 0, sm}, width, columns); }
 extern "C" int faults(const int64_t *words, int64_t most) { return agcn::plan_faults(words, most); }
 """)
     lib = str(d / "librules.so")
     subprocess.check_call(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-I" + os.path.join(PKG, "csrc"), str(src), "-o", lib])
     dll = ctypes.CDLL(lib)
     dll.few_form.argtypes = [ctypes.c_int64] * 4 + [ctypes.c_int, ctypes.c_int]
+    dll.octets.argtypes = [ctypes.c_int64] * 2 + [ctypes.c_int] * 4
     dll.faults.argtypes = [ctypes.POINTER(ctypes.c_int64), ctypes.c_int64]
     return dll
 
@@ -57,6 +59,32 @@ def test_three_blocks_per_sm_where_they_were_measured_faster(rules, graph):
     for width in (16, 20, 32, 33, 60, 64, 65, 100, 128):
         form = rules.few_form(units, rows, nnz, longest, SM, width)
         assert form == (3 if width <= widest else 4), width
+
+
+# thread blocks, nonzeros, the widths that were measured faster with 32-byte loads or no slower, those that were slower
+OCTETS = {
+    "dense 13000 x 180": (985, 2_340_000, (), (40, 64, 72, 88, 96, 112, 127, 128)),
+    "dense 10000 x 250": (1163, 2_500_000, (), (40, 72, 80, 96, 109, 128)),
+    "dense 9000 x 400": (1600, 3_600_000, (), (72, 93, 96, 104, 127)),
+    "dense 20000 x 250": (2077, 5_000_000, (72, 77, 88, 96, 103, 112, 127, 128), (40, 48, 64)),
+    "dense 60000 x 100": (2635, 6_000_000, (69, 85, 96, 109, 128), (40, 64)),
+    "dense 60000 x 150": (3899, 9_000_000, (69, 80, 96, 112, 128), (37, 40, 45, 48, 56, 64)),
+    "dense 60000 x 250": (6362, 15_000_000, (37, 40, 45, 48, 69, 88, 96, 128), (56, 64)),
+    "power law 90000 x 12": (1124, 1_170_000, (69, 72, 77, 93, 96, 104, 112, 120, 128), (40, 64, 101, 103, 109, 119, 125, 127)),
+    "power law 120000 x 10": (1445, 1_320_000, (72, 85, 96, 104, 128), (103, 110, 118, 126)),
+    "skewed 100000 x 30": (1916, 3_000_000, (69, 88, 96, 112, 128), (48, 109, 127)),
+    "power law 600000 x 15": (7731, 9_600_000, (37, 40, 48, 69, 72, 85, 88), (56, 64, 93, 96, 109, 128)),
+}
+
+
+@pytest.mark.parametrize("graph", OCTETS)
+def test_32_byte_loads_where_they_were_measured_faster(rules, graph):
+    units, nnz, faster, slower = OCTETS[graph]
+    for columns in faster + slower:
+        assert rules.octets(units, nnz, 0, SM, (columns + 7) // 8 * 8, columns) == (columns in faster), columns
+        # five blocks per SM otherwise: products of few units keep those from 97 columns on
+        if units <= 20 * SM and columns > 96:
+            assert not rules.octets(units, nnz, 1, SM, (columns + 7) // 8 * 8, columns), columns
 
 
 @pytest.mark.parametrize("words,most,faults", [
